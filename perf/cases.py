@@ -23,7 +23,7 @@ import sys
 import torch
 import torch.nn.functional as F
 
-sys.path.insert(0, os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "2by4-pretrain_b200"))
+sys.path.insert(0, os.path.join(os.getcwd(), "2by4-pretrain_b200"))      # the tree being measured is the working folder
 
 import sparse  # noqa: E402
 import train_gpt2  # noqa: E402
