@@ -87,6 +87,12 @@ __device__ __forceinline__ void tmem_relinquish() {
 __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t cols) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
 }
+// true in one lane of the (converged) warp
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(p));
+    return p != 0;
+}
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_commit(uint32_t bar) {
@@ -875,39 +881,44 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         }
     } else if (warp == 1) {
         // ---------------------------------------------------------------- MMA issuer (leader CTA only)
-        if (lane == 0 && rank == 0) {
+        // All 32 lanes walk the loop together, so that its counters, addresses and descriptors stay in uniform registers
+        // (the MMA takes all its operands from there); one elected lane issues.  Descriptors advance by an add to their
+        // address field.
+        if (rank == 0) {
             constexpr uint32_t A_LBO = A_MN ? 8192 : 16, A_KSTEP = A_MN ? 2048 : 32;
             const uint32_t idesc0 = P.idesc;   // M = 256, N = 192 set by the launcher
-            int g = 0, tl = 0;
+            const uint32_t smem0 = smem_u32(smem);
+            const uint64_t adesc0 = make_desc(smem0, A_LBO, 1024, 2), bdesc0 = make_desc(smem0 + OFF_B, 16, 1024, 2);
+            const uint64_t edesc0 = make_desc(smem0 + OFF_E, 16, 128, 0);
+            int s = 0, tl = 0;
+            uint32_t ph = 0, eslot = 0;
             bool ok = true;
             for (int tile = pair; tile < n_tiles && ok; tile += n_pairs, ++tl) {
                 const int buf = tl & 1;
+                const uint32_t acc = tmem_base + buf * BN;
                 // the epilogues of both CTAs must have drained this accumulator buffer (two tiles ago)
                 ok = mbar_wait(tmem_empty0 + 8 * buf, ((tl >> 1) & 1) ^ 1, &abort_flag, P.status, 4);
-                for (int it = 0; it < k_iters && ok; ++it, ++g) {
-                    const int s = g % STAGES;
-                    const uint32_t ph = (g / STAGES) & 1;
+                for (int it = 0; it < k_iters && ok; ++it) {
                     ok = mbar_wait(full0 + 8 * s, ph, &abort_flag, P.status, 2);
                     if (!ok) break;
-                    SP24_TRACE(1, 2 * g);
-                    const uint32_t sa = smem_u32(smem + (size_t)s * STAGE2_BYTES);
-                    const uint32_t sb = sa + OFF_B;
                     tc_fence_after();
-                    const uint32_t e_cols = E_COL0 + (g & 1) * E_SLOT;
-                    tc_cp_128x128b_pair(tmem_base + e_cols, make_desc(sa + OFF_E, 16, 128, 0));
+                    const uint32_t off = (uint32_t)s * (STAGE2_BYTES >> 4);
+                    const uint64_t ad = adesc0 + off, bd = bdesc0 + off, ed = edesc0 + off;
+                    const uint32_t e_cols = tmem_base + E_COL0 + eslot;
+                    if (elect_one()) {
+                        tc_cp_128x128b_pair(e_cols, ed);
 #pragma unroll
-                    for (int j = 0; j < KSTEPS; ++j) {
-                        const uint64_t adesc = make_desc(sa + j * A_KSTEP, A_LBO, 1024, 2);
-                        const uint32_t b_off = (uint32_t)(j >> 1) * ((BN / 2) * 128) + (j & 1) * 64;
-                        const uint64_t bdesc = make_desc(sb + b_off, 16, 1024, 2);
-                        const uint32_t ecol = e_cols + j;
-                        mma_sp_pair(tmem_base + buf * BN, adesc, bdesc, tmem_base + (ecol & ~1u), idesc0 | (ecol & 1u),
-                                    (it > 0 || j > 0) ? 1u : 0u);
+                        for (int j = 0; j < KSTEPS; ++j)
+                            mma_sp_pair(acc, ad + j * (A_KSTEP >> 4), bd + (((j >> 1) * ((BN / 2) * 128) + (j & 1) * 64) >> 4),
+                                        e_cols + (j & ~1), idesc0 | (j & 1), (it > 0 || j > 0) ? 1u : 0u);
+                        tc_commit_pair(empty0 + 8 * s);
                     }
-                    tc_commit_pair(empty0 + 8 * s);
-                    SP24_TRACE(1, 2 * g + 1);
+                    __syncwarp();
+                    eslot ^= E_SLOT;
+                    if (++s == STAGES) { s = 0; ph ^= 1; }
                 }
-                tc_commit_pair(tmem_full0 + 8 * buf);   // also arrives after an abort
+                if (elect_one()) tc_commit_pair(tmem_full0 + 8 * buf);   // also arrives after an abort
+                __syncwarp();
             }
         }
     } else {
@@ -1134,38 +1145,42 @@ spmm_pair_acc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         }
     } else if (warp == 1) {
         // ---------------------------------------------------------------- MMA issuer (leader CTA only)
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {                       // all lanes in step, one elected lane issues (as in spmm_pair_kernel)
             constexpr uint32_t A_LBO = A_MN ? 8192 : 16, A_KSTEP = A_MN ? 2048 : 32;
             const uint32_t idesc0 = P.idesc;   // M = 256, N = 256, B MN-major set by the launcher
-            int g = 0, tl = 0;
+            const uint32_t smem0 = smem_u32(smem);
+            // MN-major B: 64-column blocks 16384 bytes apart, 32 K-rows (4096 bytes) per MMA
+            const uint64_t adesc0 = make_desc(smem0, A_LBO, 1024, 2), bdesc0 = make_desc(smem0 + OFF_B, 16384, 1024, 2);
+            const uint64_t edesc0 = make_desc(smem0 + OFF_E, 16, 128, 0);
+            int s = 0, tl = 0;
+            uint32_t ph = 0, eslot = 0;
             bool ok = true;
             for (int unit = pair; unit < n_units && ok; unit += n_pairs, ++tl) {
                 const int ks = unit / n_tiles;
                 const int it0 = (int)((int64_t)ks * k_iters / P.k_splits), it1 = (int)((int64_t)(ks + 1) * k_iters / P.k_splits);
                 // the epilogues of both CTAs must have drained the accumulator of the previous unit
                 ok = mbar_wait(tmem_empty, (tl & 1) ^ 1, &abort_flag, P.status, 4);
-                for (int it = it0; it < it1 && ok; ++it, ++g) {
-                    const int s = g % STAGES;
-                    const uint32_t ph = (g / STAGES) & 1;
+                for (int it = it0; it < it1 && ok; ++it) {
                     ok = mbar_wait(full0 + 8 * s, ph, &abort_flag, P.status, 2);
                     if (!ok) break;
-                    const uint32_t sa = smem_u32(smem + (size_t)s * STAGE3_BYTES);
-                    const uint32_t sb = sa + OFF_B;
                     tc_fence_after();
-                    const uint32_t e_cols = E_COL0 + (g & 1) * E_SLOT;
-                    tc_cp_128x128b_pair(tmem_base + e_cols, make_desc(sa + OFF_E, 16, 128, 0));
+                    const uint32_t off = (uint32_t)s * (STAGE3_BYTES >> 4);
+                    const uint64_t ad = adesc0 + off, bd = bdesc0 + off, ed = edesc0 + off;
+                    const uint32_t e_cols = tmem_base + E_COL0 + eslot;
+                    if (elect_one()) {
+                        tc_cp_128x128b_pair(e_cols, ed);
 #pragma unroll
-                    for (int j = 0; j < KSTEPS; ++j) {
-                        const uint64_t adesc = make_desc(sa + j * A_KSTEP, A_LBO, 1024, 2);
-                        // MN-major B: 64-column blocks 16384 bytes apart, 32 K-rows (4096 bytes) per MMA
-                        const uint64_t bdesc = make_desc(sb + j * 4096, 16384, 1024, 2);
-                        const uint32_t ecol = e_cols + j;
-                        mma_sp_pair(tmem_base, adesc, bdesc, tmem_base + (ecol & ~1u), idesc0 | (ecol & 1u),
-                                    (it > it0 || j > 0) ? 1u : 0u);
+                        for (int j = 0; j < KSTEPS; ++j)
+                            mma_sp_pair(tmem_base, ad + j * (A_KSTEP >> 4), bd + j * (4096 >> 4), e_cols + (j & ~1), idesc0 | (j & 1),
+                                        (it > it0 || j > 0) ? 1u : 0u);
+                        tc_commit_pair(empty0 + 8 * s);
                     }
-                    tc_commit_pair(empty0 + 8 * s);
+                    __syncwarp();
+                    eslot ^= E_SLOT;
+                    if (++s == STAGES) { s = 0; ph ^= 1; }
                 }
-                tc_commit_pair(tmem_full);
+                if (elect_one()) tc_commit_pair(tmem_full);
+                __syncwarp();
             }
         }
     } else {
