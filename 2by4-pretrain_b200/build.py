@@ -4,7 +4,9 @@
 
 Every ``csrc/*.cu`` is compiled with
 ``nvcc -gencode arch=compute_100a,code=sm_100a -lineinfo`` (nvcc cross-compiles
-without a GPU) and linked into ``lib/libsparse24_b200.so``.  Object files are
+without a GPU) and linked into ``lib/libsparse24_b200.so``; the host path of the
+Python package (``csrc/torch_host.cpp``, C++ against torch) becomes
+``lib/_sp24_torch.so``, linked to that library.  Object files are
 cached under ``build/`` keyed by a hash of the source, the headers and the flags.
 """
 import concurrent.futures
@@ -20,6 +22,8 @@ CSRC = os.path.join(HERE, "csrc")
 LIBDIR = os.path.join(HERE, "lib")
 OBJDIR = os.path.join(HERE, "build")
 LIB = os.path.join(LIBDIR, "libsparse24_b200.so")
+HOST_SRC = os.path.join(CSRC, "torch_host.cpp")
+HOST_LIB = os.path.join(LIBDIR, "_sp24_torch.so")
 
 NVCC_FLAGS = ["-O3", "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo",
               "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr", "-Xptxas", "-v"]
@@ -43,6 +47,28 @@ def _digest(paths, extra=""):
 
 def sources():
     return sorted(glob.glob(os.path.join(CSRC, "*.cu")))
+
+
+def _build_host(force, headers):
+    """The host module: plain C++, so it goes through g++ (in step with the kernels' compilation)."""
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-DTORCH_EXTENSION_NAME=_sp24_torch", "-DTORCH_API_INCLUDE_EXTENSION_H",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+    cmd += ["-isystem" + p for p in cpp_extension.include_paths() + ["/usr/local/cuda/include", sysconfig.get_paths()["include"]]]
+    obj_args = [HOST_SRC, "-o", HOST_LIB, "-L" + LIBDIR, "-l:libsparse24_b200.so", "-Wl,-rpath,$ORIGIN", "-L" + cpp_extension.TORCH_LIB_PATH,
+                "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+    tag = _digest([HOST_SRC] + headers, " ".join(cmd) + torch.__version__)
+    stamp = os.path.join(OBJDIR, "host.stamp")
+    if not force and os.path.exists(HOST_LIB) and os.path.exists(stamp) and open(stamp).read() == tag:
+        return
+    r = subprocess.run(cmd + obj_args, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed on {HOST_SRC}:\n{r.stdout}\n{r.stderr}")
+    with open(stamp, "w") as f:
+        f.write(tag)
 
 
 def build(force=False, verbose=False):
@@ -80,6 +106,7 @@ def build(force=False, verbose=False):
             raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
         with open(stamp, "w") as f:
             f.write(want)
+    _build_host(force, [h for h in headers if h.endswith(".h")])
     return LIB
 
 

@@ -60,6 +60,13 @@ extern "C" const char *sp24_strerror(int code) {
 
 extern "C" int sp24_abi_version(void) { return 2; }
 
+extern "C" int sp24_zero(void *dst, int64_t bytes, void *stream) {
+    if (!dst || bytes < 0) return SP24_ERR_ARG;
+    if (cudaMemsetAsync(dst, 0, (size_t)bytes, static_cast<cudaStream_t>(stream)) == cudaSuccess) return SP24_OK;
+    sp24::launch_status();         // clears (and with SP24_DEBUG prints) the runtime's error
+    return SP24_ERR_CUDA;
+}
+
 // Peer memory for exchanges that run on the copy engines: a buffer exported by its owner (cudaIpcGetMemHandle, or a
 // framework's equivalent) is mapped into this process; copies from the returned address are ordinary device-to-device
 // copies on a stream of the current device.

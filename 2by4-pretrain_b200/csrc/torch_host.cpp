@@ -1,0 +1,900 @@
+// Native host path of the Python package: argument checks, output allocation, kernel launches through the C ABI and the
+// autograd nodes of the layers, in one call from Python each.
+//
+// A layer step launches half a dozen kernels that take 5 - 60 us each; driven from Python (argument marshalling of 20
+// words per launch, tensor views, autograd.Function objects in both directions) its host time was 300 us and bounded
+// every step below a few thousand tokens.  Nothing here computes: without the kernel library the module does not load.
+#include <ATen/ops/mm.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/saved_variable.h>
+#include <torch/extension.h>
+
+#include "../../include/sparse24_b200.h"
+
+namespace {
+
+using at::Tensor;
+using torch::autograd::variable_list;
+using OptTensor = c10::optional<Tensor>;
+using NoAutograd = at::AutoDispatchBelowADInplaceOrView;
+
+// ---------------------------------------------------------------------------------------------
+// small helpers
+// ---------------------------------------------------------------------------------------------
+void check(int rc, const char *what) { TORCH_CHECK(rc == SP24_OK, what, ": ", sp24_strerror(rc), " (code ", rc, ")"); }
+
+int dt(at::ScalarType t) {
+    switch (t) {
+        case at::kFloat: return SP24_F32;
+        case at::kHalf: return SP24_F16;
+        case at::kBFloat16: return SP24_BF16;
+        case at::kFloat8_e4m3fn: return SP24_E4M3;
+        case at::kFloat8_e5m2: return SP24_E5M2;
+        case at::kChar: return SP24_I8;
+        case at::kInt: return SP24_I32;
+        default: TORCH_CHECK(false, "Datatype ", t, " is not supported!");
+    }
+}
+bool is16(at::ScalarType t) { return t == at::kHalf || t == at::kBFloat16; }
+bool is_f8(at::ScalarType t) { return t == at::kFloat8_e4m3fn || t == at::kFloat8_e5m2; }
+
+void *cur_stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
+
+// Every tensor must live on the current device: the kernels run on its current stream and dereference raw addresses.
+void on_current_device(const Tensor &t) {
+    TORCH_CHECK(t.is_cuda(), "Error tensor.device= ", t.device(), " is not supported! Only CUDA tensors are currently supported.");
+    const auto cur = c10::cuda::current_device();
+    TORCH_CHECK(t.device().index() == cur, "tensor on ", t.device(), " but the current CUDA device is cuda:", (int)cur,
+                ": the sparse24 kernels launch on the current device; wrap the call in torch.cuda.device(tensor.device)");
+}
+void on_current_device(const OptTensor &t) { if (t.has_value()) on_current_device(*t); }
+template <typename... T> void require_cuda(const T &...t) { (on_current_device(t), ...); }
+
+void *ptr(const Tensor &t) { return t.data_ptr(); }
+const void *ptr(const OptTensor &t) { return t.has_value() ? t->data_ptr() : nullptr; }
+bool aligned(const Tensor &t, uintptr_t a = 16) { return reinterpret_cast<uintptr_t>(t.data_ptr()) % a == 0; }
+
+Tensor empty(c10::IntArrayRef shape, at::ScalarType t, const Tensor &like) { return at::empty(shape, like.options().dtype(t)); }
+
+// storage order and leading dimension of a 2-D tensor with one unit stride; order -1: neither
+struct Layout { int col; int64_t ld; };
+Layout layout_of(const Tensor &t) {
+    const int64_t rs = t.stride(0), cs = t.stride(1), m = t.size(0), k = t.size(1);
+    if (cs == 1 && (rs >= k || m == 1)) return {0, std::max(rs, k)};
+    if (rs == 1 && (cs >= m || k == 1)) return {1, std::max(cs, m)};
+    return {-1, 0};
+}
+bool usable(const Tensor &t, const Layout &l) { return l.col >= 0 && aligned(t) && (l.ld * (int64_t)t.element_size()) % 16 == 0; }
+// the same logical matrix stored densely in the requested order (no copy when it already is)
+Tensor as_layout(const Tensor &t, int col) {
+    const Layout l = layout_of(t);
+    if (l.col == col && usable(t, l)) return t;
+    return col ? t.t().contiguous().t() : t.contiguous();
+}
+
+// A view into `base`'s memory with its own type, shape and strides, sharing its version counter (a write through either
+// is seen by both); byte_off is counted from base's first element.
+Tensor carve(const Tensor &base, int64_t byte_off, at::ScalarType t, c10::IntArrayRef shape, c10::IntArrayRef strides) {
+    auto impl = c10::make_intrusive<c10::TensorImpl>(c10::Storage(base.storage()), base.key_set(), at::scalarTypeToTypeMeta(t));
+    impl->set_storage_offset(((int64_t)base.storage_offset() * base.element_size() + byte_off) / (int64_t)c10::elementSize(t));
+    impl->set_sizes_and_strides(shape, strides);
+    if (!base.is_inference()) impl->set_version_counter(base.unsafeGetTensorImpl()->version_counter());
+    return Tensor(std::move(impl));
+}
+
+// (rows, last dimension) of a contiguous or reshapeable tensor; sees later in-place writes through its version counter
+Tensor rows2d(const Tensor &t) {
+    if (t.dim() == 2) return t;
+    const int64_t k = t.size(-1);
+    if (t.is_contiguous()) return carve(t, 0, t.scalar_type(), {k ? t.numel() / k : 0, k}, {k, 1});
+    return t.reshape({-1, k});
+}
+
+int64_t align256(int64_t v) { return (v + 255) / 256 * 256; }
+
+// Word that a bounded wait of the GEMM kernels reports to, one per device.
+Tensor &status_word(c10::DeviceIndex dev) {
+    static auto &words = *new std::vector<Tensor>(64);   // never destroyed: the CUDA runtime may be gone at exit
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lock(mu);
+    Tensor &w = words.at(dev);
+    if (!w.defined()) w = at::zeros({1}, at::TensorOptions().dtype(at::kInt).device(at::kCUDA, dev));
+    return w;
+}
+int *status_ptr(const Tensor &t) { return static_cast<int *>(status_word(t.device().index()).data_ptr()); }
+
+// Device word added to the Philox offset of the MVUE draws (a step replayed from a CUDA graph bumps it), or none.
+OptTensor &rng_offset() {
+    static auto &t = *new OptTensor();
+    return t;
+}
+
+// What random.randint(0, 2**31 - 1) returns, from the same generator state: 32 random bits, drawn again until below 2^31.
+// Needs the GIL.
+uint64_t python_seed() {
+    static PyObject *getrandbits = PyObject_GetAttrString(PyImport_ImportModule("random"), "getrandbits");
+    static PyObject *bits = PyLong_FromLong(32);
+    for (;;) {
+        PyObject *r = PyObject_CallOneArg(getrandbits, bits);
+        if (!r) throw py::error_already_set();
+        const unsigned long long v = PyLong_AsUnsignedLongLong(r);
+        Py_DECREF(r);
+        if (v < (1ull << 31)) return v;
+    }
+}
+
+// ---------------------------------------------------------------------------------------------
+// sparse GEMM: input @ dense(weight).T, the contract of sparse.spmm.sparse_linear
+// ---------------------------------------------------------------------------------------------
+Tensor spmm(const Tensor &input, const Tensor &weight, const Tensor &e_tc, const OptTensor &bias_in, int64_t act, c10::optional<double> alpha,
+            bool view_result, bool bias_may_be_f32 = false) {
+    TORCH_CHECK(weight.dim() == 2, "_sparse_semi_structured_linear: Expected weight argument to be 2D tensor, got ", weight.dim(), " dims");
+    const auto wt = weight.scalar_type();
+    TORCH_CHECK(input.scalar_type() == wt, "_sparse_semi_structured_linear: Expected input datatype ", wt, ", but got ", input.scalar_type());
+    const int64_t ms = weight.size(0), kh = weight.size(1), k = 2 * kh;
+    TORCH_CHECK(input.size(-1) == k, "_sparse_semi_structured_linear: Expected weight argument to have ", input.size(-1) / 2,
+                " columns, but got ", kh);
+    Tensor x = input.dim() == 2 ? input : input.reshape({-1, k});
+    const int64_t n = x.size(0);
+    const Layout la = layout_of(weight);
+    TORCH_CHECK(la.col >= 0, "_sparse_semi_structured_linear: Invalid strides for weight argument: row stride = ", weight.stride(0),
+                ", column stride = ", weight.stride(1));
+    Layout lb = layout_of(x);
+    if (!usable(x, lb)) {
+        x = x.contiguous();
+        lb = {0, k};
+    }
+    // fp8 operands give fp32, int8 operands int32, 16-bit operands their own type
+    const bool f8 = is_f8(wt), i8 = wt == at::kChar;
+    const auto ot = f8 ? at::kFloat : (i8 ? at::kInt : wt);
+    TORCH_CHECK(!i8 || (!bias_in.has_value() && act == 0), "_sparse_semi_structured_linear: the int8 GEMM on sm_100a takes no bias and no activation");
+    OptTensor bias = bias_in;
+    bool bias_f32 = false;
+    if (bias.has_value()) {
+        TORCH_CHECK(bias->dim() == 1 && bias->size(0) == ms, "_sparse_semi_structured_linear: Expected bias argument to have ", ms,
+                    " elements, but got ", bias->numel());
+        if (bias_may_be_f32 && bias->scalar_type() != ot) {
+            // the token-major 16-bit GEMM reads a float32 bias in its epilogue; elsewhere it is cast first
+            bias_f32 = bias->scalar_type() == at::kFloat && is16(wt) && lb.col == 0 && !view_result && ms % 256 == 0;
+            if (!bias_f32) bias = bias->to(ot);
+        }
+        TORCH_CHECK(bias_f32 || bias->scalar_type() == ot, "two_four_sgemm_cutlass: Expected spars GTEMM bias datatype ", ot, ", but got ",
+                    bias->scalar_type());
+        bias = bias->contiguous();
+    }
+    TORCH_CHECK(ms % 128 == 0, "sparse GEMM on sm_100a: number of rows of the sparse matrix must be divisible by 128");
+    // k strided in the dense operand (the caller passed B.t()): D (ms, n) row-major, returned as its transposed view
+    const bool as_view = lb.col || view_result;
+    Tensor out;
+    if (as_view) {
+        out = empty({ms, n}, ot, weight);
+    } else if (input.dim() == 2) {
+        out = empty({n, ms}, ot, weight);
+    } else {
+        auto shape = input.sizes().vec();
+        shape.back() = ms;
+        out = empty(shape, ot, weight);
+    }
+    int *status = status_ptr(weight);
+    if (alpha.has_value()) {
+        TORCH_CHECK(f8 && !la.col && !lb.col, "_sparse_semi_structured_linear: alpha is for float8 operands (both K-major) only");
+        check(sp24_spmm_scaled(ptr(weight), dt(wt), la.ld, ptr(e_tc), ms, k, ptr(x), lb.ld, n, static_cast<float *>(ptr(out)), !as_view,
+                               as_view ? n : ms, static_cast<const float *>(ptr(bias)), (int)act, (float)*alpha, status, cur_stream()),
+              "sp24_spmm_scaled");
+    } else if (bias_f32) {
+        check(sp24_spmm_mlp(ptr(weight), dt(wt), la.col, la.ld, ptr(e_tc), ms, k, ptr(x), lb.ld, n, ptr(out), ms, ptr(bias), 1, 0, nullptr,
+                            ms, status, cur_stream()),
+              "sp24_spmm_mlp");
+    } else {
+        check(sp24_spmm(ptr(weight), dt(wt), la.col, la.ld, ptr(e_tc), ms, k, ptr(x), lb.col, lb.ld, n, ptr(out), dt(ot), !as_view,
+                        as_view ? n : ms, ptr(bias), (int)act, status, cur_stream()),
+              "sp24_spmm");
+    }
+    if (!as_view) return out;
+    out = out.t();
+    if (input.dim() == 2) return out;
+    auto shape = input.sizes().vec();
+    shape.back() = ms;
+    return out.reshape(shape);
+}
+
+Tensor sparse_linear(const Tensor &input, const Tensor &weight, const Tensor &e_tc, const OptTensor &bias, int64_t act,
+                     c10::optional<double> alpha, bool view_result) {
+    NoAutograd guard;
+    require_cuda(input, weight, e_tc, bias);
+    return spmm(input, weight, e_tc, bias, act, alpha, view_result);
+}
+
+// out (ms, n) float32 += sparse @ dense (k, n)
+void mm_accumulate(const Tensor &out, const Tensor &weight, const Tensor &e_tc, const Tensor &dense_in, int64_t k_splits) {
+    TORCH_CHECK(out.scalar_type() == at::kFloat && out.dim() == 2 && out.stride(1) == 1, "sparse_mm_accumulate_: out must be a row-major fp32 matrix");
+    TORCH_CHECK(is16(weight.scalar_type()) && dense_in.scalar_type() == weight.scalar_type(),
+                "sparse_mm_accumulate_: expected matching fp16 / bf16 operands, got ", weight.scalar_type(), " and ", dense_in.scalar_type());
+    const int64_t ms = weight.size(0), k = 2 * weight.size(1);
+    TORCH_CHECK(dense_in.dim() == 2 && dense_in.size(0) == k, "sparse_mm_accumulate_: dense operand must have ", k, " rows, got ", dense_in.sizes());
+    const int64_t n = dense_in.size(1);
+    TORCH_CHECK(out.size(0) == ms && out.size(1) == n, "sparse_mm_accumulate_: out must be (", ms, ", ", n, "), got ", out.sizes());
+    const Layout la = layout_of(weight);
+    TORCH_CHECK(la.col >= 0, "sparse_mm_accumulate_: invalid strides for the packed values");
+    Tensor dense = dense_in;
+    if (dense.stride(1) != 1 || !aligned(dense) || (dense.stride(0) * dense.element_size()) % 16) dense = dense.contiguous();
+    check(sp24_spmm_accumulate_f32(ptr(weight), dt(weight.scalar_type()), la.col, la.ld, ptr(e_tc), ms, k, ptr(dense), dense.stride(0), n,
+                                   static_cast<float *>(ptr(out)), out.stride(0), (int)k_splits, status_ptr(weight), cur_stream()),
+          "sp24_spmm_accumulate_f32");
+}
+void sparse_mm_accumulate(const Tensor &out, const Tensor &weight, const Tensor &e_tc, const Tensor &dense, int64_t k_splits) {
+    NoAutograd guard;
+    require_cuda(out, weight, e_tc, dense);
+    mm_accumulate(out, weight, e_tc, dense, k_splits);
+}
+
+// ---------------------------------------------------------------------------------------------
+// dense -> 2:4
+// ---------------------------------------------------------------------------------------------
+// Fills packed / meta from dense; returns the metadata in tensor-core order when it was asked for and the shape allows.
+OptTensor prune_into(const Tensor &dense_in, const Tensor &packed, const Tensor &meta, int64_t mode, const OptTensor &mask_in,
+                     const OptTensor &uniforms_in, uint64_t seed, uint64_t offset, c10::optional<bool> emit_tc, const OptTensor &row_sums,
+                     OptTensor e_tc = {}) {
+    TORCH_CHECK(dense_in.dim() == 2, "Expected 2-dimensional dense tensor, got ", dense_in.dim(), "-dimensional tensor");
+    const int64_t m = dense_in.size(0), k = dense_in.size(1);
+    const Layout lp = layout_of(packed);
+    TORCH_CHECK(lp.col >= 0, "packed output must be row- or column-major with unit inner stride");
+    const Tensor dense = as_layout(dense_in, lp.col);
+    OptTensor mask = mask_in, uniforms = uniforms_in;
+    int64_t ld_m = 0, ld_u = 0;
+    if (mask.has_value()) {
+        if (mask->scalar_type() != at::kBool && mask->scalar_type() != at::kByte) mask = mask->ne(0);
+        mask = as_layout(*mask, lp.col);
+        ld_m = layout_of(*mask).ld;
+    }
+    if (uniforms.has_value()) {
+        uniforms = as_layout(uniforms->to(at::kFloat), lp.col);
+        ld_u = layout_of(*uniforms).ld;
+    }
+    TORCH_CHECK(meta.is_contiguous(), "metadata buffer must be contiguous");
+    const bool draws = mode == SP24_PRUNE_MVUE || mode == SP24_PRUNE_MVUE_FAST;
+    const void *dev_off = draws && !uniforms.has_value() && rng_offset().has_value() ? rng_offset()->data_ptr() : nullptr;
+    // 16-bit results with whole 128-row blocks can also get their metadata in the order the GEMM reads, in the same pass.
+    // Default: for column-major results (the dY^T operand of the weight-gradient GEMM, consumed at once).
+    const bool want_tc = emit_tc.has_value() ? *emit_tc : lp.col == 1;
+    if (!e_tc.has_value() && want_tc && packed.element_size() == 2 && m % 128 == 0)
+        e_tc = empty({sp24_meta_tc_bytes(m, k)}, at::kByte, packed);
+    if (row_sums.has_value())
+        TORCH_CHECK(lp.col && row_sums->scalar_type() == at::kFloat && row_sums->numel() == m && row_sums->is_contiguous(),
+                    "row_sums: column-major input and a contiguous float32 vector of one value per row");
+    check(sp24_prune_compress_ex(ptr(dense), dt(dense.scalar_type()), m, k, layout_of(dense).ld, lp.col, ptr(packed),
+                                 dt(packed.scalar_type()), lp.ld, ptr(meta), (int)mode, ptr(mask), ld_m,
+                                 static_cast<const float *>(ptr(uniforms)), ld_u, seed, offset, static_cast<const uint64_t *>(dev_off),
+                                 const_cast<void *>(ptr(e_tc)), static_cast<float *>(const_cast<void *>(ptr(row_sums))), cur_stream()),
+          "sp24_prune_compress");
+    return e_tc;
+}
+OptTensor prune_compress(const Tensor &dense, const Tensor &packed, const Tensor &meta, int64_t mode, const OptTensor &mask,
+                         const OptTensor &uniforms, uint64_t seed, uint64_t offset, c10::optional<bool> emit_tc, const OptTensor &row_sums) {
+    NoAutograd guard;
+    require_cuda(dense, packed, meta, mask, uniforms, row_sums);
+    return prune_into(dense, packed, meta, mode, mask, uniforms, seed, offset, emit_tc, row_sums);
+}
+
+// One allocation of m*k*cf/16 elements: packed values (in the storage order asked for) first, metadata behind.
+std::pair<Tensor, Tensor> carve_compressed(int64_t m, int64_t k, at::ScalarType t, bool col, const Tensor &like) {
+    const bool b16 = c10::elementSize(t) == 2;
+    Tensor buf = empty({m * k * (b16 ? 9 : 10) / 16}, t, like);
+    const int64_t kh = k / 2, bytes = m * kh * (int64_t)c10::elementSize(t), mc = k / (b16 ? 16 : 32);
+    return {col ? carve(buf, 0, t, {m, kh}, {1, m}) : carve(buf, 0, t, {m, kh}, {kh, 1}),
+            carve(buf, bytes, b16 ? at::kShort : at::kInt, {m, mc}, {mc, 1})};
+}
+// Compression into new buffers, in the storage order of `dense` (row stride > column stride: row-major).
+std::tuple<Tensor, Tensor, OptTensor> compress(const Tensor &dense, at::ScalarType t, int64_t mode, const OptTensor &mask, uint64_t seed) {
+    NoAutograd guard;
+    require_cuda(dense, mask);
+    auto [packed, meta] = carve_compressed(dense.size(0), dense.size(1), t, !(dense.stride(0) > dense.stride(1)), dense);
+    OptTensor e = prune_into(dense, packed, meta, mode, mask, {}, seed, 0, {}, {});
+    return {packed, meta, e};
+}
+
+// ---------------------------------------------------------------------------------------------
+// mask select + both compressed copies
+// ---------------------------------------------------------------------------------------------
+// The copies of one (m, k) weight in one allocation: W values | W metadata | W^T values | W^T metadata | both metadata
+// copies in tensor-core order (whole 128 x 128 blocks only).
+struct Copies {
+    Tensor pw, mw, pt, mt, tcw, tct;
+    Copies(int64_t m, int64_t k, at::ScalarType t, const Tensor &like) {
+        TORCH_CHECK(c10::elementSize(t) == 2, "Datatype ", t, " is not supported!");
+        const int64_t vb = m * k, mb = m * k / 8;          // bytes of the values / metadata of one copy
+        const bool tc = m % 128 == 0 && k % 128 == 0;
+        const int64_t o_mw = vb, o_pt = align256(vb + mb), o_mt = o_pt + vb, o_tw = align256(o_mt + mb), o_tt = o_tw + mb;
+        Tensor buf = empty({o_tw + (tc ? 2 * mb : 0)}, at::kByte, like);
+        pw = carve(buf, 0, t, {m, k / 2}, {k / 2, 1});
+        mw = carve(buf, o_mw, at::kShort, {m, k / 16}, {k / 16, 1});
+        pt = carve(buf, o_pt, t, {k, m / 2}, {1, k});
+        mt = carve(buf, o_mt, at::kShort, {k, m / 16}, {m / 16, 1});
+        if (tc) {
+            tcw = carve(buf, o_tw, at::kByte, {mb}, {1});
+            tct = carve(buf, o_tt, at::kByte, {mb}, {1});
+        }
+    }
+};
+
+// (mask, packed_w, meta_w, packed_t, meta_t, tc_w or None, tc_t or None)
+py::tuple as_tuple(const Tensor &mask, const Copies &c) {
+    auto opt = [](const Tensor &t) { return t.defined() ? py::cast(t) : py::object(py::none()); };
+    return py::make_tuple(mask, c.pw, c.mw, c.pt, c.mt, opt(c.tcw), opt(c.tct));
+}
+
+py::tuple select_compress(const Tensor &weight, const OptTensor &mask_in, at::ScalarType t, const OptTensor &mask_out) {
+    Tensor mask;
+    c10::optional<Copies> c;
+    {
+        py::gil_scoped_release nogil;
+        NoAutograd guard;
+        require_cuda(weight, mask_in, mask_out);
+        TORCH_CHECK(weight.dim() == 2, "select_and_compress: expected a 2-D weight");
+        const int64_t m = weight.size(0), k = weight.size(1);
+        const Tensor w = as_layout(weight, 0);
+        const bool select = !mask_in.has_value();
+        if (!select) {
+            mask = *mask_in;
+            if (mask.scalar_type() != at::kBool && mask.scalar_type() != at::kByte) mask = mask.ne(0);
+            mask = as_layout(mask, 0);
+        } else if (mask_out.has_value()) {
+            mask = *mask_out;
+            TORCH_CHECK(mask.scalar_type() == at::kBool && mask.dim() == 2 && mask.size(0) == m && mask.size(1) == k && mask.is_contiguous(),
+                        "select_and_compress: mask_out must be a contiguous bool tensor of the weight's shape");
+        } else {
+            mask = empty({m, k}, at::kBool, w);
+        }
+        c.emplace(m, k, t, w);
+        const int64_t ldw = layout_of(w).ld, ldm = layout_of(mask).ld;
+        if (c->tcw.defined())
+            check(sp24_select_dual_compress_tc(ptr(w), dt(w.scalar_type()), m, k, ldw, select, ptr(mask), ldm, ptr(c->pw), dt(t), k / 2,
+                                               ptr(c->mw), ptr(c->pt), k, ptr(c->mt), ptr(c->tcw), ptr(c->tct), cur_stream()),
+                  "sp24_select_dual_compress_tc");
+        else
+            check(sp24_select_dual_compress(ptr(w), dt(w.scalar_type()), m, k, ldw, select, ptr(mask), ldm, ptr(c->pw), dt(t), k / 2,
+                                            ptr(c->mw), ptr(c->pt), k, ptr(c->mt), cur_stream()),
+                  "sp24_select_dual_compress");
+    }
+    return as_tuple(mask, *c);
+}
+
+std::vector<py::tuple> select_compress_many(const std::vector<Tensor> &weights, const std::vector<Tensor> &masks, at::ScalarType t, bool reselect) {
+    const size_t count = weights.size();
+    TORCH_CHECK(masks.size() == count, "select_and_compress_many: one mask per weight");
+    std::vector<Copies> copies;
+    std::vector<Tensor> keep;
+    copies.reserve(count);
+    {
+        py::gil_scoped_release nogil;
+        NoAutograd guard;
+        std::vector<sp24_dual_desc> descs(count);
+        for (size_t i = 0; i < count; ++i) {
+            const Tensor &weight = weights[i], &mask = masks[i];
+            require_cuda(weight, mask);
+            const int64_t m = weight.size(0), k = weight.size(1);
+            TORCH_CHECK(m % 128 == 0 && k % 128 == 0, "select_and_compress_many: shape (", m, ", ", k, ") is not a multiple of 128 x 128");
+            TORCH_CHECK(weight.scalar_type() == weights[0].scalar_type() && weight.device() == weights[0].device(),
+                        "select_and_compress_many: all weights must share dtype and device");
+            TORCH_CHECK(mask.scalar_type() == at::kBool && mask.sizes() == weight.sizes() && mask.is_contiguous(),
+                        "select_and_compress_many: masks must be contiguous bool tensors of the weights' shapes");
+            const Tensor w = as_layout(weight, 0);
+            keep.push_back(w);
+            copies.emplace_back(m, k, t, w);
+            const Copies &c = copies.back();
+            descs[i] = {ptr(w), m, k, layout_of(w).ld, ptr(mask), k, ptr(c.pw), k / 2, ptr(c.mw), ptr(c.pt), k, ptr(c.mt), ptr(c.tcw), ptr(c.tct)};
+        }
+        if (count)
+            check(sp24_select_dual_compress_batch(descs.data(), (int)count, dt(weights[0].scalar_type()), dt(t), reselect, cur_stream()),
+                  "sp24_select_dual_compress_batch");
+    }
+    std::vector<py::tuple> out;
+    out.reserve(count);
+    for (size_t i = 0; i < count; ++i) out.push_back(as_tuple(masks[i], copies[i]));
+    return out;
+}
+
+// ---------------------------------------------------------------------------------------------
+// masked decay
+// ---------------------------------------------------------------------------------------------
+// True when done; false when the tensors need what the Python wrapper does for other types, layouts and alignments.
+bool masked_add(const Tensor &grad, const Tensor &p, const Tensor &mask, double alpha) {
+    if (!grad.is_cuda() || grad.layout() != at::kStrided || p.layout() != at::kStrided || mask.layout() != at::kStrided) return false;
+    if (grad.scalar_type() != at::kFloat || p.scalar_type() != at::kFloat || mask.element_size() > 4 || mask.scalar_type() == at::kInt ||
+        mask.scalar_type() == at::kShort)
+        return false;
+    if (grad.sizes() != p.sizes() || grad.sizes() != mask.sizes() || grad.strides() != p.strides() || grad.strides() != mask.strides()) return false;
+    if (!grad.is_non_overlapping_and_dense() || !aligned(grad) || !aligned(p) || !aligned(mask, 4 * mask.element_size())) return false;
+    const auto cur = c10::cuda::current_device();
+    if (grad.device().index() != cur || p.device() != grad.device() || mask.device() != grad.device()) return false;
+    check(sp24_masked_add(ptr(grad), ptr(p), ptr(mask), (int)mask.element_size(), grad.numel(), (float)alpha, cur_stream()), "sp24_masked_add");
+    return true;
+}
+
+// ---------------------------------------------------------------------------------------------
+// FST layer
+// ---------------------------------------------------------------------------------------------
+bool accumulable(const Tensor &grad) { return grad.defined() && grad.scalar_type() == at::kFloat && grad.is_contiguous(); }
+
+// The layer's option for an exact weight gradient is a Python attribute of the weight and its GEMM is torch's.
+bool wants_dense_weight_grad(const Tensor &weight) {
+    static PyObject *name = PyUnicode_InternFromString("weight_grad");
+    py::object w = py::reinterpret_steal<py::object>(THPVariable_Wrap(weight));
+    PyObject *v = PyObject_GetAttr(w.ptr(), name);
+    if (!v) {
+        PyErr_Clear();
+        return false;
+    }
+    const bool dense = PyUnicode_Check(v) && PyUnicode_CompareWithASCIIString(v, "dense") == 0;
+    Py_DECREF(v);
+    return dense;
+}
+
+// dW = MVUE24(g^T) x and db = g.sum(0); g (tokens, out_features) and x (tokens, in_features) in 16 bits.  One pass over g
+// compresses it and takes the bias gradient.  into_grad: both are added to existing float32 .grad buffers and come back
+// undefined.
+std::pair<Tensor, Tensor> fst_weight_grads(const Tensor &g_in, const Tensor &x, const Tensor &weight, const Tensor &bias, bool into_grad,
+                                           bool need_w, bool need_b) {
+    need_b = need_b && bias.defined();
+    uint64_t seed = 0;
+    if (need_w) {
+        py::gil_scoped_acquire gil;
+        if (wants_dense_weight_grad(weight)) {
+            static PyObject *fn = py::object(py::module_::import("sparse.sparse_ops").attr("_dense_weight_grads")).release().ptr();
+            py::object r = py::reinterpret_borrow<py::object>(fn)(g_in, x, weight, bias.defined() ? py::cast(bias) : py::object(py::none()),
+                                                                  into_grad, need_w, need_b);
+            py::tuple t(r);
+            return {t[0].is_none() ? Tensor() : py::cast<Tensor>(t[0]), t[1].is_none() ? Tensor() : py::cast<Tensor>(t[1])};
+        }
+        seed = python_seed();
+    }
+    NoAutograd guard;
+    Tensor gw, gb;
+    if (need_w) {
+        const Tensor g = g_in.contiguous();
+        const int64_t tokens = g.size(0), out_f = g.size(1), in_f = x.size(1);
+        TORCH_CHECK(out_f % 32 == 0 && tokens % 64 == 0, "gradient of shape (", tokens, ", ", out_f,
+                    "): features % 32 == 0 and tokens % 64 == 0 required");
+        const bool f32 = weight.scalar_type() == at::kFloat && in_f % 8 == 0;
+        const bool into = into_grad && f32 && accumulable(weight.grad());
+        // the bias gradient: into bias.grad, or into the tail of the zeroed buffer that receives dW
+        Tensor sums, acc;
+        if (into) {
+            acc = weight.grad();
+            if (need_b && accumulable(bias.grad())) sums = bias.grad();
+        } else if (f32) {
+            const bool with_b = need_b && bias.scalar_type() == at::kFloat;
+            const int64_t nw = out_f * in_f, total = nw + (with_b ? out_f : 0);
+            Tensor buf = empty({total}, at::kFloat, g);
+            check(sp24_zero(ptr(buf), total * 4, cur_stream()), "sp24_zero");
+            acc = gw = carve(buf, 0, at::kFloat, {out_f, in_f}, {in_f, 1});
+            if (with_b) sums = gb = carve(buf, nw * 4, at::kFloat, {out_f}, {1});
+        }
+        // packed values, metadata and its tensor-core copy, all consumed by the next launch
+        const int64_t vb = out_f * tokens, mb = out_f * tokens / 8;
+        const bool tc = out_f % 128 == 0;
+        Tensor buf = empty({align256(vb + mb) + (tc ? sp24_meta_tc_bytes(out_f, tokens) : 0)}, at::kByte, g);
+        const Tensor gp = carve(buf, 0, g.scalar_type(), {out_f, tokens / 2}, {1, out_f});
+        const Tensor gm = carve(buf, vb, at::kShort, {out_f, tokens / 16}, {tokens / 16, 1});
+        OptTensor e;
+        if (tc) e = carve(buf, align256(vb + mb), at::kByte, {sp24_meta_tc_bytes(out_f, tokens)}, {1});
+        prune_into(g.t(), gp, gm, SP24_PRUNE_MVUE_FAST, {}, {}, seed, 0, false, sums.defined() ? OptTensor(sums) : OptTensor(), e);
+        if (sums.defined()) need_b = false;
+        TORCH_CHECK(tc, "sparse GEMM on sm_100a: number of rows of the sparse matrix must be divisible by 128");
+        if (acc.defined()) mm_accumulate(acc, gp, *e, x, 0);
+        else gw = spmm(x.t(), gp, *e, {}, 0, {}, false).t();
+    }
+    if (need_b) gb = g_in.sum(0);
+    return {gw, gb};
+}
+
+struct FstBackward : torch::autograd::Node {
+    torch::autograd::SavedVariable x_;
+    Tensor pt_, tct_, weight_, bias_;
+    int64_t pt_version_ = 0;
+    std::vector<int64_t> shape_;
+    bool into_grad_ = false, released_ = false;
+
+    std::string name() const override { return "FstLinearBackward"; }
+    void release_variables() override {
+        x_.reset_data();
+        pt_.reset();
+        tct_.reset();
+        released_ = true;
+    }
+    variable_list apply(variable_list &&grads) override {
+        TORCH_CHECK(!released_, torch::autograd::ERR_BACKWARD_TWICE);
+        variable_list out(3);
+        Tensor g = grads[0];
+        if (!g.defined()) return out;
+        const Tensor x = x_.unpack();
+        TORCH_CHECK(pt_._version() == pt_version_, "the compressed weight needed for gradient computation has been modified by an inplace operation");
+        {
+            NoAutograd guard;
+            // the gradient of a plain sum arrives as one expanded value; the reference layer replaces it by ones
+            if (g.dim() == 3 && g.stride(0) == 0 && g.stride(1) == 0 && g.stride(2) == 0) g = at::ones_like(g);
+            if (g.dim() != 2) g = g.reshape({-1, g.size(-1)});
+            if (g.scalar_type() != pt_.scalar_type()) g = g.to(pt_.scalar_type());
+            if (task_should_compute_output(0)) {
+                Tensor dx = spmm(g, pt_, tct_, {}, 0, {}, false);
+                out[0] = dx.dim() == (int64_t)shape_.size() ? dx : dx.view(shape_);
+            }
+        }
+        if (task_should_compute_output(1) || task_should_compute_output(2)) {
+            auto [gw, gb] = fst_weight_grads(g, x, weight_, bias_, into_grad_, task_should_compute_output(1), task_should_compute_output(2));
+            out[1] = gw;
+            out[2] = gb;
+        }
+        return out;
+    }
+};
+
+Tensor unpack(PyObject *o) {
+    TORCH_CHECK(THPVariable_Check(o), "expected a tensor");
+    return THPVariable_Unpack(o);
+}
+
+// y = x W_s^T + b on the compressed copies (packed_w, meta_w, packed_t, meta_t); tc = their metadata in tensor-core order.
+Tensor fst_linear(const Tensor &input, const Tensor &weight, const OptTensor &bias, const py::tuple &copies, const py::tuple &tc, bool into_grad) {
+    const Tensor pw = unpack(copies[0].ptr()), pt = unpack(copies[2].ptr()), tcw = unpack(tc[0].ptr()), tct = unpack(tc[1].ptr());
+    py::gil_scoped_release nogil;
+    require_cuda(input, pw, pt, tcw, tct, bias);
+    Tensor x, y;
+    {
+        NoAutograd guard;
+        x = rows2d(input);
+        if (x.scalar_type() != pw.scalar_type()) x = x.to(pw.scalar_type());
+        y = spmm(x, pw, tcw, bias, 0, {}, false, true);
+        if (input.dim() != 2) {
+            auto shape = input.sizes().vec();
+            shape.back() = pw.size(0);
+            y = y.view(shape);
+        }
+    }
+    const Tensor b = bias.has_value() ? *bias : Tensor();
+    if (torch::autograd::compute_requires_grad(input, weight, b)) {
+        auto node = std::shared_ptr<FstBackward>(new FstBackward(), torch::autograd::deleteNode);
+        node->set_next_edges(torch::autograd::collect_next_edges(input, weight, b));
+        node->x_ = torch::autograd::SavedVariable(x, false);
+        node->pt_ = pt;
+        node->pt_version_ = pt._version();
+        node->tct_ = tct;
+        node->weight_ = weight;
+        node->bias_ = b;
+        node->shape_ = input.sizes().vec();
+        node->into_grad_ = into_grad;
+        torch::autograd::set_history(y, node);
+    }
+    return y;
+}
+
+// ---------------------------------------------------------------------------------------------
+// trainer ops around the GEMMs
+// ---------------------------------------------------------------------------------------------
+// Where a backward kernel adds two parameter gradients: straight into existing float32 .grad buffers (autograd then
+// receives nothing), or into a zeroed temporary of shape (2, d).
+struct AffineGrads {
+    Tensor g, b, rg, rb;
+    AffineGrads(const Tensor &weight, const Tensor &bias, bool into, int64_t d, const Tensor &like) {
+        if (into && accumulable(weight.grad()) && accumulable(bias.grad())) {
+            g = weight.grad();
+            b = bias.grad();
+            return;
+        }
+        Tensor buf = empty({2 * d}, at::kFloat, like);
+        check(sp24_zero(ptr(buf), 2 * d * 4, cur_stream()), "sp24_zero");
+        g = rg = carve(buf, 0, at::kFloat, {d}, {1});
+        b = rb = carve(buf, d * 4, at::kFloat, {d}, {1});
+    }
+};
+
+struct LayerNormBackward : torch::autograd::Node {
+    torch::autograd::SavedVariable x_;
+    Tensor stats_, weight_, bias_;
+    std::vector<int64_t> shape_;
+    at::ScalarType x_dtype_ = at::kFloat;
+    bool into_grad_ = false, released_ = false;
+
+    std::string name() const override { return "SparseLayerNormBackward"; }
+    void release_variables() override {
+        x_.reset_data();
+        stats_.reset();
+        released_ = true;
+    }
+    variable_list apply(variable_list &&grads) override {
+        TORCH_CHECK(!released_, torch::autograd::ERR_BACKWARD_TWICE);
+        variable_list out(3);
+        if (!grads[0].defined()) return out;
+        const Tensor x = x_.unpack();
+        NoAutograd guard;
+        const int64_t rows = x.size(0), d = x.size(1);
+        Tensor dy = grads[0].reshape({rows, d});
+        if (dy.scalar_type() != at::kFloat && !is16(dy.scalar_type())) dy = dy.to(at::kFloat);
+        dy = dy.contiguous();
+        Tensor dx = at::empty_like(x);
+        AffineGrads t(weight_, bias_, into_grad_, d, x);
+        const float *st = static_cast<const float *>(ptr(stats_));
+        check(sp24_layernorm_bwd(ptr(dy), dt(dy.scalar_type()), static_cast<const float *>(ptr(x)), static_cast<const float *>(ptr(weight_)), st,
+                                 st + rows, static_cast<float *>(ptr(dx)), static_cast<float *>(ptr(t.g)), static_cast<float *>(ptr(t.b)), rows, d,
+                                 cur_stream()),
+              "sp24_layernorm_bwd");
+        out[0] = dx.view(shape_).to(x_dtype_);
+        out[1] = t.rg;
+        out[2] = t.rb;
+        return out;
+    }
+};
+
+Tensor layer_norm(const Tensor &input, const Tensor &weight, const Tensor &bias, double eps, at::ScalarType out_t, bool into_grad) {
+    require_cuda(input, weight, bias);
+    Tensor x, out, stats;
+    {
+        NoAutograd guard;
+        const int64_t d = input.size(-1);
+        x = rows2d(input);
+        if (x.scalar_type() != at::kFloat) x = x.to(at::kFloat);
+        x = x.contiguous();
+        const int64_t rows = x.size(0);
+        out = empty(input.sizes(), out_t, x);
+        stats = empty({2 * rows}, at::kFloat, x);             // mean, then reciprocal standard deviation
+        float *st = static_cast<float *>(ptr(stats));
+        check(sp24_layernorm_fwd(static_cast<const float *>(ptr(x)), static_cast<const float *>(ptr(weight)), static_cast<const float *>(ptr(bias)),
+                                 ptr(out), dt(out_t), st, st + rows, rows, d, (float)eps, cur_stream()),
+              "sp24_layernorm_fwd");
+    }
+    if (torch::autograd::compute_requires_grad(input, weight, bias)) {
+        auto node = std::shared_ptr<LayerNormBackward>(new LayerNormBackward(), torch::autograd::deleteNode);
+        node->set_next_edges(torch::autograd::collect_next_edges(input, weight, bias));
+        node->x_ = torch::autograd::SavedVariable(x, false);
+        node->stats_ = stats;
+        node->weight_ = weight;
+        node->bias_ = bias;
+        node->shape_ = input.sizes().vec();
+        node->x_dtype_ = input.scalar_type();
+        node->into_grad_ = into_grad;
+        torch::autograd::set_history(out, node);
+    }
+    return out;
+}
+
+// (x + delta, layer_norm(x + delta)); backward: the gradient arriving along the residual stream is added to the norm's
+// input gradient and the sum goes to both inputs (float32 for x, delta's type for delta).
+struct AddLayerNormBackward : torch::autograd::Node {
+    torch::autograd::SavedVariable res_;
+    Tensor stats_, weight_, bias_;
+    std::vector<int64_t> shape_;
+    at::ScalarType delta_dtype_ = at::kFloat;
+    bool into_grad_ = false, released_ = false;
+
+    std::string name() const override { return "SparseAddLayerNormBackward"; }
+    void release_variables() override {
+        res_.reset_data();
+        stats_.reset();
+        released_ = true;
+    }
+    variable_list apply(variable_list &&grads) override {
+        TORCH_CHECK(!released_, torch::autograd::ERR_BACKWARD_TWICE);
+        variable_list out(4);
+        const Tensor &grad_res = grads[0];
+        Tensor grad_out = grads[1];
+        if (!grad_res.defined() && !grad_out.defined()) return out;
+        const Tensor res = res_.unpack(shared_from_this());
+        NoAutograd guard;
+        const int64_t d = shape_.back(), rows = res.numel() / d;
+        if (!grad_out.defined()) grad_out = at::zeros(shape_, res.options().dtype(delta_dtype_));   // the normalised output was not used
+        const Tensor dy = grad_out.reshape({rows, d}).contiguous();
+        Tensor dres;
+        if (grad_res.defined()) {
+            dres = grad_res.reshape({rows, d});
+            if (dres.scalar_type() != at::kFloat || !dres.is_contiguous()) dres = dres.to(at::kFloat).contiguous();
+        }
+        Tensor dx = empty(shape_, at::kFloat, res), ddelta = empty(shape_, dy.scalar_type(), res);
+        AffineGrads t(weight_, bias_, into_grad_, d, res);
+        const float *st = static_cast<const float *>(ptr(stats_));
+        check(sp24_add_layernorm_bwd(ptr(dy), dt(dy.scalar_type()), dres.defined() ? static_cast<const float *>(ptr(dres)) : nullptr,
+                                     static_cast<const float *>(ptr(res)), static_cast<const float *>(ptr(weight_)), st, st + rows,
+                                     static_cast<float *>(ptr(dx)), ptr(ddelta), static_cast<float *>(ptr(t.g)), static_cast<float *>(ptr(t.b)),
+                                     rows, d, cur_stream()),
+              "sp24_add_layernorm_bwd");
+        out[0] = dx;
+        out[1] = ddelta;
+        out[2] = t.rg;
+        out[3] = t.rb;
+        return out;
+    }
+};
+
+std::pair<Tensor, Tensor> add_layer_norm(const Tensor &x, const Tensor &delta, const Tensor &weight, const Tensor &bias, double eps, bool into_grad) {
+    require_cuda(x, delta, weight, bias);
+    Tensor res, out, stats;
+    {
+        NoAutograd guard;
+        const int64_t d = x.size(-1), rows = x.numel() / d;
+        res = empty(x.sizes(), at::kFloat, x);
+        out = empty(x.sizes(), delta.scalar_type(), x);
+        stats = empty({2 * rows}, at::kFloat, x);
+        float *st = static_cast<float *>(ptr(stats));
+        check(sp24_add_layernorm_fwd(static_cast<const float *>(ptr(x)), ptr(delta), static_cast<float *>(ptr(res)), static_cast<const float *>(ptr(weight)),
+                                     static_cast<const float *>(ptr(bias)), ptr(out), dt(out.scalar_type()), st, st + rows, rows, d, (float)eps,
+                                     cur_stream()),
+              "sp24_add_layernorm_fwd");
+    }
+    if (torch::autograd::compute_requires_grad(x, delta, weight, bias)) {
+        auto node = std::shared_ptr<AddLayerNormBackward>(new AddLayerNormBackward(), torch::autograd::deleteNode);
+        node->set_next_edges(torch::autograd::collect_next_edges(x, delta, weight, bias));
+        node->stats_ = stats;
+        node->weight_ = weight;
+        node->bias_ = bias;
+        node->shape_ = x.sizes().vec();
+        node->delta_dtype_ = delta.scalar_type();
+        node->into_grad_ = into_grad;
+        torch::autograd::set_history(res, node);
+        torch::autograd::set_history(out, node);
+        node->res_ = torch::autograd::SavedVariable(res, true);
+    }
+    return {res, out};
+}
+
+// Mean cross entropy whose gradient for an upstream gradient of 1 is written by the forward launch; backward rescales it
+// on the device only when the upstream gradient is not 1.
+struct CrossEntropyBackward : torch::autograd::Node {
+    Tensor dlogits_;
+    std::string name() const override { return "SparseCrossEntropyBackward"; }
+    void release_variables() override { dlogits_.reset(); }
+    variable_list apply(variable_list &&grads) override {
+        variable_list out(1);
+        if (!grads[0].defined()) return out;
+        TORCH_CHECK(dlogits_.defined(), "cross_entropy: the fused gradient buffer was already handed out by an earlier backward pass");
+        NoAutograd guard;
+        Tensor g = std::move(dlogits_);                    // handed out once
+        dlogits_.reset();
+        const Tensor up = grads[0].reshape({1}).to(at::kFloat).contiguous();
+        check(sp24_scale_unless_one(ptr(g), dt(g.scalar_type()), static_cast<const float *>(ptr(up)), g.numel(), cur_stream()), "sp24_scale_unless_one");
+        out[0] = g;
+        return out;
+    }
+};
+
+Tensor cross_entropy(const Tensor &logits, const Tensor &targets) {
+    require_cuda(logits, targets);
+    Tensor loss, dlogits;
+    {
+        NoAutograd guard;
+        const int64_t rows = logits.size(0), v = logits.size(1);
+        Tensor both = empty({2 * rows}, at::kFloat, logits);   // log-sum-exp, then the rows' losses
+        dlogits = empty({rows, v}, logits.scalar_type(), logits);
+        float *lse = static_cast<float *>(ptr(both));
+        check(sp24_cross_entropy_fused(ptr(logits), dt(logits.scalar_type()), static_cast<const int64_t *>(ptr(targets)), lse, lse + rows,
+                                       (float)(1.0 / rows), ptr(dlogits), rows, v, logits.stride(0), v, cur_stream()),
+              "sp24_cross_entropy_fused");
+        loss = carve(both, rows * 4, at::kFloat, {rows}, {1}).mean();
+    }
+    auto node = std::shared_ptr<CrossEntropyBackward>(new CrossEntropyBackward(), torch::autograd::deleteNode);
+    node->set_next_edges(torch::autograd::collect_next_edges(logits));
+    node->dlogits_ = dlogits;
+    torch::autograd::set_history(loss, node);
+    return loss;
+}
+
+struct EmbedBackward : torch::autograd::Node {
+    Tensor ids_, wte_, wpe_;
+    bool into_grad_ = false;
+    std::string name() const override { return "SparseEmbedTokensBackward"; }
+    void release_variables() override { ids_.reset(); }
+    variable_list apply(variable_list &&grads) override {
+        variable_list out(2);
+        if (!grads[0].defined()) return out;
+        TORCH_CHECK(ids_.defined(), torch::autograd::ERR_BACKWARD_TWICE);
+        NoAutograd guard;
+        Tensor dx = grads[0];
+        if (dx.scalar_type() != at::kFloat || !dx.is_contiguous()) dx = dx.to(at::kFloat).contiguous();
+        Tensor gw = wte_.grad(), gp = wpe_.grad();
+        const bool into = into_grad_ && accumulable(gw) && accumulable(gp);
+        if (!into) {
+            gw = at::zeros(wte_.sizes(), wte_.options().dtype(at::kFloat));
+            gp = at::zeros(wpe_.sizes(), wpe_.options().dtype(at::kFloat));
+        }
+        const int64_t b = ids_.size(0), t = ids_.size(1);
+        check(sp24_embedding_bwd(static_cast<const float *>(ptr(dx)), static_cast<const int64_t *>(ptr(ids_)), static_cast<float *>(ptr(gw)),
+                                 static_cast<float *>(ptr(gp)), b * t, t, wte_.size(1), wte_.size(0), cur_stream()),
+              "sp24_embedding_bwd");
+        if (!into) {
+            out[0] = gw;
+            out[1] = gp;
+        }
+        return out;
+    }
+};
+
+Tensor embed_tokens(const Tensor &ids_in, const Tensor &wte, const Tensor &wpe, bool into_grad) {
+    Tensor ids, out;
+    {
+        NoAutograd guard;
+        ids = ids_in.contiguous();
+        const int64_t b = ids.size(0), t = ids.size(1), d = wte.size(1);
+        out = empty({b, t, d}, at::kFloat, wte);
+        check(sp24_embedding_fwd(static_cast<const int64_t *>(ptr(ids)), static_cast<const float *>(ptr(wte)), static_cast<const float *>(ptr(wpe)),
+                                 static_cast<float *>(ptr(out)), b * t, t, d, wte.size(0), cur_stream()),
+              "sp24_embedding_fwd");
+    }
+    if (torch::autograd::compute_requires_grad(wte, wpe)) {
+        auto node = std::shared_ptr<EmbedBackward>(new EmbedBackward(), torch::autograd::deleteNode);
+        node->set_next_edges(torch::autograd::collect_next_edges(wte, wpe));
+        node->ids_ = ids;
+        node->wte_ = wte;
+        node->wpe_ = wpe;
+        node->into_grad_ = into_grad;
+        torch::autograd::set_history(out, node);
+    }
+    return out;
+}
+
+struct GeluBackward : torch::autograd::Node {
+    torch::autograd::SavedVariable x_;
+    bool released_ = false;
+    std::string name() const override { return "SparseGeluBackward"; }
+    void release_variables() override {
+        x_.reset_data();
+        released_ = true;
+    }
+    variable_list apply(variable_list &&grads) override {
+        TORCH_CHECK(!released_, torch::autograd::ERR_BACKWARD_TWICE);
+        variable_list out(1);
+        if (!grads[0].defined()) return out;
+        const Tensor x = x_.unpack();
+        NoAutograd guard;
+        Tensor dy = grads[0].contiguous();
+        if (dy.scalar_type() != x.scalar_type()) dy = dy.to(x.scalar_type());
+        Tensor dx = at::empty_like(x);
+        check(sp24_gelu(ptr(x), ptr(dy), ptr(dx), dt(x.scalar_type()), x.numel(), cur_stream()), "sp24_gelu");
+        out[0] = dx;
+        return out;
+    }
+};
+
+Tensor gelu(const Tensor &input) {
+    require_cuda(input);
+    Tensor x, out;
+    {
+        NoAutograd guard;
+        x = input.contiguous();
+        out = at::empty_like(x);
+        check(sp24_gelu(ptr(x), nullptr, ptr(out), dt(x.scalar_type()), x.numel(), cur_stream()), "sp24_gelu");
+    }
+    if (torch::autograd::compute_requires_grad(input)) {
+        auto node = std::shared_ptr<GeluBackward>(new GeluBackward(), torch::autograd::deleteNode);
+        node->set_next_edges(torch::autograd::collect_next_edges(input));
+        node->x_ = torch::autograd::SavedVariable(x, false);
+        torch::autograd::set_history(out, node);
+    }
+    return out;
+}
+
+}  // namespace
+
+PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
+    using nogil = py::call_guard<py::gil_scoped_release>;
+    m.def("sparse_linear", &sparse_linear, nogil());
+    m.def("sparse_mm_accumulate", &sparse_mm_accumulate, nogil());
+    m.def("prune_compress", &prune_compress, nogil());
+    m.def("compress", &compress, nogil());
+    m.def("select_compress", &select_compress);
+    m.def("select_compress_many", &select_compress_many);
+    m.def("masked_add", &masked_add, nogil());
+    m.def("fst_linear", &fst_linear);
+    m.def("fst_weight_grads",
+          [](const Tensor &g, const Tensor &x, const Tensor &w, const OptTensor &b, bool into, bool nw, bool nb) {
+              auto [gw, gb] = fst_weight_grads(g, x, w, b.has_value() ? *b : Tensor(), into, nw, nb);
+              return std::make_pair(gw.defined() ? OptTensor(gw) : OptTensor(), gb.defined() ? OptTensor(gb) : OptTensor());
+          },
+          nogil());
+    m.def("layer_norm", &layer_norm, nogil());
+    m.def("add_layer_norm", &add_layer_norm, nogil());
+    m.def("cross_entropy", &cross_entropy, nogil());
+    m.def("embed_tokens", &embed_tokens, nogil());
+    m.def("gelu", &gelu, nogil());
+    m.def("python_seed", &python_seed);
+    m.def("set_rng_offset", [](const OptTensor &t) { rng_offset() = t; });
+    m.def("status_word", [](int dev) { return status_word((c10::DeviceIndex)dev); });
+}

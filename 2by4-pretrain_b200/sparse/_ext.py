@@ -5,12 +5,14 @@ not fall back.  Tensors are passed as raw device pointers plus sizes; the curren
 stream is passed as the stream handle, so calls are asynchronous like any torch op.
 """
 import ctypes
+import importlib.util
 import os
 
 import torch
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(os.path.dirname(_HERE), "lib", "libsparse24_b200.so")
+HOST_PATH = os.path.join(os.path.dirname(_HERE), "lib", "_sp24_torch.so")
 
 F32, F16, BF16, E4M3, E5M2, I8, I32 = 0, 1, 2, 3, 4, 5, 6
 PRUNE_MSE, PRUNE_MASK, PRUNE_MVUE, PRUNE_MVUE_FAST = 0, 1, 2, 3
@@ -58,6 +60,7 @@ _SIGNATURES = {
     "sp24_select_dual_compress_tc": [_vp, _i32, _i64, _i64, _i64, _i32, _vp, _i64, _vp, _i32, _i64, _vp, _vp, _i64,
                                      _vp, _vp, _vp, _vp],
     "sp24_select_dual_compress_batch": [ctypes.POINTER(DualDesc), _i32, _i32, _i32, _i32, _vp],
+    "sp24_zero": [_vp, _i64, _vp],
     "sp24_masked_add": [_vp, _vp, _vp, _i32, _i64, _f32, _vp],
     "sp24_cross_entropy_fused": [_vp, _i32, _vp, _vp, _vp, _f32, _vp, _i64, _i64, _i64, _i64, _vp],
     "sp24_scale_unless_one": [_vp, _i32, _vp, _i64, _vp],
@@ -91,6 +94,25 @@ def lib():
                 fn.argtypes = args
         _lib = h
     return _lib
+
+
+class _Host:
+    """The native host path (``csrc/torch_host.cpp``): functions that check, allocate, launch and build the autograd node
+    in one call.  Loaded on first use, so that the package imports without a build; raises when it is missing."""
+
+    def __getattr__(self, name):
+        lib()
+        if not os.path.exists(HOST_PATH):
+            raise RuntimeError(f"sparse24_b200 host module not found at {HOST_PATH}; build it with "
+                               f"`python {os.path.join(os.path.dirname(_HERE), 'build.py')}`.")
+        spec = importlib.util.spec_from_file_location("_sp24_torch", HOST_PATH)
+        mod = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(mod)
+        self.__dict__.update((k, v) for k, v in vars(mod).items() if not k.startswith("_"))
+        return self.__dict__[name]
+
+
+host = _Host()
 
 
 def register_signature(name, argtypes):

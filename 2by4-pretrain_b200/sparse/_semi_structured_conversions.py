@@ -32,6 +32,8 @@ def set_device_rng_offset(counter: Optional[Tensor]) -> None:
         if counter.dtype != torch.int64 or counter.numel() != 1 or not counter.is_cuda:
             raise RuntimeError("set_device_rng_offset: expected a one-element int64 CUDA tensor")
     _DEVICE_RNG_OFFSET = counter
+    if counter is not None or "set_rng_offset" in vars(_ext.host):      # nothing to remove before the module is loaded
+        _ext.host.set_rng_offset(counter)
 
 
 def prune_compress(dense: Tensor, sparse: Tensor, meta: Tensor, *, mode: int, mask: Optional[Tensor] = None,
@@ -44,68 +46,44 @@ def prune_compress(dense: Tensor, sparse: Tensor, meta: Tensor, *, mode: int, ma
     sparse/semi_structured.py:231-243).  ``uniforms`` (float32, logical (m, k)) is the test hook
     that drives MVUE with caller-supplied randomness; otherwise (seed, offset) key the Philox stream.
     """
-    _ext.require_cuda(dense, sparse, meta, mask, uniforms)
-    if dense.dim() != 2:
-        raise RuntimeError(f"Expected 2-dimensional dense tensor, got {dense.dim()}-dimensional tensor")
-    m, k = dense.shape
-    lay = _ext.layout_of(sparse)
-    if lay is None:
-        raise RuntimeError("packed output must be row- or column-major with unit inner stride")
-    col_major, ld_p = lay
-    dense = _ext.as_layout(dense, col_major)
-    ld_d = _ext.layout_of(dense)[1]
-    ld_m = ld_u = 0
-    if mask is not None:
-        if mask.dtype != torch.bool and mask.dtype != torch.uint8:
-            mask = mask != 0
-        mask = _ext.as_layout(mask, col_major)
-        ld_m = _ext.layout_of(mask)[1]
-    if uniforms is not None:
-        uniforms = _ext.as_layout(uniforms.float(), col_major)
-        ld_u = _ext.layout_of(uniforms)[1]
-    if not meta.is_contiguous():
-        raise RuntimeError("metadata buffer must be contiguous")
-    dev_off = _DEVICE_RNG_OFFSET if mode in (_ext.PRUNE_MVUE, _ext.PRUNE_MVUE_FAST) and uniforms is None else None
     # 16-bit results with whole 128-row blocks can also get their metadata in the order the GEMM reads, in the same
     # pass.  Default: for column-major results (the dY^T operand of the weight-gradient GEMM, consumed at once);
     # row-major results (weights converted once) get it on request, else lazily at their first GEMM.
-    e_tc = None
-    want_tc = bool(col_major) if emit_tc is None else emit_tc
-    if want_tc and sparse.element_size() == 2 and m % 128 == 0:
-        from . import spmm as _spmm
-        e_tc = torch.empty(_spmm.tc_bytes(m, k), dtype=torch.uint8, device=meta.device)
-    if row_sums is not None:
-        if not col_major or row_sums.dtype != torch.float32 or row_sums.numel() != m or not row_sums.is_contiguous():
-            raise RuntimeError("row_sums: column-major input and a contiguous float32 vector of one value per row")
-    if dev_off is not None or e_tc is not None or row_sums is not None:
-        rc = _ext.lib().sp24_prune_compress_ex(
-            dense.data_ptr(), _ext.dt(dense.dtype), m, k, ld_d, col_major, sparse.data_ptr(), _ext.dt(sparse.dtype), ld_p,
-            meta.data_ptr(), mode, _ext.ptr(mask), ld_m, _ext.ptr(uniforms), ld_u, seed & (2 ** 64 - 1),
-            offset & (2 ** 64 - 1), _ext.ptr(dev_off), _ext.ptr(e_tc), _ext.ptr(row_sums), _ext.stream())
-    else:
-        rc = _ext.lib().sp24_prune_compress(
-            dense.data_ptr(), _ext.dt(dense.dtype), m, k, ld_d, col_major, sparse.data_ptr(), _ext.dt(sparse.dtype), ld_p,
-            meta.data_ptr(), mode, _ext.ptr(mask), ld_m, _ext.ptr(uniforms), ld_u, seed & (2 ** 64 - 1),
-            offset & (2 ** 64 - 1), _ext.stream())
-    _ext.check(rc, "sp24_prune_compress")
-    from .spmm import invalidate_meta, register_tc_metadata
-    invalidate_meta(meta)  # a refilled metadata buffer must not reuse a cached tensor-core copy
-    if e_tc is not None:
-        register_tc_metadata(meta, e_tc)
+    e_tc = _ext.host.prune_compress(dense, sparse, meta, mode, mask, uniforms, seed & (2 ** 64 - 1), offset & (2 ** 64 - 1), emit_tc, row_sums)
+    note_tc_metadata(meta, e_tc)
     return sparse, meta
+
+
+def note_tc_metadata(meta: Tensor, e_tc: Optional[Tensor]) -> None:
+    """A kernel has just written ``meta`` and, unless None, its copy in tensor-core order: an older cached copy goes."""
+    from .spmm import invalidate_meta, register_tc_metadata
+    if e_tc is None:
+        invalidate_meta(meta)
+    else:
+        register_tc_metadata(meta, e_tc)
+
+
+def _prune_mode(MVUE24: bool, mask: Optional[Tensor]) -> int:
+    if mask is not None:
+        return _ext.PRUNE_MASK
+    # MVUE: production arithmetic; PRUNE_MVUE (exact) is reached through prune_compress
+    return _ext.PRUNE_MVUE_FAST if MVUE24 else _ext.PRUNE_MSE
+
+
+def compress(dense: Tensor, dtype: torch.dtype, MVUE24: bool = False, mask: Optional[Tensor] = None):
+    """2:4 compression into new buffers in the storage order of ``dense``; returns (packed, metadata).  The MVUE seed
+    comes from Python's ``random`` like in the reference (sparse/_semi_structured_conversions.py:1076)."""
+    packed, meta, e_tc = _ext.host.compress(dense, dtype, _prune_mode(MVUE24, mask), mask, random.randint(0, 2 ** 31 - 1))
+    if e_tc is not None:
+        note_tc_metadata(meta, e_tc)
+    return packed, meta
 
 
 def sparse_semi_structured_from_dense_triton(dense, sparse, meta, MVUE24: bool = False, mask: Optional[Tensor] = None):
     """Name and arguments of the reference launcher (no Triton inside).  The MVUE seed is drawn from
     Python's ``random`` like the reference does (sparse/_semi_structured_conversions.py:1076)."""
-    if mask is not None:
-        mode = _ext.PRUNE_MASK
-    elif MVUE24:
-        mode = _ext.PRUNE_MVUE_FAST   # production arithmetic; PRUNE_MVUE (exact) is reached through prune_compress
-    else:
-        mode = _ext.PRUNE_MSE
     seed = random.randint(0, 2 ** 31 - 1)
-    return prune_compress(dense, sparse, meta, mode=mode, mask=mask, seed=seed)
+    return prune_compress(dense, sparse, meta, mode=_prune_mode(MVUE24, mask), mask=mask, seed=seed)
 
 
 def sparse_semi_structured_from_dense(dense: Tensor):

@@ -23,6 +23,8 @@ def masked_add_(grad: torch.Tensor, p_data: torch.Tensor, p_mask: torch.Tensor, 
     equivalent to
     grad.add_(p.data * (1 - p.mask), alpha=decay)
     '''
+    if _ext.host.masked_add(grad, p_data, p_mask, alpha):      # float32 tensors of one dense layout
+        return
     assert grad.is_cuda and p_data.is_cuda and p_mask.is_cuda
     _ext.require_cuda(grad, p_data, p_mask)
     assert (grad.layout, p_data.layout, p_mask.layout) == (torch.strided, torch.strided, torch.strided)

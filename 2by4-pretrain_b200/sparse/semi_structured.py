@@ -13,7 +13,7 @@ from typing import Any, Optional
 
 import torch
 
-from . import _ext
+from ._semi_structured_conversions import compress
 from .sparse_semi_structured_linear import sparse_semi_structured_linear
 
 __all__ = [
@@ -32,14 +32,6 @@ _DTYPE_TO_SEMI_STRUCTURED_SPARSE_CONFIG = {
     torch.float16: _SEMI_STRUCTURED_SPARSE_CONFIG(9, 32, 64, 8, 8),
     torch.bfloat16: _SEMI_STRUCTURED_SPARSE_CONFIG(9, 32, 64, 8, 8),
 }
-
-
-def _indices_dtype(values_dtype):
-    if values_dtype in (torch.int8, torch.float8_e5m2, torch.float8_e4m3fn):
-        return torch.int32
-    if values_dtype in (torch.float16, torch.bfloat16):
-        return torch.int16
-    raise RuntimeError(f"Datatype {values_dtype}  is not supported!")
 
 
 class SparseSemiStructuredTensor(torch.Tensor):
@@ -123,20 +115,8 @@ class SparseSemiStructuredTensor(torch.Tensor):
                 raise RuntimeError("Error using MVUE24 with mask is not supported! ")
 
             # one allocation: packed values first, metadata behind (m*n*cf/16 elements of dtype)
-            compressed_size = original_tensor.nelement() * cfg.compression_factor // 16
-            compressed_tensor = torch.empty((compressed_size,), dtype=dtype, device=original_tensor.device)
-            indices_dtype = _indices_dtype(dtype)
-            row_stride, col_stride = original_tensor.stride()
-            if row_stride > col_stride:
-                sparse_tensor_cutlass = compressed_tensor[: m * n // 2].view(m, -1)
-            else:
-                sparse_tensor_cutlass = compressed_tensor[: m * n // 2].view(-1, m).t()
-            meta_tensor_cutlass = compressed_tensor[m * n // 2:].view(indices_dtype).view(m, -1)
+            sparse_tensor_cutlass, meta_tensor_cutlass = compress(original_tensor.detach(), dtype, MVUE24, mask)
             compressed_tensor_cusparselt = None
-
-            from ._semi_structured_conversions import sparse_semi_structured_from_dense_triton
-            sparse_semi_structured_from_dense_triton(original_tensor.detach(), sparse_tensor_cutlass,
-                                                     meta_tensor_cutlass, MVUE24=MVUE24, mask=mask)
 
         self.original_tensor = None
         self.compressed_tensor_cusparselt = compressed_tensor_cusparselt
@@ -236,7 +216,8 @@ class SparseSemiStructuredTensor(torch.Tensor):
 
         # inference mode does not decompose linear into t + addmm
         if func is torch.ops.aten.linear.default:
-            input_tensor, weight, bias = args
+            input_tensor, weight = args[:2]
+            bias = args[2] if len(args) > 2 else None
             shape = input_tensor.shape
             input_tensor_2d = input_tensor.view(-1, shape[-1])
             row, col = input_tensor_2d.shape

@@ -6,19 +6,16 @@ a transposable 2:4 mask, backward dX = dY W_s through the separately compressed 
 dW = MVUE24(dY^T) X with the gradient compressed on the fly.  ``MyLinear`` / ``SparseLinear`` are the
 older dense-GEMM variants of sparse/sparse_ops.py:8-87 of the reference.
 """
-import random
-
 import torch
 import torch.nn.functional as F
 from torch import autograd, nn
 from torch.amp import custom_fwd, custom_bwd
 
 from . import _ext
-from ._semi_structured_conversions import prune_compress
 from .semi_structured import SparseSemiStructuredTensor, to_sparse_semi_structured
-from .transposable_semi_structured import TransposableSparse, select_and_compress
+from .transposable_semi_structured import TransposableSparse
 from .triton_ops import MVUE24_approx_triton
-from .spmm import sparse_linear as _spmm, sparse_mm_accumulate_ as _spmm_acc, sparse_linear_mlp as _spmm_mlp, mlp_fusable
+from .spmm import sparse_linear as _spmm, sparse_linear_mlp as _spmm_mlp, register_tc_metadata, tc_metadata
 
 
 def _dense_linear(name, dx_weight, doc):
@@ -102,21 +99,6 @@ class sparse_linear_transpose(autograd.Function):
         return grad_input, grad_weight, None, None, grad_bias
 
 
-def _mvue_compress_t(g, row_sums):
-    """MVUE 2:4 compression of ``g.t()`` (features x tokens, column-major) into buffers carved like
-    ``SparseSemiStructuredTensor`` carves them, with the per-feature sums of ``g`` added to ``row_sums``
-    by the same pass.  Returns (packed values, reordered metadata)."""
-    tokens, features = g.shape
-    if features % 32 or tokens % 64:
-        raise RuntimeError(f"gradient of shape {tuple(g.shape)}: features % 32 == 0 and tokens % 64 == 0 required")
-    g = g.contiguous()
-    buf = torch.empty((features * tokens * 9 // 16,), dtype=g.dtype, device=g.device)
-    packed = buf[: features * tokens // 2].view(-1, features).t()
-    meta = buf[features * tokens // 2:].view(torch.int16).view(features, -1)
-    prune_compress(g.t(), packed, meta, mode=_ext.PRUNE_MVUE_FAST, seed=random.randint(0, 2 ** 31 - 1), row_sums=row_sums)
-    return packed, meta
-
-
 def _mm_f32(a, b, acc=None):
     """a @ b (16-bit operands) with a float32 result; added into ``acc`` in the GEMM's epilogue when given."""
     try:
@@ -130,7 +112,8 @@ def _mm_f32(a, b, acc=None):
 
 def _dense_weight_grads(g, x, weight, bias, into_grad, need_w, need_b):
     """The exact dW = g^T x as a dense GEMM with float32 output (the option ``weight_grad = "dense"`` of the layer).
-    Same contract as ``_fst_weight_grads``."""
+    Same contract as the native ``fst_weight_grads``: (grad_weight,
+    grad_bias), each None where it went straight into a ``.grad`` buffer."""
     grad_weight = grad_bias = None
     into = into_grad and weight.grad is not None and weight.grad.dtype == torch.float32 and weight.grad.is_contiguous()
     if need_w:
@@ -145,82 +128,6 @@ def _dense_weight_grads(g, x, weight, bias, into_grad, need_w, need_b):
         else:
             grad_bias = g.sum(0)
     return grad_weight, grad_bias
-
-
-def _fst_weight_grads(g, x, weight, bias, into_grad, need_w, need_b):
-    """dW = MVUE24(g^T) x and db = g.sum(0) of one FST layer; ``g`` (tokens, out_features) and ``x`` (tokens,
-    in_features) are 16-bit.  With ``into_grad`` (and an fp32 ``weight.grad`` already allocated) the GEMM adds dW
-    straight into ``weight.grad`` and the compression pass adds the column sums of ``g`` into ``bias.grad``; autograd
-    then receives None for both.  Returns (grad_weight, grad_bias)."""
-    if getattr(weight, 'weight_grad', 'mvue') == 'dense':
-        return _dense_weight_grads(g, x, weight, bias, into_grad, need_w, need_b)
-    grad_weight = grad_bias = None
-    bias_done = False
-    if need_w:
-        fp32_grad = weight.dtype == torch.float32 and x.shape[1] % 8 == 0
-        target = weight if (into_grad and fp32_grad) else None
-        into = target is not None and target.grad is not None and target.grad.dtype == torch.float32 \
-            and target.grad.is_contiguous()
-        bias_grad = None
-        if into and bias is not None and need_b and g.dtype in (torch.float16, torch.bfloat16):
-            bg = bias.grad
-            if bg is not None and bg.dtype == torch.float32 and bg.is_contiguous():
-                bias_grad = bg
-        if bias_grad is not None:
-            # the pass that compresses dY^T also adds its row sums (= grad_output.sum(0)) to bias.grad
-            gp, gm = _mvue_compress_t(g, bias_grad)
-            bias_done = True
-        else:
-            gs = to_sparse_semi_structured(g.t(), MVUE24=True, dtype=g.dtype)
-            gp, gm = gs.sparse_tensor_cutlass, gs.meta_tensor_cutlass
-        if into:
-            _spmm_acc(target.grad, gp, gm, x)
-        elif fp32_grad:
-            # split-K GEMM with fp32 accumulation: the gradient arrives in the dtype of the master weight
-            grad_weight = torch.zeros((g.shape[1], x.shape[1]), dtype=torch.float32, device=g.device)
-            _spmm_acc(grad_weight, gp, gm, x)
-        else:
-            grad_weight = _spmm(x.t(), gp, gm).t()
-    if bias is not None and need_b and not bias_done:
-        grad_bias = g.sum(0)
-    return grad_weight, grad_bias
-
-
-class _fst_linear(autograd.Function):
-    """What ``sparse_linear_transpose`` computes, on the raw compressed buffers: no tensor-subclass objects,
-    no cast of the (unused) fp32 weight.  ``weight`` only routes the gradient.  With ``into_grad`` the weight
-    gradient is accumulated by the GEMM itself into the existing fp32 ``weight.grad`` (D += A B) and autograd
-    receives no gradient for the weight: no zero-filled temporary, no separate add."""
-
-    @staticmethod
-    def forward(ctx, input, weight, pw, mw, pt, mt, bias, into_grad=False):
-        x = input.reshape(-1, input.shape[-1])
-        if x.dtype != pw.dtype:
-            x = x.to(pw.dtype)
-        ctx.save_for_backward(x, pt, mt)
-        ctx.shape = input.shape
-        ctx.weight, ctx.bias, ctx.into_grad = weight, bias, into_grad
-        if bias is not None and bias.dtype == torch.float32 and mlp_fusable(pw, x):
-            output = _spmm_mlp(x, pw, mw, bias=bias)      # float32 bias read by the epilogue: no cast launch
-        else:
-            b = None if bias is None else (bias if bias.dtype == pw.dtype else bias.to(pw.dtype))
-            output = _spmm(x, pw, mw, bias=b)             # bias added in the GEMM epilogue
-        return output.view(*input.shape[:-1], -1)
-
-    @staticmethod
-    def backward(ctx, grad_output):
-        x, pt, mt = ctx.saved_tensors
-        grad_input = None
-        if grad_output.dim() == 3 and grad_output.stride() == (0, 0, 0):
-            grad_output = torch.ones_like(grad_output)
-        g = grad_output.reshape(-1, grad_output.shape[-1])
-        if g.dtype != pt.dtype:
-            g = g.to(pt.dtype)
-        if ctx.needs_input_grad[0]:
-            grad_input = _spmm(g, pt, mt).view(ctx.shape)
-        grad_weight, grad_bias = _fst_weight_grads(g, x, ctx.weight, ctx.bias, ctx.into_grad, ctx.needs_input_grad[1],
-                                                   ctx.needs_input_grad[6])
-        return grad_input, grad_weight, None, None, None, None, grad_bias, None
 
 
 class _fst_mlp(autograd.Function):
@@ -254,9 +161,9 @@ class _fst_mlp(autograd.Function):
         g = g.contiguous()
         need = ctx.needs_input_grad
         d_pre = _spmm_mlp(g, pt2, mt2, epilogue="dgelu", aux=pre)           # gradient of fc's output, (tokens, 4 d)
-        gw2, gb2 = _fst_weight_grads(g, act, w_proj, b_proj, into_grad, need[3], need[4])
+        gw2, gb2 = _ext.host.fst_weight_grads(g, act, w_proj, b_proj, into_grad, need[3], need[4])
         grad_input = _spmm(d_pre, pt1, mt1).view(ctx.shape) if need[0] else None
-        gw1, gb1 = _fst_weight_grads(d_pre, x, w_fc, b_fc, into_grad, need[1], need[2])
+        gw1, gb1 = _ext.host.fst_weight_grads(d_pre, x, w_fc, b_fc, into_grad, need[1], need[2])
         return grad_input, gw1, gb1, gw2, gb2, None, None, None
 
 
@@ -269,8 +176,12 @@ def fst_mlp(x, fc, proj):
         and fc.bias is not None and proj.bias is not None
     if not ok:
         return proj(F.gelu(fc(x), approximate="tanh"))
-    fc._ensure_compressed()
-    proj._ensure_compressed()
+    for layer in (fc, proj):
+        layer._ensure_compressed()
+        _, mw, _, mt = layer.weight.compressed
+        tcw, tct = layer._tc_copies()
+        register_tc_metadata(mw, tcw)
+        register_tc_metadata(mt, tct)
     y = _fst_mlp.apply(x, w1, fc.bias, w2, proj.bias, w1.compressed, w2.compressed,
                        fc.accumulate_into_grad and proj.accumulate_into_grad)
     fc._advance()
@@ -316,6 +227,7 @@ class SparseLinearTranspose(nn.Linear):
         self.weight.weight_sparse = None
         self.weight.weight_sparse_T = None
         self.weight.compressed = None
+        self.weight.compressed_tc = None
         self.weight.mode = 'sparse'
         self.weight.weight_grad = self.weight_grad
         self.func = func
@@ -332,13 +244,21 @@ class SparseLinearTranspose(nn.Linear):
         dtype = torch.float16
         if torch.is_autocast_enabled('cuda') and torch.get_autocast_dtype('cuda') == torch.bfloat16:
             dtype = torch.bfloat16
-        mask, (pw, mw), (pt, mt) = select_and_compress(w, mask=None if reselect else w.mask, dtype=dtype,
-                                                       mask_out=reuse)
-        w.mask = mask
+        self._take(_ext.host.select_compress(w.detach(), None if reselect else w.mask, dtype, reuse), dtype)
+
+    def _take(self, copies, dtype):
+        """Install (mask, packed_w, meta_w, packed_t, meta_t, tc_w, tc_t) as the compressed copies of the weight."""
+        w = self.weight
+        w.mask, pw, mw, pt, mt, tcw, tct = copies
         w.compressed = (pw, mw, pt, mt)
+        # the metadata in tensor-core order, good for exactly these metadata tensors as they are now
+        w.compressed_tc = (w.compressed, mw._version, mt._version, (tcw, tct)) if tcw is not None else None
         if not self.materialize_sparse_tensors:
             w.weight_sparse = w.weight_sparse_T = None
             return
+        if tcw is not None:
+            register_tc_metadata(mw, tcw)
+            register_tc_metadata(mt, tct)
         out_f, in_f = w.shape
         w.weight_sparse = SparseSemiStructuredTensor(
             None, original_shape=torch.Size([out_f, in_f]), sparse_tensor_cutlass=pw, meta_tensor_cutlass=mw,
@@ -346,6 +266,16 @@ class SparseLinearTranspose(nn.Linear):
         w.weight_sparse_T = SparseSemiStructuredTensor(
             None, original_shape=torch.Size([in_f, out_f]), sparse_tensor_cutlass=pt, meta_tensor_cutlass=mt,
             dtype=dtype)
+
+    def _tc_copies(self):
+        """Both metadata copies in tensor-core order: what the compressing kernel wrote, or converted when it could not,
+        when the copies were replaced by hand or when their metadata was written to since."""
+        w = self.weight
+        pw, mw, pt, mt = w.compressed
+        held = w.compressed_tc
+        if held is not None and held[0] is w.compressed and held[1] == mw._version and held[2] == mt._version:
+            return held[3]
+        return tc_metadata(mw, pw.shape[0], 2 * pw.shape[1]), tc_metadata(mt, pt.shape[0], 2 * pt.shape[1])
 
     def _ensure_compressed(self):
         """Rebuild the mask and / or the compressed copies when this forward pass is due to (first micro-step after an
@@ -375,8 +305,7 @@ class SparseLinearTranspose(nn.Linear):
             x = F.linear(x, w, self.bias)
         else:
             self._ensure_compressed()
-            pw, mw, pt, mt = w.compressed
-            x = _fst_linear.apply(x, w, pw, mw, pt, mt, self.bias, self.accumulate_into_grad)
+            x = _ext.host.fst_linear(x, w, self.bias, w.compressed, self._tc_copies(), self.accumulate_into_grad)
         self._advance()
         return x
 
@@ -387,7 +316,6 @@ def refresh_sparse_layers(model: nn.Module) -> int:
     of W and W^T; done here for all those layers with one kernel launch per 48 weights instead of one per layer.
     Call it right before the forward pass, under the same autocast context.  Layers whose shapes are not
     multiples of 128 are left to refresh themselves.  Returns the number of layers refreshed."""
-    from .transposable_semi_structured import select_and_compress_many
     dtype = torch.float16
     if torch.is_autocast_enabled('cuda') and torch.get_autocast_dtype('cuda') == torch.bfloat16:
         dtype = torch.bfloat16
@@ -405,22 +333,10 @@ def refresh_sparse_layers(model: nn.Module) -> int:
         groups.setdefault((w.counter % w.freq == 0, w.dtype, w.device), []).append(mod)
     done = 0
     for (reselect, _, _), mods in groups.items():
-        res = select_and_compress_many([m.weight for m in mods], [m.weight.mask for m in mods], dtype=dtype,
-                                       reselect=reselect)
-        for mod, (mask, (pw, mw), (pt, mt)) in zip(mods, res):
-            w = mod.weight
-            w.compressed = (pw, mw, pt, mt)
-            w.refreshed = True
-            if mod.materialize_sparse_tensors:
-                out_f, in_f = w.shape
-                w.weight_sparse = SparseSemiStructuredTensor(
-                    None, original_shape=torch.Size([out_f, in_f]), sparse_tensor_cutlass=pw, meta_tensor_cutlass=mw,
-                    dtype=dtype)
-                w.weight_sparse_T = SparseSemiStructuredTensor(
-                    None, original_shape=torch.Size([in_f, out_f]), sparse_tensor_cutlass=pt, meta_tensor_cutlass=mt,
-                    dtype=dtype)
-            else:
-                w.weight_sparse = w.weight_sparse_T = None
+        res = _ext.host.select_compress_many([m.weight.detach() for m in mods], [m.weight.mask for m in mods], dtype, reselect)
+        for mod, copies in zip(mods, res):
+            mod._take(copies, dtype)
+            mod.weight.refreshed = True
             done += 1
     return done
 
@@ -449,5 +365,5 @@ def load_sparse_state(model: nn.Module, state: dict) -> None:
             raise RuntimeError(f"load_sparse_state: mask of {name} has shape {tuple(st['mask'].shape)}, expected {tuple(p.shape)}")
         p.mask = st['mask'].to(device=p.device, dtype=torch.bool)
         p.cnt, p.counter, p.step, p.freq, p.mode = st['cnt'], st['counter'], st['step'], st['freq'], st['mode']
-        p.compressed = None
+        p.compressed = p.compressed_tc = None
         p.weight_sparse = p.weight_sparse_T = None

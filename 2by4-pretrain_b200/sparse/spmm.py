@@ -45,15 +45,17 @@ _status = {}
 
 
 def _status_word(device):
+    """The word the GEMM kernels of ``device`` report a bounded wait that gave up to."""
     t = _status.get(device)
     if t is None:
-        t = torch.zeros(1, dtype=torch.int32, device=device)
-        _status[device] = t
+        t = _status[device] = _ext.host.status_word(device.index if device.index is not None else torch.cuda.current_device())
     return t
 
 
 def check_status(device=None):
     """Synchronises and raises if a bounded on-device wait of the sparse GEMM ever gave up."""
+    if torch.cuda.is_available():
+        _status_word(torch.device("cuda", torch.cuda.current_device()))
     for dev, t in _status.items():
         if device is None or dev == device:
             code = int(t.item())
@@ -101,72 +103,19 @@ def tc_metadata(meta: torch.Tensor, ms: int, k: int) -> torch.Tensor:
 
 def sparse_linear(input, weight, meta, bias=None, activation=None, alpha=None):
     """``alpha`` (float8 operands only, an addition to the reference's contract): the result is
-    alpha * (input @ dense(weight).T) (+ bias) (activation), the dequantisation scale applied in the GEMM epilogue."""
-    _ext.require_cuda(input, weight, meta, bias)
-    if activation not in _ACT:
+    alpha * (input @ dense(weight).T) (+ bias) (activation), the dequantisation scale applied in the GEMM epilogue.
+    fp8 operands give float32 and int8 operands int32 (the reference's table,
+    sparse/csrc/mySparseSemiStructuredLinear_cuda.cu:594-637,729,772), 16-bit operands their own type."""
+    act = _ACT.get(activation, -1)
+    if act < 0:
         raise RuntimeError(f"_sparse_semi_structured_linear: Invalid activation {activation}")
     if weight.dim() != 2:
         raise RuntimeError(f"_sparse_semi_structured_linear: Expected weight argument to be 2D tensor, got {weight.dim()} dims")
-    if input.dtype != weight.dtype:
-        raise RuntimeError(f"_sparse_semi_structured_linear: Expected input datatype {weight.dtype}, but got {input.dtype}")
     ms, kh = weight.shape
-    k = 2 * kh
-    sizes = list(input.shape)
-    if sizes[-1] != k:
-        raise RuntimeError(f"_sparse_semi_structured_linear: Expected weight argument to have {sizes[-1] // 2} columns, but got {kh}")
-    x2 = input.reshape(-1, k)
-    n = x2.shape[0]
-    lay_a = _ext.layout_of(weight)
-    if lay_a is None:
-        raise RuntimeError(f"_sparse_semi_structured_linear: Invalid strides for weight argument: row stride = "
-                           f"{weight.stride(0)}, column stride = {weight.stride(1)}")
-    a_mn, ld_a = lay_a
-    lay_b = _ext.layout_of(x2)
-    if lay_b is None or x2.data_ptr() % 16 or (lay_b[1] * x2.element_size()) % 16:
-        x2 = x2.contiguous()
-        lay_b = (0, k)
-    # layout_of: 0 = rows contiguous along k (K-major for the GEMM), 1 = k strided (the caller passed B.t())
-    b_mn, ld_b = lay_b
-    f8 = weight.dtype in (torch.float8_e4m3fn, torch.float8_e5m2)
-    # fp8 operands give fp32, int8 operands int32 (the reference's table,
-    # sparse/csrc/mySparseSemiStructuredLinear_cuda.cu:594-637,729,772), 16-bit operands their own type
-    out_dtype = torch.float32 if f8 else (torch.int32 if weight.dtype == torch.int8 else weight.dtype)
-    if weight.dtype == torch.int8 and (bias is not None or activation not in (None, "none")):
-        raise RuntimeError("_sparse_semi_structured_linear: the int8 GEMM on sm_100a takes no bias and no activation")
-    if bias is not None:
-        if bias.dim() != 1 or bias.shape[0] != ms:
-            raise RuntimeError(f"_sparse_semi_structured_linear: Expected bias argument to have {ms} elements, but got {bias.numel()}")
-        if bias.dtype != out_dtype:
-            raise RuntimeError(f"two_four_sgemm_cutlass: Expected spars GTEMM bias datatype {out_dtype}, but got {bias.dtype}")
-        bias = bias.contiguous()
     if ms % 128:
         raise RuntimeError("sparse GEMM on sm_100a: number of rows of the sparse matrix must be divisible by 128")
-    e_tc = tc_metadata(meta, ms, k)
-    status = _status_word(weight.device)
-    as_view = b_mn or RETURN_TRANSPOSED_VIEW
-    if as_view:
-        # D (ms, n) row-major, returned as its transposed view (the caller of mm-with-sparse-first
-        # transposes it back, so that result ends up contiguous)
-        out = torch.empty((ms, n), dtype=out_dtype, device=weight.device)
-        trans_out, ld_out = 0, n
-    else:
-        out = torch.empty((n, ms), dtype=out_dtype, device=weight.device)
-        trans_out, ld_out = 1, ms
-    if alpha is not None:
-        if not f8 or a_mn or b_mn:
-            raise RuntimeError("_sparse_semi_structured_linear: alpha is for float8 operands (both K-major) only")
-        rc = _ext.lib().sp24_spmm_scaled(weight.data_ptr(), _ext.dt(weight.dtype), ld_a, e_tc.data_ptr(), ms, k, x2.data_ptr(),
-                                         ld_b, n, out.data_ptr(), trans_out, ld_out, _ext.ptr(bias), _ACT[activation],
-                                         float(alpha), status.data_ptr(), _ext.stream())
-        _ext.check(rc, "sp24_spmm_scaled")
-    else:
-        rc = _ext.lib().sp24_spmm(weight.data_ptr(), _ext.dt(weight.dtype), a_mn, ld_a, e_tc.data_ptr(), ms, k, x2.data_ptr(),
-                                  b_mn, ld_b, n, out.data_ptr(), _ext.dt(out_dtype), trans_out, ld_out, _ext.ptr(bias),
-                                  _ACT[activation], status.data_ptr(), _ext.stream())
-        _ext.check(rc, "sp24_spmm")
-    res = out.t() if as_view else out
-    sizes[-1] = ms
-    return res.reshape(sizes) if len(sizes) != 2 else res
+    _ext.require_cuda(meta)
+    return _ext.host.sparse_linear(input, weight, tc_metadata(meta, ms, 2 * kh), bias, act, alpha, RETURN_TRANSPOSED_VIEW)
 
 
 _EPILOGUE = {"none": 0, "gelu": 1, "dgelu": 2}
@@ -231,27 +180,6 @@ def sparse_mm_accumulate_(out: torch.Tensor, weight: torch.Tensor, meta: torch.T
     operand (row- or column-major packed values), ``dense`` is row-major.  K is split over idle SMs and the
     partial products are added with fp32 reductions, so ``out`` may already hold a gradient to add to."""
     _ext.require_cuda(out, weight, meta, dense)
-    if out.dtype != torch.float32 or out.dim() != 2 or out.stride(1) != 1:
-        raise RuntimeError("sparse_mm_accumulate_: out must be a row-major fp32 matrix")
-    if weight.dtype not in (torch.float16, torch.bfloat16) or dense.dtype != weight.dtype:
-        raise RuntimeError(f"sparse_mm_accumulate_: expected matching fp16 / bf16 operands, got {weight.dtype} and {dense.dtype}")
     ms, kh = weight.shape
-    k = 2 * kh
-    if dense.dim() != 2 or dense.shape[0] != k:
-        raise RuntimeError(f"sparse_mm_accumulate_: dense operand must have {k} rows, got {tuple(dense.shape)}")
-    n = dense.shape[1]
-    if tuple(out.shape) != (ms, n):
-        raise RuntimeError(f"sparse_mm_accumulate_: out must be {(ms, n)}, got {tuple(out.shape)}")
-    lay_a = _ext.layout_of(weight)
-    if lay_a is None:
-        raise RuntimeError("sparse_mm_accumulate_: invalid strides for the packed values")
-    a_mn, ld_a = lay_a
-    if dense.stride(1) != 1 or dense.data_ptr() % 16 or (dense.stride(0) * dense.element_size()) % 16:
-        dense = dense.contiguous()
-    e_tc = tc_metadata(meta, ms, k)
-    status = _status_word(weight.device)
-    rc = _ext.lib().sp24_spmm_accumulate_f32(weight.data_ptr(), _ext.dt(weight.dtype), a_mn, ld_a, e_tc.data_ptr(), ms, k,
-                                             dense.data_ptr(), dense.stride(0), n, out.data_ptr(), out.stride(0),
-                                             k_splits, status.data_ptr(), _ext.stream())
-    _ext.check(rc, "sp24_spmm_accumulate_f32")
+    _ext.host.sparse_mm_accumulate(out, weight, tc_metadata(meta, ms, 2 * kh), dense, k_splits)
     return out

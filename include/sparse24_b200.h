@@ -65,6 +65,9 @@ const char *sp24_strerror(int code);
 /* ABI version of the loaded library (bumped when a signature changes). */
 int sp24_abi_version(void);
 
+/* Zero `bytes` bytes of device memory on `stream` (an output that a following kernel adds to). */
+int sp24_zero(void *dst, int64_t bytes, void *stream);
+
 /*
  * Peer memory for a gradient exchange that runs on the copy engines instead of on SMs (no counterpart in the
  * reference): map a buffer another process of this node exported (a 64-byte cudaIpcMemHandle_t, e.g. from
