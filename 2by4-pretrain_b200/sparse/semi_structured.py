@@ -13,8 +13,11 @@ from typing import Any, Optional
 
 import torch
 
+from . import spmm
 from ._semi_structured_conversions import compress
 from .sparse_semi_structured_linear import sparse_semi_structured_linear
+
+_aten = torch.ops.aten
 
 __all__ = [
     "SparseSemiStructuredTensor",
@@ -174,28 +177,40 @@ class SparseSemiStructuredTensor(torch.Tensor):
             return torch.nn.functional.pad(original_tensor, (0, to_pad_n, 0, to_pad_m))
         return original_tensor
 
+    def _times_dense(self, dense: torch.Tensor, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
+        """dense @ W^T (+ bias) for a token-major or k-strided ``dense`` of any rank."""
+        if dense.stride(-1) == 1 and not spmm.RETURN_TRANSPOSED_VIEW:
+            # tokens are rows of the operand and of the result: the GEMM clips a ragged last tile, nothing to pad
+            return spmm.sparse_linear(dense, self.sparse_tensor_cutlass, self.meta_tensor_cutlass, bias)
+        shape = dense.shape
+        dense = dense.view(-1, shape[-1])
+        row = dense.shape[0]
+        res = sparse_semi_structured_linear(self._pad_tensor_for_matmul(dense), self.sparse_tensor_cutlass, self.meta_tensor_cutlass,
+                                            bias_opt=bias)[:row, :]
+        return res if len(shape) == 2 else res.view(*shape[:-1], -1)
+
     @classmethod
     def __torch_dispatch__(cls, func, types, args, kwargs) -> Any:
+        # inference mode does not decompose linear into t + addmm
+        if func is _aten.linear.default:
+            if isinstance(args[1], cls):
+                return args[1]._times_dense(args[0], args[2] if len(args) > 2 else None)
+
         # below autograd: detach only rewraps the same buffers
-        if func is torch.ops.aten.detach.default:
+        elif func is _aten.detach.default:
             return args[0]._copy_with(args[0].shape, args[0].transposed)
 
         # the compressed form cannot be transposed; only the flag and the logical shape flip
-        if func is torch.ops.aten.t.default:
+        elif func is _aten.t.default:
             return args[0]._copy_with(torch.Size([args[0].shape[1], args[0].shape[0]]), not args[0].transposed)
 
-        if func is torch.ops.aten.addmm.default:
+        elif func is _aten.addmm.default:
             bias, input_A, input_B = args
             # F.linear(x) = addmm(bias, x, W.t()) = (W x' + b')'
             if isinstance(input_B, cls) and input_B.transposed:
-                row, col = input_A.shape
-                input_A_padded = input_B._pad_tensor_for_matmul(input_A)
-                assert input_B.sparse_tensor_cutlass is not None and input_B.meta_tensor_cutlass is not None
-                res = sparse_semi_structured_linear(input_A_padded, input_B.sparse_tensor_cutlass,
-                                                    input_B.meta_tensor_cutlass, bias_opt=bias)
-                return res[:row, :]
+                return input_B._times_dense(input_A, bias)
 
-        if func is torch.ops.aten.mm.default:
+        elif func is _aten.mm.default:
             input_A, input_B = args
             # first operand sparse: D = A_sparse @ B
             if isinstance(input_A, cls) and not input_A.transposed:
@@ -207,31 +222,12 @@ class SparseSemiStructuredTensor(torch.Tensor):
                 return res[:, :col]
             # second operand sparse and transposed: D = A @ W_sparse.t()
             elif isinstance(input_B, cls) and input_B.transposed:
-                row, col = input_A.shape
-                input_A_padded = input_B._pad_tensor_for_matmul(input_A)
-                assert input_B.sparse_tensor_cutlass is not None and input_B.meta_tensor_cutlass is not None
-                res = sparse_semi_structured_linear(input_A_padded, input_B.sparse_tensor_cutlass,
-                                                    input_B.meta_tensor_cutlass)
-                return res[:row, :]
+                return input_B._times_dense(input_A)
 
-        # inference mode does not decompose linear into t + addmm
-        if func is torch.ops.aten.linear.default:
-            input_tensor, weight = args[:2]
-            bias = args[2] if len(args) > 2 else None
-            shape = input_tensor.shape
-            input_tensor_2d = input_tensor.view(-1, shape[-1])
-            row, col = input_tensor_2d.shape
-            if isinstance(weight, cls):
-                input_tensor_2d_padded = weight._pad_tensor_for_matmul(input_tensor_2d)
-                assert weight.sparse_tensor_cutlass is not None and weight.meta_tensor_cutlass is not None
-                res = sparse_semi_structured_linear(input_tensor_2d_padded, weight.sparse_tensor_cutlass,
-                                                    weight.meta_tensor_cutlass, bias_opt=bias)
-                return res[:row, :].view(*shape[:-1], -1)
-
-        if func is torch.ops.aten.values.default:
+        if func is _aten.values.default:
             return args[0].sparse_tensor_cutlass.detach()
 
-        if func is torch.ops.aten.indices.default:
+        if func is _aten.indices.default:
             return args[0].meta_tensor_cutlass
 
         error_string = "\n".join(

@@ -92,6 +92,9 @@ def tc_metadata(meta: torch.Tensor, ms: int, k: int) -> torch.Tensor:
     hit = _tc_meta_cache.get(id(meta))
     e = hit[1] if hit is not None and hit[0]() is meta and hit[2] == _stamp(meta) else None
     if e is None:
+        _ext.require_cuda(meta)
+        if ms % 128:
+            raise RuntimeError("sparse GEMM on sm_100a: number of rows of the sparse matrix must be divisible by 128")
         lib = _ext.lib()
         e = torch.empty(tc_bytes(ms, k), dtype=torch.uint8, device=meta.device)
         src = meta if meta.is_contiguous() else meta.contiguous()
@@ -112,9 +115,6 @@ def sparse_linear(input, weight, meta, bias=None, activation=None, alpha=None):
     if weight.dim() != 2:
         raise RuntimeError(f"_sparse_semi_structured_linear: Expected weight argument to be 2D tensor, got {weight.dim()} dims")
     ms, kh = weight.shape
-    if ms % 128:
-        raise RuntimeError("sparse GEMM on sm_100a: number of rows of the sparse matrix must be divisible by 128")
-    _ext.require_cuda(meta)
     return _ext.host.sparse_linear(input, weight, tc_metadata(meta, ms, 2 * kh), bias, act, alpha, RETURN_TRANSPOSED_VIEW)
 
 
