@@ -409,6 +409,160 @@ extern "C" int sp24_masked_add(void *grad, const void *p, const void *mask, int 
 }
 
 // ---------------------------------------------------------------------------------------------
+// Per-tensor float8 quantisation without a trip to the host: absolute maximum, then the quantised copy (and its
+// transpose, the K-major operand of the weight-gradient GEMM) in one pass each
+// ---------------------------------------------------------------------------------------------
+namespace sp24 {
+namespace {
+
+// Bit patterns of non-negative floats order like unsigned integers (NaN above everything), so the reduction is integer.
+template <typename T> __device__ __forceinline__ uint32_t abs_bits_max(const uint4 &r) {
+    if constexpr (sizeof(T) == 2) {
+        uint32_t m = __vmaxu2(__vmaxu2(r.x & 0x7FFF7FFFu, r.y & 0x7FFF7FFFu), __vmaxu2(r.z & 0x7FFF7FFFu, r.w & 0x7FFF7FFFu));
+        m = max(m & 0xFFFFu, m >> 16);
+        return m;
+    } else {
+        return max(max(r.x & 0x7FFFFFFFu, r.y & 0x7FFFFFFFu), max(r.z & 0x7FFFFFFFu, r.w & 0x7FFFFFFFu));
+    }
+}
+
+template <typename T, bool MASK>
+__global__ void __launch_bounds__(256) absmax_kernel(const uint4 *x, const uint32_t *mask, float *amax, int64_t nvec) {
+    uint32_t m = 0;
+    const int64_t stride = (int64_t)gridDim.x * 256;
+    for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < nvec; i += 4 * stride) {
+        uint4 r[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            r[j] = make_uint4(0, 0, 0, 0);
+            const int64_t at = i + j * stride;
+            if (at < nvec) {
+                r[j] = x[at];
+                if constexpr (MASK) {   // float32 only: four values, four mask bytes
+                    const uint32_t k = mask[at];
+                    if (!(k & 0xFFu)) r[j].x = 0;
+                    if (!(k & 0xFF00u)) r[j].y = 0;
+                    if (!(k & 0xFF0000u)) r[j].z = 0;
+                    if (!(k & 0xFF000000u)) r[j].w = 0;
+                }
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) m = max(m, abs_bits_max<T>(r[j]));
+    }
+    if constexpr (sizeof(T) == 2) {
+        const uint16_t b = (uint16_t)m;
+        m = __float_as_uint(Elem<T>::to_f32(*reinterpret_cast<const T *>(&b)));
+    }
+    m = __reduce_max_sync(0xFFFFFFFFu, m);
+    __shared__ uint32_t part[8];
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int w = 1; w < 8; ++w) m = max(m, part[w]);
+        atomicMax(reinterpret_cast<unsigned int *>(amax), m);
+    }
+}
+
+// q = x * f8_quant_scale(amax) as e4m3, row-major; q_t (optional): its transpose.  A block takes 128 rows x 64 columns
+// through shared memory; a thread then owns one column's 32 rows: one whole 32-byte sector of the transposed row.
+template <typename T>
+__global__ void __launch_bounds__(256) quantize_f8_kernel(const T *x, int64_t rows, int64_t cols, int64_t ld, const float *amax, uint8_t *q,
+                                                          uint8_t *q_t, int64_t ld_t) {
+    __shared__ float sc;
+    __shared__ __align__(16) uint8_t tile[128][64 + 8];
+    if (threadIdx.x == 0) sc = f8_quant_scale(*amax);
+    __syncthreads();
+    const float scale = sc;
+    const int64_t r0 = (int64_t)blockIdx.y * 128, c0 = (int64_t)blockIdx.x * 64;
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+        const int rr = p * 32 + (threadIdx.x >> 3), cc = (threadIdx.x & 7) * 8;
+        const int64_t r = r0 + rr, c = c0 + cc;
+        if (r < rows && c < cols) {
+            float f[8];
+            constexpr int PER = 16 / sizeof(T);
+#pragma unroll
+            for (int v = 0; v < 8 / PER; ++v) {
+                const Vec<T, PER> in = load_vec<T, PER>(x + r * ld + c + v * PER);
+#pragma unroll
+                for (int j = 0; j < PER; ++j) f[v * PER + j] = __fmul_rn(Elem<T>::to_f32(in.v[j]), scale);
+            }
+            uint2 o;
+            uint16_t *h = reinterpret_cast<uint16_t *>(&o);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) h[j] = __nv_cvt_float2_to_fp8x2(make_float2(f[2 * j], f[2 * j + 1]), __NV_SATFINITE, __NV_E4M3);
+            *reinterpret_cast<uint2 *>(q + r * cols + c) = o;
+            if (q_t) *reinterpret_cast<uint2 *>(&tile[rr][cc]) = o;
+        }
+    }
+    if (!q_t) return;
+    __syncthreads();
+    const int cc = threadIdx.x & 63, rr = (threadIdx.x >> 6) * 32;
+    const int64_t c = c0 + cc, r = r0 + rr;
+    if (c >= cols || r >= rows) return;
+    if (r + 32 <= rows && ld_t % 16 == 0) {
+        uint4 o[2];
+        uint8_t *b = reinterpret_cast<uint8_t *>(o);
+#pragma unroll
+        for (int j = 0; j < 32; ++j) b[j] = tile[rr + j][cc];
+        uint4 *dst = reinterpret_cast<uint4 *>(q_t + c * ld_t + r);
+        dst[0] = o[0];
+        dst[1] = o[1];
+    } else {
+        for (int j = 0; j < 32 && r + j < rows; ++j) q_t[c * ld_t + r + j] = tile[rr + j][cc];
+    }
+}
+
+}  // namespace
+}  // namespace sp24
+
+extern "C" int sp24_absmax(const void *x, int dtype, int64_t count, const void *mask, float *amax, void *stream) {
+    using namespace sp24;
+    if (!x || !amax) return SP24_ERR_ARG;
+    if (dtype != SP24_F32 && dtype != SP24_F16 && dtype != SP24_BF16) return SP24_ERR_DTYPE;
+    if (mask && dtype != SP24_F32) return SP24_ERR_DTYPE;
+    const int per = dtype == SP24_F32 ? 4 : 8;
+    if (count <= 0 || count % per) return SP24_ERR_SHAPE;
+    if (!aligned16(x) || !aligned16(mask)) return SP24_ERR_ALIGN;
+    if (int rc = check_device()) return rc;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (cudaMemsetAsync(amax, 0, sizeof(float), st) != cudaSuccess) { launch_status(); return SP24_ERR_CUDA; }
+    const int64_t nvec = count / per;
+    int64_t blocks = (nvec + 1023) / 1024;
+    const int64_t cap = (int64_t)sm_count() * 8;
+    if (blocks > cap) blocks = cap;
+    const uint4 *xv = static_cast<const uint4 *>(x);
+    const uint32_t *mv = static_cast<const uint32_t *>(mask);
+    if (dtype == SP24_F16) absmax_kernel<__half, false><<<(unsigned)blocks, 256, 0, st>>>(xv, nullptr, amax, nvec);
+    else if (dtype == SP24_BF16) absmax_kernel<__nv_bfloat16, false><<<(unsigned)blocks, 256, 0, st>>>(xv, nullptr, amax, nvec);
+    else if (mask) absmax_kernel<float, true><<<(unsigned)blocks, 256, 0, st>>>(xv, mv, amax, nvec);
+    else absmax_kernel<float, false><<<(unsigned)blocks, 256, 0, st>>>(xv, nullptr, amax, nvec);
+    return launch_status();
+}
+
+extern "C" int sp24_quantize_f8(const void *x, int dtype, int64_t rows, int64_t cols, int64_t ld, const float *amax, void *q, void *q_t,
+                                int64_t ld_t, void *stream) {
+    using namespace sp24;
+    if (!x || !amax || !q) return SP24_ERR_ARG;
+    if (dtype != SP24_F32 && dtype != SP24_F16 && dtype != SP24_BF16) return SP24_ERR_DTYPE;
+    if (rows <= 0 || cols <= 0 || cols % 8) return SP24_ERR_SHAPE;
+    if (ld < cols || (ld * dtype_size(dtype)) % 16 || (q_t && ld_t < rows)) return SP24_ERR_STRIDE;
+    if (!aligned16(x) || !aligned16(q) || !aligned16(q_t)) return SP24_ERR_ALIGN;
+    if ((rows + 127) / 128 > 65535) return SP24_ERR_TOO_LARGE;
+    if (int rc = check_device()) return rc;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const dim3 grid((unsigned)((cols + 63) / 64), (unsigned)((rows + 127) / 128));
+    uint8_t *qb = static_cast<uint8_t *>(q), *tb = static_cast<uint8_t *>(q_t);
+    if (dtype == SP24_F16) quantize_f8_kernel<__half><<<grid, 256, 0, st>>>(static_cast<const __half *>(x), rows, cols, ld, amax, qb, tb, ld_t);
+    else if (dtype == SP24_BF16)
+        quantize_f8_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(static_cast<const __nv_bfloat16 *>(x), rows, cols, ld, amax, qb, tb, ld_t);
+    else quantize_f8_kernel<float><<<grid, 256, 0, st>>>(static_cast<const float *>(x), rows, cols, ld, amax, qb, tb, ld_t);
+    return launch_status();
+}
+
+// ---------------------------------------------------------------------------------------------
 // Masked decay + AdamW in one pass over a flat fp32 parameter range
 // ---------------------------------------------------------------------------------------------
 namespace sp24 {

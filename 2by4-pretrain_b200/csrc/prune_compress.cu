@@ -26,6 +26,9 @@ struct PcParams {
     float out_scale;                        // 8-bit outputs: stored value = value * out_scale (1 = none)
     float soft_scale;                       // soft-threshold mode: kept values are also multiplied by this ...
     int soft_use_scale;                     // ... when this is set (one more rounding in the input type)
+    const float *amax;                      // optional: 8-bit outputs take their scale from this device word (f8_store_scale)
+    void *q_dense;                          // optional (column-major input, 8-bit output): dense * f8_quant_scale in the output
+    int64_t ld_q;                           // type, same storage order, pitch ld_q
 };
 
 // internal mode code of the fused soft-threshold + compress entry point (not part of the public enum)
@@ -49,6 +52,17 @@ template <typename T, int N> __device__ __forceinline__ void store_elems(T *p, c
         for (int j = 0; j < PER; ++j) v.v[j] = in[i * PER + j];
         store_vec<T, PER>(p + i * PER, v);
     }
+}
+
+// V float32 values -> V consecutive float8 values, two per conversion instruction
+template <typename TOut, int V> __device__ __forceinline__ void store_f8(TOut *p, const float (&f)[V]) {
+    constexpr __nv_fp8_interpretation_t KIND = std::is_same<TOut, e5m2_t>::value ? __NV_E5M2 : __NV_E4M3;
+    using R = typename VecBytes<V>::type;
+    Vec<uint16_t, (V + 1) / 2> o;
+#pragma unroll
+    for (int v = 0; v < V; v += 2)
+        o.v[v / 2] = (uint16_t)__nv_cvt_float2_to_fp8x2(make_float2(f[v], v + 1 < V ? f[v + 1] : 0.f), __NV_SATFINITE, KIND);
+    *reinterpret_cast<R *>(p) = *reinterpret_cast<const R *>(&o);
 }
 
 constexpr bool is_mvue(int mode) { return mode == SP24_PRUNE_MVUE || mode == SP24_PRUNE_MVUE_FAST; }
@@ -200,9 +214,29 @@ template <typename T> __device__ __forceinline__ uint32_t mse_lookup(uint32_t lo
 // row-major storage: groups of four run along the contiguous axis.
 // Tile = 32 rows x 32 metadata columns; 8 warps, lane = metadata column, warp w owns rows 4w..4w+3.
 // ---------------------------------------------------------------------------------------------
+// Store scale of an 8-bit output: the caller's, or the reciprocal of the tensor's quantisation scale, worked out by one
+// thread from the absolute maximum that an earlier launch left on the device.  Call with all threads of the block.
+template <typename TOut> __device__ __forceinline__ float out_scale_of(const PcParams &P, float *q_scale = nullptr) {
+    if constexpr (sizeof(TOut) == 1 && !std::is_same<TOut, int8_t>::value) {
+        if (P.amax) {
+            __shared__ float sc[2];
+            if (threadIdx.x == 0) {
+                const float a = *P.amax;
+                sc[0] = f8_store_scale(a);
+                sc[1] = f8_quant_scale(a);
+            }
+            __syncthreads();
+            if (q_scale) *q_scale = sc[1];
+            return sc[0];
+        }
+    }
+    return P.out_scale;
+}
+
 template <typename TIn, typename TOut, int MODE, bool HAS_U>
 __global__ void __launch_bounds__(256, is_mvue(MODE) ? 3 : 1) pc_row_kernel(PcParams P) {
     const uint64_t rng_offset = P.offset + (P.offset_dev ? *P.offset_dev : 0ull);
+    const float out_scale = out_scale_of<TOut>(P);
     constexpr int CH = sizeof(TOut) == 2 ? 16 : 32;  // dense elements per metadata word
     constexpr int MB = sizeof(TOut) == 2 ? 2 : 4;    // bytes per metadata word
     constexpr int GROUP = MB == 2 ? 32 : 16;
@@ -290,12 +324,15 @@ __global__ void __launch_bounds__(256, is_mvue(MODE) ? 3 : 1) pc_row_kernel(PcPa
                                     ((mk[j][4 * g + 3] != 0) << 3);
                         }
                         const uint32_t nib =
-                            do_group<TIn, TOut, MODE>(grp, given, u[2 * h], u[2 * h + 1], out[2 * g], out[2 * g + 1], glut, P.out_scale);
+                            do_group<TIn, TOut, MODE>(grp, given, u[2 * h], u[2 * h + 1], out[2 * g], out[2 * g + 1], glut, out_scale);
                         word |= nib << (4 * g);
                     }
                 }
                 store_elems<TOut, CH / 2>(packed + r * P.ld_packed + c * (CH / 2), out);
                 smeta[lane >> 1][(rr / GROUP) * 2 * GROUP + meta_run_pos<MB>(rr % GROUP, lane & 1)] = (MetaT)word;
+                // 8-bit tensor-core order: 16 bytes per row and 128 columns, i.e. four lanes write one 16-byte piece
+                if constexpr (MB == 4)
+                    if (P.tc) reinterpret_cast<uint32_t *>(P.tc)[(((r >> 7) * P.k_atoms + (c >> 2)) * 128 + (r & 127)) * 4 + (c & 3)] = word;
             }
         }
     }
@@ -354,11 +391,16 @@ template <typename TIn> struct ColVec {
 };
 
 // resident blocks per SM the register budget is set for
-constexpr int col_min_blocks(int mode) { return mode == SP24_PRUNE_MVUE_FAST ? 3 : (mode == SP24_PRUNE_MVUE ? 4 : 1); }
+constexpr int col_min_blocks(int mode, int out_bytes) {
+    // 8-bit outputs hold a row-major strip of packed bytes as well: 128 registers, no spills, instead of 85 with 500 bytes
+    return mode == SP24_PRUNE_MVUE_FAST ? (out_bytes == 1 ? 2 : 3) : (mode == SP24_PRUNE_MVUE ? 4 : 1);
+}
 
 template <typename TIn, typename TOut, int MODE, bool HAS_U, int V>
-__global__ void __launch_bounds__(256, col_min_blocks(MODE)) pc_col_kernel(PcParams P) {
+__global__ void __launch_bounds__(256, col_min_blocks(MODE, sizeof(TOut))) pc_col_kernel(PcParams P) {
     const uint64_t rng_offset = P.offset + (P.offset_dev ? *P.offset_dev : 0ull);
+    float q_scale = 1.f;
+    const float out_scale = out_scale_of<TOut>(P, &q_scale);
     constexpr int CH = sizeof(TOut) == 2 ? 16 : 32;
     constexpr int MB = sizeof(TOut) == 2 ? 2 : 4;
     constexpr int GROUP = MB == 2 ? 32 : 16;
@@ -368,7 +410,8 @@ __global__ void __launch_bounds__(256, col_min_blocks(MODE)) pc_col_kernel(PcPar
     __shared__ __align__(16) MetaT smeta[4][2 * RT];
     // tensor-core order: line L = 16*(r/16) + 8*(c%2) + r%8 of 16 bytes, int16 slot 2*((c/2)%4) + (r/8)%2; the block's
     // RT rows x 8 word columns fill RT whole lines of one atom per 128-row block
-    __shared__ __align__(16) uint16_t stc[MB == 2 ? RT * 8 : 8];
+    // (8-bit outputs: RT rows x 4 32-bit words = RT lines of each of two atoms)
+    __shared__ __align__(16) MetaT stc[RT * 8];
     __shared__ float ssum[8][RT];           // per-warp partial row sums (only used when row sums are asked for)
     constexpr bool KEEP_LUT = MODE == SP24_PRUNE_MVUE_FAST && sizeof(TOut) == 2;
     __shared__ uint32_t glut[KEEP_LUT ? 16 : 1];
@@ -396,6 +439,8 @@ __global__ void __launch_bounds__(256, col_min_blocks(MODE)) pc_col_kernel(PcPar
         // 8-bit outputs can also leave row-major (the K-major operand order of the 8-bit sparse GEMM): a thread's
         // 32 logical columns are 16 contiguous packed bytes of its row
         constexpr bool CAN_RM = sizeof(TOut) == 1;
+        constexpr bool CAN_Q = CAN_RM && !std::is_same<TOut, int8_t>::value;
+        TOut *qdst = CAN_Q && P.q_dense ? static_cast<TOut *>(P.q_dense) + (c * CH) * P.ld_q + r : nullptr;
         TOut orow[CAN_RM ? V : 1][CAN_RM ? CH / 2 : 1];
         // a step = 8 consecutive storage rows = two groups of four per logical row = one Philox block
 #pragma unroll
@@ -409,6 +454,18 @@ __global__ void __launch_bounds__(256, col_min_blocks(MODE)) pc_col_kernel(PcPar
             }
             src += 8 * P.ld_dense;
             if constexpr (MODE == SP24_PRUNE_MASK) msrc += 8 * P.ld_mask;
+            if constexpr (CAN_Q) {
+                if (P.q_dense) {   // the whole tensor quantised on the way (the other operand of the layer's GEMMs)
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        float f[V];
+#pragma unroll
+                        for (int v = 0; v < V; ++v) f[v] = __fmul_rn(Elem<TIn>::to_f32(in[j].v[v]), q_scale);
+                        store_f8<TOut, V>(qdst + j * P.ld_q, f);
+                    }
+                    qdst += 8 * P.ld_q;
+                }
+            }
             if (P.row_sums) {   // sums of the unpruned values, fp32
 #pragma unroll
                 for (int v = 0; v < V; ++v) {
@@ -451,7 +508,7 @@ __global__ void __launch_bounds__(256, col_min_blocks(MODE)) pc_col_kernel(PcPar
                     float ua = 0.f, ub = 0.f;
                     if constexpr (is_mvue(MODE)) { ua = u[v][2 * h]; ub = u[v][2 * h + 1]; }
                     if constexpr (MODE == PRUNE_SOFT) { ua = P.soft_scale; ub = P.soft_use_scale ? 1.f : 0.f; }
-                    const uint32_t nib = do_group<TIn, TOut, MODE>(grp, given, ua, ub, o0.v[v], o1.v[v], glut, P.out_scale);
+                    const uint32_t nib = do_group<TIn, TOut, MODE>(grp, given, ua, ub, o0.v[v], o1.v[v], glut, out_scale);
                     word[v] |= nib << (4 * (step * 2 + h));
                     if constexpr (CAN_RM) {
                         orow[v][(step * 2 + h) * 2] = o0.v[v];
@@ -479,8 +536,11 @@ __global__ void __launch_bounds__(256, col_min_blocks(MODE)) pc_col_kernel(PcPar
         for (int v = 0; v < V; ++v) {
             const int rr = lane * V + v;
             smeta[warp >> 1][(rr / GROUP) * 2 * GROUP + meta_run_pos<MB>(rr % GROUP, warp & 1)] = (MetaT)word[v];
-            if constexpr (MB == 2)
+            if constexpr (MB == 2) {
                 if (P.tc) stc[8 * (16 * (rr >> 4) + 8 * (warp & 1) + (rr & 7)) + 2 * (warp >> 1) + ((rr >> 3) & 1)] = (uint16_t)word[v];
+            } else {
+                if (P.tc) stc[(warp >> 2) * RT * 4 + rr * 4 + (warp & 3)] = word[v];
+            }
         }
     } else {
         if (P.row_sums) {
@@ -519,6 +579,16 @@ __global__ void __launch_bounds__(256, col_min_blocks(MODE)) pc_col_kernel(PcPar
             char *dstm = static_cast<char *>(P.meta) + (cp * 2 * P.m + 2 * r0) * MB + piece * 16;
             *reinterpret_cast<uint4 *>(dstm) = *reinterpret_cast<const uint4 *>(
                 reinterpret_cast<const char *>(&smeta[pair][0]) + piece * 16);
+        }
+    }
+    if constexpr (MB == 4) {
+        if (P.tc) {
+            for (int i = threadIdx.x; i < 2 * RT; i += 256) {
+                const int half = i / RT, pline = i % RT;
+                const int64_t atom = (int64_t)blockIdx.y * 2 + half, gr = r0 + pline;
+                if (pline < rows_here && atom < P.k_atoms)
+                    reinterpret_cast<uint4 *>(P.tc)[((gr >> 7) * P.k_atoms + atom) * 128 + (gr & 127)] = reinterpret_cast<const uint4 *>(stc)[i];
+            }
         }
     }
     if constexpr (MB == 2) {
@@ -590,7 +660,8 @@ static int prune_compress_impl(const void *dense, int dense_dtype, int64_t m, in
                                int mode, const void *mask, int64_t ld_mask, const float *uniforms,
                                int64_t ld_uniforms, uint64_t seed, uint64_t offset, const uint64_t *offset_dev,
                                void *e_tc, float *row_sums, void *stream, int packed_rm = 0, float out_scale = 1.f,
-                               int soft_use_scale = 0, float soft_scale = 1.f) {
+                               int soft_use_scale = 0, float soft_scale = 1.f, const float *amax = nullptr, void *q_dense = nullptr,
+                               int64_t ld_q = 0) {
     using namespace sp24;
     if (!dense || !packed || !meta) return SP24_ERR_ARG;
     const int so = dtype_size(packed_dtype), si = dtype_size(dense_dtype);
@@ -613,12 +684,13 @@ static int prune_compress_impl(const void *dense, int dense_dtype, int64_t m, in
     if (!aligned16(dense) || !aligned16(packed) || !aligned16(meta) || (mask && !aligned16(mask)) ||
         (uniforms && !aligned16(uniforms)))
         return SP24_ERR_ALIGN;
-    if (e_tc && (so != 2 || m % 128 || !aligned16(e_tc))) return SP24_ERR_ARG;
+    if (e_tc && (packed_dtype == SP24_I8 || m % 128 || !aligned16(e_tc))) return SP24_ERR_ARG;
+    if (q_dense && (!amax || !packed_rm || ld_q < m || ld_q % 16 || !aligned16(q_dense))) return SP24_ERR_ARG;
     if (row_sums && (!col_major || (reinterpret_cast<uintptr_t>(row_sums) & 3u))) return SP24_ERR_ARG;
     if (int rc = check_device()) return rc;
     PcParams P{dense, packed, meta, static_cast<const uint8_t *>(mask), uniforms, m, k, ld_dense, ld_packed, ld_mask,
                ld_uniforms, seed, offset, reinterpret_cast<const unsigned long long *>(offset_dev),
-               static_cast<int16_t *>(e_tc), (k + 127) / 128, row_sums, packed_rm, out_scale, soft_scale, soft_use_scale};
+               static_cast<int16_t *>(e_tc), (k + 127) / 128, row_sums, packed_rm, out_scale, soft_scale, soft_use_scale, amax, q_dense, ld_q};
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     switch (dense_dtype) {
         case SP24_F32: return dispatch_out<float>(P, packed_dtype, mode, col_major, st);
@@ -672,6 +744,21 @@ extern "C" int sp24_prune_compress_q8(const void *dense, int dense_dtype, int64_
     return prune_compress_impl(dense, dense_dtype, m, k, ld_dense, col_major, packed, packed_dtype, ld_packed, meta, mode, mask,
                                ld_mask, nullptr, 0, seed, offset, nullptr, nullptr, nullptr, stream, col_major ? 1 : 0,
                                out_scale);
+}
+
+// The same conversion for a layer that never reads its scales back: the stored values' scale comes from the tensor's
+// absolute maximum on the device (sp24_absmax), and the pass that reads dense anyway also leaves the metadata in
+// tensor-core order (e_tc), the float32 row sums of the unpruned values (row_sums, column-major input, added to) and the
+// whole tensor quantised in its own storage order (q_dense, column-major input).  Each of the three may be NULL.
+extern "C" int sp24_prune_compress_q8_dev(const void *dense, int dense_dtype, int64_t m, int64_t k, int64_t ld_dense, int col_major,
+                                          void *packed, int packed_dtype, int64_t ld_packed, void *meta, int mode,
+                                          const void *mask, int64_t ld_mask, const float *amax, uint64_t seed, uint64_t offset,
+                                          void *e_tc, float *row_sums, void *q_dense, int64_t ld_q, void *stream) {
+    if (packed_dtype != SP24_E4M3 && packed_dtype != SP24_E5M2) return SP24_ERR_DTYPE;
+    if (mode > SP24_PRUNE_MVUE_FAST || !amax) return SP24_ERR_ARG;
+    return prune_compress_impl(dense, dense_dtype, m, k, ld_dense, col_major, packed, packed_dtype, ld_packed, meta, mode, mask,
+                               ld_mask, nullptr, 0, seed, offset, nullptr, e_tc, row_sums, stream, col_major ? 1 : 0, 1.f, 0, 1.f, amax,
+                               q_dense, ld_q);
 }
 
 // S-STE forward in one pass: magnitude 2:4 mask, soft threshold of the kept values (one rounding in the input type),

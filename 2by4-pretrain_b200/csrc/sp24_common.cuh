@@ -321,6 +321,16 @@ __device__ __forceinline__ uint32_t mvue24_group_fast(float (&x)[4], float u0, f
 }
 
 // ---------------------------------------------------------------------------------------------
+// float8 scales from a tensor's absolute maximum on the device: the dequantisation scale is amax / 448 in double (1 for
+// an all-zero or NaN tensor), as a host that reads amax back works it out
+// ---------------------------------------------------------------------------------------------
+__device__ __forceinline__ double f8_scale(float amax) { return amax > 0.f ? (double)amax / 448.0 : 1.0; }
+// factor of a plain quantisation pass, value * (1 / scale) in float32 ...
+__device__ __forceinline__ float f8_quant_scale(float amax) { return __fdiv_rn(1.f, (float)f8_scale(amax)); }
+// ... and the one the compressing kernels take (rounded once from double)
+__device__ __forceinline__ float f8_store_scale(float amax) { return (float)(1.0 / f8_scale(amax)); }
+
+// ---------------------------------------------------------------------------------------------
 // host-side helpers
 // ---------------------------------------------------------------------------------------------
 inline bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }

@@ -179,6 +179,8 @@ struct SpmmParams {
     int mblk_per_tile;      // 128-row blocks per tile: 2 (B staged once per 256 rows) or 1 (more, smaller tiles)
     float alpha;            // float32 outputs: D = alpha * (A * B) (+ bias); 16-bit and integer outputs ignore it
     int bias_f32;           // bias holds float32 values instead of values of the output type
+    const float *amax_a, *amax_b;   // float8: absolute maxima of the operands on the device; alpha is the product of their scales
+    int accumulate;         // float8, float32 output (ms, n): add alpha * A * B instead of storing it
     void *aux;              // fused MLP epilogues (CTA-pair kernel): second tensor shaped and pitched like out
     int64_t ld_aux;
 };
@@ -236,8 +238,9 @@ template <bool ACT> __device__ __forceinline__ float finish(float v, int act) {
 // One accumulator word -> one output value.  Integer accumulators pass through untouched: no float operation may
 // see their bits (an add of 0.0f would rewrite -0.0 and signalling-NaN patterns, which are ordinary integers).
 // float32 outputs are scaled first: alpha * acc + bias in one fused multiply-add (alpha = 1 gives acc + bias exactly).
-template <typename OutT, bool ACT> __device__ __forceinline__ OutT emit(uint32_t acc_bits, float bias, int act, float alpha) {
+template <typename OutT, bool ACT, bool SCALED = false> __device__ __forceinline__ OutT emit(uint32_t acc_bits, float bias, int act, float alpha) {
     if constexpr (std::is_same<OutT, int32_t>::value) return (int32_t)acc_bits;
+    else if constexpr (SCALED) return to_out<OutT>(finish<ACT>(fmaf(__uint_as_float(acc_bits), alpha, bias), act));
     else if constexpr (std::is_same<OutT, float>::value) return finish<ACT>(fmaf(__uint_as_float(acc_bits), alpha, bias), act);
     else return to_out<OutT>(finish<ACT>(__uint_as_float(acc_bits) + bias, act));
 }
@@ -245,6 +248,19 @@ template <typename OutT, bool ACT> __device__ __forceinline__ OutT emit(uint32_t
 template <typename OutT, bool ACT> __device__ __forceinline__ uint32_t emit_bits(uint32_t acc_bits, float bias, int act, float alpha) {
     if constexpr (std::is_same<OutT, int32_t>::value) return acc_bits;
     else return __float_as_uint(finish<ACT>(fmaf(__uint_as_float(acc_bits), alpha, bias), act));
+}
+
+template <typename OutT> __device__ __forceinline__ float load_bias(const SpmmParams &P, int64_t row) {
+    return P.bias_f32 ? static_cast<const float *>(P.bias)[row] : from_out<OutT>(static_cast<const OutT *>(P.bias)[row]);
+}
+// single-CTA kernels: float8 products take a float32 bias, the others one in the output type
+template <typename OutT, bool F8> __device__ __forceinline__ float row_bias(const SpmmParams &P, int64_t row) {
+    if constexpr (F8) return static_cast<const float *>(P.bias)[row];
+    else return from_out<OutT>(static_cast<const OutT *>(P.bias)[row]);
+}
+// alpha of a float8 product: given, or from the operands' absolute maxima
+__device__ __forceinline__ float alpha_of(const SpmmParams &P) {
+    return P.amax_a ? (float)(f8_scale(*P.amax_a) * f8_scale(*P.amax_b)) : P.alpha;
 }
 
 __device__ __forceinline__ unsigned long long globaltimer() {
@@ -467,6 +483,7 @@ spmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         const int half = (warp - 2) >> 2;   // which half of the columns
         const int tid = (warp - 2) * 32 + lane;
         OutT *out = static_cast<OutT *>(P.out);
+        const float alpha = F8 ? alpha_of(P) : P.alpha;
         OutT *stg = reinterpret_cast<OutT *>(smem + (size_t)STAGES * STAGE_BYTES);
         int tl = 0;
         for (int unit = blockIdx.x; unit < n_units; unit += gridDim.x, ++tl) {
@@ -490,8 +507,8 @@ spmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                 uint32_t held[NREG];                        // second accumulator, converted, two values per word
                 float bias0 = 0.f, bias1 = 0.f;
                 if (run && P.bias) {
-                    bias0 = from_out<OutT>(static_cast<const OutT *>(P.bias)[m0 + row_in_blk]);
-                    if (n_mblk == 2) bias1 = from_out<OutT>(static_cast<const OutT *>(P.bias)[m0 + BM + row_in_blk]);
+                    bias0 = row_bias<OutT, F8>(P, m0 + row_in_blk);
+                    if (n_mblk == 2) bias1 = row_bias<OutT, F8>(P, m0 + BM + row_in_blk);
                 }
                 const uint32_t acc = tmem_base + ((uint32_t)(quad * 32) << 16) + half * HC;
                 if (run) {
@@ -505,7 +522,7 @@ spmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                             Vec<OutT, 8> o;
 #pragma unroll
                             for (int i = 0; i < 8; ++i)
-                                o.v[i] = emit<OutT, ACT>(v[q * 8 + i], bias0, P.activation, P.alpha);
+                                o.v[i] = emit<OutT, ACT, F8>(v[q * 8 + i], bias0, P.activation, alpha);
                             const int piece = (half * HC + c * 32) / 8 + q;
                             *reinterpret_cast<uint4 *>(stg_row + ((piece ^ swz) << 4)) = *reinterpret_cast<const uint4 *>(&o);
                         }
@@ -524,8 +541,8 @@ spmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
 #pragma unroll
                             for (int i = 0; i < 16; ++i) {
                                 Vec<OutT, 2> o;
-                                o.v[0] = emit<OutT, ACT>(v[2 * i], bias1, P.activation, P.alpha);
-                                o.v[1] = emit<OutT, ACT>(v[2 * i + 1], bias1, P.activation, P.alpha);
+                                o.v[0] = emit<OutT, ACT, F8>(v[2 * i], bias1, P.activation, alpha);
+                                o.v[1] = emit<OutT, ACT, F8>(v[2 * i + 1], bias1, P.activation, alpha);
                                 held[c * 16 + i] = *reinterpret_cast<const uint32_t *>(&o);
                             }
                         }
@@ -597,7 +614,7 @@ spmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                     const int64_t mrow0 = m0 + mb * BM;
                     const int64_t m = mrow0 + row_in_blk;
                     float bias = 0.f;
-                    if (run && P.bias) bias = from_out<OutT>(static_cast<const OutT *>(P.bias)[m]);
+                    if (run && P.bias) bias = row_bias<OutT, F8>(P, m);
                     const uint32_t acc = tmem_base + ((uint32_t)(quad * 32) << 16) + mb * BN;
                     if constexpr (TRANS_OUT) {
                         // 4-byte transposed output, STG_COLS columns at a time; each warp copies its half of a chunk
@@ -617,10 +634,10 @@ spmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
 #pragma unroll
                                     for (int q = 0; q < 8; ++q) {
                                         float4 o;
-                                        o.x = __uint_as_float(emit_bits<OutT, ACT>(v[q * 4 + 0], bias, P.activation, P.alpha));
-                                        o.y = __uint_as_float(emit_bits<OutT, ACT>(v[q * 4 + 1], bias, P.activation, P.alpha));
-                                        o.z = __uint_as_float(emit_bits<OutT, ACT>(v[q * 4 + 2], bias, P.activation, P.alpha));
-                                        o.w = __uint_as_float(emit_bits<OutT, ACT>(v[q * 4 + 3], bias, P.activation, P.alpha));
+                                        o.x = __uint_as_float(emit_bits<OutT, ACT>(v[q * 4 + 0], bias, P.activation, alpha));
+                                        o.y = __uint_as_float(emit_bits<OutT, ACT>(v[q * 4 + 1], bias, P.activation, alpha));
+                                        o.z = __uint_as_float(emit_bits<OutT, ACT>(v[q * 4 + 2], bias, P.activation, alpha));
+                                        o.w = __uint_as_float(emit_bits<OutT, ACT>(v[q * 4 + 3], bias, P.activation, alpha));
                                         *reinterpret_cast<float4 *>(stg_row + (col + q * 4) * 4) = o;
                                     }
                                 }
@@ -663,7 +680,11 @@ spmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                                 tmem_ld_wait();
                                 const int64_t nb = n0 + col;
                                 OutT *row = out + m * P.ld_out + nb;
-                                if constexpr (ACCUM) {
+                                if (ACCUM || (F8 && std::is_same<OutT, float>::value && P.accumulate)) {
+                                    const float al = F8 ? alpha : 1.f;
+#pragma unroll
+                                    for (int i = 0; i < 32; ++i)
+                                        if constexpr (F8) v[i] = __float_as_uint(__uint_as_float(v[i]) * al);
                                     // D += partial product: fp32 reductions in L2, 16 bytes each, no return value
                                     if (nb + 32 <= P.n) {
 #pragma unroll
@@ -681,13 +702,13 @@ spmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                                         Vec<OutT, PER> o;
 #pragma unroll
                                         for (int i = 0; i < PER; ++i)
-                                            o.v[i] = emit<OutT, ACT>(v[q * PER + i], bias, P.activation, P.alpha);
+                                            o.v[i] = emit<OutT, ACT, F8>(v[q * PER + i], bias, P.activation, alpha);
                                         store_vec<OutT, PER>(row + q * PER, o);
                                     }
                                 } else {
                                     for (int i = 0; i < 32; ++i)
                                         if (nb + i < P.n)
-                                            row[i] = emit<OutT, ACT>(v[i], bias, P.activation, P.alpha);
+                                            row[i] = emit<OutT, ACT, F8>(v[i], bias, P.activation, alpha);
                                 }
                             }
                         }
@@ -728,11 +749,13 @@ spmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
 namespace two {
 constexpr int BN2 = 192;                                   // columns of a pair tile
 constexpr int B_HALF_BYTES = (BN2 / 2) * 256;              // 96 rows x two 128-byte K atoms
-constexpr int STAGE2_BYTES = A_STAGE_BYTES + B_HALF_BYTES + 2048;   // 43008
 constexpr int STAGES2 = 5;
-constexpr int SMEM2 = STAGES2 * STAGE2_BYTES + 1024;
-static_assert(STAGE2_BYTES % 1024 == 0, "stages must keep the 1024-byte swizzle alignment");
-static_assert(SMEM2 <= 227 * 1024, "shared memory budget");
+// 8-bit operands: the same bytes per stage (K step 256 instead of 128), twice the metadata
+constexpr int e2_bytes(bool f8) { return f8 ? 4096 : 2048; }
+constexpr int stage2_bytes(bool f8) { return A_STAGE_BYTES + B_HALF_BYTES + e2_bytes(f8); }   // 43008 / 45056
+constexpr int smem2(bool f8) { return STAGES2 * stage2_bytes(f8) + 1024; }
+static_assert(stage2_bytes(false) % 1024 == 0 && stage2_bytes(true) % 1024 == 0, "stages must keep the 1024-byte swizzle alignment");
+static_assert(smem2(true) <= 227 * 1024, "shared memory budget");
 }  // namespace two
 
 __device__ __forceinline__ uint32_t cluster_ctarank() {
@@ -785,17 +808,31 @@ __device__ __forceinline__ void mma_sp_pair(uint32_t d_tmem, uint64_t adesc, uin
         : "memory");
 }
 
-template <bool A_MN, typename OutT, int EPI>
+template <bool F8>
+__device__ __forceinline__ void mma_sp_pair_any(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t e_tmem, uint32_t idesc,
+                                                uint32_t accumulate) {
+    if constexpr (F8)
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %5, 0;\n\t"
+            "tcgen05.mma.sp.cta_group::2.kind::f8f6f4 [%0], %1, %2, [%3], %4, p;\n\t}" ::"r"(d_tmem),
+            "l"(adesc), "l"(bdesc), "r"(e_tmem), "r"(idesc), "r"(accumulate)
+            : "memory");
+    else mma_sp_pair(d_tmem, adesc, bdesc, e_tmem, idesc, accumulate);
+}
+
+template <bool A_MN, typename OutT, int EPI, bool F8>
 __global__ void __launch_bounds__(320, 1)
 spmm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                  const __grid_constant__ CUtensorMap map_e, SpmmParams P) {
     using namespace two;
     constexpr int BN = BN2;
     constexpr int STAGES = STAGES2;
+    constexpr int STAGE2_BYTES = stage2_bytes(F8);
     constexpr int OFF_B = A_STAGE_BYTES, OFF_E = OFF_B + B_HALF_BYTES;
+    constexpr int KE = F8 ? 256 : 128;            // K step of a stage
     constexpr int KSTEPS = 4;
     constexpr uint32_t TMEM_COLS = 512;
-    constexpr int E_COL0 = 2 * BN, E_SLOT = 4;    // two accumulator buffers, then two metadata slots
+    constexpr int E_COL0 = 2 * BN, E_SLOT = F8 ? 8 : 4;    // two accumulator buffers, then two metadata slots
     static_assert(sizeof(OutT) == 2, "16-bit outputs only");
     static_assert(E_COL0 + 2 * E_SLOT <= 512, "tensor memory columns exhausted");
 
@@ -811,7 +848,7 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     const int n_tiles_n = (int)((P.n + BN - 1) / BN);
     const int n_tiles_m = (int)(P.ms / (2 * BM));     // 256-row blocks: one 128-row block per CTA
     const int n_tiles = n_tiles_n * n_tiles_m;        // row block varies fastest over the tile index
-    const int k_iters = (int)((P.k + 127) / 128);
+    const int k_iters = (int)((P.k + KE - 1) / KE);
 
     const uint32_t full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[STAGES]);
     const uint32_t tmem_full0 = smem_u32(&bars[2 * STAGES]), tmem_empty0 = smem_u32(&bars[2 * STAGES + 2]);
@@ -843,7 +880,7 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         if (lane == 0) {
             int g = 0;
             bool ok = true;
-            constexpr uint32_t cta_tx = A_STAGE_BYTES + 2048 + B_HALF_BYTES;
+            constexpr uint32_t cta_tx = A_STAGE_BYTES + e2_bytes(F8) + B_HALF_BYTES;
             for (int tile = pair; tile < n_tiles && ok; tile += n_pairs) {
                 const int mblk = (tile % n_tiles_m) * 2 + (int)rank;
                 const int mrow = mblk * BM;
@@ -857,16 +894,16 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                     const uint32_t full_leader = map_to_cta(full0 + 8 * s, 0);
                     if (rank == 0) mbar_expect_tx(full0 + 8 * s, 2 * cta_tx);
                     if constexpr (!A_MN) {
-                        tma_load_2d_pair(sa, &map_a, it * 64, mrow, full_leader);
+                        tma_load_2d_pair(sa, &map_a, it * (KE / 2), mrow, full_leader);
                     } else {
                         tma_load_2d_pair(sa, &map_a, mrow, it * 64, full_leader);
                         tma_load_2d_pair(sa + 8192, &map_a, mrow + 64, it * 64, full_leader);
                     }
-                    // metadata atom of this row block and K step: two rows of 1024 bytes in the atom table
-                    tma_load_2d_pair(sa + OFF_E, &map_e, 0, (int)(((int64_t)mblk * P.k_atoms + it) * 2), full_leader);
+                    // metadata of this row block and K step: two rows of 1024 bytes per atom of the table (8-bit: two atoms)
+                    tma_load_2d_pair(sa + OFF_E, &map_e, 0, (int)(((int64_t)mblk * P.k_atoms + it * (F8 ? 2 : 1)) * 2), full_leader);
                     // this CTA's half of B: 96 rows x two 128-byte K atoms
-                    tma_load_2d_pair(sb, &map_b, it * 128, brow, full_leader);
-                    tma_load_2d_pair(sb + (BN / 2) * 128, &map_b, it * 128 + 64, brow, full_leader);
+                    tma_load_2d_pair(sb, &map_b, it * KE, brow, full_leader);
+                    tma_load_2d_pair(sb + (BN / 2) * 128, &map_b, it * KE + KE / 2, brow, full_leader);
                     SP24_TRACE(0, g);
                 }
             }
@@ -907,10 +944,12 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                     const uint32_t e_cols = tmem_base + E_COL0 + eslot;
                     if (elect_one()) {
                         tc_cp_128x128b_pair(e_cols, ed);
+                        if constexpr (F8) tc_cp_128x128b_pair(e_cols + 4, ed + (2048 >> 4));
+                        // metadata of an MMA: two columns (8-bit), or the even column of a pair plus a 1-bit selector
 #pragma unroll
                         for (int j = 0; j < KSTEPS; ++j)
-                            mma_sp_pair(acc, ad + j * (A_KSTEP >> 4), bd + (((j >> 1) * ((BN / 2) * 128) + (j & 1) * 64) >> 4),
-                                        e_cols + (j & ~1), idesc0 | (j & 1), (it > 0 || j > 0) ? 1u : 0u);
+                            mma_sp_pair_any<F8>(acc, ad + j * (A_KSTEP >> 4), bd + (((j >> 1) * ((BN / 2) * 128) + (j & 1) * 64) >> 4),
+                                                e_cols + (F8 ? 2 * j : (j & ~1)), F8 ? idesc0 : idesc0 | (j & 1), (it > 0 || j > 0) ? 1u : 0u);
                         tc_commit_pair(empty0 + 8 * s);
                     }
                     __syncwarp();
@@ -929,6 +968,7 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         const int quad = warp & 3, half = (warp - 2) >> 2;
         constexpr int HC = BN / 2, NREG = HC / 2;
         OutT *out = static_cast<OutT *>(P.out);
+        const float alpha = F8 ? alpha_of(P) : 1.f;
         const uint32_t empty_leader0 = map_to_cta(tmem_empty0, 0);
         int tl = 0;
         for (int tile = pair; tile < n_tiles; tile += n_pairs, ++tl) {
@@ -942,7 +982,7 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             uint32_t held[NREG];
             if (run) {
                 float bias = 0.f;
-                if (P.bias) bias = P.bias_f32 ? static_cast<const float *>(P.bias)[mrow] : from_out<OutT>(static_cast<const OutT *>(P.bias)[mrow]);
+                if (P.bias) bias = load_bias<OutT>(P, mrow);
                 const uint32_t acc = tmem_base + ((uint32_t)(quad * 32) << 16) + buf * BN + half * HC;
 #pragma unroll
                 for (int c = 0; c < HC / 32; ++c) {
@@ -956,8 +996,8 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                             o.v[0] = to_out<OutT>(__uint_as_float(v[2 * i]));
                             o.v[1] = to_out<OutT>(__uint_as_float(v[2 * i + 1]));
                         } else {
-                            o.v[0] = to_out<OutT>(__uint_as_float(v[2 * i]) + bias);
-                            o.v[1] = to_out<OutT>(__uint_as_float(v[2 * i + 1]) + bias);
+                            o.v[0] = emit<OutT, false, F8>(v[2 * i], bias, 0, alpha);
+                            o.v[1] = emit<OutT, false, F8>(v[2 * i + 1], bias, 0, alpha);
                         }
                         held[c * 16 + i] = *reinterpret_cast<const uint32_t *>(&o);
                     }
@@ -1345,10 +1385,10 @@ int launch_spmm(const CUtensorMap &ma, const CUtensorMap &mb, SpmmParams P, cuda
 }
 
 // Metadata atoms as a 2-D tensor for TMA: rows of 1024 bytes (256 int32), two rows per 2048-byte atom, no swizzle.
-int make_map_e(CUtensorMap *map, const void *e_tc, int64_t n_atoms) {
+int make_map_e(CUtensorMap *map, const void *e_tc, int64_t n_atoms, int atoms_per_box = 1) {
     const cuuint64_t dims[2] = {256, (cuuint64_t)(2 * n_atoms)};
     const cuuint64_t strides[1] = {1024};
-    const cuuint32_t box[2] = {256, 2};
+    const cuuint32_t box[2] = {256, (cuuint32_t)(2 * atoms_per_box)};
     const cuuint32_t estr[2] = {1, 1};
     EncodeTiledFn encode = encode_tiled_fn();
     if (!encode) return SP24_ERR_CUDA;
@@ -1364,14 +1404,15 @@ int make_map_e(CUtensorMap *map, const void *e_tc, int64_t n_atoms) {
     return r == CUDA_SUCCESS ? SP24_OK : SP24_ERR_CUDA;
 }
 
-template <bool A_MN, typename OutT, int EPI = EPI_PLAIN>
+template <bool A_MN, typename OutT, int EPI = EPI_PLAIN, bool F8 = false>
 int launch_spmm_pair(const CUtensorMap &ma, const CUtensorMap &mb, const CUtensorMap &me, SpmmParams P, cudaStream_t st) {
-    auto kern = spmm_pair_kernel<A_MN, OutT, EPI>;
+    auto kern = spmm_pair_kernel<A_MN, OutT, EPI, F8>;
+    constexpr int SMEM = two::smem2(F8);
     static bool attr_set[64];
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, two::SMEM2) != cudaSuccess)
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess)
             return SP24_ERR_CUDA;
         attr_set[dev] = true;
     }
@@ -1383,7 +1424,7 @@ int launch_spmm_pair(const CUtensorMap &ma, const CUtensorMap &mb, const CUtenso
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(2 * pairs, 1, 1);
     cfg.blockDim = dim3(320, 1, 1);
-    cfg.dynamicSmemBytes = two::SMEM2;
+    cfg.dynamicSmemBytes = SMEM;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1623,6 +1664,62 @@ extern "C" int sp24_spmm_mlp(const void *a_packed, int dtype, int a_mn_major, in
     if (epilogue == EPI_DGELU && bias) return SP24_ERR_ARG;
     return spmm_impl(a_packed, dtype, a_mn_major, ld_a, e_tc, ms, k, b, 0, ld_b, n, out, dtype, 1, ld_out, bias, 0, 1.f, status,
                      stream, bias_is_f32 ? 1 : 0, epilogue, aux, ld_aux);
+}
+
+// The GEMMs of a float8 layer whose scales stay on the device: D = alpha * (A_sparse * B) [+ float32 bias], alpha = the
+// product of the operands' scales, worked out from their absolute maxima (sp24_absmax).
+//   trans_out = 1: out (n, ms) in float32, float16 or bfloat16 (rounded once): the layer's output or input gradient
+//   without a float32 copy.  16-bit outputs of whole 256-row blocks and >= 1024 columns run on CTA pairs.
+//   trans_out = 0: out (ms, n) float32 += alpha * A * B (no bias), K cut into slices over idle SMs: the weight gradient.
+extern "C" int sp24_spmm_f8(const void *a_packed, int dtype, int64_t ld_a, const void *e_tc, int64_t ms, int64_t k, const void *b, int64_t ld_b,
+                            int64_t n, void *out, int out_dtype, int trans_out, int64_t ld_out, const float *bias, const float *amax_a,
+                            const float *amax_b, int *status, void *stream) {
+    if (dtype != SP24_E4M3 && dtype != SP24_E5M2) return SP24_ERR_DTYPE;
+    if (!e_tc || !amax_a || !amax_b || (!trans_out && bias)) return SP24_ERR_ARG;
+    if (out_dtype != SP24_F32 && (!trans_out || (out_dtype != SP24_F16 && out_dtype != SP24_BF16))) return SP24_ERR_DTYPE;
+    if (int rc = validate_spmm_args(a_packed, dtype, 0, ld_a, ms, k, b, 0, ld_b, n, out, SP24_F32, trans_out, ld_out, bias, 0)) return rc;
+    if (!aligned16(e_tc) || (ld_out * dtype_size(out_dtype)) % 16) return SP24_ERR_ALIGN;
+    if (int rc = check_device()) return rc;
+    CUtensorMap map_a, map_b;
+    if (int rc = make_map(&map_a, a_packed, dtype, ms, k / 2, ld_a, 128, 128)) return rc;
+    SpmmParams P{};
+    P.e_tc = e_tc; P.out = out; P.bias = bias; P.bias_f32 = 1; P.ms = ms; P.n = n; P.k = k; P.ld_out = ld_out;
+    P.k_atoms = (k + 127) / 128; P.status = status; P.k_splits = 1; P.alpha = 1.f; P.amax_a = amax_a; P.amax_b = amax_b;
+    const uint32_t fmt = dtype == SP24_E5M2 ? 1u : 0u;
+    P.idesc = (1u << 2) | (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(BM >> 4) << 24);
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (trans_out && out_dtype != SP24_F32 && ms % 256 == 0 && n >= 1024 && pair_kernels_enabled()) {
+        CUtensorMap map_e;
+        if (int rc = make_map(&map_b, b, dtype, n, k, ld_b, 128, two::BN2 / 2)) return rc;
+        if (int rc = make_map_e(&map_e, e_tc, (ms / 128) * P.k_atoms, 2)) return rc;
+        return out_dtype == SP24_F16 ? launch_spmm_pair<false, __half, EPI_PLAIN, true>(map_a, map_b, map_e, P, st)
+                                     : launch_spmm_pair<false, __nv_bfloat16, EPI_PLAIN, true>(map_a, map_b, map_e, P, st);
+    }
+    int bn = 128, mpt = 2;
+    const int sms = sm_count_cached();
+    pick_tile(ms, n, sms, bn, mpt);
+    if (trans_out && out_dtype != SP24_F32) {
+        // narrow tiles only: beside the 16-bit staging buffer a wide tile's stages do not fit twice
+        const int64_t tiles = ((n + 127) / 128) * ((ms / BM + 1) / 2);
+        bn = 128;
+        mpt = tiles >= sms ? 2 : 1;
+    }
+    if (!trans_out) {
+        // widest tile (least operand traffic), then as many K slices as idle SMs allow
+        bn = n >= 192 ? 192 : 128;
+        mpt = ms >= 256 ? 2 : 1;
+        const int64_t tiles = ((n + bn - 1) / bn) * ((ms / BM + mpt - 1) / mpt), k_iters = (k + 255) / 256;
+        int64_t splits = sms / tiles;
+        splits = splits < 1 ? 1 : (splits > k_iters ? k_iters : splits);
+        P.k_splits = (int)splits;
+        P.accumulate = 1;
+    }
+    P.mblk_per_tile = mpt;
+    if (!trans_out) return dispatch_bn<true, false, false, false, float>(bn, b, dtype, n, k, ld_b, map_a, P, st);
+    if (out_dtype == SP24_F32) return dispatch_bn<true, false, false, true, float>(bn, b, dtype, n, k, ld_b, map_a, P, st);
+    if (int rc = make_map(&map_b, b, dtype, n, k, ld_b, 128, 128)) return rc;
+    return out_dtype == SP24_F16 ? launch_spmm<128, true, false, false, true, __half>(map_a, map_b, P, st)
+                                 : launch_spmm<128, true, false, false, true, __nv_bfloat16>(map_a, map_b, P, st);
 }
 
 // The float8 GEMM with the dequantisation folded into the epilogue: D = alpha * (A_sparse * B) [+ bias] [activation],

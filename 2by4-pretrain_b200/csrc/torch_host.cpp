@@ -570,6 +570,180 @@ Tensor fst_linear(const Tensor &input, const Tensor &weight, const OptTensor &bi
 }
 
 // ---------------------------------------------------------------------------------------------
+// float8 FST layer: the per-tensor scales never leave the device
+// ---------------------------------------------------------------------------------------------
+Tensor absmax(const Tensor &x, const Tensor &mask = {}) {
+    Tensor a = empty({1}, at::kFloat, x);
+    check(sp24_absmax(ptr(x), dt(x.scalar_type()), x.numel(), mask.defined() ? ptr(mask) : nullptr, static_cast<float *>(ptr(a)), cur_stream()),
+          "sp24_absmax");
+    return a;
+}
+Tensor quantizable(const Tensor &t) {
+    return (t.scalar_type() == at::kFloat || is16(t.scalar_type()) ? t : t.to(at::kFloat)).contiguous();
+}
+
+struct Q8 { Tensor packed, meta, tc; };
+// e4m3 2:4 compression of the logical (m, k) matrix `dense` under the scale of *amax, packed values row-major.
+Q8 compress_q8(const Tensor &dense_in, int mode, const OptTensor &mask_in, const Tensor &amax, uint64_t seed, const Tensor &row_sums,
+               const Tensor &q_dense) {
+    const int64_t m = dense_in.size(0), k = dense_in.size(1);
+    TORCH_CHECK(m % 32 == 0 && k % 128 == 0, "compress_q8: shape (", m, ", ", k, "): rows % 32 == 0 and columns % 128 == 0 required");
+    Tensor dense = dense_in;
+    Layout l = layout_of(dense);
+    if (!usable(dense, l)) {
+        dense = dense.contiguous();
+        l = {0, k};
+    }
+    OptTensor mask = mask_in;
+    int64_t ld_m = 0;
+    if (mask.has_value()) {
+        mask = as_layout(*mask, l.col);
+        ld_m = layout_of(*mask).ld;
+    }
+    const int64_t vb = m * k / 2, mb = m * k / 8, tb = m % 128 == 0 ? sp24_meta_tc_bytes(m, k) : 0;
+    Tensor buf = empty({align256(vb) + align256(mb) + tb}, at::kByte, dense);
+    Q8 o;
+    o.packed = carve(buf, 0, at::kFloat8_e4m3fn, {m, k / 2}, {k / 2, 1});
+    o.meta = carve(buf, align256(vb), at::kInt, {m, k / 32}, {k / 32, 1});
+    if (tb) o.tc = carve(buf, align256(vb) + align256(mb), at::kByte, {tb}, {1});
+    check(sp24_prune_compress_q8_dev(ptr(dense), dt(dense.scalar_type()), m, k, l.ld, l.col, ptr(o.packed), SP24_E4M3, k / 2, ptr(o.meta), mode,
+                                     ptr(mask), ld_m, static_cast<const float *>(ptr(amax)), seed, 0, tb ? ptr(o.tc) : nullptr,
+                                     row_sums.defined() ? static_cast<float *>(ptr(row_sums)) : nullptr,
+                                     q_dense.defined() ? ptr(q_dense) : nullptr, q_dense.defined() ? q_dense.size(1) : 0, cur_stream()),
+          "sp24_prune_compress_q8");
+    return o;
+}
+
+// (absolute maximum of the masked weight, W: packed, meta, tc, W^T: packed, meta, tc)
+py::tuple fp8_weight(const Tensor &w, const Tensor &mask_in) {
+    Tensor amax;
+    Q8 a, b;
+    {
+        py::gil_scoped_release nogil;
+        NoAutograd guard;
+        require_cuda(w, mask_in);
+        const Tensor mask = mask_in.scalar_type() == at::kBool ? mask_in : mask_in.ne(0);
+        const bool direct = w.scalar_type() == at::kFloat && w.is_contiguous() && mask.is_contiguous() && w.sizes() == mask.sizes() &&
+                            w.numel() % 4 == 0 && aligned(w) && aligned(mask);
+        amax = direct ? absmax(w, mask) : absmax(quantizable(at::where(mask, w, at::zeros({}, w.options()))));
+        a = compress_q8(w, SP24_PRUNE_MASK, mask, amax, 0, {}, {});
+        b = compress_q8(w.t(), SP24_PRUNE_MASK, mask.t(), amax, 0, {}, {});
+    }
+    auto opt = [](const Tensor &t) { return t.defined() ? py::cast(t) : py::object(py::none()); };
+    return py::make_tuple(amax, a.packed, a.meta, opt(a.tc), b.packed, b.meta, opt(b.tc));
+}
+
+// input (n, k) e4m3 times the compressed weight, as (n, ms) in `out_t`
+Tensor spmm_f8(const Tensor &packed, const Tensor &tc, const Tensor &amax_w, const Tensor &xq, const Tensor &amax_x, const Tensor &bias,
+               at::ScalarType out_t) {
+    const int64_t ms = packed.size(0), k = 2 * packed.size(1), n = xq.size(0);
+    TORCH_CHECK(xq.size(1) == k, "_sparse_semi_structured_linear: Expected weight argument to have ", xq.size(1) / 2, " columns, but got ", k / 2);
+    TORCH_CHECK(tc.defined(), "sparse GEMM on sm_100a: number of rows of the sparse matrix must be divisible by 128");
+    const auto kt = is16(out_t) ? out_t : at::kFloat;
+    Tensor out = empty({n, ms}, kt, xq);
+    check(sp24_spmm_f8(ptr(packed), SP24_E4M3, packed.stride(0), ptr(tc), ms, k, ptr(xq), xq.stride(0), n, ptr(out), dt(kt), 1, ms,
+                       bias.defined() ? static_cast<const float *>(ptr(bias)) : nullptr, static_cast<const float *>(ptr(amax_w)),
+                       static_cast<const float *>(ptr(amax_x)), status_ptr(xq), cur_stream()),
+          "sp24_spmm_f8");
+    return kt == out_t ? out : out.to(out_t);
+}
+
+struct Fp8Backward : torch::autograd::Node {
+    Tensor xq_t_, amax_x_, amax_w_, pt_, tct_;
+    bool has_bias_ = false;
+    std::vector<int64_t> shape_;
+    at::ScalarType dtype_ = at::kFloat;
+
+    std::string name() const override { return "Fp8LinearBackward"; }
+    void release_variables() override {
+        xq_t_.reset();
+        pt_.reset();
+    }
+    variable_list apply(variable_list &&grads) override {
+        variable_list out(3);
+        if (!grads[0].defined()) return out;
+        TORCH_CHECK(pt_.defined(), torch::autograd::ERR_BACKWARD_TWICE);
+        const bool need_x = task_should_compute_output(0), need_w = task_should_compute_output(1);
+        bool need_b = has_bias_ && task_should_compute_output(2);
+        uint64_t seed = 0;
+        if (need_w) {
+            py::gil_scoped_acquire gil;
+            seed = python_seed();
+        }
+        NoAutograd guard;
+        const Tensor g = quantizable(grads[0].reshape({-1, grads[0].size(-1)}));
+        const int64_t n = g.size(0), of = g.size(1);
+        const Tensor amax = absmax(g);
+        Tensor gq;
+        if (need_x) gq = empty({n, of}, at::kFloat8_e4m3fn, g);
+        if (need_w) {
+            // one pass over dY: the MVUE compression of dY^T, the quantised dY and the bias gradient
+            const int64_t in_f = xq_t_.size(0), nw = of * in_f;
+            Tensor buf = empty({nw + of}, at::kFloat, g);
+            check(sp24_zero(ptr(buf), (nw + of) * 4, cur_stream()), "sp24_zero");
+            Tensor gw = carve(buf, 0, at::kFloat, {of, in_f}, {in_f, 1}), gb = carve(buf, nw * 4, at::kFloat, {of}, {1});
+            const Q8 c = compress_q8(g.t(), SP24_PRUNE_MVUE_FAST, {}, amax, seed, need_b ? gb : Tensor(), gq);
+            TORCH_CHECK(c.tc.defined(), "sparse GEMM on sm_100a: number of rows of the sparse matrix must be divisible by 128");
+            check(sp24_spmm_f8(ptr(c.packed), SP24_E4M3, n / 2, ptr(c.tc), of, n, ptr(xq_t_), n, in_f, ptr(gw), SP24_F32, 0, in_f, nullptr,
+                               static_cast<const float *>(ptr(amax)), static_cast<const float *>(ptr(amax_x_)), status_ptr(g), cur_stream()),
+                  "sp24_spmm_f8");
+            out[1] = gw;
+            if (need_b) out[2] = gb;
+            need_b = false;
+        } else if (need_x) {
+            check(sp24_quantize_f8(ptr(g), dt(g.scalar_type()), n, of, of, static_cast<const float *>(ptr(amax)), ptr(gq), nullptr, 0, cur_stream()),
+                  "sp24_quantize_f8");
+        }
+        if (need_x) out[0] = spmm_f8(pt_, tct_, amax_w_, gq, amax, {}, dtype_).view(shape_);
+        if (need_b) out[2] = g.sum(0);
+        return out;
+    }
+};
+
+Tensor fp8_linear(const Tensor &input, const Tensor &weight, const OptTensor &bias_in, const Tensor &amax_w, const Tensor &pw,
+                  const OptTensor &tcw, const Tensor &pt, const OptTensor &tct) {
+    require_cuda(input, pw, pt, bias_in);
+    const Tensor bias = bias_in.has_value() ? *bias_in : Tensor();
+    const bool tape = torch::autograd::compute_requires_grad(input, weight, bias);
+    Tensor y, xq_t, amax;
+    {
+        NoAutograd guard;
+        const Tensor x = quantizable(rows2d(input));
+        const int64_t n = x.size(0), k = x.size(1);
+        amax = absmax(x);
+        Tensor xq = empty({n, k}, at::kFloat8_e4m3fn, x);
+        if (tape && weight.requires_grad()) xq_t = empty({k, n}, at::kFloat8_e4m3fn, x);
+        check(sp24_quantize_f8(ptr(x), dt(x.scalar_type()), n, k, k, static_cast<const float *>(ptr(amax)), ptr(xq),
+                               xq_t.defined() ? ptr(xq_t) : nullptr, n, cur_stream()),
+              "sp24_quantize_f8");
+        const Tensor b = bias.defined() ? bias.to(at::kFloat).contiguous() : Tensor();
+        if (b.defined())
+            TORCH_CHECK(b.dim() == 1 && b.size(0) == pw.size(0), "_sparse_semi_structured_linear: Expected bias argument to have ", pw.size(0),
+                        " elements, but got ", b.numel());
+        y = spmm_f8(pw, tcw.has_value() ? *tcw : Tensor(), amax_w, xq, amax, b, input.scalar_type());
+        if (input.dim() != 2) {
+            auto shape = input.sizes().vec();
+            shape.back() = pw.size(0);
+            y = y.view(shape);
+        }
+    }
+    if (tape) {
+        auto node = std::shared_ptr<Fp8Backward>(new Fp8Backward(), torch::autograd::deleteNode);
+        node->set_next_edges(torch::autograd::collect_next_edges(input, weight, bias));
+        node->xq_t_ = xq_t;
+        node->amax_x_ = amax;
+        node->amax_w_ = amax_w;
+        node->pt_ = pt;
+        node->tct_ = tct.has_value() ? *tct : Tensor();
+        node->has_bias_ = bias.defined();
+        node->shape_ = input.sizes().vec();
+        node->dtype_ = input.scalar_type();
+        torch::autograd::set_history(y, node);
+    }
+    return y;
+}
+
+// ---------------------------------------------------------------------------------------------
 // trainer ops around the GEMMs
 // ---------------------------------------------------------------------------------------------
 // Where a backward kernel adds two parameter gradients: straight into existing float32 .grad buffers (autograd then
@@ -889,6 +1063,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
               return std::make_pair(gw.defined() ? OptTensor(gw) : OptTensor(), gb.defined() ? OptTensor(gb) : OptTensor());
           },
           nogil());
+    m.def("fp8_weight", &fp8_weight);
+    m.def("fp8_linear", &fp8_linear, nogil());
     m.def("layer_norm", &layer_norm, nogil());
     m.def("add_layer_norm", &add_layer_norm, nogil());
     m.def("cross_entropy", &cross_entropy, nogil());

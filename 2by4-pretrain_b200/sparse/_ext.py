@@ -39,6 +39,11 @@ _SIGNATURES = {
     "sp24_prune_compress_ex": [_vp, _i32, _i64, _i64, _i64, _i32, _vp, _i32, _i64, _vp, _i32, _vp, _i64, _vp, _i64,
                                _u64, _u64, _vp, _vp, _vp, _vp],
     "sp24_prune_compress_q8": [_vp, _i32, _i64, _i64, _i64, _i32, _vp, _i32, _i64, _vp, _i32, _vp, _i64, _f32, _u64, _u64, _vp],
+    "sp24_absmax": [_vp, _i32, _i64, _vp, _vp, _vp],
+    "sp24_quantize_f8": [_vp, _i32, _i64, _i64, _i64, _vp, _vp, _vp, _i64, _vp],
+    "sp24_prune_compress_q8_dev": [_vp, _i32, _i64, _i64, _i64, _i32, _vp, _i32, _i64, _vp, _i32, _vp, _i64, _vp, _u64, _u64, _vp, _vp,
+                                   _vp, _i64, _vp],
+    "sp24_spmm_f8": [_vp, _i32, _i64, _vp, _i64, _i64, _vp, _i64, _i64, _vp, _i32, _i32, _i64, _vp, _vp, _vp, _vp, _vp],
     "sp24_soft_threshold24_compress": [_vp, _i32, _i64, _i64, _i64, _i32, _vp, _i32, _i64, _vp, _i32, _f32, _vp, _vp],
     "sp24_layernorm_fwd": [_vp, _vp, _vp, _vp, _i32, _vp, _vp, _i64, _i64, _f32, _vp],
     "sp24_layernorm_bwd": [_vp, _i32, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _vp],
@@ -64,6 +69,7 @@ _SIGNATURES = {
     "sp24_masked_add": [_vp, _vp, _vp, _i32, _i64, _f32, _vp],
     "sp24_cross_entropy_fused": [_vp, _i32, _vp, _vp, _vp, _f32, _vp, _i64, _i64, _i64, _i64, _vp],
     "sp24_scale_unless_one": [_vp, _i32, _vp, _i64, _vp],
+    "sp24_column_sums": [_vp, _i32, _i64, _i64, _i64, _vp, _vp],
     "sp24_gelu": [_vp, _vp, _vp, _i32, _i64, _vp],
     "sp24_ipc_open": [_vp, _i32, ctypes.POINTER(ctypes.c_void_p)],
     "sp24_ipc_close": [_vp],

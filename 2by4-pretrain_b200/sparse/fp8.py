@@ -12,14 +12,14 @@ of ``sparse_linear_transpose`` (README.md:169-200 of the reference) run on the f
     dX = (dYq Wq_s)              * (sg * sw)        dYq = dY / sg
     dW = (MVUE24(dY^T)/sg  Xq)   * (sg * sx)        MVUE drawn on the 16-bit gradient, quantised on store
 
-The dequantisation scales are applied in the GEMM epilogue (``sp24_spmm_scaled``).  Scales are per tensor, ``amax / 448``, read back to the host (one synchronisation per quantised tensor): the layer is
-a functional reference of the float8 recipe, not a tuned training loop.
+Scales are per tensor, ``amax / 448``.  The layer keeps them on the device (``sp24_absmax``, ``sp24_quantize_f8``,
+``sp24_prune_compress_q8_dev``, ``sp24_spmm_f8``: no synchronisation); the functions below that take or return a scale as a
+Python float read it back.
 """
 import random
 from typing import Optional
 
 import torch
-from torch import autograd
 
 from . import _ext
 from .spmm import sparse_linear as _spmm
@@ -77,14 +77,19 @@ def compress_q8(dense: torch.Tensor, *, mode: int, mask: Optional[torch.Tensor] 
 class Fp8SparseWeight:
     """W (out_features, in_features) under a transposable 2:4 mask, compressed twice in e4m3 with one scale:
     ``pw, mw`` = W for the forward GEMM, ``pt, mt`` = W^T (K-major, from the transposed view) for the input
-    gradient."""
+    gradient.  The scale stays on the device (``amax``); reading ``scale`` brings it to the host."""
 
     def __init__(self, weight: torch.Tensor, mask: torch.Tensor):
-        w = weight.detach()
-        self.scale = scale_of(torch.where(mask, w, torch.zeros((), dtype=w.dtype, device=w.device)))
-        self.pw, self.mw = compress_q8(w, mode=_ext.PRUNE_MASK, mask=mask, scale=self.scale)
-        self.pt, self.mt = compress_q8(w.t(), mode=_ext.PRUNE_MASK, mask=mask.t(), scale=self.scale)
-        self.shape = tuple(w.shape)
+        self.amax, self.pw, self.mw, self.tcw, self.pt, self.mt, self.tct = _ext.host.fp8_weight(weight.detach(), mask)
+        self.shape = tuple(weight.shape)
+        self._scale = None
+
+    @property
+    def scale(self) -> float:
+        if self._scale is None:
+            a = float(self.amax)
+            self._scale = a / E4M3_MAX if a > 0 else 1.0
+        return self._scale
 
 
 def fst_fp8_forward(xq: torch.Tensor, sx: float, w8: Fp8SparseWeight, bias: Optional[torch.Tensor] = None):
@@ -109,33 +114,11 @@ def fst_fp8_weight_grad(g: torch.Tensor, sg: float, xq_t: torch.Tensor, sx: floa
     return _spmm(xq_t, pg, mg, alpha=sg * sx).t()
 
 
-class sparse_linear_transpose_fp8(autograd.Function):
+class sparse_linear_transpose_fp8:
     """``sparse_linear_transpose`` (README.md:169-200 of the reference) with every GEMM in e4m3.  ``weight`` only
-    routes the gradient; ``w8`` is its compressed form (``Fp8SparseWeight``)."""
+    routes the gradient; ``w8`` is its compressed form (``Fp8SparseWeight``).  The scales of x and dY are taken and
+    applied on the device; results come back in the input's dtype, the weight and bias gradients in float32."""
 
     @staticmethod
-    def forward(ctx, input, weight, w8, bias):
-        x = input.reshape(-1, input.shape[-1])
-        xq, sx = quantize(x)
-        ctx.save_for_backward(xq.t().contiguous())
-        ctx.sx, ctx.w8, ctx.shape, ctx.has_bias, ctx.dtype = sx, w8, input.shape, bias is not None, input.dtype
-        y = fst_fp8_forward(xq, sx, w8, bias)
-        return y.to(input.dtype).view(*input.shape[:-1], -1)
-
-    @staticmethod
-    def backward(ctx, grad_output):
-        (xq_t,) = ctx.saved_tensors
-        g = grad_output.reshape(-1, grad_output.shape[-1])
-        if g.dtype not in (torch.float16, torch.bfloat16, torch.float32):
-            g = g.float()
-        g = g.contiguous()
-        sg = scale_of(g)
-        grad_input = grad_weight = grad_bias = None
-        if ctx.needs_input_grad[0]:
-            gq, _ = quantize(g, sg)
-            grad_input = fst_fp8_input_grad(gq, sg, ctx.w8).to(ctx.dtype).view(ctx.shape)
-        if ctx.needs_input_grad[1]:
-            grad_weight = fst_fp8_weight_grad(g, sg, xq_t, ctx.sx)
-        if ctx.has_bias and ctx.needs_input_grad[3]:
-            grad_bias = g.sum(0)
-        return grad_input, grad_weight, None, grad_bias
+    def apply(input, weight, w8, bias):
+        return _ext.host.fp8_linear(input, weight, bias, w8.amax, w8.pw, w8.tcw, w8.pt, w8.tct)

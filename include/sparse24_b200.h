@@ -143,6 +143,26 @@ int sp24_prune_compress_q8(const void *dense, int dense_dtype, int64_t m, int64_
                            int64_t ld_mask, float out_scale, uint64_t seed, uint64_t offset, void *stream);
 
 /*
+ * Per-tensor float8 quantisation with the scale kept on the device; no counterpart in the reference, whose callers read
+ * the maximum back.  The scale of a tensor is amax / 448 worked out in double (1 for an all-zero tensor).
+ *   sp24_absmax                *amax = max |x| over `count` contiguous values (count a multiple of 16 bytes of x); mask
+ *                              (bytes, float32 x only): positions with mask 0 count as zero
+ *   sp24_quantize_f8           q (rows, cols) e4m3 = x * (1 / scale) in float32, rounded; q_t (optional) its transpose
+ *                              (cols, rows) with pitch ld_t, the K-major operand of the weight-gradient GEMM
+ *   sp24_prune_compress_q8_dev sp24_prune_compress_q8 with out_scale = 1 / scale from *amax; three optional extras from the
+ *                              same pass: the metadata in the order the GEMM reads (e_tc, m % 128 == 0), row_sums[r] +=
+ *                              sum over k of the unpruned dense[r, k] and q_dense = the whole of dense quantised like
+ *                              sp24_quantize_f8 in its own storage order (both column-major input only)
+ */
+int sp24_absmax(const void *x, int dtype, int64_t count, const void *mask, float *amax, void *stream);
+int sp24_quantize_f8(const void *x, int dtype, int64_t rows, int64_t cols, int64_t ld, const float *amax, void *q, void *q_t,
+                     int64_t ld_t, void *stream);
+int sp24_prune_compress_q8_dev(const void *dense, int dense_dtype, int64_t m, int64_t k, int64_t ld_dense, int col_major, void *packed,
+                               int packed_dtype, int64_t ld_packed, void *meta, int mode, const void *mask, int64_t ld_mask,
+                               const float *amax, uint64_t seed, uint64_t offset, void *e_tc, float *row_sums, void *q_dense,
+                               int64_t ld_q, void *stream);
+
+/*
  * 2:4 compressed -> dense (zeros at pruned positions).  Replaces
  * _sparse_semi_structured_to_dense_triton / _sparse_semi_structured_to_dense
  * (sparse/_semi_structured_conversions.py:1163-1274, :217-328).
@@ -365,6 +385,16 @@ int sp24_spmm_scaled(const void *a_packed, int dtype, int64_t ld_a, const void *
                      float alpha, int *status, void *stream);
 
 /*
+ * The GEMMs of a float8 layer whose scales stay on the device: D = alpha * (A_sparse * B) [+ bias], alpha the product of
+ * the operands' scales (see sp24_absmax).  Both operands K-major.  trans_out = 1: out (n, ms) in out_dtype F32, F16 or
+ * BF16 (rounded once from float32), bias float32 or NULL.  trans_out = 0: out (ms, n) float32 += alpha * A * B, no bias, K
+ * cut into slices over idle SMs (fixed sums are not promised: slices are added with float32 reductions).
+ */
+int sp24_spmm_f8(const void *a_packed, int dtype, int64_t ld_a, const void *e_tc, int64_t ms, int64_t k, const void *b, int64_t ld_b,
+                 int64_t n, void *out, int out_dtype, int trans_out, int64_t ld_out, const float *bias, const float *amax_a,
+                 const float *amax_b, int *status, void *stream);
+
+/*
  * Weight-gradient form of the sparse GEMM with fp32 accumulation into the output:
  *   D (ms x n, fp32, row-major, pitch ld_out) += A_sparse (ms x k) * B (k x n, stored row-major, pitch ld_b).
  * Replaces torch.mm(to_sparse_semi_structured(grad_output.t(), MVUE24=True), input) of the reference's training
@@ -435,6 +465,9 @@ int sp24_cross_entropy_bwd(const void *logits, int dtype, const int64_t *targets
 int sp24_cross_entropy_fused(const void *logits, int dtype, const int64_t *targets, float *lse, float *loss, float scale,
                              void *dlogits, int64_t rows, int64_t v, int64_t ld, int64_t ld_out, void *stream);
 int sp24_scale_unless_one(void *g, int dtype, const float *factor, int64_t count, void *stream);
+
+/* out[c] += sum over rows of x (rows, cols; 16-bit, pitch ld, cols % 8 == 0), float32: the bias gradient of a dense layer. */
+int sp24_column_sums(const void *x, int dtype, int64_t rows, int64_t cols, int64_t ld, float *out, void *stream);
 
 /*
  * GELU, tanh form, over `count` contiguous 16-bit values (count % 8 == 0), float32 arithmetic:
