@@ -744,6 +744,98 @@ Tensor fp8_linear(const Tensor &input, const Tensor &weight, const OptTensor &bi
 }
 
 // ---------------------------------------------------------------------------------------------
+// S-STE layer: forward on the sparse tensor cores, both gradients dense (the soft-threshold mask is 2:4 along the rows
+// of W only, so W_s^T has no sparse form, and the weight gradient is the straight-through dY^T X)
+// ---------------------------------------------------------------------------------------------
+struct SoftThresholdBackward : torch::autograd::Node {
+    torch::autograd::SavedVariable x_;
+    Tensor packed_, meta_;
+    bool has_bias_ = false, w_f32_ = false;
+    std::vector<int64_t> shape_;
+
+    std::string name() const override { return "SoftThresholdLinearBackward"; }
+    void release_variables() override {
+        x_.reset_data();
+        packed_.reset();
+    }
+    variable_list apply(variable_list &&grads) override {
+        variable_list out(3);
+        if (!grads[0].defined()) return out;
+        TORCH_CHECK(packed_.defined(), torch::autograd::ERR_BACKWARD_TWICE);
+        const Tensor x = x_.unpack();
+        NoAutograd guard;
+        const Tensor g = grads[0].reshape({-1, grads[0].size(-1)}).to(packed_.scalar_type());
+        const int64_t m = packed_.size(0), k = 2 * packed_.size(1);
+        if (task_should_compute_output(0)) {
+            Tensor w = empty({m, k}, packed_.scalar_type(), packed_);
+            check(sp24_to_dense(ptr(packed_), dt(w.scalar_type()), m, k, k / 2, ptr(meta_), ptr(w), k, cur_stream()), "sp24_to_dense");
+            out[0] = at::mm(g, w).view(shape_);
+        }
+        if (task_should_compute_output(1)) out[1] = w_f32_ ? at::mm(g.t(), x, at::kFloat) : at::mm(g.t(), x);
+        if (has_bias_ && task_should_compute_output(2)) {
+            if (g.is_contiguous() && g.size(1) % 8 == 0 && aligned(g)) {
+                Tensor s = empty({g.size(1)}, at::kFloat, g);
+                check(sp24_zero(ptr(s), g.size(1) * 4, cur_stream()), "sp24_zero");
+                check(sp24_column_sums(ptr(g), dt(g.scalar_type()), g.size(0), g.size(1), g.size(1), static_cast<float *>(ptr(s)), cur_stream()),
+                      "sp24_column_sums");
+                out[2] = s;
+            } else {
+                out[2] = g.sum(0);
+            }
+        }
+        return out;
+    }
+};
+
+// (packed, meta, tc or none) of S(weight) * scale
+std::tuple<Tensor, Tensor, OptTensor> soft_threshold_compress(const Tensor &weight, c10::optional<double> scale, at::ScalarType t) {
+    NoAutograd guard;
+    require_cuda(weight);
+    TORCH_CHECK(weight.dim() == 2, "Expected 2-dimensional dense tensor, got ", weight.dim(), "-dimensional tensor");
+    TORCH_CHECK(is16(t), "soft_threshold24_compress: packed dtype must be float16 or bfloat16, got ", t);
+    const int64_t m = weight.size(0), k = weight.size(1);
+    TORCH_CHECK(m % 32 == 0 && k % 64 == 0, "soft_threshold24_compress: shape (", m, ", ", k, "): rows % 32 == 0 and columns % 64 == 0 required");
+    const Tensor w = as_layout(weight, 0);
+    auto [packed, meta] = carve_compressed(m, k, t, false, w);
+    OptTensor e;
+    if (m % 128 == 0) e = empty({sp24_meta_tc_bytes(m, k)}, at::kByte, w);
+    check(sp24_soft_threshold24_compress(ptr(w), dt(w.scalar_type()), m, k, layout_of(w).ld, 0, ptr(packed), dt(t), k / 2, ptr(meta),
+                                         scale.has_value(), (float)scale.value_or(0.0), const_cast<void *>(ptr(e)), cur_stream()),
+          "sp24_soft_threshold24_compress");
+    return {packed, meta, e};
+}
+
+Tensor soft_threshold_linear(const Tensor &input, const Tensor &weight, const OptTensor &bias, double scale, at::ScalarType t) {
+    auto [packed, meta, e] = soft_threshold_compress(weight.detach(), scale, t);
+    TORCH_CHECK(e.has_value(), "sparse GEMM on sm_100a: number of rows of the sparse matrix must be divisible by 128");
+    require_cuda(input, bias);
+    Tensor x, y;
+    {
+        NoAutograd guard;
+        x = rows2d(input).to(t);
+        y = spmm(x, packed, *e, bias, 0, {}, false, true);
+        if (input.dim() != 2) {
+            auto shape = input.sizes().vec();
+            shape.back() = packed.size(0);
+            y = y.view(shape);
+        }
+    }
+    const Tensor b = bias.has_value() ? *bias : Tensor();
+    if (torch::autograd::compute_requires_grad(input, weight, b)) {
+        auto node = std::shared_ptr<SoftThresholdBackward>(new SoftThresholdBackward(), torch::autograd::deleteNode);
+        node->set_next_edges(torch::autograd::collect_next_edges(input, weight, b));
+        node->x_ = torch::autograd::SavedVariable(x, false);
+        node->packed_ = packed;
+        node->meta_ = meta;
+        node->has_bias_ = b.defined();
+        node->w_f32_ = weight.scalar_type() == at::kFloat;
+        node->shape_ = input.sizes().vec();
+        torch::autograd::set_history(y, node);
+    }
+    return y;
+}
+
+// ---------------------------------------------------------------------------------------------
 // trainer ops around the GEMMs
 // ---------------------------------------------------------------------------------------------
 // Where a backward kernel adds two parameter gradients: straight into existing float32 .grad buffers (autograd then
@@ -1063,6 +1155,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
               return std::make_pair(gw.defined() ? OptTensor(gw) : OptTensor(), gb.defined() ? OptTensor(gb) : OptTensor());
           },
           nogil());
+    m.def("soft_threshold_compress", &soft_threshold_compress, nogil());
+    m.def("soft_threshold_linear", &soft_threshold_linear, nogil());
     m.def("fp8_weight", &fp8_weight);
     m.def("fp8_linear", &fp8_linear, nogil());
     m.def("layer_norm", &layer_norm, nogil());

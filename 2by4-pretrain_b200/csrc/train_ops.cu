@@ -483,6 +483,48 @@ __global__ void __launch_bounds__(256) gelu_kernel(const uint4 *x, const uint4 *
     }
 }
 
+// out[c] += sum over rows of x[r, c] (float32): a warp reads 256 consecutive columns of a row, the block's eight warps
+// take rows in turn, one atomic per column and block at the end
+template <typename T>
+__global__ void __launch_bounds__(256) column_sums_kernel(const T *x, int64_t rows, int64_t cols, int64_t ld, int64_t rows_per_block, float *out) {
+    __shared__ float part[8][256 + 8];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t c = (int64_t)blockIdx.x * 256 + lane * 8;
+    const int64_t r0 = (int64_t)blockIdx.y * rows_per_block, r1 = r0 + rows_per_block < rows ? r0 + rows_per_block : rows;
+    float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    if (c < cols) {
+        int64_t r = r0 + warp;
+        for (; r + 24 < r1; r += 32) {      // four rows in flight
+            uint4 v[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[j] = *reinterpret_cast<const uint4 *>(x + (r + 8 * j) * ld + c);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                float f[8];
+                unpack8<T>(v[j], f);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) s[i] += f[i];
+            }
+        }
+        for (; r < r1; r += 8) {
+            float f[8];
+            unpack8<T>(*reinterpret_cast<const uint4 *>(x + r * ld + c), f);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) s[i] += f[i];
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) part[warp][lane * 8 + i] = s[i];
+    __syncthreads();
+    const int64_t col = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    if (col < cols) {
+        float t = 0.f;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) t += part[w][threadIdx.x];
+        atomicAdd(out + col, t);
+    }
+}
+
 // g *= *factor unless *factor == 1 (the usual case: nothing is read or written then)
 template <typename T>
 __global__ void __launch_bounds__(256) scale_unless_one_kernel(T *g, const float *factor, int64_t nvec) {
@@ -677,6 +719,27 @@ extern "C" int sp24_cross_entropy_fused(const void *logits, int dtype, const int
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     return dtype == SP24_F16 ? ce_fused_launch<__half>(logits, targets, lse, loss, scale, dlogits, rows, v, ld, ld_out, st)
                              : ce_fused_launch<__nv_bfloat16>(logits, targets, lse, loss, scale, dlogits, rows, v, ld, ld_out, st);
+}
+
+extern "C" int sp24_column_sums(const void *x, int dtype, int64_t rows, int64_t cols, int64_t ld, float *out, void *stream) {
+    if (!x || !out) return SP24_ERR_ARG;
+    if (dtype != SP24_F16 && dtype != SP24_BF16) return SP24_ERR_DTYPE;
+    if (rows <= 0 || cols <= 0 || cols % 8) return SP24_ERR_SHAPE;
+    if (ld < cols || ld % 8) return SP24_ERR_STRIDE;
+    if (!aligned16(x)) return SP24_ERR_ALIGN;
+    if (int rc = check_device()) return rc;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    // about four blocks per SM, each with at least one four-row trip of its eight warps
+    const int64_t cb = (cols + 255) / 256;
+    int64_t rb = ((int64_t)sm_count() * 4 + cb - 1) / cb;
+    const int64_t most = (rows + 31) / 32;
+    if (rb > most) rb = most;
+    if (rb > 65535) rb = 65535;
+    const int64_t per = (rows + rb - 1) / rb;
+    const dim3 grid((unsigned)cb, (unsigned)((rows + per - 1) / per));
+    if (dtype == SP24_F16) column_sums_kernel<__half><<<grid, 256, 0, st>>>(static_cast<const __half *>(x), rows, cols, ld, per, out);
+    else column_sums_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(static_cast<const __nv_bfloat16 *>(x), rows, cols, ld, per, out);
+    return launch_status();
 }
 
 extern "C" int sp24_scale_unless_one(void *g, int dtype, const float *factor, int64_t count, void *stream) {
