@@ -29,7 +29,7 @@ __device__ __forceinline__ void dense_group(const T (&in)[4], float u0, float u1
     if constexpr (op_is_mvue(OP)) {
         uint32_t keep;
         if constexpr (OP == OP_MVUE) keep = mvue24_group(x, u0, u1);
-        else keep = mvue24_group_fast(x, u0, u1);
+        else keep = picks_to_keep(mvue24_group_fast(x, u0, u1));
 #pragma unroll
         for (int i = 0; i < 4; ++i) s[i] = ((keep >> i) & 1u) ? Elem<T>::from_f32(x[i]) : zero;
     } else {

@@ -74,14 +74,14 @@ __device__ __forceinline__ void mode_uniform_pairs(uint64_t pair, uint64_t seed,
     else mvue_uniform_pairs(pair, seed, offset, u0a, u1a, u0b, u1b);
 }
 
-// Fast MVUE, after the arithmetic: q[] holds all four quotients, keep the keep mask.  Emits the two stored values
-// and returns the 4-bit code.  16-bit outputs: round all four, then one table lookup (keep_lut = words 64..79 of the
-// group table, in shared memory) and one byte permute gather the two stored ones.
+// Fast MVUE, after the arithmetic: q[] holds all four quotients, picks the two picks (first + 4 * second).  Emits the two
+// stored values and returns the 4-bit code.  16-bit outputs: round all four, then one table lookup (pick_lut, in shared
+// memory) and one byte permute gather the two stored ones.
 template <typename TOut>
-__device__ __forceinline__ uint32_t emit_fast(const float (&q)[4], uint32_t keep, TOut &o0, TOut &o1, const uint32_t *keep_lut,
+__device__ __forceinline__ uint32_t emit_fast(const float (&q)[4], uint32_t picks, TOut &o0, TOut &o1, const uint32_t *pick_lut,
                                               float scale = 1.f) {
     if constexpr (sizeof(TOut) == 2) {
-        const uint32_t e = keep_lut[keep];
+        const uint32_t e = pick_lut[picks];
         const uint32_t o = __byte_perm(Elem<TOut>::pack2(q[0], q[1]), Elem<TOut>::pack2(q[2], q[3]), e >> 8);
         const uint16_t lo = (uint16_t)(o & 0xFFFFu), hi = (uint16_t)(o >> 16);
         o0 = *reinterpret_cast<const TOut *>(&lo);
@@ -89,7 +89,7 @@ __device__ __forceinline__ uint32_t emit_fast(const float (&q)[4], uint32_t keep
         return e & 0xFu;
     } else {
         // 8-bit outputs: the caller's quantisation scale is applied before the cast (one more float32 rounding)
-        const uint32_t nib = encode_nibble(keep);
+        const uint32_t nib = encode_nibble(picks_to_keep(picks));
         o0 = Elem<TOut>::from_f32(__fmul_rn(pick4(nib & 3u, q[0], q[1], q[2], q[3]), scale));
         o1 = Elem<TOut>::from_f32(__fmul_rn(pick4(nib >> 2, q[0], q[1], q[2], q[3]), scale));
         return nib;
@@ -97,19 +97,19 @@ __device__ __forceinline__ uint32_t emit_fast(const float (&q)[4], uint32_t keep
 }
 
 // One group of four: decide the keep mask, emit the two stored values and the 4-bit code.
-// keep_lut: words 64..79 of the group table (indexed by a 4-bit keep mask) in shared memory; only the fast MVUE
+// pick_lut: words 80..95 of the group table (indexed by the two picks of a draw) in shared memory; only the fast MVUE
 // mode with 16-bit outputs reads it.
 template <typename TIn, typename TOut, int MODE>
 __device__ __forceinline__ uint32_t do_group(const TIn (&in)[4], uint32_t given_mask, float u0, float u1, TOut &o0,
-                                             TOut &o1, const uint32_t *keep_lut = nullptr, float scale = 1.f) {
+                                             TOut &o1, const uint32_t *pick_lut = nullptr, float scale = 1.f) {
     // `scale` only acts on 8-bit outputs (float8 quantisation); 16-bit outputs ignore it
     constexpr bool SCALED = sizeof(TOut) == 1 && !std::is_same<TOut, int8_t>::value;
     uint32_t keep;
     if constexpr (MODE == SP24_PRUNE_MVUE_FAST) {
         float x[4] = {Elem<TIn>::to_f32(in[0]), Elem<TIn>::to_f32(in[1]), Elem<TIn>::to_f32(in[2]),
                       Elem<TIn>::to_f32(in[3])};
-        keep = mvue24_group_fast(x, u0, u1);         // all four quotients in x[]
-        return emit_fast<TOut>(x, keep, o0, o1, keep_lut, scale);
+        const uint32_t picks = mvue24_group_fast(x, u0, u1);         // all four quotients in x[]
+        return emit_fast<TOut>(x, picks, o0, o1, pick_lut, scale);
     } else if constexpr (MODE == SP24_PRUNE_MVUE) {
         float x[4] = {Elem<TIn>::to_f32(in[0]), Elem<TIn>::to_f32(in[1]), Elem<TIn>::to_f32(in[2]),
                       Elem<TIn>::to_f32(in[3])};
@@ -161,10 +161,10 @@ __device__ __forceinline__ uint32_t do_group(const TIn (&in)[4], uint32_t given_
 // Table-driven group processing for 16-bit -> same 16-bit type (magnitude and mask modes).
 // Words 0..63: indexed by the six magnitude comparisons x1 | x2<<1 | x3<<2 | x4<<3 | x5<<4 | x6<<5
 // (x1 = |a0|>|a1|, x2 = |a0|>|a2|, x3 = |a0|>|a3|, x4 = |a1|>|a2|, x5 = |a1|>|a3|, x6 = |a2|>|a3|);
-// words 64..79: indexed by a 4-bit keep mask.  Each word: bits 0..3 the metadata code idx0 | idx1<<2,
+// words 64..79: indexed by a 4-bit keep mask; words 80..95: by the two picks of a draw, first + 4 * second.  Each word: bits 0..3 the metadata code idx0 | idx1<<2,
 // bits 8..23 the byte-permute selector that gathers elements idx0, idx1 from a (lo, hi) register pair.
 // ---------------------------------------------------------------------------------------------
-struct GroupLut { uint32_t v[80]; };
+struct GroupLut { uint32_t v[96]; };
 __host__ __device__ constexpr uint32_t lut_word_for_keep(uint32_t keep) {
     const uint32_t m0 = keep & 1u, m1 = (keep >> 1) & 1u, m2 = (keep >> 2) & 1u;
     const uint32_t bit0 = (m0 ^ 1u) & m1, bit1 = (m0 ^ 1u) & (m1 ^ 1u);
@@ -184,6 +184,7 @@ constexpr GroupLut make_group_lut() {
         L.v[i] = lut_word_for_keep((uint32_t)m0 | ((uint32_t)m1 << 1) | ((uint32_t)m2 << 2) | ((uint32_t)m3 << 3));
     }
     for (uint32_t k = 0; k < 16; ++k) L.v[64 + k] = lut_word_for_keep(k);
+    for (uint32_t k = 0; k < 16; ++k) L.v[80 + k] = lut_word_for_keep((1u << (k & 3u)) | (1u << (k >> 2)));
     return L;
 }
 __constant__ GroupLut kGroupLut = make_group_lut();
@@ -247,14 +248,14 @@ __global__ void __launch_bounds__(256, is_mvue(MODE) ? 3 : 1) pc_row_kernel(PcPa
 
     __shared__ __align__(16) MetaT smeta[16][64];
     constexpr bool PACKED = !is_mvue(MODE) && MODE != PRUNE_SOFT && std::is_same<TIn, TOut>::value && sizeof(TIn) == 2;
-    constexpr bool KEEP_LUT = MODE == SP24_PRUNE_MVUE_FAST && sizeof(TOut) == 2;   // words 64..79 only
-    __shared__ uint32_t glut[PACKED ? 80 : (KEEP_LUT ? 16 : 1)];
+    constexpr bool PICK_LUT = MODE == SP24_PRUNE_MVUE_FAST && sizeof(TOut) == 2;   // words 80..95 only
+    __shared__ uint32_t glut[PACKED ? 80 : (PICK_LUT ? 16 : 1)];
     if constexpr (PACKED) {
         if (threadIdx.x < 80) glut[threadIdx.x] = kGroupLut.v[threadIdx.x];
         __syncthreads();
     }
-    if constexpr (KEEP_LUT) {
-        if (threadIdx.x < 16) glut[threadIdx.x] = kGroupLut.v[64 + threadIdx.x];
+    if constexpr (PICK_LUT) {
+        if (threadIdx.x < 16) glut[threadIdx.x] = kGroupLut.v[80 + threadIdx.x];
         __syncthreads();
     }
 
@@ -413,10 +414,10 @@ __global__ void __launch_bounds__(256, col_min_blocks(MODE, sizeof(TOut))) pc_co
     // (8-bit outputs: RT rows x 4 32-bit words = RT lines of each of two atoms)
     __shared__ __align__(16) MetaT stc[RT * 8];
     __shared__ float ssum[8][RT];           // per-warp partial row sums (only used when row sums are asked for)
-    constexpr bool KEEP_LUT = MODE == SP24_PRUNE_MVUE_FAST && sizeof(TOut) == 2;
-    __shared__ uint32_t glut[KEEP_LUT ? 16 : 1];
-    if constexpr (KEEP_LUT) {
-        if (threadIdx.x < 16) glut[threadIdx.x] = kGroupLut.v[64 + threadIdx.x];
+    constexpr bool PICK_LUT = MODE == SP24_PRUNE_MVUE_FAST && sizeof(TOut) == 2;
+    __shared__ uint32_t glut[PICK_LUT ? 16 : 1];
+    if constexpr (PICK_LUT) {
+        if (threadIdx.x < 16) glut[threadIdx.x] = kGroupLut.v[80 + threadIdx.x];
         __syncthreads();
     }
 
@@ -442,7 +443,10 @@ __global__ void __launch_bounds__(256, col_min_blocks(MODE, sizeof(TOut))) pc_co
         constexpr bool CAN_Q = CAN_RM && !std::is_same<TOut, int8_t>::value;
         TOut *qdst = CAN_Q && P.q_dense ? static_cast<TOut *>(P.q_dense) + (c * CH) * P.ld_q + r : nullptr;
         TOut orow[CAN_RM ? V : 1][CAN_RM ? CH / 2 : 1];
-        // a step = 8 consecutive storage rows = two groups of four per logical row = one Philox block
+        // a step = 8 consecutive storage rows = two groups of four per logical row = one Philox block, counted along the row
+        uint64_t pair0[V];
+#pragma unroll
+        for (int v = 0; v < V; ++v) pair0[v] = (uint64_t)(r + v) * (uint64_t)(P.k / 8) + (uint64_t)(c * (CH / 8));
 #pragma unroll
         for (int step = 0; step < CH / 8; ++step) {
             Vec<TIn, V> in[8];
@@ -489,8 +493,7 @@ __global__ void __launch_bounds__(256, col_min_blocks(MODE, sizeof(TOut))) pc_co
                 } else {
 #pragma unroll
                     for (int v = 0; v < V; ++v) {
-                        const uint64_t gi = (uint64_t)(r + v) * (uint64_t)(P.k / 4) + (uint64_t)gcol;
-                        mode_uniform_pairs<MODE>(gi >> 1, P.seed, rng_offset, u[v][0], u[v][1], u[v][2], u[v][3]);
+                        mode_uniform_pairs<MODE>(pair0[v] + step, P.seed, rng_offset, u[v][0], u[v][1], u[v][2], u[v][3]);
                     }
                 }
             }

@@ -255,7 +255,7 @@ __device__ __forceinline__ uint32_t mvue24_group(float (&x)[4], float u0, float 
 //   * S - a_i and K - k_i are taken as the sum of the other three terms, not as a difference: no cancellation when one
 //     magnitude dominates its group, so p_i is good to a few float32 ulps everywhere (the reference order loses up to
 //     ~1e-4 relative there);
-//   * a draw is a count of thresholds below the scaled uniform instead of a cascade of dependent predicates;
+//   * a draw is the last threshold below the scaled uniform instead of a cascade of dependent predicates;
 //   * all four quotients are formed (two more reciprocals) so that the two stored ones can be gathered with one
 //     table-driven byte permute instead of select chains.
 // Every operation is an explicit intrinsic (no compiler contraction), so all kernels that call this function produce
@@ -269,56 +269,53 @@ __device__ __forceinline__ float rcp_fast(float v) {
 }
 constexpr int kMvueFastRounds = 7;
 
-// 23 random bits -> float32 uniform on [0, 1) with 2^-23 spacing (mantissa of a float in [1, 2), minus one)
-__device__ __forceinline__ float u32_to_uniform23(uint32_t x) {
-    return __fadd_rn(__uint_as_float((x & 0x007FFFFFu) | 0x3F800000u), -1.f);
-}
+// 23 random bits -> v = 1 + u, u a float32 uniform on [0, 1) with 2^-23 spacing (v is a float's mantissa in [1, 2)).  A scaled
+// uniform u * s is taken as fma(v, s, -s): the same real number rounded once, without the subtraction.
+__device__ __forceinline__ float u32_to_one_plus_uniform(uint32_t x) { return __uint_as_float((x & 0x007FFFFFu) | 0x3F800000u); }
 
-// Uniform pairs of groups 2*pair and 2*pair+1 for the fast mode: Philox4x32-7, 23-bit uniforms.
-__device__ __forceinline__ void mvue_uniform_pairs_fast(uint64_t pair, uint64_t seed, uint64_t offset, float &u0a,
-                                                        float &u1a, float &u0b, float &u1b) {
+// Uniform pairs (as 1 + u) of groups 2*pair and 2*pair+1 for the fast mode: Philox4x32-7, 23-bit uniforms.
+__device__ __forceinline__ void mvue_uniform_pairs_fast(uint64_t pair, uint64_t seed, uint64_t offset, float &v0a,
+                                                        float &v1a, float &v0b, float &v1b) {
     const uint4 r = philox4x32<kMvueFastRounds>(make_uint4((uint32_t)pair, (uint32_t)(pair >> 32), (uint32_t)offset,
                                                            (uint32_t)(offset >> 32)),
                                                 make_uint2((uint32_t)seed, (uint32_t)(seed >> 32)));
-    u0a = u32_to_uniform23(r.x); u1a = u32_to_uniform23(r.y);
-    u0b = u32_to_uniform23(r.z); u1b = u32_to_uniform23(r.w);
+    v0a = u32_to_one_plus_uniform(r.x); v1a = u32_to_one_plus_uniform(r.y);
+    v0b = u32_to_one_plus_uniform(r.z); v1b = u32_to_one_plus_uniform(r.w);
 }
 
-// number of thresholds c0 <= c1 <= c2 strictly below w: 0..3
-__device__ __forceinline__ uint32_t count_below(float w, float c0, float c1, float c2) {
-    return (uint32_t)(w > c0) + (uint32_t)(w > c1) + (uint32_t)(w > c2);
-}
-
-// x[] is overwritten with x_i / p_i for ALL four positions; returns the keep mask as bits 0..3.
-__device__ __forceinline__ uint32_t mvue24_group_fast(float (&x)[4], float u0, float u1) {
+// x[] is overwritten with x_i / p_i for ALL four positions; v0, v1 are one plus the two uniforms.  Returns the two picks as
+// first + 4 * second.
+//   r_j = a_j / (S - a_j), p_j = a_j (1 + sum of the other r) / S, so x_j / p_j = x_j * (S * rcp(a_j (1 + R_j)))
+__device__ __forceinline__ uint32_t mvue24_group_fast(float (&x)[4], float v0, float v1) {
     const float eps = 1.19209e-07f;
     const float a0 = __fadd_rn(fabsf(x[0]), eps), a1 = __fadd_rn(fabsf(x[1]), eps);
     const float a2 = __fadd_rn(fabsf(x[2]), eps), a3 = __fadd_rn(fabsf(x[3]), eps);
     const float a01 = __fadd_rn(a0, a1), a23 = __fadd_rn(a2, a3);
     const float s = __fadd_rn(a01, a23), a012 = __fadd_rn(a01, a2);
     // sums of the other three
-    const float s0 = __fadd_rn(a1, a23), s1 = __fadd_rn(a0, a23), s2 = __fadd_rn(a01, a3);
-    const float rs = rcp_fast(s);
-    const float t0 = __fmul_rn(a0, rs), t1 = __fmul_rn(a1, rs), t2 = __fmul_rn(a2, rs), t3 = __fmul_rn(a3, rs);
-    const float k0 = __fmul_rn(t0, rcp_fast(s0)), k1 = __fmul_rn(t1, rcp_fast(s1));
-    const float k2 = __fmul_rn(t2, rcp_fast(s2)), k3 = __fmul_rn(t3, rcp_fast(a012));
-    const float k01 = __fadd_rn(k0, k1), k23 = __fadd_rn(k2, k3);
-    const float p0 = __fmaf_rn(a0, __fadd_rn(k1, k23), t0), p1 = __fmaf_rn(a1, __fadd_rn(k0, k23), t1);
-    const float p2 = __fmaf_rn(a2, __fadd_rn(k01, k3), t2), p3 = __fmaf_rn(a3, __fadd_rn(k01, k2), t3);
+    const float r0 = __fmul_rn(a0, rcp_fast(__fadd_rn(a1, a23))), r1 = __fmul_rn(a1, rcp_fast(__fadd_rn(a0, a23)));
+    const float r2 = __fmul_rn(a2, rcp_fast(__fadd_rn(a01, a3))), r3 = __fmul_rn(a3, rcp_fast(a012));
+    const float r01 = __fadd_rn(r0, r1), r23 = __fadd_rn(r2, r3);
     // first pick: the interval of the cumulative sums (a0, a01, a012, s) that u0 * s falls into
-    const float w = __fmul_rn(u0, s);
-    const bool b0 = w > a0, b2 = w > a012;
-    const uint32_t f = (uint32_t)b0 + (uint32_t)(w > a01) + (uint32_t)b2;
+    const float w = __fmaf_rn(v0, s, -s);
+    const bool b0 = w > a0, b1 = w > a01, b2 = w > a012;
     // second pick among the other three: the same walk over the cumulative sums with the first pick's weight zeroed
-    const float d0 = b0 ? a0 : 0.f, d1 = f == 1u ? 0.f : a1, d2 = f == 2u ? 0.f : a2, d3 = b2 ? 0.f : a3;
-    const float d01 = __fadd_rn(d0, d1), d012 = __fadd_rn(d01, d2);
-    const uint32_t g = count_below(__fmul_rn(u1, __fadd_rn(d012, d3)), d0, d01, d012);
-    x[0] = __fmul_rn(x[0], rcp_fast(p0));
-    x[1] = __fmul_rn(x[1], rcp_fast(p1));
-    x[2] = __fmul_rn(x[2], rcp_fast(p2));
-    x[3] = __fmul_rn(x[3], rcp_fast(p3));
-    return (1u << f) | (1u << g);
+    const float d0 = b0 ? a0 : 0.f, d1 = (b0 && !b1) ? 0.f : a1, d2 = (b1 && !b2) ? 0.f : a2, d3 = b2 ? 0.f : a3;
+    const float d01 = __fadd_rn(d0, d1), d012 = __fadd_rn(d01, d2), ds = __fadd_rn(d012, d3);
+    const float w2 = __fmaf_rn(v1, ds, -ds);
+    // the thresholds of a walk do not decrease, so the last one passed decides
+    uint32_t f = b0 ? 1u : 0u, g = w2 > d0 ? 4u : 0u;
+    f = b1 ? 2u : f;
+    g = w2 > d01 ? 8u : g;
+    f = b2 ? 3u : f;
+    g = w2 > d012 ? 12u : g;
+    x[0] = __fmul_rn(x[0], __fmul_rn(s, rcp_fast(__fmaf_rn(a0, __fadd_rn(r1, r23), a0))));
+    x[1] = __fmul_rn(x[1], __fmul_rn(s, rcp_fast(__fmaf_rn(a1, __fadd_rn(r0, r23), a1))));
+    x[2] = __fmul_rn(x[2], __fmul_rn(s, rcp_fast(__fmaf_rn(a2, __fadd_rn(r01, r3), a2))));
+    x[3] = __fmul_rn(x[3], __fmul_rn(s, rcp_fast(__fmaf_rn(a3, __fadd_rn(r01, r2), a3))));
+    return f + g;
 }
+__device__ __forceinline__ uint32_t picks_to_keep(uint32_t picks) { return (1u << (picks & 3u)) | (1u << (picks >> 2)); }
 
 // ---------------------------------------------------------------------------------------------
 // float8 scales from a tensor's absolute maximum on the device: the dequantisation scale is amax / 448 in double (1 for
