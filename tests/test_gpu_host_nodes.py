@@ -1,0 +1,97 @@
+"""Autograd nodes of the native host path: saved tensors pass through the saved-tensor hooks, a forward-mode tangent is
+refused, and a weight's copies changed in place between the passes are noticed.  And the linear layer's unpadded route."""
+import pytest
+import torch
+import torch.autograd.forward_ad as fwAD
+import torch.nn.functional as F
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _layers():
+    import sparse
+    from sparse import train_ops
+    g = torch.Generator(device=DEV).manual_seed(3)
+    x = torch.randn(128, 256, device=DEV, generator=g).half()
+    fst = sparse.SparseLinearTranspose(256, 128, bias=True).cuda()
+    sste = sparse.SoftThresholdLinear(256, 128, bias=True, device=DEV, spmm=True)
+    sste.init_scale()
+    norm = train_ops.LayerNorm(256).cuda()
+    mask = sparse.mask_select(fst.weight.detach())[1]
+
+    def fp8(t):
+        return sparse.fp8.sparse_linear_transpose_fp8.apply(t, fst.weight, sparse.fp8.Fp8SparseWeight(fst.weight, mask), fst.bias)
+
+    def auto(layer):
+        def call(t):
+            with torch.autocast("cuda", torch.float16):
+                return layer(t)
+        return call
+    return x, {"fst": auto(fst), "sste": sste, "fp8": fp8, "norm": auto(norm), "gelu": train_ops.gelu,
+               "add_norm": auto(lambda t: train_ops.add_layer_norm(t.float(), t, norm)[1]),
+               "cross_entropy": lambda t: train_ops.cross_entropy(t, torch.arange(128, device=DEV))}
+
+
+NAMES = ["fst", "sste", "fp8", "norm", "gelu", "add_norm", "cross_entropy"]
+
+
+@pytest.mark.parametrize("name", NAMES)
+def test_saved_tensors_pass_through_hooks(name):
+    """Packed to the host and back, the gradient has the same bits; every node hands at least one tensor to the hooks."""
+    import random
+    x, calls = _layers()
+    packed, grads = [], []
+    for hooked in (False, True):
+        random.seed(5)
+        t = x.clone().requires_grad_(True)
+        if hooked:
+            def pack(v):
+                packed.append(v.shape)
+                return v.stride(), v.cpu()
+
+            def unpack(p):
+                return torch.empty_strided(p[1].shape, p[0], dtype=p[1].dtype, device=DEV).copy_(p[1])
+            with torch.autograd.graph.saved_tensors_hooks(pack, unpack):
+                y = calls[name](t)
+        else:
+            y = calls[name](t)
+        y.backward(torch.ones_like(y) * 0.5)
+        grads.append(t.grad)
+    assert packed
+    assert torch.equal(grads[0], grads[1])
+
+
+@pytest.mark.parametrize("name", NAMES)
+def test_forward_mode_is_refused(name):
+    x, calls = _layers()
+    with fwAD.dual_level(), pytest.raises(NotImplementedError):
+        calls[name](fwAD.make_dual(x, torch.ones_like(x)))
+
+
+def test_changed_copies_are_noticed():
+    import sparse
+    x, _ = _layers()
+    layer = sparse.SparseLinearTranspose(256, 128, bias=False).cuda()
+    with torch.autocast("cuda", torch.float16):
+        y = layer(x.requires_grad_(True))
+    layer.weight.compressed[2].mul_(2)
+    with pytest.raises(RuntimeError, match="inplace"):
+        y.backward(torch.ones_like(y))
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("tokens", [1, 7, 8, 127, 129, 255, 257, 1025])
+def test_ragged_tokens_equal_padded_ones(dtype, tokens):
+    """A ragged number of token-major rows is not padded; each row's result has the bits it has among padded rows.  The
+    same kernel accumulates every row in the same K order, wherever the last tile is cut."""
+    import sparse
+    g = torch.Generator(device=DEV).manual_seed(tokens)
+    w = sparse.to_sparse_semi_structured(torch.randn(256, 512, device=DEV, generator=g).to(dtype), dtype=dtype)
+    b = torch.randn(256, device=DEV, generator=g).to(dtype)
+    full = torch.randn((tokens + 7) // 8 * 8, 512, device=DEV, generator=g).to(dtype)
+    x = full[:tokens].clone()
+    with torch.inference_mode():
+        assert torch.equal(F.linear(x, w, b), F.linear(full, w, b)[:tokens])
+        assert torch.equal(F.linear(x, w), F.linear(full, w)[:tokens])
+        assert torch.equal(F.linear(full[:tokens].unsqueeze(0), w, b)[0], F.linear(full, w, b)[:tokens])
