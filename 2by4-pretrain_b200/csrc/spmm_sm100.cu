@@ -180,6 +180,7 @@ struct SpmmParams {
     float alpha;            // float32 outputs: D = alpha * (A * B) (+ bias); 16-bit and integer outputs ignore it
     int bias_f32;           // bias holds float32 values instead of values of the output type
     const float *amax_a, *amax_b;   // float8: absolute maxima of the operands on the device; alpha is the product of their scales
+    int bn, stages;         // CTA-pair kernel: tile columns and operand stages
     int accumulate;         // float8, float32 output (ms, n): add alpha * A * B instead of storing it
     void *aux;              // fused MLP epilogues (CTA-pair kernel): second tensor shaped and pitched like out
     int64_t ld_aux;
@@ -737,25 +738,31 @@ spmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
 // ------------------------------------------------------------------------------------------------
 // Two-CTA form (cluster of 2, tcgen05 cta_group::2) for 16-bit types, B stored (n, k), output (n, ms).
 // ------------------------------------------------------------------------------------------------
-// A CTA pair computes tiles of 256 sparse rows x 192 dense columns: every MMA instruction has M = 256 (128
-// rows per CTA) and N = 192, and reads half of its B operand from each CTA's shared memory, so a CTA stages
-// only 96 rows of B per stage: 42 KB per stage and 128-row block, where the single-CTA kernel needs 66 KB
-// (or 84 KB for two blocks).  One accumulator per tile leaves room for two accumulator buffers in tensor
-// memory, so the epilogue of a tile runs entirely under the next tile's MMAs, and five operand stages fit.
+// A CTA pair computes tiles of 256 sparse rows x BN dense columns (BN up to 240, chosen per problem): every MMA instruction has
+// M = 256 (128 rows per CTA) and N = BN, and reads half of its B operand from each CTA's shared memory, so a CTA stages only
+// BN / 2 rows of B per stage: 48 KB for 7.9 dense-equivalent MFLOP at 240 columns, where the single-CTA kernel needs 66 KB for
+// 6.3 (or 84 KB for two blocks).  One accumulator per tile leaves room for two accumulator buffers in tensor memory, so the
+// epilogue of a tile runs entirely under the next tile's MMAs, and four to six operand stages fit.
 // Each CTA loads its own A block, metadata and B half with TMA (cta_group::2 form, completing on the leader's
 // barrier), drains its own accumulator and reports its release to the leader's barrier.  CTA 0 of the pair
 // (the leader) issues all MMAs and metadata copies; its commits arrive on the barriers of both CTAs.  No load
 // is multicast.
 namespace two {
-constexpr int BN2 = 192;                                   // columns of a pair tile
-constexpr int B_HALF_BYTES = (BN2 / 2) * 256;              // 96 rows x two 128-byte K atoms
-constexpr int STAGES2 = 5;
-// 8-bit operands: the same bytes per stage (K step 256 instead of 128), twice the metadata
+// Columns of a pair tile: a multiple of 16 in [BN2_MIN, BN2_MAX], chosen per problem (pick_pair_bn).  Two accumulator buffers
+// of up to 240 columns start at columns 0 and 256 of tensor memory, the metadata slots sit in the 16 columns between them.
+constexpr int BN2_MIN = 32, BN2_MAX = 240, ACC_COL = 256, E_COL = 240;
+constexpr int MAX_STAGES2 = 6;
+// 8-bit operands: the same bytes per stage (K step 256 instead of 128), twice the metadata.  Stage: A block, metadata, then
+// BN / 2 rows of B as two 128-byte K atoms; every part is a multiple of the 1024-byte swizzle period.
 constexpr int e2_bytes(bool f8) { return f8 ? 4096 : 2048; }
-constexpr int stage2_bytes(bool f8) { return A_STAGE_BYTES + B_HALF_BYTES + e2_bytes(f8); }   // 43008 / 45056
-constexpr int smem2(bool f8) { return STAGES2 * stage2_bytes(f8) + 1024; }
-static_assert(stage2_bytes(false) % 1024 == 0 && stage2_bytes(true) % 1024 == 0, "stages must keep the 1024-byte swizzle alignment");
-static_assert(smem2(true) <= 227 * 1024, "shared memory budget");
+constexpr int stage2_bytes(bool f8, int bn) { return A_STAGE_BYTES + e2_bytes(f8) + bn * 128; }
+constexpr int stages2(bool f8, int bn) {
+    const int n = (227 * 1024 - 2048) / stage2_bytes(f8, bn);     // alignment slack and the static shared memory aside
+    return n < MAX_STAGES2 ? n : MAX_STAGES2;
+}
+constexpr int smem2(bool f8, int bn) { return stages2(f8, bn) * stage2_bytes(f8, bn) + 1024; }
+static_assert(stage2_bytes(false, 16) % 1024 == 0 && stage2_bytes(true, 16) % 1024 == 0, "stages must keep the 1024-byte swizzle alignment");
+static_assert(stages2(true, BN2_MAX) >= 4, "shared memory budget");
 }  // namespace two
 
 __device__ __forceinline__ uint32_t cluster_ctarank() {
@@ -825,20 +832,19 @@ __global__ void __launch_bounds__(320, 1)
 spmm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                  const __grid_constant__ CUtensorMap map_e, SpmmParams P) {
     using namespace two;
-    constexpr int BN = BN2;
-    constexpr int STAGES = STAGES2;
-    constexpr int STAGE2_BYTES = stage2_bytes(F8);
-    constexpr int OFF_B = A_STAGE_BYTES, OFF_E = OFF_B + B_HALF_BYTES;
+    const int BN = P.bn, STAGES = P.stages;       // see pick_pair_bn
+    const int STAGE2_BYTES = stage2_bytes(F8, BN);
+    constexpr int OFF_E = A_STAGE_BYTES, OFF_B = OFF_E + e2_bytes(F8);
     constexpr int KE = F8 ? 256 : 128;            // K step of a stage
     constexpr int KSTEPS = 4;
     constexpr uint32_t TMEM_COLS = 512;
-    constexpr int E_COL0 = 2 * BN, E_SLOT = F8 ? 8 : 4;    // two accumulator buffers, then two metadata slots
+    constexpr int E_SLOT = F8 ? 8 : 4;
     static_assert(sizeof(OutT) == 2, "16-bit outputs only");
-    static_assert(E_COL0 + 2 * E_SLOT <= 512, "tensor memory columns exhausted");
+    static_assert(BN2_MAX <= E_COL && E_COL + 2 * E_SLOT <= ACC_COL && ACC_COL + BN2_MAX <= 512, "tensor memory columns exhausted");
 
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    __shared__ __align__(8) uint64_t bars[2 * STAGES + 4];
+    __shared__ __align__(8) uint64_t bars[2 * MAX_STAGES2 + 4];
     __shared__ uint32_t tmem_base_smem;
     __shared__ int abort_flag;
 
@@ -850,8 +856,8 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     const int n_tiles = n_tiles_n * n_tiles_m;        // row block varies fastest over the tile index
     const int k_iters = (int)((P.k + KE - 1) / KE);
 
-    const uint32_t full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[STAGES]);
-    const uint32_t tmem_full0 = smem_u32(&bars[2 * STAGES]), tmem_empty0 = smem_u32(&bars[2 * STAGES + 2]);
+    const uint32_t full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[MAX_STAGES2]);
+    const uint32_t tmem_full0 = smem_u32(&bars[2 * MAX_STAGES2]), tmem_empty0 = smem_u32(&bars[2 * MAX_STAGES2 + 2]);
 
     if (threadIdx.x == 0) {
         abort_flag = 0;
@@ -878,18 +884,17 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     if (warp == 0) {
         // ---------------------------------------------------------------- TMA producer (one per CTA)
         if (lane == 0) {
-            int g = 0;
+            int g = 0, s = 0;
+            uint32_t ph = 1;                     // of the empty barriers: the first round passes at once
             bool ok = true;
-            constexpr uint32_t cta_tx = A_STAGE_BYTES + e2_bytes(F8) + B_HALF_BYTES;
+            const uint32_t cta_tx = (uint32_t)STAGE2_BYTES;
             for (int tile = pair; tile < n_tiles && ok; tile += n_pairs) {
                 const int mblk = (tile % n_tiles_m) * 2 + (int)rank;
                 const int mrow = mblk * BM;
                 const int brow = (tile / n_tiles_m) * BN + (int)rank * (BN / 2);
                 for (int it = 0; it < k_iters; ++it, ++g) {
-                    const int s = g % STAGES;
-                    const uint32_t ph = (g / STAGES) & 1;
-                    if (g >= STAGES && !mbar_wait(empty0 + 8 * s, ph ^ 1, &abort_flag, P.status, 1)) { ok = false; break; }
-                    const uint32_t sa = smem_u32(smem + (size_t)s * STAGE2_BYTES);
+                    if (!mbar_wait(empty0 + 8 * s, ph, &abort_flag, P.status, 1)) { ok = false; break; }
+                    const uint32_t sa = smem_u32(smem) + (uint32_t)s * (uint32_t)STAGE2_BYTES;
                     const uint32_t sb = sa + OFF_B;
                     const uint32_t full_leader = map_to_cta(full0 + 8 * s, 0);
                     if (rank == 0) mbar_expect_tx(full0 + 8 * s, 2 * cta_tx);
@@ -901,18 +906,19 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                     }
                     // metadata of this row block and K step: two rows of 1024 bytes per atom of the table (8-bit: two atoms)
                     tma_load_2d_pair(sa + OFF_E, &map_e, 0, (int)(((int64_t)mblk * P.k_atoms + it * (F8 ? 2 : 1)) * 2), full_leader);
-                    // this CTA's half of B: 96 rows x two 128-byte K atoms
+                    // this CTA's half of B: BN / 2 rows x two 128-byte K atoms
                     tma_load_2d_pair(sb, &map_b, it * KE, brow, full_leader);
                     tma_load_2d_pair(sb + (BN / 2) * 128, &map_b, it * KE + KE / 2, brow, full_leader);
                     SP24_TRACE(0, g);
+                    if (++s == STAGES) { s = 0; ph ^= 1; }
                 }
             }
             if (abort_flag && rank == 0) {
                 for (int q = (g > STAGES ? g - STAGES : 0); q < g; ++q) {
-                    const int s = q % STAGES;
-                    const uint32_t ph = (q / STAGES) & 1;
+                    const int sq = q % STAGES;
+                    const uint32_t pq = (q / STAGES) & 1;
                     for (uint32_t w = 0; w < WAIT_LIMIT; ++w)
-                        if (mbar_try_wait(full0 + 8 * s, ph)) break;
+                        if (mbar_try_wait(full0 + 8 * sq, pq)) break;
                 }
             }
         }
@@ -923,32 +929,33 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         // address field.
         if (rank == 0) {
             constexpr uint32_t A_LBO = A_MN ? 8192 : 16, A_KSTEP = A_MN ? 2048 : 32;
-            const uint32_t idesc0 = P.idesc;   // M = 256, N = 192 set by the launcher
+            const uint32_t idesc0 = P.idesc;   // M = 256, N = BN set by the launcher
             const uint32_t smem0 = smem_u32(smem);
             const uint64_t adesc0 = make_desc(smem0, A_LBO, 1024, 2), bdesc0 = make_desc(smem0 + OFF_B, 16, 1024, 2);
             const uint64_t edesc0 = make_desc(smem0 + OFF_E, 16, 128, 0);
+            const uint32_t b_atom = (uint32_t)BN * (64 >> 4);       // second K atom of a B half, in descriptor units
             int s = 0, tl = 0;
             uint32_t ph = 0, eslot = 0;
             bool ok = true;
             for (int tile = pair; tile < n_tiles && ok; tile += n_pairs, ++tl) {
                 const int buf = tl & 1;
-                const uint32_t acc = tmem_base + buf * BN;
+                const uint32_t acc = tmem_base + buf * ACC_COL;
                 // the epilogues of both CTAs must have drained this accumulator buffer (two tiles ago)
                 ok = mbar_wait(tmem_empty0 + 8 * buf, ((tl >> 1) & 1) ^ 1, &abort_flag, P.status, 4);
                 for (int it = 0; it < k_iters && ok; ++it) {
                     ok = mbar_wait(full0 + 8 * s, ph, &abort_flag, P.status, 2);
                     if (!ok) break;
                     tc_fence_after();
-                    const uint32_t off = (uint32_t)s * (STAGE2_BYTES >> 4);
+                    const uint32_t off = (uint32_t)s * ((uint32_t)STAGE2_BYTES >> 4);
                     const uint64_t ad = adesc0 + off, bd = bdesc0 + off, ed = edesc0 + off;
-                    const uint32_t e_cols = tmem_base + E_COL0 + eslot;
+                    const uint32_t e_cols = tmem_base + E_COL + eslot;
                     if (elect_one()) {
                         tc_cp_128x128b_pair(e_cols, ed);
                         if constexpr (F8) tc_cp_128x128b_pair(e_cols + 4, ed + (2048 >> 4));
                         // metadata of an MMA: two columns (8-bit), or the even column of a pair plus a 1-bit selector
 #pragma unroll
                         for (int j = 0; j < KSTEPS; ++j)
-                            mma_sp_pair_any<F8>(acc, ad + j * (A_KSTEP >> 4), bd + (((j >> 1) * ((BN / 2) * 128) + (j & 1) * 64) >> 4),
+                            mma_sp_pair_any<F8>(acc, ad + j * (A_KSTEP >> 4), bd + ((j >> 1) * b_atom + (j & 1) * (64 >> 4)),
                                                 e_cols + (F8 ? 2 * j : (j & ~1)), F8 ? idesc0 : idesc0 | (j & 1), (it > 0 || j > 0) ? 1u : 0u);
                         tc_commit_pair(empty0 + 8 * s);
                     }
@@ -962,11 +969,12 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         }
     } else {
         // ---------------------------------------------------------------- epilogue (warps 2..9 of both CTAs)
-        // No staging buffer: a warp packs its 96 columns of the accumulator into 48 registers, hands the buffer
+        // No staging buffer: a warp packs its BN / 2 columns of the accumulator into registers, hands the buffer
         // back, then stores 16-bit values directly; the 32 lanes of a store are 32 consecutive features of one
         // token, 64 contiguous bytes.
         const int quad = warp & 3, half = (warp - 2) >> 2;
-        constexpr int HC = BN / 2, NREG = HC / 2;
+        const int HC = BN / 2;                      // a multiple of 8 up to 120 (fused epilogues: of 16 up to 96)
+        constexpr int NREG = EPI == EPI_PLAIN ? 64 : 48;
         OutT *out = static_cast<OutT *>(P.out);
         const float alpha = F8 ? alpha_of(P) : 1.f;
         const uint32_t empty_leader0 = map_to_cta(tmem_empty0, 0);
@@ -983,10 +991,11 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             if (run) {
                 float bias = 0.f;
                 if (P.bias) bias = load_bias<OutT>(P, mrow);
-                const uint32_t acc = tmem_base + ((uint32_t)(quad * 32) << 16) + buf * BN + half * HC;
+                const uint32_t acc = tmem_base + ((uint32_t)(quad * 32) << 16) + buf * ACC_COL + half * HC;
 #pragma unroll
-                for (int c = 0; c < HC / 32; ++c) {
-                    uint32_t v[32];
+                for (int c = 0; c < NREG / 16; ++c) {
+                    if (c * 32 >= HC) break;
+                    uint32_t v[32];             // columns past HC belong to other tiles or to the metadata: read, never stored
                     tmem_ld32(acc + c * 32, v);
                     tmem_ld_wait();
 #pragma unroll
@@ -1014,14 +1023,16 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                     if (tok0 + HC <= P.n) {
 #pragma unroll
                         for (int c2 = 0; c2 < NREG; ++c2) {
+                            if (c2 % 4 == 0 && 2 * c2 >= HC) break;
                             dst[0] = (uint16_t)(held[c2] & 0xFFFFu);
                             dst[P.ld_out] = (uint16_t)(held[c2] >> 16);
                             dst += 2 * P.ld_out;
-                            asm volatile("" : "+l"(dst));   // one running pointer, not 96 precomputed addresses
+                            asm volatile("" : "+l"(dst));   // one running pointer, not a precomputed address per column
                         }
                     } else {
 #pragma unroll
                         for (int c2 = 0; c2 < NREG; ++c2) {
+                            if (c2 % 4 == 0 && 2 * c2 >= HC) break;
                             if (tok0 + 2 * c2 < P.n) dst[0] = (uint16_t)(held[c2] & 0xFFFFu);
                             if (tok0 + 2 * c2 + 1 < P.n) dst[P.ld_out] = (uint16_t)(held[c2] >> 16);
                             dst += 2 * P.ld_out;
@@ -1036,6 +1047,7 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                     constexpr int CHUNK = 8;
 #pragma unroll
                     for (int c0 = 0; c0 < NREG; c0 += CHUNK) {
+                        if (2 * c0 >= HC) break;
                         uint16_t a[2 * CHUNK];
                         if constexpr (EPI == EPI_DGELU) {
 #pragma unroll
@@ -1407,24 +1419,25 @@ int make_map_e(CUtensorMap *map, const void *e_tc, int64_t n_atoms, int atoms_pe
 template <bool A_MN, typename OutT, int EPI = EPI_PLAIN, bool F8 = false>
 int launch_spmm_pair(const CUtensorMap &ma, const CUtensorMap &mb, const CUtensorMap &me, SpmmParams P, cudaStream_t st) {
     auto kern = spmm_pair_kernel<A_MN, OutT, EPI, F8>;
-    constexpr int SMEM = two::smem2(F8);
+    constexpr int SMEM_MAX = 227 * 1024 - 1024;
     static bool attr_set[64];
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess)
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX) != cudaSuccess)
             return SP24_ERR_CUDA;
         attr_set[dev] = true;
     }
-    // M = 256 over the CTA pair, N = 192
-    P.idesc = (P.idesc & ~(0x1Fu << 24)) | ((uint32_t)(256 >> 4) << 24) | ((uint32_t)(two::BN2 >> 3) << 17);
-    const int64_t tiles = ((P.n + two::BN2 - 1) / two::BN2) * (P.ms / 256);
+    // M = 256 over the CTA pair, N = bn
+    P.idesc = (P.idesc & ~(0x1Fu << 24)) | ((uint32_t)(256 >> 4) << 24) | ((uint32_t)(P.bn >> 3) << 17);
+    P.stages = two::stages2(F8, P.bn);
+    const int64_t tiles = ((P.n + P.bn - 1) / P.bn) * (P.ms / 256);
     const int64_t pairs_max = sm_count_cached() / 2;
     const unsigned pairs = (unsigned)(tiles < pairs_max ? tiles : pairs_max);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(2 * pairs, 1, 1);
     cfg.blockDim = dim3(320, 1, 1);
-    cfg.dynamicSmemBytes = SMEM;
+    cfg.dynamicSmemBytes = two::smem2(F8, P.bn);
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1490,6 +1503,29 @@ void pick_tile(int64_t ms, int64_t n, int sm_count, int &bn_out, int &mpt_out) {
             if (cost < best_cost) { best_cost = cost; bn_out = bn; mpt_out = mpt; }
         }
     }
+}
+
+// Columns of a CTA-pair tile: the candidate with the lowest (rounds of tiles per CTA pair) x (bytes staged per CTA and K step).
+// The K loop is bound by the operand fill from L2 (about 14 TB/s over the chip whatever the width), so a wide tile pays only
+// where it does not leave the last round nearly empty.  fp16, us, at 192 columns -> at the width taken:
+//   ms 4096, n 2043, k 4096: 42.8 -> 33.5 (240 columns: two rounds instead of three)
+//   ms 3072, n 16384, k 768: 55.5 -> 52.0 (224); ms 768, n 16384, k 3072: 46.7 -> 43.4 (224)
+//   ms 3072, n 16384, k 3072: 148 -> 139 (240); ms 768, n 5000, k 1024: 16.5 -> 12.5 (224)
+// Few columns: the narrowest tile that still takes one round; against the single-CTA kernel, which took these before,
+//   ms 4096, k 4096: n 16 21.6 -> 16.5, n 256 23.9 -> 18.4, n 512 28.0 -> 18.9, n 768 30.8 -> 20.1; ms 768, k 3072, n 512 18.9 -> 14.4
+// (the single-CTA kernel was never faster, so it keeps the row counts that are odd multiples of 128 and the other layouts).
+// The fused epilogues hold up to 192 columns in registers and take them in chunks of 16 per half tile.
+int pick_pair_bn(int64_t ms, int64_t n, bool plain) {
+    const int step = plain ? 16 : 32, widest = plain ? two::BN2_MAX : 192;
+    const int64_t pairs = sm_count_cached() / 2;
+    int best = widest;
+    int64_t best_cost = INT64_MAX;
+    for (int bn = widest; bn >= two::BN2_MIN; bn -= step) {
+        const int64_t tiles = ((n + bn - 1) / bn) * (ms / 256);
+        const int64_t cost = ((tiles + pairs - 1) / pairs) * two::stage2_bytes(false, bn);
+        if (cost < best_cost) { best_cost = cost; best = bn; }
+    }
+    return best;
 }
 
 template <bool F8, bool A_MN, bool B_MN, bool TRANS, typename OutT>
@@ -1599,11 +1635,12 @@ static int spmm_impl(const void *a_packed, int dtype, int a_mn_major, int64_t ld
     P.idesc = (1u << 2) | ((i8 ? 2u : 1u) << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(a_mn_major ? 1 : 0) << 15) |
               ((uint32_t)(b_mn_major ? 1 : 0) << 16) | ((uint32_t)(BM >> 4) << 24);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    bool pair_form = pair_ok && n >= 1024 && pair_kernels_enabled();
+    bool pair_form = pair_ok && pair_kernels_enabled();
     if (epi != EPI_PLAIN || bias_f32) pair_form = true;      // checked above: these forms exist in the pair kernel only
     if (pair_form) {
         CUtensorMap map_b, map_e;
-        rc = make_map(&map_b, b, dtype, n, k, ld_b, 64, two::BN2 / 2);
+        P.bn = pick_pair_bn(ms, n, epi == EPI_PLAIN);
+        rc = make_map(&map_b, b, dtype, n, k, ld_b, 64, (uint32_t)P.bn / 2);
         if (rc) return rc;
         rc = make_map_e(&map_e, e_tc, (ms / 128) * P.k_atoms);
         if (rc) return rc;
@@ -1669,7 +1706,7 @@ extern "C" int sp24_spmm_mlp(const void *a_packed, int dtype, int a_mn_major, in
 // The GEMMs of a float8 layer whose scales stay on the device: D = alpha * (A_sparse * B) [+ float32 bias], alpha = the
 // product of the operands' scales, worked out from their absolute maxima (sp24_absmax).
 //   trans_out = 1: out (n, ms) in float32, float16 or bfloat16 (rounded once): the layer's output or input gradient
-//   without a float32 copy.  16-bit outputs of whole 256-row blocks and >= 1024 columns run on CTA pairs.
+//   without a float32 copy.  16-bit outputs of whole 256-row blocks run on CTA pairs.
 //   trans_out = 0: out (ms, n) float32 += alpha * A * B (no bias), K cut into slices over idle SMs: the weight gradient.
 extern "C" int sp24_spmm_f8(const void *a_packed, int dtype, int64_t ld_a, const void *e_tc, int64_t ms, int64_t k, const void *b, int64_t ld_b,
                             int64_t n, void *out, int out_dtype, int trans_out, int64_t ld_out, const float *bias, const float *amax_a,
@@ -1688,9 +1725,10 @@ extern "C" int sp24_spmm_f8(const void *a_packed, int dtype, int64_t ld_a, const
     const uint32_t fmt = dtype == SP24_E5M2 ? 1u : 0u;
     P.idesc = (1u << 2) | (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(BM >> 4) << 24);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (trans_out && out_dtype != SP24_F32 && ms % 256 == 0 && n >= 1024 && pair_kernels_enabled()) {
+    if (trans_out && out_dtype != SP24_F32 && ms % 256 == 0 && pair_kernels_enabled()) {
         CUtensorMap map_e;
-        if (int rc = make_map(&map_b, b, dtype, n, k, ld_b, 128, two::BN2 / 2)) return rc;
+        P.bn = pick_pair_bn(ms, n, true);
+        if (int rc = make_map(&map_b, b, dtype, n, k, ld_b, 128, (uint32_t)P.bn / 2)) return rc;
         if (int rc = make_map_e(&map_e, e_tc, (ms / 128) * P.k_atoms, 2)) return rc;
         return out_dtype == SP24_F16 ? launch_spmm_pair<false, __half, EPI_PLAIN, true>(map_a, map_b, map_e, P, st)
                                      : launch_spmm_pair<false, __nv_bfloat16, EPI_PLAIN, true>(map_a, map_b, map_e, P, st);

@@ -344,7 +344,7 @@ int sp24_meta_to_tc(const void *meta, int meta_itemsize, int64_t m, int64_t k, v
  *   dtype      F16 / BF16 (out_dtype = dtype), E4M3 / E5M2 (out_dtype = F32) or I8 (out_dtype = I32, no bias, no
  *              activation); the 8-bit types take K-major operands only.  The same table as the reference's
  *              (sparse/csrc/mySparseSemiStructuredLinear_cuda.cu:594-637, 729, 772).
- *              16-bit GEMMs with b_mn_major = 0, trans_out = 1, ms % 256 == 0, n >= 1024 and no activation run on
+ *              16-bit GEMMs with b_mn_major = 0, trans_out = 1, ms % 256 == 0 and no activation run on
  *              pairs of CTAs (tcgen05 cta_group::2); the result is bit-equal to the single-CTA kernel's.
  *   bias       ms values in the output type or NULL; activation 0 none, 1 relu, 2 silu, 3 gelu (tanh form; not in the reference)
  *   status     optional device int: set to a non-zero code if a bounded on-device wait gave up

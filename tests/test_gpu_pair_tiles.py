@@ -1,0 +1,74 @@
+"""Widths of the CTA-pair GEMM's tiles: every width the rule can take, at ragged ends, bit for bit against the single-CTA kernel
+(reached through the activation, which the pair kernel does not have)."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _operand(ms, k, dtype, seed, col):
+    import sparse
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    w = torch.randn(ms, k, device=DEV, generator=g).to(dtype)
+    sp = sparse.to_sparse_semi_structured(w.t().contiguous().t() if col else w, dtype=dtype)
+    return sp.sparse_tensor_cutlass, sp.meta_tensor_cutlass, g
+
+
+# (ms, n): one round at widths 32 .. 240 (n alone decides where ms is small), several rounds, and the ragged ends of tiles
+SIZES = [(256, n) for n in (1, 15, 16, 17, 31, 33, 2368, 2369, 3553, 17760, 17761)] + \
+        [(2048, n) for n in (9, 257, 288, 289, 433, 721, 1297)] + [(3072, 1100), (768, 5000), (4096, 1023)]
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("col", [False, True])
+@pytest.mark.parametrize("ms,n", SIZES)
+def test_every_tile_width_has_the_single_cta_bits(dtype, col, ms, n):
+    """Both kernels accumulate each output in the same K order: no tolerance."""
+    from sparse.spmm import check_status, sparse_linear
+    k = 832 if n < 2000 else 192
+    p, e, g = _operand(ms, k, dtype, ms + n, col)
+    x = torch.randn(n, k, device=DEV, generator=g).to(dtype)
+    b = torch.randn(ms, device=DEV, generator=g).to(dtype)
+    for sign in (1, -1):          # both signs of every output pass the relu once
+        assert torch.equal(sparse_linear(x * sign, p, e, b * sign).clamp(min=0), sparse_linear(x * sign, p, e, b * sign, "relu"))
+    check_status()
+
+
+@pytest.mark.parametrize("ms,n", [(256, 1), (512, 33), (2048, 289), (1024, 1023), (768, 5000), (3072, 2369)])
+def test_fused_epilogues_at_every_width(ms, n):
+    """The kept pre-activation has the plain product's bits; the activation's derivative stays within two bf16 roundings."""
+    import torch.nn.functional as F
+    from sparse.spmm import sparse_linear, sparse_linear_mlp
+    p, e, g = _operand(ms, 192, torch.bfloat16, n, False)
+    x = torch.randn(n, 192, device=DEV, generator=g).bfloat16()
+    b = torch.randn(ms, device=DEV, generator=g).bfloat16()
+    plain = sparse_linear(x, p, e, b)
+    act, pre = sparse_linear_mlp(x, p, e, bias=b, epilogue="gelu")
+    assert torch.equal(pre, plain)
+    ref = F.gelu(pre.float(), approximate="tanh")
+    assert float((act.float() - ref).abs().max() / ref.abs().max()) <= 2 ** -8
+    d = sparse_linear_mlp(x, p, e, epilogue="dgelu", aux=pre)
+    q = pre.float().requires_grad_(True)
+    F.gelu(q, approximate="tanh").backward(sparse_linear(x, p, e).float())
+    assert float((d.float() - q.grad).abs().max() / q.grad.abs().max()) <= 2 ** -7
+
+
+@pytest.mark.parametrize("ms,n", [(256, 128), (512, 256), (768, 1152), (256, 17792)])
+def test_float8_pair_products(ms, n):
+    """e4m3 products with the scales taken on the device, 16-bit result against float64 of the same operands: one rounding to
+    bf16 (2^-9 of the value) over float32 sums."""
+    import sparse
+    k = 256
+    g = torch.Generator(device=DEV).manual_seed(n)
+    w = torch.randn(ms, k, device=DEV, generator=g)
+    mask = sparse.mask_select(w)[1]
+    w8 = sparse.fp8.Fp8SparseWeight(w, mask)
+    x = torch.randn(n, k, device=DEV, generator=g).bfloat16()
+    y = sparse.fp8.sparse_linear_transpose_fp8.apply(x, w, w8, None)
+    sw, sx = float((w * mask).abs().max()) / 448, float(x.abs().max()) / 448
+    wq = ((w * mask) * (1 / sw)).to(torch.float8_e4m3fn).double() * sw
+    xq = (x.float() * (1 / torch.tensor(sx, device=DEV)))     # the reciprocal in float32, as the kernel takes it (ties!)
+    xq = xq.to(torch.float8_e4m3fn).double() * sx
+    ref = xq @ wq.t()
+    assert float((y.double() - ref).norm() / ref.norm()) <= 2 ** -8
