@@ -394,9 +394,13 @@ __device__ __forceinline__ void ts_dual_block(const DualParams &P, const unsigne
     }
 }
 
+// Resident CTAs per SM.  With the search: three for 16-bit inputs (80 registers), two for fp32 ones.  Without it the pass is
+// bound by memory latency between its barriers and needs fewer registers: one CTA more
+// (the 48 fp32 weights of a 12-block, 768-wide model, given masks, bf16 out: 166 -> 127 us, 3.7 -> 4.9 TB/s).
+constexpr int dual_min_blocks(bool select, int in_bytes) { return (in_bytes == 2 ? 3 : 2) + (select ? 0 : 1); }
+
 template <typename T, typename TOut, bool SELECT, bool TC>
-// three CTAs per SM for 16-bit inputs (80 registers); fp32 inputs need more registers and keep two
-__global__ void __launch_bounds__(256, sizeof(T) == 2 ? 3 : 2) ts_dual_kernel(DualParams P) {
+__global__ void __launch_bounds__(256, dual_min_blocks(SELECT, sizeof(T))) ts_dual_kernel(DualParams P) {
     ts_dual_block<T, TOut, SELECT, TC>(P, blockIdx.x, blockIdx.y);
 }
 
@@ -410,7 +414,7 @@ struct DualBatch {
     int count;
 };
 template <typename T, typename TOut, bool SELECT, bool TC>
-__global__ void __launch_bounds__(256, sizeof(T) == 2 ? 3 : 2) ts_dual_batch_kernel(const __grid_constant__ DualBatch B) {
+__global__ void __launch_bounds__(256, dual_min_blocks(SELECT, sizeof(T))) ts_dual_batch_kernel(const __grid_constant__ DualBatch B) {
     int i = 0;
     while (i + 1 < B.count && blockIdx.x >= B.first[i + 1]) ++i;
     const DualParams &P = B.p[i];
