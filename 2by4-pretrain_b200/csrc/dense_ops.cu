@@ -465,14 +465,14 @@ __global__ void __launch_bounds__(256) absmax_kernel(const uint4 *x, const uint3
     }
 }
 
-// q = x * f8_quant_scale(amax) as e4m3, row-major; q_t (optional): its transpose.  A block takes 128 rows x 64 columns
+// q = x * f8_store_scale(amax) as e4m3, row-major; q_t (optional): its transpose.  A block takes 128 rows x 64 columns
 // through shared memory; a thread then owns one column's 32 rows: one whole 32-byte sector of the transposed row.
 template <typename T>
 __global__ void __launch_bounds__(256) quantize_f8_kernel(const T *x, int64_t rows, int64_t cols, int64_t ld, const float *amax, uint8_t *q,
                                                           uint8_t *q_t, int64_t ld_t) {
     __shared__ float sc;
     __shared__ __align__(16) uint8_t tile[128][64 + 8];
-    if (threadIdx.x == 0) sc = f8_quant_scale(*amax);
+    if (threadIdx.x == 0) sc = f8_store_scale(*amax);
     __syncthreads();
     const float scale = sc;
     const int64_t r0 = (int64_t)blockIdx.y * 128, c0 = (int64_t)blockIdx.x * 64;

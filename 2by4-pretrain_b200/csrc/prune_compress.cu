@@ -27,7 +27,7 @@ struct PcParams {
     float soft_scale;                       // soft-threshold mode: kept values are also multiplied by this ...
     int soft_use_scale;                     // ... when this is set (one more rounding in the input type)
     const float *amax;                      // optional: 8-bit outputs take their scale from this device word (f8_store_scale)
-    void *q_dense;                          // optional (column-major input, 8-bit output): dense * f8_quant_scale in the output
+    void *q_dense;                          // optional (column-major input, 8-bit output): dense * f8_store_scale in the output
     int64_t ld_q;                           // type, same storage order, pitch ld_q
 };
 
@@ -217,18 +217,13 @@ template <typename T> __device__ __forceinline__ uint32_t mse_lookup(uint32_t lo
 // ---------------------------------------------------------------------------------------------
 // Store scale of an 8-bit output: the caller's, or the reciprocal of the tensor's quantisation scale, worked out by one
 // thread from the absolute maximum that an earlier launch left on the device.  Call with all threads of the block.
-template <typename TOut> __device__ __forceinline__ float out_scale_of(const PcParams &P, float *q_scale = nullptr) {
+template <typename TOut> __device__ __forceinline__ float out_scale_of(const PcParams &P) {
     if constexpr (sizeof(TOut) == 1 && !std::is_same<TOut, int8_t>::value) {
         if (P.amax) {
-            __shared__ float sc[2];
-            if (threadIdx.x == 0) {
-                const float a = *P.amax;
-                sc[0] = f8_store_scale(a);
-                sc[1] = f8_quant_scale(a);
-            }
+            __shared__ float sc;
+            if (threadIdx.x == 0) sc = f8_store_scale(*P.amax);
             __syncthreads();
-            if (q_scale) *q_scale = sc[1];
-            return sc[0];
+            return sc;
         }
     }
     return P.out_scale;
@@ -400,8 +395,7 @@ constexpr int col_min_blocks(int mode, int out_bytes) {
 template <typename TIn, typename TOut, int MODE, bool HAS_U, int V>
 __global__ void __launch_bounds__(256, col_min_blocks(MODE, sizeof(TOut))) pc_col_kernel(PcParams P) {
     const uint64_t rng_offset = P.offset + (P.offset_dev ? *P.offset_dev : 0ull);
-    float q_scale = 1.f;
-    const float out_scale = out_scale_of<TOut>(P, &q_scale);
+    const float out_scale = out_scale_of<TOut>(P);
     constexpr int CH = sizeof(TOut) == 2 ? 16 : 32;
     constexpr int MB = sizeof(TOut) == 2 ? 2 : 4;
     constexpr int GROUP = MB == 2 ? 32 : 16;
@@ -464,7 +458,7 @@ __global__ void __launch_bounds__(256, col_min_blocks(MODE, sizeof(TOut))) pc_co
                     for (int j = 0; j < 8; ++j) {
                         float f[V];
 #pragma unroll
-                        for (int v = 0; v < V; ++v) f[v] = __fmul_rn(Elem<TIn>::to_f32(in[j].v[v]), q_scale);
+                        for (int v = 0; v < V; ++v) f[v] = __fmul_rn(Elem<TIn>::to_f32(in[j].v[v]), out_scale);
                         store_f8<TOut, V>(qdst + j * P.ld_q, f);
                     }
                     qdst += 8 * P.ld_q;

@@ -324,9 +324,8 @@ __device__ __forceinline__ uint32_t picks_to_keep(uint32_t picks) { return (1u <
 // an all-zero or NaN tensor), as a host that reads amax back works it out
 // ---------------------------------------------------------------------------------------------
 __device__ __forceinline__ double f8_scale(float amax) { return amax > 0.f ? (double)amax / 448.0 : 1.0; }
-// factor of a plain quantisation pass, value * (1 / scale) in float32 ...
-__device__ __forceinline__ float f8_quant_scale(float amax) { return __fdiv_rn(1.f, (float)f8_scale(amax)); }
-// ... and the one the compressing kernels take (rounded once from double)
+// The factor every quantising kernel multiplies by: the reciprocal in double, rounded once.  Two roundings (the scale, then
+// its reciprocal) move products that are exact ties of e4m3 to the other side: 0.6 % of 16-bit values at some maxima.
 __device__ __forceinline__ float f8_store_scale(float amax) { return (float)(1.0 / f8_scale(amax)); }
 
 // ---------------------------------------------------------------------------------------------

@@ -147,7 +147,7 @@ int sp24_prune_compress_q8(const void *dense, int dense_dtype, int64_t m, int64_
  * the maximum back.  The scale of a tensor is amax / 448 worked out in double (1 for an all-zero tensor).
  *   sp24_absmax                *amax = max |x| over `count` contiguous values (count a multiple of 16 bytes of x); mask
  *                              (bytes, float32 x only): positions with mask 0 count as zero
- *   sp24_quantize_f8           q (rows, cols) e4m3 = x * (1 / scale) in float32, rounded; q_t (optional) its transpose
+ *   sp24_quantize_f8           q (rows, cols) e4m3 = x * (1 / scale rounded to float32), rounded; q_t (optional) its transpose
  *                              (cols, rows) with pitch ld_t, the K-major operand of the weight-gradient GEMM
  *   sp24_prune_compress_q8_dev sp24_prune_compress_q8 with out_scale = 1 / scale from *amax; three optional extras from the
  *                              same pass: the metadata in the order the GEMM reads (e_tc, m % 128 == 0), row_sums[r] +=

@@ -52,6 +52,31 @@ def test_quantize_matches_torch_and_transposes(dtype, rows, cols):
 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("top", [5.1875, 5.28125, 4.75, 7.125])
+def test_quantize_of_exact_ties(dtype, top):
+    """Maxima at which 16-bit values land exactly between two e4m3 values (x / scale = 84, 42, ...): the plain pass, the pass
+    beside the compression and ``fp8.quantize`` take the same side."""
+    from sparse import fp8, spmm
+    lib, _ext = _lib()
+    m, k = 256, 256
+    x = _rand((k, m), dtype, 12, 1.5).clamp(-top, top)
+    x[0, 0] = top
+    x[1] = top * 3 / 16
+    want, s = fp8.quantize(x)
+    a = _amax(x)
+    q, gq = torch.empty(k, m, dtype=E4M3, device=DEV), torch.empty(k, m, dtype=E4M3, device=DEV)
+    _ext.check(lib.sp24_quantize_f8(x.data_ptr(), _ext.dt(dtype), k, m, m, a.data_ptr(), q.data_ptr(), None, 0, _ext.stream()), "quantize")
+    packed, meta = fp8.compress_q8(x.t(), mode=_ext.PRUNE_MSE, scale=s)
+    p2, m2 = torch.empty_like(packed), torch.empty_like(meta)
+    _ext.check(lib.sp24_prune_compress_q8_dev(x.data_ptr(), _ext.dt(dtype), m, k, m, 1, p2.data_ptr(), _ext.E4M3, k // 2, m2.data_ptr(),
+                                              _ext.PRUNE_MSE, None, 0, a.data_ptr(), 0, 0, None, None, gq.data_ptr(), m, _ext.stream()),
+               "compress")
+    assert torch.equal(q.view(torch.uint8), want.view(torch.uint8))
+    assert torch.equal(gq.view(torch.uint8), want.view(torch.uint8))
+    assert torch.equal(p2.view(torch.uint8), packed.view(torch.uint8)) and torch.equal(m2, meta)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("m,k", [(128, 128), (384, 256), (256, 1152)])
 def test_compress_with_device_scale_equals_host_scale(dtype, m, k):
     """dY^T: the same packed values and metadata as with the scale read back; the extras against torch."""
