@@ -21,7 +21,8 @@ struct PcParams {
     const unsigned long long *offset_dev;   // optional device word added to offset at run time
     int16_t *tc;                            // optional metadata copy in tensor-core atom order (16-bit outputs)
     int64_t k_atoms;                        // 128-column atoms per 128-row block
-    float *row_sums;                        // optional (column-major only): row_sums[r] += sum over k of dense[r, k]
+    float *row_sums;                        // optional (column-major only): row_sums[r] += sum over k of dense[r, k] ...
+    int64_t ld_sums;                        // ... or, non-zero: block row y stores its share to row_sums[y * ld_sums + r]
     int packed_rm;                          // column-major input, 8-bit output: packed is written row-major (m, k/2)
     float out_scale;                        // 8-bit outputs: stored value = value * out_scale (1 = none)
     float soft_scale;                       // soft-threshold mode: kept values are also multiplied by this ...
@@ -563,7 +564,8 @@ __global__ void __launch_bounds__(256, col_min_blocks(MODE, sizeof(TOut))) pc_co
                 float a = 0.f;
 #pragma unroll
                 for (int w = 0; w < 8; ++w) a += ssum[w][t];
-                atomicAdd(P.row_sums + r0 + t, a);
+                if (P.ld_sums) P.row_sums[blockIdx.y * P.ld_sums + r0 + t] = a;
+                else atomicAdd(P.row_sums + r0 + t, a);
             }
         }
     }
@@ -658,7 +660,7 @@ static int prune_compress_impl(const void *dense, int dense_dtype, int64_t m, in
                                int64_t ld_uniforms, uint64_t seed, uint64_t offset, const uint64_t *offset_dev,
                                void *e_tc, float *row_sums, void *stream, int packed_rm = 0, float out_scale = 1.f,
                                int soft_use_scale = 0, float soft_scale = 1.f, const float *amax = nullptr, void *q_dense = nullptr,
-                               int64_t ld_q = 0) {
+                               int64_t ld_q = 0, bool sums_in_parts = false) {
     using namespace sp24;
     if (!dense || !packed || !meta) return SP24_ERR_ARG;
     const int so = dtype_size(packed_dtype), si = dtype_size(dense_dtype);
@@ -687,7 +689,7 @@ static int prune_compress_impl(const void *dense, int dense_dtype, int64_t m, in
     if (int rc = check_device()) return rc;
     PcParams P{dense, packed, meta, static_cast<const uint8_t *>(mask), uniforms, m, k, ld_dense, ld_packed, ld_mask,
                ld_uniforms, seed, offset, reinterpret_cast<const unsigned long long *>(offset_dev),
-               static_cast<int16_t *>(e_tc), (k + 127) / 128, row_sums, packed_rm, out_scale, soft_scale, soft_use_scale, amax, q_dense, ld_q};
+               static_cast<int16_t *>(e_tc), (k + 127) / 128, row_sums, sums_in_parts ? m : 0, packed_rm, out_scale, soft_scale, soft_use_scale, amax, q_dense, ld_q};
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     switch (dense_dtype) {
         case SP24_F32: return dispatch_out<float>(P, packed_dtype, mode, col_major, st);
@@ -756,6 +758,25 @@ extern "C" int sp24_prune_compress_q8_dev(const void *dense, int dense_dtype, in
     return prune_compress_impl(dense, dense_dtype, m, k, ld_dense, col_major, packed, packed_dtype, ld_packed, meta, mode, mask,
                                ld_mask, nullptr, 0, seed, offset, nullptr, e_tc, row_sums, stream, col_major ? 1 : 0, 1.f, 0, 1.f, amax,
                                q_dense, ld_q);
+}
+
+// Storage rows of a column-major matrix that one block of the converting kernel covers: eight metadata words.
+extern "C" int sp24_row_parts(int64_t k, int packed_dtype) {
+    const int so = sp24::dtype_size(packed_dtype);
+    const int64_t per = so == 1 ? 256 : 128;
+    return so != 1 && so != 2 ? 0 : (int)((k + per - 1) / per);
+}
+
+extern "C" int sp24_prune_compress_with(const void *dense, int dense_dtype, int64_t m, int64_t k, int64_t ld_dense, int col_major,
+                                        void *packed, int packed_dtype, int64_t ld_packed, void *meta, int mode, const void *mask,
+                                        int64_t ld_mask, const float *uniforms, int64_t ld_uniforms, uint64_t seed, uint64_t offset,
+                                        const sp24_prune_extras *x, void *stream) {
+    if (!x || mode > SP24_PRUNE_MVUE_FAST) return SP24_ERR_ARG;
+    if (x->offset_dev && (reinterpret_cast<uintptr_t>(x->offset_dev) & 7u)) return SP24_ERR_ARG;
+    if (x->amax && packed_dtype != SP24_E4M3 && packed_dtype != SP24_E5M2) return SP24_ERR_DTYPE;
+    return prune_compress_impl(dense, dense_dtype, m, k, ld_dense, col_major, packed, packed_dtype, ld_packed, meta, mode, mask, ld_mask,
+                               uniforms, ld_uniforms, seed, offset, x->offset_dev, x->e_tc, x->row_parts, stream, x->packed_row_major && col_major ? 1 : 0,
+                               1.f, 0, 1.f, x->amax, x->q_dense, x->ld_q, true);
 }
 
 // S-STE forward in one pass: magnitude 2:4 mask, soft threshold of the kept values (one rounding in the input type),

@@ -238,9 +238,20 @@ void sparse_mm_accumulate(const Tensor &out, const Tensor &weight, const Tensor 
 // ---------------------------------------------------------------------------------------------
 // dense -> 2:4
 // ---------------------------------------------------------------------------------------------
+// Row sums that the compressing pass takes along (the bias gradient): `out` is set to them, or increased by them.  `parts` is
+// scratch for partial sums (row_parts_bytes), which are added up in a fixed order: a gradient repeats bit for bit.
+struct RowSums {
+    float *out = nullptr, *parts = nullptr;
+    bool add = false;
+};
+int64_t row_parts_bytes(int64_t m, int64_t k, at::ScalarType packed) { return 4 * m * sp24_row_parts(k, dt(packed)); }
+void sum_parts(const RowSums &s, int64_t m, int64_t k, at::ScalarType packed) {
+    check(sp24_sum_parts(s.parts, sp24_row_parts(k, dt(packed)), m, s.out, s.add, cur_stream()), "sp24_sum_parts");
+}
+
 // Fills packed / meta from dense; returns the metadata in tensor-core order when it was asked for and the shape allows.
 OptTensor prune_into(const Tensor &dense_in, const Tensor &packed, const Tensor &meta, int64_t mode, const OptTensor &mask_in,
-                     const OptTensor &uniforms_in, uint64_t seed, uint64_t offset, c10::optional<bool> emit_tc, const OptTensor &row_sums,
+                     const OptTensor &uniforms_in, uint64_t seed, uint64_t offset, c10::optional<bool> emit_tc, const RowSums &sums = {},
                      OptTensor e_tc = {}) {
     TORCH_CHECK(dense_in.dim() == 2, "Expected 2-dimensional dense tensor, got ", dense_in.dim(), "-dimensional tensor");
     const int64_t m = dense_in.size(0), k = dense_in.size(1);
@@ -266,21 +277,30 @@ OptTensor prune_into(const Tensor &dense_in, const Tensor &packed, const Tensor 
     const bool want_tc = emit_tc.has_value() ? *emit_tc : lp.col == 1;
     if (!e_tc.has_value() && want_tc && packed.element_size() == 2 && m % 128 == 0)
         e_tc = empty({sp24_meta_tc_bytes(m, k)}, at::kByte, packed);
-    if (row_sums.has_value())
-        TORCH_CHECK(lp.col && row_sums->scalar_type() == at::kFloat && row_sums->numel() == m && row_sums->is_contiguous(),
-                    "row_sums: column-major input and a contiguous float32 vector of one value per row");
-    check(sp24_prune_compress_ex(ptr(dense), dt(dense.scalar_type()), m, k, layout_of(dense).ld, lp.col, ptr(packed),
-                                 dt(packed.scalar_type()), lp.ld, ptr(meta), (int)mode, ptr(mask), ld_m,
-                                 static_cast<const float *>(ptr(uniforms)), ld_u, seed, offset, static_cast<const uint64_t *>(dev_off),
-                                 const_cast<void *>(ptr(e_tc)), static_cast<float *>(const_cast<void *>(ptr(row_sums))), cur_stream()),
+    sp24_prune_extras x{};
+    x.offset_dev = static_cast<const uint64_t *>(dev_off);
+    x.e_tc = const_cast<void *>(ptr(e_tc));
+    x.row_parts = sums.parts;
+    check(sp24_prune_compress_with(ptr(dense), dt(dense.scalar_type()), m, k, layout_of(dense).ld, lp.col, ptr(packed),
+                                   dt(packed.scalar_type()), lp.ld, ptr(meta), (int)mode, ptr(mask), ld_m,
+                                   static_cast<const float *>(ptr(uniforms)), ld_u, seed, offset, &x, cur_stream()),
           "sp24_prune_compress");
+    if (sums.out) sum_parts(sums, m, k, packed.scalar_type());
     return e_tc;
 }
 OptTensor prune_compress(const Tensor &dense, const Tensor &packed, const Tensor &meta, int64_t mode, const OptTensor &mask,
                          const OptTensor &uniforms, uint64_t seed, uint64_t offset, c10::optional<bool> emit_tc, const OptTensor &row_sums) {
     NoAutograd guard;
     require_cuda(dense, packed, meta, mask, uniforms, row_sums);
-    return prune_into(dense, packed, meta, mode, mask, uniforms, seed, offset, emit_tc, row_sums);
+    RowSums sums;
+    Tensor scratch;
+    if (row_sums.has_value() && dense.dim() == 2) {
+        TORCH_CHECK(layout_of(packed).col && row_sums->scalar_type() == at::kFloat && row_sums->numel() == dense.size(0) && row_sums->is_contiguous(),
+                    "row_sums: column-major input and a contiguous float32 vector of one value per row");
+        scratch = empty({row_parts_bytes(dense.size(0), dense.size(1), packed.scalar_type())}, at::kByte, packed);
+        sums = {static_cast<float *>(ptr(*row_sums)), static_cast<float *>(ptr(scratch)), true};
+    }
+    return prune_into(dense, packed, meta, mode, mask, uniforms, seed, offset, emit_tc, sums);
 }
 
 // One allocation of m*k*cf/16 elements: packed values (in the storage order asked for) first, metadata behind.
@@ -296,7 +316,7 @@ std::tuple<Tensor, Tensor, OptTensor> compress(const Tensor &dense, at::ScalarTy
     NoAutograd guard;
     require_cuda(dense, mask);
     auto [packed, meta] = carve_compressed(dense.size(0), dense.size(1), t, !(dense.stride(0) > dense.stride(1)), dense);
-    OptTensor e = prune_into(dense, packed, meta, mode, mask, {}, seed, 0, {}, {});
+    OptTensor e = prune_into(dense, packed, meta, mode, mask, {}, seed, 0, {});
     return {packed, meta, e};
 }
 
@@ -464,28 +484,27 @@ std::pair<Tensor, Tensor> fst_weight_grads(const Tensor &g_in, const Tensor &x, 
                     "): features % 32 == 0 and tokens % 64 == 0 required");
         const bool f32 = weight.scalar_type() == at::kFloat && in_f % 8 == 0;
         const bool into = into_grad && f32 && accumulable(weight.grad());
-        // the bias gradient: into bias.grad, or into the tail of the zeroed buffer that receives dW
         Tensor sums, acc;
         if (into) {
             acc = weight.grad();
             if (need_b && accumulable(bias.grad())) sums = bias.grad();
         } else if (f32) {
-            const bool with_b = need_b && bias.scalar_type() == at::kFloat;
-            const int64_t nw = out_f * in_f, total = nw + (with_b ? out_f : 0);
-            Tensor buf = empty({total}, at::kFloat, g);
-            check(sp24_zero(ptr(buf), total * 4, cur_stream()), "sp24_zero");
-            acc = gw = carve(buf, 0, at::kFloat, {out_f, in_f}, {in_f, 1});
-            if (with_b) sums = gb = carve(buf, nw * 4, at::kFloat, {out_f}, {1});
+            acc = gw = empty({out_f, in_f}, at::kFloat, g);
+            check(sp24_zero(ptr(gw), out_f * in_f * 4, cur_stream()), "sp24_zero");
+            if (need_b && bias.scalar_type() == at::kFloat) sums = gb = empty({out_f}, at::kFloat, g);
         }
-        // packed values, metadata and its tensor-core copy, all consumed by the next launch
+        // packed values, metadata, its tensor-core copy and partial bias sums, all consumed by the next launches
         const int64_t vb = out_f * tokens, mb = out_f * tokens / 8;
         const bool tc = out_f % 128 == 0;
-        Tensor buf = empty({align256(vb + mb) + (tc ? sp24_meta_tc_bytes(out_f, tokens) : 0)}, at::kByte, g);
+        const int64_t o_tc = align256(vb + mb), o_parts = align256(o_tc + (tc ? sp24_meta_tc_bytes(out_f, tokens) : 0));
+        Tensor buf = empty({o_parts + (sums.defined() ? row_parts_bytes(out_f, tokens, g.scalar_type()) : 0)}, at::kByte, g);
         const Tensor gp = carve(buf, 0, g.scalar_type(), {out_f, tokens / 2}, {1, out_f});
         const Tensor gm = carve(buf, vb, at::kShort, {out_f, tokens / 16}, {tokens / 16, 1});
         OptTensor e;
-        if (tc) e = carve(buf, align256(vb + mb), at::kByte, {sp24_meta_tc_bytes(out_f, tokens)}, {1});
-        prune_into(g.t(), gp, gm, SP24_PRUNE_MVUE_FAST, {}, {}, seed, 0, false, sums.defined() ? OptTensor(sums) : OptTensor(), e);
+        if (tc) e = carve(buf, o_tc, at::kByte, {sp24_meta_tc_bytes(out_f, tokens)}, {1});
+        RowSums rs;
+        if (sums.defined()) rs = {static_cast<float *>(ptr(sums)), reinterpret_cast<float *>(static_cast<char *>(ptr(buf)) + o_parts), into};
+        prune_into(g.t(), gp, gm, SP24_PRUNE_MVUE_FAST, {}, {}, seed, 0, false, rs, e);
         if (sums.defined()) need_b = false;
         TORCH_CHECK(tc, "sparse GEMM on sm_100a: number of rows of the sparse matrix must be divisible by 128");
         if (acc.defined()) mm_accumulate(acc, gp, *e, x, 0);
@@ -605,16 +624,29 @@ Q8 compress_q8(const Tensor &dense_in, int mode, const OptTensor &mask_in, const
         ld_m = layout_of(*mask).ld;
     }
     const int64_t vb = m * k / 2, mb = m * k / 8, tb = m % 128 == 0 ? sp24_meta_tc_bytes(m, k) : 0;
-    Tensor buf = empty({align256(vb) + align256(mb) + tb}, at::kByte, dense);
+    const int64_t o_parts = align256(align256(vb) + align256(mb) + tb);
+    Tensor buf = empty({o_parts + (row_sums.defined() ? row_parts_bytes(m, k, at::kFloat8_e4m3fn) : 0)}, at::kByte, dense);
     Q8 o;
     o.packed = carve(buf, 0, at::kFloat8_e4m3fn, {m, k / 2}, {k / 2, 1});
     o.meta = carve(buf, align256(vb), at::kInt, {m, k / 32}, {k / 32, 1});
     if (tb) o.tc = carve(buf, align256(vb) + align256(mb), at::kByte, {tb}, {1});
-    check(sp24_prune_compress_q8_dev(ptr(dense), dt(dense.scalar_type()), m, k, l.ld, l.col, ptr(o.packed), SP24_E4M3, k / 2, ptr(o.meta), mode,
-                                     ptr(mask), ld_m, static_cast<const float *>(ptr(amax)), seed, 0, tb ? ptr(o.tc) : nullptr,
-                                     row_sums.defined() ? static_cast<float *>(ptr(row_sums)) : nullptr,
-                                     q_dense.defined() ? ptr(q_dense) : nullptr, q_dense.defined() ? q_dense.size(1) : 0, cur_stream()),
+    sp24_prune_extras x{};
+    x.amax = static_cast<const float *>(ptr(amax));
+    x.packed_row_major = 1;
+    if (tb) x.e_tc = ptr(o.tc);
+    RowSums sums;
+    if (row_sums.defined()) {
+        sums = {static_cast<float *>(ptr(row_sums)), reinterpret_cast<float *>(static_cast<char *>(ptr(buf)) + o_parts), false};
+        x.row_parts = sums.parts;
+    }
+    if (q_dense.defined()) {
+        x.q_dense = ptr(q_dense);
+        x.ld_q = q_dense.size(1);
+    }
+    check(sp24_prune_compress_with(ptr(dense), dt(dense.scalar_type()), m, k, l.ld, l.col, ptr(o.packed), SP24_E4M3, k / 2, ptr(o.meta), mode,
+                                   ptr(mask), ld_m, nullptr, 0, seed, 0, &x, cur_stream()),
           "sp24_prune_compress_q8");
+    if (sums.out) sum_parts(sums, m, k, at::kFloat8_e4m3fn);
     return o;
 }
 
@@ -684,11 +716,10 @@ struct Fp8Backward : torch::autograd::Node {
         if (need_w) {
             // one pass over dY: the MVUE compression of dY^T, the quantised dY and the bias gradient
             const Tensor xq_t = xq_t_.unpack();
-            const int64_t in_f = xq_t.size(0), nw = of * in_f;
-            Tensor buf = empty({nw + of}, at::kFloat, g);
-            check(sp24_zero(ptr(buf), (nw + of) * 4, cur_stream()), "sp24_zero");
-            Tensor gw = carve(buf, 0, at::kFloat, {of, in_f}, {in_f, 1}), gb = carve(buf, nw * 4, at::kFloat, {of}, {1});
-            const Q8 c = compress_q8(g.t(), SP24_PRUNE_MVUE_FAST, {}, amax, seed, need_b ? gb : Tensor(), gq);
+            const int64_t in_f = xq_t.size(0);
+            Tensor gw = empty({of, in_f}, at::kFloat, g), gb = need_b ? empty({of}, at::kFloat, g) : Tensor();
+            check(sp24_zero(ptr(gw), of * in_f * 4, cur_stream()), "sp24_zero");
+            const Q8 c = compress_q8(g.t(), SP24_PRUNE_MVUE_FAST, {}, amax, seed, gb, gq);
             TORCH_CHECK(c.tc.defined(), "sparse GEMM on sm_100a: number of rows of the sparse matrix must be divisible by 128");
             check(sp24_spmm_f8(ptr(c.packed), SP24_E4M3, n / 2, ptr(c.tc), of, n, ptr(xq_t), n, in_f, ptr(gw), SP24_F32, 0, in_f, nullptr,
                                static_cast<const float *>(ptr(amax)), static_cast<const float *>(ptr(amax_x_)), status_ptr(g), cur_stream()),

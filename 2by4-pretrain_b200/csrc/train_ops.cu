@@ -525,6 +525,28 @@ __global__ void __launch_bounds__(256) column_sums_kernel(const T *x, int64_t ro
     }
 }
 
+// out[c] (+)= sum of parts[p, c] over p, in a fixed order: eight threads of a block take every eighth row of a column, the first
+// adds their sums up.  Bound by latency and the launch; the layer step with 128 x 3072 partial sums (16384 x 768 -> 3072, fp16)
+// went from 242.3 us with atomics to 246.3.
+__global__ void __launch_bounds__(256) sum_parts_kernel(const float *parts, int64_t n_parts, int64_t m, float *out, int accumulate) {
+    __shared__ float part[8][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t c = (int64_t)blockIdx.x * 32 + lane;
+    float s = 0.f;
+    if (c < m) {
+#pragma unroll 8
+        for (int64_t p = warp; p < n_parts; p += 8) s += parts[p * m + c];
+    }
+    part[warp][lane] = s;
+    __syncthreads();
+    if (warp == 0 && c < m) {
+        float t = 0.f;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) t += part[w][lane];
+        out[c] = accumulate ? out[c] + t : t;
+    }
+}
+
 // g *= *factor unless *factor == 1 (the usual case: nothing is read or written then)
 template <typename T>
 __global__ void __launch_bounds__(256) scale_unless_one_kernel(T *g, const float *factor, int64_t nvec) {
@@ -739,6 +761,14 @@ extern "C" int sp24_column_sums(const void *x, int dtype, int64_t rows, int64_t 
     const dim3 grid((unsigned)cb, (unsigned)((rows + per - 1) / per));
     if (dtype == SP24_F16) column_sums_kernel<__half><<<grid, 256, 0, st>>>(static_cast<const __half *>(x), rows, cols, ld, per, out);
     else column_sums_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(static_cast<const __nv_bfloat16 *>(x), rows, cols, ld, per, out);
+    return launch_status();
+}
+
+extern "C" int sp24_sum_parts(const float *parts, int64_t n_parts, int64_t m, float *out, int accumulate, void *stream) {
+    if (!parts || !out) return SP24_ERR_ARG;
+    if (n_parts <= 0 || m <= 0 || (m + 31) / 32 > 0x7FFFFFFF) return SP24_ERR_SHAPE;
+    if (int rc = check_device()) return rc;
+    sum_parts_kernel<<<(unsigned)((m + 31) / 32), 256, 0, static_cast<cudaStream_t>(stream)>>>(parts, n_parts, m, out, accumulate);
     return launch_status();
 }
 

@@ -163,6 +163,30 @@ int sp24_prune_compress_q8_dev(const void *dense, int dense_dtype, int64_t m, in
                                int64_t ld_q, void *stream);
 
 /*
+ * sp24_prune_compress with all extras, each of which may be NULL; offset_dev, e_tc, amax and q_dense as in the two entry points
+ * above.  packed_row_major: float8 results of column-major input leave row-major, as sp24_prune_compress_q8 writes them (q_dense
+ * asks for it).  row_parts instead of row_sums:
+ * float32 (sp24_row_parts(k, packed_dtype), m), partial sums over 128 (float8: 256) consecutive k of the unpruned
+ * dense[r, k], column-major storage only.  sp24_sum_parts adds them up in a fixed order (accumulate = 1: to what out holds),
+ * so that the same gradient gives the same bits every time, which row_sums' atomics do not promise.
+ */
+typedef struct sp24_prune_extras {
+    const float *amax;
+    const uint64_t *offset_dev;
+    void *e_tc;
+    float *row_parts;
+    void *q_dense;
+    int64_t ld_q;
+    int packed_row_major;
+} sp24_prune_extras;
+int sp24_row_parts(int64_t k, int packed_dtype);
+int sp24_prune_compress_with(const void *dense, int dense_dtype, int64_t m, int64_t k, int64_t ld_dense, int col_major, void *packed,
+                             int packed_dtype, int64_t ld_packed, void *meta, int mode, const void *mask, int64_t ld_mask,
+                             const float *uniforms, int64_t ld_uniforms, uint64_t seed, uint64_t offset, const sp24_prune_extras *extras,
+                             void *stream);
+int sp24_sum_parts(const float *parts, int64_t n_parts, int64_t m, float *out, int accumulate, void *stream);
+
+/*
  * 2:4 compressed -> dense (zeros at pruned positions).  Replaces
  * _sparse_semi_structured_to_dense_triton / _sparse_semi_structured_to_dense
  * (sparse/_semi_structured_conversions.py:1163-1274, :217-328).
