@@ -3,6 +3,8 @@
 // in the same pass) and the cross-entropy loss over 16-bit logits (log-sum-exp forward, gradient written as 16-bit
 // values).  Both are HBM-bound streaming kernels on 16-byte accesses; neither has a counterpart in the reference,
 // whose training scripts live in another repository.
+#include <cooperative_groups.h>
+
 #include "sp24_common.cuh"
 
 namespace sp24 {
@@ -483,30 +485,34 @@ __global__ void __launch_bounds__(256) gelu_kernel(const uint4 *x, const uint4 *
     }
 }
 
-// out[c] += sum over rows of x[r, c] (float32): a warp reads 256 consecutive columns of a row, the block's eight warps
-// take rows in turn, one atomic per column and block at the end
+// out[c] += sum over rows of x[r, c] (float32), in a fixed order.  A cluster of eight blocks takes 64 columns, each block an
+// eighth of the rows: 8 threads read one row's 128 bytes, 64 rows in turn, four of them in flight per thread.  Block 0 adds
+// the eight blocks' sums up through distributed shared memory, so no atomics and no scratch.  Bound by latency: 4096 x 2304 in
+// 8.0 us, 8192 x 3072 in 14.1 (128 columns a cluster 8.3 and 14.6; with atomics in any order 5.6 and 11.1).
+constexpr int CS_COLS = 64, CS_BLOCKS = 8, CS_ROWS = 512 / (CS_COLS / 8), CS_FLIGHT = 4;
 template <typename T>
-__global__ void __launch_bounds__(256) column_sums_kernel(const T *x, int64_t rows, int64_t cols, int64_t ld, int64_t rows_per_block, float *out) {
-    __shared__ float part[8][256 + 8];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int64_t c = (int64_t)blockIdx.x * 256 + lane * 8;
-    const int64_t r0 = (int64_t)blockIdx.y * rows_per_block, r1 = r0 + rows_per_block < rows ? r0 + rows_per_block : rows;
+__global__ void __cluster_dims__(1, CS_BLOCKS, 1) __launch_bounds__(512) column_sums_kernel(const T *x, int64_t rows, int64_t cols, int64_t ld, float *out) {
+    __shared__ float part[CS_ROWS][CS_COLS + 4], total[CS_COLS];
+    const auto cluster = cooperative_groups::this_cluster();
+    const int piece = threadIdx.x % (CS_COLS / 8), group = threadIdx.x / (CS_COLS / 8);
+    const int64_t c = (int64_t)blockIdx.x * CS_COLS + piece * 8;
+    const int64_t per = (rows + CS_BLOCKS - 1) / CS_BLOCKS, r0 = blockIdx.y * per, r1 = r0 + per < rows ? r0 + per : rows;
     float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     if (c < cols) {
-        int64_t r = r0 + warp;
-        for (; r + 24 < r1; r += 32) {      // four rows in flight
-            uint4 v[4];
+        int64_t r = r0 + group;
+        for (; r + (CS_FLIGHT - 1) * CS_ROWS < r1; r += CS_FLIGHT * CS_ROWS) {
+            uint4 v[CS_FLIGHT];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) v[j] = *reinterpret_cast<const uint4 *>(x + (r + 8 * j) * ld + c);
+            for (int j = 0; j < CS_FLIGHT; ++j) v[j] = *reinterpret_cast<const uint4 *>(x + (r + CS_ROWS * j) * ld + c);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
+            for (int j = 0; j < CS_FLIGHT; ++j) {
                 float f[8];
                 unpack8<T>(v[j], f);
 #pragma unroll
                 for (int i = 0; i < 8; ++i) s[i] += f[i];
             }
         }
-        for (; r < r1; r += 8) {
+        for (; r < r1; r += CS_ROWS) {
             float f[8];
             unpack8<T>(*reinterpret_cast<const uint4 *>(x + r * ld + c), f);
 #pragma unroll
@@ -514,15 +520,23 @@ __global__ void __launch_bounds__(256) column_sums_kernel(const T *x, int64_t ro
         }
     }
 #pragma unroll
-    for (int i = 0; i < 8; ++i) part[warp][lane * 8 + i] = s[i];
+    for (int i = 0; i < 8; ++i) part[group][piece * 8 + i] = s[i];
     __syncthreads();
-    const int64_t col = (int64_t)blockIdx.x * 256 + threadIdx.x;
-    if (col < cols) {
+    if (threadIdx.x < CS_COLS) {
         float t = 0.f;
 #pragma unroll
-        for (int w = 0; w < 8; ++w) t += part[w][threadIdx.x];
-        atomicAdd(out + col, t);
+        for (int g = 0; g < CS_ROWS; ++g) t += part[g][threadIdx.x];
+        total[threadIdx.x] = t;
     }
+    cluster.sync();
+    const int64_t col = (int64_t)blockIdx.x * CS_COLS + threadIdx.x;
+    if (cluster.block_rank() == 0 && threadIdx.x < CS_COLS && col < cols) {
+        float t = 0.f;
+#pragma unroll
+        for (int b = 0; b < CS_BLOCKS; ++b) t += *cluster.map_shared_rank(&total[threadIdx.x], b);
+        out[col] += t;
+    }
+    cluster.sync();                         // the other blocks' shared memory stays until block 0 has read it
 }
 
 // out[c] (+)= sum of parts[p, c] over p, in a fixed order: eight threads of a block take every eighth row of a column, the first
@@ -751,16 +765,9 @@ extern "C" int sp24_column_sums(const void *x, int dtype, int64_t rows, int64_t 
     if (!aligned16(x)) return SP24_ERR_ALIGN;
     if (int rc = check_device()) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    // about four blocks per SM, each with at least one four-row trip of its eight warps
-    const int64_t cb = (cols + 255) / 256;
-    int64_t rb = ((int64_t)sm_count() * 4 + cb - 1) / cb;
-    const int64_t most = (rows + 31) / 32;
-    if (rb > most) rb = most;
-    if (rb > 65535) rb = 65535;
-    const int64_t per = (rows + rb - 1) / rb;
-    const dim3 grid((unsigned)cb, (unsigned)((rows + per - 1) / per));
-    if (dtype == SP24_F16) column_sums_kernel<__half><<<grid, 256, 0, st>>>(static_cast<const __half *>(x), rows, cols, ld, per, out);
-    else column_sums_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(static_cast<const __nv_bfloat16 *>(x), rows, cols, ld, per, out);
+    const dim3 grid((unsigned)((cols + CS_COLS - 1) / CS_COLS), CS_BLOCKS);
+    if (dtype == SP24_F16) column_sums_kernel<__half><<<grid, 512, 0, st>>>(static_cast<const __half *>(x), rows, cols, ld, out);
+    else column_sums_kernel<__nv_bfloat16><<<grid, 512, 0, st>>>(static_cast<const __nv_bfloat16 *>(x), rows, cols, ld, out);
     return launch_status();
 }
 

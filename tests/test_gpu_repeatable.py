@@ -42,7 +42,7 @@ def _step(kind, tokens, in_f, out_f, dtype, into=False):
 
 # (tokens, in, out): one partial sum, a ragged number of them, and enough blocks to finish in any order
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
-@pytest.mark.parametrize("kind,into", [("fst", False), ("fst", True), ("fp8", False)])
+@pytest.mark.parametrize("kind,into", [("fst", False), ("fst", True), ("fp8", False), ("sste", False)])
 @pytest.mark.parametrize("tokens,in_f,out_f", [(256, 256, 256), (768, 128, 384), (16384, 256, 1024)])
 def test_bias_gradient_repeats(kind, into, tokens, in_f, out_f, dtype):
     """The same bits every time, and float32 sums: within ``tokens`` roundings of the sum of magnitudes."""
