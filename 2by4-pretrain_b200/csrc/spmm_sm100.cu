@@ -1528,6 +1528,22 @@ int pick_pair_bn(int64_t ms, int64_t n, bool plain) {
     return best;
 }
 
+// Tile and K slices of the float8 weight gradient (added to out with float32 reductions).  At most two slices: two addends on a
+// zeroed buffer give the same bits in either order, three do not.  Among these, the fewest bytes staged per CTA.
+// ms 3072, n 768, k 8192: 256 x 128 tiles in two slices (144 units) instead of 256 x 192 in three.
+void pick_f8_accumulate(int64_t ms, int64_t n, int64_t k, int sms, int &bn_out, int &mpt_out, int &splits_out) {
+    const int64_t k_iters = (k + 255) / 256;
+    int64_t best = INT64_MAX;
+    for (int bn : {192, 128})
+        for (int mpt = ms >= 256 ? 2 : 1; mpt >= 1; --mpt)
+            for (int splits = 1; splits <= (k_iters > 1 ? 2 : 1); ++splits) {
+                const int64_t units = ((n + bn - 1) / bn) * ((ms / BM + mpt - 1) / mpt) * splits;
+                const int64_t stage = (int64_t)mpt * (A_STAGE_BYTES + 4096) + bn * 256;
+                const int64_t cost = ((units + sms - 1) / sms) * (((k_iters + splits - 1) / splits) * stage);
+                if (cost < best) { best = cost; bn_out = bn; mpt_out = mpt; splits_out = splits; }
+            }
+}
+
 template <bool F8, bool A_MN, bool B_MN, bool TRANS, typename OutT>
 int dispatch_bn(int bn, const void *b, int dtype, int64_t n, int64_t k, int64_t ld_b, const CUtensorMap &ma,
                 const SpmmParams &P, cudaStream_t st) {
@@ -1707,7 +1723,7 @@ extern "C" int sp24_spmm_mlp(const void *a_packed, int dtype, int a_mn_major, in
 // product of the operands' scales, worked out from their absolute maxima (sp24_absmax).
 //   trans_out = 1: out (n, ms) in float32, float16 or bfloat16 (rounded once): the layer's output or input gradient
 //   without a float32 copy.  16-bit outputs of whole 256-row blocks run on CTA pairs.
-//   trans_out = 0: out (ms, n) float32 += alpha * A * B (no bias), K cut into slices over idle SMs: the weight gradient.
+//   trans_out = 0: out (ms, n) float32 += alpha * A * B (no bias), K cut into up to two slices: the weight gradient.
 extern "C" int sp24_spmm_f8(const void *a_packed, int dtype, int64_t ld_a, const void *e_tc, int64_t ms, int64_t k, const void *b, int64_t ld_b,
                             int64_t n, void *out, int out_dtype, int trans_out, int64_t ld_out, const float *bias, const float *amax_a,
                             const float *amax_b, int *status, void *stream) {
@@ -1743,13 +1759,7 @@ extern "C" int sp24_spmm_f8(const void *a_packed, int dtype, int64_t ld_a, const
         mpt = tiles >= sms ? 2 : 1;
     }
     if (!trans_out) {
-        // widest tile (least operand traffic), then as many K slices as idle SMs allow
-        bn = n >= 192 ? 192 : 128;
-        mpt = ms >= 256 ? 2 : 1;
-        const int64_t tiles = ((n + bn - 1) / bn) * ((ms / BM + mpt - 1) / mpt), k_iters = (k + 255) / 256;
-        int64_t splits = sms / tiles;
-        splits = splits < 1 ? 1 : (splits > k_iters ? k_iters : splits);
-        P.k_splits = (int)splits;
+        pick_f8_accumulate(ms, n, k, sms, bn, mpt, P.k_splits);
         P.accumulate = 1;
     }
     P.mblk_per_tile = mpt;

@@ -412,7 +412,7 @@ int sp24_spmm_scaled(const void *a_packed, int dtype, int64_t ld_a, const void *
  * The GEMMs of a float8 layer whose scales stay on the device: D = alpha * (A_sparse * B) [+ bias], alpha the product of
  * the operands' scales (see sp24_absmax).  Both operands K-major.  trans_out = 1: out (n, ms) in out_dtype F32, F16 or
  * BF16 (rounded once from float32), bias float32 or NULL.  trans_out = 0: out (ms, n) float32 += alpha * A * B, no bias, K
- * cut into slices over idle SMs (fixed sums are not promised: slices are added with float32 reductions).
+ * cut into up to two slices, each added with float32 reductions: on a zeroed out the result repeats bit for bit.
  */
 int sp24_spmm_f8(const void *a_packed, int dtype, int64_t ld_a, const void *e_tc, int64_t ms, int64_t k, const void *b, int64_t ld_b,
                  int64_t n, void *out, int out_dtype, int trans_out, int64_t ld_out, const float *bias, const float *amax_a,

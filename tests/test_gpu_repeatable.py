@@ -62,3 +62,13 @@ def test_sum_of_parts(n_parts, m):
         _ext.check(_ext.lib().sp24_sum_parts(parts.data_ptr(), n_parts, m, out.data_ptr(), add, _ext.stream()), "sum_parts")
         want = parts.double().sum(0) + 3.0 * add
         assert float((out.double() - want).abs().max()) <= (n_parts + 1) * 2 ** -24 * float(3 + parts.double().abs().sum(0).max())
+
+
+# (tokens, in, out): one tile, tiles that would leave room for four and for three slices of K, more tiles than SMs
+@pytest.mark.parametrize("tokens,in_f,out_f", [(256, 256, 128), (4096, 512, 512), (8192, 768, 3072), (1024, 3072, 2048)])
+def test_float8_weight_gradient_repeats(tokens, in_f, out_f):
+    from sparse.spmm import check_status
+    dw = _step("fp8", tokens, in_f, out_f, torch.bfloat16)[0]
+    for _ in range(4):
+        assert torch.equal(_step("fp8", tokens, in_f, out_f, torch.bfloat16)[0], dw)
+    check_status()
