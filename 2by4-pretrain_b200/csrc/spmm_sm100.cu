@@ -19,6 +19,7 @@
 #include <cstdio>
 #include <cstdlib>
 
+#include "meta_steps.cuh"
 #include "sp24_common.cuh"
 
 namespace sp24 {
@@ -395,9 +396,14 @@ spmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                             tma_load_2d(sam + 8192, &map_a, mrow + 64, it * 64, full);
                         }
                         // metadata atoms of this 128-row block
-                        const uint8_t *e_src = static_cast<const uint8_t *>(P.e_tc) +
-                                               ((size_t)(mblk0 + mb) * P.k_atoms + (size_t)it * (E_BYTES / 2048)) * 2048;
-                        bulk_load(se + mb * E_BYTES, e_src, E_BYTES, full);
+                        const uint8_t *e_blk = static_cast<const uint8_t *>(P.e_tc) + (size_t)(mblk0 + mb) * P.k_atoms * 2048;
+                        if constexpr (F8) {
+                            const MetaAtoms at = meta_atoms_of_step(it, P.k_atoms);
+                            bulk_load(se + mb * E_BYTES, e_blk + at.first * 2048, 2048, full);
+                            bulk_load(se + mb * E_BYTES + 2048, e_blk + at.second * 2048, 2048, full);
+                        } else {
+                            bulk_load(se + mb * E_BYTES, e_blk + (size_t)it * 2048, 2048, full);
+                        }
                     }
                     // dense B: BN rows x 2 atoms of 128 bytes (K-major) or column blocks of 64 x 128 K-rows (MN-major)
                     if constexpr (!B_MN) {
