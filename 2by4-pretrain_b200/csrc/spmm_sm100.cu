@@ -754,7 +754,7 @@ spmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
 // (the leader) issues all MMAs and metadata copies; its commits arrive on the barriers of both CTAs.  No load
 // is multicast.
 namespace two {
-// Columns of a pair tile: a multiple of 16 in [BN2_MIN, BN2_MAX], chosen per problem (pick_pair_bn).  Two accumulator buffers
+// Columns of a pair tile: a multiple of 16 (8-bit operands: of 32) in [BN2_MIN, BN2_MAX], chosen per problem (pick_pair_bn).  Two accumulator buffers
 // of up to 240 columns start at columns 0 and 256 of tensor memory, the metadata slots sit in the 16 columns between them.
 constexpr int BN2_MIN = 32, BN2_MAX = 240, ACC_COL = 256, E_COL = 240;
 constexpr int MAX_STAGES2 = 6;
@@ -1516,19 +1516,21 @@ void pick_tile(int64_t ms, int64_t n, int sm_count, int &bn_out, int &mpt_out) {
 // where it does not leave the last round nearly empty.  fp16, us, at 192 columns -> at the width taken:
 //   ms 4096, n 2043, k 4096: 42.8 -> 33.5 (240 columns: two rounds instead of three)
 //   ms 3072, n 16384, k 768: 55.5 -> 52.0 (224); ms 768, n 16384, k 3072: 46.7 -> 43.4 (224)
-//   ms 3072, n 16384, k 3072: 148 -> 139 (240); ms 768, n 5000, k 1024: 16.5 -> 12.5 (224)
+//   ms 768, n 5000, k 1024: 16.5 -> 12.5 (224)
 // Few columns: the narrowest tile that still takes one round; against the single-CTA kernel, which took these before,
 //   ms 4096, k 4096: n 16 21.6 -> 16.5, n 256 23.9 -> 18.4, n 512 28.0 -> 18.9, n 768 30.8 -> 20.1; ms 768, k 3072, n 512 18.9 -> 14.4
 // (the single-CTA kernel was never faster, so it keeps the row counts that are odd multiples of 128 and the other layouts).
-// The fused epilogues hold up to 192 columns in registers and take them in chunks of 16 per half tile.
-int pick_pair_bn(int64_t ms, int64_t n, bool plain) {
-    const int step = plain ? 16 : 32, widest = plain ? two::BN2_MAX : 192;
-    const int64_t pairs = sm_count_cached() / 2;
+// The fused epilogues hold up to 192 columns in registers and take them in chunks of 16 per half tile.  8-bit operands: with
+// cta_group::2 and M = 256, kind::f8f6f4 takes N in multiples of 32 (kind::f16, sparse: of 16; the ranges of CUTLASS's
+// SM100_MMA_F8F6F4_2x1SM_SS_SPARSE and SM100_MMA_F16BF16_2x1SM_SS_SPARSE).
+int pick_pair_bn(int64_t ms, int64_t n, bool plain, bool f8, int sms) {
+    const int step = plain && !f8 ? 16 : 32, widest = !plain ? 192 : (f8 ? 224 : two::BN2_MAX);
+    const int64_t pairs = sms / 2;
     int best = widest;
     int64_t best_cost = INT64_MAX;
     for (int bn = widest; bn >= two::BN2_MIN; bn -= step) {
         const int64_t tiles = ((n + bn - 1) / bn) * (ms / 256);
-        const int64_t cost = ((tiles + pairs - 1) / pairs) * two::stage2_bytes(false, bn);
+        const int64_t cost = ((tiles + pairs - 1) / pairs) * two::stage2_bytes(f8, bn);
         if (cost < best_cost) { best_cost = cost; best = bn; }
     }
     return best;
@@ -1661,7 +1663,7 @@ static int spmm_impl(const void *a_packed, int dtype, int a_mn_major, int64_t ld
     if (epi != EPI_PLAIN || bias_f32) pair_form = true;      // checked above: these forms exist in the pair kernel only
     if (pair_form) {
         CUtensorMap map_b, map_e;
-        P.bn = pick_pair_bn(ms, n, epi == EPI_PLAIN);
+        P.bn = pick_pair_bn(ms, n, epi == EPI_PLAIN, false, sm_count_cached());
         rc = make_map(&map_b, b, dtype, n, k, ld_b, 64, (uint32_t)P.bn / 2);
         if (rc) return rc;
         rc = make_map_e(&map_e, e_tc, (ms / 128) * P.k_atoms);
@@ -1725,6 +1727,11 @@ extern "C" int sp24_spmm_mlp(const void *a_packed, int dtype, int a_mn_major, in
                      stream, bias_is_f32 ? 1 : 0, epilogue, aux, ld_aux);
 }
 
+extern "C" int sp24_pair_tile_columns(int64_t ms, int64_t n, int form, int sms) {
+    if (ms <= 0 || ms % 256 || n <= 0 || form < 0 || form > 2 || sms < 2) return 0;
+    return pick_pair_bn(ms, n, form != 1, form == 2, sms);
+}
+
 // The GEMMs of a float8 layer whose scales stay on the device: D = alpha * (A_sparse * B) [+ float32 bias], alpha = the
 // product of the operands' scales, worked out from their absolute maxima (sp24_absmax).
 //   trans_out = 1: out (n, ms) in float32, float16 or bfloat16 (rounded once): the layer's output or input gradient
@@ -1749,7 +1756,7 @@ extern "C" int sp24_spmm_f8(const void *a_packed, int dtype, int64_t ld_a, const
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (trans_out && out_dtype != SP24_F32 && ms % 256 == 0 && pair_kernels_enabled()) {
         CUtensorMap map_e;
-        P.bn = pick_pair_bn(ms, n, true);
+        P.bn = pick_pair_bn(ms, n, true, true, sm_count_cached());
         if (int rc = make_map(&map_b, b, dtype, n, k, ld_b, 128, (uint32_t)P.bn / 2)) return rc;
         if (int rc = make_map_e(&map_e, e_tc, (ms / 128) * P.k_atoms, 2)) return rc;
         return out_dtype == SP24_F16 ? launch_spmm_pair<false, __half, EPI_PLAIN, true>(map_a, map_b, map_e, P, st)

@@ -409,6 +409,13 @@ int sp24_spmm_scaled(const void *a_packed, int dtype, int64_t ld_a, const void *
                      float alpha, int *status, void *stream);
 
 /*
+ * Columns of the tile that the CTA-pair GEMM takes for (ms, n) on a GPU of `sms` SMs: host arithmetic only, for tests and for
+ * reading a profile.  form 0: 16-bit operands, plain result; 1: a fused epilogue (sp24_spmm_mlp); 2: float8 (sp24_spmm_f8).
+ * 0 when no pair tile exists.
+ */
+int sp24_pair_tile_columns(int64_t ms, int64_t n, int form, int sms);
+
+/*
  * The GEMMs of a float8 layer whose scales stay on the device: D = alpha * (A_sparse * B) [+ bias], alpha the product of
  * the operands' scales (see sp24_absmax).  Both operands K-major.  trans_out = 1: out (n, ms) in out_dtype F32, F16 or
  * BF16 (rounded once from float32), bias float32 or NULL.  trans_out = 0: out (ms, n) float32 += alpha * A * B, no bias, K

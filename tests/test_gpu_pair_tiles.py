@@ -1,7 +1,9 @@
-"""Widths of the CTA-pair GEMM's tiles: every width the rule can take, at ragged ends, bit for bit against the single-CTA kernel
-(reached through the activation, which the pair kernel does not have)."""
+"""Widths of the CTA-pair GEMM's tiles, bit for bit against the single-CTA kernel (reached through the activation, which the pair
+kernel does not have): fixed sizes at ragged ends and over several rounds, and per form one size for every width the rule takes."""
 import pytest
 import torch
+
+from _pair_tiles import FLOAT8, FUSED, PLAIN, WIDTHS, shapes
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -15,7 +17,7 @@ def _operand(ms, k, dtype, seed, col):
     return sp.sparse_tensor_cutlass, sp.meta_tensor_cutlass, g
 
 
-# (ms, n): one round at widths 32 .. 240 (n alone decides where ms is small), several rounds, and the ragged ends of tiles
+# (ms, n): one round (n alone decides where ms is small), several rounds, and the ragged ends of tiles
 SIZES = [(256, n) for n in (1, 15, 16, 17, 31, 33, 2368, 2369, 3553, 17760, 17761)] + \
         [(2048, n) for n in (9, 257, 288, 289, 433, 721, 1297)] + [(3072, 1100), (768, 5000), (4096, 1023)]
 
@@ -71,3 +73,42 @@ def test_float8_pair_products(ms, n):
     xq = sparse.fp8.quantize(x)[0].double() * sx
     ref = xq @ wq.t()
     assert float((y.double() - ref).norm() / ref.norm()) <= 2 ** -8
+
+
+def _size(form, width):
+    """(ms, n) of ``width`` on this GPU."""
+    return shapes(form, torch.cuda.get_device_properties(0).multi_processor_count)[width]
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("width", sorted(WIDTHS[PLAIN]))
+def test_plain_products_at_each_width(width, dtype):
+    test_every_tile_width_has_the_single_cta_bits(dtype, width % 32 == 0, *_size(PLAIN, width))
+
+
+@pytest.mark.parametrize("width", sorted(WIDTHS[FUSED]))
+def test_fused_epilogues_at_each_width(width):
+    test_fused_epilogues_at_every_width(*_size(FUSED, width))
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("width", sorted(WIDTHS[FLOAT8]))
+@pytest.mark.parametrize("k", [256, 640])
+def test_float8_products_at_each_width(width, k, dtype):
+    """16-bit results of the pair kernel against the float32 results of the single-CTA kernel, rounded."""
+    from sparse import _ext, fp8, spmm
+    ms, n = _size(FLOAT8, width)
+    lib = _ext.lib()
+    g = torch.Generator(device=DEV).manual_seed(width)
+    w, x = torch.randn(ms, k, device=DEV, generator=g), torch.randn(n, k, device=DEV, generator=g)
+    bias = torch.randn(ms, device=DEV, generator=g)
+    sw, (xq, sx) = fp8.scale_of(w), fp8.quantize(x)
+    aw, ax = w.abs().amax().reshape(1), x.abs().amax().reshape(1)
+    packed, meta = fp8.compress_q8(w, mode=_ext.PRUNE_MSE, scale=sw)
+    tc, status = spmm.tc_metadata(meta, ms, k), spmm._status_word(torch.device(DEV))
+    out = torch.empty(n, ms, dtype=dtype, device=DEV)
+    _ext.check(lib.sp24_spmm_f8(packed.data_ptr(), _ext.E4M3, k // 2, tc.data_ptr(), ms, k, xq.data_ptr(), k, n, out.data_ptr(),
+                                _ext.dt(dtype), 1, ms, bias.data_ptr(), aw.data_ptr(), ax.data_ptr(), status.data_ptr(), _ext.stream()),
+               "spmm_f8")
+    assert torch.equal(out, spmm.sparse_linear(xq, packed, meta, bias=bias, alpha=sw * sx).to(dtype))
+    spmm.check_status()

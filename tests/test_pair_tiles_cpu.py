@@ -1,0 +1,19 @@
+"""CPU check of the CTA-pair GEMM's tile rule: only widths that the instruction takes, and which of them are reached."""
+import random
+
+import pytest
+
+import _pair_tiles as P
+
+
+@pytest.mark.parametrize("form", [P.PLAIN, P.FUSED, P.FLOAT8])
+def test_rule_takes_legal_widths_only(form):
+    from sparse import _ext
+    rng = random.Random(form)
+    rule = _ext.lib().sp24_pair_tile_columns
+    for sms in (2, 80, 132, 148, 160):
+        for _ in range(2000):
+            ms, n = 256 * rng.randint(1, 64), int(2 ** rng.uniform(0, 22))
+            assert rule(ms, n, form, sms) in P.WIDTHS[form], (ms, n, sms)
+    assert set(P.shapes(form)) == P.WIDTHS[form]          # every width is reached, so the GPU tests' shapes cover them all
+    assert rule(128, 64, form, 148) == 0 and rule(256, 0, form, 148) == 0
