@@ -65,6 +65,12 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     if (status) atomicCAS(status, 0, code);
     return false;
 }
+// The same for a whole warp that goes on to elect a lane: one outcome for all lanes.  Each lane polls for itself, so when a
+// wait is given up some lanes may have seen the barrier flip and others not; an elect.sync that names every lane needs them all.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int *abort_flag, int *status, int code,
+                                               uint32_t limit = WAIT_LIMIT) {
+    return __all_sync(0xFFFFFFFFu, mbar_wait(bar, parity, abort_flag, status, code, limit));
+}
 __device__ __forceinline__ void fence_barrier_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
@@ -947,9 +953,9 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                 const int buf = tl & 1;
                 const uint32_t acc = tmem_base + buf * ACC_COL;
                 // the epilogues of both CTAs must have drained this accumulator buffer (two tiles ago)
-                ok = mbar_wait(tmem_empty0 + 8 * buf, ((tl >> 1) & 1) ^ 1, &abort_flag, P.status, 4);
+                ok = mbar_wait_warp(tmem_empty0 + 8 * buf, ((tl >> 1) & 1) ^ 1, &abort_flag, P.status, 4);
                 for (int it = 0; it < k_iters && ok; ++it) {
-                    ok = mbar_wait(full0 + 8 * s, ph, &abort_flag, P.status, 2);
+                    ok = mbar_wait_warp(full0 + 8 * s, ph, &abort_flag, P.status, 2);
                     if (!ok) break;
                     tc_fence_after();
                     const uint32_t off = (uint32_t)s * ((uint32_t)STAGE2_BYTES >> 4);
@@ -1217,9 +1223,9 @@ spmm_pair_acc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                 const int ks = unit / n_tiles;
                 const int it0 = (int)((int64_t)ks * k_iters / P.k_splits), it1 = (int)((int64_t)(ks + 1) * k_iters / P.k_splits);
                 // the epilogues of both CTAs must have drained the accumulator of the previous unit
-                ok = mbar_wait(tmem_empty, (tl & 1) ^ 1, &abort_flag, P.status, 4);
+                ok = mbar_wait_warp(tmem_empty, (tl & 1) ^ 1, &abort_flag, P.status, 4);
                 for (int it = it0; it < it1 && ok; ++it) {
-                    ok = mbar_wait(full0 + 8 * s, ph, &abort_flag, P.status, 2);
+                    ok = mbar_wait_warp(full0 + 8 * s, ph, &abort_flag, P.status, 2);
                     if (!ok) break;
                     tc_fence_after();
                     const uint32_t off = (uint32_t)s * (STAGE3_BYTES >> 4);
@@ -1797,14 +1803,15 @@ extern "C" int sp24_spmm_scaled(const void *a_packed, int dtype, int64_t ld_a, c
 
 // ------------------------------------------------------------------------------------------------
 // Self-test of the bounded wait: one CTA waits on a barrier that nothing ever signals, with a small
-// poll limit.  The wait must give up, record code 9 in *status and let the kernel return normally.
+// poll limit.  The wait must give up, record code 9 in *status and let the kernel return normally.  Then the whole-warp form, with
+// half of the lanes on a phase that is complete: every lane must learn that the wait was given up (code 10 otherwise).
 // ------------------------------------------------------------------------------------------------
 namespace sp24 {
 namespace {
 __global__ void wait_selftest_kernel(int *status, uint32_t limit) {
     __shared__ __align__(8) uint64_t bar;
     __shared__ int abort_flag;
-    if (threadIdx.x == 0) {
+    if (threadIdx.x == 0) {       // one warp
         abort_flag = 0;
         mbar_init(smem_u32(&bar), 1);
         fence_barrier_init();
@@ -1812,6 +1819,8 @@ __global__ void wait_selftest_kernel(int *status, uint32_t limit) {
     __syncthreads();
     if (threadIdx.x == 0) mbar_wait(smem_u32(&bar), 0, &abort_flag, status, 9, limit);
     __syncthreads();
+    const bool ok = mbar_wait_warp(smem_u32(&bar), threadIdx.x < 16 ? 1 : 0, &abort_flag, status, 9, limit);
+    if (__ballot_sync(0xFFFFFFFFu, ok) != 0 && threadIdx.x == 0) *status = 10;
 }
 }  // namespace
 }  // namespace sp24

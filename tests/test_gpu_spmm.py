@@ -334,6 +334,18 @@ def test_bounded_wait_reports_through_status_word(S):
     assert _ext.lib().sp24_selftest_bounded_wait(None, 16, None) == -5
 
 
+def test_given_up_wait_is_uniform_over_the_warp(S):
+    """A wait whose barrier has flipped for half of the lanes only: all lanes take the outcome 'gave up' (code 9; 10 if they
+    disagree), as the MMA warp must before it elects a lane."""
+    from sparse import _ext, spmm
+    status = spmm._status_word(torch.device(DEV))
+    status.zero_()
+    assert _ext.lib().sp24_selftest_bounded_wait(status.data_ptr(), 4096, _ext.stream()) == 0
+    code = int(status.item())
+    status.zero_()
+    assert code == 9
+
+
 def test_column_parallel_shards_reproduce_the_unsharded_layer(S):
     """Output-feature blocks of W, each compressed as its own matrix, give the columns of the unsharded
     product bit for bit (same masks, same K order), and the dX terms add up to the unsharded dX."""
