@@ -125,6 +125,38 @@ class _Host:
 host = _Host()
 
 
+class _Recorded(torch.autograd.Function):
+    """A native layer call as one opaque operation of a trace.  ``torch.jit.trace`` sees the outputs that the native code
+    allocates but not what its kernels write; a Python function is recorded as a call and made again on replay."""
+
+    @staticmethod
+    def forward(ctx, fn, *args):
+        # results of other operations are cut off from them (one argument may depend on another); parameters stay themselves
+        args = [a.detach().requires_grad_() if isinstance(a, torch.Tensor) and a.requires_grad and not a.is_leaf else a for a in args]
+        with torch.enable_grad():
+            out = fn(*args)
+        ctx.outs = out if isinstance(out, tuple) else (out,)
+        ctx.wrt = [(i, a) for i, a in enumerate(args) if isinstance(a, torch.Tensor) and a.requires_grad]
+        ctx.n_args = len(args)
+        detached = tuple(o.detach() for o in ctx.outs)
+        return detached if isinstance(out, tuple) else detached[0]
+
+    @staticmethod
+    def backward(ctx, *grads):
+        got = torch.autograd.grad(ctx.outs, [a for _, a in ctx.wrt], grads, retain_graph=True, allow_unused=True)
+        res = [None] * ctx.n_args
+        for (i, _), g in zip(ctx.wrt, got):
+            res[i] = g
+        return (None, *res)
+
+
+def call_layer(fn, *args):
+    """``fn(*args)`` of the native host module, recorded as a call while ``torch.jit.trace`` is running."""
+    if torch._C._get_tracing_state() is None:
+        return fn(*args)
+    return _Recorded.apply(fn, *args)
+
+
 def register_signature(name, argtypes):
     """Used by modules that bind further entry points (e.g. the sparse GEMM)."""
     _SIGNATURES[name] = argtypes

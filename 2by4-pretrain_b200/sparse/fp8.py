@@ -121,4 +121,4 @@ class sparse_linear_transpose_fp8:
 
     @staticmethod
     def apply(input, weight, w8, bias):
-        return _ext.host.fp8_linear(input, weight, bias, w8.amax, w8.pw, w8.tcw, w8.pt, w8.tct)
+        return _ext.call_layer(_ext.host.fp8_linear, input, weight, bias, w8.amax, w8.pw, w8.tcw, w8.pt, w8.tct)

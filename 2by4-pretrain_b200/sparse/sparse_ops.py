@@ -305,7 +305,7 @@ class SparseLinearTranspose(nn.Linear):
             x = F.linear(x, w, self.bias)
         else:
             self._ensure_compressed()
-            x = _ext.host.fst_linear(x, w, self.bias, w.compressed, self._tc_copies(), self.accumulate_into_grad)
+            x = _ext.call_layer(_ext.host.fst_linear, x, w, self.bias, w.compressed, self._tc_copies(), self.accumulate_into_grad)
         self._advance()
         return x
 

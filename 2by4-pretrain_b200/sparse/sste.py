@@ -83,5 +83,5 @@ class SoftThresholdLinear(nn.Linear):
         if self.spmm:
             # one kernel soft-thresholds, scales and compresses the weight; both gradients are dense GEMMs (README.md:233-267
             # of the reference): the mask is 2:4 along the rows of W only, and dW is the straight-through dY^T X
-            return _ext.host.soft_threshold_linear(x, self.weight, self.bias, self._scale(), self.spmm_dtype)
+            return _ext.call_layer(_ext.host.soft_threshold_linear, x, self.weight, self.bias, self._scale(), self.spmm_dtype)
         return F.linear(x, self.get_sparse_weights(), self.bias)

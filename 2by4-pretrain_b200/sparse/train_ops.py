@@ -18,7 +18,7 @@ class _layer_norm:
 
     @staticmethod
     def apply(x, weight, bias, eps, out_dtype, into_grad=False):
-        return _ext.host.layer_norm(x, weight, bias, eps, out_dtype, into_grad)
+        return _ext.call_layer(_ext.host.layer_norm, x, weight, bias, eps, out_dtype, into_grad)
 
 
 class _add_layer_norm:
@@ -27,7 +27,7 @@ class _add_layer_norm:
 
     @staticmethod
     def apply(x, delta, weight, bias, eps, into_grad=False):
-        return _ext.host.add_layer_norm(x, delta, weight, bias, eps, into_grad)
+        return _ext.call_layer(_ext.host.add_layer_norm, x, delta, weight, bias, eps, into_grad)
 
 
 def add_layer_norm(x: torch.Tensor, delta: torch.Tensor, norm: nn.LayerNorm):
@@ -113,7 +113,7 @@ def cross_entropy(logits: torch.Tensor, targets: torch.Tensor, fused: bool = Tru
         raise RuntimeError("cross_entropy: expected one int64 target per row")
     targets = targets.reshape(-1).contiguous()
     if fused and logits.requires_grad and torch.is_grad_enabled():
-        return _ext.host.cross_entropy(logits, targets)
+        return _ext.call_layer(_ext.host.cross_entropy, logits, targets)
     return _cross_entropy.apply(logits, targets)
 
 
@@ -131,7 +131,7 @@ def embed_tokens(ids: torch.Tensor, wte: torch.Tensor, wpe: torch.Tensor, into_g
         raise RuntimeError("embed_tokens: expected contiguous float32 tables of equal width, width % 4 == 0")
     if ids.shape[1] > wpe.shape[0]:
         raise RuntimeError(f"embed_tokens: {ids.shape[1]} positions, the position table holds {wpe.shape[0]}")
-    return _ext.host.embed_tokens(ids, wte, wpe, into_grad)
+    return _ext.call_layer(_ext.host.embed_tokens, ids, wte, wpe, into_grad)
 
 
 def gelu(x: torch.Tensor) -> torch.Tensor:
@@ -139,4 +139,4 @@ def gelu(x: torch.Tensor) -> torch.Tensor:
     kernel (float32 arithmetic, ``tanh.approx``: the formula of the GEMM epilogues); anything else goes to torch."""
     if not (x.is_cuda and x.dtype in (torch.float16, torch.bfloat16) and x.numel() % 8 == 0 and x.numel() > 0):
         return torch.nn.functional.gelu(x, approximate="tanh")
-    return _ext.host.gelu(x)
+    return _ext.call_layer(_ext.host.gelu, x)

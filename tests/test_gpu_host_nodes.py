@@ -95,3 +95,73 @@ def test_ragged_tokens_equal_padded_ones(dtype, tokens):
         assert torch.equal(F.linear(x, w, b), F.linear(full, w, b)[:tokens])
         assert torch.equal(F.linear(x, w), F.linear(full, w)[:tokens])
         assert torch.equal(F.linear(full[:tokens].unsqueeze(0), w, b)[0], F.linear(full, w, b)[:tokens])
+
+
+class _Call(torch.nn.Module):
+    """``fn(module, x)`` as a module: a trace takes the module's parameters for parameters, not for constants."""
+
+    def __init__(self, fn, module=None):
+        super().__init__()
+        self.fn, self.module = fn, module
+
+    def forward(self, t):
+        with torch.autocast("cuda", torch.float16):
+            return self.fn(self.module, t)
+
+
+def _traceable(name):
+    import sparse
+    from sparse import train_ops
+    if name in ("fst", "fst dense", "fp8"):
+        layer = sparse.SparseLinearTranspose(256, 128, bias=True).cuda()
+        if name == "fst dense":
+            layer.weight.weight_grad = "dense"
+        if name != "fp8":
+            return _Call(lambda m, t: m(t), layer)
+        w8 = sparse.fp8.Fp8SparseWeight(layer.weight, sparse.mask_select(layer.weight.detach())[1])
+        return _Call(lambda m, t: sparse.fp8.sparse_linear_transpose_fp8.apply(t, m.weight, w8, m.bias), layer)
+    if name == "sste":
+        layer = sparse.SoftThresholdLinear(256, 128, bias=True, device=DEV, spmm=True)
+        layer.init_scale()
+        return _Call(lambda m, t: m(t), layer)
+    if name == "gelu":
+        return _Call(lambda m, t: train_ops.gelu(t))
+    if name == "cross_entropy":
+        targets = torch.arange(128, device=DEV)
+        return _Call(lambda m, t: train_ops.cross_entropy(t, targets))
+    norm = train_ops.LayerNorm(256).cuda()
+    if name == "norm":
+        return _Call(lambda m, t: m(t), norm)
+    return _Call(lambda m, t: train_ops.add_layer_norm(t.float(), t, m)[1], norm)
+
+
+@pytest.mark.parametrize("name", NAMES + ["fst dense"])
+def test_traced_layers_replay(name):
+    """``torch.jit.trace`` records a layer as a call: other inputs give their own results and gradients, not what the trace's
+    output buffer happens to hold."""
+    import random
+    torch.manual_seed(6)
+    layer = _traceable(name)
+    first, second = (torch.randn(128, 256, device=DEV).half() for _ in range(2))
+    layer(first)                               # an FST layer compresses its weight before it is traced
+    traced = torch.jit.trace(layer, (first.clone().requires_grad_(True),), check_trace=False)
+    grads = []
+    for f in (layer, traced):
+        t = second.clone().requires_grad_(True)
+        layer.zero_grad(set_to_none=True)
+        random.seed(4)
+        y = f(t)
+        torch.manual_seed(7)
+        y.backward(torch.randn_like(y))
+        grads.append([y.detach(), t.grad] + [p.grad for p in layer.parameters()])
+    assert len(grads[0]) == len(grads[1])
+    for a, b in zip(*grads):
+        assert a.dtype == b.dtype and float((a.float() - b.float()).norm()) <= 1e-6 * float(a.float().norm())     # sums in any order
+
+
+def test_traced_embedding_replays():
+    from sparse import train_ops
+    wte, wpe = torch.randn(64, 32, device=DEV), torch.randn(16, 32, device=DEV)
+    first, second = (torch.randint(0, 64, (2, 16), device=DEV) for _ in range(2))
+    traced = torch.jit.trace(lambda t: train_ops.embed_tokens(t, wte, wpe), (first,), check_trace=False)
+    assert torch.equal(traced(second), train_ops.embed_tokens(second, wte, wpe))
