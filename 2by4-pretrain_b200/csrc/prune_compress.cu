@@ -774,9 +774,10 @@ extern "C" int sp24_prune_compress_with(const void *dense, int dense_dtype, int6
     if (!x || mode > SP24_PRUNE_MVUE_FAST) return SP24_ERR_ARG;
     if (x->offset_dev && (reinterpret_cast<uintptr_t>(x->offset_dev) & 7u)) return SP24_ERR_ARG;
     if (x->amax && packed_dtype != SP24_E4M3 && packed_dtype != SP24_E5M2) return SP24_ERR_DTYPE;
+    if (x->amax && x->out_scale != 0.f) return SP24_ERR_ARG;
     return prune_compress_impl(dense, dense_dtype, m, k, ld_dense, col_major, packed, packed_dtype, ld_packed, meta, mode, mask, ld_mask,
                                uniforms, ld_uniforms, seed, offset, x->offset_dev, x->e_tc, x->row_parts, stream, x->packed_row_major && col_major ? 1 : 0,
-                               1.f, 0, 1.f, x->amax, x->q_dense, x->ld_q, true);
+                               x->out_scale != 0.f ? x->out_scale : 1.f, 0, 1.f, x->amax, x->q_dense, x->ld_q, true);
 }
 
 // S-STE forward in one pass: magnitude 2:4 mask, soft threshold of the kept values (one rounding in the input type),

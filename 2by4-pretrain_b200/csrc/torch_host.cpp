@@ -116,6 +116,12 @@ OptTensor &rng_offset() {
     return t;
 }
 
+// That word for one conversion: only seeded MVUE draws read it.
+const uint64_t *rng_offset_ptr(int64_t mode) {
+    const bool draws = mode == SP24_PRUNE_MVUE || mode == SP24_PRUNE_MVUE_FAST;
+    return draws && rng_offset().has_value() ? static_cast<const uint64_t *>(rng_offset()->data_ptr()) : nullptr;
+}
+
 // What random.randint(0, 2**31 - 1) returns, from the same generator state: 32 random bits, drawn again until below 2^31.
 // Needs the GIL.
 uint64_t python_seed() {
@@ -270,15 +276,13 @@ OptTensor prune_into(const Tensor &dense_in, const Tensor &packed, const Tensor 
         ld_u = layout_of(*uniforms).ld;
     }
     TORCH_CHECK(meta.is_contiguous(), "metadata buffer must be contiguous");
-    const bool draws = mode == SP24_PRUNE_MVUE || mode == SP24_PRUNE_MVUE_FAST;
-    const void *dev_off = draws && !uniforms.has_value() && rng_offset().has_value() ? rng_offset()->data_ptr() : nullptr;
     // 16-bit results with whole 128-row blocks can also get their metadata in the order the GEMM reads, in the same pass.
     // Default: for column-major results (the dY^T operand of the weight-gradient GEMM, consumed at once).
     const bool want_tc = emit_tc.has_value() ? *emit_tc : lp.col == 1;
     if (!e_tc.has_value() && want_tc && packed.element_size() == 2 && m % 128 == 0)
         e_tc = empty({sp24_meta_tc_bytes(m, k)}, at::kByte, packed);
     sp24_prune_extras x{};
-    x.offset_dev = static_cast<const uint64_t *>(dev_off);
+    if (!uniforms.has_value()) x.offset_dev = rng_offset_ptr(mode);
     x.e_tc = const_cast<void *>(ptr(e_tc));
     x.row_parts = sums.parts;
     check(sp24_prune_compress_with(ptr(dense), dt(dense.scalar_type()), m, k, layout_of(dense).ld, lp.col, ptr(packed),
@@ -632,6 +636,7 @@ Q8 compress_q8(const Tensor &dense_in, int mode, const OptTensor &mask_in, const
     if (tb) o.tc = carve(buf, align256(vb) + align256(mb), at::kByte, {tb}, {1});
     sp24_prune_extras x{};
     x.amax = static_cast<const float *>(ptr(amax));
+    x.offset_dev = rng_offset_ptr(mode);
     x.packed_row_major = 1;
     if (tb) x.e_tc = ptr(o.tc);
     RowSums sums;

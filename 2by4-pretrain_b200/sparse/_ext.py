@@ -33,6 +33,12 @@ class DualDesc(ctypes.Structure):
                 ("meta_t", _vp), ("tc_w", _vp), ("tc_t", _vp)]
 
 
+class PruneExtras(ctypes.Structure):
+    """sp24_prune_extras"""
+    _fields_ = [("amax", ctypes.c_void_p), ("offset_dev", ctypes.c_void_p), ("e_tc", ctypes.c_void_p), ("row_parts", ctypes.c_void_p),
+                ("q_dense", ctypes.c_void_p), ("ld_q", ctypes.c_int64), ("packed_row_major", ctypes.c_int), ("out_scale", ctypes.c_float)]
+
+
 _SIGNATURES = {
     "sp24_prune_compress": [_vp, _i32, _i64, _i64, _i64, _i32, _vp, _i32, _i64, _vp, _i32, _vp, _i64, _vp, _i64,
                             _u64, _u64, _vp],
@@ -45,7 +51,8 @@ _SIGNATURES = {
                                    _vp, _i64, _vp],
     "sp24_pair_tile_columns": [_i64, _i64, _i32, _i32],
     "sp24_row_parts": [_i64, _i32],
-    "sp24_prune_compress_with": [_vp, _i32, _i64, _i64, _i64, _i32, _vp, _i32, _i64, _vp, _i32, _vp, _i64, _vp, _i64, _u64, _u64, _vp, _vp],
+    "sp24_prune_compress_with": [_vp, _i32, _i64, _i64, _i64, _i32, _vp, _i32, _i64, _vp, _i32, _vp, _i64, _vp, _i64, _u64, _u64,
+                                 ctypes.POINTER(PruneExtras), _vp],
     "sp24_sum_parts": [_vp, _i64, _i64, _vp, _i32, _vp],
     "sp24_spmm_f8": [_vp, _i32, _i64, _vp, _i64, _i64, _vp, _i64, _i64, _vp, _i32, _i32, _i64, _vp, _vp, _vp, _vp, _vp],
     "sp24_soft_threshold24_compress": [_vp, _i32, _i64, _i64, _i64, _i32, _vp, _i32, _i64, _vp, _i32, _f32, _vp, _vp],

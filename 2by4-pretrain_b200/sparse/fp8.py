@@ -21,7 +21,7 @@ from typing import Optional
 
 import torch
 
-from . import _ext
+from . import _ext, _semi_structured_conversions as _conversions
 from .spmm import sparse_linear as _spmm
 
 E4M3 = torch.float8_e4m3fn
@@ -67,9 +67,11 @@ def compress_q8(dense: torch.Tensor, *, mode: int, mask: Optional[torch.Tensor] 
         ld_m = _ext.layout_of(mask)[1]
     packed = torch.empty((m, k // 2), dtype=dtype, device=dense.device)
     meta = torch.empty((m, k // 32), dtype=torch.int32, device=dense.device)
-    rc = _ext.lib().sp24_prune_compress_q8(dense.data_ptr(), _ext.dt(dense.dtype), m, k, ld_d, col_major, packed.data_ptr(),
-                                           _ext.dt(dtype), k // 2, meta.data_ptr(), mode, _ext.ptr(mask), ld_m,
-                                           1.0 / float(scale), seed & (2 ** 64 - 1), offset & (2 ** 64 - 1), _ext.stream())
+    counter = _conversions._DEVICE_RNG_OFFSET if mode in (_ext.PRUNE_MVUE, _ext.PRUNE_MVUE_FAST) else None
+    extras = _ext.PruneExtras(offset_dev=_ext.ptr(counter), packed_row_major=1, out_scale=1.0 / float(scale))
+    rc = _ext.lib().sp24_prune_compress_with(dense.data_ptr(), _ext.dt(dense.dtype), m, k, ld_d, col_major, packed.data_ptr(),
+                                             _ext.dt(dtype), k // 2, meta.data_ptr(), mode, _ext.ptr(mask), ld_m, None, 0,
+                                             seed & (2 ** 64 - 1), offset & (2 ** 64 - 1), extras, _ext.stream())
     _ext.check(rc, "sp24_prune_compress_q8")
     return packed, meta
 

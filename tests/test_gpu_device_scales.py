@@ -151,3 +151,51 @@ def test_column_sums(dtype, rows, cols):
     _ext.check(lib.sp24_column_sums(x.data_ptr(), _ext.dt(dtype), rows, cols, cols, out.data_ptr(), _ext.stream()), "column_sums")
     want = 2.0 + x.double().sum(0)
     assert float((out.double() - want).abs().max()) <= (rows + 1) * 2 ** -24 * float(2 + x.double().abs().sum(0).max())
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_float8_draws_follow_the_device_counter(dtype):
+    """A step replayed from a graph keeps its seed; the installed counter moves the draws of the layer and of ``compress_q8``, and
+    a counter of c gives what an offset of c gives."""
+    import random
+    import sparse
+    from sparse import fp8, _ext
+    from sparse._semi_structured_conversions import set_device_rng_offset
+    tokens, in_f, out_f = 256, 256, 128
+    x, dy = _rand((tokens, in_f), dtype, 21).requires_grad_(True), _rand((tokens, out_f), dtype, 22, 1e-3)
+    w = torch.nn.Parameter(_rand((out_f, in_f), torch.float32, 23))
+    w8 = fp8.Fp8SparseWeight(w, sparse.mask_select(w.detach())[1])
+
+    def grad():
+        w.grad = x.grad = None
+        random.seed(9)
+        fp8.sparse_linear_transpose_fp8.apply(x, w, w8, None).backward(dy)
+        return w.grad
+
+    scale = fp8.scale_of(dy)
+    counter = torch.zeros(1, dtype=torch.int64, device=DEV)
+    plain = grad()
+    try:
+        set_device_rng_offset(counter)
+        at0 = grad()
+        side = torch.cuda.Stream()
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            grad()
+        torch.cuda.current_stream().wait_stream(side)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            held = grad()
+        replays = []
+        for c in (0, 3, 5):
+            counter.fill_(c)
+            graph.replay()
+            replays.append(held.clone())
+        counter.fill_(3)
+        eager3, q3 = grad(), fp8.compress_q8(dy.t(), mode=_ext.PRUNE_MVUE_FAST, scale=scale, seed=9)
+    finally:
+        set_device_rng_offset(None)
+    want3 = fp8.compress_q8(dy.t(), mode=_ext.PRUNE_MVUE_FAST, scale=scale, seed=9, offset=3)
+    assert torch.equal(at0, plain) and torch.equal(replays[0], plain) and torch.equal(replays[1], eager3)
+    assert torch.equal(q3[0].view(torch.uint8), want3[0].view(torch.uint8)) and torch.equal(q3[1], want3[1])
+    assert not torch.equal(replays[0], replays[1]) and not torch.equal(replays[1], replays[2])
