@@ -97,6 +97,10 @@ template <typename... T> void no_tangent(const T &...t) {
                                 "the layers of this package do not implement forward-mode automatic differentiation");
 }
 
+// Whether a backward pass is itself recorded (create_graph): what is linear in the incoming gradient through plain torch
+// operations then stays a function of it.
+bool recorded(const Tensor &grad) { return at::GradMode::is_enabled() && grad.requires_grad(); }
+
 int64_t align256(int64_t v) { return (v + 255) / 256 * 256; }
 
 // Word that a bounded wait of the GEMM kernels reports to, one per device.
@@ -479,8 +483,12 @@ std::pair<Tensor, Tensor> fst_weight_grads(const Tensor &g_in, const Tensor &x, 
         }
         seed = python_seed();
     }
-    NoAutograd guard;
     Tensor gw, gb;
+    if (need_b && recorded(g_in)) {
+        gb = g_in.sum({0}, false, at::kFloat);
+        need_b = false;
+    }
+    NoAutograd guard;
     if (need_w) {
         const Tensor g = g_in.contiguous();
         const int64_t tokens = g.size(0), out_f = g.size(1), in_f = x.size(1);
@@ -538,12 +546,14 @@ struct FstBackward : torch::autograd::Node {
         if (!g.defined()) return out;
         const Tensor x = x_.unpack(), pt = pt_.unpack(), tct = tct_.unpack();
         {
-            NoAutograd guard;
+            c10::optional<NoAutograd> guard;
+            if (!recorded(g)) guard.emplace();
             // the gradient of a plain sum arrives as one expanded value; the reference layer replaces it by ones
             if (g.dim() == 3 && g.stride(0) == 0 && g.stride(1) == 0 && g.stride(2) == 0) g = at::ones_like(g);
             if (g.dim() != 2) g = g.reshape({-1, g.size(-1)});
             if (g.scalar_type() != pt.scalar_type()) g = g.to(pt.scalar_type());
             if (task_should_compute_output(0)) {
+                if (!guard) guard.emplace();
                 Tensor dx = spmm(g, pt, tct, {}, 0, {}, false);
                 out[0] = dx.dim() == (int64_t)shape_.size() ? dx : dx.view(shape_);
             }
@@ -712,6 +722,10 @@ struct Fp8Backward : torch::autograd::Node {
             py::gil_scoped_acquire gil;
             seed = python_seed();
         }
+        if (need_b && recorded(grads[0])) {
+            out[2] = grads[0].reshape({-1, grads[0].size(-1)}).sum({0}, false, at::kFloat);
+            need_b = false;
+        }
         NoAutograd guard;
         const Tensor g = quantizable(grads[0].reshape({-1, grads[0].size(-1)}));
         const int64_t n = g.size(0), of = g.size(1);
@@ -807,14 +821,24 @@ struct SoftThresholdBackward : torch::autograd::Node {
         if (!grads[0].defined()) return out;
         TORCH_CHECK(!released_, torch::autograd::ERR_BACKWARD_TWICE);
         const Tensor x = x_.unpack(), packed = packed_.unpack(), meta = meta_.unpack();
+        const int64_t m = packed.size(0), k = 2 * packed.size(1);
+        Tensor w;
+        if (task_should_compute_output(0)) {
+            NoAutograd guard;
+            w = empty({m, k}, packed.scalar_type(), packed);
+            check(sp24_to_dense(ptr(packed), dt(w.scalar_type()), m, k, k / 2, ptr(meta), ptr(w), k, cur_stream()), "sp24_to_dense");
+        }
+        if (recorded(grads[0])) {
+            // all three are linear in dY; the products of 16-bit values are taken on float32 copies, exact operands either way
+            const Tensor g = grads[0].reshape({-1, grads[0].size(-1)}).to(packed.scalar_type());
+            if (w.defined()) out[0] = at::mm(g, w).view(shape_);
+            if (task_should_compute_output(1)) out[1] = w_f32_ ? at::mm(g.t().to(at::kFloat), x.to(at::kFloat)) : at::mm(g.t(), x);
+            if (has_bias_ && task_should_compute_output(2)) out[2] = g.sum({0}, false, at::kFloat);
+            return out;
+        }
         NoAutograd guard;
         const Tensor g = grads[0].reshape({-1, grads[0].size(-1)}).to(packed.scalar_type());
-        const int64_t m = packed.size(0), k = 2 * packed.size(1);
-        if (task_should_compute_output(0)) {
-            Tensor w = empty({m, k}, packed.scalar_type(), packed);
-            check(sp24_to_dense(ptr(packed), dt(w.scalar_type()), m, k, k / 2, ptr(meta), ptr(w), k, cur_stream()), "sp24_to_dense");
-            out[0] = at::mm(g, w).view(shape_);
-        }
+        if (w.defined()) out[0] = at::mm(g, w).view(shape_);
         if (task_should_compute_output(1)) out[1] = w_f32_ ? at::mm(g.t(), x, at::kFloat) : at::mm(g.t(), x);
         if (has_bias_ && task_should_compute_output(2)) {
             if (g.is_contiguous() && g.size(1) % 8 == 0 && aligned(g)) {

@@ -165,3 +165,40 @@ def test_traced_embedding_replays():
     first, second = (torch.randint(0, 64, (2, 16), device=DEV) for _ in range(2))
     traced = torch.jit.trace(lambda t: train_ops.embed_tokens(t, wte, wpe), (first,), check_trace=False)
     assert torch.equal(traced(second), train_ops.embed_tokens(second, wte, wpe))
+
+
+def _dense_of(name, layer):
+    """The weight that the layer's input gradient multiplies by, float64."""
+    return layer.get_sparse_weights().detach().half().double() if name == "sste" else None
+
+
+@pytest.mark.parametrize("name", ["sste", "fst", "fst dense", "fp8"])
+def test_gradients_stay_functions_of_the_incoming_one(name):
+    """Under ``create_graph`` whatever is a plain torch operation on dY keeps its graph (a gradient penalty differentiates it):
+    all three gradients of the S-STE layer, the bias sums of the others.  (The dense option's weight gradient has a graph too, but
+    torch's product with a float32 result has no derivative and says so.)"""
+    torch.manual_seed(8)
+    call = _traceable(name)
+    layer = call.module
+    x = torch.randn(128, 256, device=DEV).half().requires_grad_(True)
+    v = (torch.randn(128, 128, device=DEV) * 0.1).requires_grad_(True)
+    wanted = {"sste": [x, layer.weight, layer.bias], "fst dense": [layer.weight, layer.bias]}.get(name, [layer.bias])
+    y = call(x)
+    got = torch.autograd.grad(y, wanted, v.half(), create_graph=True)
+    assert all(g.requires_grad for g in got)
+    penalised = [(t, g) for t, g in zip(wanted, got) if name != "fst dense" or t is layer.bias]
+    plain = torch.autograd.grad(call(x), wanted, v.detach().half())
+    for a, b in zip(got, plain):
+        assert a.dtype == b.dtype and float((a - b).float().norm()) <= 1e-3 * float(b.float().norm())
+    # penalty = sum of squares of the gradients; its derivative in dY, in 64 bits
+    torch.autograd.backward(sum((g.float() ** 2).sum() for _, g in penalised))
+    v64, want = v.detach().half().double(), 0
+    for t, _ in penalised:
+        if t is x:
+            w = _dense_of(name, layer)
+            want = want + 2 * (v64 @ w) @ w.t()
+        elif t is layer.weight:
+            want = want + 2 * x.detach().double() @ (v64.t() @ x.detach().double()).t()
+        else:
+            want = want + 2 * v64.sum(0).expand_as(v64)
+    assert float((v.grad.double() - want).norm() / want.norm()) <= 4e-3       # fp16 roundings of the two products
