@@ -104,13 +104,29 @@ bool recorded(const Tensor &grad) { return at::GradMode::is_enabled() && grad.re
 int64_t align256(int64_t v) { return (v + 255) / 256 * 256; }
 
 // Word that a bounded wait of the GEMM kernels reports to, one per device.
+struct StatusWords {
+    std::vector<Tensor> words = std::vector<Tensor>(64);
+    std::mutex mu;
+};
+StatusWords &status_table() {
+    static auto &t = *new StatusWords();                  // never destroyed: the CUDA runtime may be gone at exit
+    return t;
+}
 Tensor &status_word(c10::DeviceIndex dev) {
-    static auto &words = *new std::vector<Tensor>(64);   // never destroyed: the CUDA runtime may be gone at exit
-    static std::mutex mu;
-    std::lock_guard<std::mutex> lock(mu);
-    Tensor &w = words.at(dev);
+    auto &t = status_table();
+    std::lock_guard<std::mutex> lock(t.mu);
+    Tensor &w = t.words.at(dev);
     if (!w.defined()) w = at::zeros({1}, at::TensorOptions().dtype(at::kInt).device(at::kCUDA, dev));
     return w;
+}
+// the words that exist, by device: those of every device that a GEMM ran on
+std::map<int, Tensor> status_words() {
+    auto &t = status_table();
+    std::lock_guard<std::mutex> lock(t.mu);
+    std::map<int, Tensor> out;
+    for (size_t i = 0; i < t.words.size(); ++i)
+        if (t.words[i].defined()) out[(int)i] = t.words[i];
+    return out;
 }
 int *status_ptr(const Tensor &t) { return static_cast<int *>(status_word(t.device().index()).data_ptr()); }
 
@@ -1249,5 +1265,6 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("gelu", &gelu, nogil());
     m.def("python_seed", &python_seed);
     m.def("set_rng_offset", [](const OptTensor &t) { rng_offset() = t; });
+    m.def("status_words", &status_words);
     m.def("status_word", [](int dev) { return status_word((c10::DeviceIndex)dev); });
 }

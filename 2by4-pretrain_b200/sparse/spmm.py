@@ -41,22 +41,20 @@ RETURN_TRANSPOSED_VIEW = False
 # made); tensors do not hash by value.  An in-place write to the metadata (copy_ on a checkpoint restore, a write
 # through another view of the same storage) bumps its version counter, and the copy is then rebuilt on the next use.
 _tc_meta_cache = {}
-_status = {}
 
 
 def _status_word(device):
     """The word the GEMM kernels of ``device`` report a bounded wait that gave up to."""
-    t = _status.get(device)
-    if t is None:
-        t = _status[device] = _ext.host.status_word(device.index if device.index is not None else torch.cuda.current_device())
-    return t
+    return _ext.host.status_word(device.index if device.index is not None else torch.cuda.current_device())
 
 
 def check_status(device=None):
-    """Synchronises and raises if a bounded on-device wait of the sparse GEMM ever gave up."""
-    if torch.cuda.is_available():
-        _status_word(torch.device("cuda", torch.cuda.current_device()))
-    for dev, t in _status.items():
+    """Synchronises and raises if a bounded on-device wait of the sparse GEMM ever gave up, on any device that ran one or on
+    ``device`` only."""
+    if "status_words" not in vars(_ext.host):       # the native module is not loaded: no GEMM has run
+        return
+    for index, t in _ext.host.status_words().items():
+        dev = torch.device("cuda", index)
         if device is None or dev == device:
             code = int(t.item())
             if code:

@@ -11,3 +11,22 @@ def test_native_seed_equals_randint_stream():
     random.seed(7)
     assert [_ext.host.python_seed() for _ in range(500)] == want
     assert random.getstate() == after
+
+
+def test_check_status_sees_every_device(monkeypatch):
+    """A wait that gave up is reported whichever device it ran on; asking for one device looks at that one only."""
+    from types import SimpleNamespace
+
+    import pytest
+    import torch
+    from sparse import _ext, spmm
+    words = {0: torch.zeros(1, dtype=torch.int32), 1: torch.tensor([2], dtype=torch.int32)}
+    monkeypatch.setattr(_ext, "host", SimpleNamespace(status_words=lambda: words, status_word=lambda i: words[i]))
+    spmm.check_status(torch.device("cuda", 0))
+    with pytest.raises(RuntimeError, match="role code 2.*cuda:1"):
+        spmm.check_status()
+    assert int(words[1]) == 0                  # reported once
+    spmm.check_status()
+    words[1].fill_(4)
+    with pytest.raises(RuntimeError, match="role code 4"):
+        spmm.check_status(device=torch.device("cuda", 1))
