@@ -631,8 +631,10 @@ Tensor absmax(const Tensor &x, const Tensor &mask = {}) {
           "sp24_absmax");
     return a;
 }
+// contiguous and on a 16-byte boundary (a view into a larger buffer may start anywhere)
 Tensor quantizable(const Tensor &t) {
-    return (t.scalar_type() == at::kFloat || is16(t.scalar_type()) ? t : t.to(at::kFloat)).contiguous();
+    const Tensor c = (t.scalar_type() == at::kFloat || is16(t.scalar_type()) ? t : t.to(at::kFloat)).contiguous();
+    return aligned(c) ? c : c.clone();
 }
 
 struct Q8 { Tensor packed, meta, tc; };

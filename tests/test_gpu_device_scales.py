@@ -199,3 +199,30 @@ def test_float8_draws_follow_the_device_counter(dtype):
     assert torch.equal(at0, plain) and torch.equal(replays[0], plain) and torch.equal(replays[1], eager3)
     assert torch.equal(q3[0].view(torch.uint8), want3[0].view(torch.uint8)) and torch.equal(q3[1], want3[1])
     assert not torch.equal(replays[0], replays[1]) and not torch.equal(replays[1], replays[2])
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("off", [1, 3])
+def test_float8_layer_takes_any_alignment(dtype, off):
+    """An input and a gradient that start off a 16-byte boundary give what their aligned copies give."""
+    import random
+    import sparse
+    from sparse import fp8
+    tokens, in_f, out_f = 256, 128, 256
+
+    def shifted(t):
+        v = torch.empty(t.numel() + off, dtype=t.dtype, device=DEV)[off:].view(t.shape)
+        return v.copy_(t)
+
+    w, b = (torch.nn.Parameter(_rand(s, torch.float32, 30)) for s in ((out_f, in_f), (out_f,)))
+    w8 = fp8.Fp8SparseWeight(w, sparse.mask_select(w.detach())[1])
+    x, dy = _rand((tokens, in_f), dtype, 31), _rand((tokens, out_f), dtype, 32, 1e-3)
+    res = []
+    for put in (torch.clone, shifted):
+        w.grad = b.grad = None
+        random.seed(3)
+        t = put(x).requires_grad_(True)
+        y = fp8.sparse_linear_transpose_fp8.apply(t, w, w8, b)
+        y.backward(put(dy))
+        res.append((y.detach(), t.grad, w.grad, b.grad))
+    assert put(x).data_ptr() % 16 and all(torch.equal(p, q) for p, q in zip(*res))
