@@ -475,7 +475,8 @@ __global__ void __launch_bounds__(256) quantize_f8_kernel(const T *x, int64_t ro
     if (threadIdx.x == 0) sc = f8_store_scale(*amax);
     __syncthreads();
     const float scale = sc;
-    const int64_t r0 = (int64_t)blockIdx.y * 128, c0 = (int64_t)blockIdx.x * 64;
+    const int64_t col_tiles = (cols + 63) / 64;       // one grid axis: the other two end at 65535 blocks
+    const int64_t r0 = blockIdx.x / col_tiles * 128, c0 = blockIdx.x % col_tiles * 64;
 #pragma unroll
     for (int p = 0; p < 4; ++p) {
         const int rr = p * 32 + (threadIdx.x >> 3), cc = (threadIdx.x & 7) * 8;
@@ -550,10 +551,11 @@ extern "C" int sp24_quantize_f8(const void *x, int dtype, int64_t rows, int64_t 
     if (rows <= 0 || cols <= 0 || cols % 8) return SP24_ERR_SHAPE;
     if (ld < cols || (ld * dtype_size(dtype)) % 16 || (q_t && ld_t < rows)) return SP24_ERR_STRIDE;
     if (!aligned16(x) || !aligned16(q) || !aligned16(q_t)) return SP24_ERR_ALIGN;
-    if ((rows + 127) / 128 > 65535) return SP24_ERR_TOO_LARGE;
+    const int64_t tiles = ((rows + 127) / 128) * ((cols + 63) / 64);
+    if (tiles > 0x7FFFFFFF) return SP24_ERR_TOO_LARGE;
     if (int rc = check_device()) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const dim3 grid((unsigned)((cols + 63) / 64), (unsigned)((rows + 127) / 128));
+    const unsigned grid = (unsigned)tiles;
     uint8_t *qb = static_cast<uint8_t *>(q), *tb = static_cast<uint8_t *>(q_t);
     if (dtype == SP24_F16) quantize_f8_kernel<__half><<<grid, 256, 0, st>>>(static_cast<const __half *>(x), rows, cols, ld, amax, qb, tb, ld_t);
     else if (dtype == SP24_BF16)

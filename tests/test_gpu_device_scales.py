@@ -226,3 +226,16 @@ def test_float8_layer_takes_any_alignment(dtype, off):
         y.backward(put(dy))
         res.append((y.detach(), t.grad, w.grad, b.grad))
     assert put(x).data_ptr() % 16 and all(torch.equal(p, q) for p, q in zip(*res))
+
+
+def test_quantize_takes_any_number_of_rows():
+    """More rows than 65535 tiles hold."""
+    from sparse import fp8
+    lib, _ext = _lib()
+    rows, cols = 65535 * 128 + 200, 8
+    x = _rand((rows, cols), torch.float16, 33)
+    q, q_t, a = torch.empty(rows, cols, dtype=E4M3, device=DEV), torch.empty(cols, rows, dtype=E4M3, device=DEV), _amax(x)
+    _ext.check(lib.sp24_quantize_f8(x.data_ptr(), _ext.dt(x.dtype), rows, cols, cols, a.data_ptr(), q.data_ptr(), q_t.data_ptr(), rows,
+                                    _ext.stream()), "quantize")
+    want = fp8.quantize(x)[0].view(torch.uint8)
+    assert torch.equal(q.view(torch.uint8), want) and torch.equal(q_t.view(torch.uint8), want.t().contiguous())
