@@ -451,9 +451,9 @@ std::vector<py::tuple> select_compress_many(const std::vector<Tensor> &weights, 
 // True when done; false when the tensors need what the Python wrapper does for other types, layouts and alignments.
 bool masked_add(const Tensor &grad, const Tensor &p, const Tensor &mask, double alpha) {
     if (!grad.is_cuda() || grad.layout() != at::kStrided || p.layout() != at::kStrided || mask.layout() != at::kStrided) return false;
-    if (grad.scalar_type() != at::kFloat || p.scalar_type() != at::kFloat || mask.element_size() > 4 || mask.scalar_type() == at::kInt ||
-        mask.scalar_type() == at::kShort)
-        return false;
+    const auto mt = mask.scalar_type();     // the types whose zero test is the kernel's: bytes, or floats with either sign of zero
+    const bool direct = mt == at::kBool || mt == at::kByte || mt == at::kChar || is16(mt) || mt == at::kFloat;
+    if (grad.scalar_type() != at::kFloat || p.scalar_type() != at::kFloat || !direct) return false;
     if (grad.sizes() != p.sizes() || grad.sizes() != mask.sizes() || grad.strides() != p.strides() || grad.strides() != mask.strides()) return false;
     if (!grad.is_non_overlapping_and_dense() || !aligned(grad) || !aligned(p) || !aligned(mask, 4 * mask.element_size())) return false;
     const auto cur = c10::cuda::current_device();

@@ -202,3 +202,22 @@ def test_gradients_stay_functions_of_the_incoming_one(name):
         else:
             want = want + 2 * v64.sum(0).expand_as(v64)
     assert float((v.grad.double() - want).norm() / want.norm()) <= 4e-3       # fp16 roundings of the two products
+
+
+@pytest.mark.parametrize("dtype", [torch.uint16, torch.uint32, torch.int16, torch.int32, torch.float8_e4m3fn, torch.float8_e5m2, torch.float16,
+                                   torch.bfloat16, torch.float32, torch.int8, torch.uint8])
+def test_masked_add_takes_a_mask_for_what_its_type_says(dtype):
+    """Zero is decided by the mask's type: -0.0 is zero in every floating type, the top bit alone is not in an integer."""
+    import sparse
+    n = 96
+    if dtype.is_floating_point:
+        m = torch.tensor([0.0, -0.0, 1.0, -2.0] * (n // 4), device=DEV).to(dtype)
+        zero = torch.tensor([True, True, False, False] * (n // 4), device=DEV)
+    else:
+        top = torch.iinfo(dtype).min or torch.iinfo(dtype).max // 2 + 1
+        m = torch.tensor([0, top, 1, 0] * (n // 4)).to(dtype).to(DEV)
+        zero = torch.tensor([True, False, False, True] * (n // 4), device=DEV)
+    g, p = torch.randn(n, device=DEV), torch.randn(n, device=DEV)
+    want = torch.where(zero, g + p * 0.5, g)
+    sparse.masked_add_(g, p, m, alpha=0.5)
+    assert torch.equal(g, want)
