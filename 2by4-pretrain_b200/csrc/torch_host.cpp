@@ -142,13 +142,17 @@ const uint64_t *rng_offset_ptr(int64_t mode) {
     return draws && rng_offset().has_value() ? static_cast<const uint64_t *>(rng_offset()->data_ptr()) : nullptr;
 }
 
+// Python objects that calls need, held from the module's load on (looked up in a function-local static they could make one
+// thread wait for the interpreter lock while another holds it and waits for the static).
+struct PyObjects {
+    PyObject *getrandbits = nullptr, *bits = nullptr, *weight_grad = nullptr, *dense_weight_grads = nullptr;
+} py_objects;
+
 // What random.randint(0, 2**31 - 1) returns, from the same generator state: 32 random bits, drawn again until below 2^31.
 // Needs the GIL.
 uint64_t python_seed() {
-    static PyObject *getrandbits = PyObject_GetAttrString(PyImport_ImportModule("random"), "getrandbits");
-    static PyObject *bits = PyLong_FromLong(32);
     for (;;) {
-        PyObject *r = PyObject_CallOneArg(getrandbits, bits);
+        PyObject *r = PyObject_CallOneArg(py_objects.getrandbits, py_objects.bits);
         if (!r) throw py::error_already_set();
         const unsigned long long v = PyLong_AsUnsignedLongLong(r);
         Py_DECREF(r);
@@ -469,9 +473,8 @@ bool accumulable(const Tensor &grad) { return grad.defined() && grad.scalar_type
 
 // The layer's option for an exact weight gradient is a Python attribute of the weight and its GEMM is torch's.
 bool wants_dense_weight_grad(const Tensor &weight) {
-    static PyObject *name = PyUnicode_InternFromString("weight_grad");
     py::object w = py::reinterpret_steal<py::object>(THPVariable_Wrap(weight));
-    PyObject *v = PyObject_GetAttr(w.ptr(), name);
+    PyObject *v = PyObject_GetAttr(w.ptr(), py_objects.weight_grad);
     if (!v) {
         PyErr_Clear();
         return false;
@@ -491,8 +494,8 @@ std::pair<Tensor, Tensor> fst_weight_grads(const Tensor &g_in, const Tensor &x, 
     if (need_w) {
         py::gil_scoped_acquire gil;
         if (wants_dense_weight_grad(weight)) {
-            static PyObject *fn = py::object(py::module_::import("sparse.sparse_ops").attr("_dense_weight_grads")).release().ptr();
-            py::object r = py::reinterpret_borrow<py::object>(fn)(g_in, x, weight, bias.defined() ? py::cast(bias) : py::object(py::none()),
+            TORCH_CHECK(py_objects.dense_weight_grads, "set_dense_weight_grads has not been called");
+            py::object r = py::reinterpret_borrow<py::object>(py_objects.dense_weight_grads)(g_in, x, weight, bias.defined() ? py::cast(bias) : py::object(py::none()),
                                                                   into_grad, need_w, need_b);
             py::tuple t(r);
             return {t[0].is_none() ? Tensor() : py::cast<Tensor>(t[0]), t[1].is_none() ? Tensor() : py::cast<Tensor>(t[1])};
@@ -1242,6 +1245,13 @@ Tensor gelu(const Tensor &input) {
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     using nogil = py::call_guard<py::gil_scoped_release>;
+    py_objects.getrandbits = py::object(py::module_::import("random").attr("getrandbits")).release().ptr();
+    py_objects.bits = PyLong_FromLong(32);
+    py_objects.weight_grad = PyUnicode_InternFromString("weight_grad");
+    m.def("set_dense_weight_grads", [](py::object fn) {
+        Py_XDECREF(py_objects.dense_weight_grads);
+        py_objects.dense_weight_grads = fn.release().ptr();
+    });
     m.def("sparse_linear", &sparse_linear, nogil());
     m.def("sparse_mm_accumulate", &sparse_mm_accumulate, nogil());
     m.def("prune_compress", &prune_compress, nogil());
