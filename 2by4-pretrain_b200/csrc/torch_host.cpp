@@ -83,6 +83,13 @@ Tensor carve(const Tensor &base, int64_t byte_off, at::ScalarType t, c10::IntArr
     return Tensor(std::move(impl));
 }
 
+// The same memory behind a version counter of its own.
+Tensor own_versions(const Tensor &t) {
+    Tensor v = carve(t, 0, t.scalar_type(), t.sizes(), t.strides());
+    if (!t.is_inference()) v.unsafeGetTensorImpl()->set_version_counter(c10::VariableVersion(0));
+    return v;
+}
+
 // (rows, last dimension) of a contiguous or reshapeable tensor; sees later in-place writes through its version counter
 Tensor rows2d(const Tensor &t) {
     if (t.dim() == 2) return t;
@@ -361,13 +368,16 @@ struct Copies {
         const bool tc = m % 128 == 0 && k % 128 == 0;
         const int64_t o_mw = vb, o_pt = align256(vb + mb), o_mt = o_pt + vb, o_tw = align256(o_mt + mb), o_tt = o_tw + mb;
         Tensor buf = empty({o_tw + (tc ? 2 * mb : 0)}, at::kByte, like);
+        // a version counter for W's tensors and one for W^T's: a write to one copy must not count as a write to the other, which
+        // a backward pass may hold
+        const Tensor buf_t = own_versions(buf);
         pw = carve(buf, 0, t, {m, k / 2}, {k / 2, 1});
         mw = carve(buf, o_mw, at::kShort, {m, k / 16}, {k / 16, 1});
-        pt = carve(buf, o_pt, t, {k, m / 2}, {1, k});
-        mt = carve(buf, o_mt, at::kShort, {k, m / 16}, {m / 16, 1});
+        pt = carve(buf_t, o_pt, t, {k, m / 2}, {1, k});
+        mt = carve(buf_t, o_mt, at::kShort, {k, m / 16}, {m / 16, 1});
         if (tc) {
             tcw = carve(buf, o_tw, at::kByte, {mb}, {1});
-            tct = carve(buf, o_tt, at::kByte, {mb}, {1});
+            tct = carve(buf_t, o_tt, at::kByte, {mb}, {1});
         }
     }
 };

@@ -221,3 +221,21 @@ def test_masked_add_takes_a_mask_for_what_its_type_says(dtype):
     want = torch.where(zero, g + p * 0.5, g)
     sparse.masked_add_(g, p, m, alpha=0.5)
     assert torch.equal(g, want)
+
+
+def test_copies_of_w_and_of_its_transpose_are_written_apart():
+    """The copies live in one allocation; a write to W's between the passes is no write to W^T's, which the backward pass holds."""
+    import sparse
+    x, _ = _layers()
+    layer = sparse.SparseLinearTranspose(256, 128, bias=False).cuda()
+    t = x.clone().requires_grad_(True)
+    with torch.autocast("cuda", torch.float16):
+        y = layer(t)
+    y.backward(torch.ones_like(y), retain_graph=True)
+    want, before = t.grad.clone(), layer.weight.compressed[3]._version
+    t.grad = None
+    layer.weight.compressed[0].mul_(2)
+    layer.weight.compressed[1].add_(0)
+    assert layer.weight.compressed[3]._version == before
+    y.backward(torch.ones_like(y))
+    assert torch.equal(t.grad, want)
