@@ -239,3 +239,30 @@ def test_copies_of_w_and_of_its_transpose_are_written_apart():
     assert layer.weight.compressed[3]._version == before
     y.backward(torch.ones_like(y))
     assert torch.equal(t.grad, want)
+
+
+@pytest.mark.parametrize("dtype", [torch.int8, torch.float8_e4m3fn])
+@pytest.mark.parametrize("tokens", [1, 7, 17, 129, 255])
+def test_ragged_tokens_of_8_bit_operands(dtype, tokens):
+    """The unpadded route with 8-bit operands: each row has the bits it has among rows padded to a multiple of 32."""
+    import sparse
+    g = torch.Generator(device=DEV).manual_seed(tokens)
+    dense = torch.randint(-9, 9, (256, 512), device=DEV, generator=g).to(torch.int8 if dtype == torch.int8 else torch.float32)
+    if dtype == torch.int8:
+        w = sparse.to_sparse_semi_structured(dense, dtype=dtype)
+    else:
+        w = sparse.to_sparse_semi_structured(dense.half(), dtype=dtype)
+    full = torch.randint(-9, 9, ((tokens + 31) // 32 * 32, 512), device=DEV, generator=g).to(dtype)
+    x = full[:tokens].clone()
+    with torch.inference_mode():
+        want = F.linear(full, w)[:tokens]
+        assert torch.equal(F.linear(x, w), want)
+        assert torch.equal(F.linear(x.unsqueeze(0), w)[0], want)
+    ref = x.double() @ _kept(w, dense).double().t()
+    assert torch.equal(want.double(), ref)             # integers of at most 9 * 9 * 512: exact in float32 and int32
+
+
+def _kept(w, dense):
+    from sparse import spmm
+    eye = torch.eye(dense.shape[1], device=DEV).to(w.sparse_tensor_cutlass.dtype)
+    return spmm.sparse_linear(eye, w.sparse_tensor_cutlass, w.meta_tensor_cutlass).t()
