@@ -74,20 +74,14 @@ Tensor as_layout(const Tensor &t, int col) {
 }
 
 // A view into `base`'s memory with its own type, shape and strides, sharing its version counter (a write through either
-// is seen by both); byte_off is counted from base's first element.
-Tensor carve(const Tensor &base, int64_t byte_off, at::ScalarType t, c10::IntArrayRef shape, c10::IntArrayRef strides) {
+// is seen by both) unless given one; byte_off is counted from base's first element.
+Tensor carve(const Tensor &base, int64_t byte_off, at::ScalarType t, c10::IntArrayRef shape, c10::IntArrayRef strides,
+             const c10::VariableVersion *version = nullptr) {
     auto impl = c10::make_intrusive<c10::TensorImpl>(c10::Storage(base.storage()), base.key_set(), at::scalarTypeToTypeMeta(t));
     impl->set_storage_offset(((int64_t)base.storage_offset() * base.element_size() + byte_off) / (int64_t)c10::elementSize(t));
     impl->set_sizes_and_strides(shape, strides);
-    if (!base.is_inference()) impl->set_version_counter(base.unsafeGetTensorImpl()->version_counter());
+    if (!base.is_inference()) impl->set_version_counter(version ? *version : base.unsafeGetTensorImpl()->version_counter());
     return Tensor(std::move(impl));
-}
-
-// The same memory behind a version counter of its own.
-Tensor own_versions(const Tensor &t) {
-    Tensor v = carve(t, 0, t.scalar_type(), t.sizes(), t.strides());
-    if (!t.is_inference()) v.unsafeGetTensorImpl()->set_version_counter(c10::VariableVersion(0));
-    return v;
 }
 
 // (rows, last dimension) of a contiguous or reshapeable tensor; sees later in-place writes through its version counter
@@ -370,14 +364,14 @@ struct Copies {
         Tensor buf = empty({o_tw + (tc ? 2 * mb : 0)}, at::kByte, like);
         // a version counter for W's tensors and one for W^T's: a write to one copy must not count as a write to the other, which
         // a backward pass may hold
-        const Tensor buf_t = own_versions(buf);
+        const c10::VariableVersion of_t(0);
         pw = carve(buf, 0, t, {m, k / 2}, {k / 2, 1});
         mw = carve(buf, o_mw, at::kShort, {m, k / 16}, {k / 16, 1});
-        pt = carve(buf_t, o_pt, t, {k, m / 2}, {1, k});
-        mt = carve(buf_t, o_mt, at::kShort, {k, m / 16}, {m / 16, 1});
+        pt = carve(buf, o_pt, t, {k, m / 2}, {1, k}, &of_t);
+        mt = carve(buf, o_mt, at::kShort, {k, m / 16}, {m / 16, 1}, &of_t);
         if (tc) {
             tcw = carve(buf, o_tw, at::kByte, {mb}, {1});
-            tct = carve(buf_t, o_tt, at::kByte, {mb}, {1});
+            tct = carve(buf, o_tt, at::kByte, {mb}, {1}, &of_t);
         }
     }
 };
