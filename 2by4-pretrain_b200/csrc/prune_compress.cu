@@ -389,7 +389,8 @@ template <typename TIn> struct ColVec {
 
 // resident blocks per SM the register budget is set for
 constexpr int col_min_blocks(int mode, int out_bytes) {
-    // 8-bit outputs hold a row-major strip of packed bytes as well: 128 registers, no spills, instead of 85 with 500 bytes
+    // 8-bit outputs hold a row-major strip of packed bytes as well: 128 registers with 28 - 36 bytes of spills (16-bit input; none
+    // for float32) instead of 85 with 500
     return mode == SP24_PRUNE_MVUE_FAST ? (out_bytes == 1 ? 2 : 3) : (mode == SP24_PRUNE_MVUE ? 4 : 1);
 }
 

@@ -96,7 +96,7 @@ int sp24_ipc_close(void *ptr);
  *              group index gi = r*(k/4)+g, counter = (gi>>1, offset), key = seed, even groups take
  *              words 0,1 and odd groups words 2,3, u = (word >> 8) * 2^-24.
  *              SP24_PRUNE_MVUE_FAST takes no uniforms and draws the same way from Philox4x32-7; its arithmetic
- *              replaces the ten IEEE divisions per group by seven reciprocal approximations (the reference's
+ *              replaces the ten IEEE divisions per group by eight reciprocal approximations (the reference's
  *              own GPU kernel also divides approximately), so kept positions and stored values can differ from
  *              SP24_PRUNE_MVUE's in the last float32 bits; it is the mode the training layer uses.
  * Shape rules (sparse/semi_structured.py:24-30,188-200): m % 32 == 0; k % 64 == 0 (16-bit) or
@@ -117,7 +117,8 @@ int sp24_prune_compress(const void *dense, int dense_dtype, int64_t m, int64_t k
  *   e_tc        a second copy of the metadata in the order sp24_spmm reads (sp24_meta_tc_bytes(m, k) bytes, 16-byte
  *               aligned), which saves the sp24_meta_to_tc launch.  16-bit packed types and m % 128 == 0 only.
  *   row_sums    m floats: row_sums[r] += sum over k of dense[r, k] (values before pruning; fp32 partial sums added
- *               with atomics, so zero the array first or pass a gradient buffer to add to).  Column-major storage
+ *               with atomics in no fixed order, so zero the array first or pass a gradient buffer to add to;
+ *               sp24_prune_compress_with has a form that repeats bit for bit).  Column-major storage
  *               only.  For dY^T these are the bias gradients of the layer (grad_output.sum(0), README.md:197-198 of
  *               the reference), taken from the pass that reads dY anyway.
  */
@@ -498,7 +499,8 @@ int sp24_cross_entropy_fused(const void *logits, int dtype, const int64_t *targe
                              void *dlogits, int64_t rows, int64_t v, int64_t ld, int64_t ld_out, void *stream);
 int sp24_scale_unless_one(void *g, int dtype, const float *factor, int64_t count, void *stream);
 
-/* out[c] += sum over rows of x (rows, cols; 16-bit, pitch ld, cols % 8 == 0), float32: the bias gradient of a dense layer. */
+/* out[c] += sum over rows of x (rows, cols; 16-bit, pitch ld, cols % 8 == 0), float32, in a fixed order: the bias gradient of a
+ * dense layer. */
 int sp24_column_sums(const void *x, int dtype, int64_t rows, int64_t cols, int64_t ld, float *out, void *stream);
 
 /*
