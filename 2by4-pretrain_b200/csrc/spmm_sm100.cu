@@ -152,6 +152,17 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
         : "r"(taddr)
         : "memory");
 }
+// shared memory -> global through a tensor map, one element-wise float32 add per element in L2; parts of the box past the tensor are left out
+__device__ __forceinline__ void tma_reduce_add_2d(const CUtensorMap *map, int x, int y, uint32_t src) {
+    asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%1, %2}], [%3];" ::"l"(map), "r"(x), "r"(y), "r"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+// all but the newest N groups of this thread have read their shared memory
+template <int N> __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory"); }
+__device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
 // fp32 vector reduction into global memory (sm_90+), address 16-byte aligned
 __device__ __forceinline__ void red_add_v4(float *addr, float a, float b, float c, float d) {
     asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
@@ -1104,14 +1115,26 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 // Tiles of 256 sparse rows x 256 dense columns per CTA pair (M = 256, N = 256 per instruction); a CTA stages its 128
 // rows of A (16 KB), its 128 columns of B as two 64-column boxes of 128 K-rows (32 KB) and 2 KB of metadata per K
 // step of 128: 50 KB for 8.4 dense-equivalent MFLOP, four stages.  K is cut into slices (work unit = tile x slice)
-// so that the units fill the pairs; every unit adds its partial product with fp32 vector reductions.  One
+// so that the units fill the pairs; every unit adds its partial product with fp32 reductions in L2.  One
 // accumulator of 256 columns per CTA: a pair that owns more than one unit drains it before the next unit's MMAs.
+//
+// Epilogue: tensor memory -> shared memory -> TMA reductions of 16 rows x 32 columns.  Its cost is exposed (nothing is left to
+// multiply): 128 KB a CTA take about 2 us at the 32 bytes a clock that an SM writes.  red.global.add.v4 from the registers, 32
+// rows of 16 bytes an instruction, took 4 us even for one tile (64-byte rows: 0.6 us more than 128-byte ones); before -> now:
+// ms 512, n 256, k 256 9.5 -> 8.2 us; ms 3072, n 768, k 8192 / 16384 25.1 -> 22.1 / 40.7 -> 38.3 us; ms 768, n 768, k 8192 15.0 -> 11.9 us.
+// Where every pair has one unit at most (any output up to 74 tiles) the operand ring is idle by then and holds the whole tile,
+// so that no chunk waits for another; a pair with more units stages chunk by chunk beside its ring, which is filling again.
 namespace two {
 constexpr int BN3 = 256;
 constexpr int B3_BYTES = (BN3 / 2) * 256;                  // 128 columns x 128 K-rows x 2 bytes
 constexpr int STAGE3_BYTES = A_STAGE_BYTES + B3_BYTES + 2048;   // 51200
 constexpr int STAGES3 = 4;
-constexpr int SMEM3 = STAGES3 * STAGE3_BYTES + 1024;
+// Epilogue staging: a box is 16 rows x 32 columns, 128-byte rows in the 128-byte swizzle of the output's tensor map; a chunk is
+// the two boxes of a warp's 32 rows.
+constexpr int BOX3_BYTES = 16 * 128, CHUNKS3 = BN3 / 2 / 32;
+constexpr int STAGING3 = 8 * BOX3_BYTES;                    // one box per epilogue warp
+constexpr int SMEM3 = STAGES3 * STAGE3_BYTES + STAGING3 + 1024;
+static_assert(8 * CHUNKS3 * 2 * BOX3_BYTES <= STAGES3 * STAGE3_BYTES, "an idle operand ring holds a whole tile");
 static_assert(STAGE3_BYTES % 1024 == 0, "stages must keep the 1024-byte swizzle alignment");
 static_assert(SMEM3 <= 227 * 1024, "shared memory budget");
 }  // namespace two
@@ -1119,7 +1142,7 @@ static_assert(SMEM3 <= 227 * 1024, "shared memory budget");
 template <bool A_MN>
 __global__ void __launch_bounds__(320, 1)
 spmm_pair_acc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                     const __grid_constant__ CUtensorMap map_e, SpmmParams P) {
+                     const __grid_constant__ CUtensorMap map_e, const __grid_constant__ CUtensorMap map_d, SpmmParams P) {
     using namespace two;
     constexpr int BN = BN3;
     constexpr int STAGES = STAGES3;
@@ -1251,33 +1274,54 @@ spmm_pair_acc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         // ---------------------------------------------------------------- epilogue (warps 2..9 of both CTAs)
         const int quad = warp & 3, half = (warp - 2) >> 2;
         constexpr int HC = BN / 2;                     // 128 columns per warp
-        float *out = static_cast<float *>(P.out);
         const uint32_t empty_leader = map_to_cta(tmem_empty, 0);
+        const bool idle_ring = n_units <= n_pairs;     // this pair's only unit: the operand ring is free when it is complete
+        const uint32_t stg = smem_u32(smem) + (idle_ring ? (warp - 2) * CHUNKS3 * 2 * BOX3_BYTES
+                                                         : STAGES3 * STAGE3_BYTES + (warp - 2) * BOX3_BYTES);
         int tl = 0;
         for (int unit = pair; unit < n_units; unit += n_pairs, ++tl) {
             const int tile = unit % n_tiles;
-            const int mrow = ((tile % n_tiles_m) * 2 + (int)rank) * BM + quad * 32 + lane;
-            const int64_t col0 = (int64_t)(tile / n_tiles_m) * BN + half * HC;
+            const int mrow = ((tile % n_tiles_m) * 2 + (int)rank) * BM + quad * 32;
+            const int col0 = (tile / n_tiles_m) * BN + half * HC;
             const bool ok = mbar_wait(tmem_full, tl & 1, &abort_flag, P.status, 3);
             tc_fence_after();
-            const bool run = ok && !abort_flag;
+            const bool run = __all_sync(0xFFFFFFFFu, ok && !abort_flag);
             if (run) {
                 const uint32_t acc = tmem_base + ((uint32_t)(quad * 32) << 16) + half * HC;
-                float *row = out + (int64_t)mrow * P.ld_out + col0;
 #pragma unroll 1
-                for (int c = 0; c < HC / 32; ++c) {
+                for (int c = 0; c < CHUNKS3; ++c) {
                     uint32_t v[32];
                     tmem_ld32(acc + c * 32, v);
                     tmem_ld_wait();
-                    const int64_t nb = col0 + c * 32;
-                    if (nb + 32 <= P.n) {
+                    const int x = col0 + c * 32;
+                    // a lane's row of 128 bytes at `row`, its eight 16-byte pieces in the map's 128-byte swizzle
+                    auto put = [&](uint32_t row) {
 #pragma unroll
                         for (int q = 0; q < 8; ++q)
-                            red_add_v4(row + c * 32 + q * 4, __uint_as_float(v[q * 4]), __uint_as_float(v[q * 4 + 1]),
-                                       __uint_as_float(v[q * 4 + 2]), __uint_as_float(v[q * 4 + 3]));
+                            st_shared_v4(row + ((q ^ (lane & 7)) << 4), v[q * 4], v[q * 4 + 1], v[q * 4 + 2], v[q * 4 + 3]);
+                        fence_proxy_async();
+                    };
+                    if (idle_ring) {
+                        const uint32_t buf = stg + c * 2 * BOX3_BYTES;
+                        put(buf + lane * 128);
+                        __syncwarp();
+                        if (lane == 0 && x < P.n) {
+                            tma_reduce_add_2d(&map_d, x, mrow, buf);
+                            tma_reduce_add_2d(&map_d, x, mrow + 16, buf + BOX3_BYTES);
+                            bulk_commit();
+                        }
                     } else {
-                        for (int i = 0; i < 32; ++i)
-                            if (nb + i < P.n) atomicAdd(row + c * 32 + i, __uint_as_float(v[i]));
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            if (lane == 0) bulk_wait_read<0>();      // the box before has left
+                            __syncwarp();
+                            if ((lane >> 4) == h) put(stg + (lane & 15) * 128);
+                            __syncwarp();
+                            if (lane == 0 && x < P.n) {
+                                tma_reduce_add_2d(&map_d, x, mrow + 16 * h, stg);
+                                bulk_commit();
+                            }
+                        }
                     }
                 }
             }
@@ -1285,6 +1329,7 @@ spmm_pair_acc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(empty_leader);
         }
+        if (lane == 0) bulk_wait_read<0>();            // shared memory stays until it has been read
         tc_fence_before();
     }
     __syncthreads();
@@ -1351,29 +1396,34 @@ EncodeTiledFn encode_tiled_fn() {
     return fn;
 }
 
-// 2-D tensor map over a row-major (rows, cols) array with leading dimension ld (elements), 128-byte swizzle.
-int make_map(CUtensorMap *map, const void *base, int dt, int64_t rows, int64_t cols, int64_t ld, uint32_t box_cols,
-             uint32_t box_rows) {
+// 2-D tensor map over rows of `cols` elements, row_bytes apart.
+int encode_map(CUtensorMap *map, CUtensorMapDataType type, const void *base, int64_t cols, int64_t rows, int64_t row_bytes, uint32_t box_cols,
+               uint32_t box_rows, CUtensorMapSwizzle swizzle) {
     const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)ld * dtype_size(dt)};
+    const cuuint64_t strides[1] = {(cuuint64_t)row_bytes};
     const cuuint32_t box[2] = {box_cols, box_rows};
     const cuuint32_t estr[2] = {1, 1};
     EncodeTiledFn encode = encode_tiled_fn();
     if (!encode) return SP24_ERR_CUDA;
-    CUresult r = encode(map, tmap_dtype(dt), 2, const_cast<void *>(base), dims, strides, box, estr,
-                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r == CUDA_ERROR_INVALID_CONTEXT) {
+    CUresult r = CUDA_SUCCESS;
+    for (int attempt = 0; attempt < 2; ++attempt) {
+        r = encode(map, type, 2, const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (r != CUDA_ERROR_INVALID_CONTEXT) break;
         // a host thread that has made no runtime call yet (an autograd worker) has no current context for this
         // driver entry point: let the runtime bind the primary context, then encode again
         cudaFree(nullptr);
-        r = encode(map, tmap_dtype(dt), 2, const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     }
     if (r != CUDA_SUCCESS && getenv("SP24_DEBUG"))
-        fprintf(stderr, "sparse24_b200: cuTensorMapEncodeTiled failed (%d): base %p rows %lld cols %lld ld %lld box %u x %u\n",
-                (int)r, base, (long long)rows, (long long)cols, (long long)ld, box_cols, box_rows);
+        fprintf(stderr, "sparse24_b200: cuTensorMapEncodeTiled failed (%d): base %p rows %lld cols %lld pitch %lld box %u x %u\n",
+                (int)r, base, (long long)rows, (long long)cols, (long long)row_bytes, box_cols, box_rows);
     return r == CUDA_SUCCESS ? SP24_OK : SP24_ERR_CUDA;
+}
+
+// Operand (rows, cols) with leading dimension ld (elements), 128-byte swizzle.
+int make_map(CUtensorMap *map, const void *base, int dt, int64_t rows, int64_t cols, int64_t ld, uint32_t box_cols,
+             uint32_t box_rows) {
+    return encode_map(map, tmap_dtype(dt), base, cols, rows, ld * dtype_size(dt), box_cols, box_rows, CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
 // SP24_SPMM_PAIR=0 in the environment keeps every GEMM on the single-CTA kernels (read once per process)
@@ -1410,22 +1460,7 @@ int launch_spmm(const CUtensorMap &ma, const CUtensorMap &mb, SpmmParams P, cuda
 
 // Metadata atoms as a 2-D tensor for TMA: rows of 1024 bytes (256 int32), two rows per 2048-byte atom, no swizzle.
 int make_map_e(CUtensorMap *map, const void *e_tc, int64_t n_atoms, int atoms_per_box = 1) {
-    const cuuint64_t dims[2] = {256, (cuuint64_t)(2 * n_atoms)};
-    const cuuint64_t strides[1] = {1024};
-    const cuuint32_t box[2] = {256, (cuuint32_t)(2 * atoms_per_box)};
-    const cuuint32_t estr[2] = {1, 1};
-    EncodeTiledFn encode = encode_tiled_fn();
-    if (!encode) return SP24_ERR_CUDA;
-    CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_INT32, 2, const_cast<void *>(e_tc), dims, strides, box, estr,
-                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r == CUDA_ERROR_INVALID_CONTEXT) {
-        cudaFree(nullptr);   // see make_map
-        r = encode(map, CU_TENSOR_MAP_DATA_TYPE_INT32, 2, const_cast<void *>(e_tc), dims, strides, box, estr,
-                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    }
-    return r == CUDA_SUCCESS ? SP24_OK : SP24_ERR_CUDA;
+    return encode_map(map, CU_TENSOR_MAP_DATA_TYPE_INT32, e_tc, 256, 2 * n_atoms, 1024, 256, 2 * atoms_per_box, CU_TENSOR_MAP_SWIZZLE_NONE);
 }
 
 template <bool A_MN, typename OutT, int EPI = EPI_PLAIN, bool F8 = false>
@@ -1463,8 +1498,8 @@ int launch_spmm_pair(const CUtensorMap &ma, const CUtensorMap &mb, const CUtenso
 }
 
 template <bool A_MN>
-int launch_spmm_pair_acc(const CUtensorMap &ma, const CUtensorMap &mb, const CUtensorMap &me, SpmmParams P, int k_splits,
-                         cudaStream_t st) {
+int launch_spmm_pair_acc(const CUtensorMap &ma, const CUtensorMap &mb, const CUtensorMap &me, const CUtensorMap &md, SpmmParams P,
+                         int k_splits, cudaStream_t st) {
     auto kern = spmm_pair_acc_kernel<A_MN>;
     static bool attr_set[64];
     int dev = 0;
@@ -1497,7 +1532,7 @@ int launch_spmm_pair_acc(const CUtensorMap &ma, const CUtensorMap &mb, const CUt
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if (cudaLaunchKernelEx(&cfg, kern, ma, mb, me, P) != cudaSuccess) return launch_status();
+    if (cudaLaunchKernelEx(&cfg, kern, ma, mb, me, md, P) != cudaSuccess) return launch_status();
     return launch_status();
 }
 
@@ -1928,8 +1963,11 @@ extern "C" int sp24_spmm_accumulate_f32(const void *a_packed, int dtype, int a_m
         CUtensorMap map_e;
         rc = make_map_e(&map_e, e_tc, (ms / 128) * P.k_atoms);
         if (rc) return rc;
-        return a_mn_major ? launch_spmm_pair_acc<true>(map_a, map_b, map_e, P, k_splits, st)
-                          : launch_spmm_pair_acc<false>(map_a, map_b, map_e, P, k_splits, st);
+        CUtensorMap map_d;
+        rc = encode_map(&map_d, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, out, n, ms, ld_out * 4, 32, 16, CU_TENSOR_MAP_SWIZZLE_128B);
+        if (rc) return rc;
+        return a_mn_major ? launch_spmm_pair_acc<true>(map_a, map_b, map_e, map_d, P, k_splits, st)
+                          : launch_spmm_pair_acc<false>(map_a, map_b, map_e, map_d, P, k_splits, st);
     }
     // widest tile (least operand traffic per output), then as many K slices as idle SMs allow
     const int sms = sm_count_cached();
