@@ -163,6 +163,24 @@ template <int N> __device__ __forceinline__ void bulk_wait_read() { asm volatile
 __device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
     asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
+// 16 lanes (the lower or upper half of the warp's quadrant) x 16 columns: register 4 c + 2 h + e of lane L holds row 8 h + L / 4,
+// column 8 c + 2 (L % 4) + e
+__device__ __forceinline__ void tmem_ld_16x256b_x2(uint32_t taddr, uint32_t (&v)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                 : "r"(taddr)
+                 : "memory");
+}
+// four 8 x 8 matrices of 16-bit values, each written transposed; lane 8 i + j gives the address of row j of matrix i as stored
+__device__ __forceinline__ void stmatrix_x4_trans(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared::cta.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d)
+                 : "memory");
+}
+__device__ __forceinline__ uint4 ld_shared_v4(uint32_t addr) {
+    uint4 v;
+    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+    return v;
+}
 // fp32 vector reduction into global memory (sm_90+), address 16-byte aligned
 __device__ __forceinline__ void red_add_v4(float *addr, float a, float b, float c, float d) {
     asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
@@ -779,11 +797,21 @@ constexpr int MAX_STAGES2 = 6;
 // BN / 2 rows of B as two 128-byte K atoms; every part is a multiple of the 1024-byte swizzle period.
 constexpr int e2_bytes(bool f8) { return f8 ? 4096 : 2048; }
 constexpr int stage2_bytes(bool f8, int bn) { return A_STAGE_BYTES + e2_bytes(f8) + bn * 128; }
+// Output staging of the plain epilogue: a chunk is 16 tokens x 32 features of 16 bits, two per epilogue warp.
+constexpr int MAX_CHUNKS2 = (BN2_MAX / 16 + 1) / 2;         // of a tile and a warp
+constexpr int CHUNK2_BYTES = 16 * 64, STAGING2 = 8 * 2 * CHUNK2_BYTES;
+// barriers and flags behind the staging, so that no static shared memory shifts the (1024-byte aligned) start of the stages
+struct Ctl2 {
+    uint64_t bars[2 * MAX_STAGES2 + 4];
+    uint32_t tmem_base;
+    int abort_flag;
+};
+constexpr int SMEM_LIMIT = 227 * 1024;
 constexpr int stages2(bool f8, int bn) {
-    const int n = (227 * 1024 - 2048) / stage2_bytes(f8, bn);     // alignment slack and the static shared memory aside
+    const int n = (SMEM_LIMIT - STAGING2 - (int)sizeof(Ctl2)) / stage2_bytes(f8, bn);
     return n < MAX_STAGES2 ? n : MAX_STAGES2;
 }
-constexpr int smem2(bool f8, int bn) { return stages2(f8, bn) * stage2_bytes(f8, bn) + 1024; }
+constexpr int smem2(bool f8, int bn) { return stages2(f8, bn) * stage2_bytes(f8, bn) + STAGING2 + (int)sizeof(Ctl2); }
 static_assert(stage2_bytes(false, 16) % 1024 == 0 && stage2_bytes(true, 16) % 1024 == 0, "stages must keep the 1024-byte swizzle alignment");
 static_assert(stages2(true, BN2_MAX) >= 4, "shared memory budget");
 }  // namespace two
@@ -866,10 +894,14 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     static_assert(BN2_MAX <= E_COL && E_COL + 2 * E_SLOT <= ACC_COL && ACC_COL + BN2_MAX <= 512, "tensor memory columns exhausted");
 
     extern __shared__ __align__(1024) uint8_t smem_raw[];
-    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    __shared__ __align__(8) uint64_t bars[2 * MAX_STAGES2 + 4];
-    __shared__ uint32_t tmem_base_smem;
-    __shared__ int abort_flag;
+    uint8_t *smem = smem_raw;
+    if (smem_u32(smem) & 1023) {              // the same in every CTA; not seen, but the swizzled stages depend on it
+        if (threadIdx.x == 0 && P.status) atomicCAS(P.status, 0, 11);
+        return;
+    }
+    Ctl2 &ctl = *reinterpret_cast<Ctl2 *>(smem + STAGES * STAGE2_BYTES + STAGING2);
+    uint64_t *const bars = ctl.bars;
+    volatile int &abort_flag = ctl.abort_flag;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();          // 0 = leader
@@ -895,14 +927,14 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         fence_barrier_init();
     }
     if (warp == 1) {
-        tmem_alloc_pair(smem_u32(&tmem_base_smem), TMEM_COLS);
+        tmem_alloc_pair(smem_u32(&ctl.tmem_base), TMEM_COLS);
         tmem_relinquish_pair();
     }
     tc_fence_before();
     __syncthreads();
     cluster_sync_all();                       // the peer's barriers are initialised before anything targets them
     tc_fence_after();
-    const uint32_t tmem_base = tmem_base_smem;
+    const uint32_t tmem_base = ctl.tmem_base;
 
     if (warp == 0) {
         // ---------------------------------------------------------------- TMA producer (one per CTA)
@@ -992,77 +1024,130 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         }
     } else {
         // ---------------------------------------------------------------- epilogue (warps 2..9 of both CTAs)
-        // No staging buffer: a warp packs its BN / 2 columns of the accumulator into registers, hands the buffer
-        // back, then stores 16-bit values directly; the 32 lanes of a store are 32 consecutive features of one
-        // token, 64 contiguous bytes.
+        // Plain form: a warp takes every other 16-token chunk of its 32 features.  tcgen05.ld in the 16x256b shape leaves 8 x 8
+        // fragments, packed to 16 bits in registers (64 of them), and the accumulator goes back to the MMAs at once.  stmatrix then
+        // writes the fragments token-major into the warp's two chunks of shared memory, from where 16-byte stores take them: 8 tokens
+        // x 64 bytes an instruction instead of one token's 32 two-byte values.  What bounds it is the chip's writes, about 3.4 TB/s
+        // however they are issued (128-byte rows and TMA stores were no faster), shared with the operand fill.  fp16 / bf16, us,
+        // two-byte stores -> now: ms 3072, k 768, n 8192 27.2 -> 26.2; ms 2304 23.3 -> 21.7; ms 768, k 3072 23.7 -> 22.9;
+        // ms 4096, k 4096, n 2043 30.7 -> 29.5, n 16 14.4 -> 13.4.
+        // Fused forms: a warp packs its BN / 2 columns of the accumulator into registers, hands the buffer back, then stores
+        // 16-bit values directly; the 32 lanes of a store are 32 consecutive features of one token.
         const int quad = warp & 3, half = (warp - 2) >> 2;
-        const int HC = BN / 2;                      // a multiple of 8 up to 120 (fused epilogues: of 16 up to 96)
-        constexpr int NREG = EPI == EPI_PLAIN ? 64 : 48;
+        const int HC = BN / 2;                      // fused epilogues: a multiple of 16 up to 96
+        constexpr int NREG = 48;
         OutT *out = static_cast<OutT *>(P.out);
         const float alpha = F8 ? alpha_of(P) : 1.f;
         const uint32_t empty_leader0 = map_to_cta(tmem_empty0, 0);
+        // plain form: the warp's staging, and where a lane's stmatrix row goes in a chunk: token 8 (lane / 16) + lane % 8 in rows of
+        // 64 bytes, features 16 h + 8 (lane / 8 % 2) in 16-byte pieces, permuted by token / 2 % 4 against bank conflicts
+        const uint32_t stg = smem_u32(smem) + STAGES * STAGE2_BYTES + (warp - 2) * 2 * CHUNK2_BYTES;
+        const uint32_t ld_off = (lane >> 2) * 64 + (((lane & 3) ^ ((lane >> 3) & 3)) << 4);
+        uint32_t stm_off[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int tok = 8 * (lane >> 4) + (lane & 7), piece = 2 * h + ((lane >> 3) & 1);
+            stm_off[h] = tok * 64 + ((piece ^ ((tok >> 1) & 3)) << 4);
+        }
         int tl = 0;
         for (int tile = pair; tile < n_tiles; tile += n_pairs, ++tl) {
             const int buf = tl & 1;
-            const int mrow = ((tile % n_tiles_m) * 2 + (int)rank) * BM + quad * 32 + lane;
-            const int64_t tok0 = (int64_t)(tile / n_tiles_m) * BN + half * HC;
+            const int mrow = ((tile % n_tiles_m) * 2 + (int)rank) * BM + quad * 32;
+            const int64_t row0 = (int64_t)(tile / n_tiles_m) * BN;
             const bool ok = mbar_wait(tmem_full0 + 8 * buf, (tl >> 1) & 1, &abort_flag, P.status, 3);
             tc_fence_after();
             if (threadIdx.x == 64) SP24_TRACE(2, 4 * tl);
-            const bool run = ok && !abort_flag;
-            uint32_t held[NREG];
-            if (run) {
-                float bias = 0.f;
-                if (P.bias) bias = load_bias<OutT>(P, mrow);
-                const uint32_t acc = tmem_base + ((uint32_t)(quad * 32) << 16) + buf * ACC_COL + half * HC;
+            const bool run = __all_sync(0xFFFFFFFFu, ok && !abort_flag);      // the warp reads tensor memory together
+            if constexpr (EPI == EPI_PLAIN) {
+                const int64_t left = P.n - row0;
+                const int limit = left < BN ? (int)left : BN, chunks = (limit + 15) / 16;
+                uint32_t held[MAX_CHUNKS2][8];      // chunk half + 2 i: word 4 h + j has features 16 h + 8 (j % 2), tokens 8 (j / 2)
+                if (run) {
+                    float bias[4] = {0.f, 0.f, 0.f, 0.f};       // of features 8 h + lane / 4
+                    if (P.bias) {
 #pragma unroll
-                for (int c = 0; c < NREG / 16; ++c) {
-                    if (c * 32 >= HC) break;
-                    uint32_t v[32];             // columns past HC belong to other tiles or to the metadata: read, never stored
-                    tmem_ld32(acc + c * 32, v);
-                    tmem_ld_wait();
+                        for (int h = 0; h < 4; ++h) bias[h] = load_bias<OutT>(P, mrow + 8 * h + (lane >> 2));
+                    }
+                    const uint32_t acc = tmem_base + ((uint32_t)(quad * 32) << 16) + buf * ACC_COL + half * 16;
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) {
-                        Vec<OutT, 2> o;
-                        if constexpr (EPI == EPI_DGELU) {   // no bias; the factor gelu'(aux) is applied at store time
-                            o.v[0] = to_out<OutT>(__uint_as_float(v[2 * i]));
-                            o.v[1] = to_out<OutT>(__uint_as_float(v[2 * i + 1]));
-                        } else {
-                            o.v[0] = emit<OutT, false, F8>(v[2 * i], bias, 0, alpha);
-                            o.v[1] = emit<OutT, false, F8>(v[2 * i + 1], bias, 0, alpha);
+                    for (int i0 = 0; i0 < MAX_CHUNKS2; i0 += 2) {
+                        if (half + 2 * i0 >= chunks) break;
+                        uint32_t v[2][2][8];
+#pragma unroll
+                        for (int i = 0; i < 2; ++i) {           // past the last chunk: other columns, read but not stored
+                            tmem_ld_16x256b_x2(acc + (i0 + i) * 32, v[i][0]);
+                            tmem_ld_16x256b_x2(acc + (16u << 16) + (i0 + i) * 32, v[i][1]);
                         }
-                        held[c * 16 + i] = *reinterpret_cast<const uint32_t *>(&o);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int i = 0; i < 2; ++i)
+#pragma unroll
+                            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                                for (int j = 0; j < 4; ++j) {
+                                    Vec<OutT, 2> o;
+                                    o.v[0] = emit<OutT, false, F8>(v[i][h][2 * j], bias[2 * h + (j & 1)], 0, alpha);
+                                    o.v[1] = emit<OutT, false, F8>(v[i][h][2 * j + 1], bias[2 * h + (j & 1)], 0, alpha);
+                                    held[i0 + i][4 * h + j] = *reinterpret_cast<const uint32_t *>(&o);
+                                }
                     }
                 }
-            }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(empty_leader0 + 8 * buf);
-            if (threadIdx.x == 64) SP24_TRACE(2, 4 * tl + 1);
-            if (run) {
-                uint16_t *dst = reinterpret_cast<uint16_t *>(out) + tok0 * P.ld_out + mrow;
-                uint16_t *aux = reinterpret_cast<uint16_t *>(P.aux) + tok0 * P.ld_aux + mrow;
-                if constexpr (EPI == EPI_PLAIN) {
-                    if (tok0 + HC <= P.n) {
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_cluster(empty_leader0 + 8 * buf);
+                if (threadIdx.x == 64) SP24_TRACE(2, 4 * tl + 1);
+                if (run) {
+                    uint4 *const dst = reinterpret_cast<uint4 *>(out + (row0 + half * 16 + (lane >> 2)) * P.ld_out + mrow) + (lane & 3);
+                    const int mine = limit - half * 16 - (lane >> 2);       // tokens of the tile from this lane's first one on
 #pragma unroll
-                        for (int c2 = 0; c2 < NREG; ++c2) {
-                            if (c2 % 4 == 0 && 2 * c2 >= HC) break;
-                            dst[0] = (uint16_t)(held[c2] & 0xFFFFu);
-                            dst[P.ld_out] = (uint16_t)(held[c2] >> 16);
-                            dst += 2 * P.ld_out;
-                            asm volatile("" : "+l"(dst));   // one running pointer, not a precomputed address per column
-                        }
-                    } else {
+                    for (int i = 0; i < MAX_CHUNKS2; ++i) {
+                        if (half + 2 * i >= chunks) break;
+                        const uint32_t at = stg + (i & 1) * CHUNK2_BYTES;
 #pragma unroll
-                        for (int c2 = 0; c2 < NREG; ++c2) {
-                            if (c2 % 4 == 0 && 2 * c2 >= HC) break;
-                            if (tok0 + 2 * c2 < P.n) dst[0] = (uint16_t)(held[c2] & 0xFFFFu);
-                            if (tok0 + 2 * c2 + 1 < P.n) dst[P.ld_out] = (uint16_t)(held[c2] >> 16);
-                            dst += 2 * P.ld_out;
-                            asm volatile("" : "+l"(dst));
+                        for (int h = 0; h < 2; ++h)
+                            stmatrix_x4_trans(at + stm_off[h], held[i][4 * h], held[i][4 * h + 1], held[i][4 * h + 2], held[i][4 * h + 3]);
+                        __syncwarp();                           // also: the chunk before the last one has left its half
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {           // 8 tokens x 64 bytes an instruction
+                            const uint4 o = ld_shared_v4(at + ld_off + h * 512);
+                            if (32 * i + 8 * h < mine) dst[(32 * i + 8 * h) * (P.ld_out / 8)] = o;
                         }
                     }
-                } else {
+                    __syncwarp();
+                }
+            } else {
+                const int64_t tok0 = row0 + half * HC;
+                uint32_t held[NREG];
+                if (run) {
+                    float bias = 0.f;
+                    if (P.bias) bias = load_bias<OutT>(P, mrow + lane);
+                    const uint32_t acc = tmem_base + ((uint32_t)(quad * 32) << 16) + buf * ACC_COL + half * HC;
+#pragma unroll
+                    for (int c = 0; c < NREG / 16; ++c) {
+                        if (c * 32 >= HC) break;
+                        uint32_t v[32];             // columns past HC belong to other tiles or to the metadata: read, never stored
+                        tmem_ld32(acc + c * 32, v);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) {
+                            Vec<OutT, 2> o;
+                            if constexpr (EPI == EPI_DGELU) {   // no bias; the factor gelu'(aux) is applied at store time
+                                o.v[0] = to_out<OutT>(__uint_as_float(v[2 * i]));
+                                o.v[1] = to_out<OutT>(__uint_as_float(v[2 * i + 1]));
+                            } else {
+                                o.v[0] = emit<OutT, false, F8>(v[2 * i], bias, 0, alpha);
+                                o.v[1] = emit<OutT, false, F8>(v[2 * i + 1], bias, 0, alpha);
+                            }
+                            held[c * 16 + i] = *reinterpret_cast<const uint32_t *>(&o);
+                        }
+                    }
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_cluster(empty_leader0 + 8 * buf);
+                if (run) {
+                    uint16_t *dst = reinterpret_cast<uint16_t *>(out) + tok0 * P.ld_out + mrow + lane;
+                    uint16_t *aux = reinterpret_cast<uint16_t *>(P.aux) + tok0 * P.ld_aux + mrow + lane;
                     const bool full = tok0 + HC <= P.n;
                     auto as_f = [](uint16_t bits) { return from_out<OutT>(*reinterpret_cast<const OutT *>(&bits)); };
                     auto as_b = [](float v) { const OutT o = to_out<OutT>(v); return *reinterpret_cast<const uint16_t *>(&o); };
@@ -1466,7 +1551,7 @@ int make_map_e(CUtensorMap *map, const void *e_tc, int64_t n_atoms, int atoms_pe
 template <bool A_MN, typename OutT, int EPI = EPI_PLAIN, bool F8 = false>
 int launch_spmm_pair(const CUtensorMap &ma, const CUtensorMap &mb, const CUtensorMap &me, SpmmParams P, cudaStream_t st) {
     auto kern = spmm_pair_kernel<A_MN, OutT, EPI, F8>;
-    constexpr int SMEM_MAX = 227 * 1024 - 1024;
+    constexpr int SMEM_MAX = two::SMEM_LIMIT;
     static bool attr_set[64];
     int dev = 0;
     cudaGetDevice(&dev);
