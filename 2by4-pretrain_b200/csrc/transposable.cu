@@ -394,10 +394,11 @@ __device__ __forceinline__ void ts_dual_block(const DualParams &P, const unsigne
     }
 }
 
-// Resident CTAs per SM.  With the search: three for 16-bit inputs (80 registers), two for fp32 ones.  Without it the pass is
-// bound by memory latency between its barriers and needs fewer registers: one CTA more
-// (the 48 fp32 weights of a 12-block, 768-wide model, given masks, bf16 out: 166 -> 127 us, 3.7 -> 4.9 TB/s).
-constexpr int dual_min_blocks(bool select, int in_bytes) { return (in_bytes == 2 ? 3 : 2) + (select ? 0 : 1); }
+// Resident CTAs per SM.  Between its barriers the pass waits for memory, so a CTA more pays as long as the registers hold (with
+// the search 64 for 16-bit inputs, 12 bytes of spills, 80 for float32; without it 39 - 48 and 56).  us, one CTA fewer -> now -> one more:
+//   the 48 float32 weights of a 12-block, 768-wide model, bf16 out: given masks 124.7 -> 109.3 -> 115.1, search 208 -> 166
+//   eight 4096 x 4096 of 16 bits: given masks 134.9 -> 124.0 -> 135.3, search 230 -> 222
+constexpr int dual_min_blocks(bool select, int in_bytes) { return (in_bytes == 2 ? 4 : 3) + (select ? 0 : 1); }
 
 template <typename T, typename TOut, bool SELECT, bool TC>
 __global__ void __launch_bounds__(256, dual_min_blocks(SELECT, sizeof(T))) ts_dual_kernel(DualParams P) {
