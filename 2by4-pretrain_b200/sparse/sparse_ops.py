@@ -313,17 +313,27 @@ class SparseLinearTranspose(nn.Linear):
 
 def _modules(model: nn.Module):
     """``model.modules()``, each once and in the same order, without a generator per level of nesting: with 48 layers the walk was
-    a fifth of the host time of their refresh."""
-    if type(model).modules is not nn.Module.modules or type(model).named_modules is not nn.Module.named_modules:
+    a fifth of the host time of their refresh.  torch's walk asks every module for its ``named_modules``, so a module that has
+    one of its own, in its class or on the instance, decides what is below it; ``modules`` counts at the root only."""
+    if type(model).modules is not nn.Module.modules or 'modules' in model.__dict__:
         return list(model.modules())
-    seen, out, stack = set(), [], [model]
+    seen, out, stack, plain = set(), [], [model], set()
     while stack:
         mod = stack.pop()
         if mod is None or mod in seen:
             continue
+        cls = type(mod)
+        if cls not in plain:
+            if cls.named_modules is not nn.Module.named_modules:
+                return list(model.modules())
+            plain.add(cls)
+        if 'named_modules' in mod.__dict__:
+            return list(model.modules())
         seen.add(mod)
         out.append(mod)
-        stack.extend(reversed(mod._modules.values()))
+        children = mod._modules
+        if children:
+            stack.extend(reversed(children.values()))
     return out
 
 

@@ -20,9 +20,29 @@ class _Narrow(nn.Module):
         yield self.a
 
 
+class _Hides(nn.Module):
+    """A module that shows one of its two children to a walk."""
+    def __init__(self):
+        super().__init__()
+        self.shown, self.hidden = nn.Linear(2, 2), nn.Linear(2, 2)
+
+    def named_modules(self, memo=None, prefix="", remove_duplicate=True):
+        yield prefix, self
+        yield prefix + ".shown", self.shown
+
+
+def _own(name, value):
+    """A module with ``name`` of its own on the instance, not in the class."""
+    model = nn.Sequential(nn.Linear(2, 2), nn.ReLU())
+    model.__dict__[name] = lambda *a, **k: iter(value(model))
+    return model
+
+
 def test_same_modules_in_the_same_order():
     from sparse.sparse_ops import _modules
-    for model in (nn.Linear(2, 2), _nested(), _Narrow(), nn.ModuleList()):
+    own_modules, own_named = _own("modules", lambda m: [m[0]]), _own("named_modules", lambda m: [("", m), ("1", m[1])])
+    for model in (nn.Linear(2, 2), _nested(), _Narrow(), nn.ModuleList(), _Hides(), nn.Sequential(nn.ReLU(), nn.ModuleList([_Hides()])),
+                  nn.Sequential(_Narrow(), nn.ReLU()), own_modules, own_named, nn.Sequential(own_modules, own_named)):
         assert [id(m) for m in _modules(model)] == [id(m) for m in model.modules()]
 
 
