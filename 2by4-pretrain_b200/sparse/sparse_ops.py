@@ -350,9 +350,7 @@ def refresh_sparse_layers(model: nn.Module) -> int:
     for mod in _modules(model):
         if not isinstance(mod, SparseLinearTranspose):
             continue
-        w = mod._parameters.get('weight')
-        if w is None:                        # a parametrized weight is an attribute of another kind
-            w = mod.weight
+        w = mod.weight                       # the attribute: a subclass or a parametrization may answer for the parameter
         if w.mode != 'sparse' or w.cnt != 0 or not w.is_cuda:
             continue
         m, k = w.shape

@@ -1,4 +1,7 @@
 """The walk over a model's modules that the batched refresh of sparse layers makes: what ``modules()`` yields, in its order."""
+from types import SimpleNamespace
+
+import pytest
 import torch
 from torch import nn
 
@@ -55,3 +58,44 @@ def test_parametrized_weight_is_found():
     layer.__dict__["weight"] = w
     assert sparse.refresh_sparse_layers(nn.ModuleList([layer])) == 0
     assert torch.equal(layer.weight.mask, torch.ones(128, 128, dtype=torch.bool))
+
+
+def _gpu_weight(shape, counter=1):
+    """What the refresh reads of a weight on the GPU."""
+    return SimpleNamespace(mode="sparse", cnt=0, counter=counter, freq=40, is_cuda=True, shape=torch.Size(shape), dtype=torch.float32,
+                           device=torch.device("cpu"), mask=torch.ones(shape, dtype=torch.bool))
+
+
+@pytest.fixture
+def refreshed(monkeypatch):
+    """The weights that reach the native call, by the refresh's option ``reselect``."""
+    import sparse.sparse_ops as ops
+    calls = {}
+
+    def native(weights, masks, dtype, reselect):
+        calls[reselect] = list(weights)
+        return [(m, *[torch.empty(0)] * 4, None, None) for m in masks]
+
+    monkeypatch.setattr(ops, "_ext", SimpleNamespace(host=SimpleNamespace(select_compress_many=native)))
+    return calls
+
+
+def test_refresh_takes_the_weight_that_the_layer_uses(refreshed):
+    """A plain parameter, an attribute in the place of a parameter that was taken out (what a parametrization leaves), one that
+    hides the parameter, and a subclass that answers itself."""
+    import sparse
+
+    class Viewed(sparse.SparseLinearTranspose):
+        def __getattribute__(self, name):
+            if name == "weight" and "seen" in object.__getattribute__(self, "__dict__"):
+                return self.seen
+            return super().__getattribute__(name)
+
+    plain, replaced, hidden = (sparse.SparseLinearTranspose(128, 128) for _ in range(3))
+    viewed = Viewed(128, 128)
+    del replaced._parameters["weight"]
+    weights = [_gpu_weight((128, 256), c) for c in (1, 40, 1)]
+    replaced.__dict__["weight"], hidden.__dict__["weight"], viewed.__dict__["seen"] = weights
+    assert sparse.refresh_sparse_layers(nn.ModuleList([plain, replaced, hidden, viewed])) == 3        # `plain` is on the CPU
+    assert [id(w) for w in refreshed[False]] == [id(weights[0]), id(weights[2])] and refreshed[True] == [weights[1]]
+    assert all(w.refreshed for w in weights) and torch.equal(plain.weight.mask, torch.ones(128, 128, dtype=torch.bool))
