@@ -353,8 +353,8 @@ def refresh_sparse_layers(model: nn.Module) -> int:
         w = mod.weight                       # the attribute: a subclass or a parametrization may answer for the parameter
         if w.mode != 'sparse' or w.cnt != 0 or not w.is_cuda:
             continue
-        m, k = w.shape
-        if m % 128 or k % 128:
+        shape = w.shape                      # rows decide first: a trainer's flat shard of odd size is passed over too
+        if shape[0] % 128 or shape[1] % 128:
             continue
         mask, device = w.mask, w.device
         if mask.device != device:

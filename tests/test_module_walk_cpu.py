@@ -99,3 +99,12 @@ def test_refresh_takes_the_weight_that_the_layer_uses(refreshed):
     assert sparse.refresh_sparse_layers(nn.ModuleList([plain, replaced, hidden, viewed])) == 3        # `plain` is on the CPU
     assert [id(w) for w in refreshed[False]] == [id(weights[0]), id(weights[2])] and refreshed[True] == [weights[1]]
     assert all(w.refreshed for w in weights) and torch.equal(plain.weight.mask, torch.ones(128, 128, dtype=torch.bool))
+
+
+@pytest.mark.parametrize("shape", [(100,), (130, 128), (128, 130), (2, 128, 128)])
+def test_refresh_leaves_other_shapes_alone(refreshed, shape):
+    """Sizes off 128, and shards that a trainer keeps flat: left to the layer itself."""
+    import sparse
+    layer = sparse.SparseLinearTranspose(128, 128)
+    layer.__dict__["weight"] = _gpu_weight(shape)
+    assert sparse.refresh_sparse_layers(layer) == 0 and not refreshed
