@@ -895,7 +895,7 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *smem = smem_raw;
-    if (smem_u32(smem) & 1023) {              // the same in every CTA; not seen, but the swizzled stages depend on it
+    if (smem_u32(smem) & 1023) {              // the same in every CTA; the launcher looks first, the swizzled stages depend on it
         if (threadIdx.x == 0 && P.status) atomicCAS(P.status, 0, 11);
         return;
     }
@@ -1556,6 +1556,11 @@ int launch_spmm_pair(const CUtensorMap &ma, const CUtensorMap &mb, const CUtenso
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !attr_set[dev]) {
+        // the kernel takes its dynamic shared memory as it comes: it starts on 1024 bytes only behind none, or whole kilobytes, of
+        // static shared memory
+        cudaFuncAttributes fa{};
+        if (cudaFuncGetAttributes(&fa, kern) != cudaSuccess) return launch_status();
+        if (fa.sharedSizeBytes % 1024) return SP24_ERR_ALIGN;
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX) != cudaSuccess)
             return SP24_ERR_CUDA;
         attr_set[dev] = true;

@@ -44,13 +44,22 @@ _tc_meta_cache = {}
 
 
 def _status_word(device):
-    """The word the GEMM kernels of ``device`` report a bounded wait that gave up to."""
+    """The word to which the GEMM kernels of ``device`` report that they stopped early."""
     return _ext.host.status_word(device.index if device.index is not None else torch.cuda.current_device())
 
 
+_MISPLACED = 11       # the status code of a kernel whose shared memory starts off a 1024-byte boundary
+
+
+def _stopped(code):
+    if code == _MISPLACED:
+        return "shared memory off its 1024-byte boundary, the result was not written,"
+    return f"an on-device wait gave up (role code {code})"
+
+
 def check_status(device=None):
-    """Synchronises and raises if a bounded on-device wait of the sparse GEMM ever gave up, on any device that ran one or on
-    ``device`` only."""
+    """Synchronises and raises if a sparse GEMM ever stopped early, on any device that ran one or on ``device`` only: a bounded
+    on-device wait gave up, or its shared memory did not start where its operands need it."""
     if "status_words" not in vars(_ext.host):       # the native module is not loaded: no GEMM has run
         return
     for index, t in _ext.host.status_words().items():
@@ -59,7 +68,7 @@ def check_status(device=None):
             code = int(t.item())
             if code:
                 t.zero_()
-                raise RuntimeError(f"sp24_spmm: an on-device wait gave up (role code {code}) on {dev}")
+                raise RuntimeError(f"sp24_spmm: {_stopped(code)} on {dev}")
 
 
 def invalidate_meta(meta):

@@ -373,7 +373,9 @@ int sp24_meta_to_tc(const void *meta, int meta_itemsize, int64_t m, int64_t k, v
  *              16-bit GEMMs with b_mn_major = 0, trans_out = 1, ms % 256 == 0 and no activation run on
  *              pairs of CTAs (tcgen05 cta_group::2); the result is bit-equal to the single-CTA kernel's.
  *   bias       ms values in the output type or NULL; activation 0 none, 1 relu, 2 silu, 3 gelu (tanh form; not in the reference)
- *   status     optional device int: set to a non-zero code if a bounded on-device wait gave up
+ *   status     optional device int: set to a non-zero code if a bounded on-device wait gave up (11: the shared memory of a
+ *              CTA-pair kernel did not start on 1024 bytes and nothing was written; a build in which that could be
+ *              returns SP24_ERR_ALIGN at the launch)
  * Shape rules: ms % 128 == 0, k % 64 == 0 (16-bit) or k % 128 == 0 (8-bit); n % 8 == 0 unless B is stored (n, k)
  * and the output (n, ms) (b_mn_major == 0 and trans_out == 1), where any n > 0 is accepted.
  */

@@ -17,3 +17,18 @@ def test_rule_takes_legal_widths_only(form):
             assert rule(ms, n, form, sms) in P.WIDTHS[form], (ms, n, sms)
     assert set(P.shapes(form)) == P.WIDTHS[form]          # every width is reached, so the GPU tests' shapes cover them all
     assert rule(128, 64, form, 148) == 0 and rule(256, 0, form, 148) == 0
+
+
+@pytest.mark.parametrize("code,says", [(3, "wait gave up (role code 3)"), (11, "1024-byte boundary")])
+def test_status_codes_say_what_happened(monkeypatch, code, says):
+    """A kernel that could not start is not reported as a wait that gave up; the word is cleared once it was reported."""
+    from types import SimpleNamespace
+
+    import torch
+    from sparse import spmm
+    word = torch.tensor([code], dtype=torch.int32)
+    monkeypatch.setattr(spmm, "_ext", SimpleNamespace(host=SimpleNamespace(status_words=lambda: {0: word})))
+    with pytest.raises(RuntimeError) as e:
+        spmm.check_status()
+    assert says in str(e.value) and ("wait" in str(e.value)) == (code != 11) and "cuda:0" in str(e.value)
+    spmm.check_status()
