@@ -395,13 +395,27 @@ __device__ __forceinline__ void ts_dual_block(const DualParams &P, const unsigne
 }
 
 // Resident CTAs per SM.  Between its barriers the pass waits for memory, so a CTA more pays as long as the registers hold (with
-// the search 64 for 16-bit inputs, 12 bytes of spills, 80 for float32; without it 39 - 48 and 56).  us, one CTA fewer -> now -> one more:
+// the search 64 for 16-bit inputs, over a list 12 bytes of spills, 80 for float32; without it 39 - 48 and 56 - 63).  us, one CTA fewer -> now -> one more:
 //   the 48 float32 weights of a 12-block, 768-wide model, bf16 out: given masks 124.7 -> 109.3 -> 115.1, search 208 -> 166
 //   eight 4096 x 4096 of 16 bits: given masks 134.9 -> 124.0 -> 135.3, search 230 -> 222
-constexpr int dual_min_blocks(bool select, int in_bytes) { return (in_bytes == 2 ? 4 : 3) + (select ? 0 : 1); }
+// A grid that the SMs hold at once, or nearly, has no use for the CTA and pays for its registers: with FEW it has one fewer.
+constexpr int dual_min_blocks(bool select, int in_bytes, bool few) { return (in_bytes == 2 ? 4 : 3) + (select ? 0 : 1) - (few ? 1 : 0); }
 
-template <typename T, typename TOut, bool SELECT, bool TC>
-__global__ void __launch_bounds__(256, dual_min_blocks(SELECT, sizeof(T))) ts_dual_kernel(DualParams P) {
+// Blocks per SM up to which the form with fewer resident CTAs is taken: about its own resident count, and more for the 16-bit
+// search over a list, whose 64-register form spills most.  us, few -> many:
+//   float32 search 2304 x 768 6.1 -> 6.4, 2048 x 2048 10.4 -> 10.2; 16-bit search 768 x 3072 6.23 -> 6.27, 2048 x 2048 9.9 -> 9.7,
+//   over a list: one 768 x 768 4.9 -> 5.4, four 3072 x 768 (1152 blocks) 17.9 -> 18.4, four 2048 x 2048 (2048) 31.4 -> 31.3
+//   16-bit given masks 2048 x 2048 (512 blocks) 6.3 -> 6.4, four 2304 x 768 (864) 9.0 -> 8.8; float32 ones are faster at every size
+//   16-bit given masks into the other 16-bit type: slower at every size, 2048 x 2048 7.4 -> 8.0, four 4096 x 4096 76.3 -> 78.0
+constexpr int ALWAYS_FEW = 1 << 20;
+template <typename T, typename TOut> constexpr int dual_few_limit(bool select, bool list) {
+    if (sizeof(T) == 4) return select ? 2 : 0;
+    if (!select) return std::is_same<T, TOut>::value ? 4 : ALWAYS_FEW;
+    return list ? 13 : 3;
+}
+
+template <typename T, typename TOut, bool SELECT, bool TC, bool FEW>
+__global__ void __launch_bounds__(256, dual_min_blocks(SELECT, sizeof(T), FEW)) ts_dual_kernel(DualParams P) {
     ts_dual_block<T, TOut, SELECT, TC>(P, blockIdx.x, blockIdx.y);
 }
 
@@ -414,8 +428,8 @@ struct DualBatch {
     unsigned first[kDualBatchMax + 1];
     int count;
 };
-template <typename T, typename TOut, bool SELECT, bool TC>
-__global__ void __launch_bounds__(256, dual_min_blocks(SELECT, sizeof(T))) ts_dual_batch_kernel(const __grid_constant__ DualBatch B) {
+template <typename T, typename TOut, bool SELECT, bool TC, bool FEW>
+__global__ void __launch_bounds__(256, dual_min_blocks(SELECT, sizeof(T), FEW)) ts_dual_batch_kernel(const __grid_constant__ DualBatch B) {
     int i = 0;
     while (i + 1 < B.count && blockIdx.x >= B.first[i + 1]) ++i;
     const DualParams &P = B.p[i];
@@ -424,29 +438,37 @@ __global__ void __launch_bounds__(256, dual_min_blocks(SELECT, sizeof(T))) ts_du
     ts_dual_block<T, TOut, SELECT, TC>(P, local % ncb, local / ncb);
 }
 
-template <typename T, typename TOut> int launch_dual(const DualParams &P, int select, cudaStream_t st) {
+template <typename T, typename TOut, bool SELECT, bool TC> int launch_dual_form(const DualParams &P, cudaStream_t st) {
     dim3 grid((unsigned)((P.k + 127) / 128), (unsigned)(P.m / 64));
-    const bool tc = P.tc_w != nullptr;
-    if (select) {
-        if (tc) ts_dual_kernel<T, TOut, true, true><<<grid, 256, 0, st>>>(P);
-        else ts_dual_kernel<T, TOut, true, false><<<grid, 256, 0, st>>>(P);
+    constexpr int limit = dual_few_limit<T, TOut>(SELECT, false);
+    if (limit == ALWAYS_FEW || (uint64_t)grid.x * grid.y <= (uint64_t)limit * sm_count()) {
+        if constexpr (limit > 0) ts_dual_kernel<T, TOut, SELECT, TC, true><<<grid, 256, 0, st>>>(P);
     } else {
-        if (tc) ts_dual_kernel<T, TOut, false, true><<<grid, 256, 0, st>>>(P);
-        else ts_dual_kernel<T, TOut, false, false><<<grid, 256, 0, st>>>(P);
+        if constexpr (limit < ALWAYS_FEW) ts_dual_kernel<T, TOut, SELECT, TC, false><<<grid, 256, 0, st>>>(P);
     }
     return launch_status();
 }
 
-template <typename T, typename TOut> int launch_dual_batch(const DualBatch &B, int select, bool tc, cudaStream_t st) {
+template <typename T, typename TOut, bool SELECT, bool TC> int launch_dual_list(const DualBatch &B, cudaStream_t st) {
     const unsigned grid = B.first[B.count];
-    if (select) {
-        if (tc) ts_dual_batch_kernel<T, TOut, true, true><<<grid, 256, 0, st>>>(B);
-        else ts_dual_batch_kernel<T, TOut, true, false><<<grid, 256, 0, st>>>(B);
+    constexpr int limit = dual_few_limit<T, TOut>(SELECT, true);
+    if (limit == ALWAYS_FEW || grid <= (uint64_t)limit * sm_count()) {
+        if constexpr (limit > 0) ts_dual_batch_kernel<T, TOut, SELECT, TC, true><<<grid, 256, 0, st>>>(B);
     } else {
-        if (tc) ts_dual_batch_kernel<T, TOut, false, true><<<grid, 256, 0, st>>>(B);
-        else ts_dual_batch_kernel<T, TOut, false, false><<<grid, 256, 0, st>>>(B);
+        if constexpr (limit < ALWAYS_FEW) ts_dual_batch_kernel<T, TOut, SELECT, TC, false><<<grid, 256, 0, st>>>(B);
     }
     return launch_status();
+}
+
+template <typename T, typename TOut> int launch_dual(const DualParams &P, int select, cudaStream_t st) {
+    const bool tc = P.tc_w != nullptr;
+    if (select) return tc ? launch_dual_form<T, TOut, true, true>(P, st) : launch_dual_form<T, TOut, true, false>(P, st);
+    return tc ? launch_dual_form<T, TOut, false, true>(P, st) : launch_dual_form<T, TOut, false, false>(P, st);
+}
+
+template <typename T, typename TOut> int launch_dual_batch(const DualBatch &B, int select, bool tc, cudaStream_t st) {
+    if (select) return tc ? launch_dual_list<T, TOut, true, true>(B, st) : launch_dual_list<T, TOut, true, false>(B, st);
+    return tc ? launch_dual_list<T, TOut, false, true>(B, st) : launch_dual_list<T, TOut, false, false>(B, st);
 }
 
 template <typename T> int dispatch_dual_batch(const DualBatch &B, int packed_dtype, int select, bool tc, cudaStream_t st) {
