@@ -112,3 +112,50 @@ def test_float8_products_at_each_width(width, k, dtype):
                "spmm_f8")
     assert torch.equal(out, spmm.sparse_linear(xq, packed, meta, bias=bias, alpha=sw * sx).to(dtype))
     spmm.check_status()
+
+
+def _window(n, ms, dtype):
+    """A pre-filled buffer with a row more above and below and 8 values more on either side, its bits, and the (n, ms) window."""
+    buf = torch.randn(n + 2, ms + 16, device=DEV).to(dtype)
+    return buf, buf.view(torch.int16).clone(), buf[1:-1, 8:-8]
+
+
+def _only_the_window_changed(buf, before, window, result):
+    assert torch.equal(window, result)
+    window.view(torch.int16).copy_(before[1:-1, 8:-8])
+    assert torch.equal(buf.view(torch.int16), before)
+
+
+@pytest.mark.parametrize("ms,n", [(256, 1), (256, 7), (512, 17), (1024, 33)] + [(0, w) for w in sorted(WIDTHS[PLAIN])])
+def test_plain_products_stay_in_their_window(ms, n):
+    """16-byte stores of a pitched output at few tokens and at each width's ragged end (ms 0: the shape of that width)."""
+    from sparse import _ext, spmm
+    ms, n = (ms, n) if ms else _size(PLAIN, n)
+    k = 192
+    p, e, g = _operand(ms, k, torch.bfloat16, ms + n, False)
+    x = torch.randn(n, k, device=DEV, generator=g).bfloat16()
+    b = torch.randn(ms, device=DEV, generator=g).bfloat16()
+    buf, before, out = _window(n, ms, torch.bfloat16)
+    status = spmm._status_word(torch.device(DEV))
+    _ext.check(_ext.lib().sp24_spmm(p.data_ptr(), _ext.BF16, 0, k // 2, spmm.tc_metadata(e, ms, k).data_ptr(), ms, k, x.data_ptr(), 0, k, n,
+                                    out.data_ptr(), _ext.BF16, 1, ms + 16, b.data_ptr(), 0, status.data_ptr(), _ext.stream()), "spmm")
+    _only_the_window_changed(buf, before, out, spmm.sparse_linear(x, p, e, b))
+    spmm.check_status()
+
+
+@pytest.mark.parametrize("ms,n", [(256, 1), (256, 7), (512, 17)] + [(0, w) for w in sorted(WIDTHS[FLOAT8])])
+def test_float8_products_stay_in_their_window(ms, n):
+    from sparse import _ext, fp8, spmm
+    ms, n = (ms, n) if ms else _size(FLOAT8, n)
+    k = 384
+    g = torch.Generator(device=DEV).manual_seed(ms + n)
+    w, x = torch.randn(ms, k, device=DEV, generator=g), torch.randn(n, k, device=DEV, generator=g)
+    sw, (xq, sx) = fp8.scale_of(w), fp8.quantize(x)
+    aw, ax = w.abs().amax().reshape(1), x.abs().amax().reshape(1)
+    packed, meta = fp8.compress_q8(w, mode=_ext.PRUNE_MSE, scale=sw)
+    buf, before, out = _window(n, ms, torch.float16)
+    tc, status = spmm.tc_metadata(meta, ms, k), spmm._status_word(torch.device(DEV))
+    _ext.check(_ext.lib().sp24_spmm_f8(packed.data_ptr(), _ext.E4M3, k // 2, tc.data_ptr(), ms, k, xq.data_ptr(), k, n, out.data_ptr(),
+                                       _ext.F16, 1, ms + 16, None, aw.data_ptr(), ax.data_ptr(), status.data_ptr(), _ext.stream()), "spmm_f8")
+    _only_the_window_changed(buf, before, out, spmm.sparse_linear(xq, packed, meta, alpha=sw * sx).half())
+    spmm.check_status()
