@@ -797,10 +797,18 @@ constexpr int MAX_STAGES2 = 6;
 // BN / 2 rows of B as two 128-byte K atoms; every part is a multiple of the 1024-byte swizzle period.
 constexpr int e2_bytes(bool f8) { return f8 ? 4096 : 2048; }
 constexpr int stage2_bytes(bool f8, int bn) { return A_STAGE_BYTES + e2_bytes(f8) + bn * 128; }
-// Output staging of the plain epilogue: a chunk is 16 tokens x 32 features of 16 bits, two per epilogue warp.
+// Output staging of the plain epilogue: a chunk is 16 tokens x 32 features of 16 bits, two per epilogue warp.  Four widths have one
+// operand stage fewer for it: 16-bit 144 and 208, float8 128 and 192.  Against the direct stores before it the calls
+// measured at 208, 128 and 192 lost no more than 1 % (ms 2304, k 3072, n 8192 57.0 -> 57.6 us; float8 ms 768, k 3072, n 8192 15.7 both) but for float8 at width
+// 128 with three K steps in one round, 6.4 -> 6.5.  Pieces of 8 tokens, one or two a warp, gave the stages back and were not kept:
+// up to 3 % faster at widths 208 and 192 from k 3072 on (57.6 -> 55.4, 15.7 -> 15.4), 1 - 2 % slower at most others.
 constexpr int MAX_CHUNKS2 = (BN2_MAX / 16 + 1) / 2;         // of a tile and a warp
 constexpr int CHUNK2_BYTES = 16 * 64, STAGING2 = 8 * 2 * CHUNK2_BYTES;
-// barriers and flags behind the staging, so that no static shared memory shifts the (1024-byte aligned) start of the stages
+// Barriers and flags behind the staging, at addresses known at run time only.  With the same kernel's barriers in static shared
+// memory a K step takes about 30 ns longer where it is bound by latency; us, static -> here: fp16 ms 4096, k 3072, n 16 12.5 -> 11.5;
+// ms 1536, k 3072, n 4096 22.8 -> 21.5; float8 ms 256, k 3072, n 16 7.9 -> 7.5; over all shapes 3 % (fp16), 2 % (float8), 1 % (fused).
+// Where the stages start makes no difference, so it is the code of the loops.  One form is slower with it: the gelu epilogue at
+// k 3072 and 16384 tokens, ms 3072 170 -> 176, ms 4096 224 -> 234 (at k 768, or up to 4096 tokens, the same or faster).
 struct Ctl2 {
     uint64_t bars[2 * MAX_STAGES2 + 4];
     uint32_t tmem_base;
@@ -1028,9 +1036,9 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         // fragments, packed to 16 bits in registers (64 of them), and the accumulator goes back to the MMAs at once.  stmatrix then
         // writes the fragments token-major into the warp's two chunks of shared memory, from where 16-byte stores take them: 8 tokens
         // x 64 bytes an instruction instead of one token's 32 two-byte values.  What bounds it is the chip's writes, about 3.4 TB/s
-        // however they are issued (128-byte rows and TMA stores were no faster), shared with the operand fill.  fp16 / bf16, us,
-        // two-byte stores -> now: ms 3072, k 768, n 8192 27.2 -> 26.2; ms 2304 23.3 -> 21.7; ms 768, k 3072 23.7 -> 22.9;
-        // ms 4096, k 4096, n 2043 30.7 -> 29.5, n 16 14.4 -> 13.4.
+        // however they are issued (128-byte rows and TMA stores were no faster), shared with the operand fill: taken by itself it
+        // gains where many tiles are written, fp16 us, two-byte stores -> now: ms 3072, k 768, n 8192 28.0 -> 26.6, n 16384
+        // 50.0 -> 49.3; float8 ms 768, k 768, n 4096 7.5 -> 7.3; with few short tiles its chain costs up to 0.2 us (see Ctl2 for the rest).
         // Fused forms: a warp packs its BN / 2 columns of the accumulator into registers, hands the buffer back, then stores
         // 16-bit values directly; the 32 lanes of a store are 32 consecutive features of one token.
         const int quad = warp & 3, half = (warp - 2) >> 2;
@@ -1203,10 +1211,13 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 // so that the units fill the pairs; every unit adds its partial product with fp32 reductions in L2.  One
 // accumulator of 256 columns per CTA: a pair that owns more than one unit drains it before the next unit's MMAs.
 //
-// Epilogue: tensor memory -> shared memory -> TMA reductions of 16 rows x 32 columns.  Its cost is exposed (nothing is left to
-// multiply): 128 KB a CTA take about 2 us at the 32 bytes a clock that an SM writes.  red.global.add.v4 from the registers, 32
-// rows of 16 bytes an instruction, took 4 us even for one tile (64-byte rows: 0.6 us more than 128-byte ones); before -> now:
-// ms 512, n 256, k 256 9.5 -> 8.2 us; ms 3072, n 768, k 8192 / 16384 25.1 -> 22.1 / 40.7 -> 38.3 us; ms 768, n 768, k 8192 15.0 -> 11.9 us.
+// Epilogue: tensor memory -> shared memory -> TMA reductions of 16 rows x 32 columns.  Its cost is exposed where a pair has one unit
+// (nothing is left to multiply): under 3 us for a few tiles, 7 of 41 with all pairs writing at once (ms 3072, n 768, k 16384, by a
+// build without it), where the chip's writes bound it.  red.global.add.v4 from the registers, 32 rows of 16 bytes an instruction, took
+// 4 us even for one tile (64-byte rows: 0.6 us more than 128-byte ones).  us, before -> now, one unit per pair: ms 512, n 256, k 256
+// 9.5 -> 7.8; ms 768, n 768, k 8192 15.3 -> 11.8; ms 3072, n 768, k 8192 / 16384 24.6 -> 21.3 / 40.5 -> 37.4; several units (outputs
+// of more tiles than pairs, or given slices): ms 3072, n 3072, k 2048 / 8192 31.4 -> 25.4 / 80.6 -> 71.6; ms 4096, n 4096, k 2048
+// 67.2 -> 49.3; ms 512, n 512, k 16384 in 40 slices 29.6 -> 21.0.
 // Where every pair has one unit at most (any output up to 74 tiles) the operand ring is idle by then and holds the whole tile,
 // so that no chunk waits for another; a pair with more units stages chunk by chunk beside its ring, which is filling again.
 namespace two {
@@ -1644,12 +1655,13 @@ void pick_tile(int64_t ms, int64_t n, int sm_count, int &bn_out, int &mpt_out) {
 
 // Columns of a CTA-pair tile: the candidate with the lowest (rounds of tiles per CTA pair) x (bytes staged per CTA and K step).
 // The K loop is bound by the operand fill from L2 (about 14 TB/s over the chip whatever the width), so a wide tile pays only
-// where it does not leave the last round nearly empty.  fp16, us, at 192 columns -> at the width taken:
-//   ms 4096, n 2043, k 4096: 42.8 -> 33.5 (240 columns: two rounds instead of three)
-//   ms 3072, n 16384, k 768: 55.5 -> 52.0 (224); ms 768, n 16384, k 3072: 46.7 -> 43.4 (224)
-//   ms 768, n 5000, k 1024: 16.5 -> 12.5 (224)
-// Few columns: the narrowest tile that still takes one round; against the single-CTA kernel, which took these before,
-//   ms 4096, k 4096: n 16 21.6 -> 16.5, n 256 23.9 -> 18.4, n 512 28.0 -> 18.9, n 768 30.8 -> 20.1; ms 768, k 3072, n 512 18.9 -> 14.4
+// where it does not leave the last round nearly empty.  The number of stages is left out: one stage of five is worth 3 % at most,
+// and no other width makes up for it with the rounds it costs.  fp16, us, at 192 columns -> at the width taken:
+//   ms 4096, n 2043, k 4096: 39.3 -> 31.7 (240 columns: two rounds instead of three)
+//   ms 3072, n 16384, k 768: 52.2 -> 49.5 (224); ms 768, n 16384, k 3072: 44.5 -> 42.5 (224)
+//   ms 768, n 5000, k 1024: 11.8 -> 9.2 (224)
+// Few columns: the narrowest tile that still takes one round; single-CTA kernel -> here:
+//   ms 4096, k 4096: n 16 19.8 -> 13.2, n 256 20.8 -> 14.6, n 512 21.7 -> 15.5, n 768 24.0 -> 16.2; ms 768, k 3072, n 512 16.4 -> 11.5
 // (the single-CTA kernel was never faster, so it keeps the row counts that are odd multiples of 128 and the other layouts).
 // The fused epilogues hold up to 192 columns in registers and take them in chunks of 16 per half tile.  8-bit operands: with
 // cta_group::2 and M = 256, kind::f8f6f4 takes N in multiples of 32 (kind::f16, sparse: of 16; the ranges of CUTLASS's
