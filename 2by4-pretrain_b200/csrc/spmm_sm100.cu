@@ -1562,7 +1562,7 @@ int launch_spmm_pair(const CUtensorMap &ma, const CUtensorMap &mb, const CUtenso
         // the kernel takes its dynamic shared memory as it comes: it starts on 1024 bytes only behind none, or whole kilobytes, of
         // static shared memory
         cudaFuncAttributes fa{};
-        if (cudaFuncGetAttributes(&fa, kern) != cudaSuccess) return launch_status();
+        if (cudaFuncGetAttributes(&fa, kern) != cudaSuccess) return SP24_ERR_CUDA;
         if (fa.sharedSizeBytes % 1024) return SP24_ERR_ALIGN;
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX) != cudaSuccess)
             return SP24_ERR_CUDA;
