@@ -799,8 +799,9 @@ constexpr int CHUNK2_BYTES = 16 * 64, STAGING2 = 8 * 2 * CHUNK2_BYTES;
 // Barriers and flags behind the staging, at addresses known at run time only.  With the same kernel's barriers in static shared
 // memory a K step takes about 30 ns longer where it is bound by latency; us, static -> here: fp16 ms 4096, k 3072, n 16 12.5 -> 11.5;
 // ms 1536, k 3072, n 4096 22.8 -> 21.5; float8 ms 256, k 3072, n 16 7.9 -> 7.5; over all shapes 3 % (fp16), 2 % (float8), 1 % (fused).
-// Where the stages start makes no difference, so it is the code of the loops.  One form is slower with it: the gelu epilogue at
-// k 3072 and 16384 tokens, ms 3072 170 -> 176, ms 4096 224 -> 234 (at k 768, or up to 4096 tokens, the same or faster).
+// Where the stages start makes no difference, so it is the code of the loops.  One place is slower with it: the gelu epilogue at
+// k 3072 with 8192 tokens and more, 1 - 8 % (ms 4096, n 16384 229 -> 237; the same with operands of zeros, so not the power limit);
+// at k 2048 and 4096 the same sizes are 2 - 5 % faster (197 -> 192, 287 -> 286), at k 768 alike, so no rule on sizes follows.
 struct Ctl2 {
     uint64_t bars[2 * MAX_STAGES2 + 4];
     uint32_t tmem_base;
