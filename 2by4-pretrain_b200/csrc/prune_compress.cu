@@ -75,31 +75,52 @@ __device__ __forceinline__ void mode_uniform_pairs(uint64_t pair, uint64_t seed,
     else mvue_uniform_pairs(pair, seed, offset, u0a, u1a, u0b, u1b);
 }
 
-// Fast MVUE, after the arithmetic: q[] holds all four quotients, picks the two picks (first + 4 * second).  Emits the two
-// stored values and returns the 4-bit code.  16-bit outputs: round all four, then one table lookup (pick_lut, in shared
-// memory) and one byte permute gather the two stored ones.
+// Entry of the pick table (16 entries in shared memory): byte-permute selector that gathers the two stored values from the four
+// rounded quotients, and the metadata code.
+struct PickEntry { uint32_t sel, code; };
+__device__ __forceinline__ uint2 pick_entry(uint32_t addr) {      // written once, before a barrier
+    uint2 e;
+    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(e.x), "=r"(e.y) : "r"(addr));
+    return e;
+}
+// Two groups of the fast MVUE mode.  x[] as mvue24_two_groups_fast takes it.  The quotients are rounded (8-bit outputs: times the
+// caller's quantisation scale first, one more float32 rounding), then one table lookup and one byte permute a group gather the two
+// stored values into oa, ob (low 16 / 8 bits: the lower position).  Returns the two 4-bit codes, the second group's in bits 4..7.
 template <typename TOut>
-__device__ __forceinline__ uint32_t emit_fast(const float (&q)[4], uint32_t picks, TOut &o0, TOut &o1, const uint32_t *pick_lut,
-                                              float scale = 1.f) {
+__device__ __forceinline__ uint32_t two_groups_fast(float2 (&x)[4], float2 v0, float2 v1, uint32_t picks, float scale, uint32_t &oa, uint32_t &ob) {
+    const uint2 at = mvue24_two_groups_fast(x, v0, v1, picks);
+    const uint2 ea = pick_entry(at.x), eb = pick_entry(at.y);
     if constexpr (sizeof(TOut) == 2) {
-        const uint32_t e = pick_lut[picks];
-        const uint32_t o = __byte_perm(Elem<TOut>::pack2(q[0], q[1]), Elem<TOut>::pack2(q[2], q[3]), e >> 8);
-        const uint16_t lo = (uint16_t)(o & 0xFFFFu), hi = (uint16_t)(o >> 16);
-        o0 = *reinterpret_cast<const TOut *>(&lo);
-        o1 = *reinterpret_cast<const TOut *>(&hi);
-        return e & 0xFu;
+        oa = __byte_perm(Elem<TOut>::pack2(x[0].x, x[1].x), Elem<TOut>::pack2(x[2].x, x[3].x), ea.x);
+        ob = __byte_perm(Elem<TOut>::pack2(x[0].y, x[1].y), Elem<TOut>::pack2(x[2].y, x[3].y), eb.x);
     } else {
-        // 8-bit outputs: the caller's quantisation scale is applied before the cast (one more float32 rounding)
-        const uint32_t nib = encode_nibble(picks_to_keep(picks));
-        o0 = Elem<TOut>::from_f32(__fmul_rn(pick4(nib & 3u, q[0], q[1], q[2], q[3]), scale));
-        o1 = Elem<TOut>::from_f32(__fmul_rn(pick4(nib >> 2, q[0], q[1], q[2], q[3]), scale));
-        return nib;
+        static_assert(!std::is_same<TOut, int8_t>::value, "no integer form");
+        constexpr __nv_fp8_interpretation_t KIND = std::is_same<TOut, e5m2_t>::value ? __NV_E5M2 : __NV_E4M3;
+        const float2 sc = make_float2(scale, scale);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) x[j] = __fmul2_rn(x[j], sc);
+        auto two = [](float lo, float hi) { return (uint32_t)__nv_cvt_float2_to_fp8x2(make_float2(lo, hi), __NV_SATFINITE, KIND); };
+        oa = __byte_perm(two(x[0].x, x[1].x) | (two(x[2].x, x[3].x) << 16), 0u, ea.x);
+        ob = __byte_perm(two(x[0].y, x[1].y) | (two(x[2].y, x[3].y) << 16), 0u, eb.x);
     }
+    return ea.y + eb.y * 16u;
+}
+
+// One group of the fast MVUE mode with a 16-bit result, after the arithmetic: q[] holds all four quotients, picks the two picks
+// (first + 4 * second).  Round all four, then one table lookup (pick_lut, in shared memory) and one byte permute gather the stored two.
+template <typename TOut>
+__device__ __forceinline__ uint32_t emit_fast(const float (&q)[4], uint32_t picks, TOut &o0, TOut &o1, const uint32_t *pick_lut) {
+    const uint32_t e = pick_lut[picks];
+    const uint32_t o = __byte_perm(Elem<TOut>::pack2(q[0], q[1]), Elem<TOut>::pack2(q[2], q[3]), e >> 8);
+    const uint16_t lo = (uint16_t)(o & 0xFFFFu), hi = (uint16_t)(o >> 16);
+    o0 = *reinterpret_cast<const TOut *>(&lo);
+    o1 = *reinterpret_cast<const TOut *>(&hi);
+    return e & 0xFu;
 }
 
 // One group of four: decide the keep mask, emit the two stored values and the 4-bit code.
-// pick_lut: words 80..95 of the group table (indexed by the two picks of a draw) in shared memory; only the fast MVUE
-// mode with 16-bit outputs reads it.
+// pick_lut: words 80..95 of the group table (indexed by the two picks of a draw) in shared memory; only the fast MVUE mode, which
+// comes here with 16-bit results of row-major input, reads it.
 template <typename TIn, typename TOut, int MODE>
 __device__ __forceinline__ uint32_t do_group(const TIn (&in)[4], uint32_t given_mask, float u0, float u1, TOut &o0,
                                              TOut &o1, const uint32_t *pick_lut = nullptr, float scale = 1.f) {
@@ -107,10 +128,11 @@ __device__ __forceinline__ uint32_t do_group(const TIn (&in)[4], uint32_t given_
     constexpr bool SCALED = sizeof(TOut) == 1 && !std::is_same<TOut, int8_t>::value;
     uint32_t keep;
     if constexpr (MODE == SP24_PRUNE_MVUE_FAST) {
+        static_assert(sizeof(TOut) == 2, "8-bit results go two groups at a time");
         float x[4] = {Elem<TIn>::to_f32(in[0]), Elem<TIn>::to_f32(in[1]), Elem<TIn>::to_f32(in[2]),
                       Elem<TIn>::to_f32(in[3])};
         const uint32_t picks = mvue24_group_fast(x, u0, u1);         // all four quotients in x[]
-        return emit_fast<TOut>(x, picks, o0, o1, pick_lut, scale);
+        return emit_fast<TOut>(x, picks, o0, o1, pick_lut);
     } else if constexpr (MODE == SP24_PRUNE_MVUE) {
         float x[4] = {Elem<TIn>::to_f32(in[0]), Elem<TIn>::to_f32(in[1]), Elem<TIn>::to_f32(in[2]),
                       Elem<TIn>::to_f32(in[3])};
@@ -190,6 +212,27 @@ constexpr GroupLut make_group_lut() {
 }
 __constant__ GroupLut kGroupLut = make_group_lut();
 
+// Pick tables: indexed by the two picks of a draw, first + 4 * second; selectors over four 16-bit (0) or 8-bit (1) values.
+struct PickLut { uint32_t v[2][16][2]; };
+constexpr PickLut make_pick_lut() {
+    PickLut L{};
+    for (uint32_t k = 0; k < 16; ++k) {
+        const uint32_t w = lut_word_for_keep((1u << (k & 3u)) | (1u << (k >> 2))), code = w & 0xFu;
+        L.v[0][k][0] = w >> 8;
+        L.v[1][k][0] = (code & 3u) | (code >> 2) << 4 | 0x4400u;
+        L.v[0][k][1] = L.v[1][k][1] = code;
+    }
+    return L;
+}
+__constant__ PickLut kPickLut = make_pick_lut();
+template <typename TOut> __device__ __forceinline__ void load_pick_lut(PickEntry *to) {
+    if (threadIdx.x < 16) {
+        constexpr int which = sizeof(TOut) == 2 ? 0 : 1;
+        to[threadIdx.x] = PickEntry{kPickLut.v[which][threadIdx.x][0], kPickLut.v[which][threadIdx.x][1]};
+    }
+    __syncthreads();
+}
+
 template <typename T> struct Packed16;
 template <> struct Packed16<__half> {
     __device__ static uint32_t gt_mask(uint32_t a, uint32_t b) {
@@ -245,7 +288,9 @@ __global__ void __launch_bounds__(256, is_mvue(MODE) ? 3 : 1) pc_row_kernel(PcPa
     __shared__ __align__(16) MetaT smeta[16][64];
     constexpr bool PACKED = !is_mvue(MODE) && MODE != PRUNE_SOFT && std::is_same<TIn, TOut>::value && sizeof(TIn) == 2;
     constexpr bool PICK_LUT = MODE == SP24_PRUNE_MVUE_FAST && sizeof(TOut) == 2;   // words 80..95 only
+    constexpr bool PAIRS = MODE == SP24_PRUNE_MVUE_FAST && sizeof(TOut) == 1;      // two groups at a time
     __shared__ uint32_t glut[PACKED ? 80 : (PICK_LUT ? 16 : 1)];
+    __shared__ __align__(8) PickEntry picks[PAIRS ? 16 : 1];
     if constexpr (PACKED) {
         if (threadIdx.x < 80) glut[threadIdx.x] = kGroupLut.v[threadIdx.x];
         __syncthreads();
@@ -254,6 +299,8 @@ __global__ void __launch_bounds__(256, is_mvue(MODE) ? 3 : 1) pc_row_kernel(PcPa
         if (threadIdx.x < 16) glut[threadIdx.x] = kGroupLut.v[80 + threadIdx.x];
         __syncthreads();
     }
+    if constexpr (PAIRS) load_pick_lut<TOut>(picks);
+    const uint32_t picks_at = (uint32_t)__cvta_generic_to_shared(picks);
 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t ncols = P.k / CH;
@@ -277,7 +324,7 @@ __global__ void __launch_bounds__(256, is_mvue(MODE) ? 3 : 1) pc_row_kernel(PcPa
             for (int j = 0; j < RPI; ++j) {
                 const int rr = warp * 4 + it * RPI + j;
                 const int64_t r = r0 + rr;
-                TOut out[CH / 2];
+                alignas(16) TOut out[CH / 2];
                 uint32_t word = 0;
                 if constexpr (PACKED) {
                     // one table lookup and one byte permute per group of four
@@ -294,6 +341,19 @@ __global__ void __launch_bounds__(256, is_mvue(MODE) ? 3 : 1) pc_row_kernel(PcPa
                         }
                         o32[g] = __byte_perm(raw[2 * g], raw[2 * g + 1], e >> 8);
                         word |= (e & 0xFu) << (4 * g);
+                    }
+                } else if constexpr (PAIRS) {
+#pragma unroll
+                    for (int g2 = 0; g2 < CH / 8; ++g2) {
+                        const uint64_t gi = (uint64_t)r * (uint64_t)(P.k / 4) + (uint64_t)(c * (CH / 4) + g2 * 2);
+                        float2 v0, v1, x[4];
+                        mode_uniform_pairs<MODE>(gi >> 1, P.seed, rng_offset, v0.x, v1.x, v0.y, v1.y);
+#pragma unroll
+                        for (int e = 0; e < 4; ++e)
+                            x[e] = make_float2(Elem<TIn>::to_f32(in[j][8 * g2 + e]), Elem<TIn>::to_f32(in[j][8 * g2 + 4 + e]));
+                        uint32_t oa, ob;
+                        word += two_groups_fast<TOut>(x, v0, v1, picks_at, out_scale, oa, ob) << (8 * g2);
+                        reinterpret_cast<uint32_t *>(&out[0])[g2] = oa | (ob << 16);
                     }
                 } else
 #pragma unroll
@@ -382,20 +442,19 @@ template <typename TIn> struct ColVec {
     // Exact MVUE is bound by instruction issue, not by load width: one row per thread makes blocks of 32 rows, which
     // balances the SMs better on short matrices and is never slower on long ones.
     static constexpr int narrow = 1;
-    // Fast MVUE has a third of the arithmetic, so its loads and stores weigh more: four rows per thread (8-byte
-    // accesses for 16-bit inputs) is the fastest from 768 x 8192 to 4096 x 8192 (one / two rows: +7 % / +3 %).
-    static constexpr int fast = 4;
+    // Fast MVUE with 8-bit results: two rows, two groups at a time, three blocks per SM, where one group at a time took four rows at two
+    // blocks: the quantised bytes are gathered by one permute a group.  bf16 -> e4m3 with row sums and the quantised tensor, us:
+    // 3072 x 8192 49.9 -> 41.4, 768 x 8192 18.6 -> 13.9, 1024 x 1024 11.0 -> 6.8.
+    static constexpr int fast8 = 2;
 };
 
 // resident blocks per SM the register budget is set for
-constexpr int col_min_blocks(int mode, int out_bytes) {
-    // 8-bit outputs hold a row-major strip of packed bytes as well: 128 registers with 28 - 36 bytes of spills (16-bit input; none
-    // for float32) instead of 85 with 500
-    return mode == SP24_PRUNE_MVUE_FAST ? (out_bytes == 1 ? 2 : 3) : (mode == SP24_PRUNE_MVUE ? 4 : 1);
+constexpr int col_min_blocks(int mode) {
+    return mode == SP24_PRUNE_MVUE_FAST ? 3 : (mode == SP24_PRUNE_MVUE ? 4 : 1);
 }
 
 template <typename TIn, typename TOut, int MODE, bool HAS_U, int V>
-__global__ void __launch_bounds__(256, col_min_blocks(MODE, sizeof(TOut))) pc_col_kernel(PcParams P) {
+__global__ void __launch_bounds__(256, col_min_blocks(MODE)) pc_col_kernel(PcParams P) {
     const uint64_t rng_offset = P.offset + (P.offset_dev ? *P.offset_dev : 0ull);
     const float out_scale = out_scale_of<TOut>(P);
     constexpr int CH = sizeof(TOut) == 2 ? 16 : 32;
@@ -410,12 +469,10 @@ __global__ void __launch_bounds__(256, col_min_blocks(MODE, sizeof(TOut))) pc_co
     // (8-bit outputs: RT rows x 4 32-bit words = RT lines of each of two atoms)
     __shared__ __align__(16) MetaT stc[RT * 8];
     __shared__ float ssum[8][RT];           // per-warp partial row sums (only used when row sums are asked for)
-    constexpr bool PICK_LUT = MODE == SP24_PRUNE_MVUE_FAST && sizeof(TOut) == 2;
-    __shared__ uint32_t glut[PICK_LUT ? 16 : 1];
-    if constexpr (PICK_LUT) {
-        if (threadIdx.x < 16) glut[threadIdx.x] = kGroupLut.v[80 + threadIdx.x];
-        __syncthreads();
-    }
+    constexpr bool PAIRS = MODE == SP24_PRUNE_MVUE_FAST;      // two groups at a time, see ColVec
+    __shared__ __align__(8) PickEntry picks[PAIRS ? 16 : 1];
+    if constexpr (PAIRS) load_pick_lut<TOut>(picks);
+    const uint32_t picks_at = (uint32_t)__cvta_generic_to_shared(picks);
 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t ncols = P.k / CH;
@@ -438,7 +495,7 @@ __global__ void __launch_bounds__(256, col_min_blocks(MODE, sizeof(TOut))) pc_co
         constexpr bool CAN_RM = sizeof(TOut) == 1;
         constexpr bool CAN_Q = CAN_RM && !std::is_same<TOut, int8_t>::value;
         TOut *qdst = CAN_Q && P.q_dense ? static_cast<TOut *>(P.q_dense) + (c * CH) * P.ld_q + r : nullptr;
-        TOut orow[CAN_RM ? V : 1][CAN_RM ? CH / 2 : 1];
+        alignas(16) TOut orow[CAN_RM ? V : 1][CAN_RM ? CH / 2 : 1];
         // a step = 8 consecutive storage rows = two groups of four per logical row = one Philox block, counted along the row
         uint64_t pair0[V];
 #pragma unroll
@@ -466,58 +523,86 @@ __global__ void __launch_bounds__(256, col_min_blocks(MODE, sizeof(TOut))) pc_co
                     qdst += 8 * P.ld_q;
                 }
             }
-            if (P.row_sums) {   // sums of the unpruned values, fp32
+            if constexpr (PAIRS) {
+                uint32_t o[2][V];                // per group and row: the two stored values
 #pragma unroll
                 for (int v = 0; v < V; ++v) {
-                    float a = 0.f;
+                    float2 v0, v1, x[4];
+                    mode_uniform_pairs<MODE>(pair0[v] | step, P.seed, rng_offset, v0.x, v1.x, v0.y, v1.y);
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) a += Elem<TIn>::to_f32(in[j].v[v]);
-                    rsum[v] += a;
+                    for (int j = 0; j < 4; ++j) x[j] = make_float2(Elem<TIn>::to_f32(in[j].v[v]), Elem<TIn>::to_f32(in[4 + j].v[v]));
+                    if (P.row_sums) {   // sums of the unpruned values, fp32
+                        const float2 a = __fadd2_rn(__fadd2_rn(x[0], x[1]), __fadd2_rn(x[2], x[3]));
+                        rsum[v] += a.x + a.y;
+                    }
+                    word[v] += two_groups_fast<TOut>(x, v0, v1, picks_at, out_scale, o[0][v], o[1][v]) << (8 * step);
                 }
-            }
-            float u[V][4];
-            if constexpr (is_mvue(MODE)) {
-                const int64_t gcol = c * (CH / 4) + step * 2;  // first of the two groups
-                if constexpr (HAS_U) {
-                    float t0[V], t1[V], t2[V], t3[V];
-                    load_elems<float, V>(P.uniforms + (gcol * 4 + 0) * P.ld_u + r, t0);
-                    load_elems<float, V>(P.uniforms + (gcol * 4 + 1) * P.ld_u + r, t1);
-                    load_elems<float, V>(P.uniforms + (gcol * 4 + 4) * P.ld_u + r, t2);
-                    load_elems<float, V>(P.uniforms + (gcol * 4 + 5) * P.ld_u + r, t3);
+                static_assert(CAN_RM && V == 2, "8-bit results, two rows a thread");
 #pragma unroll
-                    for (int v = 0; v < V; ++v) { u[v][0] = t0[v]; u[v][1] = t1[v]; u[v][2] = t2[v]; u[v][3] = t3[v]; }
-                } else {
+                for (int v = 0; v < V; ++v) *reinterpret_cast<uint32_t *>(&orow[v][4 * step]) = o[0][v] | (o[1][v] << 16);
+                if (!P.packed_rm) {
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {       // the lower and the higher stored values of two rows
+                        const uint32_t both = __byte_perm(o[h][0], o[h][1], 0x5140u);
+                        *reinterpret_cast<uint16_t *>(dst) = (uint16_t)both;
+                        *reinterpret_cast<uint16_t *>(dst + P.ld_packed) = (uint16_t)(both >> 16);
+                        dst += 2 * P.ld_packed;
+                    }
+                }
+            } else {
+                if (P.row_sums) {   // sums of the unpruned values, fp32
 #pragma unroll
                     for (int v = 0; v < V; ++v) {
-                        mode_uniform_pairs<MODE>(pair0[v] + step, P.seed, rng_offset, u[v][0], u[v][1], u[v][2], u[v][3]);
+                        float a = 0.f;
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) a += Elem<TIn>::to_f32(in[j].v[v]);
+                        rsum[v] += a;
                     }
                 }
-            }
+                float u[V][4];
+                if constexpr (is_mvue(MODE)) {
+                    const int64_t gcol = c * (CH / 4) + step * 2;  // first of the two groups
+                    if constexpr (HAS_U) {
+                        float t0[V], t1[V], t2[V], t3[V];
+                        load_elems<float, V>(P.uniforms + (gcol * 4 + 0) * P.ld_u + r, t0);
+                        load_elems<float, V>(P.uniforms + (gcol * 4 + 1) * P.ld_u + r, t1);
+                        load_elems<float, V>(P.uniforms + (gcol * 4 + 4) * P.ld_u + r, t2);
+                        load_elems<float, V>(P.uniforms + (gcol * 4 + 5) * P.ld_u + r, t3);
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                Vec<TOut, V> o0, o1;
+                        for (int v = 0; v < V; ++v) { u[v][0] = t0[v]; u[v][1] = t1[v]; u[v][2] = t2[v]; u[v][3] = t3[v]; }
+                    } else {
 #pragma unroll
-                for (int v = 0; v < V; ++v) {
-                    const TIn grp[4] = {in[4 * h].v[v], in[4 * h + 1].v[v], in[4 * h + 2].v[v], in[4 * h + 3].v[v]};
-                    uint32_t given = 0;
-                    if constexpr (MODE == SP24_PRUNE_MASK) {
-                        given = (mk[4 * h].v[v] != 0) | ((mk[4 * h + 1].v[v] != 0) << 1) | ((mk[4 * h + 2].v[v] != 0) << 2) |
-                                ((mk[4 * h + 3].v[v] != 0) << 3);
-                    }
-                    float ua = 0.f, ub = 0.f;
-                    if constexpr (is_mvue(MODE)) { ua = u[v][2 * h]; ub = u[v][2 * h + 1]; }
-                    if constexpr (MODE == PRUNE_SOFT) { ua = P.soft_scale; ub = P.soft_use_scale ? 1.f : 0.f; }
-                    const uint32_t nib = do_group<TIn, TOut, MODE>(grp, given, ua, ub, o0.v[v], o1.v[v], glut, out_scale);
-                    word[v] |= nib << (4 * (step * 2 + h));
-                    if constexpr (CAN_RM) {
-                        orow[v][(step * 2 + h) * 2] = o0.v[v];
-                        orow[v][(step * 2 + h) * 2 + 1] = o1.v[v];
+                        for (int v = 0; v < V; ++v) {
+                            mode_uniform_pairs<MODE>(pair0[v] + step, P.seed, rng_offset, u[v][0], u[v][1], u[v][2], u[v][3]);
+                        }
                     }
                 }
-                if (!CAN_RM || !P.packed_rm) {
-                    store_vec<TOut, V>(dst, o0);
-                    store_vec<TOut, V>(dst + P.ld_packed, o1);
-                    dst += 2 * P.ld_packed;
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    Vec<TOut, V> o0, o1;
+#pragma unroll
+                    for (int v = 0; v < V; ++v) {
+                        const TIn grp[4] = {in[4 * h].v[v], in[4 * h + 1].v[v], in[4 * h + 2].v[v], in[4 * h + 3].v[v]};
+                        uint32_t given = 0;
+                        if constexpr (MODE == SP24_PRUNE_MASK) {
+                            given = (mk[4 * h].v[v] != 0) | ((mk[4 * h + 1].v[v] != 0) << 1) | ((mk[4 * h + 2].v[v] != 0) << 2) |
+                                    ((mk[4 * h + 3].v[v] != 0) << 3);
+                        }
+                        float ua = 0.f, ub = 0.f;
+                        if constexpr (is_mvue(MODE)) { ua = u[v][2 * h]; ub = u[v][2 * h + 1]; }
+                        if constexpr (MODE == PRUNE_SOFT) { ua = P.soft_scale; ub = P.soft_use_scale ? 1.f : 0.f; }
+                        const uint32_t nib = do_group<TIn, TOut, MODE>(grp, given, ua, ub, o0.v[v], o1.v[v], nullptr, out_scale);
+                        word[v] |= nib << (4 * (step * 2 + h));
+                        if constexpr (CAN_RM) {
+                            orow[v][(step * 2 + h) * 2] = o0.v[v];
+                            orow[v][(step * 2 + h) * 2 + 1] = o1.v[v];
+                        }
+                    }
+                    if (!CAN_RM || !P.packed_rm) {
+                        store_vec<TOut, V>(dst, o0);
+                        store_vec<TOut, V>(dst + P.ld_packed, o1);
+                        dst += 2 * P.ld_packed;
+                    }
                 }
             }
         }
@@ -606,14 +691,215 @@ __global__ void __launch_bounds__(256, col_min_blocks(MODE, sizeof(TOut))) pc_co
     }
 }
 
+// ---------------------------------------------------------------------------------------------
+// Fast MVUE, column-major storage, 16-bit results: dY^T, the sparse operand of every weight-gradient GEMM.
+// ---------------------------------------------------------------------------------------------
+// Bound by arithmetic: about 80 instructions a group of four for the draws, quotients and random numbers, which by themselves (operands
+// in shared memory, no traffic) take 115 cycles a warp and group, 67 % of the time measured here; the rest are copies, addresses and
+// metadata.  So: persistent blocks, whose warps fetch their 16 columns of the next two tiles by asynchronous copies (no registers hold
+// loads, no warp waits at the start of a block), compressed rows written over the storage rows that the same lane has read and stored
+// 16 bytes a lane, one barrier a tile (for the metadata, which eight warps assemble), and two groups at a time in two-lane arithmetic.
+// Two blocks of 128 registers: with three (80) or four (64) the loop's constants no longer fit and the same work is 106 and 109
+// instructions a group instead of 98.  us, one group at a time in a block per tile -> here: bf16 4096 x 8192 45.7 -> 39.4, fp16
+// 3072 x 16384 64.1 -> 56.8, bf16 with row sums 3072 x 8192 38.0 -> 31.7, 768 x 8192 12.5 -> 11.1, fp16 512 x 256 5.5 -> 3.7.
+// Three or four stages of copies instead of two, and tiles of two or four 16-column slices a warp, gained nothing.
+template <typename TIn> struct MvueCol {
+    static constexpr int RT = 64, KT = 128;                      // a tile: rows x logical columns; a warp takes 16 of the columns
+    static constexpr int ROW = RT * sizeof(TIn);                 // bytes of one storage row of a tile
+    static constexpr int SLICE = 16 * ROW, STAGES = 2;           // a warp's share, and how many of them are under way
+    static constexpr int RUN = 0, LINE = 4 * 2 * RT * 2, SUMS = LINE + RT * 16, OUT = SUMS + 8 * RT * 4;     // staged results
+    static constexpr int SMEM = STAGES * 8 * SLICE + 2 * OUT;
+    static constexpr int BLOCKS = 2;
+};
+
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+// Keeps a value that a loop needs in its register: worked out anew in every pass, such values cost more than the arithmetic they serve.
+template <typename T> __device__ __forceinline__ void pin(T &v) {
+    if constexpr (sizeof(T) == 8) asm volatile("" : "+l"(v));
+    else asm volatile("" : "+r"(v));
+}
+__device__ __forceinline__ void st_shared16(uint32_t addr, uint32_t v) { asm volatile("st.shared.u16 [%0], %1;" ::"r"(addr), "h"((uint16_t)v) : "memory"); }
+
+template <typename TIn, typename TOut>
+__global__ void __launch_bounds__(256, MvueCol<TIn>::BLOCKS)
+mvue_col_kernel(const __grid_constant__ PcParams P, const __grid_constant__ PhiloxKeys<kMvueFastRounds> keys) {
+    using Cfg = MvueCol<TIn>;
+    constexpr int RT = Cfg::RT, ROW = Cfg::ROW, STAGES = Cfg::STAGES, V = 2;
+    extern __shared__ __align__(16) uint8_t smem[];
+    __shared__ __align__(8) PickEntry picks[16];
+    load_pick_lut<TOut>(picks);
+    const uint32_t picks_at = (uint32_t)__cvta_generic_to_shared(picks);
+    const uint64_t rng_offset = P.offset + (P.offset_dev ? *P.offset_dev : 0ull);
+
+    const int lane = threadIdx.x & 31, warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0);
+    const int m = (int)P.m, ncols = (int)(P.k / 16);
+    const int n_rt = (m + RT - 1) / RT, n_ct = (ncols + 7) / 8;
+    // tile -> (row tile, column tile), the row tile varying fastest; both advance by the grid without a division
+    const int grid_r = (int)(gridDim.x % n_rt), grid_c = (int)(gridDim.x / n_rt);
+    auto advance = [&](int &tr, int &tc) {
+        tr += grid_r;
+        tc += grid_c;
+        if (tr >= n_rt) { tr -= n_rt; ++tc; }
+    };
+    // asynchronous copies of a slice's 16 storage rows, 16 bytes a lane and copy
+    constexpr int PIECES = ROW / 16, AT_ONCE = 32 / PIECES;
+    const uint32_t ld_in = (uint32_t)P.ld_dense * (uint32_t)sizeof(TIn), ld_out = (uint32_t)P.ld_packed * 2u;      // bytes
+    uint8_t *const slices = smem + warp * (STAGES * Cfg::SLICE);
+    uint32_t fetch_to = (uint32_t)__cvta_generic_to_shared(slices) + lane * 16;
+    const char *fetch_from = static_cast<const char *>(P.dense) + (uint64_t)(lane / PIECES) * ld_in + lane % PIECES * 16;
+    int fetch_row = lane % PIECES * (16 / (int)sizeof(TIn));
+    pin(fetch_to);
+    pin(fetch_from);
+    pin(fetch_row);
+    int ftr = blockIdx.x % n_rt, ftc = blockIdx.x / n_rt;
+    auto fetch = [&](int buf) {
+        const int c = ftc * 8 + warp;
+        if (fetch_row + ftr * RT < m && c < ncols) {
+            const char *src = fetch_from + ((uint64_t)(uint32_t)(c * 16) * ld_in + (uint32_t)(ftr * ROW));
+#pragma unroll
+            for (int i = 0; i < 16 / AT_ONCE; ++i, src += (uint64_t)AT_ONCE * ld_in) cp_async16(fetch_to + buf * Cfg::SLICE + i * 512, src);
+        }
+        cp_async_commit();
+        advance(ftr, ftc);
+    };
+    // where a lane's two words go in the staged metadata (the second 8 words behind the first in both orders), and its 16 bytes of the
+    // stored rows
+    const int rr = lane * V;
+    uint32_t run_at = (uint32_t)__cvta_generic_to_shared(smem + STAGES * 8 * Cfg::SLICE) + Cfg::RUN +
+                      2 * ((warp >> 1) * 2 * RT + (rr / 32) * 64 + meta_run_pos<2>(rr % 32, warp & 1));
+    uint32_t line_at = (uint32_t)__cvta_generic_to_shared(smem + STAGES * 8 * Cfg::SLICE) + Cfg::LINE +
+                       2 * (8 * (16 * (rr >> 4) + 8 * (warp & 1) + (rr & 7)) + 2 * (warp >> 1) + ((rr >> 3) & 1));
+    char *store_to = static_cast<char *>(P.packed) + (uint64_t)(lane >> 3) * ld_out + (lane & 7) * 16;
+    pin(run_at);
+    pin(line_at);
+    pin(store_to);
+
+    for (int i = 0; i < STAGES; ++i) fetch(i);
+    int tr = blockIdx.x % n_rt, tc = blockIdx.x / n_rt, buf = 0;
+    uint32_t out_off = 0;
+    const uint32_t row_pairs = (uint32_t)(P.k / 8);
+#pragma unroll 1
+    for (; tc < n_ct; advance(tr, tc)) {
+        const int r0 = tr * RT, c = tc * 8 + warp;
+        uint8_t *const sl = slices + buf * Cfg::SLICE;
+        cp_async_wait<STAGES - 1>();
+        __syncwarp();
+        uint32_t word[V] = {0, 0};
+        float rsum[V] = {0.f, 0.f};
+        if (r0 + lane * V < m && c < ncols) {
+            uint64_t pair[V];
+            pair[0] = (uint64_t)(uint32_t)(r0 + lane * V) * row_pairs + (uint32_t)(c * 2);
+            pair[1] = pair[0] + row_pairs;
+#pragma unroll
+            for (int step = 0; step < 2; ++step) {
+                Vec<TIn, V> in[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) in[j] = load_vec<TIn, V>(reinterpret_cast<const TIn *>(sl + (8 * step + j) * ROW) + lane * V);
+                uint32_t o[2][V];
+#pragma unroll
+                for (int v = 0; v < V; ++v) {
+                    // the count of blocks before the slice is even: K is a multiple of 64
+                    const uint4 u = philox4x32<kMvueFastRounds>(make_uint4((uint32_t)pair[v] | step, (uint32_t)(pair[v] >> 32), (uint32_t)rng_offset, (uint32_t)(rng_offset >> 32)), keys);
+                    const float2 v0 = make_float2(u32_to_one_plus_uniform(u.x), u32_to_one_plus_uniform(u.z));
+                    const float2 v1 = make_float2(u32_to_one_plus_uniform(u.y), u32_to_one_plus_uniform(u.w));
+                    float2 x[4];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) x[j] = make_float2(Elem<TIn>::to_f32(in[j].v[v]), Elem<TIn>::to_f32(in[4 + j].v[v]));
+                    if (P.row_sums) {   // sums of the unpruned values, fp32
+                        const float2 a = __fadd2_rn(__fadd2_rn(x[0], x[1]), __fadd2_rn(x[2], x[3]));
+                        rsum[v] += a.x + a.y;
+                    }
+                    word[v] += two_groups_fast<TOut>(x, v0, v1, picks_at, 1.f, o[0][v], o[1][v]) << (8 * step);
+                }
+                // stored rows take the place of the storage rows that this lane has read
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    uint32_t *to = reinterpret_cast<uint32_t *>(sl + (4 * step + 2 * h) * 128) + lane;
+                    to[0] = __byte_perm(o[h][0], o[h][1], 0x5410u);
+                    to[32] = __byte_perm(o[h][0], o[h][1], 0x7632u);
+                }
+            }
+        }
+        // word columns past the matrix (K not a multiple of 128) are zeros in the tensor-core copy: the GEMM multiplies them by
+        // zero-filled operands
+        st_shared16(run_at + out_off, word[0]);
+        st_shared16(run_at + out_off + 16, word[1]);
+        st_shared16(line_at + out_off, word[0]);
+        st_shared16(line_at + out_off + 16, word[1]);
+        if (P.row_sums) *reinterpret_cast<float2 *>(smem + STAGES * 8 * Cfg::SLICE + out_off + Cfg::SUMS + (warp * RT + rr) * 4) = make_float2(rsum[0], rsum[1]);
+        __syncwarp();
+        if (r0 + (lane & 7) * 8 < m && c < ncols) {       // 8 rows of 128 bytes, 16 bytes a lane and store
+            char *dst = store_to + ((uint64_t)(uint32_t)(c * 8) * ld_out + (uint32_t)(r0 * 2));
+            *reinterpret_cast<uint4 *>(dst) = *reinterpret_cast<const uint4 *>(sl + lane * 16);
+            *reinterpret_cast<uint4 *>(dst + 4ull * ld_out) = *reinterpret_cast<const uint4 *>(sl + 512 + lane * 16);
+        }
+        __syncwarp();
+        fetch(buf);
+        if (++buf == STAGES) buf = 0;
+        __syncthreads();
+        // metadata and row sums of the tile, one piece a thread; the next tile's are staged in the other buffer, and nobody is two
+        // tiles ahead
+        const uint8_t *out = smem + STAGES * 8 * Cfg::SLICE + out_off;
+        const int t = threadIdx.x & 63, rows_here = m - r0;
+        if (warp < 2) {
+            // 4 column pairs x 2 RT words
+            const int cp = tc * 4 + (t >> 4), pc = t & 15;
+            if (pc * 4 < rows_here && cp * 2 < ncols)
+                *reinterpret_cast<uint4 *>(static_cast<char *>(P.meta) + ((uint64_t)(uint32_t)cp * (uint32_t)m + (uint32_t)r0) * 4 + pc * 16) =
+                    *reinterpret_cast<const uint4 *>(out + Cfg::RUN + t * 16);
+        } else if (warp < 4) {
+            const int gr = r0 + t;    // line index inside the 128-row block = row index of its first writer
+            if (P.tc && t < rows_here) {
+                const int64_t off = ((gr >> 7) * P.k_atoms + tc) * 2048 + (gr & 127) * 16;
+                if (off + 16 <= (P.m >> 7) * P.k_atoms * 2048)   // every store is checked against the buffer size
+                    *reinterpret_cast<uint4 *>(reinterpret_cast<char *>(P.tc) + off) = *reinterpret_cast<const uint4 *>(out + Cfg::LINE + t * 16);
+            }
+        } else if (warp < 6) {
+            if (P.row_sums && t < rows_here) {
+                const float *ssum = reinterpret_cast<const float *>(out + Cfg::SUMS);
+                float a = 0.f;
+#pragma unroll
+                for (int w = 0; w < 8; ++w) a += ssum[w * RT + t];
+                if (P.ld_sums) P.row_sums[tc * P.ld_sums + r0 + t] = a;
+                else atomicAdd(P.row_sums + r0 + t, a);
+            }
+        }
+        out_off ^= Cfg::OUT;
+    }
+    cp_async_wait<0>();
+}
+
+// Lets a kernel take more than 48 KB of dynamic shared memory, once per kernel and device.
+template <auto KERN> int allow_shared_memory(int bytes) {
+    static bool done[64];
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64 || !done[dev]) {
+        if (cudaFuncSetAttribute(KERN, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) return SP24_ERR_CUDA;
+        if (dev >= 0 && dev < 64) done[dev] = true;
+    }
+    return SP24_OK;
+}
+
 template <typename TIn, typename TOut, int MODE, bool HAS_U>
 int launch(const PcParams &P, int col_major, cudaStream_t st) {
     constexpr int CH = sizeof(TOut) == 2 ? 16 : 32;
     if (!col_major) {
         dim3 grid((unsigned)((P.k / CH + 31) / 32), (unsigned)(P.m / 32));
         pc_row_kernel<TIn, TOut, MODE, HAS_U><<<grid, 256, 0, st>>>(P);
+    } else if constexpr (MODE == SP24_PRUNE_MVUE_FAST && sizeof(TOut) == 2) {
+        using Cfg = MvueCol<TIn>;
+        constexpr auto kern = mvue_col_kernel<TIn, TOut>;
+        if (int rc = allow_shared_memory<mvue_col_kernel<TIn, TOut>>(Cfg::SMEM)) return rc;
+        const int64_t tiles = ((P.m + Cfg::RT - 1) / Cfg::RT) * ((P.k / 16 + 7) / 8), most = (int64_t)sm_count() * Cfg::BLOCKS;
+        kern<<<(unsigned)(tiles < most ? tiles : most), 256, Cfg::SMEM, st>>>(P, PhiloxKeys<kMvueFastRounds>(P.seed));
     } else {
-        constexpr int V = MODE == SP24_PRUNE_MVUE_FAST ? ColVec<TIn>::fast : (MODE == SP24_PRUNE_MVUE ? ColVec<TIn>::narrow : ColVec<TIn>::wide);
+        constexpr int V = MODE == SP24_PRUNE_MVUE_FAST ? ColVec<TIn>::fast8
+                                                       : (MODE == SP24_PRUNE_MVUE ? ColVec<TIn>::narrow : ColVec<TIn>::wide);
         constexpr int RT = 32 * V;
         dim3 grid((unsigned)((P.m + RT - 1) / RT), (unsigned)((P.k / CH + 7) / 8));
         pc_col_kernel<TIn, TOut, MODE, HAS_U, V><<<grid, 256, 0, st>>>(P);

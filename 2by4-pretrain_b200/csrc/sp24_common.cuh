@@ -162,16 +162,36 @@ template <int META_BYTES> __device__ __forceinline__ int meta_run_pos(int rr, in
 // ---------------------------------------------------------------------------------------------
 // Philox4x32 with ROUNDS rounds: 10 for the exact MVUE mode; 7 (the fewest rounds Salmon et al. report as passing
 // BigCrush) for the fast mode.  The reference draws with five (tl.rand4x(..., n_rounds=5)).
+__device__ __forceinline__ uint4 philox_round(uint4 c, uint32_t k0, uint32_t k1) {
+    // both halves of a product from one wide multiplication (written as two, they are two instructions)
+    uint32_t hi0, lo0, hi1, lo1;
+    asm("{\n\t.reg .b64 t;\n\tmul.wide.u32 t, %2, %3;\n\tmov.b64 {%0, %1}, t;\n\t}" : "=r"(lo0), "=r"(hi0) : "r"(c.x), "n"(0xD2511F53u));
+    asm("{\n\t.reg .b64 t;\n\tmul.wide.u32 t, %2, %3;\n\tmov.b64 {%0, %1}, t;\n\t}" : "=r"(lo1), "=r"(hi1) : "r"(c.z), "n"(0xCD9E8D57u));
+    return make_uint4(hi1 ^ c.y ^ k0, lo1, hi0 ^ c.w ^ k1, lo0);
+}
 template <int ROUNDS = 10> __device__ __forceinline__ uint4 philox4x32(uint4 c, uint2 k) {
-    constexpr uint32_t M0 = 0xD2511F53u, M1 = 0xCD9E8D57u, W0 = 0x9E3779B9u, W1 = 0xBB67AE85u;
 #pragma unroll
     for (int i = 0; i < ROUNDS; ++i) {
-        const uint32_t hi0 = __umulhi(M0, c.x), lo0 = M0 * c.x;
-        const uint32_t hi1 = __umulhi(M1, c.z), lo1 = M1 * c.z;
-        c = make_uint4(hi1 ^ c.y ^ k.x, lo1, hi0 ^ c.w ^ k.y, lo0);
-        k.x += W0;
-        k.y += W1;
+        c = philox_round(c, k.x, k.y);
+        k.x += 0x9E3779B9u;
+        k.y += 0xBB67AE85u;
     }
+    return c;
+}
+// The same with the round keys worked out beforehand (two words a round): kept in a kernel's parameters they are constant operands,
+// where the schedule above takes two instructions of the uniform path a round.
+template <int ROUNDS> struct PhiloxKeys {
+    uint32_t k[2 * ROUNDS];
+    __host__ __device__ explicit PhiloxKeys(uint64_t seed = 0) {
+        for (int i = 0; i < ROUNDS; ++i) {
+            k[2 * i] = (uint32_t)seed + (uint32_t)i * 0x9E3779B9u;
+            k[2 * i + 1] = (uint32_t)(seed >> 32) + (uint32_t)i * 0xBB67AE85u;
+        }
+    }
+};
+template <int ROUNDS> __device__ __forceinline__ uint4 philox4x32(uint4 c, const PhiloxKeys<ROUNDS> &keys) {
+#pragma unroll
+    for (int i = 0; i < ROUNDS; ++i) c = philox_round(c, keys.k[2 * i], keys.k[2 * i + 1]);
     return c;
 }
 
@@ -316,6 +336,54 @@ __device__ __forceinline__ uint32_t mvue24_group_fast(float (&x)[4], float v0, f
     x[2] = __fmul_rn(x[2], __fmul_rn(s, rcp_fast(__fmaf_rn(a2, __fadd_rn(r01, r3), a2))));
     x[3] = __fmul_rn(x[3], __fmul_rn(s, rcp_fast(__fmaf_rn(a3, __fadd_rn(r01, r2), a3))));
     return f + g;
+}
+// The same arithmetic, bit for bit, for two groups at once: .x of every operand belongs to the first group, .y to the second.  Sums,
+// multiply-adds and most products are the two-lane instructions of sm_100: half the issue slots, the same time on the FMA pipe.  The
+// draws are counted instead of selected: a passed threshold is 1.0, the first pick's weight is taken out by products with 0 or 1 (NaN
+// where an infinity is behind the first position, which makes the second uniform NaN in the form above too), and the picks are added up as denormal floats, whose bits are the
+// shared-memory address of the pick's table entry.  That leaves 7 instead of 19 instructions a group to the integer pipe, the busiest
+// one with the form above (64 % of its rate at 73 % of the issue slots); the whole is 47 instructions a group instead of 64.
+__device__ __forceinline__ float passed(float v, float limit) {      // 1.0 or 0.0
+    float r;
+    asm("set.gt.f32.f32 %0, %1, %2;" : "=f"(r) : "f"(v), "f"(limit));
+    return r;
+}
+// at: address of entry 0; returns the addresses of the two groups' entries (8 bytes each, entry first + 4 * second)
+__device__ __forceinline__ uint2 mvue24_two_groups_fast(float2 (&x)[4], float2 v0, float2 v1, uint32_t at) {
+    const float eps = 1.19209e-07f;
+    auto abs_eps = [&](float2 v) { return make_float2(__fadd_rn(fabsf(v.x), eps), __fadd_rn(fabsf(v.y), eps)); };
+    auto rcp2 = [](float2 v) { return make_float2(rcp_fast(v.x), rcp_fast(v.y)); };
+    // scalar products: a two-lane one that feeds a two-lane sum is fused with it, which is one float32 ulp off the form above
+    auto times = [](float2 a, float2 b) { return make_float2(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y)); };
+    auto neg = [](float2 v) { return make_float2(-v.x, -v.y); };
+    auto scaled = [&](float2 v, float2 s_) { return __ffma2_rn(v, s_, neg(s_)); };
+    auto above = [](float2 v, float2 limit) { return make_float2(passed(v.x, limit.x), passed(v.y, limit.y)); };
+    auto both = [](float v) { return make_float2(v, v); };
+    const float2 a0 = abs_eps(x[0]), a1 = abs_eps(x[1]), a2 = abs_eps(x[2]), a3 = abs_eps(x[3]);
+    const float2 a01 = __fadd2_rn(a0, a1), a23 = __fadd2_rn(a2, a3);
+    const float2 s = __fadd2_rn(a01, a23), a012 = __fadd2_rn(a01, a2);
+    const float2 r0 = times(a0, rcp2(__fadd2_rn(a1, a23))), r1 = times(a1, rcp2(__fadd2_rn(a0, a23)));
+    const float2 r2 = times(a2, rcp2(__fadd2_rn(a01, a3))), r3 = times(a3, rcp2(a012));
+    const float2 r01 = __fadd2_rn(r0, r1), r23 = __fadd2_rn(r2, r3);
+    const float2 w = scaled(v0, s);
+    const float2 t0 = above(w, a0), t1 = above(w, a01), t2 = above(w, a012);     // not increasing
+    const float2 most = __fmul2_rn(t0, both(3.4028235e38f));       // an infinite or NaN a0 is never passed: minima, not products
+    const float2 d0 = make_float2(fminf(a0.x, most.x), fminf(a0.y, most.y)), d1 = __ffma2_rn(__fadd2_rn(t1, neg(t0)), a1, a1);
+    const float2 d2 = __ffma2_rn(__fadd2_rn(t2, neg(t1)), a2, a2), d3 = __ffma2_rn(neg(t2), a3, a3);
+    const float2 d01 = __fadd2_rn(d0, d1), d012 = __fadd2_rn(d01, d2), ds = __fadd2_rn(d012, d3);
+    const float2 w2 = scaled(v1, ds);
+    const float2 e8 = both(__uint_as_float(8u)), e32 = both(__uint_as_float(32u));
+    float2 p = __ffma2_rn(t0, e8, both(__uint_as_float(at)));
+    p = __ffma2_rn(t1, e8, p);
+    p = __ffma2_rn(t2, e8, p);
+    p = __ffma2_rn(above(w2, d0), e32, p);
+    p = __ffma2_rn(above(w2, d01), e32, p);
+    p = __ffma2_rn(above(w2, d012), e32, p);
+    x[0] = __fmul2_rn(x[0], __fmul2_rn(s, rcp2(__ffma2_rn(a0, __fadd2_rn(r1, r23), a0))));
+    x[1] = __fmul2_rn(x[1], __fmul2_rn(s, rcp2(__ffma2_rn(a1, __fadd2_rn(r0, r23), a1))));
+    x[2] = __fmul2_rn(x[2], __fmul2_rn(s, rcp2(__ffma2_rn(a2, __fadd2_rn(r01, r3), a2))));
+    x[3] = __fmul2_rn(x[3], __fmul2_rn(s, rcp2(__ffma2_rn(a3, __fadd2_rn(r01, r2), a3))));
+    return make_uint2(__float_as_uint(p.x), __float_as_uint(p.y));
 }
 __device__ __forceinline__ uint32_t picks_to_keep(uint32_t picks) { return (1u << (picks & 3u)) | (1u << (picks >> 2)); }
 
