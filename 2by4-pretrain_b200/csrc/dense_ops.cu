@@ -54,6 +54,7 @@ __device__ __forceinline__ void dense_group(const T (&in)[4], float u0, float u1
 
 // row-major: one item = 8 consecutive elements of a row (two groups, one Philox block).
 template <typename T, int OP, bool HAS_U> __global__ void __launch_bounds__(256) dense_row_kernel(DenseParams P) {
+    chain_enter();
     constexpr int ITEMS = 2;
     const int64_t per_row = P.k / 8;
     const int64_t total = P.m * per_row;
@@ -123,6 +124,7 @@ template <typename T, int OP, bool HAS_U> __global__ void __launch_bounds__(256)
 
 // column-major storage: element (r, c) at c*ld + r; thread = V consecutive r x 8 storage rows.
 template <typename T, int OP, bool HAS_U> __global__ void __launch_bounds__(256) dense_col_kernel(DenseParams P) {
+    chain_enter();
     constexpr int V = 16 / sizeof(T);
     const int64_t r = ((int64_t)blockIdx.x * 256 + threadIdx.x) * V;
     const int64_t c8 = (int64_t)blockIdx.y * 8;
@@ -182,11 +184,11 @@ template <typename T, int OP, bool HAS_U> __global__ void __launch_bounds__(256)
 template <typename T, int OP, bool HAS_U> int launch_dense(const DenseParams &P, int col_major, cudaStream_t st) {
     if (!col_major) {
         const int64_t total = P.m * (P.k / 8);
-        dense_row_kernel<T, OP, HAS_U><<<(unsigned)((total + 511) / 512), 256, 0, st>>>(P);
+        launch_chained(st, dense_row_kernel<T, OP, HAS_U>, (unsigned)((total + 511) / 512), 256, 0, P);
     } else {
         constexpr int V = 16 / sizeof(T);
         dim3 grid((unsigned)((P.m / V + 255) / 256), (unsigned)(P.k / 8));
-        dense_col_kernel<T, OP, HAS_U><<<grid, 256, 0, st>>>(P);
+        launch_chained(st, dense_col_kernel<T, OP, HAS_U>, grid, 256, 0, P);
     }
     return launch_status();
 }
@@ -226,6 +228,7 @@ int check_dense_args(const void *x, int dtype, int64_t m, int64_t k, int64_t ld_
 template <typename T> __global__ void __launch_bounds__(256) to_dense_kernel(const T *packed, const void *meta, T *dense,
                                                                               int64_t m, int64_t k, int64_t ld_p,
                                                                               int64_t ld_d) {
+    chain_enter();
     constexpr int CH = sizeof(T) == 2 ? 16 : 32;
     constexpr int MB = sizeof(T) == 2 ? 2 : 4;
     using MetaT = typename VecBytes<MB>::type;
@@ -287,6 +290,7 @@ template <int MS> __device__ __forceinline__ uint32_t load_keep4(const void *mas
 template <int MS>
 __global__ void __launch_bounds__(256) masked_add_kernel(float *grad, const float *p, const void *mask, int64_t n,
                                                          float alpha) {
+    chain_enter();
     constexpr int UNR = 4;
     const int64_t n4 = n / 4;
     const int64_t base = (int64_t)blockIdx.x * (256 * UNR) + threadIdx.x;
@@ -378,11 +382,11 @@ extern "C" int sp24_to_dense(const void *packed, int dtype, int64_t m, int64_t k
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (sz == 2) {
         const int64_t total = m * (k / 16);
-        to_dense_kernel<uint16_t><<<(unsigned)((total + 255) / 256), 256, 0, st>>>(
+        launch_chained(st, to_dense_kernel<uint16_t>, (unsigned)((total + 255) / 256), 256, 0,
             static_cast<const uint16_t *>(packed), meta, static_cast<uint16_t *>(dense), m, k, ld_packed, ld_dense);
     } else {
         const int64_t total = m * (k / 32);
-        to_dense_kernel<uint8_t><<<(unsigned)((total + 255) / 256), 256, 0, st>>>(
+        launch_chained(st, to_dense_kernel<uint8_t>, (unsigned)((total + 255) / 256), 256, 0,
             static_cast<const uint8_t *>(packed), meta, static_cast<uint8_t *>(dense), m, k, ld_packed, ld_dense);
     }
     return launch_status();
@@ -402,9 +406,9 @@ extern "C" int sp24_masked_add(void *grad, const void *p, const void *mask, int 
     const unsigned blocks = (unsigned)((n4 + 1023) / 1024 > 0 ? (n4 + 1023) / 1024 : 1);
     float *g = static_cast<float *>(grad);
     const float *q = static_cast<const float *>(p);
-    if (mask_itemsize == 1) masked_add_kernel<1><<<blocks, 256, 0, st>>>(g, q, mask, n, alpha);
-    else if (mask_itemsize == 2) masked_add_kernel<2><<<blocks, 256, 0, st>>>(g, q, mask, n, alpha);
-    else masked_add_kernel<4><<<blocks, 256, 0, st>>>(g, q, mask, n, alpha);
+    if (mask_itemsize == 1) launch_chained(st, masked_add_kernel<1>, blocks, 256, 0, g, q, mask, n, alpha);
+    else if (mask_itemsize == 2) launch_chained(st, masked_add_kernel<2>, blocks, 256, 0, g, q, mask, n, alpha);
+    else launch_chained(st, masked_add_kernel<4>, blocks, 256, 0, g, q, mask, n, alpha);
     return launch_status();
 }
 
@@ -428,6 +432,7 @@ template <typename T> __device__ __forceinline__ uint32_t abs_bits_max(const uin
 
 template <typename T, bool MASK>
 __global__ void __launch_bounds__(256) absmax_kernel(const uint4 *x, const uint32_t *mask, float *amax, int64_t nvec) {
+    chain_enter();
     uint32_t m = 0;
     const int64_t stride = (int64_t)gridDim.x * 256;
     for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < nvec; i += 4 * stride) {
@@ -470,6 +475,7 @@ __global__ void __launch_bounds__(256) absmax_kernel(const uint4 *x, const uint3
 template <typename T>
 __global__ void __launch_bounds__(256) quantize_f8_kernel(const T *x, int64_t rows, int64_t cols, int64_t ld, const float *amax, uint8_t *q,
                                                           uint8_t *q_t, int64_t ld_t) {
+    chain_enter();
     __shared__ float sc;
     __shared__ __align__(16) uint8_t tile[128][64 + 8];
     if (threadIdx.x == 0) sc = f8_store_scale(*amax);
@@ -536,10 +542,10 @@ extern "C" int sp24_absmax(const void *x, int dtype, int64_t count, const void *
     if (blocks > cap) blocks = cap;
     const uint4 *xv = static_cast<const uint4 *>(x);
     const uint32_t *mv = static_cast<const uint32_t *>(mask);
-    if (dtype == SP24_F16) absmax_kernel<__half, false><<<(unsigned)blocks, 256, 0, st>>>(xv, nullptr, amax, nvec);
-    else if (dtype == SP24_BF16) absmax_kernel<__nv_bfloat16, false><<<(unsigned)blocks, 256, 0, st>>>(xv, nullptr, amax, nvec);
-    else if (mask) absmax_kernel<float, true><<<(unsigned)blocks, 256, 0, st>>>(xv, mv, amax, nvec);
-    else absmax_kernel<float, false><<<(unsigned)blocks, 256, 0, st>>>(xv, nullptr, amax, nvec);
+    if (dtype == SP24_F16) launch_chained(st, absmax_kernel<__half, false>, (unsigned)blocks, 256, 0, xv, nullptr, amax, nvec);
+    else if (dtype == SP24_BF16) launch_chained(st, absmax_kernel<__nv_bfloat16, false>, (unsigned)blocks, 256, 0, xv, nullptr, amax, nvec);
+    else if (mask) launch_chained(st, absmax_kernel<float, true>, (unsigned)blocks, 256, 0, xv, mv, amax, nvec);
+    else launch_chained(st, absmax_kernel<float, false>, (unsigned)blocks, 256, 0, xv, nullptr, amax, nvec);
     return launch_status();
 }
 
@@ -557,10 +563,10 @@ extern "C" int sp24_quantize_f8(const void *x, int dtype, int64_t rows, int64_t 
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const unsigned grid = (unsigned)tiles;
     uint8_t *qb = static_cast<uint8_t *>(q), *tb = static_cast<uint8_t *>(q_t);
-    if (dtype == SP24_F16) quantize_f8_kernel<__half><<<grid, 256, 0, st>>>(static_cast<const __half *>(x), rows, cols, ld, amax, qb, tb, ld_t);
+    if (dtype == SP24_F16) launch_chained(st, quantize_f8_kernel<__half>, grid, 256, 0, static_cast<const __half *>(x), rows, cols, ld, amax, qb, tb, ld_t);
     else if (dtype == SP24_BF16)
-        quantize_f8_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(static_cast<const __nv_bfloat16 *>(x), rows, cols, ld, amax, qb, tb, ld_t);
-    else quantize_f8_kernel<float><<<grid, 256, 0, st>>>(static_cast<const float *>(x), rows, cols, ld, amax, qb, tb, ld_t);
+        launch_chained(st, quantize_f8_kernel<__nv_bfloat16>, grid, 256, 0, static_cast<const __nv_bfloat16 *>(x), rows, cols, ld, amax, qb, tb, ld_t);
+    else launch_chained(st, quantize_f8_kernel<float>, grid, 256, 0, static_cast<const float *>(x), rows, cols, ld, amax, qb, tb, ld_t);
     return launch_status();
 }
 
@@ -607,6 +613,7 @@ __device__ __forceinline__ void adam_one(float &p, float g, float &m, float &v, 
 }
 
 __global__ void __launch_bounds__(256) adamw_masked_decay_kernel(AdamParams P) {
+    chain_enter();
     const float t = P.step_dev ? *P.step_dev : P.step;
     const float inv_bc1 = 1.f / (1.f - powf(P.beta1, t));
     const float inv_sqrt_bc2 = 1.f / sqrtf(1.f - powf(P.beta2, t));
@@ -670,7 +677,7 @@ extern "C" int sp24_adamw_masked_decay_ex(void *p, const void *grad, int grad_dt
     int64_t blocks = (n4 + 255) / 256;
     if (blocks < 1) blocks = 1;
     if (blocks > 148 * 16) blocks = 148 * 16;
-    adamw_masked_decay_kernel<<<(unsigned)blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(P);
+    launch_chained(static_cast<cudaStream_t>(stream), adamw_masked_decay_kernel, (unsigned)blocks, 256, 0, P);
     return launch_status();
 }
 

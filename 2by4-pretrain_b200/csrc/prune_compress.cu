@@ -275,6 +275,7 @@ template <typename TOut> __device__ __forceinline__ float out_scale_of(const PcP
 
 template <typename TIn, typename TOut, int MODE, bool HAS_U>
 __global__ void __launch_bounds__(256, is_mvue(MODE) ? 3 : 1) pc_row_kernel(PcParams P) {
+    chain_enter();
     const uint64_t rng_offset = P.offset + (P.offset_dev ? *P.offset_dev : 0ull);
     const float out_scale = out_scale_of<TOut>(P);
     constexpr int CH = sizeof(TOut) == 2 ? 16 : 32;  // dense elements per metadata word
@@ -455,6 +456,7 @@ constexpr int col_min_blocks(int mode) {
 
 template <typename TIn, typename TOut, int MODE, bool HAS_U, int V>
 __global__ void __launch_bounds__(256, col_min_blocks(MODE)) pc_col_kernel(PcParams P) {
+    chain_enter();
     const uint64_t rng_offset = P.offset + (P.offset_dev ? *P.offset_dev : 0ull);
     const float out_scale = out_scale_of<TOut>(P);
     constexpr int CH = sizeof(TOut) == 2 ? 16 : 32;
@@ -727,6 +729,7 @@ __device__ __forceinline__ void st_shared16(uint32_t addr, uint32_t v) { asm vol
 template <typename TIn, typename TOut>
 __global__ void __launch_bounds__(256, MvueCol<TIn>::BLOCKS)
 mvue_col_kernel(const __grid_constant__ PcParams P, const __grid_constant__ PhiloxKeys<kMvueFastRounds> keys) {
+    chain_enter();
     using Cfg = MvueCol<TIn>;
     constexpr int RT = Cfg::RT, ROW = Cfg::ROW, STAGES = Cfg::STAGES, V = 2;
     extern __shared__ __align__(16) uint8_t smem[];
@@ -890,19 +893,19 @@ int launch(const PcParams &P, int col_major, cudaStream_t st) {
     constexpr int CH = sizeof(TOut) == 2 ? 16 : 32;
     if (!col_major) {
         dim3 grid((unsigned)((P.k / CH + 31) / 32), (unsigned)(P.m / 32));
-        pc_row_kernel<TIn, TOut, MODE, HAS_U><<<grid, 256, 0, st>>>(P);
+        launch_chained(st, pc_row_kernel<TIn, TOut, MODE, HAS_U>, grid, 256, 0, P);
     } else if constexpr (MODE == SP24_PRUNE_MVUE_FAST && sizeof(TOut) == 2) {
         using Cfg = MvueCol<TIn>;
         constexpr auto kern = mvue_col_kernel<TIn, TOut>;
         if (int rc = allow_shared_memory<mvue_col_kernel<TIn, TOut>>(Cfg::SMEM)) return rc;
         const int64_t tiles = ((P.m + Cfg::RT - 1) / Cfg::RT) * ((P.k / 16 + 7) / 8), most = (int64_t)sm_count() * Cfg::BLOCKS;
-        kern<<<(unsigned)(tiles < most ? tiles : most), 256, Cfg::SMEM, st>>>(P, PhiloxKeys<kMvueFastRounds>(P.seed));
+        launch_chained(st, kern, (unsigned)(tiles < most ? tiles : most), 256, Cfg::SMEM, P, PhiloxKeys<kMvueFastRounds>(P.seed));
     } else {
         constexpr int V = MODE == SP24_PRUNE_MVUE_FAST ? ColVec<TIn>::fast8
                                                        : (MODE == SP24_PRUNE_MVUE ? ColVec<TIn>::narrow : ColVec<TIn>::wide);
         constexpr int RT = 32 * V;
         dim3 grid((unsigned)((P.m + RT - 1) / RT), (unsigned)((P.k / CH + 7) / 8));
-        pc_col_kernel<TIn, TOut, MODE, HAS_U, V><<<grid, 256, 0, st>>>(P);
+        launch_chained(st, pc_col_kernel<TIn, TOut, MODE, HAS_U, V>, grid, 256, 0, P);
     }
     return launch_status();
 }

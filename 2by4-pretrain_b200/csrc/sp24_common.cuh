@@ -9,6 +9,7 @@
 #include <stdint.h>
 
 #include <type_traits>
+#include <utility>
 
 #include "../../include/sparse24_b200.h"
 
@@ -412,5 +413,29 @@ inline int dtype_size(int dt) {
 int check_device();            // SP24_OK when the current device is compute capability 10.x
 int launch_status();           // maps cudaGetLastError() to SP24_OK / SP24_ERR_CUDA
 int sm_count();                // SMs of the current device
+
+// Programmatic dependent launch.  A kernel launched by launch_chained may start while the kernel before it on the stream is still
+// finishing (as soon as all blocks of that one have called chain_enter or left), so its launch latency and set-up are hidden behind
+// the other's last wave.  chain_enter first waits until everything before on the stream is complete and visible: no kernel touches
+// global memory before it, and every thread calls it, so a kernel's completion implies that of all kernels before it.
+__device__ __forceinline__ void chain_enter() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+// Errors are left for launch_status, as with a <<<>>> launch.
+template <typename... P, typename... A>
+inline void launch_chained(cudaStream_t st, void (*kern)(P...), dim3 grid, unsigned threads, size_t smem, A &&...args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    (void)cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...);
+}
 
 }  // namespace sp24

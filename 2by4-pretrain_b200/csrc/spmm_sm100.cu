@@ -390,6 +390,7 @@ spmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = tmem_base_smem;
+    chain_enter();
 
     if (warp == 0) {
         // ---------------------------------------------------------------- TMA producer
@@ -897,6 +898,7 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *smem = smem_raw;
     if (smem_u32(smem) & 1023) {              // the same in every CTA; the launcher looks first, the swizzled stages depend on it
+        chain_enter();
         if (threadIdx.x == 0 && P.status) atomicCAS(P.status, 0, 11);
         return;
     }
@@ -936,6 +938,7 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     cluster_sync_all();                       // the peer's barriers are initialised before anything targets them
     tc_fence_after();
     const uint32_t tmem_base = ctl.tmem_base;
+    chain_enter();
 
     if (warp == 0) {
         // ---------------------------------------------------------------- TMA producer (one per CTA)
@@ -1277,6 +1280,7 @@ spmm_pair_acc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     cluster_sync_all();
     tc_fence_after();
     const uint32_t tmem_base = tmem_base_smem;
+    chain_enter();
 
     if (warp == 0) {
         // ---------------------------------------------------------------- TMA producer (one per CTA)
@@ -1437,6 +1441,7 @@ spmm_pair_acc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
 // 16-column metadata word c.  8-bit types: atom = 128 rows x 16 bytes, row-major.
 template <int MB>
 __global__ void meta_to_tc_kernel(const void *meta_api, uint8_t *e_tc, int64_t m, int64_t ncols, int64_t k_atoms) {
+    chain_enter();
     const int64_t words_per_atom = 2048 / MB;
     const int64_t total = (m / 128) * k_atoms * words_per_atom;
     const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1543,7 +1548,7 @@ int launch_spmm(const CUtensorMap &ma, const CUtensorMap &mb, SpmmParams P, cuda
     P.idesc |= (uint32_t)(BN >> 3) << 17;
     const int64_t tiles = ((P.n + BN - 1) / BN) * ((P.ms / BM + P.mblk_per_tile - 1) / P.mblk_per_tile) * P.k_splits;
     const int sms = sm_count_cached();
-    kern<<<(unsigned)(tiles < sms ? tiles : sms), 320, Cfg::SMEM, st>>>(ma, mb, P);
+    launch_chained(st, kern, (unsigned)(tiles < sms ? tiles : sms), 320, Cfg::SMEM, ma, mb, P);
     return launch_status();
 }
 
@@ -1580,13 +1585,15 @@ int launch_spmm_pair(const CUtensorMap &ma, const CUtensorMap &mb, const CUtenso
     cfg.blockDim = dim3(320, 1, 1);
     cfg.dynamicSmemBytes = two::smem2(F8, P.bn);
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;      // see launch_chained
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
     if (cudaLaunchKernelEx(&cfg, kern, ma, mb, me, P) != cudaSuccess) return SP24_ERR_CUDA;
     return launch_status();
 }
@@ -1619,13 +1626,15 @@ int launch_spmm_pair_acc(const CUtensorMap &ma, const CUtensorMap &mb, const CUt
     cfg.blockDim = dim3(320, 1, 1);
     cfg.dynamicSmemBytes = two::SMEM3;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;      // see launch_chained
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
     if (cudaLaunchKernelEx(&cfg, kern, ma, mb, me, md, P) != cudaSuccess) return launch_status();
     return launch_status();
 }
@@ -1716,9 +1725,9 @@ extern "C" int sp24_meta_to_tc(const void *meta, int meta_itemsize, int64_t m, i
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const unsigned blocks = (unsigned)((total + 255) / 256);
     if (meta_itemsize == 2)
-        meta_to_tc_kernel<2><<<blocks, 256, 0, st>>>(meta, static_cast<uint8_t *>(e_tc), m, k / 16, k_atoms);
+        launch_chained(st, meta_to_tc_kernel<2>, blocks, 256, 0, meta, static_cast<uint8_t *>(e_tc), m, k / 16, k_atoms);
     else
-        meta_to_tc_kernel<4><<<blocks, 256, 0, st>>>(meta, static_cast<uint8_t *>(e_tc), m, k / 32, k_atoms);
+        launch_chained(st, meta_to_tc_kernel<4>, blocks, 256, 0, meta, static_cast<uint8_t *>(e_tc), m, k / 32, k_atoms);
     return launch_status();
 }
 

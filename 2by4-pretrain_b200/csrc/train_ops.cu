@@ -63,6 +63,7 @@ template <typename TOut, int NV>
 __global__ void __launch_bounds__(256) layernorm_fwd_kernel(const float *x, const TOut *delta, float *res_out, const float *gamma,
                                                             const float *beta, TOut *out, float *mean_out, float *rstd_out,
                                                             int64_t rows, float eps) {
+    chain_enter();
     constexpr int d = NV * 128, nv = NV;
     const int lane = threadIdx.x & 31;
     const int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -121,6 +122,7 @@ template <typename TDy, int NV>
 __global__ void __launch_bounds__(32 * LnBwdWarps<NV>::value, 1)
     layernorm_bwd_kernel(const TDy *dy, const float *x, const float *gamma, const float *mean, const float *rstd, const float *dres,
                          float *dx, TDy *ddelta, float *dgamma, float *dbeta, int64_t rows) {
+    chain_enter();
     extern __shared__ float red[];           // 2 x W x d floats: [gamma sums | beta sums] x warp x column
     constexpr int d = NV * 128, W = LnBwdWarps<NV>::value;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -213,6 +215,7 @@ template <typename T> __device__ __forceinline__ void unpack8(const uint4 &r, fl
 template <typename T>
 __global__ void __launch_bounds__(256) ce_fwd_kernel(const T *logits, const int64_t *targets, float *lse, float *loss,
                                                      int64_t v, int64_t ld) {
+    chain_enter();
     __shared__ float scratch[8];
     const int64_t row = blockIdx.x;
     const T *p = logits + row * ld;
@@ -246,6 +249,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) ce_bwd_kernel(const T *logits, const int64_t *targets, const float *lse,
                                                      const float *upstream, float scale, T *dlogits, int64_t v, int64_t ld,
                                                      int64_t ld_out) {
+    chain_enter();
     const int64_t row = blockIdx.x;
     const T *p = logits + row * ld;
     T *q = dlogits + row * ld_out;
@@ -304,6 +308,7 @@ template <> struct Pair16<__half> {
 template <typename T, bool STAGED>
 __global__ void __launch_bounds__(512) ce_fused_kernel(const T *logits, const int64_t *targets, float *lse, float *loss,
                                                        float scale, T *dlogits, int64_t v, int64_t ld, int64_t ld_out) {
+    chain_enter();
     extern __shared__ uint4 staged[];        // the row as 16-byte pieces (STAGED only)
     __shared__ float scratch[16];
     typedef typename Pair16<T>::type P2;
@@ -399,6 +404,7 @@ __device__ __forceinline__ void red_add_v4(float *addr, const float4 &v) {
 // out[row, :] = wte[ids[row], :] + wpe[row % t, :]; an id outside [0, vocab) contributes zeros
 __global__ void __launch_bounds__(256) embedding_fwd_kernel(const int64_t *ids, const float *wte, const float *wpe, float *out,
                                                             int64_t rows, int64_t t, int64_t d, int64_t vocab) {
+    chain_enter();
     const int lane = threadIdx.x & 31;
     const int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
     if (row >= rows) return;
@@ -415,6 +421,7 @@ __global__ void __launch_bounds__(256) embedding_fwd_kernel(const int64_t *ids, 
 // which rows that share a token or a position are added is not fixed)
 __global__ void __launch_bounds__(256) embedding_bwd_kernel(const float *dx, const int64_t *ids, float *dwte, float *dwpe,
                                                             int64_t rows, int64_t t, int64_t d, int64_t vocab) {
+    chain_enter();
     const int lane = threadIdx.x & 31;
     const int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
     if (row >= rows) return;
@@ -450,6 +457,7 @@ __device__ __forceinline__ float dgelu_f(float x) {
 // BWD: out = dy * gelu'(x); otherwise out = gelu(x).  Two 16-byte pieces per thread and trip.
 template <typename T, bool BWD>
 __global__ void __launch_bounds__(256) gelu_kernel(const uint4 *x, const uint4 *dy, uint4 *out, int64_t nvec) {
+    chain_enter();
     const int64_t stride = (int64_t)gridDim.x * 256;
     for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < nvec; i += 2 * stride) {
         const int64_t i2 = i + stride;
@@ -492,6 +500,7 @@ __global__ void __launch_bounds__(256) gelu_kernel(const uint4 *x, const uint4 *
 constexpr int CS_COLS = 64, CS_BLOCKS = 8, CS_ROWS = 512 / (CS_COLS / 8), CS_FLIGHT = 4;
 template <typename T>
 __global__ void __cluster_dims__(1, CS_BLOCKS, 1) __launch_bounds__(512) column_sums_kernel(const T *x, int64_t rows, int64_t cols, int64_t ld, float *out) {
+    chain_enter();
     __shared__ float part[CS_ROWS][CS_COLS + 4], total[CS_COLS];
     const auto cluster = cooperative_groups::this_cluster();
     const int piece = threadIdx.x % (CS_COLS / 8), group = threadIdx.x / (CS_COLS / 8);
@@ -543,6 +552,7 @@ __global__ void __cluster_dims__(1, CS_BLOCKS, 1) __launch_bounds__(512) column_
 // adds their sums up.  Bound by latency and the launch; the layer step with 128 x 3072 partial sums (16384 x 768 -> 3072, fp16)
 // went from 242.3 us with atomics to 246.3.
 __global__ void __launch_bounds__(256) sum_parts_kernel(const float *parts, int64_t n_parts, int64_t m, float *out, int accumulate) {
+    chain_enter();
     __shared__ float part[8][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t c = (int64_t)blockIdx.x * 32 + lane;
@@ -564,6 +574,7 @@ __global__ void __launch_bounds__(256) sum_parts_kernel(const float *parts, int6
 // g *= *factor unless *factor == 1 (the usual case: nothing is read or written then)
 template <typename T>
 __global__ void __launch_bounds__(256) scale_unless_one_kernel(T *g, const float *factor, int64_t nvec) {
+    chain_enter();
     const float f = *factor;
     if (f == 1.f) return;
     for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < nvec; i += (int64_t)gridDim.x * 256) {
@@ -595,7 +606,7 @@ static int layernorm_fwd_impl(const float *x, const void *delta, float *res_out,
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const unsigned blocks = (unsigned)((rows + 7) / 8);
 #define SP24_LN_FWD(T_, NV_) \
-    layernorm_fwd_kernel<T_, NV_><<<blocks, 256, 0, st>>>(x, static_cast<const T_ *>(delta), res_out, gamma, beta, \
+    launch_chained(st, layernorm_fwd_kernel<T_, NV_>, blocks, 256, 0, x, static_cast<const T_ *>(delta), res_out, gamma, beta, \
                                                           static_cast<T_ *>(out), mean, rstd, rows, eps)
 #define SP24_LN_FWD_NV(T_) \
     switch (d / 128) { \
@@ -652,7 +663,7 @@ static int layernorm_bwd_impl(const void *dy, int dy_dtype, const float *dres, c
         int64_t blocks = (rows + W - 1) / W; \
         const int64_t cap = (int64_t)sm_count() * resident; \
         if (blocks > cap) blocks = cap; \
-        kern<<<(unsigned)blocks, 32 * W, smem, st>>>(static_cast<const T_ *>(dy), x, gamma, mean, rstd, dres, dx, \
+        launch_chained(st, kern, (unsigned)blocks, 32 * W, smem, static_cast<const T_ *>(dy), x, gamma, mean, rstd, dres, dx, \
                                                   static_cast<T_ *>(ddelta), dgamma, dbeta, rows); \
     } while (0)
 #define SP24_LN_BWD_NV(T_) \
@@ -692,9 +703,9 @@ extern "C" int sp24_cross_entropy_fwd(const void *logits, int dtype, const int64
     if (int rc = check_device()) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (dtype == SP24_F16)
-        ce_fwd_kernel<__half><<<(unsigned)rows, 256, 0, st>>>(static_cast<const __half *>(logits), targets, lse, loss, v, ld);
+        launch_chained(st, ce_fwd_kernel<__half>, (unsigned)rows, 256, 0, static_cast<const __half *>(logits), targets, lse, loss, v, ld);
     else
-        ce_fwd_kernel<__nv_bfloat16><<<(unsigned)rows, 256, 0, st>>>(static_cast<const __nv_bfloat16 *>(logits), targets, lse, loss, v, ld);
+        launch_chained(st, ce_fwd_kernel<__nv_bfloat16>, (unsigned)rows, 256, 0, static_cast<const __nv_bfloat16 *>(logits), targets, lse, loss, v, ld);
     return launch_status();
 }
 
@@ -710,10 +721,10 @@ extern "C" int sp24_cross_entropy_bwd(const void *logits, int dtype, const int64
     if (int rc = check_device()) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (dtype == SP24_F16)
-        ce_bwd_kernel<__half><<<(unsigned)rows, 256, 0, st>>>(static_cast<const __half *>(logits), targets, lse, upstream, scale,
+        launch_chained(st, ce_bwd_kernel<__half>, (unsigned)rows, 256, 0, static_cast<const __half *>(logits), targets, lse, upstream, scale,
                                                              static_cast<__half *>(dlogits), v, ld, ld_out);
     else
-        ce_bwd_kernel<__nv_bfloat16><<<(unsigned)rows, 256, 0, st>>>(static_cast<const __nv_bfloat16 *>(logits), targets, lse, upstream,
+        launch_chained(st, ce_bwd_kernel<__nv_bfloat16>, (unsigned)rows, 256, 0, static_cast<const __nv_bfloat16 *>(logits), targets, lse, upstream,
                                                                     scale, static_cast<__nv_bfloat16 *>(dlogits), v, ld, ld_out);
     return launch_status();
 }
@@ -733,10 +744,10 @@ static int ce_fused_launch(const void *logits, const int64_t *targets, float *ls
                 return launch_status();
             attr_set[dev] = true;
         }
-        kern<<<(unsigned)rows, 512, row_bytes, st>>>(static_cast<const T *>(logits), targets, lse, loss, scale,
+        launch_chained(st, kern, (unsigned)rows, 512, row_bytes, static_cast<const T *>(logits), targets, lse, loss, scale,
                                                      static_cast<T *>(dlogits), v, ld, ld_out);
     } else {
-        ce_fused_kernel<T, false><<<(unsigned)rows, 512, 0, st>>>(static_cast<const T *>(logits), targets, lse, loss, scale,
+        launch_chained(st, ce_fused_kernel<T, false>, (unsigned)rows, 512, 0, static_cast<const T *>(logits), targets, lse, loss, scale,
                                                                   static_cast<T *>(dlogits), v, ld, ld_out);
     }
     return launch_status();
@@ -766,8 +777,8 @@ extern "C" int sp24_column_sums(const void *x, int dtype, int64_t rows, int64_t 
     if (int rc = check_device()) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const dim3 grid((unsigned)((cols + CS_COLS - 1) / CS_COLS), CS_BLOCKS);
-    if (dtype == SP24_F16) column_sums_kernel<__half><<<grid, 512, 0, st>>>(static_cast<const __half *>(x), rows, cols, ld, out);
-    else column_sums_kernel<__nv_bfloat16><<<grid, 512, 0, st>>>(static_cast<const __nv_bfloat16 *>(x), rows, cols, ld, out);
+    if (dtype == SP24_F16) launch_chained(st, column_sums_kernel<__half>, grid, 512, 0, static_cast<const __half *>(x), rows, cols, ld, out);
+    else launch_chained(st, column_sums_kernel<__nv_bfloat16>, grid, 512, 0, static_cast<const __nv_bfloat16 *>(x), rows, cols, ld, out);
     return launch_status();
 }
 
@@ -775,7 +786,7 @@ extern "C" int sp24_sum_parts(const float *parts, int64_t n_parts, int64_t m, fl
     if (!parts || !out) return SP24_ERR_ARG;
     if (n_parts <= 0 || m <= 0 || (m + 31) / 32 > 0x7FFFFFFF) return SP24_ERR_SHAPE;
     if (int rc = check_device()) return rc;
-    sum_parts_kernel<<<(unsigned)((m + 31) / 32), 256, 0, static_cast<cudaStream_t>(stream)>>>(parts, n_parts, m, out, accumulate);
+    launch_chained(static_cast<cudaStream_t>(stream), sum_parts_kernel, (unsigned)((m + 31) / 32), 256, 0, parts, n_parts, m, out, accumulate);
     return launch_status();
 }
 
@@ -791,9 +802,9 @@ extern "C" int sp24_scale_unless_one(void *g, int dtype, const float *factor, in
     const int64_t cap = (int64_t)sm_count() * 8;
     if (blocks > cap) blocks = cap;
     if (dtype == SP24_F16)
-        scale_unless_one_kernel<__half><<<(unsigned)blocks, 256, 0, st>>>(static_cast<__half *>(g), factor, nvec);
+        launch_chained(st, scale_unless_one_kernel<__half>, (unsigned)blocks, 256, 0, static_cast<__half *>(g), factor, nvec);
     else
-        scale_unless_one_kernel<__nv_bfloat16><<<(unsigned)blocks, 256, 0, st>>>(static_cast<__nv_bfloat16 *>(g), factor, nvec);
+        launch_chained(st, scale_unless_one_kernel<__nv_bfloat16>, (unsigned)blocks, 256, 0, static_cast<__nv_bfloat16 *>(g), factor, nvec);
     return launch_status();
 }
 
@@ -804,7 +815,7 @@ extern "C" int sp24_embedding_fwd(const int64_t *ids, const float *wte, const fl
     if (!aligned16(wte) || !aligned16(wpe) || !aligned16(out)) return SP24_ERR_ALIGN;
     if ((rows + 7) / 8 > 0x7FFFFFFF) return SP24_ERR_TOO_LARGE;
     if (int rc = check_device()) return rc;
-    embedding_fwd_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(ids, wte, wpe, out, rows, t, d,
+    launch_chained(static_cast<cudaStream_t>(stream), embedding_fwd_kernel, (unsigned)((rows + 7) / 8), 256, 0, ids, wte, wpe, out, rows, t, d,
                                                                                                      vocab);
     return launch_status();
 }
@@ -816,7 +827,7 @@ extern "C" int sp24_embedding_bwd(const float *dx, const int64_t *ids, float *dw
     if (!aligned16(dx) || !aligned16(dwte) || !aligned16(dwpe)) return SP24_ERR_ALIGN;
     if ((rows + 7) / 8 > 0x7FFFFFFF) return SP24_ERR_TOO_LARGE;
     if (int rc = check_device()) return rc;
-    embedding_bwd_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(dx, ids, dwte, dwpe, rows, t, d,
+    launch_chained(static_cast<cudaStream_t>(stream), embedding_bwd_kernel, (unsigned)((rows + 7) / 8), 256, 0, dx, ids, dwte, dwpe, rows, t, d,
                                                                                                      vocab);
     return launch_status();
 }
@@ -835,11 +846,11 @@ extern "C" int sp24_gelu(const void *x, const void *dy, void *out, int dtype, in
     const uint4 *xv = static_cast<const uint4 *>(x), *gv = static_cast<const uint4 *>(dy);
     uint4 *ov = static_cast<uint4 *>(out);
     if (dtype == SP24_F16) {
-        if (dy) gelu_kernel<__half, true><<<(unsigned)blocks, 256, 0, st>>>(xv, gv, ov, nvec);
-        else gelu_kernel<__half, false><<<(unsigned)blocks, 256, 0, st>>>(xv, gv, ov, nvec);
+        if (dy) launch_chained(st, gelu_kernel<__half, true>, (unsigned)blocks, 256, 0, xv, gv, ov, nvec);
+        else launch_chained(st, gelu_kernel<__half, false>, (unsigned)blocks, 256, 0, xv, gv, ov, nvec);
     } else {
-        if (dy) gelu_kernel<__nv_bfloat16, true><<<(unsigned)blocks, 256, 0, st>>>(xv, gv, ov, nvec);
-        else gelu_kernel<__nv_bfloat16, false><<<(unsigned)blocks, 256, 0, st>>>(xv, gv, ov, nvec);
+        if (dy) launch_chained(st, gelu_kernel<__nv_bfloat16, true>, (unsigned)blocks, 256, 0, xv, gv, ov, nvec);
+        else launch_chained(st, gelu_kernel<__nv_bfloat16, false>, (unsigned)blocks, 256, 0, xv, gv, ov, nvec);
     }
     return launch_status();
 }

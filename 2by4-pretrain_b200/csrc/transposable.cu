@@ -158,6 +158,7 @@ __device__ __forceinline__ uint32_t gather_mask_bytes(uint32_t mw) {
 template <typename T>
 __global__ void __launch_bounds__(256) ts_select_kernel(const T *x, T *sparse, uint8_t *mask, int64_t k, int64_t ld_x,
                                                         int64_t ld_s, int64_t ld_m, int use_abs) {
+    chain_enter();
     __shared__ uint32_t lut[64];
     load_select_lut(lut);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -416,6 +417,7 @@ template <typename T, typename TOut> constexpr int dual_few_limit(bool select, b
 
 template <typename T, typename TOut, bool SELECT, bool TC, bool FEW>
 __global__ void __launch_bounds__(256, dual_min_blocks(SELECT, sizeof(T), FEW)) ts_dual_kernel(DualParams P) {
+    chain_enter();
     ts_dual_block<T, TOut, SELECT, TC>(P, blockIdx.x, blockIdx.y);
 }
 
@@ -430,6 +432,7 @@ struct DualBatch {
 };
 template <typename T, typename TOut, bool SELECT, bool TC, bool FEW>
 __global__ void __launch_bounds__(256, dual_min_blocks(SELECT, sizeof(T), FEW)) ts_dual_batch_kernel(const __grid_constant__ DualBatch B) {
+    chain_enter();
     int i = 0;
     while (i + 1 < B.count && blockIdx.x >= B.first[i + 1]) ++i;
     const DualParams &P = B.p[i];
@@ -442,9 +445,9 @@ template <typename T, typename TOut, bool SELECT, bool TC> int launch_dual_form(
     dim3 grid((unsigned)((P.k + 127) / 128), (unsigned)(P.m / 64));
     constexpr int limit = dual_few_limit<T, TOut>(SELECT, false);
     if (limit == ALWAYS_FEW || (uint64_t)grid.x * grid.y <= (uint64_t)limit * sm_count()) {
-        if constexpr (limit > 0) ts_dual_kernel<T, TOut, SELECT, TC, true><<<grid, 256, 0, st>>>(P);
+        if constexpr (limit > 0) launch_chained(st, ts_dual_kernel<T, TOut, SELECT, TC, true>, grid, 256, 0, P);
     } else {
-        if constexpr (limit < ALWAYS_FEW) ts_dual_kernel<T, TOut, SELECT, TC, false><<<grid, 256, 0, st>>>(P);
+        if constexpr (limit < ALWAYS_FEW) launch_chained(st, ts_dual_kernel<T, TOut, SELECT, TC, false>, grid, 256, 0, P);
     }
     return launch_status();
 }
@@ -453,9 +456,9 @@ template <typename T, typename TOut, bool SELECT, bool TC> int launch_dual_list(
     const unsigned grid = B.first[B.count];
     constexpr int limit = dual_few_limit<T, TOut>(SELECT, true);
     if (limit == ALWAYS_FEW || grid <= (uint64_t)limit * sm_count()) {
-        if constexpr (limit > 0) ts_dual_batch_kernel<T, TOut, SELECT, TC, true><<<grid, 256, 0, st>>>(B);
+        if constexpr (limit > 0) launch_chained(st, ts_dual_batch_kernel<T, TOut, SELECT, TC, true>, grid, 256, 0, B);
     } else {
-        if constexpr (limit < ALWAYS_FEW) ts_dual_batch_kernel<T, TOut, SELECT, TC, false><<<grid, 256, 0, st>>>(B);
+        if constexpr (limit < ALWAYS_FEW) launch_chained(st, ts_dual_batch_kernel<T, TOut, SELECT, TC, false>, grid, 256, 0, B);
     }
     return launch_status();
 }
@@ -504,15 +507,15 @@ extern "C" int sp24_transposable_select(const void *x, int dtype, int64_t m, int
     uint8_t *mk = static_cast<uint8_t *>(mask_out);
     switch (dtype) {
         case SP24_F32:
-            ts_select_kernel<float><<<grid, 256, 0, st>>>(static_cast<const float *>(x), static_cast<float *>(sparse_out), mk,
+            launch_chained(st, ts_select_kernel<float>, grid, 256, 0, static_cast<const float *>(x), static_cast<float *>(sparse_out), mk,
                                                           k, ld_x, ld_sparse, ld_mask, use_abs);
             break;
         case SP24_F16:
-            ts_select_kernel<__half><<<grid, 256, 0, st>>>(static_cast<const __half *>(x), static_cast<__half *>(sparse_out),
+            launch_chained(st, ts_select_kernel<__half>, grid, 256, 0, static_cast<const __half *>(x), static_cast<__half *>(sparse_out),
                                                            mk, k, ld_x, ld_sparse, ld_mask, use_abs);
             break;
         default:
-            ts_select_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(static_cast<const __nv_bfloat16 *>(x),
+            launch_chained(st, ts_select_kernel<__nv_bfloat16>, grid, 256, 0, static_cast<const __nv_bfloat16 *>(x),
                                                                   static_cast<__nv_bfloat16 *>(sparse_out), mk, k, ld_x,
                                                                   ld_sparse, ld_mask, use_abs);
     }
