@@ -30,6 +30,8 @@ struct PcParams {
     const float *amax;                      // optional: 8-bit outputs take their scale from this device word (f8_store_scale)
     void *q_dense;                          // optional (column-major input, 8-bit output): dense * f8_store_scale in the output
     int64_t ld_q;                           // type, same storage order, pitch ld_q
+    uint4 *zero;                            // optional (fast MVUE, column-major input): a buffer of n_zero 16-byte pieces that is
+    int64_t n_zero;                         // cleared on the way
 };
 
 // internal mode code of the fused soft-threshold + compress entry point (not part of the public enum)
@@ -259,6 +261,14 @@ template <typename T> __device__ __forceinline__ uint32_t mse_lookup(uint32_t lo
 // row-major storage: groups of four run along the contiguous axis.
 // Tile = 32 rows x 32 metadata columns; 8 warps, lane = metadata column, warp w owns rows 4w..4w+3.
 // ---------------------------------------------------------------------------------------------
+// Clears this block's share of the buffer that the launch was given: the weight gradient that the next kernel adds to.  The stores go
+// out beside the arithmetic, where a memset of its own (9.4 MB: 3.1 us) held up the stream.
+__device__ __forceinline__ void clear_share(const PcParams &P, int64_t block, int64_t blocks) {
+    if (!P.zero) return;
+    const int64_t per = (P.n_zero + blocks - 1) / blocks, end = min(P.n_zero, (block + 1) * per);
+    for (int64_t i = block * per + threadIdx.x; i < end; i += 256) P.zero[i] = make_uint4(0, 0, 0, 0);
+}
+
 // Store scale of an 8-bit output: the caller's, or the reciprocal of the tensor's quantisation scale, worked out by one
 // thread from the absolute maximum that an earlier launch left on the device.  Call with all threads of the block.
 template <typename TOut> __device__ __forceinline__ float out_scale_of(const PcParams &P) {
@@ -475,6 +485,7 @@ __global__ void __launch_bounds__(256, col_min_blocks(MODE)) pc_col_kernel(PcPar
     __shared__ __align__(8) PickEntry picks[PAIRS ? 16 : 1];
     if constexpr (PAIRS) load_pick_lut<TOut>(picks);
     const uint32_t picks_at = (uint32_t)__cvta_generic_to_shared(picks);
+    if constexpr (PAIRS) clear_share(P, (int64_t)blockIdx.y * gridDim.x + blockIdx.x, (int64_t)gridDim.x * gridDim.y);
 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t ncols = P.k / CH;
@@ -782,6 +793,7 @@ mvue_col_kernel(const __grid_constant__ PcParams P, const __grid_constant__ Phil
     pin(store_to);
 
     for (int i = 0; i < STAGES; ++i) fetch(i);
+    clear_share(P, blockIdx.x, gridDim.x);
     int tr = blockIdx.x % n_rt, tc = blockIdx.x / n_rt, buf = 0;
     uint32_t out_off = 0;
     const uint32_t row_pairs = (uint32_t)(P.k / 8);
@@ -950,7 +962,7 @@ static int prune_compress_impl(const void *dense, int dense_dtype, int64_t m, in
                                int64_t ld_uniforms, uint64_t seed, uint64_t offset, const uint64_t *offset_dev,
                                void *e_tc, float *row_sums, void *stream, int packed_rm = 0, float out_scale = 1.f,
                                int soft_use_scale = 0, float soft_scale = 1.f, const float *amax = nullptr, void *q_dense = nullptr,
-                               int64_t ld_q = 0, bool sums_in_parts = false) {
+                               int64_t ld_q = 0, bool sums_in_parts = false, void *zero = nullptr, int64_t zero_bytes = 0) {
     using namespace sp24;
     if (!dense || !packed || !meta) return SP24_ERR_ARG;
     const int so = dtype_size(packed_dtype), si = dtype_size(dense_dtype);
@@ -975,11 +987,13 @@ static int prune_compress_impl(const void *dense, int dense_dtype, int64_t m, in
         return SP24_ERR_ALIGN;
     if (e_tc && (packed_dtype == SP24_I8 || m % 128 || !aligned16(e_tc))) return SP24_ERR_ARG;
     if (q_dense && (!amax || !packed_rm || ld_q < m || ld_q % 16 || !aligned16(q_dense))) return SP24_ERR_ARG;
+    if (zero && (mode != SP24_PRUNE_MVUE_FAST || !col_major || zero_bytes <= 0 || zero_bytes % 16 || !aligned16(zero))) return SP24_ERR_ARG;
     if (row_sums && (!col_major || (reinterpret_cast<uintptr_t>(row_sums) & 3u))) return SP24_ERR_ARG;
     if (int rc = check_device()) return rc;
     PcParams P{dense, packed, meta, static_cast<const uint8_t *>(mask), uniforms, m, k, ld_dense, ld_packed, ld_mask,
                ld_uniforms, seed, offset, reinterpret_cast<const unsigned long long *>(offset_dev),
-               static_cast<int16_t *>(e_tc), (k + 127) / 128, row_sums, sums_in_parts ? m : 0, packed_rm, out_scale, soft_scale, soft_use_scale, amax, q_dense, ld_q};
+               static_cast<int16_t *>(e_tc), (k + 127) / 128, row_sums, sums_in_parts ? m : 0, packed_rm, out_scale, soft_scale, soft_use_scale, amax, q_dense, ld_q,
+               static_cast<uint4 *>(zero), zero_bytes / 16};
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     switch (dense_dtype) {
         case SP24_F32: return dispatch_out<float>(P, packed_dtype, mode, col_major, st);
@@ -1057,17 +1071,33 @@ extern "C" int sp24_row_parts(int64_t k, int packed_dtype) {
     return so != 1 && so != 2 ? 0 : (int)((k + per - 1) / per);
 }
 
-extern "C" int sp24_prune_compress_with(const void *dense, int dense_dtype, int64_t m, int64_t k, int64_t ld_dense, int col_major,
-                                        void *packed, int packed_dtype, int64_t ld_packed, void *meta, int mode, const void *mask,
-                                        int64_t ld_mask, const float *uniforms, int64_t ld_uniforms, uint64_t seed, uint64_t offset,
-                                        const sp24_prune_extras *x, void *stream) {
+static int prune_compress_with(const void *dense, int dense_dtype, int64_t m, int64_t k, int64_t ld_dense, int col_major, void *packed,
+                               int packed_dtype, int64_t ld_packed, void *meta, int mode, const void *mask, int64_t ld_mask,
+                               const float *uniforms, int64_t ld_uniforms, uint64_t seed, uint64_t offset, const sp24_prune_extras *x,
+                               void *zero, int64_t zero_bytes, void *stream) {
     if (!x || mode > SP24_PRUNE_MVUE_FAST) return SP24_ERR_ARG;
     if (x->offset_dev && (reinterpret_cast<uintptr_t>(x->offset_dev) & 7u)) return SP24_ERR_ARG;
     if (x->amax && packed_dtype != SP24_E4M3 && packed_dtype != SP24_E5M2) return SP24_ERR_DTYPE;
     if (x->amax && x->out_scale != 0.f) return SP24_ERR_ARG;
     return prune_compress_impl(dense, dense_dtype, m, k, ld_dense, col_major, packed, packed_dtype, ld_packed, meta, mode, mask, ld_mask,
                                uniforms, ld_uniforms, seed, offset, x->offset_dev, x->e_tc, x->row_parts, stream, x->packed_row_major && col_major ? 1 : 0,
-                               x->out_scale != 0.f ? x->out_scale : 1.f, 0, 1.f, x->amax, x->q_dense, x->ld_q, true);
+                               x->out_scale != 0.f ? x->out_scale : 1.f, 0, 1.f, x->amax, x->q_dense, x->ld_q, true, zero, zero_bytes);
+}
+
+extern "C" int sp24_prune_compress_with(const void *dense, int dense_dtype, int64_t m, int64_t k, int64_t ld_dense, int col_major,
+                                        void *packed, int packed_dtype, int64_t ld_packed, void *meta, int mode, const void *mask,
+                                        int64_t ld_mask, const float *uniforms, int64_t ld_uniforms, uint64_t seed, uint64_t offset,
+                                        const sp24_prune_extras *x, void *stream) {
+    return prune_compress_with(dense, dense_dtype, m, k, ld_dense, col_major, packed, packed_dtype, ld_packed, meta, mode, mask, ld_mask,
+                               uniforms, ld_uniforms, seed, offset, x, nullptr, 0, stream);
+}
+
+extern "C" int sp24_mvue_compress_clearing(const void *dense, int dense_dtype, int64_t m, int64_t k, int64_t ld_dense, void *packed,
+                                           int packed_dtype, int64_t ld_packed, void *meta, uint64_t seed, uint64_t offset,
+                                           const sp24_prune_extras *x, void *zero, int64_t zero_bytes, void *stream) {
+    if (!zero) return SP24_ERR_ARG;
+    return prune_compress_with(dense, dense_dtype, m, k, ld_dense, 1, packed, packed_dtype, ld_packed, meta, SP24_PRUNE_MVUE_FAST, nullptr, 0,
+                               nullptr, 0, seed, offset, x, zero, zero_bytes, stream);
 }
 
 // S-STE forward in one pass: magnitude 2:4 mask, soft threshold of the kept values (one rounding in the input type),

@@ -397,6 +397,14 @@ __device__ __forceinline__ double f8_scale(float amax) { return amax > 0.f ? (do
 // its reciprocal) move products that are exact ties of e4m3 to the other side: 0.6 % of 16-bit values at some maxima.
 __device__ __forceinline__ float f8_store_scale(float amax) { return (float)(1.0 / f8_scale(amax)); }
 
+// Rows first, first + 8, ... of one column of parts (rows of `pitch` values) added up in that order: an eighth of a fixed-order sum.
+__device__ __forceinline__ float sum_every_eighth(const float *column, int64_t n_parts, int64_t pitch, int first) {
+    float s = 0.f;
+#pragma unroll 8
+    for (int64_t p = first; p < n_parts; p += 8) s += column[p * pitch];
+    return s;
+}
+
 // ---------------------------------------------------------------------------------------------
 // host-side helpers
 // ---------------------------------------------------------------------------------------------

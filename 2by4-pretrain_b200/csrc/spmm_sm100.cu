@@ -212,6 +212,10 @@ struct SpmmParams {
     int accumulate;         // float8, float32 output (ms, n): add alpha * A * B instead of storing it
     void *aux;              // fused MLP epilogues (CTA-pair kernel): second tensor shaped and pitched like out
     int64_t ld_aux;
+    const float *row_parts; // weight-gradient form: row_sums[r] (+)= sum over p of row_parts[p * ms + r]
+    float *row_sums;
+    int64_t n_parts;
+    int sums_accumulate;
 };
 
 // Epilogue forms of the CTA-pair kernel.  PRE_GELU: aux = h = acc + bias rounded to the output type, out = gelu(h)
@@ -1371,6 +1375,23 @@ spmm_pair_acc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         const bool idle_ring = n_units <= n_pairs;     // this pair's only unit: the operand ring is free when it is complete
         const uint32_t stg = smem_u32(smem) + (idle_ring ? (warp - 2) * CHUNKS3 * 2 * BOX3_BYTES
                                                          : STAGES3 * STAGE3_BYTES + (warp - 2) * BOX3_BYTES);
+        // The row sums that the compression left in parts (the bias gradient), while the first operands are on their way: 32 rows a
+        // CTA and turn, in the order of sum_parts_kernel, through the staging that nothing uses yet.  As a launch of its own between
+        // the compression and this kernel it took 2.6 us of a replayed step and 4 of an eager one.
+        if (P.row_sums) {
+            float *const part = reinterpret_cast<float *>(smem + STAGES3 * STAGE3_BYTES);
+            for (int64_t r = (int64_t)blockIdx.x * 32; r < P.ms; r += (int64_t)gridDim.x * 32) {
+                part[(warp - 2) * 32 + lane] = sum_every_eighth(P.row_parts + r + lane, P.n_parts, P.ms, warp - 2);
+                epilogue_bar_sync();
+                if (warp == 2) {
+                    float t = 0.f;
+#pragma unroll
+                    for (int w = 0; w < 8; ++w) t += part[w * 32 + lane];
+                    P.row_sums[r + lane] = P.sums_accumulate ? P.row_sums[r + lane] + t : t;
+                }
+                epilogue_bar_sync();
+            }
+        }
         int tl = 0;
         for (int unit = pair; unit < n_units; unit += n_pairs, ++tl) {
             const int tile = unit % n_tiles;
@@ -2032,13 +2053,14 @@ extern "C" int sp24_spmm_noalloc(const void *a_packed, int dtype, int a_mn_major
 // D (ms x n, fp32, row-major) += A_sparse (ms x k) * B (k x n, stored row-major): the weight-gradient form.
 // K is cut into slices so that tiles x slices fills the SMs; every slice adds its partial product with fp32
 // reductions, so the caller zeroes D for a plain product or passes a gradient buffer to accumulate into.
-extern "C" int sp24_spmm_accumulate_f32(const void *a_packed, int dtype, int a_mn_major, int64_t ld_a, const void *e_tc,
-                                        int64_t ms, int64_t k, const void *b, int64_t ld_b, int64_t n, float *out,
-                                        int64_t ld_out, int k_splits, int *status, void *stream) {
+static int spmm_accumulate_impl(const void *a_packed, int dtype, int a_mn_major, int64_t ld_a, const void *e_tc, int64_t ms, int64_t k,
+                                const void *b, int64_t ld_b, int64_t n, float *out, int64_t ld_out, int k_splits, const float *row_parts,
+                                int64_t n_parts, float *row_sums, int sums_accumulate, int *status, void *stream) {
     if (!a_packed || !e_tc || !b || !out || !status) return SP24_ERR_ARG;
     if (dtype != SP24_F16 && dtype != SP24_BF16) return SP24_ERR_DTYPE;
     if (ms <= 0 || n <= 0 || k <= 0 || ms % 128 || k % 64 || n % 8) return SP24_ERR_SHAPE;
     if (k_splits < 0) return SP24_ERR_ARG;
+    if (row_sums && (!row_parts || n_parts <= 0)) return SP24_ERR_ARG;
     const int64_t a_inner = a_mn_major ? ms : k / 2;
     if (ld_a < a_inner || (ld_a * 2) % 16 || ld_b < n || (ld_b * 2) % 16 || ld_out < n || (ld_out * 4) % 16) return SP24_ERR_STRIDE;
     if (!aligned16(a_packed) || !aligned16(e_tc) || !aligned16(b) || !aligned16(out)) return SP24_ERR_ALIGN;
@@ -2070,9 +2092,12 @@ extern "C" int sp24_spmm_accumulate_f32(const void *a_packed, int dtype, int a_m
         CUtensorMap map_d;
         rc = encode_map(&map_d, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, out, n, ms, ld_out * 4, 32, 16, CU_TENSOR_MAP_SWIZZLE_128B);
         if (rc) return rc;
+        P.row_parts = row_parts; P.row_sums = row_sums; P.n_parts = n_parts; P.sums_accumulate = sums_accumulate;
         return a_mn_major ? launch_spmm_pair_acc<true>(map_a, map_b, map_e, map_d, P, k_splits, st)
                           : launch_spmm_pair_acc<false>(map_a, map_b, map_e, map_d, P, k_splits, st);
     }
+    if (row_sums)
+        if (int rc2 = sp24_sum_parts(row_parts, n_parts, ms, row_sums, sums_accumulate, stream)) return rc2;
     // widest tile (least operand traffic per output), then as many K slices as idle SMs allow
     const int sms = sm_count_cached();
     const bool wide = n >= 192;
@@ -2090,4 +2115,20 @@ extern "C" int sp24_spmm_accumulate_f32(const void *a_packed, int dtype, int a_m
                                 : launch_spmm<128, false, true, true, false, float>(map_a, map_b, P, st);
     return wide ? launch_spmm<192, false, false, true, false, float>(map_a, map_b, P, st)
                 : launch_spmm<128, false, false, true, false, float>(map_a, map_b, P, st);
+}
+
+extern "C" int sp24_spmm_accumulate_f32(const void *a_packed, int dtype, int a_mn_major, int64_t ld_a, const void *e_tc,
+                                        int64_t ms, int64_t k, const void *b, int64_t ld_b, int64_t n, float *out,
+                                        int64_t ld_out, int k_splits, int *status, void *stream) {
+    return spmm_accumulate_impl(a_packed, dtype, a_mn_major, ld_a, e_tc, ms, k, b, ld_b, n, out, ld_out, k_splits, nullptr, 0, nullptr, 0,
+                                status, stream);
+}
+
+extern "C" int sp24_spmm_accumulate_sums_f32(const void *a_packed, int dtype, int a_mn_major, int64_t ld_a, const void *e_tc, int64_t ms,
+                                             int64_t k, const void *b, int64_t ld_b, int64_t n, float *out, int64_t ld_out, int k_splits,
+                                             const float *row_parts, int64_t n_parts, float *row_sums, int sums_accumulate, int *status,
+                                             void *stream) {
+    if (!row_sums) return SP24_ERR_ARG;
+    return spmm_accumulate_impl(a_packed, dtype, a_mn_major, ld_a, e_tc, ms, k, b, ld_b, n, out, ld_out, k_splits, row_parts, n_parts, row_sums,
+                                sums_accumulate, status, stream);
 }

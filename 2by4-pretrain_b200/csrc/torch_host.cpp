@@ -244,7 +244,20 @@ Tensor sparse_linear(const Tensor &input, const Tensor &weight, const Tensor &e_
 }
 
 // out (ms, n) float32 += sparse @ dense (k, n)
-void mm_accumulate(const Tensor &out, const Tensor &weight, const Tensor &e_tc, const Tensor &dense_in, int64_t k_splits) {
+// Row sums that the compressing pass takes along (the bias gradient): `out` is set to them, or increased by them.  `parts` is
+// scratch for partial sums (row_parts_bytes), which are added up in a fixed order: a gradient repeats bit for bit.
+struct RowSums {
+    float *out = nullptr, *parts = nullptr;
+    bool add = false;
+};
+int64_t row_parts_bytes(int64_t m, int64_t k, at::ScalarType packed) { return 4 * m * sp24_row_parts(k, dt(packed)); }
+void sum_parts(const RowSums &s, int64_t m, int64_t k, at::ScalarType packed) {
+    check(sp24_sum_parts(s.parts, sp24_row_parts(k, dt(packed)), m, s.out, s.add, cur_stream()), "sp24_sum_parts");
+}
+
+// sums: the partial row sums of the compressed operand, added up by the same launch
+void mm_accumulate(const Tensor &out, const Tensor &weight, const Tensor &e_tc, const Tensor &dense_in, int64_t k_splits,
+                   const RowSums &sums = {}) {
     TORCH_CHECK(out.scalar_type() == at::kFloat && out.dim() == 2 && out.stride(1) == 1, "sparse_mm_accumulate_: out must be a row-major fp32 matrix");
     TORCH_CHECK(is16(weight.scalar_type()) && dense_in.scalar_type() == weight.scalar_type(),
                 "sparse_mm_accumulate_: expected matching fp16 / bf16 operands, got ", weight.scalar_type(), " and ", dense_in.scalar_type());
@@ -256,6 +269,13 @@ void mm_accumulate(const Tensor &out, const Tensor &weight, const Tensor &e_tc, 
     TORCH_CHECK(la.col >= 0, "sparse_mm_accumulate_: invalid strides for the packed values");
     Tensor dense = dense_in;
     if (dense.stride(1) != 1 || !aligned(dense) || (dense.stride(0) * dense.element_size()) % 16) dense = dense.contiguous();
+    if (sums.out) {
+        check(sp24_spmm_accumulate_sums_f32(ptr(weight), dt(weight.scalar_type()), la.col, la.ld, ptr(e_tc), ms, k, ptr(dense), dense.stride(0), n,
+                                            static_cast<float *>(ptr(out)), out.stride(0), (int)k_splits, sums.parts,
+                                            sp24_row_parts(k, dt(weight.scalar_type())), sums.out, sums.add, status_ptr(weight), cur_stream()),
+              "sp24_spmm_accumulate_sums_f32");
+        return;
+    }
     check(sp24_spmm_accumulate_f32(ptr(weight), dt(weight.scalar_type()), la.col, la.ld, ptr(e_tc), ms, k, ptr(dense), dense.stride(0), n,
                                    static_cast<float *>(ptr(out)), out.stride(0), (int)k_splits, status_ptr(weight), cur_stream()),
           "sp24_spmm_accumulate_f32");
@@ -269,21 +289,11 @@ void sparse_mm_accumulate(const Tensor &out, const Tensor &weight, const Tensor 
 // ---------------------------------------------------------------------------------------------
 // dense -> 2:4
 // ---------------------------------------------------------------------------------------------
-// Row sums that the compressing pass takes along (the bias gradient): `out` is set to them, or increased by them.  `parts` is
-// scratch for partial sums (row_parts_bytes), which are added up in a fixed order: a gradient repeats bit for bit.
-struct RowSums {
-    float *out = nullptr, *parts = nullptr;
-    bool add = false;
-};
-int64_t row_parts_bytes(int64_t m, int64_t k, at::ScalarType packed) { return 4 * m * sp24_row_parts(k, dt(packed)); }
-void sum_parts(const RowSums &s, int64_t m, int64_t k, at::ScalarType packed) {
-    check(sp24_sum_parts(s.parts, sp24_row_parts(k, dt(packed)), m, s.out, s.add, cur_stream()), "sp24_sum_parts");
-}
-
+// clear (fast MVUE of column-major values): a dense tensor that the same launch sets to zero.
 // Fills packed / meta from dense; returns the metadata in tensor-core order when it was asked for and the shape allows.
 OptTensor prune_into(const Tensor &dense_in, const Tensor &packed, const Tensor &meta, int64_t mode, const OptTensor &mask_in,
                      const OptTensor &uniforms_in, uint64_t seed, uint64_t offset, c10::optional<bool> emit_tc, const RowSums &sums = {},
-                     OptTensor e_tc = {}) {
+                     OptTensor e_tc = {}, const Tensor &clear = {}) {
     TORCH_CHECK(dense_in.dim() == 2, "Expected 2-dimensional dense tensor, got ", dense_in.dim(), "-dimensional tensor");
     const int64_t m = dense_in.size(0), k = dense_in.size(1);
     const Layout lp = layout_of(packed);
@@ -310,10 +320,15 @@ OptTensor prune_into(const Tensor &dense_in, const Tensor &packed, const Tensor 
     if (!uniforms.has_value()) x.offset_dev = rng_offset_ptr(mode);
     x.e_tc = const_cast<void *>(ptr(e_tc));
     x.row_parts = sums.parts;
-    check(sp24_prune_compress_with(ptr(dense), dt(dense.scalar_type()), m, k, layout_of(dense).ld, lp.col, ptr(packed),
-                                   dt(packed.scalar_type()), lp.ld, ptr(meta), (int)mode, ptr(mask), ld_m,
-                                   static_cast<const float *>(ptr(uniforms)), ld_u, seed, offset, &x, cur_stream()),
-          "sp24_prune_compress");
+    if (clear.defined())
+        check(sp24_mvue_compress_clearing(ptr(dense), dt(dense.scalar_type()), m, k, layout_of(dense).ld, ptr(packed), dt(packed.scalar_type()),
+                                          lp.ld, ptr(meta), seed, offset, &x, ptr(clear), clear.nbytes(), cur_stream()),
+              "sp24_mvue_compress_clearing");
+    else
+        check(sp24_prune_compress_with(ptr(dense), dt(dense.scalar_type()), m, k, layout_of(dense).ld, lp.col, ptr(packed),
+                                       dt(packed.scalar_type()), lp.ld, ptr(meta), (int)mode, ptr(mask), ld_m,
+                                       static_cast<const float *>(ptr(uniforms)), ld_u, seed, offset, &x, cur_stream()),
+              "sp24_prune_compress");
     if (sums.out) sum_parts(sums, m, k, packed.scalar_type());
     return e_tc;
 }
@@ -524,8 +539,7 @@ std::pair<Tensor, Tensor> fst_weight_grads(const Tensor &g_in, const Tensor &x, 
             acc = weight.grad();
             if (need_b && accumulable(bias.grad())) sums = bias.grad();
         } else if (f32) {
-            acc = gw = empty({out_f, in_f}, at::kFloat, g);
-            check(sp24_zero(ptr(gw), out_f * in_f * 4, cur_stream()), "sp24_zero");
+            acc = gw = empty({out_f, in_f}, at::kFloat, g);      // the compression clears it for the GEMM that adds to it
             if (need_b && bias.scalar_type() == at::kFloat) sums = gb = empty({out_f}, at::kFloat, g);
         }
         // packed values, metadata, its tensor-core copy and partial bias sums, all consumed by the next launches
@@ -539,10 +553,10 @@ std::pair<Tensor, Tensor> fst_weight_grads(const Tensor &g_in, const Tensor &x, 
         if (tc) e = carve(buf, o_tc, at::kByte, {sp24_meta_tc_bytes(out_f, tokens)}, {1});
         RowSums rs;
         if (sums.defined()) rs = {static_cast<float *>(ptr(sums)), reinterpret_cast<float *>(static_cast<char *>(ptr(buf)) + o_parts), into};
-        prune_into(g.t(), gp, gm, SP24_PRUNE_MVUE_FAST, {}, {}, seed, 0, false, rs, e);
+        prune_into(g.t(), gp, gm, SP24_PRUNE_MVUE_FAST, {}, {}, seed, 0, false, {nullptr, rs.parts, false}, e, gw);
         if (sums.defined()) need_b = false;
         TORCH_CHECK(tc, "sparse GEMM on sm_100a: number of rows of the sparse matrix must be divisible by 128");
-        if (acc.defined()) mm_accumulate(acc, gp, *e, x, 0);
+        if (acc.defined()) mm_accumulate(acc, gp, *e, x, 0, rs);
         else gw = spmm(x.t(), gp, *e, {}, 0, {}, false).t();
     }
     if (need_b) gb = g_in.sum(0);
@@ -647,7 +661,7 @@ Tensor quantizable(const Tensor &t) {
 struct Q8 { Tensor packed, meta, tc; };
 // e4m3 2:4 compression of the logical (m, k) matrix `dense` under the scale of *amax, packed values row-major.
 Q8 compress_q8(const Tensor &dense_in, int mode, const OptTensor &mask_in, const Tensor &amax, uint64_t seed, const Tensor &row_sums,
-               const Tensor &q_dense) {
+               const Tensor &q_dense, const Tensor &clear = {}) {
     const int64_t m = dense_in.size(0), k = dense_in.size(1);
     TORCH_CHECK(m % 32 == 0 && k % 128 == 0, "compress_q8: shape (", m, ", ", k, "): rows % 32 == 0 and columns % 128 == 0 required");
     Tensor dense = dense_in;
@@ -683,9 +697,16 @@ Q8 compress_q8(const Tensor &dense_in, int mode, const OptTensor &mask_in, const
         x.q_dense = ptr(q_dense);
         x.ld_q = q_dense.size(1);
     }
-    check(sp24_prune_compress_with(ptr(dense), dt(dense.scalar_type()), m, k, l.ld, l.col, ptr(o.packed), SP24_E4M3, k / 2, ptr(o.meta), mode,
-                                   ptr(mask), ld_m, nullptr, 0, seed, 0, &x, cur_stream()),
-          "sp24_prune_compress_q8");
+    if (clear.defined() && l.col)
+        check(sp24_mvue_compress_clearing(ptr(dense), dt(dense.scalar_type()), m, k, l.ld, ptr(o.packed), SP24_E4M3, k / 2, ptr(o.meta), seed, 0,
+                                          &x, ptr(clear), clear.nbytes(), cur_stream()),
+              "sp24_mvue_compress_clearing");
+    else {
+        if (clear.defined()) check(sp24_zero(ptr(clear), clear.nbytes(), cur_stream()), "sp24_zero");
+        check(sp24_prune_compress_with(ptr(dense), dt(dense.scalar_type()), m, k, l.ld, l.col, ptr(o.packed), SP24_E4M3, k / 2, ptr(o.meta),
+                                       mode, ptr(mask), ld_m, nullptr, 0, seed, 0, &x, cur_stream()),
+              "sp24_prune_compress_q8");
+    }
     if (sums.out) sum_parts(sums, m, k, at::kFloat8_e4m3fn);
     return o;
 }
@@ -762,8 +783,7 @@ struct Fp8Backward : torch::autograd::Node {
             const Tensor xq_t = xq_t_.unpack();
             const int64_t in_f = xq_t.size(0);
             Tensor gw = empty({of, in_f}, at::kFloat, g), gb = need_b ? empty({of}, at::kFloat, g) : Tensor();
-            check(sp24_zero(ptr(gw), of * in_f * 4, cur_stream()), "sp24_zero");
-            const Q8 c = compress_q8(g.t(), SP24_PRUNE_MVUE_FAST, {}, amax, seed, gb, gq);
+            const Q8 c = compress_q8(g.t(), SP24_PRUNE_MVUE_FAST, {}, amax, seed, gb, gq, gw);
             TORCH_CHECK(c.tc.defined(), "sparse GEMM on sm_100a: number of rows of the sparse matrix must be divisible by 128");
             check(sp24_spmm_f8(ptr(c.packed), SP24_E4M3, n / 2, ptr(c.tc), of, n, ptr(xq_t), n, in_f, ptr(gw), SP24_F32, 0, in_f, nullptr,
                                static_cast<const float *>(ptr(amax)), static_cast<const float *>(ptr(amax_x_)), status_ptr(g), cur_stream()),

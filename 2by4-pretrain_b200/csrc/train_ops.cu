@@ -556,12 +556,7 @@ __global__ void __launch_bounds__(256) sum_parts_kernel(const float *parts, int6
     __shared__ float part[8][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t c = (int64_t)blockIdx.x * 32 + lane;
-    float s = 0.f;
-    if (c < m) {
-#pragma unroll 8
-        for (int64_t p = warp; p < n_parts; p += 8) s += parts[p * m + c];
-    }
-    part[warp][lane] = s;
+    part[warp][lane] = c < m ? sum_every_eighth(parts + c, n_parts, m, warp) : 0.f;
     __syncthreads();
     if (warp == 0 && c < m) {
         float t = 0.f;

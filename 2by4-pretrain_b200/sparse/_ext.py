@@ -53,6 +53,10 @@ _SIGNATURES = {
     "sp24_row_parts": [_i64, _i32],
     "sp24_prune_compress_with": [_vp, _i32, _i64, _i64, _i64, _i32, _vp, _i32, _i64, _vp, _i32, _vp, _i64, _vp, _i64, _u64, _u64,
                                  ctypes.POINTER(PruneExtras), _vp],
+    "sp24_mvue_compress_clearing": [_vp, _i32, _i64, _i64, _i64, _vp, _i32, _i64, _vp, _u64, _u64, ctypes.POINTER(PruneExtras), _vp, _i64,
+                                    _vp],
+    "sp24_spmm_accumulate_sums_f32": [_vp, _i32, _i32, _i64, _vp, _i64, _i64, _vp, _i64, _i64, _vp, _i64, _i32, _vp, _i64, _vp, _i32, _vp,
+                                      _vp],
     "sp24_sum_parts": [_vp, _i64, _i64, _vp, _i32, _vp],
     "sp24_spmm_f8": [_vp, _i32, _i64, _vp, _i64, _i64, _vp, _i64, _i64, _vp, _i32, _i32, _i64, _vp, _vp, _vp, _vp, _vp],
     "sp24_soft_threshold24_compress": [_vp, _i32, _i64, _i64, _i64, _i32, _vp, _i32, _i64, _vp, _i32, _f32, _vp, _vp],

@@ -187,6 +187,13 @@ int sp24_prune_compress_with(const void *dense, int dense_dtype, int64_t m, int6
                              const float *uniforms, int64_t ld_uniforms, uint64_t seed, uint64_t offset, const sp24_prune_extras *extras,
                              void *stream);
 int sp24_sum_parts(const float *parts, int64_t n_parts, int64_t m, float *out, int accumulate, void *stream);
+/*
+ * SP24_PRUNE_MVUE_FAST of a column-major matrix (dY^T), as sp24_prune_compress_with does it, which also clears zero_bytes
+ * (a multiple of 16) at `zero` (16-byte aligned): the buffer that the weight-gradient GEMM after it adds to.
+ */
+int sp24_mvue_compress_clearing(const void *dense, int dense_dtype, int64_t m, int64_t k, int64_t ld_dense, void *packed,
+                                int packed_dtype, int64_t ld_packed, void *meta, uint64_t seed, uint64_t offset,
+                                const sp24_prune_extras *extras, void *zero, int64_t zero_bytes, void *stream);
 
 /*
  * 2:4 compressed -> dense (zeros at pruned positions).  Replaces
@@ -442,6 +449,14 @@ int sp24_spmm_f8(const void *a_packed, int dtype, int64_t ld_a, const void *e_tc
 int sp24_spmm_accumulate_f32(const void *a_packed, int dtype, int a_mn_major, int64_t ld_a, const void *e_tc,
                              int64_t ms, int64_t k, const void *b, int64_t ld_b, int64_t n, float *out,
                              int64_t ld_out, int k_splits, int *status, void *stream);
+/*
+ * The same, and row_sums[r] = sum over p of row_parts[p * ms + r] (sums_accumulate = 1: added to what row_sums holds), in the
+ * order of sp24_sum_parts: the bias gradient from the parts that the compression of dY^T left.
+ */
+int sp24_spmm_accumulate_sums_f32(const void *a_packed, int dtype, int a_mn_major, int64_t ld_a, const void *e_tc, int64_t ms,
+                                  int64_t k, const void *b, int64_t ld_b, int64_t n, float *out, int64_t ld_out, int k_splits,
+                                  const float *row_parts, int64_t n_parts, float *row_sums, int sums_accumulate, int *status,
+                                  void *stream);
 
 /*
  * Two streaming kernels of the trainer around the sparse GEMMs.  No counterpart in the reference, whose model and
