@@ -914,7 +914,9 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     const uint32_t rank = cluster_ctarank();          // 0 = leader
     const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
     const int n_tiles_n = (int)((P.n + BN - 1) / BN);
-    const int n_tiles_m = (int)(P.ms / (2 * BM));     // 256-row blocks: one 128-row block per CTA
+    // 256-row blocks, one 128-row block per CTA.  Where ms is an odd multiple of 128 the last one's second block lies past the operand:
+    // its loads give zeros and its results are not stored.
+    const int n_tiles_m = (int)((P.ms + 2 * BM - 1) / (2 * BM));
     const int n_tiles = n_tiles_n * n_tiles_m;        // row block varies fastest over the tile index
     const int k_iters = (int)((P.k + KE - 1) / KE);
 
@@ -1065,7 +1067,7 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             const bool ok = mbar_wait(tmem_full0 + 8 * buf, (tl >> 1) & 1, &abort_flag, P.status, 3);
             tc_fence_after();
             if (threadIdx.x == 64) SP24_TRACE(2, 4 * tl);
-            const bool run = __all_sync(0xFFFFFFFFu, ok && !abort_flag);      // the warp reads tensor memory together
+            const bool run = __all_sync(0xFFFFFFFFu, ok && !abort_flag) && mrow < P.ms;      // the warp reads tensor memory together
             if constexpr (EPI == EPI_PLAIN) {
                 const int64_t left = P.n - row0;
                 const int limit = left < BN ? (int)left : BN, chunks = (limit + 15) / 16;
@@ -1257,7 +1259,7 @@ spmm_pair_acc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     const uint32_t rank = cluster_ctarank();
     const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
     const int n_tiles_n = (int)((P.n + BN - 1) / BN);
-    const int n_tiles_m = (int)(P.ms / (2 * BM));
+    const int n_tiles_m = (int)((P.ms + 2 * BM - 1) / (2 * BM));      // as in spmm_pair_kernel
     const int n_tiles = n_tiles_n * n_tiles_m;
     const int n_units = n_tiles * P.k_splits;     // unit u = (tile u % n_tiles, K slice u / n_tiles)
     const int k_iters = (int)((P.k + 127) / 128);
@@ -1399,7 +1401,7 @@ spmm_pair_acc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
             const int col0 = (tile / n_tiles_m) * BN + half * HC;
             const bool ok = mbar_wait(tmem_full, tl & 1, &abort_flag, P.status, 3);
             tc_fence_after();
-            const bool run = __all_sync(0xFFFFFFFFu, ok && !abort_flag);
+            const bool run = __all_sync(0xFFFFFFFFu, ok && !abort_flag) && mrow < P.ms;
             if (run) {
                 const uint32_t acc = tmem_base + ((uint32_t)(quad * 32) << 16) + half * HC;
 #pragma unroll 1
@@ -1598,7 +1600,7 @@ int launch_spmm_pair(const CUtensorMap &ma, const CUtensorMap &mb, const CUtenso
     // M = 256 over the CTA pair, N = bn
     P.idesc = (P.idesc & ~(0x1Fu << 24)) | ((uint32_t)(256 >> 4) << 24) | ((uint32_t)(P.bn >> 3) << 17);
     P.stages = two::stages2(F8, P.bn);
-    const int64_t tiles = ((P.n + P.bn - 1) / P.bn) * (P.ms / 256);
+    const int64_t tiles = ((P.n + P.bn - 1) / P.bn) * ((P.ms + 255) / 256);
     const int64_t pairs_max = sm_count_cached() / 2;
     const unsigned pairs = (unsigned)(tiles < pairs_max ? tiles : pairs_max);
     cudaLaunchConfig_t cfg{};
@@ -1633,7 +1635,7 @@ int launch_spmm_pair_acc(const CUtensorMap &ma, const CUtensorMap &mb, const CUt
     }
     // M = 256 over the CTA pair, N = 256
     P.idesc = (P.idesc & ~(0x1Fu << 24)) | ((uint32_t)(256 >> 4) << 24) | ((uint32_t)(two::BN3 >> 3) << 17);
-    const int64_t tiles = ((P.n + two::BN3 - 1) / two::BN3) * (P.ms / 256);
+    const int64_t tiles = ((P.n + two::BN3 - 1) / two::BN3) * ((P.ms + 255) / 256);
     const int64_t pairs_max = sm_count_cached() / 2;
     const int64_t k_iters = (P.k + 127) / 128;
     int64_t splits = k_splits ? k_splits : pairs_max / tiles;
@@ -1685,7 +1687,7 @@ void pick_tile(int64_t ms, int64_t n, int sm_count, int &bn_out, int &mpt_out) {
 //   ms 768, n 5000, k 1024: 11.8 -> 9.2 (224)
 // Few columns: the narrowest tile that still takes one round; single-CTA kernel -> here:
 //   ms 4096, k 4096: n 16 19.8 -> 13.2, n 256 20.8 -> 14.6, n 512 21.7 -> 15.5, n 768 24.0 -> 16.2; ms 768, k 3072, n 512 16.4 -> 11.5
-// (the single-CTA kernel was never faster, so it keeps the row counts that are odd multiples of 128 and the other layouts).
+// (the single-CTA kernel was never faster, so it keeps what pair_takes_rows leaves it and the other layouts).
 // The fused epilogues hold up to 192 columns in registers and take them in chunks of 16 per half tile.  8-bit operands: with
 // cta_group::2 and M = 256, kind::f8f6f4 takes N in multiples of 32 (kind::f16, sparse: of 16; the ranges of CUTLASS's
 // SM100_MMA_F8F6F4_2x1SM_SS_SPARSE and SM100_MMA_F16BF16_2x1SM_SS_SPARSE).
@@ -1695,11 +1697,24 @@ int pick_pair_bn(int64_t ms, int64_t n, bool plain, bool f8, int sms) {
     int best = widest;
     int64_t best_cost = INT64_MAX;
     for (int bn = widest; bn >= two::BN2_MIN; bn -= step) {
-        const int64_t tiles = ((n + bn - 1) / bn) * (ms / 256);
+        const int64_t tiles = ((n + bn - 1) / bn) * ((ms + 255) / 256);
         const int64_t cost = ((tiles + pairs - 1) / pairs) * two::stage2_bytes(f8, bn);
         if (cost < best_cost) { best_cost = cost; best = bn; }
     }
     return best;
+}
+
+// Whether the CTA-pair kernel takes an operand whose last 256-row block is half empty (ms an odd multiple of 128).  Mostly yes, us,
+// single-CTA kernel -> pairs: fp16 ms 896, n 1984, k 1152 8.7 -> 7.9, n 8192, k 3072 43.5 -> 27.7; ms 2944, n 16384, k 768 53.7 -> 49.2;
+// ms 128, n 256, k 512 5.4 -> 4.4; float8 ms 1152, n 8192, k 3072 46.1 -> 20.8.  Not where many columns meet few K steps, so that the
+// epilogue decides and the empty half's does nothing: ms 384, n 16384, k 256 9.1 -> 10.3; ms 384, n 4096, k 512 6.0 -> 6.3; ms 1152,
+// n 16384, k 256 17.1 -> 18.3; ms 128, n 8192, k 512 6.1 -> 6.7; float8 ms 128, n 16384, k 1024 8.5 -> 8.9.  (Also left to the single
+// CTAs by the third line although pairs are faster there: ms 384, n 16384, k 512 13.0 -> 11.6.)
+bool pair_takes_rows(int64_t ms, int64_t n, int64_t k, bool f8) {
+    if (ms % 256 == 0 || n <= 2560) return true;
+    if (k <= 256) return false;
+    if (k <= 512 && ms <= 384) return false;
+    return ms > 128 || n <= 5120 || k > (f8 ? 1024 : 768);
 }
 
 // Tile and K slices of the float8 weight gradient (added to out with float32 reductions).  At most two slices: two addends on a
@@ -1792,9 +1807,9 @@ static int spmm_impl(const void *a_packed, int dtype, int a_mn_major, int64_t ld
     if (!aligned16(e_tc)) return SP24_ERR_ALIGN;
     const bool i8 = dtype == SP24_I8;
     const bool f8 = dtype == SP24_E4M3 || dtype == SP24_E5M2 || i8;   // 8-bit operand geometry
-    // CTA-pair kernel: 16-bit types, token-major B and output, whole 256-row blocks, no activation; the fused MLP
-    // epilogues and the float32 bias exist in that kernel only
-    const bool pair_ok = !f8 && !b_mn_major && trans_out && ms % 256 == 0 && activation == 0;
+    // CTA-pair kernel: 16-bit types, token-major B and output, no activation; the fused MLP epilogues and the float32 bias exist in
+    // that kernel only and for whole 256-row blocks
+    const bool pair_layout = !f8 && !b_mn_major && trans_out && activation == 0, pair_ok = pair_layout && ms % 256 == 0;
     if (epi != EPI_PLAIN && (!pair_ok || !aux || ld_aux < ms || (ld_aux * 2) % 16 || !aligned16(aux))) return SP24_ERR_ARG;
     if (bias_f32 && !pair_ok) return SP24_ERR_ARG;
     if (int rc = check_device()) return rc;
@@ -1825,7 +1840,7 @@ static int spmm_impl(const void *a_packed, int dtype, int a_mn_major, int64_t ld
     P.idesc = (1u << 2) | ((i8 ? 2u : 1u) << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(a_mn_major ? 1 : 0) << 15) |
               ((uint32_t)(b_mn_major ? 1 : 0) << 16) | ((uint32_t)(BM >> 4) << 24);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    bool pair_form = pair_ok && pair_kernels_enabled();
+    bool pair_form = pair_layout && pair_takes_rows(ms, n, k, false) && pair_kernels_enabled();
     if (epi != EPI_PLAIN || bias_f32) pair_form = true;      // checked above: these forms exist in the pair kernel only
     if (pair_form) {
         CUtensorMap map_b, map_e;
@@ -1901,7 +1916,7 @@ extern "C" int sp24_pair_tile_columns(int64_t ms, int64_t n, int form, int sms) 
 // The GEMMs of a float8 layer whose scales stay on the device: D = alpha * (A_sparse * B) [+ float32 bias], alpha = the
 // product of the operands' scales, worked out from their absolute maxima (sp24_absmax).
 //   trans_out = 1: out (n, ms) in float32, float16 or bfloat16 (rounded once): the layer's output or input gradient
-//   without a float32 copy.  16-bit outputs of whole 256-row blocks run on CTA pairs.
+//   without a float32 copy.  16-bit outputs run on CTA pairs (see pair_takes_rows).
 //   trans_out = 0: out (ms, n) float32 += alpha * A * B (no bias), K cut into up to two slices: the weight gradient.
 extern "C" int sp24_spmm_f8(const void *a_packed, int dtype, int64_t ld_a, const void *e_tc, int64_t ms, int64_t k, const void *b, int64_t ld_b,
                             int64_t n, void *out, int out_dtype, int trans_out, int64_t ld_out, const float *bias, const float *amax_a,
@@ -1920,7 +1935,7 @@ extern "C" int sp24_spmm_f8(const void *a_packed, int dtype, int64_t ld_a, const
     const uint32_t fmt = dtype == SP24_E5M2 ? 1u : 0u;
     P.idesc = (1u << 2) | (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(BM >> 4) << 24);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (trans_out && out_dtype != SP24_F32 && ms % 256 == 0 && pair_kernels_enabled()) {
+    if (trans_out && out_dtype != SP24_F32 && pair_takes_rows(ms, n, k, true) && pair_kernels_enabled()) {
         CUtensorMap map_e;
         P.bn = pick_pair_bn(ms, n, true, true, sm_count_cached());
         if (int rc = make_map(&map_b, b, dtype, n, k, ld_b, 128, (uint32_t)P.bn / 2)) return rc;
@@ -2082,8 +2097,10 @@ static int spmm_accumulate_impl(const void *a_packed, int dtype, int a_mn_major,
     P.idesc = (1u << 2) | (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(a_mn_major ? 1 : 0) << 15) | (1u << 16) |
               ((uint32_t)(BM >> 4) << 24);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    // CTA-pair kernel for whole 256-row blocks and at least one full tile of columns
-    bool pair_form = ms % 256 == 0 && n >= 256;
+    // CTA-pair kernel for at least one full tile of columns, also where the last 256-row block is half empty: us, single CTAs -> pairs,
+    // ms 384, n 256, k 1024 10.3 -> 6.7; ms 1152, n 1152, k 1984 15.2 -> 9.9; ms 2944, n 768, k 16384 51.6 -> 38.5; ms 128, n 768, k 2048
+    // 7.3 -> 7.2
+    bool pair_form = n >= 256;
     pair_form = pair_form && pair_kernels_enabled();
     if (pair_form) {
         CUtensorMap map_e;
