@@ -1224,30 +1224,32 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 // so that no chunk waits for another; a pair with more units stages chunk by chunk beside its ring, which is filling again.
 namespace two {
 constexpr int BN3 = 256;
-constexpr int B3_BYTES = (BN3 / 2) * 256;                  // 128 columns x 128 K-rows x 2 bytes
-constexpr int STAGE3_BYTES = A_STAGE_BYTES + B3_BYTES + 2048;   // 51200
+constexpr int B3_BYTES = (BN3 / 2) * 256;                  // 128 columns x 128 K-rows x 2 bytes (float8: x 256 x 1)
 constexpr int STAGES3 = 4;
+constexpr int stage3_bytes(bool f8) { return A_STAGE_BYTES + B3_BYTES + e2_bytes(f8); }   // 51200, float8 53248
 // Epilogue staging: a box is 16 rows x 32 columns, 128-byte rows in the 128-byte swizzle of the output's tensor map; a chunk is
 // the two boxes of a warp's 32 rows.
 constexpr int BOX3_BYTES = 16 * 128, CHUNKS3 = BN3 / 2 / 32;
 constexpr int STAGING3 = 8 * BOX3_BYTES;                    // one box per epilogue warp
-constexpr int SMEM3 = STAGES3 * STAGE3_BYTES + STAGING3 + 1024;
-static_assert(8 * CHUNKS3 * 2 * BOX3_BYTES <= STAGES3 * STAGE3_BYTES, "an idle operand ring holds a whole tile");
-static_assert(STAGE3_BYTES % 1024 == 0, "stages must keep the 1024-byte swizzle alignment");
-static_assert(SMEM3 <= 227 * 1024, "shared memory budget");
+constexpr int smem3(bool f8) { return STAGES3 * stage3_bytes(f8) + STAGING3 + 1024; }
+static_assert(8 * CHUNKS3 * 2 * BOX3_BYTES <= STAGES3 * stage3_bytes(false), "an idle operand ring holds a whole tile");
+static_assert(stage3_bytes(false) % 1024 == 0 && stage3_bytes(true) % 1024 == 0, "stages must keep the 1024-byte swizzle alignment");
+static_assert(smem3(true) <= SMEM_LIMIT, "shared memory budget");
 }  // namespace two
 
-template <bool A_MN>
+// Float8 (F8): both operands K-major (B stored (n, k)), K step 256, the accumulator times the product of the operands' scales.
+template <bool A_MN, bool F8>
 __global__ void __launch_bounds__(320, 1)
 spmm_pair_acc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                      const __grid_constant__ CUtensorMap map_e, const __grid_constant__ CUtensorMap map_d, SpmmParams P) {
     using namespace two;
+    static_assert(!(A_MN && F8), "8-bit operands are K-major");
     constexpr int BN = BN3;
-    constexpr int STAGES = STAGES3;
+    constexpr int STAGES = STAGES3, STAGE3_BYTES = stage3_bytes(F8), KE = F8 ? 256 : 128;
     constexpr int OFF_B = A_STAGE_BYTES, OFF_E = OFF_B + B3_BYTES;
     constexpr int KSTEPS = 4;
     constexpr uint32_t TMEM_COLS = 512;
-    constexpr int E_COL0 = BN, E_SLOT = 4;       // one accumulator, then two metadata slots
+    constexpr int E_COL0 = BN, E_SLOT = F8 ? 8 : 4;       // one accumulator, then two metadata slots
 
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -1262,7 +1264,7 @@ spmm_pair_acc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     const int n_tiles_m = (int)((P.ms + 2 * BM - 1) / (2 * BM));      // as in spmm_pair_kernel
     const int n_tiles = n_tiles_n * n_tiles_m;
     const int n_units = n_tiles * P.k_splits;     // unit u = (tile u % n_tiles, K slice u / n_tiles)
-    const int k_iters = (int)((P.k + 127) / 128);
+    const int k_iters = (int)((P.k + KE - 1) / KE);
 
     const uint32_t full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[STAGES]);
     const uint32_t tmem_full = smem_u32(&bars[2 * STAGES]), tmem_empty = smem_u32(&bars[2 * STAGES + 1]);
@@ -1293,7 +1295,7 @@ spmm_pair_acc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         if (lane == 0) {
             int g = 0;
             bool ok = true;
-            constexpr uint32_t cta_tx = A_STAGE_BYTES + 2048 + B3_BYTES;
+            constexpr uint32_t cta_tx = STAGE3_BYTES;
             for (int unit = pair; unit < n_units && ok; unit += n_pairs) {
                 const int tile = unit % n_tiles, ks = unit / n_tiles;
                 const int it0 = (int)((int64_t)ks * k_iters / P.k_splits), it1 = (int)((int64_t)(ks + 1) * k_iters / P.k_splits);
@@ -1309,15 +1311,20 @@ spmm_pair_acc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                     const uint32_t full_leader = map_to_cta(full0 + 8 * s, 0);
                     if (rank == 0) mbar_expect_tx(full0 + 8 * s, 2 * cta_tx);
                     if constexpr (!A_MN) {
-                        tma_load_2d_pair(sa, &map_a, it * 64, mrow, full_leader);
+                        tma_load_2d_pair(sa, &map_a, it * (KE / 2), mrow, full_leader);
                     } else {
                         tma_load_2d_pair(sa, &map_a, mrow, it * 64, full_leader);
                         tma_load_2d_pair(sa + 8192, &map_a, mrow + 64, it * 64, full_leader);
                     }
-                    tma_load_2d_pair(sa + OFF_E, &map_e, 0, (int)(((int64_t)mblk * P.k_atoms + it) * 2), full_leader);
-                    // this CTA's 128 columns of B: two boxes of 64 columns x 128 K-rows
-                    tma_load_2d_pair(sb, &map_b, bcol, it * 128, full_leader);
-                    tma_load_2d_pair(sb + 16384, &map_b, bcol + 64, it * 128, full_leader);
+                    tma_load_2d_pair(sa + OFF_E, &map_e, 0, (int)(((int64_t)mblk * P.k_atoms + it * (F8 ? 2 : 1)) * 2), full_leader);
+                    // this CTA's 128 columns of B: two boxes of 64 columns x 128 K-rows, or of 128 columns x 128 bytes of K
+                    if constexpr (F8) {
+                        tma_load_2d_pair(sb, &map_b, it * KE, bcol, full_leader);
+                        tma_load_2d_pair(sb + 16384, &map_b, it * KE + 128, bcol, full_leader);
+                    } else {
+                        tma_load_2d_pair(sb, &map_b, bcol, it * 128, full_leader);
+                        tma_load_2d_pair(sb + 16384, &map_b, bcol + 64, it * 128, full_leader);
+                    }
                 }
             }
             if (abort_flag && rank == 0) {
@@ -1333,10 +1340,10 @@ spmm_pair_acc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         // ---------------------------------------------------------------- MMA issuer (leader CTA only)
         if (rank == 0) {                       // all lanes in step, one elected lane issues (as in spmm_pair_kernel)
             constexpr uint32_t A_LBO = A_MN ? 8192 : 16, A_KSTEP = A_MN ? 2048 : 32;
-            const uint32_t idesc0 = P.idesc;   // M = 256, N = 256, B MN-major set by the launcher
+            const uint32_t idesc0 = P.idesc;   // M = 256, N = 256, operand majors set by the launcher
             const uint32_t smem0 = smem_u32(smem);
-            // MN-major B: 64-column blocks 16384 bytes apart, 32 K-rows (4096 bytes) per MMA
-            const uint64_t adesc0 = make_desc(smem0, A_LBO, 1024, 2), bdesc0 = make_desc(smem0 + OFF_B, 16384, 1024, 2);
+            // MN-major B: 64-column blocks 16384 bytes apart, 32 K-rows (4096 bytes) per MMA; K-major: 64 bytes per MMA, two K atoms
+            const uint64_t adesc0 = make_desc(smem0, A_LBO, 1024, 2), bdesc0 = make_desc(smem0 + OFF_B, F8 ? 16 : 16384, 1024, 2);
             const uint64_t edesc0 = make_desc(smem0 + OFF_E, 16, 128, 0);
             int s = 0, tl = 0;
             uint32_t ph = 0, eslot = 0;
@@ -1355,10 +1362,13 @@ spmm_pair_acc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                     const uint32_t e_cols = tmem_base + E_COL0 + eslot;
                     if (elect_one()) {
                         tc_cp_128x128b_pair(e_cols, ed);
+                        if constexpr (F8) tc_cp_128x128b_pair(e_cols + 4, ed + (2048 >> 4));
 #pragma unroll
                         for (int j = 0; j < KSTEPS; ++j)
-                            mma_sp_pair(tmem_base, ad + j * (A_KSTEP >> 4), bd + j * (4096 >> 4), e_cols + (j & ~1), idesc0 | (j & 1),
-                                        (it > it0 || j > 0) ? 1u : 0u);
+                            mma_sp_pair_any<F8>(tmem_base, ad + j * (A_KSTEP >> 4),
+                                                bd + (F8 ? (j >> 1) * (16384 >> 4) + (j & 1) * (64 >> 4) : j * (4096 >> 4)),
+                                                e_cols + (F8 ? 2 * j : (j & ~1)), F8 ? idesc0 : idesc0 | (j & 1),
+                                                (it > it0 || j > 0) ? 1u : 0u);
                         tc_commit_pair(empty0 + 8 * s);
                     }
                     __syncwarp();
@@ -1374,6 +1384,7 @@ spmm_pair_acc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         const int quad = warp & 3, half = (warp - 2) >> 2;
         constexpr int HC = BN / 2;                     // 128 columns per warp
         const uint32_t empty_leader = map_to_cta(tmem_empty, 0);
+        const float alpha = F8 ? alpha_of(P) : 1.f;
         const bool idle_ring = n_units <= n_pairs;     // this pair's only unit: the operand ring is free when it is complete
         const uint32_t stg = smem_u32(smem) + (idle_ring ? (warp - 2) * CHUNKS3 * 2 * BOX3_BYTES
                                                          : STAGES3 * STAGE3_BYTES + (warp - 2) * BOX3_BYTES);
@@ -1409,6 +1420,10 @@ spmm_pair_acc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                     uint32_t v[32];
                     tmem_ld32(acc + c * 32, v);
                     tmem_ld_wait();
+                    if constexpr (F8) {
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * alpha);
+                    }
                     const int x = col0 + c * 32;
                     // a lane's row of 128 bytes at `row`, its eight 16-byte pieces in the map's 128-byte swizzle
                     auto put = [&](uint32_t row) {
@@ -1621,15 +1636,15 @@ int launch_spmm_pair(const CUtensorMap &ma, const CUtensorMap &mb, const CUtenso
     return launch_status();
 }
 
-template <bool A_MN>
+template <bool A_MN, bool F8 = false>
 int launch_spmm_pair_acc(const CUtensorMap &ma, const CUtensorMap &mb, const CUtensorMap &me, const CUtensorMap &md, SpmmParams P,
                          int k_splits, cudaStream_t st) {
-    auto kern = spmm_pair_acc_kernel<A_MN>;
+    auto kern = spmm_pair_acc_kernel<A_MN, F8>;
     static bool attr_set[64];
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, two::SMEM3) != cudaSuccess)
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, two::smem3(F8)) != cudaSuccess)
             return launch_status();
         attr_set[dev] = true;
     }
@@ -1637,17 +1652,18 @@ int launch_spmm_pair_acc(const CUtensorMap &ma, const CUtensorMap &mb, const CUt
     P.idesc = (P.idesc & ~(0x1Fu << 24)) | ((uint32_t)(256 >> 4) << 24) | ((uint32_t)(two::BN3 >> 3) << 17);
     const int64_t tiles = ((P.n + two::BN3 - 1) / two::BN3) * ((P.ms + 255) / 256);
     const int64_t pairs_max = sm_count_cached() / 2;
-    const int64_t k_iters = (P.k + 127) / 128;
+    const int64_t k_iters = (P.k + (F8 ? 255 : 127)) / (F8 ? 256 : 128);
     int64_t splits = k_splits ? k_splits : pairs_max / tiles;
     if (splits < 1) splits = 1;
     if (splits > k_iters) splits = k_iters;
+    if (F8 && splits > 2) splits = 2;       // two addends on a cleared buffer give the same bits in either order, three do not
     P.k_splits = (int)splits;
     const int64_t units = tiles * splits;
     const unsigned pairs = (unsigned)(units < pairs_max ? units : pairs_max);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(2 * pairs, 1, 1);
     cfg.blockDim = dim3(320, 1, 1);
-    cfg.dynamicSmemBytes = two::SMEM3;
+    cfg.dynamicSmemBytes = two::smem3(F8);
     cfg.stream = st;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1951,6 +1967,16 @@ extern "C" int sp24_spmm_f8(const void *a_packed, int dtype, int64_t ld_a, const
         const int64_t tiles = ((n + 127) / 128) * ((ms / BM + 1) / 2);
         bn = 128;
         mpt = tiles >= sms ? 2 : 1;
+    }
+    // Weight gradient on CTA pairs: us, single CTAs -> pairs, ms 3072, n 768, k 8192 28.4 -> 15.3; ms 3072, n 3072, k 8192 89.8 -> 41.1;
+    // ms 768, n 768, k 8192 16.2 -> 12.2; ms 1280, n 640, k 4096 11.3 -> 8.9; ms 2304, n 768, k 256 6.9 both.  Below these sizes the pair
+    // kernel's longer start counts: ms 1024, n 1024, k 1024 7.0 -> 7.2; ms 2048, n 512, k 512 6.4 -> 6.9; ms 256, n 256, k 256 5.7 -> 6.4.
+    if (!trans_out && n >= 256 && (k >= 2048 || ms * n >= 3 << 19) && pair_kernels_enabled()) {
+        CUtensorMap map_e, map_d;
+        if (int rc = make_map(&map_b, b, dtype, n, k, ld_b, 128, 128)) return rc;
+        if (int rc = make_map_e(&map_e, e_tc, (ms / 128) * P.k_atoms, 2)) return rc;
+        if (int rc = encode_map(&map_d, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, out, n, ms, ld_out * 4, 32, 16, CU_TENSOR_MAP_SWIZZLE_128B)) return rc;
+        return launch_spmm_pair_acc<false, true>(map_a, map_b, map_e, map_d, P, 0, st);
     }
     if (!trans_out) {
         pick_f8_accumulate(ms, n, k, sms, bn, mpt, P.k_splits);
