@@ -60,8 +60,25 @@ extern "C" const char *sp24_strerror(int code) {
 
 extern "C" int sp24_abi_version(void) { return 2; }
 
+namespace sp24 {
+namespace {
+__global__ void __launch_bounds__(256) clear_kernel(uint32_t *dst, int64_t words) {
+    chain_enter();
+    for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < words; i += (int64_t)gridDim.x * 256) dst[i] = 0;
+}
+}  // namespace
+}  // namespace sp24
+
+// Small buffers are cleared by a kernel: a memset in the stream ends the overlap of the kernels around it (launch_chained).
+// The float8 layer step, with three such words: 153.8 -> 146.5 us (8192 tokens, 768 -> 3072).
 extern "C" int sp24_zero(void *dst, int64_t bytes, void *stream) {
     if (!dst || bytes < 0) return SP24_ERR_ARG;
+    if (bytes > 0 && bytes <= 1 << 18 && bytes % 4 == 0 && (reinterpret_cast<uintptr_t>(dst) & 3u) == 0) {
+        const int64_t words = bytes / 4;
+        sp24::launch_chained(static_cast<cudaStream_t>(stream), sp24::clear_kernel, (unsigned)((words + 1023) / 1024), 256, 0,
+                             static_cast<uint32_t *>(dst), words);
+        return sp24::launch_status();
+    }
     if (cudaMemsetAsync(dst, 0, (size_t)bytes, static_cast<cudaStream_t>(stream)) == cudaSuccess) return SP24_OK;
     sp24::launch_status();         // clears (and with SP24_DEBUG prints) the runtime's error
     return SP24_ERR_CUDA;
