@@ -18,6 +18,7 @@
 
 #include <cstdio>
 #include <cstdlib>
+#include <mutex>
 
 #include "meta_steps.cuh"
 #include "sp24_common.cuh"
@@ -854,10 +855,11 @@ __device__ __forceinline__ void tmem_relinquish_pair() {
 __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t cols) {
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
 }
-// arrives on the barrier at this shared-memory offset in both CTAs of the pair once the MMAs issued so far are done
-__device__ __forceinline__ void tc_commit_pair(uint32_t bar) {
+// arrives on the barrier at this shared-memory offset in both CTAs of the pair once the MMAs issued so far are done; first: the
+// leader's rank, where the cluster has more than one pair
+__device__ __forceinline__ void tc_commit_pair(uint32_t bar, uint32_t first = 0) {
     asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
-                 "h"((uint16_t)3)
+                 "h"((uint16_t)(3u << first))
                  : "memory");
 }
 __device__ __forceinline__ void tc_cp_128x128b_pair(uint32_t taddr, uint64_t sdesc) {
@@ -1198,6 +1200,198 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     // nobody leaves while the peer may still read this CTA's shared memory or signal its barriers
     __syncthreads();
     cluster_sync_all();
+    if (warp == 1) {
+        tc_fence_after();
+        tmem_dealloc_pair(tmem_base, TMEM_COLS);
+    }
+}
+
+// ------------------------------------------------------------------------------------------------
+// Few tokens: K cut into slices over the pairs of a cluster.
+// ------------------------------------------------------------------------------------------------
+// A handful of dense columns gives one tile per 256 rows: 16 pairs of 74 walk 32 K steps each for a 4096 x 4096 weight, and a step
+// takes the ring's latency whatever it computes.  Here a cluster of S pairs (S <= 4: eight CTAs) takes one tile, each pair every S-th
+// part of K with a ring of its own.  Every pair finishes a share of the tile's columns: it gets the others' float32 partial sums of
+// them in its shared memory, and after one cluster barrier adds them to its own in a fixed order, so results repeat bit for bit.
+// (One pair finishing the whole tile took 1 us more at 32 columns and 2.5 at 64.)
+namespace two {
+constexpr int SPLIT_MAX = 4, BN_SPLIT = 64;                 // pairs a cluster, columns of a tile at most
+constexpr int64_t SPLIT_N = 4096;                           // more columns are more tiles than clusters at any row count
+__host__ __device__ constexpr int share(int bn, int slices) { return (bn + 4 * slices - 1) / (4 * slices) * 4; }     // columns a pair finishes
+// a partial share: columns in fours, 128 rows x 16 bytes each, so that a warp's remote store is 512 bytes in one piece
+__host__ __device__ constexpr int part_bytes(int bn, int slices) { return share(bn, slices) * BM * 4; }
+constexpr int split_stages(int bn, int slices) {
+    const int n = (SMEM_LIMIT - (slices - 1) * part_bytes(bn, slices) - (int)sizeof(Ctl2)) / stage2_bytes(false, bn);
+    return n < MAX_STAGES2 ? n : MAX_STAGES2;
+}
+constexpr int split_smem(int bn, int slices) {
+    return split_stages(bn, slices) * stage2_bytes(false, bn) + (slices - 1) * part_bytes(bn, slices) + (int)sizeof(Ctl2);
+}
+static_assert(split_stages(BN_SPLIT, SPLIT_MAX) >= 4, "shared memory budget");
+}  // namespace two
+
+__device__ __forceinline__ void st_cluster_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+
+template <bool A_MN, typename OutT>
+__global__ void __launch_bounds__(320, 1)
+spmm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+                  const __grid_constant__ CUtensorMap map_e, SpmmParams P) {
+    using namespace two;
+    const int BN = P.bn, STAGES = P.stages, S = P.k_splits;
+    const int STAGE_BYTES = stage2_bytes(false, BN);
+    constexpr int OFF_E = A_STAGE_BYTES, OFF_B = OFF_E + e2_bytes(false);
+    constexpr uint32_t TMEM_COLS = 512;
+
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    uint8_t *const smem = smem_raw;                // on 1024 bytes: checked by the launcher, the same in every CTA
+    uint8_t *const parts = smem + STAGES * STAGE_BYTES;
+    Ctl2 &ctl = *reinterpret_cast<Ctl2 *>(parts + (S - 1) * part_bytes(BN, S));
+    uint64_t *const bars = ctl.bars;
+    volatile int &abort_flag = ctl.abort_flag;
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t cta = cluster_ctarank(), rank = cta & 1u, leader = cta & ~1u;      // rank in the pair; the pair's first CTA
+    const int slice = (int)(cta >> 1);
+    const int n_tiles_m = (int)((P.ms + 2 * BM - 1) / (2 * BM));
+    const int tile = (int)blockIdx.x / (2 * S);
+    const int k_iters = (int)((P.k + 127) / 128), it0 = slice * k_iters / S, it1 = (slice + 1) * k_iters / S;
+    const int mblk = (tile % n_tiles_m) * 2 + (int)rank;
+    const int64_t row0 = (int64_t)(tile / n_tiles_m) * BN;
+
+    const uint32_t full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[MAX_STAGES2]), tmem_full = smem_u32(&bars[2 * MAX_STAGES2]);
+    if (threadIdx.x == 0) {
+        abort_flag = 0;
+        for (int s = 0; s < STAGES; ++s) {
+            mbar_init(full0 + 8 * s, 1);
+            mbar_init(empty0 + 8 * s, 1);
+        }
+        mbar_init(tmem_full, 1);
+        fence_barrier_init();
+    }
+    if (warp == 1) {
+        tmem_alloc_pair(smem_u32(&ctl.tmem_base), TMEM_COLS);
+        tmem_relinquish_pair();
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();
+    tc_fence_after();
+    const uint32_t tmem_base = ctl.tmem_base;
+    chain_enter();
+
+    float acc[32];
+    bool run = false;
+    const int quad = warp & 3, half = (warp - 2) >> 2, HC = BN / 2, CW = share(BN, S);
+    const int mrow = mblk * BM + quad * 32, left = P.n - row0 < BN ? (int)(P.n - row0) : BN;
+    auto owner_of = [&](int col) { return (col >= CW) + (col >= 2 * CW) + (col >= 3 * CW); };      // the pair that finishes a column
+    if (warp == 0) {
+        if (lane == 0) {
+            int s = 0, g = 0;
+            uint32_t ph = 1;
+            for (int it = it0; it < it1; ++it, ++g) {
+                if (!mbar_wait(empty0 + 8 * s, ph, &abort_flag, P.status, 1)) break;
+                const uint32_t sa = smem_u32(smem) + (uint32_t)(s * STAGE_BYTES), sb = sa + OFF_B;
+                const uint32_t full_leader = map_to_cta(full0 + 8 * s, leader);
+                if (rank == 0) mbar_expect_tx(full0 + 8 * s, 2 * (uint32_t)STAGE_BYTES);
+                if constexpr (!A_MN) {
+                    tma_load_2d_pair(sa, &map_a, it * 64, mblk * BM, full_leader);
+                } else {
+                    tma_load_2d_pair(sa, &map_a, mblk * BM, it * 64, full_leader);
+                    tma_load_2d_pair(sa + 8192, &map_a, mblk * BM + 64, it * 64, full_leader);
+                }
+                tma_load_2d_pair(sa + OFF_E, &map_e, 0, (int)(((int64_t)mblk * P.k_atoms + it) * 2), full_leader);
+                tma_load_2d_pair(sb, &map_b, it * 128, (int)row0 + (int)rank * (BN / 2), full_leader);
+                tma_load_2d_pair(sb + (BN / 2) * 128, &map_b, it * 128 + 64, (int)row0 + (int)rank * (BN / 2), full_leader);
+                if (++s == STAGES) { s = 0; ph ^= 1; }
+            }
+            if (abort_flag && rank == 0) {
+                for (int q = (g > STAGES ? g - STAGES : 0); q < g; ++q)
+                    for (uint32_t w = 0; w < WAIT_LIMIT; ++w)
+                        if (mbar_try_wait(full0 + 8 * (q % STAGES), (q / STAGES) & 1)) break;
+            }
+        }
+        __syncwarp();
+    } else if (warp == 1) {
+        if (rank == 0) {                       // all lanes in step, one elected lane issues (as in spmm_pair_kernel)
+            const uint32_t idesc0 = P.idesc, smem0 = smem_u32(smem);
+            constexpr uint32_t A_LBO = A_MN ? 8192 : 16, A_KSTEP = A_MN ? 2048 : 32;
+            const uint64_t adesc0 = make_desc(smem0, A_LBO, 1024, 2), bdesc0 = make_desc(smem0 + OFF_B, 16, 1024, 2);
+            const uint64_t edesc0 = make_desc(smem0 + OFF_E, 16, 128, 0);
+            const uint32_t b_atom = (uint32_t)BN * (64 >> 4);
+            int s = 0;
+            uint32_t ph = 0, eslot = 0;
+            for (int it = it0; it < it1; ++it) {
+                if (!mbar_wait_warp(full0 + 8 * s, ph, &abort_flag, P.status, 2)) break;
+                tc_fence_after();
+                const uint32_t off = (uint32_t)s * ((uint32_t)STAGE_BYTES >> 4), e_cols = tmem_base + E_COL + eslot;
+                if (elect_one()) {
+                    tc_cp_128x128b_pair(e_cols, edesc0 + off);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        mma_sp_pair(tmem_base, adesc0 + off + j * (A_KSTEP >> 4), bdesc0 + off + ((j >> 1) * b_atom + (j & 1) * (64 >> 4)),
+                                    e_cols + (j & ~1), idesc0 | (j & 1), (it > it0 || j > 0) ? 1u : 0u);
+                    tc_commit_pair(empty0 + 8 * s, leader);
+                }
+                __syncwarp();
+                eslot ^= 4;
+                if (++s == STAGES) { s = 0; ph ^= 1; }
+            }
+            if (elect_one()) tc_commit_pair(tmem_full, leader);      // also arrives after an abort
+            __syncwarp();
+        }
+    } else {
+        const bool ok = mbar_wait(tmem_full, 0, &abort_flag, P.status, 3);
+        tc_fence_after();
+        run = __all_sync(0xFFFFFFFFu, ok && !abort_flag);      // the warp reads tensor memory together
+        if (run) {
+            uint32_t v[32];                    // a lane: one row, 32 columns; those past HC are read, never used
+            tmem_ld32(tmem_base + ((uint32_t)(quad * 32) << 16) + half * HC, v);
+            tmem_ld_wait();
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                const int col = half * HC + 4 * q, owner = owner_of(col);
+                if (4 * q < HC && col < left && owner != slice)
+                    st_cluster_v4(map_to_cta(smem_u32(parts + (slice - (slice > owner)) * part_bytes(BN, S)) +
+                                                 (col - owner * CW) * BM * 4 + (quad * 32 + lane) * 16, 2 * owner + rank),
+                                  v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+            }
+#pragma unroll
+            for (int i = 0; i < 32; ++i) acc[i] = __uint_as_float(v[i]);
+        }
+        tc_fence_before();
+    }
+    // the partial tiles have arrived; also: nobody leaves while a peer may still signal its barriers or read its operands
+    __syncthreads();
+    cluster_sync_all();
+    if (warp >= 2 && run && mrow < P.ms) {
+        const float bias = P.bias ? load_bias<OutT>(P, mrow + lane) : 0.f;
+        const int c0 = half * HC;
+        // columns of other pairs read the first 16 bytes instead, so that no load waits for a branch
+        const uint32_t from = smem_u32(parts) + (quad * 32 + lane) * 16;
+        for (int p = 0; p < S - 1; ++p) {
+            uint4 o[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                const int col = c0 + 4 * q;
+                const bool mine = 4 * q < HC && col < left && owner_of(col) == slice;
+                o[q] = ld_shared_v4(from + p * part_bytes(BN, S) + (mine ? (col - slice * CW) * BM * 4 : 0));
+            }
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                acc[4 * q] += __uint_as_float(o[q].x);
+                acc[4 * q + 1] += __uint_as_float(o[q].y);
+                acc[4 * q + 2] += __uint_as_float(o[q].z);
+                acc[4 * q + 3] += __uint_as_float(o[q].w);
+            }
+        }
+        OutT *dst = static_cast<OutT *>(P.out) + (row0 + c0) * P.ld_out + mrow + lane;      // 32 features of a token a store
+        const int first = max(slice * CW, c0) - c0, last = min(min((slice + 1) * CW, left), c0 + HC) - c0;      // this warp's columns
+#pragma unroll
+        for (int i = 0; i < 32; ++i, dst += P.ld_out)
+            if (i >= first && i < last) *dst = to_out<OutT>(acc[i] + bias);
+    }
     if (warp == 1) {
         tc_fence_after();
         tmem_dealloc_pair(tmem_base, TMEM_COLS);
@@ -1678,6 +1872,76 @@ int launch_spmm_pair_acc(const CUtensorMap &ma, const CUtensorMap &mb, const CUt
     return launch_status();
 }
 
+// spmm_split_kernel: a cluster of 2 * slices CTAs a tile.
+void split_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute (&attr)[2], int slices, int64_t tiles, int smem, cudaStream_t st) {
+    cfg.gridDim = dim3((unsigned)(2 * slices * tiles), 1, 1);
+    cfg.blockDim = dim3(320, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2 * slices;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;      // see launch_chained
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+}
+
+// Clusters of 2 s CTAs that the device holds at once (entry s; zeros where the kernel cannot run), worked out on its first call.
+struct SplitRoom { int64_t clusters[two::SPLIT_MAX + 1]; };
+template <bool A_MN, typename OutT> const SplitRoom *split_room() {
+    static SplitRoom room[64];
+    static bool done[64];
+    static std::mutex mu;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+    std::lock_guard<std::mutex> lock(mu);
+    if (!done[dev]) {
+        auto kern = spmm_split_kernel<A_MN, OutT>;
+        cudaFuncAttributes fa{};
+        // dynamic shared memory on 1024 bytes, as in launch_spmm_pair
+        if (cudaFuncGetAttributes(&fa, kern) == cudaSuccess && fa.sharedSizeBytes % 1024 == 0 &&
+            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, two::SMEM_LIMIT) == cudaSuccess)
+            for (int s = 2; s <= two::SPLIT_MAX; ++s) {
+                cudaLaunchConfig_t cfg{};
+                cudaLaunchAttribute attr[2];
+                split_config(cfg, attr, s, 1, two::split_smem(two::BN_SPLIT, s), nullptr);
+                int n = 0;
+                if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess) room[dev].clusters[s] = n;
+            }
+        cudaGetLastError();
+        done[dev] = true;
+    }
+    return &room[dev];
+}
+
+// Slices of K for few columns (1: the pair kernel takes the call): the most that leave every tile a cluster at once, from eight K
+// steps (two a slice) on.  us, pair kernel -> here:
+//   ms 4096, k 4096: n 1 12.3 -> 7.6, n 64 12.7 -> 8.3, n 128 13.3 -> 9.5; ms 512, k 4096: n 16 11.9 -> 5.8, n 256 12.1 -> 8.2
+//   ms 1024, k 1024: n 16 5.3 -> 3.8, n 256 5.5 -> 5.3; ms 512, k 2048, n 768 8.2 -> 6.4; ms 256, k 1024, n 1000 5.5 -> 5.3
+// Shorter K keeps the order of sums that the pair and single-CTA kernels share bit for bit; slices would gain 0.1 - 0.6 us there
+// (ms 512, n 16, k 512 4.1 -> 3.5) and lose with one step each (ms 512, n 512, k 512 in four 4.4 -> 5.0).
+int pick_slices(int64_t ms, int64_t n, int64_t k, int bn, const SplitRoom &room) {
+    if (k <= 7 * 128) return 1;
+    const int64_t tiles = ((ms + 255) / 256) * ((n + bn - 1) / bn);
+    for (int s = two::SPLIT_MAX; s >= 2; --s)
+        if (tiles <= room.clusters[s]) return s;
+    return 1;
+}
+int split_bn(int64_t n) { return n <= 32 ? 32 : (n <= 48 ? 48 : 64); }
+
+template <bool A_MN, typename OutT>
+int launch_spmm_split(const CUtensorMap &ma, const CUtensorMap &mb, const CUtensorMap &me, SpmmParams P, cudaStream_t st) {
+    P.idesc = (P.idesc & ~(0x1Fu << 24)) | ((uint32_t)(256 >> 4) << 24) | ((uint32_t)(P.bn >> 3) << 17);
+    P.stages = two::split_stages(P.bn, P.k_splits);
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr[2];
+    split_config(cfg, attr, P.k_splits, ((P.ms + 255) / 256) * ((P.n + P.bn - 1) / P.bn), two::split_smem(P.bn, P.k_splits), st);
+    if (cudaLaunchKernelEx(&cfg, spmm_split_kernel<A_MN, OutT>, ma, mb, me, P) != cudaSuccess) return SP24_ERR_CUDA;
+    return launch_status();
+}
+
 // Tile shape: wide / tall tiles stage fewer operand bytes per output, small ones fill the SMs more evenly.
 // Cost model per candidate (BN, row blocks per tile): rounds of tiles per CTA x bytes staged per K iteration.
 void pick_tile(int64_t ms, int64_t n, int sm_count, int &bn_out, int &mpt_out) {
@@ -1861,10 +2125,21 @@ static int spmm_impl(const void *a_packed, int dtype, int a_mn_major, int64_t ld
     if (pair_form) {
         CUtensorMap map_b, map_e;
         P.bn = pick_pair_bn(ms, n, epi == EPI_PLAIN, false, sm_count_cached());
+        if (epi == EPI_PLAIN && n <= two::SPLIT_N && pair_kernels_enabled()) {
+            const SplitRoom *room = out_dtype == SP24_F16 ? (a_mn_major ? split_room<true, __half>() : split_room<false, __half>())
+                                                          : (a_mn_major ? split_room<true, __nv_bfloat16>() : split_room<false, __nv_bfloat16>());
+            P.k_splits = room ? pick_slices(ms, n, k, split_bn(n), *room) : 1;
+            if (P.k_splits > 1) P.bn = split_bn(n);
+        }
         rc = make_map(&map_b, b, dtype, n, k, ld_b, 64, (uint32_t)P.bn / 2);
         if (rc) return rc;
         rc = make_map_e(&map_e, e_tc, (ms / 128) * P.k_atoms);
         if (rc) return rc;
+        if (P.k_splits > 1)
+            return out_dtype == SP24_F16 ? (a_mn_major ? launch_spmm_split<true, __half>(map_a, map_b, map_e, P, st)
+                                                       : launch_spmm_split<false, __half>(map_a, map_b, map_e, P, st))
+                                         : (a_mn_major ? launch_spmm_split<true, __nv_bfloat16>(map_a, map_b, map_e, P, st)
+                                                       : launch_spmm_split<false, __nv_bfloat16>(map_a, map_b, map_e, P, st));
 #define SP24_PAIR(EPI_) \
         do { \
             if (out_dtype == SP24_F16) \
