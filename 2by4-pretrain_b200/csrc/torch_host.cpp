@@ -433,39 +433,146 @@ py::tuple select_compress(const Tensor &weight, const OptTensor &mask_in, at::Sc
     return as_tuple(mask, *c);
 }
 
-std::vector<py::tuple> select_compress_many(const std::vector<Tensor> &weights, const std::vector<Tensor> &masks, at::ScalarType t, bool reselect) {
+// Both copies of every weight in one launch; without the GIL.
+std::vector<Copies> compress_all(const std::vector<Tensor> &weights, const std::vector<Tensor> &masks, at::ScalarType t, bool reselect) {
     const size_t count = weights.size();
     TORCH_CHECK(masks.size() == count, "select_and_compress_many: one mask per weight");
     std::vector<Copies> copies;
     std::vector<Tensor> keep;
     copies.reserve(count);
+    NoAutograd guard;
+    std::vector<sp24_dual_desc> descs(count);
+    for (size_t i = 0; i < count; ++i) {
+        const Tensor &weight = weights[i], &mask = masks[i];
+        require_cuda(weight, mask);
+        const int64_t m = weight.size(0), k = weight.size(1);
+        TORCH_CHECK(m % 128 == 0 && k % 128 == 0, "select_and_compress_many: shape (", m, ", ", k, ") is not a multiple of 128 x 128");
+        TORCH_CHECK(weight.scalar_type() == weights[0].scalar_type() && weight.device() == weights[0].device(),
+                    "select_and_compress_many: all weights must share dtype and device");
+        TORCH_CHECK(mask.scalar_type() == at::kBool && mask.sizes() == weight.sizes() && mask.is_contiguous(),
+                    "select_and_compress_many: masks must be contiguous bool tensors of the weights' shapes");
+        const Tensor w = as_layout(weight, 0);
+        keep.push_back(w);
+        copies.emplace_back(m, k, t, w);
+        const Copies &c = copies.back();
+        descs[i] = {ptr(w), m, k, layout_of(w).ld, ptr(mask), k, ptr(c.pw), k / 2, ptr(c.mw), ptr(c.pt), k, ptr(c.mt), ptr(c.tcw), ptr(c.tct)};
+    }
+    if (count)
+        check(sp24_select_dual_compress_batch(descs.data(), (int)count, dt(weights[0].scalar_type()), dt(t), reselect, cur_stream()),
+              "sp24_select_dual_compress_batch");
+    return copies;
+}
+
+std::vector<py::tuple> select_compress_many(const std::vector<Tensor> &weights, const std::vector<Tensor> &masks, at::ScalarType t, bool reselect) {
+    std::vector<Copies> copies;
     {
         py::gil_scoped_release nogil;
-        NoAutograd guard;
-        std::vector<sp24_dual_desc> descs(count);
-        for (size_t i = 0; i < count; ++i) {
-            const Tensor &weight = weights[i], &mask = masks[i];
-            require_cuda(weight, mask);
-            const int64_t m = weight.size(0), k = weight.size(1);
-            TORCH_CHECK(m % 128 == 0 && k % 128 == 0, "select_and_compress_many: shape (", m, ", ", k, ") is not a multiple of 128 x 128");
-            TORCH_CHECK(weight.scalar_type() == weights[0].scalar_type() && weight.device() == weights[0].device(),
-                        "select_and_compress_many: all weights must share dtype and device");
-            TORCH_CHECK(mask.scalar_type() == at::kBool && mask.sizes() == weight.sizes() && mask.is_contiguous(),
-                        "select_and_compress_many: masks must be contiguous bool tensors of the weights' shapes");
-            const Tensor w = as_layout(weight, 0);
-            keep.push_back(w);
-            copies.emplace_back(m, k, t, w);
-            const Copies &c = copies.back();
-            descs[i] = {ptr(w), m, k, layout_of(w).ld, ptr(mask), k, ptr(c.pw), k / 2, ptr(c.mw), ptr(c.pt), k, ptr(c.mt), ptr(c.tcw), ptr(c.tct)};
-        }
-        if (count)
-            check(sp24_select_dual_compress_batch(descs.data(), (int)count, dt(weights[0].scalar_type()), dt(t), reselect, cur_stream()),
-                  "sp24_select_dual_compress_batch");
+        copies = compress_all(weights, masks, t, reselect);
     }
     std::vector<py::tuple> out;
-    out.reserve(count);
-    for (size_t i = 0; i < count; ++i) out.push_back(as_tuple(masks[i], copies[i]));
+    out.reserve(copies.size());
+    for (size_t i = 0; i < copies.size(); ++i) out.push_back(as_tuple(masks[i], copies[i]));
     return out;
+}
+
+// ---------------------------------------------------------------------------------------------
+// refresh of a model's layers
+// ---------------------------------------------------------------------------------------------
+// What sparse_ops.refresh_sparse_layers does for layers of the plain class: reads each weight's state, launches once per group and
+// installs the copies.  In Python these 20 attribute accesses a layer were more host time than 48 layers' kernel on the GPU (109 us).
+// Returns the number of layers refreshed and those it leaves to the caller: any whose class, weight, mask or counters are not plain.
+struct RefreshNames {
+    PyObject *weight, *parameters, *mode, *cnt, *mask, *counter, *freq, *compressed, *compressed_tc, *weight_sparse, *weight_sparse_T, *refreshed, *take,
+        *materialize;
+};
+const RefreshNames &refresh_names() {       // made by the module's load, see PyObjects
+    static const RefreshNames n = [] {
+        auto s = [](const char *t) { return PyUnicode_InternFromString(t); };
+        return RefreshNames{s("weight"), s("_parameters"), s("mode"), s("cnt"), s("mask"), s("counter"), s("freq"), s("compressed"), s("compressed_tc"),
+                            s("weight_sparse"), s("weight_sparse_T"), s("refreshed"), s("_take"), s("materialize_sparse_tensors")};
+    }();
+    return n;
+}
+
+std::pair<int64_t, py::list> refresh_layers(const py::list &mods, at::ScalarType t, const py::object &plain) {
+    const RefreshNames &N = refresh_names();
+    auto attr = [](PyObject *o, PyObject *name) {
+        PyObject *v = PyObject_GetAttr(o, name);
+        if (!v) throw py::error_already_set();
+        return py::reinterpret_steal<py::object>(v);
+    };
+    auto set = [](PyObject *o, PyObject *name, PyObject *v) {
+        if (PyObject_SetAttr(o, name, v) < 0) throw py::error_already_set();
+    };
+    struct Group { bool reselect; at::ScalarType type; c10::Device device; std::vector<Tensor> weights, masks; std::vector<py::object> owners; };
+    std::vector<Group> groups;
+    py::list left;
+    const bool plain_class = !PyObject_IsTrue(attr(plain.ptr(), N.materialize).ptr());
+    for (const py::handle mod : mods) {
+        PyObject *dict = nullptr, *params = nullptr, *w = nullptr;
+        py::object held;
+        if (plain_class && (PyObject *)Py_TYPE(mod.ptr()) == plain.ptr()) {
+            held = py::reinterpret_steal<py::object>(PyObject_GenericGetDict(mod.ptr(), nullptr));
+            dict = held.ptr();
+            if (!dict) PyErr_Clear();
+        }
+        // plain: the weight is the registered parameter, and nothing of its handling is replaced on the instance
+        if (dict && !PyDict_GetItemWithError(dict, N.weight) && !PyDict_GetItemWithError(dict, N.take) && !PyDict_GetItemWithError(dict, N.materialize) &&
+            (params = PyDict_GetItemWithError(dict, N.parameters)) && PyDict_Check(params))
+            w = PyDict_GetItemWithError(params, N.weight);
+        if (PyErr_Occurred()) throw py::error_already_set();
+        if (!w || !THPVariable_Check(w)) {
+            left.append(mod);
+            continue;
+        }
+        const Tensor &weight = THPVariable_Unpack(w);
+        const py::object mode = attr(w, N.mode), cnt = attr(w, N.cnt), mask_o = attr(w, N.mask), counter = attr(w, N.counter), freq = attr(w, N.freq);
+        if (!PyUnicode_CheckExact(mode.ptr()) || !PyLong_CheckExact(cnt.ptr()) || !PyLong_CheckExact(counter.ptr()) || !PyLong_CheckExact(freq.ptr()) ||
+            !THPVariable_Check(mask_o.ptr()) || weight.dim() != 2) {
+            left.append(mod);
+            continue;
+        }
+        if (PyUnicode_CompareWithASCIIString(mode.ptr(), "sparse") != 0 || PyObject_IsTrue(cnt.ptr()) || !weight.is_cuda()) continue;
+        if (weight.size(0) % 128 || weight.size(1) % 128) continue;
+        const Tensor &mask = THPVariable_Unpack(mask_o.ptr());
+        int over1 = 0, over2 = 0;
+        const long long c = PyLong_AsLongLongAndOverflow(counter.ptr(), &over1), f = PyLong_AsLongLongAndOverflow(freq.ptr(), &over2);
+        if (mask.device() != weight.device() || mask.scalar_type() != at::kBool || !mask.is_contiguous() || over1 || over2 || f == 0) {
+            left.append(mod);
+            continue;
+        }
+        const bool reselect = c % f == 0;
+        Group *g = nullptr;
+        for (Group &have : groups)
+            if (have.reselect == reselect && have.type == weight.scalar_type() && have.device == weight.device()) g = &have;
+        if (!g) {
+            groups.push_back({reselect, weight.scalar_type(), weight.device(), {}, {}, {}});
+            g = &groups.back();
+        }
+        g->weights.push_back(weight);
+        g->masks.push_back(mask);
+        g->owners.push_back(py::reinterpret_borrow<py::object>(w));
+    }
+    int64_t done = 0;
+    for (const Group &g : groups) {
+        std::vector<Copies> copies;
+        {
+            py::gil_scoped_release nogil;
+            copies = compress_all(g.weights, g.masks, t, g.reselect);
+        }
+        for (size_t i = 0; i < copies.size(); ++i) {       // what SparseLinearTranspose._take does
+            const Copies &k = copies[i];
+            PyObject *w = g.owners[i].ptr();
+            const py::tuple held = py::make_tuple(k.pw, k.mw, k.pt, k.mt);
+            set(w, N.compressed, held.ptr());
+            set(w, N.compressed_tc, py::make_tuple(held, (int64_t)k.mw._version(), (int64_t)k.mt._version(), py::make_tuple(k.tcw, k.tct)).ptr());
+            set(w, N.weight_sparse, Py_None);
+            set(w, N.weight_sparse_T, Py_None);
+            set(w, N.refreshed, Py_True);
+            ++done;
+        }
+    }
+    return {done, left};
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1282,6 +1389,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("compress", &compress, nogil());
     m.def("select_compress", &select_compress);
     m.def("select_compress_many", &select_compress_many);
+    refresh_names();
+    m.def("refresh_layers", &refresh_layers);
     m.def("masked_add", &masked_add, nogil());
     m.def("fst_linear", &fst_linear);
     m.def("fst_weight_grads",

@@ -12,6 +12,7 @@ from torch import autograd, nn
 from torch.amp import custom_fwd, custom_bwd
 
 from . import _ext
+from ._ext import host as _host
 from .semi_structured import SparseSemiStructuredTensor, to_sparse_semi_structured
 from .transposable_semi_structured import TransposableSparse
 from .triton_ops import MVUE24_approx_triton
@@ -346,10 +347,10 @@ def refresh_sparse_layers(model: nn.Module) -> int:
     dtype = torch.float16
     if torch.is_autocast_enabled('cuda') and torch.get_autocast_dtype('cuda') == torch.bfloat16:
         dtype = torch.bfloat16
+    layers = [mod for mod in _modules(model) if isinstance(mod, SparseLinearTranspose)]
+    done, layers = _host.refresh_layers(layers, dtype, SparseLinearTranspose)
     groups = {}
-    for mod in _modules(model):
-        if not isinstance(mod, SparseLinearTranspose):
-            continue
+    for mod in layers:                       # those with a class, weight, mask or counters of their own
         w = mod.weight                       # the attribute: a subclass or a parametrization may answer for the parameter
         if w.mode != 'sparse' or w.cnt != 0 or not w.is_cuda:
             continue
@@ -368,7 +369,6 @@ def refresh_sparse_layers(model: nn.Module) -> int:
         group[0].append(mod)
         group[1].append(w)
         group[2].append(mask)
-    done = 0
     for (reselect, _, _), (mods, weights, masks) in groups.items():
         res = _ext.host.select_compress_many(weights, masks, dtype, reselect)
         for mod, w, copies in zip(mods, weights, res):
