@@ -1039,10 +1039,11 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         // Plain form: a warp takes every other 16-token chunk of its 32 features.  tcgen05.ld in the 16x256b shape leaves 8 x 8
         // fragments, packed to 16 bits in registers (64 of them), and the accumulator goes back to the MMAs at once.  stmatrix then
         // writes the fragments token-major into the warp's two chunks of shared memory, from where 16-byte stores take them: 8 tokens
-        // x 64 bytes an instruction instead of one token's 32 two-byte values.  What bounds it is the chip's writes, about 3.4 TB/s
-        // however they are issued (128-byte rows and TMA stores were no faster), shared with the operand fill: taken by itself it
-        // gains where many tiles are written, fp16 us, two-byte stores -> now: ms 3072, k 768, n 8192 28.0 -> 26.6, n 16384
-        // 50.0 -> 49.3; float8 ms 768, k 768, n 4096 7.5 -> 7.3; with few short tiles its chain costs up to 0.2 us (see Ctl2 for the rest).
+        // x 64 bytes an instruction instead of one token's 32 two-byte values.  128-byte rows and TMA stores were no faster: 148 blocks
+        // that only write such tiles reach 5.3 TB/s in pieces of 64 to 256 bytes, and here the stores share the way to L2 with the
+        // operand fill.  Taken by itself it gains where many tiles are written, fp16 us, two-byte stores -> now: ms 3072, k 768,
+        // n 8192 28.0 -> 26.6, n 16384 50.0 -> 49.3; float8 ms 768, k 768, n 4096 7.5 -> 7.3; with few short tiles its chain costs up
+        // to 0.2 us (see Ctl2 for the rest).
         // Fused forms: a warp packs its BN / 2 columns of the accumulator into registers, hands the buffer back, then stores
         // 16-bit values directly; the 32 lanes of a store are 32 consecutive features of one token.
         const int quad = warp & 3, half = (warp - 2) >> 2;
@@ -1216,7 +1217,10 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 // (One pair finishing the whole tile took 1 us more at 32 columns and 2.5 at 64.)
 namespace two {
 constexpr int SPLIT_MAX = 4, BN_SPLIT = 64;                 // pairs a cluster, columns of a tile at most
-constexpr int64_t SPLIT_N = 4096;                           // more columns are more tiles than clusters at any row count
+// Columns at most.  A training step of the FST and float8 layers has at least 64 tokens (their MVUE compression takes multiples of
+// 64) and keeps one order of sums whatever the kernel: an output rounded the other way makes other MVUE draws, which moves a
+// model's gradients by several percent.
+constexpr int64_t SPLIT_N = 63;
 __host__ __device__ constexpr int share(int bn, int slices) { return (bn + 4 * slices - 1) / (4 * slices) * 4; }     // columns a pair finishes
 // a partial share: columns in fours, 128 rows x 16 bytes each, so that a warp's remote store is 512 bytes in one piece
 __host__ __device__ constexpr int part_bytes(int bn, int slices) { return share(bn, slices) * BM * 4; }
@@ -1409,11 +1413,11 @@ spmm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
 //
 // Epilogue: tensor memory -> shared memory -> TMA reductions of 16 rows x 32 columns.  Its cost is exposed where a pair has one unit
 // (nothing is left to multiply): under 3 us for a few tiles, 7 of 41 with all pairs writing at once (ms 3072, n 768, k 16384, by a
-// build without it), where the chip's writes bound it.  red.global.add.v4 from the registers, 32 rows of 16 bytes an instruction, took
-// 4 us even for one tile (64-byte rows: 0.6 us more than 128-byte ones).  us, before -> now, one unit per pair: ms 512, n 256, k 256
-// 9.5 -> 7.8; ms 768, n 768, k 8192 15.3 -> 11.8; ms 3072, n 768, k 8192 / 16384 24.6 -> 21.3 / 40.5 -> 37.4; several units (outputs
-// of more tiles than pairs, or given slices): ms 3072, n 3072, k 2048 / 8192 31.4 -> 25.4 / 80.6 -> 71.6; ms 4096, n 4096, k 2048
-// 67.2 -> 49.3; ms 512, n 512, k 16384 in 40 slices 29.6 -> 21.0.
+// build without it).  red.global.add.v4 from the registers, 32 rows of 16 bytes an instruction, took 4 us even for one tile (64-byte
+// rows: 0.6 us more than 128-byte ones).  us, before -> now, one unit per pair: ms 512, n 256, k 256 9.5 -> 7.8; ms 768, n 768, k 8192
+// 15.3 -> 11.8; ms 3072, n 768, k 8192 / 16384 24.6 -> 21.3 / 40.5 -> 37.4; several units (outputs of more tiles than pairs, or given
+// slices): ms 3072, n 3072, k 2048 / 8192 31.4 -> 25.4 / 80.6 -> 71.6; ms 4096, n 4096, k 2048 67.2 -> 49.3; ms 512, n 512, k 16384 in
+// 40 slices 29.6 -> 21.0.  Barriers at run-time addresses (see Ctl2) made no difference here.
 // Where every pair has one unit at most (any output up to 74 tiles) the operand ring is idle by then and holds the whole tile,
 // so that no chunk waits for another; a pair with more units stages chunk by chunk beside its ring, which is filling again.
 namespace two {
@@ -1918,10 +1922,10 @@ template <bool A_MN, typename OutT> const SplitRoom *split_room() {
 
 // Slices of K for few columns (1: the pair kernel takes the call): the most that leave every tile a cluster at once, from eight K
 // steps (two a slice) on.  us, pair kernel -> here:
-//   ms 4096, k 4096: n 1 12.3 -> 7.6, n 64 12.7 -> 8.3, n 128 13.3 -> 9.5; ms 512, k 4096: n 16 11.9 -> 5.8, n 256 12.1 -> 8.2
-//   ms 1024, k 1024: n 16 5.3 -> 3.8, n 256 5.5 -> 5.3; ms 512, k 2048, n 768 8.2 -> 6.4; ms 256, k 1024, n 1000 5.5 -> 5.3
+//   ms 4096, k 4096: n 1 12.3 -> 7.6, n 33 12.5 -> 7.9; ms 512, k 4096, n 16 11.9 -> 5.8; ms 2304, k 3072, n 16 9.7 -> 5.7
+//   ms 1024, k 1024: n 1 5.2 -> 3.8, n 33 5.5 -> 4.2; ms 4096, k 1024, n 16 5.3 -> 4.9
 // Shorter K keeps the order of sums that the pair and single-CTA kernels share bit for bit; slices would gain 0.1 - 0.6 us there
-// (ms 512, n 16, k 512 4.1 -> 3.5) and lose with one step each (ms 512, n 512, k 512 in four 4.4 -> 5.0).
+// (ms 512, n 16, k 512 4.1 -> 3.5).
 int pick_slices(int64_t ms, int64_t n, int64_t k, int bn, const SplitRoom &room) {
     if (k <= 7 * 128) return 1;
     const int64_t tiles = ((ms + 255) / 256) * ((n + bn - 1) / bn);

@@ -1,5 +1,5 @@
 """The GEMM for few columns, K cut into slices over the pairs of a cluster: two to four slices, tiles of 32, 48 and 64 columns with ragged
-ends, odd row blocks, K that ends inside a step, and one K too short for it: against float64, inside the output's window, and the same
+ends, odd row blocks, K that ends inside a step, and a K too short and a width too large for it: against float64, inside the output's window, and the same
 bits every time."""
 import pytest
 import torch
@@ -11,8 +11,8 @@ ROUND = {torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8}
 
 @pytest.mark.parametrize("dtype", list(ROUND), ids=["f16", "bf16"])
 @pytest.mark.parametrize("col", [False, True])
-@pytest.mark.parametrize("ms,n,k", [(256, 1, 1024), (512, 17, 960), (384, 33, 1152), (128, 64, 4096), (1024, 48, 1088), (640, 65, 2048),
-                                    (2304, 130, 1600), (256, 1030, 1088), (2048, 200, 1024), (512, 16, 896)])
+@pytest.mark.parametrize("ms,n,k", [(256, 1, 1024), (512, 17, 960), (384, 33, 1152), (128, 63, 4096), (1024, 48, 1088), (640, 49, 2048),
+                                    (2304, 32, 1600), (4096, 8, 1088), (6144, 63, 1024), (2048, 64, 1024), (512, 16, 896)])
 def test_few_columns(ms, n, k, col, dtype):
     import sparse
     from sparse import _ext, spmm
