@@ -213,10 +213,13 @@ struct SpmmParams {
     int accumulate;         // float8, float32 output (ms, n): add alpha * A * B instead of storing it
     void *aux;              // fused MLP epilogues (CTA-pair kernel): second tensor shaped and pitched like out
     int64_t ld_aux;
-    const float *row_parts; // weight-gradient form: row_sums[r] (+)= sum over p of row_parts[p * ms + r]
-    float *row_sums;
+};
+// Row sums that the weight-gradient form alone takes along: out[r] (+)= sum over p of parts[p * ms + r]
+struct SumsParams {
+    const float *parts;
+    float *out;
     int64_t n_parts;
-    int sums_accumulate;
+    int accumulate;
 };
 
 // Epilogue forms of the CTA-pair kernel.  PRE_GELU: aux = h = acc + bias rounded to the output type, out = gelu(h)
@@ -1220,7 +1223,7 @@ constexpr int SPLIT_MAX = 4, BN_SPLIT = 64;                 // pairs a cluster, 
 // Columns at most.  A training step of the FST and float8 layers has at least 64 tokens (their MVUE compression takes multiples of
 // 64) and keeps one order of sums whatever the kernel: an output rounded the other way makes other MVUE draws, which moves a
 // model's gradients by several percent.
-constexpr int64_t SPLIT_N = 63;
+constexpr int64_t SPLIT_N = 63, SPLIT_K = 7 * 128;          // K above: see pick_slices
 __host__ __device__ constexpr int share(int bn, int slices) { return (bn + 4 * slices - 1) / (4 * slices) * 4; }     // columns a pair finishes
 // a partial share: columns in fours, 128 rows x 16 bytes each, so that a warp's remote store is 512 bytes in one piece
 __host__ __device__ constexpr int part_bytes(int bn, int slices) { return share(bn, slices) * BM * 4; }
@@ -1439,7 +1442,7 @@ static_assert(smem3(true) <= SMEM_LIMIT, "shared memory budget");
 template <bool A_MN, bool F8>
 __global__ void __launch_bounds__(320, 1)
 spmm_pair_acc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                     const __grid_constant__ CUtensorMap map_e, const __grid_constant__ CUtensorMap map_d, SpmmParams P) {
+                     const __grid_constant__ CUtensorMap map_e, const __grid_constant__ CUtensorMap map_d, SpmmParams P, SumsParams sums) {
     using namespace two;
     static_assert(!(A_MN && F8), "8-bit operands are K-major");
     constexpr int BN = BN3;
@@ -1589,16 +1592,16 @@ spmm_pair_acc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         // The row sums that the compression left in parts (the bias gradient), while the first operands are on their way: 32 rows a
         // CTA and turn, in the order of sum_parts_kernel, through the staging that nothing uses yet.  As a launch of its own between
         // the compression and this kernel it took 2.6 us of a replayed step and 4 of an eager one.
-        if (P.row_sums) {
+        if (sums.out) {
             float *const part = reinterpret_cast<float *>(smem + STAGES3 * STAGE3_BYTES);
             for (int64_t r = (int64_t)blockIdx.x * 32; r < P.ms; r += (int64_t)gridDim.x * 32) {
-                part[(warp - 2) * 32 + lane] = sum_every_eighth(P.row_parts + r + lane, P.n_parts, P.ms, warp - 2);
+                part[(warp - 2) * 32 + lane] = sum_every_eighth(sums.parts + r + lane, sums.n_parts, P.ms, warp - 2);
                 epilogue_bar_sync();
                 if (warp == 2) {
                     float t = 0.f;
 #pragma unroll
                     for (int w = 0; w < 8; ++w) t += part[w * 32 + lane];
-                    P.row_sums[r + lane] = P.sums_accumulate ? P.row_sums[r + lane] + t : t;
+                    sums.out[r + lane] = sums.accumulate ? sums.out[r + lane] + t : t;
                 }
                 epilogue_bar_sync();
             }
@@ -1836,7 +1839,7 @@ int launch_spmm_pair(const CUtensorMap &ma, const CUtensorMap &mb, const CUtenso
 
 template <bool A_MN, bool F8 = false>
 int launch_spmm_pair_acc(const CUtensorMap &ma, const CUtensorMap &mb, const CUtensorMap &me, const CUtensorMap &md, SpmmParams P,
-                         int k_splits, cudaStream_t st) {
+                         const SumsParams &sums, int k_splits, cudaStream_t st) {
     auto kern = spmm_pair_acc_kernel<A_MN, F8>;
     static bool attr_set[64];
     int dev = 0;
@@ -1872,7 +1875,7 @@ int launch_spmm_pair_acc(const CUtensorMap &ma, const CUtensorMap &mb, const CUt
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    if (cudaLaunchKernelEx(&cfg, kern, ma, mb, me, md, P) != cudaSuccess) return launch_status();
+    if (cudaLaunchKernelEx(&cfg, kern, ma, mb, me, md, P, sums) != cudaSuccess) return launch_status();
     return launch_status();
 }
 
@@ -1926,8 +1929,7 @@ template <bool A_MN, typename OutT> const SplitRoom *split_room() {
 //   ms 1024, k 1024: n 1 5.2 -> 3.8, n 33 5.5 -> 4.2; ms 4096, k 1024, n 16 5.3 -> 4.9
 // Shorter K keeps the order of sums that the pair and single-CTA kernels share bit for bit; slices would gain 0.1 - 0.6 us there
 // (ms 512, n 16, k 512 4.1 -> 3.5).
-int pick_slices(int64_t ms, int64_t n, int64_t k, int bn, const SplitRoom &room) {
-    if (k <= 7 * 128) return 1;
+int pick_slices(int64_t ms, int64_t n, int bn, const SplitRoom &room) {
     const int64_t tiles = ((ms + 255) / 256) * ((n + bn - 1) / bn);
     for (int s = two::SPLIT_MAX; s >= 2; --s)
         if (tiles <= room.clusters[s]) return s;
@@ -2129,10 +2131,10 @@ static int spmm_impl(const void *a_packed, int dtype, int a_mn_major, int64_t ld
     if (pair_form) {
         CUtensorMap map_b, map_e;
         P.bn = pick_pair_bn(ms, n, epi == EPI_PLAIN, false, sm_count_cached());
-        if (epi == EPI_PLAIN && n <= two::SPLIT_N && pair_kernels_enabled()) {
+        if (epi == EPI_PLAIN && n <= two::SPLIT_N && k > two::SPLIT_K && pair_kernels_enabled()) {
             const SplitRoom *room = out_dtype == SP24_F16 ? (a_mn_major ? split_room<true, __half>() : split_room<false, __half>())
                                                           : (a_mn_major ? split_room<true, __nv_bfloat16>() : split_room<false, __nv_bfloat16>());
-            P.k_splits = room ? pick_slices(ms, n, k, split_bn(n), *room) : 1;
+            P.k_splits = room ? pick_slices(ms, n, split_bn(n), *room) : 1;
             if (P.k_splits > 1) P.bn = split_bn(n);
         }
         rc = make_map(&map_b, b, dtype, n, k, ld_b, 64, (uint32_t)P.bn / 2);
@@ -2255,7 +2257,7 @@ extern "C" int sp24_spmm_f8(const void *a_packed, int dtype, int64_t ld_a, const
         if (int rc = make_map(&map_b, b, dtype, n, k, ld_b, 128, 128)) return rc;
         if (int rc = make_map_e(&map_e, e_tc, (ms / 128) * P.k_atoms, 2)) return rc;
         if (int rc = encode_map(&map_d, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, out, n, ms, ld_out * 4, 32, 16, CU_TENSOR_MAP_SWIZZLE_128B)) return rc;
-        return launch_spmm_pair_acc<false, true>(map_a, map_b, map_e, map_d, P, 0, st);
+        return launch_spmm_pair_acc<false, true>(map_a, map_b, map_e, map_d, P, SumsParams{}, 0, st);
     }
     if (!trans_out) {
         pick_f8_accumulate(ms, n, k, sms, bn, mpt, P.k_splits);
@@ -2414,9 +2416,9 @@ static int spmm_accumulate_impl(const void *a_packed, int dtype, int a_mn_major,
         CUtensorMap map_d;
         rc = encode_map(&map_d, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, out, n, ms, ld_out * 4, 32, 16, CU_TENSOR_MAP_SWIZZLE_128B);
         if (rc) return rc;
-        P.row_parts = row_parts; P.row_sums = row_sums; P.n_parts = n_parts; P.sums_accumulate = sums_accumulate;
-        return a_mn_major ? launch_spmm_pair_acc<true>(map_a, map_b, map_e, map_d, P, k_splits, st)
-                          : launch_spmm_pair_acc<false>(map_a, map_b, map_e, map_d, P, k_splits, st);
+        const SumsParams sums{row_parts, row_sums, n_parts, sums_accumulate};
+        return a_mn_major ? launch_spmm_pair_acc<true>(map_a, map_b, map_e, map_d, P, sums, k_splits, st)
+                          : launch_spmm_pair_acc<false>(map_a, map_b, map_e, map_d, P, sums, k_splits, st);
     }
     if (row_sums)
         if (int rc2 = sp24_sum_parts(row_parts, n_parts, ms, row_sums, sums_accumulate, stream)) return rc2;
