@@ -16,6 +16,7 @@
 // bounded), frees its tensor memory and returns.  Nothing traps.
 #include <cuda.h>
 
+#include <algorithm>
 #include <cstdio>
 #include <cstdlib>
 #include <mutex>
@@ -1837,6 +1838,12 @@ int launch_spmm_pair(const CUtensorMap &ma, const CUtensorMap &mb, const CUtenso
     return launch_status();
 }
 
+// K slices of the weight gradient on CTA pairs: as many as idle pairs allow.
+int64_t pair_slices(int64_t ms, int64_t n, int64_t k, int k_step, int sms) {
+    const int64_t tiles = ((n + two::BN3 - 1) / two::BN3) * ((ms + 255) / 256), k_iters = (k + k_step - 1) / k_step;
+    return std::max<int64_t>(1, std::min(sms / 2 / tiles, k_iters));
+}
+
 template <bool A_MN, bool F8 = false>
 int launch_spmm_pair_acc(const CUtensorMap &ma, const CUtensorMap &mb, const CUtensorMap &me, const CUtensorMap &md, SpmmParams P,
                          const SumsParams &sums, int k_splits, cudaStream_t st) {
@@ -1853,11 +1860,8 @@ int launch_spmm_pair_acc(const CUtensorMap &ma, const CUtensorMap &mb, const CUt
     P.idesc = (P.idesc & ~(0x1Fu << 24)) | ((uint32_t)(256 >> 4) << 24) | ((uint32_t)(two::BN3 >> 3) << 17);
     const int64_t tiles = ((P.n + two::BN3 - 1) / two::BN3) * ((P.ms + 255) / 256);
     const int64_t pairs_max = sm_count_cached() / 2;
-    const int64_t k_iters = (P.k + (F8 ? 255 : 127)) / (F8 ? 256 : 128);
-    int64_t splits = k_splits ? k_splits : pairs_max / tiles;
-    if (splits < 1) splits = 1;
-    if (splits > k_iters) splits = k_iters;
-    if (F8 && splits > 2) splits = 2;       // two addends on a cleared buffer give the same bits in either order, three do not
+    constexpr int KE = F8 ? 256 : 128;
+    const int64_t splits = k_splits ? std::min<int64_t>(k_splits, (P.k + KE - 1) / KE) : pair_slices(P.ms, P.n, P.k, KE, sm_count_cached());
     P.k_splits = (int)splits;
     const int64_t units = tiles * splits;
     const unsigned pairs = (unsigned)(units < pairs_max ? units : pairs_max);
@@ -2001,6 +2005,14 @@ bool pair_takes_rows(int64_t ms, int64_t n, int64_t k, bool f8) {
     if (k <= 256) return false;
     if (k <= 512 && ms <= 384) return false;
     return ms > 128 || n <= 5120 || k > (f8 ? 1024 : 768);
+}
+
+// Row blocks of a tile and K slices of the 16-bit weight gradient on single CTAs.
+int single_row_blocks(int64_t ms) { return ms >= 256 ? 2 : 1; }
+int64_t single_slices(int64_t ms, int64_t n, int64_t k, int sms) {
+    const int64_t bn = n >= 192 ? 192 : 128, mpt = single_row_blocks(ms), k_iters = (k + 127) / 128;
+    const int64_t tiles = ((n + bn - 1) / bn) * ((ms / BM + mpt - 1) / mpt);
+    return std::max<int64_t>(1, std::min(sms / tiles, k_iters));
 }
 
 // Tile and K slices of the float8 weight gradient (added to out with float32 reductions).  At most two slices: two addends on a
@@ -2249,7 +2261,7 @@ extern "C" int sp24_spmm_f8(const void *a_packed, int dtype, int64_t ld_a, const
         bn = 128;
         mpt = tiles >= sms ? 2 : 1;
     }
-    // Weight gradient on CTA pairs: us, single CTAs -> pairs, ms 3072, n 768, k 8192 28.4 -> 15.3; ms 3072, n 3072, k 8192 89.8 -> 41.1;
+    // Weight gradient on CTA pairs: us, single CTAs -> pairs, ms 3072, n 768, k 8192 28.4 -> 15.3; ms 3072, n 3072, k 8192 91.7 -> 49.4;
     // ms 768, n 768, k 8192 16.2 -> 12.2; ms 1280, n 640, k 4096 11.3 -> 8.9; ms 2304, n 768, k 256 6.9 both.  Below these sizes the pair
     // kernel's longer start counts: ms 1024, n 1024, k 1024 7.0 -> 7.2; ms 2048, n 512, k 512 6.4 -> 6.9; ms 256, n 256, k 256 5.7 -> 6.4.
     if (!trans_out && n >= 256 && (k >= 2048 || ms * n >= 3 << 19) && pair_kernels_enabled()) {
@@ -2257,7 +2269,12 @@ extern "C" int sp24_spmm_f8(const void *a_packed, int dtype, int64_t ld_a, const
         if (int rc = make_map(&map_b, b, dtype, n, k, ld_b, 128, 128)) return rc;
         if (int rc = make_map_e(&map_e, e_tc, (ms / 128) * P.k_atoms, 2)) return rc;
         if (int rc = encode_map(&map_d, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, out, n, ms, ld_out * 4, 32, 16, CU_TENSOR_MAP_SWIZZLE_128B)) return rc;
-        return launch_spmm_pair_acc<false, true>(map_a, map_b, map_e, map_d, P, SumsParams{}, 0, st);
+        // slices: what the single-CTA kernel takes at least (the error grows with the length of a float32 accumulation), two at most
+        // (two addends on a cleared buffer give the same bits in either order, three do not)
+        int bn = 0, mpt = 0, slices = 1;
+        pick_f8_accumulate(ms, n, k, sm_count_cached(), bn, mpt, slices);
+        if (slices < 2 && pair_slices(ms, n, k, 256, sm_count_cached()) >= 2) slices = 2;
+        return launch_spmm_pair_acc<false, true>(map_a, map_b, map_e, map_d, P, SumsParams{}, slices, st);
     }
     if (!trans_out) {
         pick_f8_accumulate(ms, n, k, sms, bn, mpt, P.k_splits);
@@ -2404,10 +2421,10 @@ static int spmm_accumulate_impl(const void *a_packed, int dtype, int a_mn_major,
     P.idesc = (1u << 2) | (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(a_mn_major ? 1 : 0) << 15) | (1u << 16) |
               ((uint32_t)(BM >> 4) << 24);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    // CTA-pair kernel for at least one full tile of columns, also where the last 256-row block is half empty: us, single CTAs -> pairs,
-    // ms 384, n 256, k 1024 10.3 -> 6.7; ms 1152, n 1152, k 1984 15.2 -> 9.9; ms 2944, n 768, k 16384 51.6 -> 38.5; ms 128, n 768, k 2048
-    // 7.3 -> 7.2
-    bool pair_form = n >= 256;
+    // CTA-pair kernel for at least one full tile of columns, also where the last of several 256-row blocks is half empty: us, single CTAs
+    // -> pairs with as many slices, ms 384, n 256, k 1024 11.2 -> 6.8; ms 1152, n 1152, k 1984 15.9 -> 14.4, n 3072, k 8192 68.2 -> 35.3;
+    // ms 2944, n 768, k 16384 55.9 -> 47.1.  A single half-empty block lost: ms 128, n 1920, k 6016 13.2 -> 15.3.
+    bool pair_form = n >= 256 && ms > 128;
     pair_form = pair_form && pair_kernels_enabled();
     if (pair_form) {
         CUtensorMap map_e;
@@ -2417,22 +2434,18 @@ static int spmm_accumulate_impl(const void *a_packed, int dtype, int a_mn_major,
         rc = encode_map(&map_d, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, out, n, ms, ld_out * 4, 32, 16, CU_TENSOR_MAP_SWIZZLE_128B);
         if (rc) return rc;
         const SumsParams sums{row_parts, row_sums, n_parts, sums_accumulate};
+        // The error of a float32 accumulation on the tensor cores grows with its length: an output of 2176 x 768 over k 8128 in two
+        // slices is 2.4e-6 off, in four 1.2e-6.  Row counts that the single-CTA kernel took before keep its number of slices at least.
+        if (ms % 256 && !k_splits) k_splits = (int)std::max(single_slices(ms, n, k, sm_count_cached()), pair_slices(ms, n, k, 128, sm_count_cached()));
         return a_mn_major ? launch_spmm_pair_acc<true>(map_a, map_b, map_e, map_d, P, sums, k_splits, st)
                           : launch_spmm_pair_acc<false>(map_a, map_b, map_e, map_d, P, sums, k_splits, st);
     }
     if (row_sums)
         if (int rc2 = sp24_sum_parts(row_parts, n_parts, ms, row_sums, sums_accumulate, stream)) return rc2;
     // widest tile (least operand traffic per output), then as many K slices as idle SMs allow
-    const int sms = sm_count_cached();
     const bool wide = n >= 192;
-    const int bn = wide ? 192 : 128;
-    P.mblk_per_tile = ms >= 256 ? 2 : 1;
-    const int64_t tiles = ((n + bn - 1) / bn) * ((ms / BM + P.mblk_per_tile - 1) / P.mblk_per_tile);
-    const int64_t k_iters = (k + 127) / 128;
-    int64_t splits = k_splits ? k_splits : sms / tiles;
-    if (splits < 1) splits = 1;
-    if (splits > k_iters) splits = k_iters;
-    P.k_splits = (int)splits;
+    P.mblk_per_tile = single_row_blocks(ms);
+    P.k_splits = (int)(k_splits ? std::min<int64_t>(k_splits, (k + 127) / 128) : single_slices(ms, n, k, sm_count_cached()));
     // fp16 and bf16 operands share these kernels: the element type only enters through the tensor maps and the
     // instruction descriptor
     if (a_mn_major) return wide ? launch_spmm<192, false, true, true, false, float>(map_a, map_b, P, st)
