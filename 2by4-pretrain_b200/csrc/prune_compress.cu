@@ -710,7 +710,7 @@ __global__ void __launch_bounds__(256, col_min_blocks(MODE)) pc_col_kernel(PcPar
 // Bound by arithmetic: about 80 instructions a group of four for the draws, quotients and random numbers, which by themselves (operands
 // in shared memory, no traffic) take 115 cycles a warp and group, 67 % of the time measured here; the rest are copies, addresses and
 // metadata.  So: persistent blocks, whose warps fetch their 16 columns of the next two tiles by asynchronous copies (no registers hold
-// loads, no warp waits at the start of a block), compressed rows written over the storage rows that the same lane has read and stored
+// loads, no warp waits at the start of a block), compressed rows written over storage rows that have been read and stored
 // 16 bytes a lane, one barrier a tile (for the metadata, which eight warps assemble), and two groups at a time in two-lane arithmetic.
 // Two blocks of 128 registers: with three (80) or four (64) the loop's constants no longer fit and the same work is 106 and 109
 // instructions a group instead of 98.  us, one group at a time in a block per tile -> here: bf16 4096 x 8192 45.7 -> 39.4, fp16
@@ -743,6 +743,9 @@ mvue_col_kernel(const __grid_constant__ PcParams P, const __grid_constant__ Phil
     chain_enter();
     using Cfg = MvueCol<TIn>;
     constexpr int RT = Cfg::RT, ROW = Cfg::ROW, STAGES = Cfg::STAGES, V = 2;
+    // 16-bit input: a lane writes only over the four bytes of a row that it alone reads.  Float32 rows are twice as long: other lanes
+    // read where it writes.
+    constexpr bool OWN_BYTES = ROW == RT * sizeof(TOut) && V * sizeof(TIn) == 4;
     extern __shared__ __align__(16) uint8_t smem[];
     __shared__ __align__(8) PickEntry picks[16];
     load_pick_lut<TOut>(picks);
@@ -805,7 +808,9 @@ mvue_col_kernel(const __grid_constant__ PcParams P, const __grid_constant__ Phil
         __syncwarp();
         uint32_t word[V] = {0, 0};
         float rsum[V] = {0.f, 0.f};
-        if (r0 + lane * V < m && c < ncols) {
+        const bool mine = r0 + lane * V < m && c < ncols;      // all lanes, the first 16 or none
+        const uint32_t together = OWN_BYTES ? 0u : __ballot_sync(0xFFFFFFFFu, mine);
+        if (mine) {
             uint64_t pair[V];
             pair[0] = (uint64_t)(uint32_t)(r0 + lane * V) * row_pairs + (uint32_t)(c * 2);
             pair[1] = pair[0] + row_pairs;
@@ -830,7 +835,8 @@ mvue_col_kernel(const __grid_constant__ PcParams P, const __grid_constant__ Phil
                     }
                     word[v] += two_groups_fast<TOut>(x, v0, v1, picks_at, 1.f, o[0][v], o[1][v]) << (8 * step);
                 }
-                // stored rows take the place of the storage rows that this lane has read
+                // stored rows (128 bytes) take the place of the first storage rows, which all lanes have read by now
+                if constexpr (!OWN_BYTES) __syncwarp(together);
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     uint32_t *to = reinterpret_cast<uint32_t *>(sl + (4 * step + 2 * h) * 128) + lane;

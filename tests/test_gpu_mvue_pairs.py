@@ -49,6 +49,14 @@ def test_compression_has_the_dense_kernels_bits(m, k, dtype, col, special):
     assert bool((same | (odd & (want == 0) & back.isnan())).all())
 
 
+@pytest.mark.parametrize("dtype", list(NAMES), ids=NAMES.get)
+@pytest.mark.parametrize("m,k", [(1184, 8256), (2080, 4160)])
+def test_blocks_of_many_tiles_have_the_dense_kernels_bits(m, k, dtype):
+    """19 x 65 and 33 x 33 tiles on two blocks an SM: every stage is refilled after its operands were written over, and both buffers of
+    staged metadata are used again; remainders of 32 rows and 64 columns."""
+    test_compression_has_the_dense_kernels_bits(m, k, dtype, True, False)
+
+
 @pytest.mark.parametrize("m,k", [(32, 64), (96, 192), (1056, 2624)])
 def test_row_sums(m, k):
     """The row sums taken along the way: k float32 additions of exact values, against float64."""
