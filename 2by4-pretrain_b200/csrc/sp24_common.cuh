@@ -425,7 +425,9 @@ int sm_count();                // SMs of the current device
 // Programmatic dependent launch.  A kernel launched by launch_chained may start while the kernel before it on the stream is still
 // finishing (as soon as all blocks of that one have called chain_enter or left), so its launch latency and set-up are hidden behind
 // the other's last wave.  chain_enter first waits until everything before on the stream is complete and visible: no kernel touches
-// global memory before it, and every thread calls it, so a kernel's completion implies that of all kernels before it.
+// global memory before it, and every thread calls it, so a kernel's completion implies that of all kernels before it.  Its memory clobber
+// holds plain loads back.  It does not bind loads that promise read-only data (__ldg, ld.global.nc, __restrict__): the kernel before may
+// still be writing during this one's life, so there are none.
 __device__ __forceinline__ void chain_enter() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

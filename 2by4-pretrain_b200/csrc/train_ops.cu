@@ -105,6 +105,14 @@ __global__ void __launch_bounds__(256) layernorm_fwd_kernel(const float *x, cons
     }
 }
 
+// A load that is made wherever it is written: the compiler neither keeps the value for the next use (d values held over a row's two
+// passes spill up to 660 bytes a thread) nor moves the load ahead of chain_enter, as it may with one that promises read-only data.
+__device__ __forceinline__ float4 load4_again(const float4 *p) {
+    float4 v;
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
+
 // dx = rstd * (g dy - mean(g dy) - xhat mean(g dy xhat)) (+ dres);  dgamma += sum_rows dy xhat;  dbeta += sum_rows dy.
 // dres (optional): the gradient that reaches the norm's input along the residual stream, added before the store;
 // ddelta (optional): the same dx again in dy's element type, the gradient of the branch that was added in front.
@@ -144,7 +152,7 @@ __global__ void __launch_bounds__(32 * LnBwdWarps<NV>::value, 1)
         for (int i = 0; i < NV; ++i) {
             const float4 xv = load4<float>(x + base + i * 128);
             const float4 dv = load4<TDy>(dy + base + i * 128);
-            const float4 g = __ldg(g4 + i * 32);
+            const float4 g = load4_again(g4 + i * 32);
             const float4 xh = make_float4(fmaf(xv.x, rs, shift), fmaf(xv.y, rs, shift), fmaf(xv.z, rs, shift), fmaf(xv.w, rs, shift));
             const float4 gy = make_float4(dv.x * g.x, dv.y * g.y, dv.z * g.z, dv.w * g.w);
             s1 += (gy.x + gy.y) + (gy.z + gy.w);
@@ -162,7 +170,7 @@ __global__ void __launch_bounds__(32 * LnBwdWarps<NV>::value, 1)
             const int64_t at = base + i * 128;
             const float4 xv = load4<float>(x + at);
             const float4 dv = load4<TDy>(dy + at);
-            const float4 g = __ldg(g4 + i * 32);
+            const float4 g = load4_again(g4 + i * 32);
             // rs (g dy - m1 - xhat m2) = (rs g) dy + c1 + c2 xhat
             float4 o = make_float4(fmaf(c2, fmaf(xv.x, rs, shift), fmaf(rs * g.x, dv.x, c1)),
                                    fmaf(c2, fmaf(xv.y, rs, shift), fmaf(rs * g.y, dv.y, c1)),
