@@ -1216,8 +1216,9 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 // ------------------------------------------------------------------------------------------------
 // A handful of dense columns gives one tile per 256 rows: 16 pairs of 74 walk 32 K steps each for a 4096 x 4096 weight, and a step
 // takes the ring's latency whatever it computes.  Here a cluster of S pairs (S <= 4: eight CTAs) takes one tile, each pair every S-th
-// part of K with a ring of its own.  Every pair finishes a share of the tile's columns: it gets the others' float32 partial sums of
-// them in its shared memory, and after one cluster barrier adds them to its own in a fixed order, so results repeat bit for bit.
+// part of K with a ring of its own.  Every pair finishes a share of the tile's columns: all pairs leave their float32 partial sums of
+// them in its shared memory, and after one cluster barrier it adds them up in the order of the slices, its own like the others', so
+// results repeat bit for bit and equal tokens of a call have equal outputs.
 // (One pair finishing the whole tile took 1 us more at 32 columns and 2.5 at 64.)
 namespace two {
 constexpr int SPLIT_MAX = 4, BN_SPLIT = 64;                 // pairs a cluster, columns of a tile at most
@@ -1229,11 +1230,11 @@ __host__ __device__ constexpr int share(int bn, int slices) { return (bn + 4 * s
 // a partial share: columns in fours, 128 rows x 16 bytes each, so that a warp's remote store is 512 bytes in one piece
 __host__ __device__ constexpr int part_bytes(int bn, int slices) { return share(bn, slices) * BM * 4; }
 constexpr int split_stages(int bn, int slices) {
-    const int n = (SMEM_LIMIT - (slices - 1) * part_bytes(bn, slices) - (int)sizeof(Ctl2)) / stage2_bytes(false, bn);
+    const int n = (SMEM_LIMIT - slices * part_bytes(bn, slices) - (int)sizeof(Ctl2)) / stage2_bytes(false, bn);
     return n < MAX_STAGES2 ? n : MAX_STAGES2;
 }
 constexpr int split_smem(int bn, int slices) {
-    return split_stages(bn, slices) * stage2_bytes(false, bn) + (slices - 1) * part_bytes(bn, slices) + (int)sizeof(Ctl2);
+    return split_stages(bn, slices) * stage2_bytes(false, bn) + slices * part_bytes(bn, slices) + (int)sizeof(Ctl2);
 }
 static_assert(split_stages(BN_SPLIT, SPLIT_MAX) >= 4, "shared memory budget");
 }  // namespace two
@@ -1255,7 +1256,7 @@ spmm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *const smem = smem_raw;                // on 1024 bytes: checked by the launcher, the same in every CTA
     uint8_t *const parts = smem + STAGES * STAGE_BYTES;
-    Ctl2 &ctl = *reinterpret_cast<Ctl2 *>(parts + (S - 1) * part_bytes(BN, S));
+    Ctl2 &ctl = *reinterpret_cast<Ctl2 *>(parts + S * part_bytes(BN, S));
     uint64_t *const bars = ctl.bars;
     volatile int &abort_flag = ctl.abort_flag;
 
@@ -1289,7 +1290,6 @@ spmm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     const uint32_t tmem_base = ctl.tmem_base;
     chain_enter();
 
-    float acc[32];
     bool run = false;
     const int quad = warp & 3, half = (warp - 2) >> 2, HC = BN / 2, CW = share(BN, S);
     const int mrow = mblk * BM + quad * 32, left = P.n - row0 < BN ? (int)(P.n - row0) : BN;
@@ -1360,13 +1360,11 @@ spmm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
 #pragma unroll
             for (int q = 0; q < 8; ++q) {
                 const int col = half * HC + 4 * q, owner = owner_of(col);
-                if (4 * q < HC && col < left && owner != slice)
-                    st_cluster_v4(map_to_cta(smem_u32(parts + (slice - (slice > owner)) * part_bytes(BN, S)) +
-                                                 (col - owner * CW) * BM * 4 + (quad * 32 + lane) * 16, 2 * owner + rank),
+                if (4 * q < HC && col < left)
+                    st_cluster_v4(map_to_cta(smem_u32(parts + slice * part_bytes(BN, S)) + (col - owner * CW) * BM * 4 + (quad * 32 + lane) * 16,
+                                             2 * owner + rank),
                                   v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
             }
-#pragma unroll
-            for (int i = 0; i < 32; ++i) acc[i] = __uint_as_float(v[i]);
         }
         tc_fence_before();
     }
@@ -1378,7 +1376,10 @@ spmm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         const int c0 = half * HC;
         // columns of other pairs read the first 16 bytes instead, so that no load waits for a branch
         const uint32_t from = smem_u32(parts) + (quad * 32 + lane) * 16;
-        for (int p = 0; p < S - 1; ++p) {
+        float sum[32];
+#pragma unroll
+        for (int i = 0; i < 32; ++i) sum[i] = -0.f;            // plus x: x, whatever its sign
+        for (int p = 0; p < S; ++p) {
             uint4 o[8];
 #pragma unroll
             for (int q = 0; q < 8; ++q) {
@@ -1388,17 +1389,23 @@ spmm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             }
 #pragma unroll
             for (int q = 0; q < 8; ++q) {
-                acc[4 * q] += __uint_as_float(o[q].x);
-                acc[4 * q + 1] += __uint_as_float(o[q].y);
-                acc[4 * q + 2] += __uint_as_float(o[q].z);
-                acc[4 * q + 3] += __uint_as_float(o[q].w);
+                sum[4 * q] += __uint_as_float(o[q].x);
+                sum[4 * q + 1] += __uint_as_float(o[q].y);
+                sum[4 * q + 2] += __uint_as_float(o[q].z);
+                sum[4 * q + 3] += __uint_as_float(o[q].w);
             }
         }
-        OutT *dst = static_cast<OutT *>(P.out) + (row0 + c0) * P.ld_out + mrow + lane;      // 32 features of a token a store
-        const int first = max(slice * CW, c0) - c0, last = min(min((slice + 1) * CW, left), c0 + HC) - c0;      // this warp's columns
+        // this warp's columns, four a branch (a condition for each took 0.1 us more); a store: 32 features of a token
+        OutT *dst = static_cast<OutT *>(P.out) + (row0 + c0) * P.ld_out + mrow + lane;
+        const int first = max(slice * CW, c0) - c0, last = min(min((slice + 1) * CW, left), c0 + HC) - c0;
 #pragma unroll
-        for (int i = 0; i < 32; ++i, dst += P.ld_out)
-            if (i >= first && i < last) *dst = to_out<OutT>(acc[i] + bias);
+        for (int q = 0; q < 8; ++q, dst += 4 * P.ld_out)
+            if (4 * q >= first && 4 * q < last) {
+                OutT *d = dst;
+#pragma unroll
+                for (int i = 0; i < 4; ++i, d += P.ld_out)
+                    if (4 * q + i < last) *d = to_out<OutT>(sum[4 * q + i] + bias);
+            }
     }
     if (warp == 1) {
         tc_fence_after();

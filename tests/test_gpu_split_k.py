@@ -36,3 +36,26 @@ def test_few_columns(ms, n, k, col, dtype):
     assert bool(((out.double() - ref).abs() <= ROUND[dtype] * ref.abs() * 1.01 + (k + 4) * 2.0 ** -24 * mag).all())
     out.copy_(before[1:-1, 8:-8])
     assert torch.equal(buf, before)
+
+
+@pytest.mark.parametrize("bias", [False, True])
+@pytest.mark.parametrize("ms", [512, 4096, 7168])      # four, three and two slices of K where 15, 22 and 33 clusters of them fit
+def test_equal_tokens_have_equal_outputs(ms, bias):
+    """Products of 2^24, -2^24, 0.5 and 0.25 in different slices: every token's sum is 0.75 where the first two slices are added
+    up first, and one of the small products is lost where another slice comes between them.  Random tokens beside them: equal ones give the same bits."""
+    import sparse
+    from sparse import spmm
+    k, n = 4096, 63
+    w = torch.zeros(ms, k, device=DEV)
+    w[:, 0], w[:, 12 * 128], w[:, 22 * 128], w[:, 28 * 128] = 4096.0, -4096.0, 1.0, 1.0
+    x = torch.zeros(1, k, device=DEV)
+    x[:, 0], x[:, 12 * 128], x[:, 22 * 128], x[:, 28 * 128] = 4096.0, 4096.0, 0.5, 0.25
+    b = torch.zeros(ms, device=DEV).half() if bias else None
+    sp = sparse.to_sparse_semi_structured(w.half(), dtype=torch.float16)
+    y = spmm.sparse_linear(x.half().expand(n, k).contiguous(), sp.sparse_tensor_cutlass, sp.meta_tensor_cutlass, bias=b)
+    assert bool((y == 0.75).all())
+    sp = sparse.to_sparse_semi_structured(torch.randn(ms, k, device=DEV).half(), dtype=torch.float16)
+    x = torch.randn(1, k, device=DEV).half()
+    y = spmm.sparse_linear(x.expand(n, k).contiguous(), sp.sparse_tensor_cutlass, sp.meta_tensor_cutlass, bias=b)
+    spmm.check_status()
+    assert torch.equal(y, y[:1].expand(n, ms))
