@@ -1906,44 +1906,54 @@ void split_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute (&attr)[2], int s
     cfg.numAttrs = 2;
 }
 
-// Clusters of 2 s CTAs that the device holds at once (entry s; zeros where the kernel cannot run), worked out on its first call.
-struct SplitRoom { int64_t clusters[two::SPLIT_MAX + 1]; };
-template <bool A_MN, typename OutT> const SplitRoom *split_room() {
-    static SplitRoom room[64];
-    static bool done[64];
+// Whether the split kernel can run on the current device at all, worked out on the first call there.
+template <bool A_MN, typename OutT> bool split_runs() {
+    static bool runs[64], done[64];
     static std::mutex mu;
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
     std::lock_guard<std::mutex> lock(mu);
     if (!done[dev]) {
         auto kern = spmm_split_kernel<A_MN, OutT>;
         cudaFuncAttributes fa{};
         // dynamic shared memory on 1024 bytes, as in launch_spmm_pair
-        if (cudaFuncGetAttributes(&fa, kern) == cudaSuccess && fa.sharedSizeBytes % 1024 == 0 &&
-            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, two::SMEM_LIMIT) == cudaSuccess)
-            for (int s = 2; s <= two::SPLIT_MAX; ++s) {
-                cudaLaunchConfig_t cfg{};
-                cudaLaunchAttribute attr[2];
-                split_config(cfg, attr, s, 1, two::split_smem(two::BN_SPLIT, s), nullptr);
-                int n = 0;
-                if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess) room[dev].clusters[s] = n;
-            }
-        cudaGetLastError();
+        bool ok = cudaFuncGetAttributes(&fa, kern) == cudaSuccess && fa.sharedSizeBytes % 1024 == 0 &&
+                  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, two::SMEM_LIMIT) == cudaSuccess;
+        for (int s = 2; s <= two::SPLIT_MAX && ok; ++s) {
+            cudaLaunchConfig_t cfg{};
+            cudaLaunchAttribute attr[2];
+            split_config(cfg, attr, s, 1, two::split_smem(two::BN_SPLIT, s), nullptr);
+            int n = 0;
+            ok = cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess && n > 0;
+        }
+        if (!ok) cudaGetLastError();
+        runs[dev] = ok;
         done[dev] = true;
     }
-    return &room[dev];
+    return runs[dev];
 }
 
+// Clusters of this many CTAs, one CTA per SM, that a device of eight GPCs holds at once however its SMs (an even number in each) are
+// spread over them: a GPC leaves at most cluster - 2 of its SMs over.  On 148 SMs 33 clusters of four, 20 of six, 13 of eight; the
+// device measured here holds 33, 22 and 15.
+constexpr int64_t clusters_for_sure(int64_t cluster, int64_t sms) {
+    const int64_t used = sms - 8 * (cluster - 2);
+    return used > 0 ? (used + cluster - 1) / cluster : 0;
+}
+static_assert(clusters_for_sure(4, 148) == 33 && clusters_for_sure(6, 148) == 20 && clusters_for_sure(8, 148) == 13, "");
+
 // Slices of K for few columns (1: the pair kernel takes the call): the most that leave every tile a cluster at once, from eight K
-// steps (two a slice) on.  us, pair kernel -> here:
+// steps (two a slice) on.  They decide the order of the sums, so the rule knows sizes and the number of SMs only: the same bits on every
+// device with as many.  us, pair kernel -> here:
 //   ms 4096, k 4096: n 1 12.3 -> 7.6, n 33 12.5 -> 7.9; ms 512, k 4096, n 16 11.9 -> 5.8; ms 2304, k 3072, n 16 9.7 -> 5.7
 //   ms 1024, k 1024: n 1 5.2 -> 3.8, n 33 5.5 -> 4.2; ms 4096, k 1024, n 16 5.3 -> 4.9
 // Shorter K keeps the order of sums that the pair and single-CTA kernels share bit for bit; slices would gain 0.1 - 0.6 us there
 // (ms 512, n 16, k 512 4.1 -> 3.5).
-int pick_slices(int64_t ms, int64_t n, int bn, const SplitRoom &room) {
-    const int64_t tiles = ((ms + 255) / 256) * ((n + bn - 1) / bn);
+int pick_slices(int64_t ms, int64_t n, int64_t k, int sms) {
+    if (n > two::SPLIT_N || k <= two::SPLIT_K) return 1;
+    const int64_t tiles = (ms + 255) / 256;
     for (int s = two::SPLIT_MAX; s >= 2; --s)
-        if (tiles <= room.clusters[s]) return s;
+        if (tiles <= clusters_for_sure(2 * s, sms)) return s;
     return 1;
 }
 int split_bn(int64_t n) { return n <= 32 ? 32 : (n <= 48 ? 48 : 64); }
@@ -2150,11 +2160,11 @@ static int spmm_impl(const void *a_packed, int dtype, int a_mn_major, int64_t ld
     if (pair_form) {
         CUtensorMap map_b, map_e;
         P.bn = pick_pair_bn(ms, n, epi == EPI_PLAIN, false, sm_count_cached());
-        if (epi == EPI_PLAIN && n <= two::SPLIT_N && k > two::SPLIT_K && pair_kernels_enabled()) {
-            const SplitRoom *room = out_dtype == SP24_F16 ? (a_mn_major ? split_room<true, __half>() : split_room<false, __half>())
-                                                          : (a_mn_major ? split_room<true, __nv_bfloat16>() : split_room<false, __nv_bfloat16>());
-            P.k_splits = room ? pick_slices(ms, n, split_bn(n), *room) : 1;
-            if (P.k_splits > 1) P.bn = split_bn(n);
+        const int slices = epi == EPI_PLAIN && pair_kernels_enabled() ? pick_slices(ms, n, k, sm_count_cached()) : 1;
+        if (slices > 1 && (out_dtype == SP24_F16 ? (a_mn_major ? split_runs<true, __half>() : split_runs<false, __half>())
+                                                 : (a_mn_major ? split_runs<true, __nv_bfloat16>() : split_runs<false, __nv_bfloat16>()))) {
+            P.k_splits = slices;
+            P.bn = split_bn(n);
         }
         rc = make_map(&map_b, b, dtype, n, k, ld_b, 64, (uint32_t)P.bn / 2);
         if (rc) return rc;
@@ -2222,6 +2232,11 @@ extern "C" int sp24_spmm_mlp(const void *a_packed, int dtype, int a_mn_major, in
     if (epilogue == EPI_DGELU && bias) return SP24_ERR_ARG;
     return spmm_impl(a_packed, dtype, a_mn_major, ld_a, e_tc, ms, k, b, 0, ld_b, n, out, dtype, 1, ld_out, bias, 0, 1.f, status,
                      stream, bias_is_f32 ? 1 : 0, epilogue, aux, ld_aux);
+}
+
+extern "C" int sp24_k_slices(int64_t ms, int64_t n, int64_t k, int sms) {
+    if (ms <= 0 || ms % 128 || n <= 0 || k <= 0 || k % 64 || sms < 2) return 0;
+    return pick_slices(ms, n, k, sms);
 }
 
 extern "C" int sp24_pair_tile_columns(int64_t ms, int64_t n, int form, int sms) {

@@ -425,6 +425,12 @@ int sp24_spmm_scaled(const void *a_packed, int dtype, int64_t ld_a, const void *
  * 0 when no pair tile exists.
  */
 int sp24_pair_tile_columns(int64_t ms, int64_t n, int form, int sms);
+/*
+ * Slices that the 16-bit GEMM with token-major B and output (plain result, no activation) cuts K into for (ms, n, k) on a GPU of `sms`
+ * SMs: host arithmetic only.  1: no slices, the order of sums that all other kernels share.  Two or more: partial sums of consecutive
+ * slices, added up in their order.  0 for sizes that it does not take.
+ */
+int sp24_k_slices(int64_t ms, int64_t n, int64_t k, int sms);
 
 /*
  * The GEMMs of a float8 layer whose scales stay on the device: D = alpha * (A_sparse * B) [+ bias], alpha the product of

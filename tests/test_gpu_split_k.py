@@ -39,7 +39,7 @@ def test_few_columns(ms, n, k, col, dtype):
 
 
 @pytest.mark.parametrize("bias", [False, True])
-@pytest.mark.parametrize("ms", [512, 4096, 7168])      # four, three and two slices of K where 15, 22 and 33 clusters of them fit
+@pytest.mark.parametrize("ms", [512, 4096, 7168])      # four, three and two slices of K
 def test_equal_tokens_have_equal_outputs(ms, bias):
     """Products of 2^24, -2^24, 0.5 and 0.25 in different slices: every token's sum is 0.75 where the first two slices are added
     up first, and one of the small products is lost where another slice comes between them.  Random tokens beside them: equal ones give the same bits."""

@@ -32,3 +32,21 @@ def test_status_codes_say_what_happened(monkeypatch, code, says):
         spmm.check_status()
     assert says in str(e.value) and ("wait" in str(e.value)) == (code != 11) and "cuda:0" in str(e.value)
     spmm.check_status()
+
+
+def test_slices_of_k_fit_every_floor_plan():
+    """The number of slices, which decides the order of the sums, follows from sizes and the number of SMs alone, and its clusters all fit
+    at once whichever way the SMs (an even number in each of eight GPCs) are spread."""
+    from sparse import _ext
+    rule, rng = _ext.lib().sp24_k_slices, random.Random(1)
+    edges = [(13, 4), (14, 3), (20, 3), (21, 2), (33, 2), (34, 1)]
+    assert [rule(256 * t, 1, 1024, 148) for t, _ in edges] == [s for _, s in edges]
+    assert rule(13 * 256 + 128, 63, 960, 148) == 3 and rule(512, 64, 4096, 148) == 1 and rule(512, 1, 896, 148) == 1
+    assert rule(100, 1, 1024, 148) == 0 and rule(256, 0, 1024, 148) == 0
+    for _ in range(3000):
+        sms, plan = rng.choice([132, 144, 148, 152, 160]), [0] * 8
+        for _ in range(sms // 2):
+            plan[min(rng.randrange(8), rng.randrange(8))] += 2
+        tiles = rng.randint(1, 40)
+        s = rule(256 * tiles, rng.randint(1, 63), 128 * rng.randint(8, 40), sms)
+        assert s == 1 or tiles <= sum(gpc // (2 * s) for gpc in plan)
