@@ -421,6 +421,7 @@ inline int dtype_size(int dt) {
 int check_device();            // SP24_OK when the current device is compute capability 10.x
 int launch_status();           // maps cudaGetLastError() to SP24_OK / SP24_ERR_CUDA
 int sm_count();                // SMs of the current device
+int clear_words(void *dst, int64_t words, cudaStream_t st);      // zeros at dst, 4-byte aligned memory of the current device
 
 // Programmatic dependent launch.  A kernel launched by launch_chained may start while the kernel before it on the stream is still
 // finishing (as soon as all blocks of that one have called chain_enter or left), so its launch latency and set-up are hidden behind
