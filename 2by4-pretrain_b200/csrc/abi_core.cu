@@ -12,10 +12,10 @@ int check_device() {
     // with the same value, so concurrent first calls are harmless.
     static int cached[64];
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return SP24_ERR_CUDA;
+    if (cudaGetDevice(&dev) != cudaSuccess) return runtime_error();
     if (dev >= 0 && dev < 64 && cached[dev]) return cached[dev] == 1 ? SP24_OK : SP24_ERR_DEVICE;
     int major = 0;
-    if (cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev) != cudaSuccess) return SP24_ERR_CUDA;
+    if (cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev) != cudaSuccess) return runtime_error();
     const int ok = major == 10;
     if (dev >= 0 && dev < 64) cached[dev] = ok ? 1 : 2;
     return ok ? SP24_OK : SP24_ERR_DEVICE;
@@ -25,10 +25,15 @@ int check_device() {
 int sm_count() {
     static int cached[64];
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+    if (cudaGetDevice(&dev) != cudaSuccess) {
+        runtime_error();
+        return 148;
+    }
+    if (dev < 0 || dev >= 64) return 148;
     if (!cached[dev]) {
         int n = 0;
-        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) runtime_error();
+        if (n <= 0) n = 148;
         cached[dev] = n;
     }
     return cached[dev];
@@ -38,6 +43,11 @@ int launch_status() {
     const cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) return SP24_OK;
     if (getenv("SP24_DEBUG")) fprintf(stderr, "sparse24_b200: CUDA error %d: %s\n", (int)e, cudaGetErrorString(e));
+    return SP24_ERR_CUDA;
+}
+
+int runtime_error() {
+    launch_status();
     return SP24_ERR_CUDA;
 }
 
@@ -84,13 +94,12 @@ extern "C" int sp24_zero(void *dst, int64_t bytes, void *stream) {
         cudaPointerAttributes at{};
         int dev = -1;
         const bool known = cudaGetDevice(&dev) == cudaSuccess && cudaPointerGetAttributes(&at, dst) == cudaSuccess;
-        if (!known) sp24::launch_status();      // the memset says what is wrong
+        if (!known) sp24::runtime_error();      // the memset says what is wrong
         if (known && at.type == cudaMemoryTypeDevice && at.device == dev && sp24::check_device() == SP24_OK)
             return sp24::clear_words(dst, bytes / 4, st);
     }
     if (cudaMemsetAsync(dst, 0, (size_t)bytes, st) == cudaSuccess) return SP24_OK;
-    sp24::launch_status();         // clears (and with SP24_DEBUG prints) the runtime's error
-    return SP24_ERR_CUDA;
+    return sp24::runtime_error();
 }
 
 // Peer memory for exchanges that run on the copy engines: a buffer exported by its owner (cudaIpcGetMemHandle, or a
@@ -102,14 +111,11 @@ extern "C" int sp24_ipc_open(const void *handle, int handle_bytes, void **ptr) {
     cudaIpcMemHandle_t h;
     memcpy(&h, handle, sizeof(h));
     *ptr = nullptr;
-    if (cudaIpcOpenMemHandle(ptr, h, cudaIpcMemLazyEnablePeerAccess) != cudaSuccess) {
-        sp24::launch_status();     // clears (and with SP24_DEBUG prints) the runtime's error
-        return SP24_ERR_CUDA;
-    }
+    if (cudaIpcOpenMemHandle(ptr, h, cudaIpcMemLazyEnablePeerAccess) != cudaSuccess) return sp24::runtime_error();
     return SP24_OK;
 }
 
 extern "C" int sp24_ipc_close(void *ptr) {
     if (!ptr) return SP24_ERR_ARG;
-    return cudaIpcCloseMemHandle(ptr) == cudaSuccess ? SP24_OK : SP24_ERR_CUDA;
+    return cudaIpcCloseMemHandle(ptr) == cudaSuccess ? SP24_OK : sp24::runtime_error();
 }

@@ -900,7 +900,7 @@ template <auto KERN> int allow_shared_memory(int bytes) {
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64 || !done[dev]) {
-        if (cudaFuncSetAttribute(KERN, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) return SP24_ERR_CUDA;
+        if (cudaFuncSetAttribute(KERN, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) return runtime_error();
         if (dev >= 0 && dev < 64) done[dev] = true;
     }
     return SP24_OK;

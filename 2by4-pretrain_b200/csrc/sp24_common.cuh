@@ -420,6 +420,8 @@ inline int dtype_size(int dt) {
 }
 int check_device();            // SP24_OK when the current device is compute capability 10.x
 int launch_status();           // maps cudaGetLastError() to SP24_OK / SP24_ERR_CUDA
+int runtime_error();           // for a failed runtime call: takes its error out of the runtime (and with SP24_DEBUG prints it), so
+                               // that no later call reports it; always SP24_ERR_CUDA
 int sm_count();                // SMs of the current device
 int clear_words(void *dst, int64_t words, cudaStream_t st);      // zeros at dst, 4-byte aligned memory of the current device
 

@@ -1745,7 +1745,7 @@ int encode_map(CUtensorMap *map, CUtensorMapDataType type, const void *base, int
     const cuuint32_t box[2] = {box_cols, box_rows};
     const cuuint32_t estr[2] = {1, 1};
     EncodeTiledFn encode = encode_tiled_fn();
-    if (!encode) return SP24_ERR_CUDA;
+    if (!encode) return runtime_error();
     CUresult r = CUDA_SUCCESS;
     for (int attempt = 0; attempt < 2; ++attempt) {
         r = encode(map, type, 2, const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
@@ -1789,7 +1789,7 @@ int launch_spmm(const CUtensorMap &ma, const CUtensorMap &mb, SpmmParams P, cuda
     const int which = P.activation ? 1 : 0;
     if (dev >= 0 && dev < 64 && !attr_set[dev][which]) {
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM) != cudaSuccess)
-            return launch_status();
+            return runtime_error();
         attr_set[dev][which] = true;
     }
     P.idesc |= (uint32_t)(BN >> 3) << 17;
@@ -1815,10 +1815,10 @@ int launch_spmm_pair(const CUtensorMap &ma, const CUtensorMap &mb, const CUtenso
         // the kernel takes its dynamic shared memory as it comes: it starts on 1024 bytes only behind none, or whole kilobytes, of
         // static shared memory
         cudaFuncAttributes fa{};
-        if (cudaFuncGetAttributes(&fa, kern) != cudaSuccess) return SP24_ERR_CUDA;
+        if (cudaFuncGetAttributes(&fa, kern) != cudaSuccess) return runtime_error();
         if (fa.sharedSizeBytes % 1024) return SP24_ERR_ALIGN;
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX) != cudaSuccess)
-            return SP24_ERR_CUDA;
+            return runtime_error();
         attr_set[dev] = true;
     }
     // M = 256 over the CTA pair, N = bn
@@ -1841,7 +1841,7 @@ int launch_spmm_pair(const CUtensorMap &ma, const CUtensorMap &mb, const CUtenso
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    if (cudaLaunchKernelEx(&cfg, kern, ma, mb, me, P) != cudaSuccess) return SP24_ERR_CUDA;
+    if (cudaLaunchKernelEx(&cfg, kern, ma, mb, me, P) != cudaSuccess) return runtime_error();
     return launch_status();
 }
 
@@ -1860,7 +1860,7 @@ int launch_spmm_pair_acc(const CUtensorMap &ma, const CUtensorMap &mb, const CUt
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !attr_set[dev]) {
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, two::smem3(F8)) != cudaSuccess)
-            return launch_status();
+            return runtime_error();
         attr_set[dev] = true;
     }
     // M = 256 over the CTA pair, N = 256
@@ -1886,7 +1886,7 @@ int launch_spmm_pair_acc(const CUtensorMap &ma, const CUtensorMap &mb, const CUt
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    if (cudaLaunchKernelEx(&cfg, kern, ma, mb, me, md, P, sums) != cudaSuccess) return launch_status();
+    if (cudaLaunchKernelEx(&cfg, kern, ma, mb, me, md, P, sums) != cudaSuccess) return runtime_error();
     return launch_status();
 }
 
@@ -1910,8 +1910,9 @@ void split_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute (&attr)[2], int s
 template <bool A_MN, typename OutT> bool split_runs() {
     static bool runs[64], done[64];
     static std::mutex mu;
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
+    int dev = -1;
+    if (cudaGetDevice(&dev) != cudaSuccess) runtime_error();
+    if (dev < 0 || dev >= 64) return false;
     std::lock_guard<std::mutex> lock(mu);
     if (!done[dev]) {
         auto kern = spmm_split_kernel<A_MN, OutT>;
@@ -1926,7 +1927,7 @@ template <bool A_MN, typename OutT> bool split_runs() {
             int n = 0;
             ok = cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess && n > 0;
         }
-        if (!ok) cudaGetLastError();
+        if (!ok) runtime_error();
         runs[dev] = ok;
         done[dev] = true;
     }
@@ -1965,7 +1966,7 @@ int launch_spmm_split(const CUtensorMap &ma, const CUtensorMap &mb, const CUtens
     cudaLaunchConfig_t cfg{};
     cudaLaunchAttribute attr[2];
     split_config(cfg, attr, P.k_splits, ((P.ms + 255) / 256) * ((P.n + P.bn - 1) / P.bn), two::split_smem(P.bn, P.k_splits), st);
-    if (cudaLaunchKernelEx(&cfg, spmm_split_kernel<A_MN, OutT>, ma, mb, me, P) != cudaSuccess) return SP24_ERR_CUDA;
+    if (cudaLaunchKernelEx(&cfg, spmm_split_kernel<A_MN, OutT>, ma, mb, me, P) != cudaSuccess) return runtime_error();
     return launch_status();
 }
 
@@ -2372,11 +2373,11 @@ namespace {
 int noalloc_scratch(void **out) {
     static void *cached[64];
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return SP24_ERR_CUDA;
+    if (cudaGetDevice(&dev) != cudaSuccess) return runtime_error();
     if (dev < 0 || dev >= 64) return SP24_ERR_DEVICE;
     if (!cached[dev]) {
         void *p = nullptr;
-        if (cudaGetSymbolAddress(&p, g_noalloc_scratch) != cudaSuccess || !p) return SP24_ERR_CUDA;
+        if (cudaGetSymbolAddress(&p, g_noalloc_scratch) != cudaSuccess || !p) return runtime_error();
         cached[dev] = p;
     }
     *out = cached[dev];

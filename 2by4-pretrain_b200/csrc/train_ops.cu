@@ -658,11 +658,12 @@ static int layernorm_bwd_impl(const void *dy, int dy_dtype, const float *dres, c
         auto kern = layernorm_bwd_kernel<T_, NV_>; \
         if (smem > 48 * 1024 && dev >= 0 && dev < 64 && !attr_set[which][NV_ - 1][dev]) { \
             if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) \
-                return launch_status(); \
+                return runtime_error(); \
             attr_set[which][NV_ - 1][dev] = true; \
         } \
         int resident = 0;                                                /* persistent grid: every block resident at once */ \
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kern, 32 * W, smem) != cudaSuccess || resident < 1) resident = 1; \
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kern, 32 * W, smem) != cudaSuccess) runtime_error(); \
+        if (resident < 1) resident = 1; \
         int64_t blocks = (rows + W - 1) / W; \
         const int64_t cap = (int64_t)sm_count() * resident; \
         if (blocks > cap) blocks = cap; \
@@ -744,7 +745,7 @@ static int ce_fused_launch(const void *logits, const int64_t *targets, float *ls
         cudaGetDevice(&dev);
         if (dev >= 0 && dev < 64 && !attr_set[dev]) {
             if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 110 * 1024) != cudaSuccess)
-                return launch_status();
+                return runtime_error();
             attr_set[dev] = true;
         }
         launch_chained(st, kern, (unsigned)rows, 512, row_bytes, static_cast<const T *>(logits), targets, lse, loss, scale,
