@@ -8,12 +8,12 @@
 namespace sp24 {
 
 int check_device() {
-    // The answer is cached per device ordinal; the cache is written once per device and only ever
-    // with the same value, so concurrent first calls are harmless.
-    static int cached[64];
+    // The answer is cached per device ordinal; concurrent first calls write the same value.
+    static std::atomic<int> cached[64];
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return runtime_error();
-    if (dev >= 0 && dev < 64 && cached[dev]) return cached[dev] == 1 ? SP24_OK : SP24_ERR_DEVICE;
+    if (dev >= 0 && dev < 64)
+        if (const int known = cached[dev]) return known == 1 ? SP24_OK : SP24_ERR_DEVICE;
     int major = 0;
     if (cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev) != cudaSuccess) return runtime_error();
     const int ok = major == 10;
@@ -23,7 +23,7 @@ int check_device() {
 
 // Number of SMs of the current device (cached per device ordinal; 148 if the query fails).
 int sm_count() {
-    static int cached[64];
+    static std::atomic<int> cached[64];
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) {
         runtime_error();

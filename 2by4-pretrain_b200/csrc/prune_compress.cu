@@ -896,7 +896,7 @@ mvue_col_kernel(const __grid_constant__ PcParams P, const __grid_constant__ Phil
 
 // Lets a kernel take more than 48 KB of dynamic shared memory, once per kernel and device.
 template <auto KERN> int allow_shared_memory(int bytes) {
-    static bool done[64];
+    static std::atomic<bool> done[64];
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64 || !done[dev]) {

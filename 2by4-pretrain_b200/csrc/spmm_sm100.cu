@@ -1726,7 +1726,7 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t
                                   const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 EncodeTiledFn encode_tiled_fn() {
-    static EncodeTiledFn fn = nullptr;
+    static std::atomic<EncodeTiledFn> fn{nullptr};
     if (!fn) {
         void *p = nullptr;
         cudaDriverEntryPointQueryResult q;
@@ -1783,7 +1783,7 @@ int launch_spmm(const CUtensorMap &ma, const CUtensorMap &mb, SpmmParams P, cuda
     using Cfg = SpmmCfg<BN, F8, TRANS, OutT>;
     auto kern = P.activation ? spmm_kernel<BN, F8, A_MN, B_MN, TRANS, OutT, true>
                              : spmm_kernel<BN, F8, A_MN, B_MN, TRANS, OutT, false>;
-    static bool attr_set[64][2];
+    static std::atomic<bool> attr_set[64][2];
     int dev = 0;
     cudaGetDevice(&dev);
     const int which = P.activation ? 1 : 0;
@@ -1808,7 +1808,7 @@ template <bool A_MN, typename OutT, int EPI = EPI_PLAIN, bool F8 = false>
 int launch_spmm_pair(const CUtensorMap &ma, const CUtensorMap &mb, const CUtensorMap &me, SpmmParams P, cudaStream_t st) {
     auto kern = spmm_pair_kernel<A_MN, OutT, EPI, F8>;
     constexpr int SMEM_MAX = two::SMEM_LIMIT;
-    static bool attr_set[64];
+    static std::atomic<bool> attr_set[64];
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !attr_set[dev]) {
@@ -1855,7 +1855,7 @@ template <bool A_MN, bool F8 = false>
 int launch_spmm_pair_acc(const CUtensorMap &ma, const CUtensorMap &mb, const CUtensorMap &me, const CUtensorMap &md, SpmmParams P,
                          const SumsParams &sums, int k_splits, cudaStream_t st) {
     auto kern = spmm_pair_acc_kernel<A_MN, F8>;
-    static bool attr_set[64];
+    static std::atomic<bool> attr_set[64];
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !attr_set[dev]) {
@@ -2371,7 +2371,7 @@ namespace {
 // Device address of the array, looked up once per device.  In host code the array's name is only a
 // handle; the address a kernel can use comes from cudaGetSymbolAddress with that device current.
 int noalloc_scratch(void **out) {
-    static void *cached[64];
+    static std::atomic<void *> cached[64];
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return runtime_error();
     if (dev < 0 || dev >= 64) return SP24_ERR_DEVICE;

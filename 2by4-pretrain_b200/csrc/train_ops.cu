@@ -647,7 +647,7 @@ static int layernorm_bwd_impl(const void *dy, int dy_dtype, const float *dres, c
         return SP24_ERR_ALIGN;
     if (int rc = check_device()) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    static bool attr_set[3][8][64];
+    static std::atomic<bool> attr_set[3][8][64];
     int dev = 0;
     cudaGetDevice(&dev);
     const int which = dy_dtype == SP24_F32 ? 0 : (dy_dtype == SP24_F16 ? 1 : 2);
@@ -740,7 +740,7 @@ static int ce_fused_launch(const void *logits, const int64_t *targets, float *ls
     const bool staged = row_bytes <= 110 * 1024;           // two resident blocks per SM
     if (staged) {
         auto kern = ce_fused_kernel<T, true>;
-        static bool attr_set[64];
+        static std::atomic<bool> attr_set[64];
         int dev = 0;
         cudaGetDevice(&dev);
         if (dev >= 0 && dev < 64 && !attr_set[dev]) {
