@@ -40,9 +40,10 @@ def test_compression_clears_exactly_the_buffer(pieces, f8):
 
 
 @pytest.mark.parametrize("accumulate", [0, 1])
-@pytest.mark.parametrize("m,n,k", [(256, 256, 64), (384, 512, 1152), (1024, 256, 1088), (2304, 264, 2048)])
+@pytest.mark.parametrize("m,n,k", [(256, 256, 64), (384, 512, 1152), (1024, 256, 1088), (2304, 264, 2048), (128, 512, 1152), (384, 128, 1088)])
 def test_gemm_adds_up_the_row_sums(m, n, k, accumulate):
-    """The same bits as the launch of its own (one fixed order), for row blocks that the pair kernel takes and one that it does not."""
+    """The same bits as the launch of its own (one fixed order), for sizes that the pair kernel takes and two that it does not (a single row
+    block, few columns)."""
     from sparse import _ext
     from sparse.spmm import check_status
     lib = _ext.lib()

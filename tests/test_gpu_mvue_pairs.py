@@ -57,6 +57,40 @@ def test_blocks_of_many_tiles_have_the_dense_kernels_bits(m, k, dtype):
     test_compression_has_the_dense_kernels_bits(m, k, dtype, True, False)
 
 
+@pytest.mark.parametrize("dtype", list(NAMES), ids=NAMES.get)
+@pytest.mark.parametrize("m,k", [(128, 64), (384, 1088), (2176, 2112)])
+def test_pitches_metadata_copy_and_sums(m, k, dtype):
+    """Row pitches wider than the matrix on either side (16-byte steps), the metadata copy in tensor-core order where K ends inside an
+    atom, and row sums added by the same launch: the bits of the plain call, nothing written beside the rows."""
+    from sparse import _ext
+    lib, out = _ext.lib(), torch.float16 if dtype == torch.float32 else dtype
+    x = _x(m, k, dtype, True).t()                        # storage (k, m)
+    wide = torch.full((k, m + 24), float("nan"), dtype=dtype, device=DEV)
+    wide[:, 8:m + 8] = x
+    atoms = lib.sp24_meta_tc_bytes(m, k)
+
+    def call(src, packed, ld, ld_p):
+        meta, e_tc = torch.zeros(m * k // 16, dtype=torch.int16, device=DEV), torch.full((atoms,), 0x5A, dtype=torch.uint8, device=DEV)
+        sums = torch.full((m,), 3.0, device=DEV)
+        _ext.check(lib.sp24_prune_compress_ex(src.data_ptr(), _ext.dt(dtype), m, k, ld, 1, packed.data_ptr(), _ext.dt(out), ld_p, meta.data_ptr(),
+                                              _ext.PRUNE_MVUE_FAST, None, 0, None, 0, 7, 2, None, e_tc.data_ptr(), sums.data_ptr(), _ext.stream()),
+                   "prune_compress_ex")
+        return meta, e_tc, sums
+
+    plain = torch.empty(k // 2, m, dtype=out, device=DEV)
+    room = torch.full((k // 2, m + 40), 7.0, dtype=out, device=DEV)
+    meta, e_tc, sums = call(x, plain, m, m)
+    meta2, e_tc2, sums2 = call(wide[:, 8:], room[:, 16:], m + 24, m + 40)
+    assert torch.equal(_bits(room[:, 16:m + 16]), _bits(plain)) and torch.equal(meta, meta2) and torch.equal(e_tc, e_tc2)
+    assert bool((room[:, :16] == 7).all()) and bool((room[:, m + 16:] == 7).all())
+    want = torch.empty_like(e_tc)
+    _ext.check(lib.sp24_meta_to_tc(meta.data_ptr(), 2, m, k, want.data_ptr(), _ext.stream()), "meta_to_tc")
+    assert torch.equal(e_tc, want)
+    ref, mag = 3.0 + x.double().sum(0), 3.0 + x.double().abs().sum(0)
+    for s in (sums, sums2):                              # k float32 additions in whatever order the blocks come
+        assert bool(((s.double() - ref).abs() <= (k + 1) * 2.0 ** -24 * mag).all())
+
+
 @pytest.mark.parametrize("m,k", [(32, 64), (96, 192), (1056, 2624)])
 def test_row_sums(m, k):
     """The row sums taken along the way: k float32 additions of exact values, against float64."""

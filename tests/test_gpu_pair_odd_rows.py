@@ -43,6 +43,13 @@ def test_products(ms, n, k, col, dtype):
     _check(buf, before, out, ref, ROUND[dtype] * ref.abs() * 1.01 + (k + 2) * 2.0 ** -24 * mag)      # float32 sums, one rounding
 
 
+@pytest.mark.parametrize("col", [False, True])
+@pytest.mark.parametrize("ms,n,k", [(1152, 8200, 576), (640, 16390, 1088)])
+def test_products_of_more_tiles_than_pairs(ms, n, k, col):
+    """About 185 and 210 tiles on 74 pairs: the persistent loop, the second accumulator and a half-empty block that hands both back early."""
+    test_products(ms, n, k, col, torch.float16)
+
+
 @pytest.mark.parametrize("ms,n,k,splits", [(128, 256, 192, 0), (384, 264, 1088, 3), (1152, 1152, 1984, 0)])
 @pytest.mark.parametrize("col", [False, True])
 def test_weight_gradient(ms, n, k, splits, col):
@@ -75,3 +82,8 @@ def test_float8_products(ms, n, k):
     spmm.check_status()
     ref = spmm.sparse_linear(xq, packed, meta, alpha=sw * sx)
     _check(buf, before, out, ref.half().double(), torch.zeros(1, device=DEV, dtype=torch.float64))
+
+
+@pytest.mark.parametrize("ms,n,k", [(1152, 8200, 640), (640, 16390, 1152)])
+def test_float8_products_of_more_tiles_than_pairs(ms, n, k):
+    test_float8_products(ms, n, k)
