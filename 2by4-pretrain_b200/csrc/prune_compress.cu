@@ -717,7 +717,7 @@ __global__ void __launch_bounds__(256, col_min_blocks(MODE)) pc_col_kernel(PcPar
 // 3072 x 16384 64.1 -> 56.8, bf16 with row sums 3072 x 8192 38.0 -> 31.7, 768 x 8192 12.5 -> 11.1, fp16 512 x 256 5.5 -> 3.7.
 // Three or four stages of copies instead of two, and tiles of two or four 16-column slices a warp, gained nothing.
 template <typename TIn> struct MvueCol {
-    static constexpr int RT = 64, KT = 128;                      // a tile: rows x logical columns; a warp takes 16 of the columns
+    static constexpr int RT = 64;                                // rows of a tile; each of its eight warps takes 16 logical columns
     static constexpr int ROW = RT * sizeof(TIn);                 // bytes of one storage row of a tile
     static constexpr int SLICE = 16 * ROW, STAGES = 2;           // a warp's share, and how many of them are under way
     static constexpr int RUN = 0, LINE = 4 * 2 * RT * 2, SUMS = LINE + RT * 16, OUT = SUMS + 8 * RT * 4;     // staged results

@@ -1221,11 +1221,13 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 // results repeat bit for bit and equal tokens of a call have equal outputs.
 // (One pair finishing the whole tile took 1 us more at 32 columns and 2.5 at 64.)
 namespace two {
-constexpr int SPLIT_MAX = 4, BN_SPLIT = 64;                 // pairs a cluster, columns of a tile at most
+constexpr int SPLIT_MAX = 4, BN_SPLIT = 64;                 // pairs a cluster at most, the widest tile
 // Columns at most.  A training step of the FST and float8 layers has at least 64 tokens (their MVUE compression takes multiples of
 // 64) and keeps one order of sums whatever the kernel: an output rounded the other way makes other MVUE draws, which moves a
-// model's gradients by several percent.
+// model's gradients by several percent.  The bound is not where slices stop gaining: inference, which has no such reason, stops here
+// with it (ms 4096, k 4096: n 64 12.7 us, 8.3 in slices; n 128 13.3, 9.5).
 constexpr int64_t SPLIT_N = 63, SPLIT_K = 7 * 128;          // K above: see pick_slices
+static_assert(SPLIT_N <= BN_SPLIT, "one tile takes all columns");
 __host__ __device__ constexpr int share(int bn, int slices) { return (bn + 4 * slices - 1) / (4 * slices) * 4; }     // columns a pair finishes
 // a partial share: columns in fours, 128 rows x 16 bytes each, so that a warp's remote store is 512 bytes in one piece
 __host__ __device__ constexpr int part_bytes(int bn, int slices) { return share(bn, slices) * BM * 4; }
@@ -1263,11 +1265,8 @@ spmm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t cta = cluster_ctarank(), rank = cta & 1u, leader = cta & ~1u;      // rank in the pair; the pair's first CTA
     const int slice = (int)(cta >> 1);
-    const int n_tiles_m = (int)((P.ms + 2 * BM - 1) / (2 * BM));
-    const int tile = (int)blockIdx.x / (2 * S);
     const int k_iters = (int)((P.k + 127) / 128), it0 = slice * k_iters / S, it1 = (slice + 1) * k_iters / S;
-    const int mblk = (tile % n_tiles_m) * 2 + (int)rank;
-    const int64_t row0 = (int64_t)(tile / n_tiles_m) * BN;
+    const int mblk = (int)blockIdx.x / (2 * S) * 2 + (int)rank;      // a tile: 256 rows, all columns
 
     const uint32_t full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[MAX_STAGES2]), tmem_full = smem_u32(&bars[2 * MAX_STAGES2]);
     if (threadIdx.x == 0) {
@@ -1292,7 +1291,7 @@ spmm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
 
     bool run = false;
     const int quad = warp & 3, half = (warp - 2) >> 2, HC = BN / 2, CW = share(BN, S);
-    const int mrow = mblk * BM + quad * 32, left = P.n - row0 < BN ? (int)(P.n - row0) : BN;
+    const int mrow = mblk * BM + quad * 32, n = (int)P.n;
     auto owner_of = [&](int col) { return (col >= CW) + (col >= 2 * CW) + (col >= 3 * CW); };      // the pair that finishes a column
     if (warp == 0) {
         if (lane == 0) {
@@ -1310,8 +1309,8 @@ spmm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                     tma_load_2d_pair(sa + 8192, &map_a, mblk * BM + 64, it * 64, full_leader);
                 }
                 tma_load_2d_pair(sa + OFF_E, &map_e, 0, (int)(((int64_t)mblk * P.k_atoms + it) * 2), full_leader);
-                tma_load_2d_pair(sb, &map_b, it * 128, (int)row0 + (int)rank * (BN / 2), full_leader);
-                tma_load_2d_pair(sb + (BN / 2) * 128, &map_b, it * 128 + 64, (int)row0 + (int)rank * (BN / 2), full_leader);
+                tma_load_2d_pair(sb, &map_b, it * 128, (int)rank * (BN / 2), full_leader);
+                tma_load_2d_pair(sb + (BN / 2) * 128, &map_b, it * 128 + 64, (int)rank * (BN / 2), full_leader);
                 if (++s == STAGES) { s = 0; ph ^= 1; }
             }
             if (abort_flag && rank == 0) {
@@ -1360,7 +1359,7 @@ spmm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
 #pragma unroll
             for (int q = 0; q < 8; ++q) {
                 const int col = half * HC + 4 * q, owner = owner_of(col);
-                if (4 * q < HC && col < left)
+                if (4 * q < HC && col < n)
                     st_cluster_v4(map_to_cta(smem_u32(parts + slice * part_bytes(BN, S)) + (col - owner * CW) * BM * 4 + (quad * 32 + lane) * 16,
                                              2 * owner + rank),
                                   v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
@@ -1384,7 +1383,7 @@ spmm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
 #pragma unroll
             for (int q = 0; q < 8; ++q) {
                 const int col = c0 + 4 * q;
-                const bool mine = 4 * q < HC && col < left && owner_of(col) == slice;
+                const bool mine = 4 * q < HC && col < n && owner_of(col) == slice;
                 o[q] = ld_shared_v4(from + p * part_bytes(BN, S) + (mine ? (col - slice * CW) * BM * 4 : 0));
             }
 #pragma unroll
@@ -1396,8 +1395,8 @@ spmm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             }
         }
         // this warp's columns, four a branch (a condition for each took 0.1 us more); a store: 32 features of a token
-        OutT *dst = static_cast<OutT *>(P.out) + (row0 + c0) * P.ld_out + mrow + lane;
-        const int first = max(slice * CW, c0) - c0, last = min(min((slice + 1) * CW, left), c0 + HC) - c0;
+        OutT *dst = static_cast<OutT *>(P.out) + c0 * P.ld_out + mrow + lane;
+        const int first = max(slice * CW, c0) - c0, last = min(min((slice + 1) * CW, n), c0 + HC) - c0;
 #pragma unroll
         for (int q = 0; q < 8; ++q, dst += 4 * P.ld_out)
             if (4 * q >= first && 4 * q < last) {
@@ -1965,7 +1964,7 @@ int launch_spmm_split(const CUtensorMap &ma, const CUtensorMap &mb, const CUtens
     P.stages = two::split_stages(P.bn, P.k_splits);
     cudaLaunchConfig_t cfg{};
     cudaLaunchAttribute attr[2];
-    split_config(cfg, attr, P.k_splits, ((P.ms + 255) / 256) * ((P.n + P.bn - 1) / P.bn), two::split_smem(P.bn, P.k_splits), st);
+    split_config(cfg, attr, P.k_splits, (P.ms + 255) / 256, two::split_smem(P.bn, P.k_splits), st);
     if (cudaLaunchKernelEx(&cfg, spmm_split_kernel<A_MN, OutT>, ma, mb, me, P) != cudaSuccess) return runtime_error();
     return launch_status();
 }
