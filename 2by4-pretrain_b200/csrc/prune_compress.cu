@@ -455,7 +455,7 @@ template <typename TIn> struct ColVec {
     static constexpr int narrow = 1;
     // Fast MVUE with 8-bit results: two rows, two groups at a time, three blocks per SM, where one group at a time took four rows at two
     // blocks: the quantised bytes are gathered by one permute a group.  bf16 -> e4m3 with row sums and the quantised tensor, us:
-    // 3072 x 8192 49.9 -> 41.4, 768 x 8192 18.6 -> 13.9, 1024 x 1024 11.0 -> 6.8.
+    // 3072 x 8192 49.2 -> 41.0, 768 x 8192 17.3 -> 12.1, 1024 x 1024 10.6 -> 6.4.
     static constexpr int fast8 = 2;
 };
 
@@ -713,8 +713,9 @@ __global__ void __launch_bounds__(256, col_min_blocks(MODE)) pc_col_kernel(PcPar
 // loads, no warp waits at the start of a block), compressed rows written over storage rows that have been read and stored
 // 16 bytes a lane, one barrier a tile (for the metadata, which eight warps assemble), and two groups at a time in two-lane arithmetic.
 // Two blocks of 128 registers: with three (80) or four (64) the loop's constants no longer fit and the same work is 106 and 109
-// instructions a group instead of 98.  us, one group at a time in a block per tile -> here: bf16 4096 x 8192 45.7 -> 39.4, fp16
-// 3072 x 16384 64.1 -> 56.8, bf16 with row sums 3072 x 8192 38.0 -> 31.7, 768 x 8192 12.5 -> 11.1, fp16 512 x 256 5.5 -> 3.7.
+// instructions a group instead of 98.  us a replayed launch, one group at a time in a block per tile -> here: bf16 4096 x 8192 45.0 -> 38.0,
+// fp16 3072 x 16384 63.9 -> 55.9, bf16 with row sums 3072 x 8192 37.0 -> 29.2, 768 x 8192 11.2 -> 9.4, fp16 512 x 256 5.1 -> 3.1, float32
+// 4096 x 8192 42.7 -> 42.4, 512 x 256 5.0 -> 3.3.
 // Three or four stages of copies instead of two, and tiles of two or four 16-column slices a warp, gained nothing.
 template <typename TIn> struct MvueCol {
     static constexpr int RT = 64;                                // rows of a tile; each of its eight warps takes 16 logical columns

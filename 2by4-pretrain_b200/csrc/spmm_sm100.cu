@@ -2283,10 +2283,11 @@ extern "C" int sp24_spmm_f8(const void *a_packed, int dtype, int64_t ld_a, const
         bn = 128;
         mpt = tiles >= sms ? 2 : 1;
     }
-    // Weight gradient on CTA pairs: us, single CTAs -> pairs, ms 3072, n 768, k 8192 28.4 -> 15.3; ms 3072, n 3072, k 8192 91.7 -> 49.4;
-    // ms 768, n 768, k 8192 16.2 -> 12.2; ms 1280, n 640, k 4096 11.3 -> 8.9; ms 2304, n 768, k 256 6.9 both.  Below these sizes the pair
-    // kernel's longer start counts: ms 1024, n 1024, k 1024 7.0 -> 7.2; ms 2048, n 512, k 512 6.4 -> 6.9; ms 256, n 256, k 256 5.7 -> 6.4.
-    if (!trans_out && n >= 256 && (k >= 2048 || ms * n >= 3 << 19) && pair_kernels_enabled()) {
+    // Weight gradient on CTA pairs: us, single CTAs -> pairs, ms 3072, n 768, k 8192 27.3 -> 13.5; ms 3072, n 3072, k 8192 80.9 -> 45.1;
+    // ms 768, n 768, k 8192 15.9 -> 11.3; ms 1280, n 640, k 4096 11.1 -> 8.9; ms 3072, n 640, k 512 10.1 -> 7.5; ms 1024, n 3072, k 256
+    // 8.2 -> 7.3.  Below these sizes the pair kernel's longer start counts: ms 1024, n 1024, k 1024 6.8 -> 7.0; ms 2048, n 512, k 512
+    // 6.1 -> 6.7; ms 2048, n 1024, k 256 6.1 -> 6.7; ms 256, n 256, k 256 5.6 -> 6.3.
+    if (!trans_out && n >= 256 && (k >= 2048 || ms * n >= (k > 256 ? 3 << 19 : 3 << 20)) && pair_kernels_enabled()) {
         CUtensorMap map_e, map_d;
         if (int rc = make_map(&map_b, b, dtype, n, k, ld_b, 128, 128)) return rc;
         if (int rc = make_map_e(&map_e, e_tc, (ms / 128) * P.k_atoms, 2)) return rc;
