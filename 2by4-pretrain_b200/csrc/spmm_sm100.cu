@@ -2011,17 +2011,43 @@ int pick_pair_bn(int64_t ms, int64_t n, bool plain, bool f8, int sms) {
     return best;
 }
 
-// Whether the CTA-pair kernel takes an operand whose last 256-row block is half empty (ms an odd multiple of 128).  Mostly yes, us,
-// single-CTA kernel -> pairs: fp16 ms 896, n 1984, k 1152 8.7 -> 7.9, n 8192, k 3072 43.5 -> 27.7; ms 2944, n 16384, k 768 53.7 -> 49.2;
-// ms 128, n 256, k 512 5.4 -> 4.4; float8 ms 1152, n 8192, k 3072 46.1 -> 20.8.  Not where many columns meet few K steps, so that the
-// epilogue decides and the empty half's does nothing: ms 384, n 16384, k 256 9.1 -> 10.3; ms 384, n 4096, k 512 6.0 -> 6.3; ms 1152,
-// n 16384, k 256 17.1 -> 18.3; ms 128, n 8192, k 512 6.1 -> 6.7; float8 ms 128, n 16384, k 1024 8.5 -> 8.9.  (Also left to the single
-// CTAs by the third line although pairs are faster there: ms 384, n 16384, k 512 13.0 -> 11.6.)
-bool pair_takes_rows(int64_t ms, int64_t n, int64_t k, bool f8) {
-    if (ms % 256 == 0 || n <= 2560) return true;
-    if (k <= 256) return false;
-    if (k <= 512 && ms <= 384) return false;
-    return ms > 128 || n <= 5120 || k > (f8 ? 1024 : 768);
+// The single-CTA tile of a float8 product with 16-bit results: narrow, since beside the 16-bit staging buffer a wide tile's stages do not
+// fit twice.
+void pick_f8_tile(int64_t ms, int64_t n, int sms, int &bn, int &mpt) {
+    bn = 128;
+    mpt = ((n + 127) / 128) * ((ms / BM + 1) / 2) >= sms ? 2 : 1;
+}
+
+// Whether the CTA-pair kernel takes an operand whose last 256-row block is half empty (ms an odd multiple of 128): where its estimated
+// time is lower.  Both estimates, ns, are a start and, for every round of tiles, what the columns of a CTA's tile take to write and the
+// K steps to stage, less what the two overlap; fitted to a map over 8 row counts (128 .. 2944), 16 widths (64 .. 16384) and K from 64 to
+// 1536, which they meet by 3 % on average.  Pairs gain by the bytes that a K step stages and lose by a wide tile's epilogue, of which
+// the empty half does nothing.  us, single CTAs -> pairs, taken: fp16 ms 896, n 1984, k 1152 8.7 -> 7.9, n 8192, k 3072 43.5 -> 27.7;
+// ms 128, n 256, k 512 5.4 -> 4.4; float8 ms 1152, n 8192, k 3072 46.1 -> 20.8; left alone: ms 2176, n 1024, k 128 4.4 -> 5.3; ms 640,
+// n 3496, k 320 5.5 -> 6.2; float8 ms 896, n 2537, k 128 4.8 -> 5.6.  Over the map pairs are taken and up to 9 % slower at 22 of 1536
+// sizes in fp16 and at none of 1024 in float8.  Up to 320 columns they were never slower by more than 4 %.  Many columns and few K steps
+// (the lines in the middle) stay with single CTAs without an estimate.
+bool pair_takes_rows(int64_t ms, int64_t n, int64_t k, bool f8, int sms) {
+    if (ms % 256 == 0 || n <= 320) return true;
+    if (n > 2560) {
+        if (k <= 256 || (k <= 512 && ms <= 384)) return false;
+        if (ms == 128 && n > 5120 && k <= (f8 ? 1024 : 768)) return false;
+    }
+    const int64_t steps = (k + (f8 ? 255 : 127)) / (f8 ? 256 : 128);
+    auto rounds = [&](int64_t columns, int64_t row_blocks, int64_t units) {
+        const int64_t tiles = ((n + columns - 1) / columns) * ((ms / BM + row_blocks - 1) / row_blocks);
+        return (tiles + units - 1) / units;
+    };
+    const int64_t pair_bn = pick_pair_bn(ms, n, true, f8, sms);
+    const int64_t pair = 4100 + rounds(pair_bn, 2, sms / 2) * (f8 ? 12 * pair_bn + 340 * steps - 800 : 13 * pair_bn + 260 * steps - 800);
+    int bn = 128, mpt = 2;
+    if (f8) {
+        pick_f8_tile(ms, n, sms, bn, mpt);
+        return pair <= 3100 + rounds(bn, mpt, sms) * (7 * mpt * bn + (mpt == 2 ? 1000 : 650) * steps);
+    }
+    pick_tile(ms, n, sms, bn, mpt);
+    const int64_t step = 150 + (mpt * (A_STAGE_BYTES + 2048) + bn * 256) / 150;
+    return pair <= 3600 + rounds(bn, mpt, sms) * (11 * mpt * bn + step * steps - 1200);
 }
 
 // Row blocks of a tile and K slices of the 16-bit weight gradient on single CTAs.
@@ -2155,7 +2181,7 @@ static int spmm_impl(const void *a_packed, int dtype, int a_mn_major, int64_t ld
     P.idesc = (1u << 2) | ((i8 ? 2u : 1u) << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(a_mn_major ? 1 : 0) << 15) |
               ((uint32_t)(b_mn_major ? 1 : 0) << 16) | ((uint32_t)(BM >> 4) << 24);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    bool pair_form = pair_layout && pair_takes_rows(ms, n, k, false) && pair_kernels_enabled();
+    bool pair_form = pair_layout && pair_takes_rows(ms, n, k, false, sm_count_cached()) && pair_kernels_enabled();
     if (epi != EPI_PLAIN || bias_f32) pair_form = true;      // checked above: these forms exist in the pair kernel only
     if (pair_form) {
         CUtensorMap map_b, map_e;
@@ -2266,7 +2292,7 @@ extern "C" int sp24_spmm_f8(const void *a_packed, int dtype, int64_t ld_a, const
     const uint32_t fmt = dtype == SP24_E5M2 ? 1u : 0u;
     P.idesc = (1u << 2) | (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(BM >> 4) << 24);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (trans_out && out_dtype != SP24_F32 && pair_takes_rows(ms, n, k, true) && pair_kernels_enabled()) {
+    if (trans_out && out_dtype != SP24_F32 && pair_takes_rows(ms, n, k, true, sm_count_cached()) && pair_kernels_enabled()) {
         CUtensorMap map_e;
         P.bn = pick_pair_bn(ms, n, true, true, sm_count_cached());
         if (int rc = make_map(&map_b, b, dtype, n, k, ld_b, 128, (uint32_t)P.bn / 2)) return rc;
@@ -2277,12 +2303,7 @@ extern "C" int sp24_spmm_f8(const void *a_packed, int dtype, int64_t ld_a, const
     int bn = 128, mpt = 2;
     const int sms = sm_count_cached();
     pick_tile(ms, n, sms, bn, mpt);
-    if (trans_out && out_dtype != SP24_F32) {
-        // narrow tiles only: beside the 16-bit staging buffer a wide tile's stages do not fit twice
-        const int64_t tiles = ((n + 127) / 128) * ((ms / BM + 1) / 2);
-        bn = 128;
-        mpt = tiles >= sms ? 2 : 1;
-    }
+    if (trans_out && out_dtype != SP24_F32) pick_f8_tile(ms, n, sms, bn, mpt);
     // Weight gradient on CTA pairs: us, single CTAs -> pairs, ms 3072, n 768, k 8192 27.3 -> 13.5; ms 3072, n 3072, k 8192 80.9 -> 45.1;
     // ms 768, n 768, k 8192 15.9 -> 11.3; ms 1280, n 640, k 4096 11.1 -> 8.9; ms 3072, n 640, k 512 10.1 -> 7.5; ms 1024, n 3072, k 256
     // 8.2 -> 7.3.  Below these sizes the pair kernel's longer start counts: ms 1024, n 1024, k 1024 6.8 -> 7.0; ms 2048, n 512, k 512
