@@ -2465,11 +2465,26 @@ static int spmm_accumulate_impl(const void *a_packed, int dtype, int a_mn_major,
     P.idesc = (1u << 2) | (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(a_mn_major ? 1 : 0) << 15) | (1u << 16) |
               ((uint32_t)(BM >> 4) << 24);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    // CTA-pair kernel for at least one full tile of columns, also where the last of several 256-row blocks is half empty: us, single CTAs
-    // -> pairs with as many slices, ms 384, n 256, k 1024 11.2 -> 6.8; ms 1152, n 1152, k 1984 15.9 -> 14.4, n 3072, k 8192 68.2 -> 35.3;
-    // ms 2944, n 768, k 16384 55.9 -> 47.1.  A single half-empty block lost: ms 128, n 1920, k 6016 13.2 -> 15.3.
-    bool pair_form = n >= 256 && ms > 128;
-    pair_form = pair_form && pair_kernels_enabled();
+    // CTA-pair kernel for at least one full tile of columns
+    bool pair_form = n >= 256 && ms > 128 && pair_kernels_enabled();
+    if (pair_form && ms % 256) {
+        // The last of several 256-row blocks is half empty (a single one lost: ms 128, n 1920, k 6016 13.2 -> 15.3).  The error of a float32
+        // accumulation on the tensor cores grows with its length (2176 x 768 over k 8128: 2.4e-6 in two slices, 1.2e-6 in four), so these
+        // keep the single-CTA kernel's number of slices at least.  Where that makes more rounds of pairs than of CTAs the two are about
+        // even, pairs 17 % slower to 13 % faster over a map, and the single CTAs keep it, except that the row sums would be a launch of
+        // their own then (2.6 us).  us, single CTAs -> pairs, as many rounds: ms 384, n 256, k 1024 10.7 -> 7.6, ms 1152, n 3072, k 8192
+        // 65.0 -> 33.1; more rounds: ms 384, n 520, k 1984 11.4 -> 13.7, ms 2944, n 768, k 16384 51.4 -> 45.8.
+        const int sms = sm_count_cached();
+        const int64_t slices = k_splits ? std::min<int64_t>(k_splits, (k + 127) / 128) : single_slices(ms, n, k, sms);
+        if (!k_splits) k_splits = (int)std::max(slices, pair_slices(ms, n, k, 128, sms));
+        auto rounds = [&](int64_t columns, int64_t splits, int64_t units) {
+            return (((n + columns - 1) / columns) * ((ms + 255) / 256) * splits + units - 1) / units;
+        };
+        if (!row_sums && rounds(two::BN3, std::min<int64_t>(k_splits, (k + 127) / 128), sms / 2) > rounds(192, slices, sms)) {
+            pair_form = false;
+            k_splits = (int)slices;
+        }
+    }
     if (pair_form) {
         CUtensorMap map_e;
         rc = make_map_e(&map_e, e_tc, (ms / 128) * P.k_atoms);
@@ -2478,9 +2493,6 @@ static int spmm_accumulate_impl(const void *a_packed, int dtype, int a_mn_major,
         rc = encode_map(&map_d, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, out, n, ms, ld_out * 4, 32, 16, CU_TENSOR_MAP_SWIZZLE_128B);
         if (rc) return rc;
         const SumsParams sums{row_parts, row_sums, n_parts, sums_accumulate};
-        // The error of a float32 accumulation on the tensor cores grows with its length: an output of 2176 x 768 over k 8128 in two
-        // slices is 2.4e-6 off, in four 1.2e-6.  Row counts that the single-CTA kernel took before keep its number of slices at least.
-        if (ms % 256 && !k_splits) k_splits = (int)std::max(single_slices(ms, n, k, sm_count_cached()), pair_slices(ms, n, k, 128, sm_count_cached()));
         return a_mn_major ? launch_spmm_pair_acc<true>(map_a, map_b, map_e, map_d, P, sums, k_splits, st)
                           : launch_spmm_pair_acc<false>(map_a, map_b, map_e, map_d, P, sums, k_splits, st);
     }

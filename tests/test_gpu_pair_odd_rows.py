@@ -50,7 +50,7 @@ def test_products_of_more_tiles_than_pairs(ms, n, k, col):
     test_products(ms, n, k, col, torch.float16)
 
 
-@pytest.mark.parametrize("ms,n,k,splits", [(128, 256, 192, 0), (384, 264, 1088, 3), (1152, 1152, 1984, 0)])
+@pytest.mark.parametrize("ms,n,k,splits", [(128, 256, 192, 0), (384, 264, 1088, 3), (1152, 1152, 1984, 0), (384, 520, 1024, 0), (640, 264, 1088, 0), (384, 264, 64, 5)])
 @pytest.mark.parametrize("col", [False, True])
 def test_weight_gradient(ms, n, k, splits, col):
     import sparse
