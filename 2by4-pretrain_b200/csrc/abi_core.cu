@@ -84,7 +84,7 @@ int clear_words(void *dst, int64_t words, cudaStream_t st) {
 }
 }  // namespace sp24
 
-// Small buffers in the current device's memory are cleared by a kernel: a memset in the stream ends the chain of the kernels around
+// Small buffers in the current device's memory are cleared by a kernel: a memset in the stream ends the overlap of the kernels around
 // it (launch_chained).  The runtime's memset keeps what a kernel of this device may not be able to reach: memory of the host, of another
 // device or managed, and pointers that the runtime does not know.
 extern "C" int sp24_zero(void *dst, int64_t bytes, void *stream) {

@@ -426,16 +426,16 @@ int runtime_error();           // for a failed runtime call: takes its error out
 int sm_count();                // SMs of the current device
 int clear_words(void *dst, int64_t words, cudaStream_t st);      // zeros at dst, 4-byte aligned memory of the current device
 
-// Programmatic dependent launch.  A kernel launched by launch_chained is placed as soon as all blocks of the kernel before it on the
-// stream have left, before that one counts as complete, so its launch latency and set-up are hidden.  chain_enter waits until everything
-// before on the stream is complete and visible: no kernel touches global memory before it, and every thread calls it, so a kernel's
-// completion implies that of all kernels before it.  Its memory clobber holds plain loads back.  It does not bind loads that promise
-// read-only data (__ldg, ld.global.nc, __restrict__), which are not for a kernel whose input may not be visible yet, so there are none.
-// Nothing lets the next kernel in earlier (griddepcontrol.launch_dependents): its blocks would fill the SMs that have room first, up to
-// their resident limit, where a balanced placement takes fewer a SM.  us, early -> here, replayed back to back: exact MVUE 2048 x 2048
-// 17.7 -> 13.0, dense MVUE fp16 2048 x 1024 5.5 -> 4.3, selection 2048 x 1024 7.2 -> 5.6 (before chained launches 13.3, 4.6, 6.1); of 576
-// kernels and sizes 29 had become slower by more than 4 %, now one.  A GEMM after a GEMM loses 1 % (2043 tokens, 4096 x 4096 38.3 -> 38.8).
-__device__ __forceinline__ void chain_enter() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Programmatic dependent launch.  A kernel launched by launch_chained may start while the kernel before it on the stream is still
+// finishing (as soon as all blocks of that one have called chain_enter or left), so its launch latency and set-up are hidden behind
+// the other's last wave.  chain_enter first waits until everything before on the stream is complete and visible: no kernel touches
+// global memory before it, and every thread calls it, so a kernel's completion implies that of all kernels before it.  Its memory clobber
+// holds plain loads back.  It does not bind loads that promise read-only data (__ldg, ld.global.nc, __restrict__): the kernel before may
+// still be writing during this one's life, so there are none.
+__device__ __forceinline__ void chain_enter() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 // Errors are left for launch_status, as with a <<<>>> launch.
 template <typename... P, typename... A>
 inline void launch_chained(cudaStream_t st, void (*kern)(P...), dim3 grid, unsigned threads, size_t smem, A &&...args) {
