@@ -78,6 +78,23 @@ __global__ void __launch_bounds__(256) clear_kernel(uint32_t *dst, int64_t words
 }
 }  // namespace
 
+int resident_blocks(const void *kern, unsigned threads, size_t smem) {
+    struct Known {
+        const void *kern;
+        unsigned threads;
+        size_t smem;
+        int blocks;
+    };
+    static thread_local Known known[64];      // by a hash of the kernel's address; what falls together is asked for again
+    Known &k = known[(reinterpret_cast<uintptr_t>(kern) >> 4) * 0x9E3779B97F4A7C15ull >> 58];
+    if (k.kern != kern || k.threads != threads || k.smem != smem) {
+        int n = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, (int)threads, smem) != cudaSuccess) runtime_error();
+        k = {kern, threads, smem, n};
+    }
+    return k.blocks;
+}
+
 int clear_words(void *dst, int64_t words, cudaStream_t st) {
     launch_chained(st, clear_kernel, (unsigned)((words + 1023) / 1024), 256, 0, static_cast<uint32_t *>(dst), words);
     return launch_status();
