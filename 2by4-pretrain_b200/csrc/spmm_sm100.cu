@@ -1944,9 +1944,9 @@ static_assert(clusters_for_sure(4, 148) == 33 && clusters_for_sure(6, 148) == 20
 
 // Slices of K for few columns (1: the pair kernel takes the call): the most that leave every tile a cluster at once, from eight K
 // steps (two a slice) on.  They decide the order of the sums, so the rule knows sizes and the number of SMs only: the same bits on every
-// device with as many.  us, pair kernel -> here:
-//   ms 4096, k 4096: n 1 12.3 -> 7.6, n 33 12.5 -> 7.9; ms 512, k 4096, n 16 11.9 -> 5.8; ms 2304, k 3072, n 16 9.7 -> 5.7
-//   ms 1024, k 1024: n 1 5.2 -> 3.8, n 33 5.5 -> 4.2; ms 4096, k 1024, n 16 5.3 -> 4.9
+// device with as many.  us a replayed launch, pair kernel -> here:
+//   ms 4096, k 4096: n 1 11.8 -> 6.8, n 33 12.1 -> 7.2; ms 512, k 4096, n 16 11.7 -> 5.6; ms 2304, k 3072, n 16 9.5 -> 5.5
+//   ms 1024, k 1024: n 1 5.0 -> 3.5, n 33 5.3 -> 4.0; ms 4096, k 1024, n 16 5.1 -> 4.7; ms 5632, k 4096, n 16 11.8 -> 8.1
 // Shorter K keeps the order of sums that the pair and single-CTA kernels share bit for bit; slices would gain 0.1 - 0.6 us there
 // (ms 512, n 16, k 512 4.1 -> 3.5).
 int pick_slices(int64_t ms, int64_t n, int64_t k, int sms) {
@@ -2181,12 +2181,13 @@ static int spmm_impl(const void *a_packed, int dtype, int a_mn_major, int64_t ld
     P.idesc = (1u << 2) | ((i8 ? 2u : 1u) << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(a_mn_major ? 1 : 0) << 15) |
               ((uint32_t)(b_mn_major ? 1 : 0) << 16) | ((uint32_t)(BM >> 4) << 24);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    bool pair_form = pair_layout && pair_takes_rows(ms, n, k, false, sm_count_cached()) && pair_kernels_enabled();
+    const int sms = sm_count_cached();
+    bool pair_form = pair_layout && pair_takes_rows(ms, n, k, false, sms) && pair_kernels_enabled();
     if (epi != EPI_PLAIN || bias_f32) pair_form = true;      // checked above: these forms exist in the pair kernel only
     if (pair_form) {
         CUtensorMap map_b, map_e;
-        P.bn = pick_pair_bn(ms, n, epi == EPI_PLAIN, false, sm_count_cached());
-        const int slices = epi == EPI_PLAIN && pair_kernels_enabled() ? pick_slices(ms, n, k, sm_count_cached()) : 1;
+        P.bn = pick_pair_bn(ms, n, epi == EPI_PLAIN, false, sms);
+        const int slices = epi == EPI_PLAIN && pair_kernels_enabled() ? pick_slices(ms, n, k, sms) : 1;
         if (slices > 1 && (out_dtype == SP24_F16 ? (a_mn_major ? split_runs<true, __half>() : split_runs<false, __half>())
                                                  : (a_mn_major ? split_runs<true, __nv_bfloat16>() : split_runs<false, __nv_bfloat16>()))) {
             P.k_splits = slices;
@@ -2215,7 +2216,7 @@ static int spmm_impl(const void *a_packed, int dtype, int a_mn_major, int64_t ld
 #undef SP24_PAIR
     }
     int bn = 128, mpt = 2;
-    pick_tile(ms, n, sm_count_cached(), bn, mpt);
+    pick_tile(ms, n, sms, bn, mpt);
     P.mblk_per_tile = mpt;
 #define SP24_GO(F8_, AMN_, BMN_, TR_, OT_) return dispatch_bn<F8_, AMN_, BMN_, TR_, OT_>(bn, b, dtype, n, k, ld_b, map_a, P, st)
     if (i8) {
@@ -2292,16 +2293,16 @@ extern "C" int sp24_spmm_f8(const void *a_packed, int dtype, int64_t ld_a, const
     const uint32_t fmt = dtype == SP24_E5M2 ? 1u : 0u;
     P.idesc = (1u << 2) | (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(BM >> 4) << 24);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (trans_out && out_dtype != SP24_F32 && pair_takes_rows(ms, n, k, true, sm_count_cached()) && pair_kernels_enabled()) {
+    const int sms = sm_count_cached();
+    if (trans_out && out_dtype != SP24_F32 && pair_takes_rows(ms, n, k, true, sms) && pair_kernels_enabled()) {
         CUtensorMap map_e;
-        P.bn = pick_pair_bn(ms, n, true, true, sm_count_cached());
+        P.bn = pick_pair_bn(ms, n, true, true, sms);
         if (int rc = make_map(&map_b, b, dtype, n, k, ld_b, 128, (uint32_t)P.bn / 2)) return rc;
         if (int rc = make_map_e(&map_e, e_tc, (ms / 128) * P.k_atoms, 2)) return rc;
         return out_dtype == SP24_F16 ? launch_spmm_pair<false, __half, EPI_PLAIN, true>(map_a, map_b, map_e, P, st)
                                      : launch_spmm_pair<false, __nv_bfloat16, EPI_PLAIN, true>(map_a, map_b, map_e, P, st);
     }
     int bn = 128, mpt = 2;
-    const int sms = sm_count_cached();
     pick_tile(ms, n, sms, bn, mpt);
     if (trans_out && out_dtype != SP24_F32) pick_f8_tile(ms, n, sms, bn, mpt);
     // Weight gradient on CTA pairs: us, single CTAs -> pairs, ms 3072, n 768, k 8192 27.3 -> 13.5; ms 3072, n 3072, k 8192 80.9 -> 45.1;
@@ -2316,8 +2317,8 @@ extern "C" int sp24_spmm_f8(const void *a_packed, int dtype, int64_t ld_a, const
         // slices: what the single-CTA kernel takes at least (the error grows with the length of a float32 accumulation), two at most
         // (two addends on a cleared buffer give the same bits in either order, three do not)
         int bn = 0, mpt = 0, slices = 1;
-        pick_f8_accumulate(ms, n, k, sm_count_cached(), bn, mpt, slices);
-        if (slices < 2 && pair_slices(ms, n, k, 256, sm_count_cached()) >= 2) slices = 2;
+        pick_f8_accumulate(ms, n, k, sms, bn, mpt, slices);
+        if (slices < 2 && pair_slices(ms, n, k, 256, sms) >= 2) slices = 2;
         return launch_spmm_pair_acc<false, true>(map_a, map_b, map_e, map_d, P, SumsParams{}, slices, st);
     }
     if (!trans_out) {

@@ -65,7 +65,7 @@ const char *sp24_strerror(int code);
 /* ABI version of the loaded library (bumped when a signature changes). */
 int sp24_abi_version(void);
 
-/* Zero `bytes` bytes of device memory on `stream` (an output that a following kernel adds to). */
+/* Zero `bytes` bytes of device memory on `stream` (an output that a following kernel adds to).  Any memory that cudaMemsetAsync takes. */
 int sp24_zero(void *dst, int64_t bytes, void *stream);
 
 /*
@@ -420,9 +420,10 @@ int sp24_spmm_scaled(const void *a_packed, int dtype, int64_t ld_a, const void *
                      float alpha, int *status, void *stream);
 
 /*
- * Columns of the tile that the CTA-pair GEMM takes for (ms, n) on a GPU of `sms` SMs: host arithmetic only, for tests and for
- * reading a profile.  form 0: 16-bit operands, plain result; 1: a fused epilogue (sp24_spmm_mlp); 2: float8 (sp24_spmm_f8).
- * 0 when no pair tile exists.
+ * Columns of the tile that the CTA-pair GEMM takes for (ms, n), ms a multiple of 256, on a GPU of `sms` SMs: host arithmetic only, for
+ * tests and for reading a profile.  form 0: 16-bit operands, plain result; 1: a fused epilogue (sp24_spmm_mlp); 2: float8 (sp24_spmm_f8).
+ * 0 for other arguments: whether an odd multiple of 128 rows runs on CTA pairs depends on k too, and its tile is then that of ms + 128.
+ * Where sp24_k_slices tells of slices, form 0 runs on another kernel, whose tile is 32, 48 or 64 columns.
  */
 int sp24_pair_tile_columns(int64_t ms, int64_t n, int form, int sms);
 /*
