@@ -184,11 +184,11 @@ template <typename T, int OP, bool HAS_U> __global__ void __launch_bounds__(256)
 template <typename T, int OP, bool HAS_U> int launch_dense(const DenseParams &P, int col_major, cudaStream_t st) {
     if (!col_major) {
         const int64_t total = P.m * (P.k / 8);
-        launch_chained(st, dense_row_kernel<T, OP, HAS_U>, (unsigned)((total + 511) / 512), 256, 0, P);
+        launch_balanced(st, dense_row_kernel<T, OP, HAS_U>, (unsigned)((total + 511) / 512), 256, 0, P);
     } else {
         constexpr int V = 16 / sizeof(T);
         dim3 grid((unsigned)((P.m / V + 255) / 256), (unsigned)(P.k / 8));
-        launch_chained(st, dense_col_kernel<T, OP, HAS_U>, grid, 256, 0, P);
+        launch_balanced(st, dense_col_kernel<T, OP, HAS_U>, grid, 256, 0, P);
     }
     return launch_status();
 }

@@ -926,7 +926,8 @@ int launch(const PcParams &P, int col_major, cudaStream_t st) {
     constexpr int CH = sizeof(TOut) == 2 ? 16 : 32;
     if (!col_major) {
         dim3 grid((unsigned)((P.k / CH + 31) / 32), (unsigned)(P.m / 32));
-        launch_chained(st, pc_row_kernel<TIn, TOut, MODE, HAS_U>, grid, 256, 0, P);
+        if constexpr (is_mvue(MODE)) launch_balanced(st, pc_row_kernel<TIn, TOut, MODE, HAS_U>, grid, 256, 0, P);
+        else launch_chained(st, pc_row_kernel<TIn, TOut, MODE, HAS_U>, grid, 256, 0, P);
     } else if constexpr (MODE == SP24_PRUNE_MVUE_FAST && sizeof(TOut) == 2) {
         using Cfg = MvueCol<TIn>;
         constexpr auto kern = mvue_col_kernel<TIn, TOut>;
@@ -938,7 +939,8 @@ int launch(const PcParams &P, int col_major, cudaStream_t st) {
                                                        : (MODE == SP24_PRUNE_MVUE ? ColVec<TIn>::narrow : ColVec<TIn>::wide);
         constexpr int RT = 32 * V;
         dim3 grid((unsigned)((P.m + RT - 1) / RT), (unsigned)((P.k / CH + 7) / 8));
-        launch_chained(st, pc_col_kernel<TIn, TOut, MODE, HAS_U, V>, grid, 256, 0, P);
+        if constexpr (is_mvue(MODE)) launch_balanced(st, pc_col_kernel<TIn, TOut, MODE, HAS_U, V>, grid, 256, 0, P);
+        else launch_chained(st, pc_col_kernel<TIn, TOut, MODE, HAS_U, V>, grid, 256, 0, P);
     }
     return launch_status();
 }

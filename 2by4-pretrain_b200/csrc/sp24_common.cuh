@@ -426,7 +426,7 @@ int runtime_error();           // for a failed runtime call: takes its error out
 int sm_count();                // SMs of the current device
 int clear_words(void *dst, int64_t words, cudaStream_t st);      // zeros at dst, 4-byte aligned memory of the current device
 
-// Programmatic dependent launch.  A kernel launched by launch_chained, for most grids, may start while the kernel before it on the
+// Programmatic dependent launch.  A kernel launched by launch_chained may start while the kernel before it on the
 // stream is still finishing (as soon as all blocks of that one have called chain_enter or left), so its launch latency and set-up are
 // hidden behind the other's last wave.  chain_enter first waits until everything before on the stream is complete and visible: no kernel
 // touches global memory before it, and every thread calls it, so a kernel's completion implies that of all kernels before it.  Its memory
@@ -436,14 +436,6 @@ __device__ __forceinline__ void chain_enter() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
-// Blocks of a kernel that an SM holds at once (kept per thread; the runtime's answer is the same for every device this library runs on).
-int resident_blocks(const void *kern, unsigned threads, size_t smem);
-// Plain stream order for a grid of more blocks than SMs that leaves SMs room for more than an even share: placed while the kernel before
-// it still holds some SMs, its blocks fill the others up to their resident limit, three on some and one on others where two each take
-// two thirds of the time.  us, replayed back to back, chained -> in plain order: exact MVUE 2048 x 2048 17.7 -> 13.4, dense MVUE fp16
-// 2048 x 1024 5.5 -> 4.6, selection fp16 2048 x 1024 7.2 -> 6.1; a float8 layer step of 4096 tokens, 1024 -> 1024, 71.7 -> 66.7.  Letting
-// the next kernel in at the end of each kernel only (no launch_dependents) mends these too, but takes 2 - 10 % from layer steps: fst
-// 256 tokens, 256 -> 512, 22.7 -> 25.4.
 // Errors are left for launch_status, as with a <<<>>> launch.
 template <typename... P, typename... A>
 inline void launch_chained(cudaStream_t st, void (*kern)(P...), dim3 grid, unsigned threads, size_t smem, A &&...args) {
@@ -457,9 +449,25 @@ inline void launch_chained(cudaStream_t st, void (*kern)(P...), dim3 grid, unsig
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    const int64_t blocks = (int64_t)grid.x * grid.y * grid.z, sms = sm_count();
-    if (blocks > sms && (blocks + sms - 1) / sms < resident_blocks(reinterpret_cast<const void *>(kern), threads, smem)) cfg.numAttrs = 0;
     (void)cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...);
+}
+
+// Blocks of a kernel that an SM holds at once (kept per thread; the runtime's answer is the same for every device this library runs on).
+int resident_blocks(const void *kern, unsigned threads, size_t smem);
+// For kernels whose blocks compute for long: plain stream order where the grid has more blocks than the GPU SMs and an SM has room for more
+// than its even share.  Placed while the kernel before it still holds some SMs, its blocks fill the others up to their resident limit, three
+// on some and one on others where two each take two thirds of the time.  us, replayed back to back, chained -> here: exact MVUE
+// 2048 x 2048 17.7 -> 13.4, dense MVUE fp16 2048 x 1024 5.5 -> 4.6, selection fp16 2048 x 1024 7.2 -> 6.1; layer steps of 4096 tokens,
+// float8 1024 -> 1024 71.5 -> 68.7, fst 3072 -> 768 60.0 -> 57.3.  Kernels that stream keep their 0.4 us from the chain at most sizes (layer norm 2048 x 512 2.4,
+// here 2.8) and lose more than that at a few (4096 x 512 3.1 -> 3.6).  Letting the next kernel in at the end of each kernel only (no
+// launch_dependents) mends all of these, but takes 2 - 10 % from layer steps: fst 256 tokens, 256 -> 512, 22.7 -> 25.4.
+template <typename... P, typename... A>
+inline void launch_balanced(cudaStream_t st, void (*kern)(P...), dim3 grid, unsigned threads, size_t smem, A &&...args) {
+    const int64_t blocks = (int64_t)grid.x * grid.y * grid.z, sms = sm_count();
+    if (blocks > sms && (blocks + sms - 1) / sms < resident_blocks(reinterpret_cast<const void *>(kern), threads, smem))
+        kern<<<grid, threads, smem, st>>>(std::forward<A>(args)...);
+    else
+        launch_chained(st, kern, grid, threads, smem, std::forward<A>(args)...);
 }
 
 }  // namespace sp24

@@ -445,9 +445,9 @@ template <typename T, typename TOut, bool SELECT, bool TC> int launch_dual_form(
     dim3 grid((unsigned)((P.k + 127) / 128), (unsigned)(P.m / 64));
     constexpr int limit = dual_few_limit<T, TOut>(SELECT, false);
     if (limit == ALWAYS_FEW || (uint64_t)grid.x * grid.y <= (uint64_t)limit * sm_count()) {
-        if constexpr (limit > 0) launch_chained(st, ts_dual_kernel<T, TOut, SELECT, TC, true>, grid, 256, 0, P);
+        if constexpr (limit > 0) launch_balanced(st, ts_dual_kernel<T, TOut, SELECT, TC, true>, grid, 256, 0, P);
     } else {
-        if constexpr (limit < ALWAYS_FEW) launch_chained(st, ts_dual_kernel<T, TOut, SELECT, TC, false>, grid, 256, 0, P);
+        if constexpr (limit < ALWAYS_FEW) launch_balanced(st, ts_dual_kernel<T, TOut, SELECT, TC, false>, grid, 256, 0, P);
     }
     return launch_status();
 }
@@ -456,9 +456,9 @@ template <typename T, typename TOut, bool SELECT, bool TC> int launch_dual_list(
     const unsigned grid = B.first[B.count];
     constexpr int limit = dual_few_limit<T, TOut>(SELECT, true);
     if (limit == ALWAYS_FEW || grid <= (uint64_t)limit * sm_count()) {
-        if constexpr (limit > 0) launch_chained(st, ts_dual_batch_kernel<T, TOut, SELECT, TC, true>, grid, 256, 0, B);
+        if constexpr (limit > 0) launch_balanced(st, ts_dual_batch_kernel<T, TOut, SELECT, TC, true>, grid, 256, 0, B);
     } else {
-        if constexpr (limit < ALWAYS_FEW) launch_chained(st, ts_dual_batch_kernel<T, TOut, SELECT, TC, false>, grid, 256, 0, B);
+        if constexpr (limit < ALWAYS_FEW) launch_balanced(st, ts_dual_batch_kernel<T, TOut, SELECT, TC, false>, grid, 256, 0, B);
     }
     return launch_status();
 }
@@ -507,15 +507,15 @@ extern "C" int sp24_transposable_select(const void *x, int dtype, int64_t m, int
     uint8_t *mk = static_cast<uint8_t *>(mask_out);
     switch (dtype) {
         case SP24_F32:
-            launch_chained(st, ts_select_kernel<float>, grid, 256, 0, static_cast<const float *>(x), static_cast<float *>(sparse_out), mk,
+            launch_balanced(st, ts_select_kernel<float>, grid, 256, 0, static_cast<const float *>(x), static_cast<float *>(sparse_out), mk,
                                                           k, ld_x, ld_sparse, ld_mask, use_abs);
             break;
         case SP24_F16:
-            launch_chained(st, ts_select_kernel<__half>, grid, 256, 0, static_cast<const __half *>(x), static_cast<__half *>(sparse_out),
+            launch_balanced(st, ts_select_kernel<__half>, grid, 256, 0, static_cast<const __half *>(x), static_cast<__half *>(sparse_out),
                                                            mk, k, ld_x, ld_sparse, ld_mask, use_abs);
             break;
         default:
-            launch_chained(st, ts_select_kernel<__nv_bfloat16>, grid, 256, 0, static_cast<const __nv_bfloat16 *>(x),
+            launch_balanced(st, ts_select_kernel<__nv_bfloat16>, grid, 256, 0, static_cast<const __nv_bfloat16 *>(x),
                                                                   static_cast<__nv_bfloat16 *>(sparse_out), mk, k, ld_x,
                                                                   ld_sparse, ld_mask, use_abs);
     }

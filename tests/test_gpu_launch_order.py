@@ -1,5 +1,5 @@
 """Which launches of the library may start behind the last wave of the one before (programmatic edges in a captured graph) and which go
-in plain stream order: grids that would crowd on the SMs with room."""
+in plain stream order: grids of long blocks that would crowd on the SMs with room."""
 import ctypes
 
 import pytest
