@@ -212,6 +212,7 @@ struct SpmmParams {
     const float *amax_a, *amax_b;   // float8: absolute maxima of the operands on the device; alpha is the product of their scales
     int bn, stages;         // CTA-pair kernel: tile columns and operand stages
     int accumulate;         // float8, float32 output (ms, n): add alpha * A * B instead of storing it
+    int whole_columns;      // CTA-pair weight gradient: map_b is one of make_map_columns
     void *aux;              // fused MLP epilogues (CTA-pair kernel): second tensor shaped and pitched like out
     int64_t ld_aux;
 };
@@ -850,6 +851,13 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap
         "l"(map), "r"(x), "r"(y), "r"(bar_cluster)
         : "memory");
 }
+// a box of two 128-byte columns (see make_map_columns), one behind the other in shared memory
+__device__ __forceinline__ void tma_load_columns_pair(uint32_t dst, const CUtensorMap *map, int row, int column, uint32_t bar_cluster) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
+        "l"(map), "r"(0), "r"(row), "r"(column), "r"(bar_cluster)
+        : "memory");
+}
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t dst_smem, uint32_t cols) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst_smem), "r"(cols) : "memory");
 }
@@ -972,14 +980,12 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                     if constexpr (!A_MN) {
                         tma_load_2d_pair(sa, &map_a, it * (KE / 2), mrow, full_leader);
                     } else {
-                        tma_load_2d_pair(sa, &map_a, mrow, it * 64, full_leader);
-                        tma_load_2d_pair(sa + 8192, &map_a, mrow + 64, it * 64, full_leader);
+                        tma_load_columns_pair(sa, &map_a, it * 64, mrow / 64, full_leader);
                     }
                     // metadata of this row block and K step: two rows of 1024 bytes per atom of the table (8-bit: two atoms)
                     tma_load_2d_pair(sa + OFF_E, &map_e, 0, (int)(((int64_t)mblk * P.k_atoms + it * (F8 ? 2 : 1)) * 2), full_leader);
                     // this CTA's half of B: BN / 2 rows x two 128-byte K atoms
-                    tma_load_2d_pair(sb, &map_b, it * KE, brow, full_leader);
-                    tma_load_2d_pair(sb + (BN / 2) * 128, &map_b, it * KE + KE / 2, brow, full_leader);
+                    tma_load_columns_pair(sb, &map_b, brow, 2 * it, full_leader);
                     SP24_TRACE(0, g);
                     if (++s == STAGES) { s = 0; ph ^= 1; }
                 }
@@ -1305,12 +1311,10 @@ spmm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                 if constexpr (!A_MN) {
                     tma_load_2d_pair(sa, &map_a, it * 64, mblk * BM, full_leader);
                 } else {
-                    tma_load_2d_pair(sa, &map_a, mblk * BM, it * 64, full_leader);
-                    tma_load_2d_pair(sa + 8192, &map_a, mblk * BM + 64, it * 64, full_leader);
+                    tma_load_columns_pair(sa, &map_a, it * 64, mblk * 2, full_leader);
                 }
                 tma_load_2d_pair(sa + OFF_E, &map_e, 0, (int)(((int64_t)mblk * P.k_atoms + it) * 2), full_leader);
-                tma_load_2d_pair(sb, &map_b, it * 128, (int)rank * (BN / 2), full_leader);
-                tma_load_2d_pair(sb + (BN / 2) * 128, &map_b, it * 128 + 64, (int)rank * (BN / 2), full_leader);
+                tma_load_columns_pair(sb, &map_b, (int)rank * (BN / 2), 2 * it, full_leader);
                 if (++s == STAGES) { s = 0; ph ^= 1; }
             }
             if (abort_flag && rank == 0) {
@@ -1521,14 +1525,14 @@ spmm_pair_acc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                     if constexpr (!A_MN) {
                         tma_load_2d_pair(sa, &map_a, it * (KE / 2), mrow, full_leader);
                     } else {
-                        tma_load_2d_pair(sa, &map_a, mrow, it * 64, full_leader);
-                        tma_load_2d_pair(sa + 8192, &map_a, mrow + 64, it * 64, full_leader);
+                        tma_load_columns_pair(sa, &map_a, it * 64, mrow / 64, full_leader);
                     }
                     tma_load_2d_pair(sa + OFF_E, &map_e, 0, (int)(((int64_t)mblk * P.k_atoms + it * (F8 ? 2 : 1)) * 2), full_leader);
                     // this CTA's 128 columns of B: two boxes of 64 columns x 128 K-rows, or of 128 columns x 128 bytes of K
                     if constexpr (F8) {
-                        tma_load_2d_pair(sb, &map_b, it * KE, bcol, full_leader);
-                        tma_load_2d_pair(sb + 16384, &map_b, it * KE + 128, bcol, full_leader);
+                        tma_load_columns_pair(sb, &map_b, bcol, 2 * it, full_leader);
+                    } else if (P.whole_columns) {
+                        tma_load_columns_pair(sb, &map_b, it * 128, bcol / 64, full_leader);
                     } else {
                         tma_load_2d_pair(sb, &map_b, bcol, it * 128, full_leader);
                         tma_load_2d_pair(sb + 16384, &map_b, bcol + 64, it * 128, full_leader);
@@ -1736,18 +1740,18 @@ EncodeTiledFn encode_tiled_fn() {
     return fn;
 }
 
-// 2-D tensor map over rows of `cols` elements, row_bytes apart.
+// Tensor map over rows of `cols` elements, row_bytes apart; a third dimension where depth is given: depth_bytes apart, box_depth of them a box.
 int encode_map(CUtensorMap *map, CUtensorMapDataType type, const void *base, int64_t cols, int64_t rows, int64_t row_bytes, uint32_t box_cols,
-               uint32_t box_rows, CUtensorMapSwizzle swizzle) {
-    const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)row_bytes};
-    const cuuint32_t box[2] = {box_cols, box_rows};
-    const cuuint32_t estr[2] = {1, 1};
+               uint32_t box_rows, CUtensorMapSwizzle swizzle, int64_t depth = 0, int64_t depth_bytes = 0, uint32_t box_depth = 0) {
+    const cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, (cuuint64_t)depth};
+    const cuuint64_t strides[2] = {(cuuint64_t)row_bytes, (cuuint64_t)depth_bytes};
+    const cuuint32_t box[3] = {box_cols, box_rows, box_depth};
+    const cuuint32_t estr[3] = {1, 1, 1};
     EncodeTiledFn encode = encode_tiled_fn();
     if (!encode) return runtime_error();
     CUresult r = CUDA_SUCCESS;
     for (int attempt = 0; attempt < 2; ++attempt) {
-        r = encode(map, type, 2, const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+        r = encode(map, type, depth ? 3 : 2, const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (r != CUDA_ERROR_INVALID_CONTEXT) break;
         // a host thread that has made no runtime call yet (an autograd worker) has no current context for this
@@ -1764,6 +1768,16 @@ int encode_map(CUtensorMap *map, CUtensorMapDataType type, const void *base, int
 int make_map(CUtensorMap *map, const void *base, int dt, int64_t rows, int64_t cols, int64_t ld, uint32_t box_cols,
              uint32_t box_rows) {
     return encode_map(map, tmap_dtype(dt), base, cols, rows, ld * dtype_size(dt), box_cols, box_rows, CU_TENSOR_MAP_SWIZZLE_128B);
+}
+
+// The same operand as columns of 128 bytes, two a box: one request of an SM's copy engine instead of two, each of which holds the next one up
+// (a K step is bound by the requests' latency).  us a launch, two boxes -> one: ms 4096, k 4096, n 16 / 64 / 256 / 2043 7.7 / 13.4 /
+// 14.0 / 28.0 -> 7.3 / 12.2 / 13.0 / 27.3; ms 768, n 8192: k 2304 (column-major A) 20.2 -> 18.2, k 3072 23.3 -> 22.0; weight gradient
+// ms 2304, n 768, k 8192 20.8 -> 19.5; K of 768, which the epilogue bounds, 0 - 3 %.  cols must fill whole columns: a last one reaching past
+// them would read the next row.  An operand of an odd number of columns gets zeros for the second half of its last box.
+int make_map_columns(CUtensorMap *map, const void *base, int dt, int64_t rows, int64_t cols, int64_t ld, uint32_t box_rows) {
+    const int64_t es = dtype_size(dt), w = 128 / es;
+    return encode_map(map, tmap_dtype(dt), base, w, rows, ld * es, (uint32_t)w, box_rows, CU_TENSOR_MAP_SWIZZLE_128B, cols / w, 128, 2);
 }
 
 // SP24_SPMM_PAIR=0 in the environment keeps every GEMM on the single-CTA kernels (read once per process)
@@ -2157,9 +2171,6 @@ static int spmm_impl(const void *a_packed, int dtype, int a_mn_major, int64_t ld
 
     CUtensorMap map_a;
     int rc;
-    if (!a_mn_major) rc = make_map(&map_a, a_packed, dtype, ms, k / 2, ld_a, f8 ? 128 : 64, 128);
-    else rc = make_map(&map_a, a_packed, dtype, k / 2, ms, ld_a, 64, 64);
-    if (rc) return rc;
 
     SpmmParams P{};
     P.e_tc = e_tc; P.out = out; P.bias = bias; P.ms = ms; P.n = n; P.k = k; P.ld_out = ld_out;
@@ -2184,6 +2195,9 @@ static int spmm_impl(const void *a_packed, int dtype, int a_mn_major, int64_t ld
     const int sms = sm_count_cached();
     bool pair_form = pair_layout && pair_takes_rows(ms, n, k, false, sms) && pair_kernels_enabled();
     if (epi != EPI_PLAIN || bias_f32) pair_form = true;      // checked above: these forms exist in the pair kernel only
+    if (a_mn_major) rc = pair_form ? make_map_columns(&map_a, a_packed, dtype, k / 2, ms, ld_a, 64) : make_map(&map_a, a_packed, dtype, k / 2, ms, ld_a, 64, 64);
+    else rc = make_map(&map_a, a_packed, dtype, ms, k / 2, ld_a, f8 ? 128 : 64, 128);
+    if (rc) return rc;
     if (pair_form) {
         CUtensorMap map_b, map_e;
         P.bn = pick_pair_bn(ms, n, epi == EPI_PLAIN, false, sms);
@@ -2193,7 +2207,7 @@ static int spmm_impl(const void *a_packed, int dtype, int a_mn_major, int64_t ld
             P.k_splits = slices;
             P.bn = split_bn(n);
         }
-        rc = make_map(&map_b, b, dtype, n, k, ld_b, 64, (uint32_t)P.bn / 2);
+        rc = make_map_columns(&map_b, b, dtype, n, k, ld_b, (uint32_t)P.bn / 2);
         if (rc) return rc;
         rc = make_map_e(&map_e, e_tc, (ms / 128) * P.k_atoms);
         if (rc) return rc;
@@ -2297,7 +2311,7 @@ extern "C" int sp24_spmm_f8(const void *a_packed, int dtype, int64_t ld_a, const
     if (trans_out && out_dtype != SP24_F32 && pair_takes_rows(ms, n, k, true, sms) && pair_kernels_enabled()) {
         CUtensorMap map_e;
         P.bn = pick_pair_bn(ms, n, true, true, sms);
-        if (int rc = make_map(&map_b, b, dtype, n, k, ld_b, 128, (uint32_t)P.bn / 2)) return rc;
+        if (int rc = make_map_columns(&map_b, b, dtype, n, k, ld_b, (uint32_t)P.bn / 2)) return rc;
         if (int rc = make_map_e(&map_e, e_tc, (ms / 128) * P.k_atoms, 2)) return rc;
         return out_dtype == SP24_F16 ? launch_spmm_pair<false, __half, EPI_PLAIN, true>(map_a, map_b, map_e, P, st)
                                      : launch_spmm_pair<false, __nv_bfloat16, EPI_PLAIN, true>(map_a, map_b, map_e, P, st);
@@ -2311,7 +2325,7 @@ extern "C" int sp24_spmm_f8(const void *a_packed, int dtype, int64_t ld_a, const
     // 6.1 -> 6.7; ms 2048, n 1024, k 256 6.1 -> 6.7; ms 256, n 256, k 256 5.6 -> 6.3.
     if (!trans_out && n >= 256 && (k >= 2048 || ms * n >= (k > 256 ? 3 << 19 : 3 << 20)) && pair_kernels_enabled()) {
         CUtensorMap map_e, map_d;
-        if (int rc = make_map(&map_b, b, dtype, n, k, ld_b, 128, 128)) return rc;
+        if (int rc = make_map_columns(&map_b, b, dtype, n, k, ld_b, 128)) return rc;
         if (int rc = make_map_e(&map_e, e_tc, (ms / 128) * P.k_atoms, 2)) return rc;
         if (int rc = encode_map(&map_d, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, out, n, ms, ld_out * 4, 32, 16, CU_TENSOR_MAP_SWIZZLE_128B)) return rc;
         // slices: what the single-CTA kernel takes at least (the error grows with the length of a float32 accumulation), two at most
@@ -2450,14 +2464,6 @@ static int spmm_accumulate_impl(const void *a_packed, int dtype, int a_mn_major,
     if (!aligned16(a_packed) || !aligned16(e_tc) || !aligned16(b) || !aligned16(out)) return SP24_ERR_ALIGN;
     if (int rc = check_device()) return rc;
 
-    CUtensorMap map_a, map_b;
-    int rc;
-    if (!a_mn_major) rc = make_map(&map_a, a_packed, dtype, ms, k / 2, ld_a, 64, 128);
-    else rc = make_map(&map_a, a_packed, dtype, k / 2, ms, ld_a, 64, 64);
-    if (rc) return rc;
-    rc = make_map(&map_b, b, dtype, k, n, ld_b, 64, 128);
-    if (rc) return rc;
-
     SpmmParams P{};
     P.e_tc = e_tc; P.out = out; P.bias = nullptr; P.ms = ms; P.n = n; P.k = k; P.ld_out = ld_out;
     P.k_atoms = (k + 127) / 128; P.status = status; P.activation = 0; P.trace = nullptr;
@@ -2486,6 +2492,14 @@ static int spmm_accumulate_impl(const void *a_packed, int dtype, int a_mn_major,
             k_splits = (int)slices;
         }
     }
+    CUtensorMap map_a, map_b;
+    int rc;
+    if (!a_mn_major) rc = make_map(&map_a, a_packed, dtype, ms, k / 2, ld_a, 64, 128);
+    else rc = pair_form ? make_map_columns(&map_a, a_packed, dtype, k / 2, ms, ld_a, 64) : make_map(&map_a, a_packed, dtype, k / 2, ms, ld_a, 64, 64);
+    if (rc) return rc;
+    P.whole_columns = pair_form && n % 64 == 0;
+    rc = P.whole_columns ? make_map_columns(&map_b, b, dtype, k, n, ld_b, 128) : make_map(&map_b, b, dtype, k, n, ld_b, 64, 128);
+    if (rc) return rc;
     if (pair_form) {
         CUtensorMap map_e;
         rc = make_map_e(&map_e, e_tc, (ms / 128) * P.k_atoms);
