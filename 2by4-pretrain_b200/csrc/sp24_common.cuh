@@ -429,13 +429,16 @@ int clear_words(void *dst, int64_t words, cudaStream_t st);      // zeros at dst
 // Programmatic dependent launch.  A kernel launched by launch_chained may start while the kernel before it on the
 // stream is still finishing (as soon as all blocks of that one have called chain_enter or left), so its launch latency and set-up are
 // hidden behind the other's last wave.  chain_enter first waits until everything before on the stream is complete and visible: no kernel
-// touches global memory before it, and every thread calls it, so a kernel's completion implies that of all kernels before it.  Its memory
+// reads or writes global memory before it, and every thread calls it, so a kernel's completion implies that of all kernels before it.  Its memory
 // clobber holds plain loads back.  It does not bind loads that promise read-only data (__ldg, ld.global.nc, __restrict__): the kernel
 // before may still be writing during this one's life, so there are none.
 __device__ __forceinline__ void chain_enter() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
+// Asks L2 for the line of an address.  No value is read: the one access that may come before chain_enter, since what the kernel before still
+// writes arrives in L2 as well.
+__device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 // Errors are left for launch_status, as with a <<<>>> launch.
 template <typename... P, typename... A>
 inline void launch_chained(cudaStream_t st, void (*kern)(P...), dim3 grid, unsigned threads, size_t smem, A &&...args) {
