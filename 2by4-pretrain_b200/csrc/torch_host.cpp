@@ -765,7 +765,19 @@ Tensor quantizable(const Tensor &t) {
     return aligned(c) ? c : c.clone();
 }
 
-struct Q8 { Tensor packed, meta, tc; };
+struct Q8 {
+    Tensor packed, meta, tc;
+    // room for the compressed (m, k) matrix, `extra` bytes behind the result
+    Tensor make(int64_t m, int64_t k, int64_t extra, const Tensor &like) {
+        const int64_t vb = m * k / 2, mb = m * k / 8, tb = m % 128 == 0 ? sp24_meta_tc_bytes(m, k) : 0;
+        const int64_t end = align256(align256(vb) + align256(mb) + tb);
+        const Tensor buf = empty({end + extra}, at::kByte, like);
+        packed = carve(buf, 0, at::kFloat8_e4m3fn, {m, k / 2}, {k / 2, 1});
+        meta = carve(buf, align256(vb), at::kInt, {m, k / 32}, {k / 32, 1});
+        if (tb) tc = carve(buf, align256(vb) + align256(mb), at::kByte, {tb}, {1});
+        return carve(buf, end, at::kByte, {extra}, {1});
+    }
+};
 // e4m3 2:4 compression of the logical (m, k) matrix `dense` under the scale of *amax, packed values row-major.
 Q8 compress_q8(const Tensor &dense_in, int mode, const OptTensor &mask_in, const Tensor &amax, uint64_t seed, const Tensor &row_sums,
                const Tensor &q_dense, const Tensor &clear = {}) {
@@ -783,21 +795,16 @@ Q8 compress_q8(const Tensor &dense_in, int mode, const OptTensor &mask_in, const
         mask = as_layout(*mask, l.col);
         ld_m = layout_of(*mask).ld;
     }
-    const int64_t vb = m * k / 2, mb = m * k / 8, tb = m % 128 == 0 ? sp24_meta_tc_bytes(m, k) : 0;
-    const int64_t o_parts = align256(align256(vb) + align256(mb) + tb);
-    Tensor buf = empty({o_parts + (row_sums.defined() ? row_parts_bytes(m, k, at::kFloat8_e4m3fn) : 0)}, at::kByte, dense);
     Q8 o;
-    o.packed = carve(buf, 0, at::kFloat8_e4m3fn, {m, k / 2}, {k / 2, 1});
-    o.meta = carve(buf, align256(vb), at::kInt, {m, k / 32}, {k / 32, 1});
-    if (tb) o.tc = carve(buf, align256(vb) + align256(mb), at::kByte, {tb}, {1});
+    const Tensor parts = o.make(m, k, row_sums.defined() ? row_parts_bytes(m, k, at::kFloat8_e4m3fn) : 0, dense);
     sp24_prune_extras x{};
     x.amax = static_cast<const float *>(ptr(amax));
     x.offset_dev = rng_offset_ptr(mode);
     x.packed_row_major = 1;
-    if (tb) x.e_tc = ptr(o.tc);
+    if (o.tc.defined()) x.e_tc = ptr(o.tc);
     RowSums sums;
     if (row_sums.defined()) {
-        sums = {static_cast<float *>(ptr(row_sums)), reinterpret_cast<float *>(static_cast<char *>(ptr(buf)) + o_parts), false};
+        sums = {static_cast<float *>(ptr(row_sums)), static_cast<float *>(ptr(parts)), false};
         x.row_parts = sums.parts;
     }
     if (q_dense.defined()) {
@@ -830,8 +837,20 @@ py::tuple fp8_weight(const Tensor &w, const Tensor &mask_in) {
         const bool direct = w.scalar_type() == at::kFloat && w.is_contiguous() && mask.is_contiguous() && w.sizes() == mask.sizes() &&
                             w.numel() % 4 == 0 && aligned(w) && aligned(mask);
         amax = direct ? absmax(w, mask) : absmax(quantizable(at::where(mask, w, at::zeros({}, w.options()))));
-        a = compress_q8(w, SP24_PRUNE_MASK, mask, amax, 0, {}, {});
-        b = compress_q8(w.t(), SP24_PRUNE_MASK, mask.t(), amax, 0, {}, {});
+        const int64_t m = w.size(0), k = w.size(1);
+        const Layout l = layout_of(w);
+        // one read for both where W is row-major in whole 128 x 128 blocks
+        if (l.col == 0 && usable(w, l) && (w.scalar_type() == at::kFloat || is16(w.scalar_type())) && mask.is_contiguous() && aligned(mask, 4) &&
+            mask.sizes() == w.sizes() && m % 128 == 0 && k % 128 == 0 && m <= 64 * 65535 && m && k) {
+            a.make(m, k, 0, w);
+            b.make(k, m, 0, w);
+            check(sp24_dual_compress_f8(ptr(w), dt(w.scalar_type()), m, k, l.ld, ptr(mask), k, static_cast<const float *>(ptr(amax)), ptr(a.packed),
+                                        ptr(a.meta), ptr(a.tc), ptr(b.packed), ptr(b.meta), ptr(b.tc), cur_stream()),
+                  "sp24_dual_compress_f8");
+        } else {
+            a = compress_q8(w, SP24_PRUNE_MASK, mask, amax, 0, {}, {});
+            b = compress_q8(w.t(), SP24_PRUNE_MASK, mask.t(), amax, 0, {}, {});
+        }
     }
     auto opt = [](const Tensor &t) { return t.defined() ? py::cast(t) : py::object(py::none()); };
     return py::make_tuple(amax, a.packed, a.meta, opt(a.tc), b.packed, b.meta, opt(b.tc));

@@ -49,6 +49,7 @@ _SIGNATURES = {
     "sp24_quantize_f8": [_vp, _i32, _i64, _i64, _i64, _vp, _vp, _vp, _i64, _vp],
     "sp24_prune_compress_q8_dev": [_vp, _i32, _i64, _i64, _i64, _i32, _vp, _i32, _i64, _vp, _i32, _vp, _i64, _vp, _u64, _u64, _vp, _vp,
                                    _vp, _i64, _vp],
+    "sp24_dual_compress_f8": [_vp, _i32, _i64, _i64, _i64, _vp, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp],
     "sp24_pair_tile_columns": [_i64, _i64, _i32, _i32],
     "sp24_k_slices": [_i64, _i64, _i64, _i32],
     "sp24_row_parts": [_i64, _i32],

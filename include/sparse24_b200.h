@@ -162,6 +162,14 @@ int sp24_prune_compress_q8_dev(const void *dense, int dense_dtype, int64_t m, in
                                int packed_dtype, int64_t ld_packed, void *meta, int mode, const void *mask, int64_t ld_mask,
                                const float *amax, uint64_t seed, uint64_t offset, void *e_tc, float *row_sums, void *q_dense,
                                int64_t ld_q, void *stream);
+/*
+ * Both compressed copies of a float8 layer's weight from one read: what sp24_prune_compress_q8_dev writes for W (row-major, mask mode)
+ * and for its transposed view W.T under the same mask, with e_tc.  W (m, k) row-major F32, F16 or BF16, mask bytes; m and k multiples
+ * of 128, m at most 64 * 65535.  packed_w (m, k/2), packed_t (k, m/2) e4m3, contiguous; meta_w (m, k/32), meta_t (k, m/32) int32;
+ * tc_w, tc_t: sp24_meta_tc_bytes(m, k) and (k, m) bytes.
+ */
+int sp24_dual_compress_f8(const void *w, int dtype, int64_t m, int64_t k, int64_t ld_w, const void *mask, int64_t ld_mask, const float *amax,
+                          void *packed_w, void *meta_w, void *tc_w, void *packed_t, void *meta_t, void *tc_t, void *stream);
 
 /*
  * sp24_prune_compress with all extras, each of which may be NULL; offset_dev, e_tc, amax and q_dense as in the two entry points
