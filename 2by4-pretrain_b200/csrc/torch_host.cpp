@@ -767,6 +767,7 @@ Tensor quantizable(const Tensor &t) {
 
 struct Q8 {
     Tensor packed, meta, tc;
+    RowSums sums;
     // room for the compressed (m, k) matrix, `extra` bytes behind the result
     Tensor make(int64_t m, int64_t k, int64_t extra, const Tensor &like) {
         const int64_t vb = m * k / 2, mb = m * k / 8, tb = m % 128 == 0 ? sp24_meta_tc_bytes(m, k) : 0;
@@ -779,6 +780,7 @@ struct Q8 {
     }
 };
 // e4m3 2:4 compression of the logical (m, k) matrix `dense` under the scale of *amax, packed values row-major.
+// row_sums: o.sums says how the next launch gets them; its parts live as long as o.packed.
 Q8 compress_q8(const Tensor &dense_in, int mode, const OptTensor &mask_in, const Tensor &amax, uint64_t seed, const Tensor &row_sums,
                const Tensor &q_dense, const Tensor &clear = {}) {
     const int64_t m = dense_in.size(0), k = dense_in.size(1);
@@ -802,10 +804,9 @@ Q8 compress_q8(const Tensor &dense_in, int mode, const OptTensor &mask_in, const
     x.offset_dev = rng_offset_ptr(mode);
     x.packed_row_major = 1;
     if (o.tc.defined()) x.e_tc = ptr(o.tc);
-    RowSums sums;
     if (row_sums.defined()) {
-        sums = {static_cast<float *>(ptr(row_sums)), static_cast<float *>(ptr(parts)), false};
-        x.row_parts = sums.parts;
+        o.sums = {static_cast<float *>(ptr(row_sums)), static_cast<float *>(ptr(parts)), false};
+        x.row_parts = o.sums.parts;
     }
     if (q_dense.defined()) {
         x.q_dense = ptr(q_dense);
@@ -821,7 +822,6 @@ Q8 compress_q8(const Tensor &dense_in, int mode, const OptTensor &mask_in, const
                                        mode, ptr(mask), ld_m, nullptr, 0, seed, 0, &x, cur_stream()),
               "sp24_prune_compress_q8");
     }
-    if (sums.out) sum_parts(sums, m, k, at::kFloat8_e4m3fn);
     return o;
 }
 
@@ -911,9 +911,16 @@ struct Fp8Backward : torch::autograd::Node {
             Tensor gw = empty({of, in_f}, at::kFloat, g), gb = need_b ? empty({of}, at::kFloat, g) : Tensor();
             const Q8 c = compress_q8(g.t(), SP24_PRUNE_MVUE_FAST, {}, amax, seed, gb, gq, gw);
             TORCH_CHECK(c.tc.defined(), "sparse GEMM on sm_100a: number of rows of the sparse matrix must be divisible by 128");
-            check(sp24_spmm_f8(ptr(c.packed), SP24_E4M3, n / 2, ptr(c.tc), of, n, ptr(xq_t), n, in_f, ptr(gw), SP24_F32, 0, in_f, nullptr,
-                               static_cast<const float *>(ptr(amax)), static_cast<const float *>(ptr(amax_x_)), status_ptr(g), cur_stream()),
-                  "sp24_spmm_f8");
+            const float *scale_g = static_cast<const float *>(ptr(amax)), *scale_x = static_cast<const float *>(ptr(amax_x_));
+            if (c.sums.out)
+                check(sp24_spmm_f8_sums(ptr(c.packed), SP24_E4M3, n / 2, ptr(c.tc), of, n, ptr(xq_t), n, in_f, static_cast<float *>(ptr(gw)), in_f,
+                                        scale_g, scale_x, c.sums.parts, sp24_row_parts(n, SP24_E4M3), c.sums.out, c.sums.add, status_ptr(g),
+                                        cur_stream()),
+                      "sp24_spmm_f8_sums");
+            else
+                check(sp24_spmm_f8(ptr(c.packed), SP24_E4M3, n / 2, ptr(c.tc), of, n, ptr(xq_t), n, in_f, ptr(gw), SP24_F32, 0, in_f, nullptr, scale_g,
+                                   scale_x, status_ptr(g), cur_stream()),
+                      "sp24_spmm_f8");
             out[1] = gw;
             if (need_b) out[2] = gb;
             need_b = false;

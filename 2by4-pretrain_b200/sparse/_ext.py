@@ -61,6 +61,7 @@ _SIGNATURES = {
                                       _vp],
     "sp24_sum_parts": [_vp, _i64, _i64, _vp, _i32, _vp],
     "sp24_spmm_f8": [_vp, _i32, _i64, _vp, _i64, _i64, _vp, _i64, _i64, _vp, _i32, _i32, _i64, _vp, _vp, _vp, _vp, _vp],
+    "sp24_spmm_f8_sums": [_vp, _i32, _i64, _vp, _i64, _i64, _vp, _i64, _i64, _vp, _i64, _vp, _vp, _vp, _i64, _vp, _i32, _vp, _vp],
     "sp24_soft_threshold24_compress": [_vp, _i32, _i64, _i64, _i64, _i32, _vp, _i32, _i64, _vp, _i32, _f32, _vp, _vp],
     "sp24_layernorm_fwd": [_vp, _vp, _vp, _vp, _i32, _vp, _vp, _i64, _i64, _f32, _vp],
     "sp24_layernorm_bwd": [_vp, _i32, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _vp],

@@ -451,6 +451,11 @@ int sp24_spmm_f8(const void *a_packed, int dtype, int64_t ld_a, const void *e_tc
                  int64_t n, void *out, int out_dtype, int trans_out, int64_t ld_out, const float *bias, const float *amax_a,
                  const float *amax_b, int *status, void *stream);
 
+/* trans_out = 0, and row_sums as sp24_spmm_accumulate_sums_f32 takes them along. */
+int sp24_spmm_f8_sums(const void *a_packed, int dtype, int64_t ld_a, const void *e_tc, int64_t ms, int64_t k, const void *b, int64_t ld_b,
+                      int64_t n, float *out, int64_t ld_out, const float *amax_a, const float *amax_b, const float *row_parts, int64_t n_parts,
+                      float *row_sums, int sums_accumulate, int *status, void *stream);
+
 /*
  * Weight-gradient form of the sparse GEMM with fp32 accumulation into the output:
  *   D (ms x n, fp32, row-major, pitch ld_out) += A_sparse (ms x k) * B (k x n, stored row-major, pitch ld_b).
