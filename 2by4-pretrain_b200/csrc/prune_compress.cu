@@ -467,9 +467,8 @@ template <typename TIn> struct ColVec {
     // Exact MVUE is bound by instruction issue, not by load width: one row per thread makes blocks of 32 rows, which
     // balances the SMs better on short matrices and is never slower on long ones.
     static constexpr int narrow = 1;
-    // Fast MVUE with 8-bit results: two rows, two groups at a time, three blocks per SM, where one group at a time took four rows at two
-    // blocks: the quantised bytes are gathered by one permute a group.  bf16 -> e4m3 with row sums and the quantised tensor, us:
-    // 3072 x 8192 49.2 -> 41.0, 768 x 8192 17.3 -> 12.1, 1024 x 1024 10.6 -> 6.4.
+    // Fast MVUE with 8-bit results of float32 input, or stored in columns: two rows, two groups at a time, three blocks per SM, where one
+    // group at a time took four rows at two blocks: the quantised bytes are gathered by one permute a group.
     static constexpr int fast8 = 2;
 };
 
@@ -674,11 +673,17 @@ __global__ void __launch_bounds__(256, col_min_blocks(MODE)) pc_col_kernel(PcPar
         // the eight warps hold eight K ranges of the same rows: one reduction per row and block
         for (int t = threadIdx.x; t < RT; t += 256) {
             if (r0 + t < P.m) {
-                float a = 0.f;
+                // parts are of 128 storage rows: the block's eight words of 16 bits are one, of 32 bits two
+                constexpr int HALVES = MB == 4 ? 2 : 1;
 #pragma unroll
-                for (int w = 0; w < 8; ++w) a += ssum[w][t];
-                if (P.ld_sums) P.row_sums[blockIdx.y * P.ld_sums + r0 + t] = a;
-                else atomicAdd(P.row_sums + r0 + t, a);
+                for (int h = 0; h < HALVES; ++h) {
+                    float a = 0.f;
+#pragma unroll
+                    for (int w = 0; w < 8 / HALVES; ++w) a += ssum[h * 4 + w][t];
+                    const int64_t part = (int64_t)blockIdx.y * HALVES + h;
+                    if (!P.ld_sums) atomicAdd(P.row_sums + r0 + t, a);
+                    else if (part < P.k_atoms) P.row_sums[part * P.ld_sums + r0 + t] = a;
+                }
             }
         }
     }
@@ -719,7 +724,8 @@ __global__ void __launch_bounds__(256, col_min_blocks(MODE)) pc_col_kernel(PcPar
 }
 
 // ---------------------------------------------------------------------------------------------
-// Fast MVUE, column-major storage, 16-bit results: dY^T, the sparse operand of every weight-gradient GEMM.
+// Fast MVUE, column-major storage, 16-bit results, or row-major float8 ones of 16-bit input: dY^T, the sparse operand of every
+// weight-gradient GEMM.
 // ---------------------------------------------------------------------------------------------
 // Bound by arithmetic: about 80 instructions a group of four for the draws, quotients and random numbers, which by themselves (operands
 // in shared memory, no traffic) take 115 cycles a warp and group, 67 % of the time measured here; the rest are copies, addresses and
@@ -730,13 +736,19 @@ __global__ void __launch_bounds__(256, col_min_blocks(MODE)) pc_col_kernel(PcPar
 // instructions a group instead of 98.  us a replayed launch, one group at a time in a block per tile -> here: bf16 4096 x 8192 45.0 -> 38.0,
 // fp16 3072 x 16384 63.9 -> 55.9, bf16 with row sums 3072 x 8192 37.0 -> 29.2, 768 x 8192 11.2 -> 9.4, fp16 512 x 256 5.1 -> 3.1, float32
 // 4096 x 8192 42.7 -> 42.4, 512 x 256 5.0 -> 3.3.
+// Float8 results with the quantised tensor and row sums (stored rows staged for one 16-byte store a thread, quantised rows for two a
+// lane), blocks of their own tile each -> here: bf16 3072 x 8192 40.8 -> 34.8, 768 x 8192 12.3 -> 11.7, 1024 x 4096 9.8 -> 8.8, 1024 x 1024
+// 6.6 -> 4.2.  Float32 input keeps the other kernel for them (its operands and the quantised ones do not fit the registers).
 // Three or four stages of copies instead of two, and tiles of two or four 16-column slices a warp, gained nothing.
-template <typename TIn> struct MvueCol {
+template <typename TIn, typename TOut> struct MvueCol {
+    static constexpr bool F8 = sizeof(TOut) == 1;
     static constexpr int RT = 64;                                // rows of a tile; each of its eight warps takes 16 logical columns
     static constexpr int ROW = RT * sizeof(TIn);                 // bytes of one storage row of a tile
     static constexpr int SLICE = 16 * ROW, STAGES = 2;           // a warp's share, and how many of them are under way
-    static constexpr int RUN = 0, LINE = 4 * 2 * RT * 2, SUMS = LINE + RT * 16, OUT = SUMS + 8 * RT * 4;     // staged results
-    static constexpr int SMEM = STAGES * 8 * SLICE + 2 * OUT;
+    static constexpr int RUN = 0, LINE = 4 * 2 * RT * 2, SUMS = LINE + RT * 16, PACK = SUMS + 8 * RT * 4;     // staged results
+    static constexpr int OUT = PACK + (F8 ? RT * 64 : 0);
+    static constexpr int QUANT = STAGES * 8 * SLICE + 2 * OUT;   // float8: a warp's 16 storage rows quantised
+    static constexpr int SMEM = QUANT + (F8 ? 8 * 16 * RT : 0);
     static constexpr int BLOCKS = 2;
 };
 
@@ -753,11 +765,14 @@ template <typename T> __device__ __forceinline__ void pin(T &v) {
 __device__ __forceinline__ void st_shared16(uint32_t addr, uint32_t v) { asm volatile("st.shared.u16 [%0], %1;" ::"r"(addr), "h"((uint16_t)v) : "memory"); }
 
 template <typename TIn, typename TOut>
-__global__ void __launch_bounds__(256, MvueCol<TIn>::BLOCKS)
+__global__ void __launch_bounds__(256, MvueCol<TIn, TOut>::BLOCKS)
 mvue_col_kernel(const __grid_constant__ PcParams P, const __grid_constant__ PhiloxKeys<kMvueFastRounds> keys) {
     chain_enter();
-    using Cfg = MvueCol<TIn>;
+    using Cfg = MvueCol<TIn, TOut>;
+    constexpr bool F8 = Cfg::F8;
     constexpr int RT = Cfg::RT, ROW = Cfg::ROW, STAGES = Cfg::STAGES, V = 2;
+    static_assert(!F8 || sizeof(TIn) == 2, "float8 from 16-bit values only");
+    const float out_scale = out_scale_of<TOut>(P);
     // 16-bit input: a lane writes only over the four bytes of a row that it alone reads.  Float32 rows are twice as long: other lanes
     // read where it writes.
     constexpr bool OWN_BYTES = ROW == RT * sizeof(TOut) && V * sizeof(TIn) == 4;
@@ -801,11 +816,21 @@ mvue_col_kernel(const __grid_constant__ PcParams P, const __grid_constant__ Phil
     // where a lane's two words go in the staged metadata (the second 8 words behind the first in both orders), and its 16 bytes of the
     // stored rows
     const int rr = lane * V;
-    uint32_t run_at = (uint32_t)__cvta_generic_to_shared(smem + STAGES * 8 * Cfg::SLICE) + Cfg::RUN +
-                      2 * ((warp >> 1) * 2 * RT + (rr / 32) * 64 + meta_run_pos<2>(rr % 32, warp & 1));
-    uint32_t line_at = (uint32_t)__cvta_generic_to_shared(smem + STAGES * 8 * Cfg::SLICE) + Cfg::LINE +
-                       2 * (8 * (16 * (rr >> 4) + 8 * (warp & 1) + (rr & 7)) + 2 * (warp >> 1) + ((rr >> 3) & 1));
+    // (float8: half a 32-bit word each; the row after is 16 bytes further in either order and either type)
+    const uint32_t staged = (uint32_t)__cvta_generic_to_shared(smem + STAGES * 8 * Cfg::SLICE);
+    uint32_t run_at = staged + Cfg::RUN + (F8 ? 4 * ((warp >> 2) * 2 * RT + (rr / 16) * 32 + meta_run_pos<4>(rr % 16, (warp >> 1) & 1)) + 2 * (warp & 1)
+                                              : 2 * ((warp >> 1) * 2 * RT + (rr / 32) * 64 + meta_run_pos<2>(rr % 32, warp & 1)));
+    uint32_t line_at = staged + Cfg::LINE + (F8 ? rr * 16 + warp * 2
+                                                : 2 * (8 * (16 * (rr >> 4) + 8 * (warp & 1) + (rr & 7)) + 2 * (warp >> 1) + ((rr >> 3) & 1)));
     char *store_to = static_cast<char *>(P.packed) + (uint64_t)(lane >> 3) * ld_out + (lane & 7) * 16;
+    // float8: a row's 64 stored bytes of a tile are eight pieces of 8, one a warp; rows 2 l and 2 l + 1 share 128 bytes whose halves change
+    // places every eight l, the pieces exchanged by l % 8: no bank is met twice
+    auto pack_at = [](int row, int piece) {
+        const int l = row >> 1;
+        return Cfg::PACK + l * 128 + (((row & 1) ^ ((l >> 3) & 1)) << 6) + ((piece ^ (l & 7)) << 3);
+    };
+    uint32_t pack_to[2] = {staged + pack_at(rr, warp), staged + pack_at(rr + 1, warp)};
+    uint8_t *const quant = smem + Cfg::QUANT + warp * (16 * RT);
     pin(run_at);
     pin(line_at);
     pin(store_to);
@@ -829,11 +854,21 @@ mvue_col_kernel(const __grid_constant__ PcParams P, const __grid_constant__ Phil
             uint64_t pair[V];
             pair[0] = (uint64_t)(uint32_t)(r0 + lane * V) * row_pairs + (uint32_t)(c * 2);
             pair[1] = pair[0] + row_pairs;
+            uint32_t stored[F8 ? V : 1][2];
 #pragma unroll
             for (int step = 0; step < 2; ++step) {
                 Vec<TIn, V> in[8];
 #pragma unroll
                 for (int j = 0; j < 8; ++j) in[j] = load_vec<TIn, V>(reinterpret_cast<const TIn *>(sl + (8 * step + j) * ROW) + lane * V);
+                if constexpr (F8) {
+                    if (P.q_dense) {
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) {
+                            const float f[V] = {__fmul_rn(Elem<TIn>::to_f32(in[j].v[0]), out_scale), __fmul_rn(Elem<TIn>::to_f32(in[j].v[1]), out_scale)};
+                            store_f8<TOut, V>(reinterpret_cast<TOut *>(quant + (8 * step + j) * RT + lane * V), f);
+                        }
+                    }
+                }
                 uint32_t o[2][V];
 #pragma unroll
                 for (int v = 0; v < V; ++v) {
@@ -848,8 +883,10 @@ mvue_col_kernel(const __grid_constant__ PcParams P, const __grid_constant__ Phil
                         const float2 a = __fadd2_rn(__fadd2_rn(x[0], x[1]), __fadd2_rn(x[2], x[3]));
                         rsum[v] += a.x + a.y;
                     }
-                    word[v] += two_groups_fast<TOut>(x, v0, v1, picks_at, 1.f, o[0][v], o[1][v]) << (8 * step);
+                    word[v] += two_groups_fast<TOut>(x, v0, v1, picks_at, out_scale, o[0][v], o[1][v]) << (8 * step);
+                    if constexpr (F8) stored[v][step] = o[0][v] | (o[1][v] << 16);
                 }
+                if constexpr (F8) continue;
                 // stored rows (128 bytes) take the place of the first storage rows, which all lanes have read by now
                 if constexpr (!OWN_BYTES) __syncwarp(together);
 #pragma unroll
@@ -858,6 +895,11 @@ mvue_col_kernel(const __grid_constant__ PcParams P, const __grid_constant__ Phil
                     to[0] = __byte_perm(o[h][0], o[h][1], 0x5410u);
                     to[32] = __byte_perm(o[h][0], o[h][1], 0x7632u);
                 }
+            }
+            if constexpr (F8) {
+#pragma unroll
+                for (int v = 0; v < V; ++v)
+                    asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(pack_to[v] + out_off), "r"(stored[v][0]), "r"(stored[v][1]) : "memory");
             }
         }
         // word columns past the matrix (K not a multiple of 128) are zeros in the tensor-core copy: the GEMM multiplies them by
@@ -868,7 +910,13 @@ mvue_col_kernel(const __grid_constant__ PcParams P, const __grid_constant__ Phil
         st_shared16(line_at + out_off + 16, word[1]);
         if (P.row_sums) *reinterpret_cast<float2 *>(smem + STAGES * 8 * Cfg::SLICE + out_off + Cfg::SUMS + (warp * RT + rr) * 4) = make_float2(rsum[0], rsum[1]);
         __syncwarp();
-        if (r0 + (lane & 7) * 8 < m && c < ncols) {       // 8 rows of 128 bytes, 16 bytes a lane and store
+        if constexpr (F8) {
+            if (P.q_dense && r0 + (lane & 3) * 16 < m) {       // 16 rows of 64 bytes (float8: columns come in whole tiles)
+                char *dst = static_cast<char *>(P.q_dense) + (c * 16 + (lane >> 2)) * P.ld_q + r0 + (lane & 3) * 16;
+                *reinterpret_cast<uint4 *>(dst) = *reinterpret_cast<const uint4 *>(quant + lane * 16);
+                *reinterpret_cast<uint4 *>(dst + 8 * P.ld_q) = *reinterpret_cast<const uint4 *>(quant + 512 + lane * 16);
+            }
+        } else if (r0 + (lane & 7) * 8 < m && c < ncols) {       // 8 rows of 128 bytes, 16 bytes a lane and store
             char *dst = store_to + ((uint64_t)(uint32_t)(c * 8) * ld_out + (uint32_t)(r0 * 2));
             *reinterpret_cast<uint4 *>(dst) = *reinterpret_cast<const uint4 *>(sl + lane * 16);
             *reinterpret_cast<uint4 *>(dst + 4ull * ld_out) = *reinterpret_cast<const uint4 *>(sl + 512 + lane * 16);
@@ -881,7 +929,21 @@ mvue_col_kernel(const __grid_constant__ PcParams P, const __grid_constant__ Phil
         // tiles ahead
         const uint8_t *out = smem + STAGES * 8 * Cfg::SLICE + out_off;
         const int t = threadIdx.x & 63, rows_here = m - r0;
-        if (warp < 2) {
+        if constexpr (F8) {
+            const int row = threadIdx.x >> 2, piece = threadIdx.x & 3;       // 16 bytes a thread
+            if (row < rows_here) {
+                const uint2 lo = *reinterpret_cast<const uint2 *>(out + pack_at(row, 2 * piece)), hi = *reinterpret_cast<const uint2 *>(out + pack_at(row, 2 * piece + 1));
+                *reinterpret_cast<uint4 *>(static_cast<char *>(P.packed) + (int64_t)(r0 + row) * P.ld_packed + tc * 64 + piece * 16) =
+                    make_uint4(lo.x, lo.y, hi.x, hi.y);
+            }
+        }
+        if (F8 && warp < 2) {
+            // 2 column pairs x 2 RT words of 4 bytes
+            const int cp = tc * 2 + (t >> 5), pc = t & 31;
+            if (pc * 2 < rows_here)
+                *reinterpret_cast<uint4 *>(static_cast<char *>(P.meta) + ((uint64_t)(uint32_t)cp * (uint32_t)m + (uint32_t)r0) * 8 + pc * 16) =
+                    *reinterpret_cast<const uint4 *>(out + Cfg::RUN + t * 16);
+        } else if (warp < 2) {
             // 4 column pairs x 2 RT words
             const int cp = tc * 4 + (t >> 4), pc = t & 15;
             if (pc * 4 < rows_here && cp * 2 < ncols)
@@ -1019,6 +1081,15 @@ template <auto KERN> int allow_shared_memory(int bytes) {
     return SP24_OK;
 }
 
+template <typename TIn, typename TOut> int launch_mvue_col(const PcParams &P, cudaStream_t st) {
+    using Cfg = MvueCol<TIn, TOut>;
+    constexpr auto kern = mvue_col_kernel<TIn, TOut>;
+    if (int rc = allow_shared_memory<mvue_col_kernel<TIn, TOut>>(Cfg::SMEM)) return rc;
+    const int64_t tiles = ((P.m + Cfg::RT - 1) / Cfg::RT) * ((P.k / 16 + 7) / 8), most = (int64_t)sm_count() * Cfg::BLOCKS;
+    launch_chained(st, kern, (unsigned)(tiles < most ? tiles : most), 256, Cfg::SMEM, P, PhiloxKeys<kMvueFastRounds>(P.seed));
+    return launch_status();
+}
+
 template <typename TIn, typename TOut, int MODE, bool HAS_U>
 int launch(const PcParams &P, int col_major, cudaStream_t st) {
     constexpr int CH = sizeof(TOut) == 2 ? 16 : 32;
@@ -1027,12 +1098,10 @@ int launch(const PcParams &P, int col_major, cudaStream_t st) {
         if constexpr (is_mvue(MODE)) launch_balanced(st, pc_row_kernel<TIn, TOut, MODE, HAS_U>, grid, 256, 0, P);
         else launch_chained(st, pc_row_kernel<TIn, TOut, MODE, HAS_U>, grid, 256, 0, P);
     } else if constexpr (MODE == SP24_PRUNE_MVUE_FAST && sizeof(TOut) == 2) {
-        using Cfg = MvueCol<TIn>;
-        constexpr auto kern = mvue_col_kernel<TIn, TOut>;
-        if (int rc = allow_shared_memory<mvue_col_kernel<TIn, TOut>>(Cfg::SMEM)) return rc;
-        const int64_t tiles = ((P.m + Cfg::RT - 1) / Cfg::RT) * ((P.k / 16 + 7) / 8), most = (int64_t)sm_count() * Cfg::BLOCKS;
-        launch_chained(st, kern, (unsigned)(tiles < most ? tiles : most), 256, Cfg::SMEM, P, PhiloxKeys<kMvueFastRounds>(P.seed));
+        return launch_mvue_col<TIn, TOut>(P, st);
     } else {
+        if constexpr (MODE == SP24_PRUNE_MVUE_FAST && sizeof(TIn) == 2)
+            if (P.packed_rm) return launch_mvue_col<TIn, TOut>(P, st);
         constexpr int V = MODE == SP24_PRUNE_MVUE_FAST ? ColVec<TIn>::fast8
                                                        : (MODE == SP24_PRUNE_MVUE ? ColVec<TIn>::narrow : ColVec<TIn>::wide);
         constexpr int RT = 32 * V;
@@ -1185,11 +1254,10 @@ extern "C" int sp24_prune_compress_q8_dev(const void *dense, int dense_dtype, in
                                q_dense, ld_q);
 }
 
-// Storage rows of a column-major matrix that one block of the converting kernel covers: eight metadata words.
+// One part for every 128 storage rows of a column-major matrix.
 extern "C" int sp24_row_parts(int64_t k, int packed_dtype) {
     const int so = sp24::dtype_size(packed_dtype);
-    const int64_t per = so == 1 ? 256 : 128;
-    return so != 1 && so != 2 ? 0 : (int)((k + per - 1) / per);
+    return so != 1 && so != 2 ? 0 : (int)((k + 127) / 128);
 }
 
 static int prune_compress_with(const void *dense, int dense_dtype, int64_t m, int64_t k, int64_t ld_dense, int col_major, void *packed,

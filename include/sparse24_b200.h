@@ -175,7 +175,7 @@ int sp24_dual_compress_f8(const void *w, int dtype, int64_t m, int64_t k, int64_
  * sp24_prune_compress with all extras, each of which may be NULL; offset_dev, e_tc, amax and q_dense as in the two entry points
  * above.  packed_row_major: float8 results of column-major input leave row-major, as sp24_prune_compress_q8 writes them (q_dense
  * asks for it).  out_scale: float8 without amax, as for sp24_prune_compress_q8 (0: none).  row_parts instead of row_sums:
- * float32 (sp24_row_parts(k, packed_dtype), m), partial sums over 128 (float8: 256) consecutive k of the unpruned
+ * float32 (sp24_row_parts(k, packed_dtype), m), partial sums over 128 consecutive k of the unpruned
  * dense[r, k], column-major storage only.  sp24_sum_parts adds them up in a fixed order (accumulate = 1: to what out holds),
  * so that the same gradient gives the same bits every time, which row_sums' atomics do not promise.
  */
