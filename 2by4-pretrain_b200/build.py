@@ -59,7 +59,7 @@ def _build_host(force, headers):
            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
     cmd += ["-isystem" + p for p in cpp_extension.include_paths() + ["/usr/local/cuda/include", sysconfig.get_paths()["include"]]]
     obj_args = [HOST_SRC, "-o", HOST_LIB, "-L" + LIBDIR, "-l:libsparse24_b200.so", "-Wl,-rpath,$ORIGIN", "-L" + cpp_extension.TORCH_LIB_PATH,
-                "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+                "-ltorch_python", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda"]
     tag = _digest([HOST_SRC] + headers, " ".join(cmd) + torch.__version__)
     stamp = os.path.join(OBJDIR, "host.stamp")
     if not force and os.path.exists(HOST_LIB) and os.path.exists(stamp) and open(stamp).read() == tag:

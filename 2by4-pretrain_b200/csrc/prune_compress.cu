@@ -738,7 +738,7 @@ __global__ void __launch_bounds__(256, col_min_blocks(MODE)) pc_col_kernel(PcPar
 // 4096 x 8192 42.7 -> 42.4, 512 x 256 5.0 -> 3.3.
 // Float8 results with the quantised tensor and row sums (stored rows staged for one 16-byte store a thread, quantised rows for two a
 // lane), blocks of their own tile each -> here: bf16 3072 x 8192 40.8 -> 34.8, 768 x 8192 12.3 -> 11.7, 1024 x 4096 9.8 -> 8.8, 1024 x 1024
-// 6.6 -> 4.2.  Float32 input keeps the other kernel for them (its operands and the quantised ones do not fit the registers).
+// 6.6 -> 4.2.  Float8 results of float32 input stay with the other kernel.
 // Three or four stages of copies instead of two, and tiles of two or four 16-column slices a warp, gained nothing.
 template <typename TIn, typename TOut> struct MvueCol {
     static constexpr bool F8 = sizeof(TOut) == 1;

@@ -4,10 +4,15 @@
 // A layer step launches half a dozen kernels that take 5 - 60 us each; driven from Python (argument marshalling of 20
 // words per launch, tensor views, autograd.Function objects in both directions) its host time was 300 us and bounded
 // every step below a few thousand tokens.  Nothing here computes: without the kernel library the module does not load.
+#include <ATen/autocast_mode.h>
+#include <ATen/cuda/EmptyTensor.h>
 #include <ATen/ops/mm.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/saved_variable.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 #include <torch/extension.h>
 
 #include "../../include/sparse24_b200.h"
@@ -55,7 +60,17 @@ void *ptr(const Tensor &t) { return t.data_ptr(); }
 const void *ptr(const OptTensor &t) { return t.has_value() ? t->data_ptr() : nullptr; }
 bool aligned(const Tensor &t, uintptr_t a = 16) { return reinterpret_cast<uintptr_t>(t.data_ptr()) % a == 0; }
 
-Tensor empty(c10::IntArrayRef shape, at::ScalarType t, const Tensor &like) { return at::empty(shape, like.options().dtype(t)); }
+// Whether somebody wants to see or change what is allocated: a trace, a dispatch mode, a functorch level, memory filled for determinism.
+bool allocations_watched() {
+    return torch::jit::tracer::isTracing() || c10::impl::TorchDispatchModeTLS::any_modes_set() ||
+           c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode) ||
+           (at::globalContext().deterministicAlgorithms() && at::globalContext().deterministicFillUninitializedMemory());
+}
+// Otherwise straight from the allocator: through the dispatcher an allocation took 0.2 us more, and a layer step makes eight.
+Tensor empty(c10::IntArrayRef shape, at::ScalarType t, const Tensor &like) {
+    if (!like.is_cuda() || allocations_watched()) return at::empty(shape, like.options().dtype(t));
+    return at::detail::empty_cuda(shape, t, like.device(), c10::nullopt);
+}
 
 // storage order and leading dimension of a 2-D tensor with one unit stride; order -1: neither
 struct Layout { int col; int64_t ld; };
@@ -397,38 +412,43 @@ py::tuple as_tuple(const Tensor &mask, const Copies &c) {
     return py::make_tuple(mask, c.pw, c.mw, c.pt, c.mt, opt(c.tcw), opt(c.tct));
 }
 
+// Both copies of one weight, without the GIL; the mask that they follow goes to `mask`.
+Copies select_copies(const Tensor &weight, const OptTensor &mask_in, at::ScalarType t, const OptTensor &mask_out, Tensor &mask) {
+    NoAutograd guard;
+    require_cuda(weight, mask_in, mask_out);
+    TORCH_CHECK(weight.dim() == 2, "select_and_compress: expected a 2-D weight");
+    const int64_t m = weight.size(0), k = weight.size(1);
+    const Tensor w = as_layout(weight, 0);
+    const bool select = !mask_in.has_value();
+    if (!select) {
+        mask = *mask_in;
+        if (mask.scalar_type() != at::kBool && mask.scalar_type() != at::kByte) mask = mask.ne(0);
+        mask = as_layout(mask, 0);
+    } else if (mask_out.has_value()) {
+        mask = *mask_out;
+        TORCH_CHECK(mask.scalar_type() == at::kBool && mask.dim() == 2 && mask.size(0) == m && mask.size(1) == k && mask.is_contiguous(),
+                    "select_and_compress: mask_out must be a contiguous bool tensor of the weight's shape");
+    } else {
+        mask = empty({m, k}, at::kBool, w);
+    }
+    Copies c(m, k, t, w);
+    const int64_t ldw = layout_of(w).ld, ldm = layout_of(mask).ld;
+    if (c.tcw.defined())
+        check(sp24_select_dual_compress_tc(ptr(w), dt(w.scalar_type()), m, k, ldw, select, ptr(mask), ldm, ptr(c.pw), dt(t), k / 2, ptr(c.mw),
+                                           ptr(c.pt), k, ptr(c.mt), ptr(c.tcw), ptr(c.tct), cur_stream()),
+              "sp24_select_dual_compress_tc");
+    else
+        check(sp24_select_dual_compress(ptr(w), dt(w.scalar_type()), m, k, ldw, select, ptr(mask), ldm, ptr(c.pw), dt(t), k / 2, ptr(c.mw),
+                                        ptr(c.pt), k, ptr(c.mt), cur_stream()),
+              "sp24_select_dual_compress");
+    return c;
+}
 py::tuple select_compress(const Tensor &weight, const OptTensor &mask_in, at::ScalarType t, const OptTensor &mask_out) {
     Tensor mask;
     c10::optional<Copies> c;
     {
         py::gil_scoped_release nogil;
-        NoAutograd guard;
-        require_cuda(weight, mask_in, mask_out);
-        TORCH_CHECK(weight.dim() == 2, "select_and_compress: expected a 2-D weight");
-        const int64_t m = weight.size(0), k = weight.size(1);
-        const Tensor w = as_layout(weight, 0);
-        const bool select = !mask_in.has_value();
-        if (!select) {
-            mask = *mask_in;
-            if (mask.scalar_type() != at::kBool && mask.scalar_type() != at::kByte) mask = mask.ne(0);
-            mask = as_layout(mask, 0);
-        } else if (mask_out.has_value()) {
-            mask = *mask_out;
-            TORCH_CHECK(mask.scalar_type() == at::kBool && mask.dim() == 2 && mask.size(0) == m && mask.size(1) == k && mask.is_contiguous(),
-                        "select_and_compress: mask_out must be a contiguous bool tensor of the weight's shape");
-        } else {
-            mask = empty({m, k}, at::kBool, w);
-        }
-        c.emplace(m, k, t, w);
-        const int64_t ldw = layout_of(w).ld, ldm = layout_of(mask).ld;
-        if (c->tcw.defined())
-            check(sp24_select_dual_compress_tc(ptr(w), dt(w.scalar_type()), m, k, ldw, select, ptr(mask), ldm, ptr(c->pw), dt(t), k / 2,
-                                               ptr(c->mw), ptr(c->pt), k, ptr(c->mt), ptr(c->tcw), ptr(c->tct), cur_stream()),
-                  "sp24_select_dual_compress_tc");
-        else
-            check(sp24_select_dual_compress(ptr(w), dt(w.scalar_type()), m, k, ldw, select, ptr(mask), ldm, ptr(c->pw), dt(t), k / 2,
-                                            ptr(c->mw), ptr(c->pt), k, ptr(c->mt), cur_stream()),
-                  "sp24_select_dual_compress");
+        c.emplace(select_copies(weight, mask_in, t, mask_out, mask));
     }
     return as_tuple(mask, *c);
 }
@@ -481,77 +501,141 @@ std::vector<py::tuple> select_compress_many(const std::vector<Tensor> &weights, 
 // What sparse_ops.refresh_sparse_layers does for layers of the plain class: reads each weight's state, launches once per group and
 // installs the copies.  In Python these 20 attribute accesses a layer were more host time than 48 layers' kernel on the GPU (109 us).
 // Returns the number of layers refreshed and those it leaves to the caller: any whose class, weight, mask or counters are not plain.
-struct RefreshNames {
-    PyObject *weight, *parameters, *mode, *cnt, *mask, *counter, *freq, *compressed, *compressed_tc, *weight_sparse, *weight_sparse_T, *refreshed, *take,
-        *materialize;
+struct LayerNames {
+    PyObject *weight, *bias, *parameters, *training, *mode, *cnt, *mask, *counter, *freq, *step, *compressed, *compressed_tc, *weight_sparse, *weight_sparse_T,
+        *refreshed, *take, *refresh, *ensure, *tc_copies, *advance, *materialize, *into_grad, *parameter_type;
 };
-const RefreshNames &refresh_names() {       // made by the module's load, see PyObjects
-    static const RefreshNames n = [] {
+const LayerNames &layer_names() {       // made by the module's load, see PyObjects
+    static const LayerNames n = [] {
         auto s = [](const char *t) { return PyUnicode_InternFromString(t); };
-        return RefreshNames{s("weight"), s("_parameters"), s("mode"), s("cnt"), s("mask"), s("counter"), s("freq"), s("compressed"), s("compressed_tc"),
-                            s("weight_sparse"), s("weight_sparse_T"), s("refreshed"), s("_take"), s("materialize_sparse_tensors")};
+        return LayerNames{s("weight"), s("bias"), s("_parameters"), s("training"), s("mode"), s("cnt"), s("mask"), s("counter"), s("freq"), s("step"),
+                          s("compressed"), s("compressed_tc"), s("weight_sparse"), s("weight_sparse_T"), s("refreshed"), s("_take"), s("_refresh"),
+                          s("_ensure_compressed"), s("_tc_copies"), s("_advance"), s("materialize_sparse_tensors"), s("accumulate_into_grad"),
+                          py::module_::import("torch.nn").attr("Parameter").cast<py::object>().release().ptr()};
     }();
     return n;
 }
+// What an instance holds itself, a new reference or null.
+py::object own_dict(PyObject *o) {
+    py::object d = py::reinterpret_steal<py::object>(PyObject_GenericGetDict(o, nullptr));
+    if (!d) PyErr_Clear();
+    return d;
+}
+PyObject *item(const py::object &dict, PyObject *name) {      // borrowed, null where there is none
+    PyObject *v = PyDict_GetItemWithError(dict.ptr(), name);
+    if (!v && PyErr_Occurred()) throw py::error_already_set();
+    return v;
+}
+void put(const py::object &dict, PyObject *name, PyObject *v) {
+    if (PyDict_SetItem(dict.ptr(), name, v) < 0) throw py::error_already_set();
+}
+// The dictionary of a weight that is a plain torch.nn.Parameter, whose attributes of this package are kept there and nowhere else.
+py::object weight_dict(PyObject *w) { return (PyObject *)Py_TYPE(w) == layer_names().parameter_type ? own_dict(w) : py::object(); }
+// c % f == 0 as Python has it; -1 where the two are not plain integers of 64 bits
+int due(PyObject *counter, PyObject *freq) {
+    if (!counter || !freq || !PyLong_CheckExact(counter) || !PyLong_CheckExact(freq)) return -1;
+    int over1 = 0, over2 = 0;
+    const long long c = PyLong_AsLongLongAndOverflow(counter, &over1), f = PyLong_AsLongLongAndOverflow(freq, &over2);
+    return over1 || over2 || f == 0 ? -1 : (f == -1 || c % f == 0);
+}
+bool is_sparse_mode(PyObject *mode) { return mode && PyUnicode_CheckExact(mode) && PyUnicode_CompareWithASCIIString(mode, "sparse") == 0; }
+// What SparseLinearTranspose._take leaves on the weight, but for the mask.
+void install(const py::object &w, const Copies &k) {
+    const LayerNames &N = layer_names();
+    const py::tuple held = py::make_tuple(k.pw, k.mw, k.pt, k.mt);
+    put(w, N.compressed, held.ptr());
+    if (k.tcw.defined())
+        put(w, N.compressed_tc, py::make_tuple(held, (int64_t)k.mw._version(), (int64_t)k.mt._version(), py::make_tuple(k.tcw, k.tct)).ptr());
+    else put(w, N.compressed_tc, Py_None);
+    put(w, N.weight_sparse, Py_None);
+    put(w, N.weight_sparse_T, Py_None);
+}
+
+struct Walk { PyObject *base_modules, *base_named, *modules, *named, *children; };
+const Walk &walk_names() {       // made by the module's load, see PyObjects
+    static const Walk w = [] {
+        auto s = [](const char *t) { return PyUnicode_InternFromString(t); };
+        const py::object cls = py::module_::import("torch.nn").attr("Module");
+        return Walk{py::object(cls.attr("modules")).release().ptr(), py::object(cls.attr("named_modules")).release().ptr(), s("modules"), s("named_modules"),
+                    s("_modules")};
+    }();
+    return w;
+}
+// ``model.modules()``, each once and in the same order, or None where a module has a walk of its own: torch's asks every module for its
+// ``named_modules``, so one that has another, in its class or on the instance, decides what is below it; ``modules`` counts at the root
+// only.  Without a generator per level of nesting, which for 48 layers took as long as the launch that refreshes them (in Python 25 us).
+py::object modules(const py::object &model) {
+    const Walk &W = walk_names();
+    const py::object root = own_dict(model.ptr());
+    if (!root || _PyType_Lookup(Py_TYPE(model.ptr()), W.modules) != W.base_modules || item(root, W.modules)) return py::none();
+    const py::object seen = py::reinterpret_steal<py::object>(PySet_New(nullptr));
+    py::list out;
+    std::vector<py::object> stack{model};
+    while (!stack.empty()) {
+        const py::object mod = std::move(stack.back());
+        stack.pop_back();
+        if (mod.is_none()) continue;
+        const int known = PySet_Contains(seen.ptr(), mod.ptr());
+        if (known < 0) throw py::error_already_set();
+        if (known) continue;
+        PyTypeObject *const cls = Py_TYPE(mod.ptr());
+        const py::object dict = own_dict(mod.ptr());
+        if (!dict || _PyType_Lookup(cls, W.named) != W.base_named || item(dict, W.named) || _PyType_Lookup(cls, W.children)) return py::none();
+        PyObject *const children = item(dict, W.children);
+        if (!children || !PyDict_CheckExact(children)) return py::none();
+        if (PySet_Add(seen.ptr(), mod.ptr()) < 0) throw py::error_already_set();
+        out.append(mod);
+        const size_t below = stack.size();
+        PyObject *key, *child;
+        for (Py_ssize_t at = 0; PyDict_Next(children, &at, &key, &child);) stack.push_back(py::reinterpret_borrow<py::object>(child));
+        std::reverse(stack.begin() + below, stack.end());
+    }
+    return out;
+}
 
 std::pair<int64_t, py::list> refresh_layers(const py::list &mods, at::ScalarType t, const py::object &plain) {
-    const RefreshNames &N = refresh_names();
-    auto attr = [](PyObject *o, PyObject *name) {
-        PyObject *v = PyObject_GetAttr(o, name);
-        if (!v) throw py::error_already_set();
-        return py::reinterpret_steal<py::object>(v);
-    };
-    auto set = [](PyObject *o, PyObject *name, PyObject *v) {
-        if (PyObject_SetAttr(o, name, v) < 0) throw py::error_already_set();
-    };
+    const LayerNames &N = layer_names();
     struct Group { bool reselect; at::ScalarType type; c10::Device device; std::vector<Tensor> weights, masks; std::vector<py::object> owners; };
     std::vector<Group> groups;
     py::list left;
-    const bool plain_class = !PyObject_IsTrue(attr(plain.ptr(), N.materialize).ptr());
+    const py::object materialize = py::reinterpret_steal<py::object>(PyObject_GetAttr(plain.ptr(), N.materialize));
+    if (!materialize) throw py::error_already_set();
+    const bool plain_class = !PyObject_IsTrue(materialize.ptr());
     for (const py::handle mod : mods) {
-        PyObject *dict = nullptr, *params = nullptr, *w = nullptr;
-        py::object held;
-        if (plain_class && (PyObject *)Py_TYPE(mod.ptr()) == plain.ptr()) {
-            held = py::reinterpret_steal<py::object>(PyObject_GenericGetDict(mod.ptr(), nullptr));
-            dict = held.ptr();
-            if (!dict) PyErr_Clear();
-        }
+        PyObject *params = nullptr, *w = nullptr;
+        const py::object dict = plain_class && (PyObject *)Py_TYPE(mod.ptr()) == plain.ptr() ? own_dict(mod.ptr()) : py::object();
         // plain: the weight is the registered parameter, and nothing of its handling is replaced on the instance
-        if (dict && !PyDict_GetItemWithError(dict, N.weight) && !PyDict_GetItemWithError(dict, N.take) && !PyDict_GetItemWithError(dict, N.materialize) &&
-            (params = PyDict_GetItemWithError(dict, N.parameters)) && PyDict_Check(params))
-            w = PyDict_GetItemWithError(params, N.weight);
-        if (PyErr_Occurred()) throw py::error_already_set();
-        if (!w || !THPVariable_Check(w)) {
+        if (dict && !item(dict, N.weight) && !item(dict, N.take) && !item(dict, N.materialize) && (params = item(dict, N.parameters)) && PyDict_Check(params))
+            w = item(py::reinterpret_borrow<py::object>(params), N.weight);
+        const py::object wd = w && THPVariable_Check(w) ? weight_dict(w) : py::object();
+        if (!wd) {
             left.append(mod);
             continue;
         }
         const Tensor &weight = THPVariable_Unpack(w);
-        const py::object mode = attr(w, N.mode), cnt = attr(w, N.cnt), mask_o = attr(w, N.mask), counter = attr(w, N.counter), freq = attr(w, N.freq);
-        if (!PyUnicode_CheckExact(mode.ptr()) || !PyLong_CheckExact(cnt.ptr()) || !PyLong_CheckExact(counter.ptr()) || !PyLong_CheckExact(freq.ptr()) ||
-            !THPVariable_Check(mask_o.ptr()) || weight.dim() != 2) {
+        PyObject *mode = item(wd, N.mode), *cnt = item(wd, N.cnt), *mask_o = item(wd, N.mask);
+        const int reselect = due(item(wd, N.counter), item(wd, N.freq));
+        if (!mode || !PyUnicode_CheckExact(mode) || !cnt || !PyLong_CheckExact(cnt) || !mask_o || !THPVariable_Check(mask_o) || weight.dim() != 2) {
             left.append(mod);
             continue;
         }
-        if (PyUnicode_CompareWithASCIIString(mode.ptr(), "sparse") != 0 || PyObject_IsTrue(cnt.ptr()) || !weight.is_cuda()) continue;
+        if (!is_sparse_mode(mode) || PyObject_IsTrue(cnt) || !weight.is_cuda()) continue;
         if (weight.size(0) % 128 || weight.size(1) % 128) continue;
-        const Tensor &mask = THPVariable_Unpack(mask_o.ptr());
-        int over1 = 0, over2 = 0;
-        const long long c = PyLong_AsLongLongAndOverflow(counter.ptr(), &over1), f = PyLong_AsLongLongAndOverflow(freq.ptr(), &over2);
-        if (mask.device() != weight.device() || mask.scalar_type() != at::kBool || !mask.is_contiguous() || over1 || over2 || f == 0) {
+        const Tensor &mask = THPVariable_Unpack(mask_o);
+        if (mask.device() != weight.device() || mask.scalar_type() != at::kBool || !mask.is_contiguous() || reselect < 0) {
             left.append(mod);
             continue;
         }
-        const bool reselect = c % f == 0;
         Group *g = nullptr;
         for (Group &have : groups)
-            if (have.reselect == reselect && have.type == weight.scalar_type() && have.device == weight.device()) g = &have;
+            if (have.reselect == (bool)reselect && have.type == weight.scalar_type() && have.device == weight.device()) g = &have;
         if (!g) {
-            groups.push_back({reselect, weight.scalar_type(), weight.device(), {}, {}, {}});
+            groups.push_back({(bool)reselect, weight.scalar_type(), weight.device(), {}, {}, {}});
             g = &groups.back();
         }
         g->weights.push_back(weight);
         g->masks.push_back(mask);
-        g->owners.push_back(py::reinterpret_borrow<py::object>(w));
+        g->owners.push_back(wd);
     }
     int64_t done = 0;
     for (const Group &g : groups) {
@@ -560,15 +644,9 @@ std::pair<int64_t, py::list> refresh_layers(const py::list &mods, at::ScalarType
             py::gil_scoped_release nogil;
             copies = compress_all(g.weights, g.masks, t, g.reselect);
         }
-        for (size_t i = 0; i < copies.size(); ++i) {       // what SparseLinearTranspose._take does
-            const Copies &k = copies[i];
-            PyObject *w = g.owners[i].ptr();
-            const py::tuple held = py::make_tuple(k.pw, k.mw, k.pt, k.mt);
-            set(w, N.compressed, held.ptr());
-            set(w, N.compressed_tc, py::make_tuple(held, (int64_t)k.mw._version(), (int64_t)k.mt._version(), py::make_tuple(k.tcw, k.tct)).ptr());
-            set(w, N.weight_sparse, Py_None);
-            set(w, N.weight_sparse_T, Py_None);
-            set(w, N.refreshed, Py_True);
+        for (size_t i = 0; i < copies.size(); ++i) {
+            install(g.owners[i], copies[i]);
+            put(g.owners[i], N.refreshed, Py_True);
             ++done;
         }
     }
@@ -590,6 +668,24 @@ bool masked_add(const Tensor &grad, const Tensor &p, const Tensor &mask, double 
     if (grad.device().index() != cur || p.device() != grad.device() || mask.device() != grad.device()) return false;
     check(sp24_masked_add(ptr(grad), ptr(p), ptr(mask), (int)mask.element_size(), grad.numel(), (float)alpha, cur_stream()), "sp24_masked_add");
     return true;
+}
+
+// masked_add(grad, p, mask, alpha) as a plain C function of the module: a model's decays are one call a weight, and the general
+// argument conversion was a tenth of each.
+PyObject *py_masked_add(PyObject *, PyObject *const *args, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    TORCH_CHECK_TYPE(n == 4 && THPVariable_Check(args[0]) && THPVariable_Check(args[1]) && THPVariable_Check(args[2]),
+                     "masked_add: expected three tensors and a number");
+    const double alpha = PyFloat_AsDouble(args[3]);
+    if (alpha == -1.0 && PyErr_Occurred()) return nullptr;
+    const Tensor &grad = THPVariable_Unpack(args[0]), &p = THPVariable_Unpack(args[1]), &mask = THPVariable_Unpack(args[2]);
+    bool done;
+    {
+        py::gil_scoped_release nogil;
+        done = masked_add(grad, p, mask, alpha);
+    }
+    return PyBool_FromLong(done);
+    END_HANDLE_TH_ERRORS
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -716,10 +812,9 @@ Tensor unpack(PyObject *o) {
     return THPVariable_Unpack(o);
 }
 
-// y = x W_s^T + b on the compressed copies (packed_w, meta_w, packed_t, meta_t); tc = their metadata in tensor-core order.
-Tensor fst_linear(const Tensor &input, const Tensor &weight, const OptTensor &bias, const py::tuple &copies, const py::tuple &tc, bool into_grad) {
-    const Tensor pw = unpack(copies[0].ptr()), pt = unpack(copies[2].ptr()), tcw = unpack(tc[0].ptr()), tct = unpack(tc[1].ptr());
-    py::gil_scoped_release nogil;
+// y = x W_s^T + b on the compressed copies
+Tensor fst_product(const Tensor &input, const Tensor &weight, const OptTensor &bias, const Tensor &pw, const Tensor &pt, const Tensor &tcw, const Tensor &tct,
+                   bool into_grad) {
     require_cuda(input, pw, pt, tcw, tct, bias);
     no_tangent(input, weight, bias);
     Tensor x, y;
@@ -748,6 +843,134 @@ Tensor fst_linear(const Tensor &input, const Tensor &weight, const OptTensor &bi
         torch::autograd::set_history(y, node);
     }
     return y;
+}
+// copies: (packed_w, meta_w, packed_t, meta_t); tc = their metadata in tensor-core order.
+Tensor fst_linear(const Tensor &input, const Tensor &weight, const OptTensor &bias, const py::tuple &copies, const py::tuple &tc, bool into_grad) {
+    const Tensor pw = unpack(copies[0].ptr()), pt = unpack(copies[2].ptr()), tcw = unpack(tc[0].ptr()), tct = unpack(tc[1].ptr());
+    py::gil_scoped_release nogil;
+    return fst_product(input, weight, bias, pw, pt, tcw, tct, into_grad);
+}
+
+// The class whose forward fst_forward knows, and its five methods that take part: replaced ones are called by Python instead.
+struct LayerClass {
+    PyTypeObject *type = nullptr;
+    PyObject *methods[5] = {};
+} layer_class;
+void set_layer_class(const py::object &cls) {
+    const LayerNames &N = layer_names();
+    PyObject *const names[5] = {N.take, N.refresh, N.ensure, N.tc_copies, N.advance};
+    for (int i = 0; i < 5; ++i) {
+        layer_class.methods[i] = PyObject_GetAttr(cls.ptr(), names[i]);
+        if (!layer_class.methods[i]) throw py::error_already_set();
+    }
+    layer_class.type = (PyTypeObject *)cls.inc_ref().ptr();
+}
+bool layer_class_untouched() {
+    const LayerNames &N = layer_names();
+    PyObject *const names[5] = {N.take, N.refresh, N.ensure, N.tc_copies, N.advance};
+    for (int i = 0; i < 5; ++i)
+        if (_PyType_Lookup(layer_class.type, names[i]) != layer_class.methods[i]) return false;
+    return _PyType_Lookup(layer_class.type, N.materialize) == Py_False;
+}
+void add_one(const py::object &dict, PyObject *name, PyObject *v) {
+    const py::object one = py::reinterpret_steal<py::object>(PyLong_FromLong(1)), sum = py::reinterpret_steal<py::object>(PyNumber_Add(v, one.ptr()));
+    if (!sum) throw py::error_already_set();
+    put(dict, name, sum.ptr());
+}
+
+// fst_forward(layer, x): SparseLinearTranspose.forward of a plain layer in sparse mode, state and all; None where anything about the call is
+// not plain, before anything was changed: the class's own Python takes the call then.  In Python the attributes, tuples and frames
+// of a call were a third of a small layer's forward.
+PyObject *py_fst_forward(PyObject *, PyObject *const *args, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    const LayerNames &N = layer_names();
+    if (n != 2 || Py_TYPE(args[0]) != layer_class.type || !THPVariable_Check(args[1]) || torch::jit::tracer::isTracing() || !layer_class_untouched())
+        Py_RETURN_NONE;
+    const py::object dict = own_dict(args[0]);
+    if (!dict || item(dict, N.weight) || item(dict, N.bias) || item(dict, N.take) || item(dict, N.refresh) || item(dict, N.ensure) ||
+        item(dict, N.tc_copies) || item(dict, N.advance) || item(dict, N.materialize))
+        Py_RETURN_NONE;
+    PyObject *const params_o = item(dict, N.parameters), *const training = item(dict, N.training);
+    if (!params_o || !PyDict_Check(params_o) || (training != Py_True && training != Py_False)) Py_RETURN_NONE;
+    const py::object params = py::reinterpret_borrow<py::object>(params_o);
+    PyObject *const w_o = item(params, N.weight), *const b_o = item(params, N.bias);
+    if (!w_o || !THPVariable_Check(w_o) || !b_o || (b_o != Py_None && !THPVariable_Check(b_o))) Py_RETURN_NONE;
+    const py::object wd = weight_dict(w_o);
+    if (!wd) Py_RETURN_NONE;
+    PyObject *const cnt = item(wd, N.cnt), *const mask_o = item(wd, N.mask), *const step = item(wd, N.step), *const counter = item(wd, N.counter);
+    if (!is_sparse_mode(item(wd, N.mode)) || !cnt || !PyLong_CheckExact(cnt) || !step || !PyLong_CheckExact(step) || !counter || !PyLong_CheckExact(counter) ||
+        !mask_o || !THPVariable_Check(mask_o))
+        Py_RETURN_NONE;
+    const Tensor weight = THPVariable_Unpack(w_o), mask = THPVariable_Unpack(mask_o), x = THPVariable_Unpack(args[1]);
+    const OptTensor bias = b_o == Py_None ? OptTensor() : OptTensor(THPVariable_Unpack(b_o));
+    if (mask.device() != weight.device()) Py_RETURN_NONE;
+    PyObject *into = item(dict, N.into_grad);
+    if (!into) into = _PyType_Lookup(layer_class.type, N.into_grad);
+    if (into != Py_True && into != Py_False) Py_RETURN_NONE;
+    const bool first = PyObject_IsTrue(cnt) == 0;
+    PyObject *const refreshed = item(wd, N.refreshed);
+    if (refreshed && refreshed != Py_True && refreshed != Py_False) Py_RETURN_NONE;
+    const bool compress_now = first && refreshed != Py_True;
+
+    Tensor pw, pt, tcw, tct;
+    if (compress_now) {
+        const int reselect = due(counter, item(wd, N.freq));
+        // whole 128 x 128 blocks: the launch leaves the metadata in the GEMM's order too
+        if (reselect < 0 || weight.dim() != 2 || weight.size(0) % 128 || weight.size(1) % 128) Py_RETURN_NONE;
+        // a reselected mask overwrites the existing buffer, so that it keeps one address for the whole run
+        const bool reuse = reselect && mask.is_cuda() && mask.is_contiguous() && mask.scalar_type() == at::kBool;
+        const bool bf16 = at::autocast::is_autocast_enabled(at::kCUDA) && at::autocast::get_autocast_dtype(at::kCUDA) == at::kBFloat16;
+        Tensor used;
+        c10::optional<Copies> c;
+        {
+            py::gil_scoped_release nogil;
+            c.emplace(select_copies(weight, reselect ? OptTensor() : OptTensor(mask), bf16 ? at::kBFloat16 : at::kHalf,
+                                    reuse ? OptTensor(mask) : OptTensor(), used));
+        }
+        if (!used.is_same(mask)) put(wd, N.mask, py::cast(used).ptr());
+        install(wd, *c);
+        pw = c->pw;
+        pt = c->pt;
+        tcw = c->tcw;
+        tct = c->tct;
+    } else {
+        // the copies at hand and their metadata in the GEMM's order, if both are still what the compression left
+        PyObject *const held = item(wd, N.compressed), *const tc = item(wd, N.compressed_tc);
+        if (!held || !PyTuple_CheckExact(held) || PyTuple_GET_SIZE(held) != 4 || !tc || !PyTuple_CheckExact(tc) || PyTuple_GET_SIZE(tc) != 4 ||
+            PyTuple_GET_ITEM(tc, 0) != held)
+            Py_RETURN_NONE;
+        for (int i = 0; i < 4; ++i)
+            if (!THPVariable_Check(PyTuple_GET_ITEM(held, i))) Py_RETURN_NONE;
+        PyObject *const order = PyTuple_GET_ITEM(tc, 3);
+        auto version = [](const Tensor &t, PyObject *v) { return !t.is_inference() && PyLong_CheckExact(v) && PyLong_AsLongLong(v) == (long long)t._version(); };
+        if (!PyTuple_CheckExact(order) || PyTuple_GET_SIZE(order) != 2 || !THPVariable_Check(PyTuple_GET_ITEM(order, 0)) ||
+            !THPVariable_Check(PyTuple_GET_ITEM(order, 1)) || !version(THPVariable_Unpack(PyTuple_GET_ITEM(held, 1)), PyTuple_GET_ITEM(tc, 1)) ||
+            !version(THPVariable_Unpack(PyTuple_GET_ITEM(held, 3)), PyTuple_GET_ITEM(tc, 2)))
+            Py_RETURN_NONE;
+        pw = THPVariable_Unpack(PyTuple_GET_ITEM(held, 0));
+        pt = THPVariable_Unpack(PyTuple_GET_ITEM(held, 2));
+        tcw = THPVariable_Unpack(PyTuple_GET_ITEM(order, 0));
+        tct = THPVariable_Unpack(PyTuple_GET_ITEM(order, 1));
+        if (first) put(wd, N.refreshed, Py_False);
+    }
+    Tensor y;
+    {
+        py::gil_scoped_release nogil;
+        y = fst_product(x, weight, bias, pw, pt, tcw, tct, into == Py_True);
+    }
+    if (training == Py_True) {
+        // read again: a saved-tensor hook may have run Python since
+        PyObject *const c = item(wd, N.cnt), *const s = item(wd, N.step), *const o = item(wd, N.counter);
+        if (!c || !s || !o) {
+            PyErr_SetString(PyExc_AttributeError, "the weight's counters are gone");
+            return nullptr;
+        }
+        if (PyObject_IsTrue(c) == 0) add_one(wd, N.counter, o);
+        add_one(wd, N.step, s);
+        add_one(wd, N.cnt, c);
+    }
+    return THPVariable_Wrap(std::move(y));
+    END_HANDLE_TH_ERRORS
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1415,9 +1638,15 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("compress", &compress, nogil());
     m.def("select_compress", &select_compress);
     m.def("select_compress_many", &select_compress_many);
-    refresh_names();
+    layer_names();
+    walk_names();
+    m.def("modules", &modules);
     m.def("refresh_layers", &refresh_layers);
-    m.def("masked_add", &masked_add, nogil());
+    static PyMethodDef calls[] = {{"masked_add", (PyCFunction)(void (*)(void))py_masked_add, METH_FASTCALL, nullptr},
+                                  {"fst_forward", (PyCFunction)(void (*)(void))py_fst_forward, METH_FASTCALL, nullptr},
+                                  {nullptr, nullptr, 0, nullptr}};
+    if (PyModule_AddFunctions(m.ptr(), calls) < 0) throw py::error_already_set();
+    m.def("set_layer_class", &set_layer_class);
     m.def("fst_linear", &fst_linear);
     m.def("fst_weight_grads",
           [](const Tensor &g, const Tensor &x, const Tensor &w, const OptTensor &b, bool into, bool nw, bool nb) {

@@ -132,8 +132,9 @@ class _Host:
         spec = importlib.util.spec_from_file_location("_sp24_torch", HOST_PATH)
         mod = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(mod)
-        from .sparse_ops import _dense_weight_grads
+        from .sparse_ops import SparseLinearTranspose, _dense_weight_grads
         mod.set_dense_weight_grads(_dense_weight_grads)
+        mod.set_layer_class(SparseLinearTranspose)
         self.__dict__.update((k, v) for k, v in vars(mod).items() if not k.startswith("_"))
         return self.__dict__[name]
 

@@ -306,6 +306,9 @@ class SparseLinearTranspose(nn.Linear):
         if w.mode == 'dense':
             x = F.linear(x, w, self.bias)
         else:
+            y = _host.fst_forward(self, x)   # all of what follows and _advance for a plain layer; None where anything is not plain
+            if y is not None:
+                return y
             self._ensure_compressed()
             x = _ext.call_layer(_ext.host.fst_linear, x, w, self.bias, w.compressed, self._tc_copies(), self.accumulate_into_grad)
         self._advance()
@@ -313,29 +316,8 @@ class SparseLinearTranspose(nn.Linear):
 
 
 def _modules(model: nn.Module):
-    """``model.modules()``, each once and in the same order, without a generator per level of nesting: with 48 layers the walk was
-    a fifth of the host time of their refresh.  torch's walk asks every module for its ``named_modules``, so a module that has
-    one of its own, in its class or on the instance, decides what is below it; ``modules`` counts at the root only."""
-    if type(model).modules is not nn.Module.modules or 'modules' in model.__dict__:
-        return list(model.modules())
-    seen, out, stack, plain = set(), [], [model], set()
-    while stack:
-        mod = stack.pop()
-        if mod is None or mod in seen:
-            continue
-        cls = type(mod)
-        if cls not in plain:
-            if cls.named_modules is not nn.Module.named_modules:
-                return list(model.modules())
-            plain.add(cls)
-        if 'named_modules' in mod.__dict__:
-            return list(model.modules())
-        seen.add(mod)
-        out.append(mod)
-        children = mod._modules
-        if children:
-            stack.extend(reversed(children.values()))
-    return out
+    """``list(model.modules())``, walked by native code where no module has a walk of its own."""
+    return _host.modules(model) or list(model.modules())
 
 
 def refresh_sparse_layers(model: nn.Module) -> int:

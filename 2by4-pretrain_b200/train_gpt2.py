@@ -179,7 +179,8 @@ def masked_decay_(model, alpha):
     with torch.no_grad():
         for p in model.parameters():
             if hasattr(p, "mask") and p.mode == "sparse" and p.grad is not None:
-                p.grad = p.grad.float()
+                if p.grad.dtype != torch.float32:
+                    p.grad = p.grad.float()
                 sparse.masked_add_(p.grad.data, p.data, p.mask, alpha=alpha)
                 p.cnt = 0
 
