@@ -945,7 +945,7 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(tmem_full0 + 8 * b, 1);
-            mbar_init(tmem_empty0 + 8 * b, 16);   // used in the leader only: eight epilogue warps of each CTA
+            mbar_init(tmem_empty0 + 8 * b, EPI == EPI_PLAIN ? 8 : 16);   // used in the leader only: four or eight epilogue warps of each CTA
         }
         fence_barrier_init();
     }
@@ -1046,14 +1046,15 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         }
     } else {
         // ---------------------------------------------------------------- epilogue (warps 2..9 of both CTAs)
-        // Plain form: a warp takes every other 16-token chunk of its 32 features.  tcgen05.ld in the 16x256b shape leaves 8 x 8
-        // fragments, packed to 16 bits in registers (64 of them), and the accumulator goes back to the MMAs at once.  stmatrix then
-        // writes the fragments token-major into the warp's two chunks of shared memory, from where 16-byte stores take them: 8 tokens
-        // x 64 bytes an instruction instead of one token's 32 two-byte values.  128-byte rows and TMA stores were no faster: 148 blocks
-        // that only write such tiles reach 5.3 TB/s in pieces of 64 to 256 bytes, and here the stores share the way to L2 with the
-        // operand fill.  Taken by itself it gains where many tiles are written, fp16 us, two-byte stores -> now: ms 3072, k 768,
-        // n 8192 28.0 -> 26.6, n 16384 50.0 -> 49.3; float8 ms 768, k 768, n 4096 7.5 -> 7.3; with few short tiles its chain costs up
-        // to 0.2 us (see Ctl2 for the rest).
+        // Plain form: 16-token chunks of a warp's 32 features, two read and packed to 16 bits while the two before are stored.
+        // tcgen05.ld in the 16x256b shape leaves 8 x 8 fragments; stmatrix writes them token-major into the warp's two chunks of shared
+        // memory, from where 16-byte stores take them, 8 tokens x 64 bytes an instruction (128-byte rows and TMA stores were no faster).
+        // While a later tile will want the accumulator again, the four warps of one half take all of it and the other four the next
+        // tile's; of a pair's last two tiles, which nobody waits for, each half takes every other chunk.  With all eight warps on one tile,
+        // an accumulator first read whole into registers and then stored, the stores stood still while it was read: 4500 clocks a tile
+        // without any operand loads, where stores by themselves take 2640.  us, that -> now: ms 3072, k 768, n 8192 30.4 -> 27.9 (float8
+        // 22.6 -> 19.2), n 16384 47.6 -> 46.9; ms 768, n 8192, k 3072 24.6 -> 23.5; ms 4096, n 2043, k 4096 28.2 -> 27.1; ms 1024, n 1024,
+        // k 1024 7.4 -> 6.8; ms 512, n 256, k 256 4.8 -> 4.25 (a third of that from the shorter code).  One loop for both cases: 2 - 5 % slower.
         // Fused forms: a warp packs its BN / 2 columns of the accumulator into registers, hands the buffer back, then stores
         // 16-bit values directly; the 32 lanes of a store are 32 consecutive features of one token.
         const int quad = warp & 3, half = (warp - 2) >> 2;
@@ -1084,59 +1085,92 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             if constexpr (EPI == EPI_PLAIN) {
                 const int64_t left = P.n - row0;
                 const int limit = left < BN ? (int)left : BN, chunks = (limit + 15) / 16;
-                uint32_t held[MAX_CHUNKS2][8];      // chunk half + 2 i: word 4 h + j has features 16 h + 8 (j % 2), tokens 8 (j / 2)
-                if (run) {
-                    float bias[4] = {0.f, 0.f, 0.f, 0.f};       // of features 8 h + lane / 4
-                    if (P.bias) {
+                float bias[4] = {0.f, 0.f, 0.f, 0.f};       // of features 8 h + lane / 4
+                if (run && P.bias) {
 #pragma unroll
-                        for (int h = 0; h < 4; ++h) bias[h] = load_bias<OutT>(P, mrow + 8 * h + (lane >> 2));
-                    }
-                    const uint32_t acc = tmem_base + ((uint32_t)(quad * 32) << 16) + buf * ACC_COL + half * 16;
-#pragma unroll
-                    for (int i0 = 0; i0 < MAX_CHUNKS2; i0 += 2) {
-                        if (half + 2 * i0 >= chunks) break;
-                        uint32_t v[2][2][8];
-#pragma unroll
-                        for (int i = 0; i < 2; ++i) {           // past the last chunk: other columns, read but not stored
-                            tmem_ld_16x256b_x2(acc + (i0 + i) * 32, v[i][0]);
-                            tmem_ld_16x256b_x2(acc + (16u << 16) + (i0 + i) * 32, v[i][1]);
-                        }
-                        tmem_ld_wait();
-#pragma unroll
-                        for (int i = 0; i < 2; ++i)
-#pragma unroll
-                            for (int h = 0; h < 2; ++h)
-#pragma unroll
-                                for (int j = 0; j < 4; ++j) {
-                                    Vec<OutT, 2> o;
-                                    o.v[0] = emit<OutT, false, F8>(v[i][h][2 * j], bias[2 * h + (j & 1)], 0, alpha);
-                                    o.v[1] = emit<OutT, false, F8>(v[i][h][2 * j + 1], bias[2 * h + (j & 1)], 0, alpha);
-                                    held[i0 + i][4 * h + j] = *reinterpret_cast<const uint32_t *>(&o);
-                                }
-                    }
+                    for (int h = 0; h < 4; ++h) bias[h] = load_bias<OutT>(P, mrow + 8 * h + (lane >> 2));
                 }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive_cluster(empty_leader0 + 8 * buf);
-                if (threadIdx.x == 64) SP24_TRACE(2, 4 * tl + 1);
-                if (run) {
-                    uint4 *const dst = reinterpret_cast<uint4 *>(out + (row0 + half * 16 + (lane >> 2)) * P.ld_out + mrow) + (lane & 3);
-                    const int mine = limit - half * 16 - (lane >> 2);       // tokens of the tile from this lane's first one on
+                const uint32_t acc = tmem_base + ((uint32_t)(quad * 32) << 16) + buf * ACC_COL;
+                const int64_t row = P.ld_out / 8;           // of 16-byte pieces
+                auto read = [&](uint32_t column, uint32_t (&v)[2][8]) {      // a chunk past the last one: other columns, read but not stored
+                    tmem_ld_16x256b_x2(acc + column, v[0]);
+                    tmem_ld_16x256b_x2(acc + (16u << 16) + column, v[1]);
+                };
+                auto pack = [&](const uint32_t (&v)[2][8], uint32_t (&held)[8]) {      // word 4 h + j: features 16 h + 8 (j % 2), tokens 8 (j / 2)
 #pragma unroll
-                    for (int i = 0; i < MAX_CHUNKS2; ++i) {
-                        if (half + 2 * i >= chunks) break;
-                        const uint32_t at = stg + (i & 1) * CHUNK2_BYTES;
+                    for (int h = 0; h < 2; ++h)
 #pragma unroll
-                        for (int h = 0; h < 2; ++h)
-                            stmatrix_x4_trans(at + stm_off[h], held[i][4 * h], held[i][4 * h + 1], held[i][4 * h + 2], held[i][4 * h + 3]);
-                        __syncwarp();                           // also: the chunk before the last one has left its half
-#pragma unroll
-                        for (int h = 0; h < 2; ++h) {           // 8 tokens x 64 bytes an instruction
-                            const uint4 o = ld_shared_v4(at + ld_off + h * 512);
-                            if (32 * i + 8 * h < mine) dst[(32 * i + 8 * h) * (P.ld_out / 8)] = o;
+                        for (int j = 0; j < 4; ++j) {
+                            Vec<OutT, 2> o;
+                            o.v[0] = emit<OutT, false, F8>(v[h][2 * j], bias[2 * h + (j & 1)], 0, alpha);
+                            o.v[1] = emit<OutT, false, F8>(v[h][2 * j + 1], bias[2 * h + (j & 1)], 0, alpha);
+                            held[4 * h + j] = *reinterpret_cast<const uint32_t *>(&o);
                         }
+                };
+                auto store = [&](uint32_t at, const uint32_t (&held)[8], uint4 *to, int tokens) {
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) stmatrix_x4_trans(at + stm_off[h], held[4 * h], held[4 * h + 1], held[4 * h + 2], held[4 * h + 3]);
+                    __syncwarp();                           // also: the chunk before the last one has left its half
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {           // 8 tokens x 64 bytes an instruction
+                        const uint4 o = ld_shared_v4(at + ld_off + h * 512);
+                        if (8 * h < tokens) to[8 * h * row] = o;
                     }
-                    __syncwarp();
+                };
+                uint4 *const dst = reinterpret_cast<uint4 *>(out + (row0 + (lane >> 2)) * P.ld_out + mrow) + (lane & 3);
+                const int mine = limit - (lane >> 2);       // tokens of the tile from this lane's first one on
+                uint32_t v[2][2][8], held[2][8];
+                if (tile + 2 * n_pairs < n_tiles) {
+                    // the tile after the next wants this accumulator
+                    if ((tl & 1) == half) {
+                        if (run) {
+                            read(0, v[0]);
+                            read(16, v[1]);
+                        }
+#pragma unroll 1
+                        for (int c = 0; c < chunks; c += 2) {
+                            if (run) {
+                                tmem_ld_wait();
+                                pack(v[0], held[0]);
+                                pack(v[1], held[1]);
+                                if (c + 2 < chunks) {
+                                    read((c + 2) * 16, v[0]);
+                                    read((c + 3) * 16, v[1]);
+                                }
+                            }
+                            if (c + 2 >= chunks) {          // all read
+                                tc_fence_before();
+                                __syncwarp();
+                                if (lane == 0) mbar_arrive_cluster(empty_leader0 + 8 * buf);
+                            }
+                            if (run) {
+                                store(stg, held[0], dst + 16 * c * row, mine - 16 * c);
+                                if (c + 1 < chunks) store(stg + CHUNK2_BYTES, held[1], dst + 16 * (c + 1) * row, mine - 16 * (c + 1));
+                            }
+                        }
+                        __syncwarp();
+                    }
+                } else {
+                    if (run && half < chunks) {
+                        read(half * 16, v[0]);
+                        read(half * 16 + 32, v[1]);
+#pragma unroll
+                        for (int i = 0; i < MAX_CHUNKS2; i += 2) {
+                            if (half + 2 * i >= chunks) break;
+                            tmem_ld_wait();
+                            pack(v[0], held[0]);
+                            pack(v[1], held[1]);
+                            if (i + 2 < MAX_CHUNKS2 && half + 2 * (i + 2) < chunks) {
+                                read(half * 16 + 32 * (i + 2), v[0]);
+                                read(half * 16 + 32 * (i + 3), v[1]);
+                            }
+                            uint4 *const to = dst + half * 16 * row;
+                            store(stg, held[0], to + 32 * i * row, mine - half * 16 - 32 * i);
+                            if (half + 2 * (i + 1) < chunks) store(stg + CHUNK2_BYTES, held[1], to + 32 * (i + 1) * row, mine - half * 16 - 32 * (i + 1));
+                        }
+                        __syncwarp();
+                    }
+                    tc_fence_before();
                 }
             } else {
                 const int64_t tok0 = row0 + half * HC;

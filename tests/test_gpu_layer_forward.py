@@ -1,5 +1,6 @@
 """SparseLinearTranspose.forward in native code: results, gradients and the state on the weight of a run are those of the class's own Python
 (which a subclass takes), through new masks, accumulation windows, a batched refresh, evaluation, edited copies and replaced methods."""
+import gc
 import random
 
 import pytest
@@ -8,6 +9,13 @@ import torch
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
 STATE = ("mode", "cnt", "counter", "freq", "step", "weight_sparse", "weight_sparse_T")
+
+
+@pytest.fixture(autouse=True)
+def _nothing_left():
+    """Caught exceptions hold layers in cycles; other tests count the memory in use."""
+    yield
+    gc.collect()
 
 
 def _pair(i, o, bias=True):

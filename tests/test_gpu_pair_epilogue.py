@@ -1,0 +1,36 @@
+"""The CTA-pair GEMM's plain epilogue over several tiles a pair: accumulators that are wanted again (all columns by four warps) and a pair's
+last two (every other chunk by eight), widths of an odd and an even number of chunks, last tiles of one and of seventeen tokens, a bias, a
+half-empty row block, inside the output's window."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+ROUND = {torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8}
+
+
+# tiles a pair: 3 to 6, 12, 2 and 1
+@pytest.mark.parametrize("dtype", list(ROUND), ids=["f16", "bf16"])
+@pytest.mark.parametrize("ms,n,k", [(3072, 8193, 64), (2304, 8081, 128), (768, 16385, 192), (3072, 16384, 64), (1152, 8225, 320), (512, 8191, 64), (256, 17, 64)])
+def test_several_tiles_a_pair(ms, n, k, dtype):
+    import sparse
+    from sparse import _ext, spmm
+    g = torch.Generator(device=DEV).manual_seed(ms + n + k)
+    sp = sparse.to_sparse_semi_structured(torch.randn(ms, k, device=DEV, generator=g).to(dtype), dtype=dtype)
+    x, bias = torch.randn(n, k, device=DEV, generator=g).to(dtype), torch.randn(ms, device=DEV, generator=g).to(dtype)
+    buf = torch.randn(n + 2, ms + 16, device=DEV, generator=g).to(dtype)
+    before, out = buf.clone(), buf[1:-1, 8:-8]
+    p, e, status = sp.sparse_tensor_cutlass, spmm.tc_metadata(sp.meta_tensor_cutlass, ms, k), spmm._status_word(torch.device(DEV))
+    dt = _ext.dt(dtype)
+    for b in (bias, None):
+        _ext.check(_ext.lib().sp24_spmm(p.data_ptr(), dt, 0, k // 2, e.data_ptr(), ms, k, x.data_ptr(), 0, k, n, out.data_ptr(), dt, 1, ms + 16,
+                                        _ext.ptr(b), 0, status.data_ptr(), _ext.stream()), "spmm")
+        spmm.check_status()
+        a = sp.to_dense().double()
+        ref, mag = x.double() @ a.t(), x.double().abs() @ a.abs().t()
+        if b is not None:
+            ref, mag = ref + b.double(), mag + b.double().abs()
+        # float32 sums, one rounding
+        assert bool(((out.double() - ref).abs() <= ROUND[dtype] * ref.abs() * 1.01 + (k + 2) * 2.0 ** -24 * mag).all())
+    out.copy_(before[1:-1, 8:-8])
+    assert torch.equal(buf, before)
