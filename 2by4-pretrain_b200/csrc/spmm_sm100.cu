@@ -2066,37 +2066,12 @@ void pick_f8_tile(int64_t ms, int64_t n, int sms, int &bn, int &mpt) {
     mpt = ((n + 127) / 128) * ((ms / BM + 1) / 2) >= sms ? 2 : 1;
 }
 
-// Whether the CTA-pair kernel takes an operand whose last 256-row block is half empty (ms an odd multiple of 128): where its estimated
-// time is lower.  Both estimates, ns, are a start and, for every round of tiles, what the columns of a CTA's tile take to write and the
-// K steps to stage, less what the two overlap; fitted to a map over 8 row counts (128 .. 2944), 16 widths (64 .. 16384) and K from 64 to
-// 1536, which they meet by 3 % on average.  Pairs gain by the bytes that a K step stages and lose by a wide tile's epilogue, of which
-// the empty half does nothing.  us, single CTAs -> pairs, taken: fp16 ms 896, n 1984, k 1152 8.7 -> 7.9, n 8192, k 3072 43.5 -> 27.7;
-// ms 128, n 256, k 512 5.4 -> 4.4; float8 ms 1152, n 8192, k 3072 46.1 -> 20.8; left alone: ms 2176, n 1024, k 128 4.4 -> 5.3; ms 640,
-// n 3496, k 320 5.5 -> 6.2; float8 ms 896, n 2537, k 128 4.8 -> 5.6.  Over the map pairs are taken and up to 9 % slower at 22 of 1536
-// sizes in fp16 and at none of 1024 in float8.  Up to 320 columns they were never slower by more than 4 %.  Many columns and few K steps
-// (the lines in the middle) stay with single CTAs without an estimate.
-bool pair_takes_rows(int64_t ms, int64_t n, int64_t k, bool f8, int sms) {
-    if (ms % 256 == 0 || n <= 320) return true;
-    if (n > 2560) {
-        if (k <= 256 || (k <= 512 && ms <= 384)) return false;
-        if (ms == 128 && n > 5120 && k <= (f8 ? 1024 : 768)) return false;
-    }
-    const int64_t steps = (k + (f8 ? 255 : 127)) / (f8 ? 256 : 128);
-    auto rounds = [&](int64_t columns, int64_t row_blocks, int64_t units) {
-        const int64_t tiles = ((n + columns - 1) / columns) * ((ms / BM + row_blocks - 1) / row_blocks);
-        return (tiles + units - 1) / units;
-    };
-    const int64_t pair_bn = pick_pair_bn(ms, n, true, f8, sms);
-    const int64_t pair = 4100 + rounds(pair_bn, 2, sms / 2) * (f8 ? 12 * pair_bn + 340 * steps - 800 : 13 * pair_bn + 260 * steps - 800);
-    int bn = 128, mpt = 2;
-    if (f8) {
-        pick_f8_tile(ms, n, sms, bn, mpt);
-        return pair <= 3100 + rounds(bn, mpt, sms) * (7 * mpt * bn + (mpt == 2 ? 1000 : 650) * steps);
-    }
-    pick_tile(ms, n, sms, bn, mpt);
-    const int64_t step = 150 + (mpt * (A_STAGE_BYTES + 2048) + bn * 256) / 150;
-    return pair <= 3600 + rounds(bn, mpt, sms) * (11 * mpt * bn + step * steps - 1200);
-}
+// Whether the CTA-pair kernel takes an operand of whole or half 256-row blocks.  A half-empty last block costs its MMAs, not its stores, and
+// over a map of 9 odd row counts (128 .. 2944), 12 widths (384 .. 16384) and K from 128 to 3072 pairs are faster or alike, except where
+// the one block there is is half empty and many tiles are to be written: ms 128, n 16384, k 128 single CTAs 5.1, pairs 5.8; k 3072 19.6 / 20.5;
+// n 8192 5.3 / 5.5.  Elsewhere in fp16 up to 6 % slower at 5 of 972 sizes (384 x 6000, k 128 5.1 / 5.4) and up to 35 % faster at 211 that
+// an earlier rule left to single CTAs, us: 1152 x 12000, k 256 16.6 / 12.6; 384 x 12000, k 512 10.3 / 8.0; float8 384 x 12000, k 384 11.7 / 7.6.
+bool pair_takes_rows(int64_t ms, int64_t n) { return ms > BM || n <= 8192; }
 
 // Row blocks of a tile and K slices of the 16-bit weight gradient on single CTAs.
 int single_row_blocks(int64_t ms) { return ms >= 256 ? 2 : 1; }
@@ -2227,7 +2202,7 @@ static int spmm_impl(const void *a_packed, int dtype, int a_mn_major, int64_t ld
               ((uint32_t)(b_mn_major ? 1 : 0) << 16) | ((uint32_t)(BM >> 4) << 24);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int sms = sm_count_cached();
-    bool pair_form = pair_layout && pair_takes_rows(ms, n, k, false, sms) && pair_kernels_enabled();
+    bool pair_form = pair_layout && pair_takes_rows(ms, n) && pair_kernels_enabled();
     if (epi != EPI_PLAIN || bias_f32) pair_form = true;      // checked above: these forms exist in the pair kernel only
     if (a_mn_major) rc = pair_form ? make_map_columns(&map_a, a_packed, dtype, k / 2, ms, ld_a, 64) : make_map(&map_a, a_packed, dtype, k / 2, ms, ld_a, 64, 64);
     else rc = make_map(&map_a, a_packed, dtype, ms, k / 2, ld_a, f8 ? 128 : 64, 128);
@@ -2342,7 +2317,7 @@ static int spmm_f8_impl(const void *a_packed, int dtype, int64_t ld_a, const voi
     P.idesc = (1u << 2) | (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(BM >> 4) << 24);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int sms = sm_count_cached();
-    if (trans_out && out_dtype != SP24_F32 && pair_takes_rows(ms, n, k, true, sms) && pair_kernels_enabled()) {
+    if (trans_out && out_dtype != SP24_F32 && pair_takes_rows(ms, n) && pair_kernels_enabled()) {
         CUtensorMap map_e;
         P.bn = pick_pair_bn(ms, n, true, true, sms);
         if (int rc = make_map_columns(&map_b, b, dtype, n, k, ld_b, (uint32_t)P.bn / 2)) return rc;

@@ -34,3 +34,8 @@ def test_several_tiles_a_pair(ms, n, k, dtype):
         assert bool(((out.double() - ref).abs() <= ROUND[dtype] * ref.abs() * 1.01 + (k + 2) * 2.0 ** -24 * mag).all())
     out.copy_(before[1:-1, 8:-8])
     assert torch.equal(buf, before)
+
+
+@pytest.mark.parametrize("ms,n,k", [(128, 8192, 64), (128, 8200, 64), (384, 12008, 128), (1408, 4100, 256)])
+def test_either_side_of_the_rule_for_odd_row_blocks(ms, n, k):
+    test_several_tiles_a_pair(ms, n, k, torch.float16)
