@@ -2503,17 +2503,23 @@ static int spmm_accumulate_impl(const void *a_packed, int dtype, int a_mn_major,
     if (pair_form && ms % 256) {
         // The last of several 256-row blocks is half empty (a single one lost: ms 128, n 1920, k 6016 13.2 -> 15.3).  The error of a float32
         // accumulation on the tensor cores grows with its length (2176 x 768 over k 8128: 2.4e-6 in two slices, 1.2e-6 in four), so these
-        // keep the single-CTA kernel's number of slices at least.  Where that makes more rounds of pairs than of CTAs the two are about
-        // even, pairs 17 % slower to 13 % faster over a map, and the single CTAs keep it, except that the row sums would be a launch of
-        // their own then (2.6 us).  us, single CTAs -> pairs, as many rounds: ms 384, n 256, k 1024 10.7 -> 7.6, ms 1152, n 3072, k 8192
-        // 65.0 -> 33.1; more rounds: ms 384, n 520, k 1984 11.4 -> 13.7, ms 2944, n 768, k 16384 51.4 -> 45.8.
+        // keep the single-CTA kernel's number of slices at least.  That may make more rounds of pairs than of CTAs, a pair's round being
+        // less than half as long: both times are estimated, ns, from rounds and K steps, by a fit to a map of 504 sizes (8 row counts, 9
+        // widths, K from 256 to 16384) that they meet by 3.6 % on average, pairs with 6 % added; the row sums would be a launch of their own
+        // beside single CTAs.  us, single CTAs / pairs, pairs taken: ms 2944, n 768, k 16384 52.7 / 43.9, ms 2176, n 2304, k 8192 69.0 /
+        // 56.8, ms 384, n 256, k 1024 10.7 / 7.6; left alone: ms 384, n 520, k 1984 11.7 / 13.6, ms 1152, n 1024, k 512 11.8 / 12.7.  Against the
+        // rounds alone, which decided before, 2 sizes are more than 3 % slower (n 520) and 82 faster, up to 21 %.
         const int sms = sm_count_cached();
-        const int64_t slices = k_splits ? std::min<int64_t>(k_splits, (k + 127) / 128) : single_slices(ms, n, k, sms);
+        const int64_t k_iters = (k + 127) / 128;
+        const int64_t slices = k_splits ? std::min<int64_t>(k_splits, k_iters) : single_slices(ms, n, k, sms);
         if (!k_splits) k_splits = (int)std::max(slices, pair_slices(ms, n, k, 128, sms));
-        auto rounds = [&](int64_t columns, int64_t splits, int64_t units) {
-            return (((n + columns - 1) / columns) * ((ms + 255) / 256) * splits + units - 1) / units;
+        const int64_t splits = std::min<int64_t>(k_splits, k_iters);
+        auto rounds = [&](int64_t columns, int64_t parts, int64_t units) {
+            return (((n + columns - 1) / columns) * ((ms + 255) / 256) * parts + units - 1) / units;
         };
-        if (!row_sums && rounds(two::BN3, std::min<int64_t>(k_splits, (k + 127) / 128), sms / 2) > rounds(192, slices, sms)) {
+        const int64_t pairs = 3250 + rounds(two::BN3, splits, sms / 2) * (4930 + 392 * ((k_iters + splits - 1) / splits));
+        const int64_t singles = 6000 + rounds(192, slices, sms) * (6080 + 860 * ((k_iters + slices - 1) / slices)) + (row_sums ? 2600 : 0);
+        if (pairs > singles && rounds(two::BN3, splits, sms / 2) > rounds(192, slices, sms)) {
             pair_form = false;
             k_splits = (int)slices;
         }

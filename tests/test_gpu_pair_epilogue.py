@@ -39,3 +39,25 @@ def test_several_tiles_a_pair(ms, n, k, dtype):
 @pytest.mark.parametrize("ms,n,k", [(128, 8192, 64), (128, 8200, 64), (384, 12008, 128), (1408, 4100, 256)])
 def test_either_side_of_the_rule_for_odd_row_blocks(ms, n, k):
     test_several_tiles_a_pair(ms, n, k, torch.float16)
+
+
+@pytest.mark.parametrize("sums", [False, True])
+@pytest.mark.parametrize("ms,n,k", [(896, 1152, 1984), (2176, 640, 4096), (384, 520, 1984), (2944, 2944, 384), (1920, 1152, 8192)])
+def test_weight_gradients_of_odd_row_blocks(ms, n, k, sums):
+    """With fewer and more units than pairs, on pairs and on single CTAs, against float64; the row sums with them or on their own."""
+    import sparse
+    from sparse import _ext, spmm
+    lib, g = _ext.lib(), torch.Generator(device=DEV).manual_seed(ms + n + k)
+    sp = sparse.to_sparse_semi_structured(torch.randn(ms, k, device=DEV, generator=g).half().t().contiguous().t(), dtype=torch.float16)
+    x, parts = torch.randn(k, n, device=DEV, generator=g).half(), torch.randn(3, ms, device=DEV, generator=g)
+    p, e, status = sp.sparse_tensor_cutlass, spmm.tc_metadata(sp.meta_tensor_cutlass, ms, k), spmm._status_word(torch.device(DEV))
+    out, got = torch.zeros(ms, n, device=DEV), torch.zeros(ms, device=DEV)
+    a = (p.data_ptr(), _ext.F16, 1, ms, e.data_ptr(), ms, k, x.data_ptr(), n, n, out.data_ptr(), n, 0)
+    if sums:
+        _ext.check(lib.sp24_spmm_accumulate_sums_f32(*a, parts.data_ptr(), 3, got.data_ptr(), 0, status.data_ptr(), _ext.stream()), "spmm")
+        assert bool(((got.double() - parts.double().sum(0)).abs() <= 4 * 2.0 ** -24 * parts.double().abs().sum(0)).all())
+    else:
+        _ext.check(lib.sp24_spmm_accumulate_f32(*a, status.data_ptr(), _ext.stream()), "spmm")
+    spmm.check_status()
+    d = sp.to_dense().double()
+    assert bool(((out.double() - d @ x.double()).abs() <= (k + 16) * 2.0 ** -24 * (d.abs() @ x.double().abs())).all())
