@@ -1244,9 +1244,8 @@ struct SoftThresholdBackward : torch::autograd::Node {
         if (has_bias_ && task_should_compute_output(2)) {
             if (g.is_contiguous() && g.size(1) % 8 == 0 && aligned(g)) {
                 Tensor s = empty({g.size(1)}, at::kFloat, g);
-                check(sp24_zero(ptr(s), g.size(1) * 4, cur_stream()), "sp24_zero");
-                check(sp24_column_sums(ptr(g), dt(g.scalar_type()), g.size(0), g.size(1), g.size(1), static_cast<float *>(ptr(s)), cur_stream()),
-                      "sp24_column_sums");
+                check(sp24_column_sums_set(ptr(g), dt(g.scalar_type()), g.size(0), g.size(1), g.size(1), static_cast<float *>(ptr(s)), cur_stream()),
+                      "sp24_column_sums_set");
                 out[2] = s;
             } else {
                 out[2] = g.sum(0);

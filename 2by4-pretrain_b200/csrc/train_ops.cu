@@ -501,13 +501,14 @@ __global__ void __launch_bounds__(256) gelu_kernel(const uint4 *x, const uint4 *
     }
 }
 
-// out[c] += sum over rows of x[r, c] (float32), in a fixed order.  A cluster of eight blocks takes 64 columns, each block an
+// out[c] (add: +)= sum over rows of x[r, c] (float32), in a fixed order.  A cluster of eight blocks takes 64 columns, each block an
 // eighth of the rows: 8 threads read one row's 128 bytes, 64 rows in turn, four of them in flight per thread.  Block 0 adds
 // the eight blocks' sums up through distributed shared memory, so no atomics and no scratch.  Bound by latency: 4096 x 2304 in
-// 8.0 us, 8192 x 3072 in 14.1 (128 columns a cluster 8.3 and 14.6; with atomics in any order 5.6 and 11.1).
+// 8.0 us, 8192 x 3072 in 14.1 (128 columns a cluster 8.3 and 14.6; with atomics in any order 5.6 and 11.1).  Set instead of added to, the
+// sums need no launch that clears them: the S-STE step of the committed workload 51.9 us replayed (54.1 with it), 116.0 a call (119.6).
 constexpr int CS_COLS = 64, CS_BLOCKS = 8, CS_ROWS = 512 / (CS_COLS / 8), CS_FLIGHT = 4;
 template <typename T>
-__global__ void __cluster_dims__(1, CS_BLOCKS, 1) __launch_bounds__(512) column_sums_kernel(const T *x, int64_t rows, int64_t cols, int64_t ld, float *out) {
+__global__ void __cluster_dims__(1, CS_BLOCKS, 1) __launch_bounds__(512) column_sums_kernel(const T *x, int64_t rows, int64_t cols, int64_t ld, float *out, bool add) {
     chain_enter();
     __shared__ float part[CS_ROWS][CS_COLS + 4], total[CS_COLS];
     const auto cluster = cooperative_groups::this_cluster();
@@ -551,7 +552,7 @@ __global__ void __cluster_dims__(1, CS_BLOCKS, 1) __launch_bounds__(512) column_
         float t = 0.f;
 #pragma unroll
         for (int b = 0; b < CS_BLOCKS; ++b) t += *cluster.map_shared_rank(&total[threadIdx.x], b);
-        out[col] += t;
+        out[col] = add ? out[col] + t : t;
     }
     cluster.sync();                         // the other blocks' shared memory stays until block 0 has read it
 }
@@ -772,7 +773,7 @@ extern "C" int sp24_cross_entropy_fused(const void *logits, int dtype, const int
                              : ce_fused_launch<__nv_bfloat16>(logits, targets, lse, loss, scale, dlogits, rows, v, ld, ld_out, st);
 }
 
-extern "C" int sp24_column_sums(const void *x, int dtype, int64_t rows, int64_t cols, int64_t ld, float *out, void *stream) {
+static int column_sums(const void *x, int dtype, int64_t rows, int64_t cols, int64_t ld, float *out, bool add, void *stream) {
     if (!x || !out) return SP24_ERR_ARG;
     if (dtype != SP24_F16 && dtype != SP24_BF16) return SP24_ERR_DTYPE;
     if (rows <= 0 || cols <= 0 || cols % 8) return SP24_ERR_SHAPE;
@@ -781,9 +782,15 @@ extern "C" int sp24_column_sums(const void *x, int dtype, int64_t rows, int64_t 
     if (int rc = check_device()) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const dim3 grid((unsigned)((cols + CS_COLS - 1) / CS_COLS), CS_BLOCKS);
-    if (dtype == SP24_F16) launch_chained(st, column_sums_kernel<__half>, grid, 512, 0, static_cast<const __half *>(x), rows, cols, ld, out);
-    else launch_chained(st, column_sums_kernel<__nv_bfloat16>, grid, 512, 0, static_cast<const __nv_bfloat16 *>(x), rows, cols, ld, out);
+    if (dtype == SP24_F16) launch_chained(st, column_sums_kernel<__half>, grid, 512, 0, static_cast<const __half *>(x), rows, cols, ld, out, add);
+    else launch_chained(st, column_sums_kernel<__nv_bfloat16>, grid, 512, 0, static_cast<const __nv_bfloat16 *>(x), rows, cols, ld, out, add);
     return launch_status();
+}
+extern "C" int sp24_column_sums(const void *x, int dtype, int64_t rows, int64_t cols, int64_t ld, float *out, void *stream) {
+    return column_sums(x, dtype, rows, cols, ld, out, true, stream);
+}
+extern "C" int sp24_column_sums_set(const void *x, int dtype, int64_t rows, int64_t cols, int64_t ld, float *out, void *stream) {
+    return column_sums(x, dtype, rows, cols, ld, out, false, stream);
 }
 
 extern "C" int sp24_sum_parts(const float *parts, int64_t n_parts, int64_t m, float *out, int accumulate, void *stream) {

@@ -537,8 +537,9 @@ int sp24_cross_entropy_fused(const void *logits, int dtype, const int64_t *targe
 int sp24_scale_unless_one(void *g, int dtype, const float *factor, int64_t count, void *stream);
 
 /* out[c] += sum over rows of x (rows, cols; 16-bit, pitch ld, cols % 8 == 0), float32, in a fixed order: the bias gradient of a
- * dense layer. */
+ * dense layer.  _set: out is written, whatever it holds. */
 int sp24_column_sums(const void *x, int dtype, int64_t rows, int64_t cols, int64_t ld, float *out, void *stream);
+int sp24_column_sums_set(const void *x, int dtype, int64_t rows, int64_t cols, int64_t ld, float *out, void *stream);
 
 /*
  * GELU, tanh form, over `count` contiguous 16-bit values (count % 8 == 0), float32 arithmetic:
