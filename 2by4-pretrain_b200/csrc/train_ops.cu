@@ -117,14 +117,24 @@ __device__ __forceinline__ float4 load4_again(const float4 *p) {
 // dres (optional): the gradient that reaches the norm's input along the residual stream, added before the store;
 // ddelta (optional): the same dx again in dy's element type, the gradient of the branch that was added in front.
 // Persistent warps: each walks rows warp, warp + nwarps, ... and keeps its column sums in its own slice of shared
-// memory; one reduction over the block's eight warps at the end, then one atomic per column and block.
-// The kernel is bound by the latency of a row's two dependent memory round trips (statistics, then outputs), so what
-// counts is the number of rows in flight: with the column sums in shared memory instead of registers a thread needs
-// under 64 registers and an SM holds 32 warps instead of 16; they form ONE block per SM (LnBwdWarps<NV> warps: 32 up
-// to d = 768, 16 beyond, by the shared memory their sums take), so that the closing atomics are one set per SM.
-// A row is read twice: once for the two row-wide sums and the column sums, once more (L1 / L2) together with the
-// residual-stream gradient.  (L2 prefetches of that gradient and of the warp's next row made it slower.)
-template <int NV> struct LnBwdWarps { static constexpr int value = NV <= 6 ? 32 : 16; };
+// memory; one reduction over the block's warps at the end, then one atomic per column and block.
+// The kernel is bound by the latency of a row, so all of a row's loads (x, dy and the residual-stream gradient) go out at
+// once and stay in registers until its outputs are written.  That takes up to 128 registers and 16 warps (12 at d = 1024,
+// where 16 spill); 32 warps that read x and dy again for the outputs, and the gradient only then, had more rows in
+// flight and two dependent round trips each.  us a launch over buffers larger than L2, that form -> this one:
+// 8192 x 768 bf16 with both extras 25.8 -> 21.0 (100 MB, 15.4 at the copy rate), without 18.1 -> 15.7; 2048 x 768
+// 12.0 -> 7.1, 512 x 256 4.5 -> 2.5, 8192 x 1024 37.4 -> 26.9.  8192 x 768 with 20 warps 23.2, with 8 21.7; with the next
+// row's pieces copied to shared memory meanwhile 25.6.
+template <int NV> struct LnBwdWarps { static constexpr int value = NV <= 7 ? 16 : 12; };
+// Four elements as they lie in memory.
+template <typename T> struct Four {
+    uint2 v;
+    __device__ __forceinline__ float4 get() const { return load4<T>(reinterpret_cast<const T *>(&v)); }
+};
+template <> struct Four<float> {
+    float4 v;
+    __device__ __forceinline__ float4 get() const { return v; }
+};
 
 template <typename TDy, int NV>
 __global__ void __launch_bounds__(32 * LnBwdWarps<NV>::value, 1)
@@ -147,11 +157,21 @@ __global__ void __launch_bounds__(32 * LnBwdWarps<NV>::value, 1)
         const float mu = mean[row], rs = rstd[row];
         const float shift = -mu * rs;
         const int64_t base = row * d + lane * 4;
+        float4 xs[NV], res[NV];
+        Four<TDy> ds[NV];
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+            xs[i] = load4<float>(x + base + i * 128);
+            ds[i] = *reinterpret_cast<const Four<TDy> *>(dy + base + i * 128);
+        }
+        if (dres) {
+#pragma unroll
+            for (int i = 0; i < NV; ++i) res[i] = load4<float>(dres + base + i * 128);
+        }
         float s1 = 0.f, s2 = 0.f;
 #pragma unroll
         for (int i = 0; i < NV; ++i) {
-            const float4 xv = load4<float>(x + base + i * 128);
-            const float4 dv = load4<TDy>(dy + base + i * 128);
+            const float4 xv = xs[i], dv = ds[i].get();
             const float4 g = load4_again(g4 + i * 32);
             const float4 xh = make_float4(fmaf(xv.x, rs, shift), fmaf(xv.y, rs, shift), fmaf(xv.z, rs, shift), fmaf(xv.w, rs, shift));
             const float4 gy = make_float4(dv.x * g.x, dv.y * g.y, dv.z * g.z, dv.w * g.w);
@@ -168,8 +188,7 @@ __global__ void __launch_bounds__(32 * LnBwdWarps<NV>::value, 1)
 #pragma unroll
         for (int i = 0; i < NV; ++i) {
             const int64_t at = base + i * 128;
-            const float4 xv = load4<float>(x + at);
-            const float4 dv = load4<TDy>(dy + at);
+            const float4 xv = xs[i], dv = ds[i].get();
             const float4 g = load4_again(g4 + i * 32);
             // rs (g dy - m1 - xhat m2) = (rs g) dy + c1 + c2 xhat
             float4 o = make_float4(fmaf(c2, fmaf(xv.x, rs, shift), fmaf(rs * g.x, dv.x, c1)),
@@ -177,8 +196,7 @@ __global__ void __launch_bounds__(32 * LnBwdWarps<NV>::value, 1)
                                    fmaf(c2, fmaf(xv.z, rs, shift), fmaf(rs * g.z, dv.z, c1)),
                                    fmaf(c2, fmaf(xv.w, rs, shift), fmaf(rs * g.w, dv.w, c1)));
             if (dres) {
-                const float4 r = load4<float>(dres + at);
-                o = make_float4(o.x + r.x, o.y + r.y, o.z + r.z, o.w + r.w);
+                o = make_float4(o.x + res[i].x, o.y + res[i].y, o.z + res[i].z, o.w + res[i].w);
             }
             store4<float>(dx + at, o.x, o.y, o.z, o.w);
             if (ddelta) store4<TDy>(ddelta + at, o.x, o.y, o.z, o.w);
@@ -655,7 +673,7 @@ static int layernorm_bwd_impl(const void *dy, int dy_dtype, const float *dres, c
 #define SP24_LN_BWD(T_, NV_) \
     do { \
         constexpr int W = LnBwdWarps<NV_>::value; \
-        const size_t smem = (size_t)2 * W * d * sizeof(float);           /* 32 warps x 6 KB = 192 KB at d = 768 */ \
+        const size_t smem = (size_t)2 * W * d * sizeof(float);           /* 16 warps x 6 KB = 96 KB at d = 768 */ \
         auto kern = layernorm_bwd_kernel<T_, NV_>; \
         if (smem > 48 * 1024 && dev >= 0 && dev < 64 && !attr_set[which][NV_ - 1][dev]) { \
             if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) \
