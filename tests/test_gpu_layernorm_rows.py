@@ -38,3 +38,22 @@ def test_against_float64(d, rows, extras, dtype):
     for got, terms in ((dg, y * xh), (db, y)):
         mag = (y.abs() * (xh.abs() + 1)).sum(0)
         assert bool(((got.double() - terms.sum(0)).abs() <= (rows + 4) * 2.0 ** -24 * mag).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("rows,d", [(1, 128), (9, 768), (2369, 896), (1003, 1024)])
+def test_the_residual_stream_may_be_written_in_place(rows, d, dtype):
+    """res_out = x gives the bits of a separate buffer; the sum is float32's own, and the output that of the plain norm of it."""
+    from sparse import _ext
+    g = torch.Generator(device=DEV).manual_seed(rows + d)
+    x, delta = torch.randn(rows, d, device=DEV, generator=g), torch.randn(rows, d, device=DEV, generator=g).to(dtype)
+    gamma, beta = torch.randn(d, device=DEV, generator=g), torch.randn(d, device=DEV, generator=g)
+    p, lib, got = lambda t: t.data_ptr(), _ext.lib(), []  # noqa: E731
+    want = x + delta.float()
+    for inp, branch, res in ((x, delta, torch.empty_like(x)), (x, delta, x), (want, None, None)):
+        out, mean, rstd = torch.empty(rows, d, device=DEV, dtype=dtype), torch.empty(rows, device=DEV), torch.empty(rows, device=DEV)
+        tail = (p(gamma), p(beta), p(out), _ext.dt(dtype), p(mean), p(rstd), rows, d, 1e-5, _ext.stream())
+        rc = lib.sp24_add_layernorm_fwd(p(inp), p(branch), p(res), *tail) if res is not None else lib.sp24_layernorm_fwd(p(inp), *tail)
+        assert rc == 0 and (res is None or torch.equal(res, want))
+        got.append((out, mean, rstd))
+    assert all(torch.equal(a, b) for run in got[1:] for a, b in zip(run, got[0]))
