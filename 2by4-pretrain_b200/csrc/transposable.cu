@@ -160,14 +160,18 @@ __global__ void __launch_bounds__(256) ts_select_kernel(const T *x, T *sparse, u
                                                         int64_t ld_s, int64_t ld_m, int use_abs) {
     chain_enter();
     __shared__ uint32_t lut[64];
-    load_select_lut(lut);
+    constexpr bool LATE = sizeof(T) == 4;   // as in ts_dual_block: float32 768 x 768 3.2 -> 3.0 us, fp16 4096 x 4096 24.8 -> 28.5
+    if constexpr (!LATE) load_select_lut(lut);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t r = (int64_t)blockIdx.y * 32 + warp * 4;
     const int64_t c = (int64_t)blockIdx.x * 128 + lane * 4;
-    if (c >= k) return;
     T w[4][4];
+    if (c < k) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) load_row4<T>(x + (r + i) * ld_x + c, w[i]);
+        for (int i = 0; i < 4; ++i) load_row4<T>(x + (r + i) * ld_x + c, w[i]);
+    }
+    if constexpr (LATE) load_select_lut(lut);
+    if (c >= k) return;
     float v[4][4];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
@@ -230,7 +234,12 @@ __device__ __forceinline__ void ts_dual_block(const DualParams &P, const unsigne
     __shared__ __align__(4) uint16_t tlin[2 * 128];     // W^T: [word column parity][W column]
     __shared__ __align__(4) uint8_t nib_t[8][128];      // [block row][W column]
     __shared__ uint32_t lut[64];
-    load_select_lut(lut);
+    // The table's barrier goes behind the loads, so that they do not wait for it; 16-bit given masks, with little else to do,
+    // have it in front.  us, in front -> behind: float32 to bf16, given masks, 768 x 768 4.29 -> 4.02, 512 x 256 3.48 -> 3.30, 48
+    // weights of a 12-block, 768-wide model 112.8 -> 113.1; search 3072 x 768 7.9 -> 7.4, those 48 170.1 -> 168.7; 16-bit search
+    // 4096 x 4096 32.4 -> 31.8, eight of them over a list 226.4 -> 225.7; 16-bit given masks 2048 x 2048 7.8 -> 8.0.
+    constexpr bool LATE = SELECT || sizeof(T) == 4;
+    if constexpr (!LATE) load_select_lut(lut);
 
     // A block covers 64 rows x 128 columns as two 32-row halves.  Both halves are loaded up front so that
     // the second half's global loads are in flight while the first half is being searched.
@@ -255,6 +264,7 @@ __device__ __forceinline__ void ts_dual_block(const DualParams &P, const unsigne
             }
         }
     }
+    if constexpr (LATE) load_select_lut(lut);
 
 #pragma unroll 1
     for (int half = 0; half < 2; ++half) {
