@@ -814,7 +814,7 @@ constexpr int CHUNK2_BYTES = 16 * 64, STAGING2 = 8 * 2 * CHUNK2_BYTES;
 // k 3072 with 8192 tokens and more, 1 - 8 % (ms 4096, n 16384 229 -> 237; the same with operands of zeros, so not the power limit);
 // at k 2048 and 4096 the same sizes are 2 - 5 % faster (197 -> 192, 287 -> 286), at k 768 alike, so no rule on sizes follows.
 struct Ctl2 {
-    uint64_t bars[2 * MAX_STAGES2 + 4];
+    uint64_t bars[2 * MAX_STAGES2 + 6];
     uint32_t tmem_base;
     int abort_flag;
 };
@@ -936,6 +936,12 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 
     const uint32_t full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[MAX_STAGES2]);
     const uint32_t tmem_full0 = smem_u32(&bars[2 * MAX_STAGES2]), tmem_empty0 = smem_u32(&bars[2 * MAX_STAGES2 + 2]);
+    // Plain form: a pair's last two tiles are complete on barriers of their own.  Before them a warp waits for the tiles of its half only,
+    // each of which holds that accumulator back until the warp has read it, so a barrier is never more than one phase from what the
+    // warp waits for.  The last two are for all warps, and one that has not waited for the other accumulator before does not know its
+    // phase; waiting for every tile instead would stall a warp that two tiles of the other half have passed meanwhile.
+    const uint32_t tmem_last0 = smem_u32(&bars[2 * MAX_STAGES2 + 4]);
+    auto ends = [&](int tile) { return EPI == EPI_PLAIN && tile + 2 * n_pairs >= n_tiles; };
 
     if (threadIdx.x == 0) {
         abort_flag = 0;
@@ -945,6 +951,7 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(tmem_full0 + 8 * b, 1);
+            mbar_init(tmem_last0 + 8 * b, 1);
             mbar_init(tmem_empty0 + 8 * b, EPI == EPI_PLAIN ? 8 : 16);   // used in the leader only: four or eight epilogue warps of each CTA
         }
         fence_barrier_init();
@@ -1040,7 +1047,7 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                     eslot ^= E_SLOT;
                     if (++s == STAGES) { s = 0; ph ^= 1; }
                 }
-                if (elect_one()) tc_commit_pair(tmem_full0 + 8 * buf);   // also arrives after an abort
+                if (elect_one()) tc_commit_pair((ends(tile) ? tmem_last0 : tmem_full0) + 8 * buf);   // also arrives after an abort
                 __syncwarp();
             }
         }
@@ -1076,9 +1083,11 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         int tl = 0;
         for (int tile = pair; tile < n_tiles; tile += n_pairs, ++tl) {
             const int buf = tl & 1;
+            const bool last = ends(tile);
+            if (EPI == EPI_PLAIN && !last && (tl & 1) != half) continue;      // the other half's tile
             const int mrow = ((tile % n_tiles_m) * 2 + (int)rank) * BM + quad * 32;
             const int64_t row0 = (int64_t)(tile / n_tiles_m) * BN;
-            const bool ok = mbar_wait(tmem_full0 + 8 * buf, (tl >> 1) & 1, &abort_flag, P.status, 3);
+            const bool ok = mbar_wait((last ? tmem_last0 : tmem_full0) + 8 * buf, last ? 0 : (tl >> 1) & 1, &abort_flag, P.status, 3);
             tc_fence_after();
             if (threadIdx.x == 64) SP24_TRACE(2, 4 * tl);
             const bool run = __all_sync(0xFFFFFFFFu, ok && !abort_flag) && mrow < P.ms;      // the warp reads tensor memory together
@@ -1120,36 +1129,34 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                 uint4 *const dst = reinterpret_cast<uint4 *>(out + (row0 + (lane >> 2)) * P.ld_out + mrow) + (lane & 3);
                 const int mine = limit - (lane >> 2);       // tokens of the tile from this lane's first one on
                 uint32_t v[2][2][8], held[2][8];
-                if (tile + 2 * n_pairs < n_tiles) {
+                if (!last) {
                     // the tile after the next wants this accumulator
-                    if ((tl & 1) == half) {
-                        if (run) {
-                            read(0, v[0]);
-                            read(16, v[1]);
-                        }
-#pragma unroll 1
-                        for (int c = 0; c < chunks; c += 2) {
-                            if (run) {
-                                tmem_ld_wait();
-                                pack(v[0], held[0]);
-                                pack(v[1], held[1]);
-                                if (c + 2 < chunks) {
-                                    read((c + 2) * 16, v[0]);
-                                    read((c + 3) * 16, v[1]);
-                                }
-                            }
-                            if (c + 2 >= chunks) {          // all read
-                                tc_fence_before();
-                                __syncwarp();
-                                if (lane == 0) mbar_arrive_cluster(empty_leader0 + 8 * buf);
-                            }
-                            if (run) {
-                                store(stg, held[0], dst + 16 * c * row, mine - 16 * c);
-                                if (c + 1 < chunks) store(stg + CHUNK2_BYTES, held[1], dst + 16 * (c + 1) * row, mine - 16 * (c + 1));
-                            }
-                        }
-                        __syncwarp();
+                    if (run) {
+                        read(0, v[0]);
+                        read(16, v[1]);
                     }
+#pragma unroll 1
+                    for (int c = 0; c < chunks; c += 2) {
+                        if (run) {
+                            tmem_ld_wait();
+                            pack(v[0], held[0]);
+                            pack(v[1], held[1]);
+                            if (c + 2 < chunks) {
+                                read((c + 2) * 16, v[0]);
+                                read((c + 3) * 16, v[1]);
+                            }
+                        }
+                        if (c + 2 >= chunks) {          // all read
+                            tc_fence_before();
+                            __syncwarp();
+                            if (lane == 0) mbar_arrive_cluster(empty_leader0 + 8 * buf);
+                        }
+                        if (run) {
+                            store(stg, held[0], dst + 16 * c * row, mine - 16 * c);
+                            if (c + 1 < chunks) store(stg + CHUNK2_BYTES, held[1], dst + 16 * (c + 1) * row, mine - 16 * (c + 1));
+                        }
+                    }
+                    __syncwarp();
                 } else {
                     if (run && half < chunks) {
                         read(half * 16, v[0]);

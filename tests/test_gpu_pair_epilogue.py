@@ -41,6 +41,36 @@ def test_either_side_of_the_rule_for_odd_row_blocks(ms, n, k):
     test_several_tiles_a_pair(ms, n, k, torch.float16)
 
 
+# one K step a tile, where the MMAs of two tiles are shortest against a warp's stores: five and nine tiles a pair of 16 to 240 columns
+@pytest.mark.parametrize("ms,n,k", [(94720, 16, 64), (94720, 48, 64), (94720, 112, 128), (170240, 33, 64), (3072, 16384, 128), (4096, 20011, 64)])
+def test_short_tiles_again_and_again(ms, n, k):
+    test_several_tiles_a_pair(ms, n, k, torch.float16)
+
+
+# float8: a K step is 256 long
+@pytest.mark.parametrize("dtype", list(ROUND), ids=["f16", "bf16"])
+@pytest.mark.parametrize("ms,n,k", [(3072, 16384, 128), (3072, 8193, 256), (768, 30011, 128), (94720, 48, 128), (1152, 12001, 384)])
+def test_float8_tiles(ms, n, k, dtype):
+    """Against the single-CTA kernel's float32 result, rounded: exact products, float32 sums in the same order."""
+    from sparse import _ext, fp8, spmm
+    g = torch.Generator(device=DEV).manual_seed(ms + n)
+    w, x = torch.randn(ms, k, device=DEV, generator=g), torch.randn(n, k, device=DEV, generator=g)
+    (xq, sx), aw, ax = fp8.quantize(x), w.abs().amax().reshape(1), x.abs().amax().reshape(1)
+    packed, meta = fp8.compress_q8(w, mode=_ext.PRUNE_MSE, scale=fp8.scale_of(w))
+    tc, status = spmm.tc_metadata(meta, ms, k), spmm._status_word(torch.device(DEV))
+    buf = torch.randn(n + 2, ms + 16, device=DEV, generator=g).to(dtype)
+    before, out = buf.clone(), buf[1:-1, 8:-8]
+    for _ in range(3):
+        out.fill_(float("nan"))
+        _ext.check(_ext.lib().sp24_spmm_f8(packed.data_ptr(), _ext.E4M3, k // 2, tc.data_ptr(), ms, k, xq.data_ptr(), k, n, out.data_ptr(),
+                                           _ext.dt(dtype), 1, ms + 16, None, aw.data_ptr(), ax.data_ptr(), status.data_ptr(), _ext.stream()), "spmm_f8")
+        spmm.check_status()
+        ref = spmm.sparse_linear(xq, packed, meta, alpha=fp8.scale_of(w) * sx)
+        assert torch.equal(out, ref.to(dtype))
+    out.copy_(before[1:-1, 8:-8])
+    assert torch.equal(buf, before)
+
+
 @pytest.mark.parametrize("sums", [False, True])
 @pytest.mark.parametrize("ms,n,k", [(896, 1152, 1984), (2176, 640, 4096), (384, 520, 1984), (2944, 2944, 384), (1920, 1152, 8192)])
 def test_weight_gradients_of_odd_row_blocks(ms, n, k, sums):
