@@ -287,44 +287,68 @@ template <int MS> __device__ __forceinline__ uint32_t load_keep4(const void *mas
     }
 }
 
+// How many blocks, from the first and whole ones, ask L2 for their operands before the kernel before has ended, and whether for the
+// gradient and the mask too.
+struct Ahead { int64_t blocks; int grad, mask; };
+
+// A model's 48 weights are as many launches of 1 - 5 us, each of which would begin with an idle DRAM.  Tensors that L2 holds already only pay for
+// the requests, and nothing tells the launch which it has.  So: grids of up to two blocks an SM, where they cost next to nothing, ask for
+// all three arrays; arrays that L2 cannot hold as well, in every block; in between the first five blocks an SM (four have room at once)
+// ask for parameter and mask, the gradient being what the pass before is likely to have left in L2, and later blocks are placed too late to
+// gain.  16 KB of an array are one request of the copy engine; a request for every 128 bytes, by all blocks, cost tensors in L2 more.  us a
+// replayed launch, none / a line each / here, tensors larger than L2 by turns: 768 x 256 2.4 / 1.9 / 1.9, 768 x 768 2.9 / 2.3 / 2.25 (its
+// bytes 1.2), 2304 x 768 5.1 / 4.2 / 4.1 (3.5), 3072 x 768 6.1 / 5.2 / 4.7 (4.7), 3072 x 1024 7.5 / 6.6 / 6.6, 4096 x 1024 9.4 / 8.3 / 8.2,
+// 4096 x 2048 17.1 / 16.0 / 16.2, 4096 x 4096 32.5 / 31.0 / 30.9; the 48 weights of a 12-block model 768 wide 248 / 217 / 195 (169), 384 wide 137 /
+// 109 / 107.  One tensor over and over: 768 x 256 1.76 / 1.78 / 1.74, 768 x 768 1.95 / 1.95 / 1.96, 1024 x 1024 2.5 / 2.5 / 2.6, 2304 x 768
+// 2.82 / 3.18 / 2.98, 3072 x 768 2.85 / 3.36 / 3.10, 3072 x 1024 3.73 / 4.59 / 4.10, 4096 x 1024 4.48 / 5.36 / 4.69, 4096 x 2048 8.1 / 9.9 / 8.4.
+Ahead decay_ahead(int64_t n, int mask_itemsize, const void *mask) {
+    const int64_t blocks = n / 4096, few = 2 * (int64_t)sm_count();
+    const int whole_mask = aligned16(mask);
+    if (blocks <= few || n * (8 + mask_itemsize) > 96 << 20) return {blocks, 1, whole_mask};
+    return {std::min(blocks, few / 2 * 5), 0, whole_mask};
+}
+
 template <int MS>
 __global__ void __launch_bounds__(256) masked_add_kernel(float *grad, const float *p, const void *mask, int64_t n,
-                                                         float alpha) {
+                                                         float alpha, Ahead ahead) {
     constexpr int UNR = 4;
     const int64_t n4 = n / 4;
-    // The block's 36 KB (one mask byte an element) are under way from DRAM before the kernel before has ended: a model's 48 weights are as many
-    // launches of 1 - 5 us, each of which began with an idle DRAM.  us a replayed launch over tensors larger than L2, without -> with: n
-    // 768 x 768 3.1 -> 2.5 (its bytes 1.2), 2304 x 768 5.3 -> 4.2 (3.5), 3072 x 768 6.3 -> 5.1 (4.7), 4096 x 4096 32.4 -> 30.8; the 48
-    // weights of GPT-2 249 -> 207 (169).  One tensor over and over, all of it in L2: 1.9 -> 2.0, 3.1 -> 3.5, 3.1 -> 3.6, 30.2 -> 30.0.  One
-    // request of the copy engine an array and block instead: 214.
-    const int64_t first = (int64_t)blockIdx.x * (256 * UNR), pieces = min((int64_t)(256 * UNR), n4 - first);      // of four elements
-    const int line = (threadIdx.x & 127) * 8, mask_line = threadIdx.x * (32 / MS);                                  // of 128 bytes
-    if (line < pieces) prefetch_l2((threadIdx.x < 128 ? grad : p) + 4 * (first + line));
-    if (mask_line < pieces) prefetch_l2(static_cast<const uint8_t *>(mask) + 4 * MS * (first + mask_line));
+    if (threadIdx.x == 0 && blockIdx.x < ahead.blocks) {
+        const int64_t first = (int64_t)blockIdx.x * (1024 * UNR);
+        if (ahead.grad) prefetch_l2(grad + first, 4096 * UNR);
+        prefetch_l2(p + first, 4096 * UNR);
+        if (ahead.mask) prefetch_l2(static_cast<const uint8_t *>(mask) + MS * first, 1024 * UNR * MS);
+    }
     chain_enter();
     const int64_t base = (int64_t)blockIdx.x * (256 * UNR) + threadIdx.x;
-    float4 g[UNR], q[UNR];
-    uint32_t keep[UNR];
+    // whole blocks without a condition on any load: a load behind a branch waits for those before it (48 weights 768 wide: 235 us instead of 195)
+    auto pass = [&](auto whole) {
+        constexpr bool WHOLE = decltype(whole)::value;
+        float4 g[UNR], q[UNR];
+        uint32_t keep[UNR];
 #pragma unroll
-    for (int j = 0; j < UNR; ++j) {
-        const int64_t i = base + j * 256;
-        if (i < n4) {
-            keep[j] = load_keep4<MS>(mask, i * 4);
-            g[j] = reinterpret_cast<const float4 *>(grad)[i];
-            q[j] = reinterpret_cast<const float4 *>(p)[i];
+        for (int j = 0; j < UNR; ++j) {
+            const int64_t i = base + j * 256;
+            if (WHOLE || i < n4) {
+                keep[j] = load_keep4<MS>(mask, i * 4);
+                g[j] = reinterpret_cast<const float4 *>(grad)[i];
+                q[j] = reinterpret_cast<const float4 *>(p)[i];
+            }
         }
-    }
 #pragma unroll
-    for (int j = 0; j < UNR; ++j) {
-        const int64_t i = base + j * 256;
-        if (i < n4 && keep[j] != 0xFu) {
-            if (!(keep[j] & 1u)) g[j].x = __fadd_rn(g[j].x, __fmul_rn(q[j].x, alpha));
-            if (!(keep[j] & 2u)) g[j].y = __fadd_rn(g[j].y, __fmul_rn(q[j].y, alpha));
-            if (!(keep[j] & 4u)) g[j].z = __fadd_rn(g[j].z, __fmul_rn(q[j].z, alpha));
-            if (!(keep[j] & 8u)) g[j].w = __fadd_rn(g[j].w, __fmul_rn(q[j].w, alpha));
-            reinterpret_cast<float4 *>(grad)[i] = g[j];
+        for (int j = 0; j < UNR; ++j) {
+            const int64_t i = base + j * 256;
+            if ((WHOLE || i < n4) && keep[j] != 0xFu) {
+                if (!(keep[j] & 1u)) g[j].x = __fadd_rn(g[j].x, __fmul_rn(q[j].x, alpha));
+                if (!(keep[j] & 2u)) g[j].y = __fadd_rn(g[j].y, __fmul_rn(q[j].y, alpha));
+                if (!(keep[j] & 4u)) g[j].z = __fadd_rn(g[j].z, __fmul_rn(q[j].z, alpha));
+                if (!(keep[j] & 8u)) g[j].w = __fadd_rn(g[j].w, __fmul_rn(q[j].w, alpha));
+                reinterpret_cast<float4 *>(grad)[i] = g[j];
+            }
         }
-    }
+    };
+    if (((int64_t)blockIdx.x + 1) * (256 * UNR) <= n4) pass(std::true_type{});
+    else pass(std::false_type{});
     // ragged tail (n not a multiple of 4): handled by the first threads of block 0
     if (blockIdx.x == 0 && threadIdx.x < (int)(n - n4 * 4)) {
         const int64_t i = n4 * 4 + threadIdx.x;
@@ -415,9 +439,10 @@ extern "C" int sp24_masked_add(void *grad, const void *p, const void *mask, int 
     const unsigned blocks = (unsigned)((n4 + 1023) / 1024 > 0 ? (n4 + 1023) / 1024 : 1);
     float *g = static_cast<float *>(grad);
     const float *q = static_cast<const float *>(p);
-    if (mask_itemsize == 1) launch_chained(st, masked_add_kernel<1>, blocks, 256, 0, g, q, mask, n, alpha);
-    else if (mask_itemsize == 2) launch_chained(st, masked_add_kernel<2>, blocks, 256, 0, g, q, mask, n, alpha);
-    else launch_chained(st, masked_add_kernel<4>, blocks, 256, 0, g, q, mask, n, alpha);
+    const Ahead ahead = decay_ahead(n, mask_itemsize, mask);
+    if (mask_itemsize == 1) launch_chained(st, masked_add_kernel<1>, blocks, 256, 0, g, q, mask, n, alpha, ahead);
+    else if (mask_itemsize == 2) launch_chained(st, masked_add_kernel<2>, blocks, 256, 0, g, q, mask, n, alpha, ahead);
+    else launch_chained(st, masked_add_kernel<4>, blocks, 256, 0, g, q, mask, n, alpha, ahead);
     return launch_status();
 }
 

@@ -436,9 +436,11 @@ __device__ __forceinline__ void chain_enter() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
-// Asks L2 for the line of an address.  No value is read: the one access that may come before chain_enter, since what the kernel before still
-// writes arrives in L2 as well.
-__device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+// Asks L2 for `bytes` at p (both multiples of 16, more than none).  No value is read: the one access that may come before chain_enter, since what
+// the kernel before still writes arrives in L2 as well.
+__device__ __forceinline__ void prefetch_l2(const void *p, uint32_t bytes) {
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
 // Errors are left for launch_status, as with a <<<>>> launch.
 template <typename... P, typename... A>
 inline void launch_chained(cudaStream_t st, void (*kern)(P...), dim3 grid, unsigned threads, size_t smem, A &&...args) {

@@ -24,3 +24,10 @@ def test_decays_in_a_row(n, mask_dtype):
         ra = torch.where(keep != 0, ra, ra + rb * (0.5 + i))
         rb = torch.where(keep != 0, rb, rb + ra * -0.25)
     assert torch.equal(a, ra) and torch.equal(b, rb)
+
+
+@pytest.mark.parametrize("mask_dtype", [torch.bool, torch.float32])
+@pytest.mark.parametrize("blocks", [296, 297, 740, 741, 2100, 2800])
+def test_decays_whose_blocks_ask_ahead_or_not(blocks, mask_dtype):
+    """Either side of two and of five blocks an SM, and of what L2 holds of the three arrays (float32 masks: from 2049 blocks, bool from 2731)."""
+    test_decays_in_a_row(blocks * 4096 - 2048 + 7, mask_dtype)
