@@ -68,7 +68,7 @@ extern "C" const char *sp24_strerror(int code) {
     }
 }
 
-extern "C" int sp24_abi_version(void) { return 2; }
+extern "C" int sp24_abi_version(void) { return SP24_ABI_VERSION; }
 
 namespace sp24 {
 namespace {

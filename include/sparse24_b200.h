@@ -62,7 +62,12 @@ enum {
 /* Human-readable text for an error code (static storage). */
 const char *sp24_strerror(int code);
 
-/* ABI version of the loaded library (bumped when a signature changes). */
+/*
+ * ABI version of the loaded library, raised when a signature or the meaning of an argument changes.
+ *   3: row_parts of float8 results hold one part for every 128 k, as those of 16-bit ones, where version 2 had one for every 256
+ *      (sp24_row_parts): a buffer of half the parts is written past its end.
+ */
+#define SP24_ABI_VERSION 3
 int sp24_abi_version(void);
 
 /* Zero `bytes` bytes of device memory on `stream` (an output that a following kernel adds to).  Any memory that cudaMemsetAsync takes. */
@@ -175,8 +180,8 @@ int sp24_dual_compress_f8(const void *w, int dtype, int64_t m, int64_t k, int64_
  * sp24_prune_compress with all extras, each of which may be NULL; offset_dev, e_tc, amax and q_dense as in the two entry points
  * above.  packed_row_major: float8 results of column-major input leave row-major, as sp24_prune_compress_q8 writes them (q_dense
  * asks for it).  out_scale: float8 without amax, as for sp24_prune_compress_q8 (0: none).  row_parts instead of row_sums:
- * float32 (sp24_row_parts(k, packed_dtype), m), partial sums over 128 consecutive k of the unpruned
- * dense[r, k], column-major storage only.  sp24_sum_parts adds them up in a fixed order (accumulate = 1: to what out holds),
+ * float32 (sp24_row_parts(k, packed_dtype), m), a partial sum for every 128 consecutive k, whatever the type (see
+ * SP24_ABI_VERSION), of the unpruned dense[r, k], column-major storage only.  sp24_sum_parts adds them up in a fixed order (accumulate = 1: to what out holds),
  * so that the same gradient gives the same bits every time, which row_sums' atomics do not promise.
  */
 typedef struct sp24_prune_extras {
@@ -189,7 +194,7 @@ typedef struct sp24_prune_extras {
     int packed_row_major;
     float out_scale;
 } sp24_prune_extras;
-int sp24_row_parts(int64_t k, int packed_dtype);
+int sp24_row_parts(int64_t k, int packed_dtype);       /* (k + 127) / 128 for 8- and 16-bit types, 0 for others */
 int sp24_prune_compress_with(const void *dense, int dense_dtype, int64_t m, int64_t k, int64_t ld_dense, int col_major, void *packed,
                              int packed_dtype, int64_t ld_packed, void *meta, int mode, const void *mask, int64_t ld_mask,
                              const float *uniforms, int64_t ld_uniforms, uint64_t seed, uint64_t offset, const sp24_prune_extras *extras,

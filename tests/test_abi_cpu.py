@@ -179,3 +179,11 @@ def test_missing_library_fails_loudly(monkeypatch):
     monkeypatch.setattr(_ext, "LIB_PATH", "/nonexistent/libsparse24_b200.so")
     with pytest.raises(RuntimeError, match="no CPU or Triton fallback"):
         _ext.lib()
+
+
+def test_row_parts_and_the_version_that_says_so(lib):
+    """Float8 results have as many parts as 16-bit ones from version 3 on: a caller that reckons with version 2 can tell."""
+    assert lib.sp24_abi_version() == int(re.search(r"#define SP24_ABI_VERSION (\d+)", open(HEADER).read()).group(1)) >= 3
+    for dtype in range(1, 6):
+        assert [lib.sp24_row_parts(k, dtype) for k in (64, 128, 192, 256, 4224)] == [1, 1, 2, 2, 33]
+    assert lib.sp24_row_parts(256, 0) == lib.sp24_row_parts(256, 6) == 0
