@@ -2074,11 +2074,20 @@ void pick_f8_tile(int64_t ms, int64_t n, int sms, int &bn, int &mpt) {
 }
 
 // Whether the CTA-pair kernel takes an operand of whole or half 256-row blocks.  A half-empty last block costs its MMAs, not its stores, and
-// over a map of 9 odd row counts (128 .. 2944), 12 widths (384 .. 16384) and K from 128 to 3072 pairs are faster or alike, except where
-// the one block there is is half empty and many tiles are to be written: ms 128, n 16384, k 128 single CTAs 5.1, pairs 5.8; k 3072 19.6 / 20.5;
-// n 8192 5.3 / 5.5.  Elsewhere in fp16 up to 6 % slower at 5 of 972 sizes (384 x 6000, k 128 5.1 / 5.4) and up to 35 % faster at 211 that
-// an earlier rule left to single CTAs, us: 1152 x 12000, k 256 16.6 / 12.6; 384 x 12000, k 512 10.3 / 8.0; float8 384 x 12000, k 384 11.7 / 7.6.
-bool pair_takes_rows(int64_t ms, int64_t n) { return ms > BM || n <= 8192; }
+// over a map of 9 odd row counts (128 .. 2944), 12 widths (384 .. 16384) and K from 128 to 3072 pairs are faster or alike, us, single CTAs /
+// pairs: 1152 x 12000, k 256 16.3 / 12.2; 384 x 12000, k 512 10.3 / 8.0; float8 384 x 12000, k 384 11.7 / 7.6.  Two exceptions.  The one
+// block there is is half empty and many tiles are to be written: ms 128, n 16384, k 128 5.1 / 5.8, k 3072 19.6 / 20.5; n 8192 5.3 / 5.5.
+// And 16-bit operands of one whole K step whose 128 x 128 tiles fill one round of single CTAs by two thirds or more: n * ms of 1.6 to 2.4
+// million, over 9 odd row counts 0 - 12 % slower on pairs, e.g. 384 x 6000 4.3 / 4.8, 896 x 2510 4.29 / 4.64, 2176 x 1011 4.22 / 4.45;
+// with fewer tiles or a second round pairs gain again (384 x 2395 4.13 / 3.97, 896 x 2790 4.96 / 4.70).
+bool pair_takes_rows(int64_t ms, int64_t n, int64_t k, bool f8, int sms) {
+    if (ms % 256 == 0) return true;
+    if (!f8 && k == 128) {
+        const int64_t tiles = (ms / BM) * ((n + 127) / 128);
+        if (tiles <= sms && 3 * tiles >= 2 * sms) return false;
+    }
+    return ms > BM || n <= 8192;
+}
 
 // Row blocks of a tile and K slices of the 16-bit weight gradient on single CTAs.
 int single_row_blocks(int64_t ms) { return ms >= 256 ? 2 : 1; }
@@ -2209,7 +2218,7 @@ static int spmm_impl(const void *a_packed, int dtype, int a_mn_major, int64_t ld
               ((uint32_t)(b_mn_major ? 1 : 0) << 16) | ((uint32_t)(BM >> 4) << 24);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int sms = sm_count_cached();
-    bool pair_form = pair_layout && pair_takes_rows(ms, n) && pair_kernels_enabled();
+    bool pair_form = pair_layout && pair_takes_rows(ms, n, k, false, sms) && pair_kernels_enabled();
     if (epi != EPI_PLAIN || bias_f32) pair_form = true;      // checked above: these forms exist in the pair kernel only
     if (a_mn_major) rc = pair_form ? make_map_columns(&map_a, a_packed, dtype, k / 2, ms, ld_a, 64) : make_map(&map_a, a_packed, dtype, k / 2, ms, ld_a, 64, 64);
     else rc = make_map(&map_a, a_packed, dtype, ms, k / 2, ld_a, f8 ? 128 : 64, 128);
@@ -2324,7 +2333,7 @@ static int spmm_f8_impl(const void *a_packed, int dtype, int64_t ld_a, const voi
     P.idesc = (1u << 2) | (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(BM >> 4) << 24);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int sms = sm_count_cached();
-    if (trans_out && out_dtype != SP24_F32 && pair_takes_rows(ms, n) && pair_kernels_enabled()) {
+    if (trans_out && out_dtype != SP24_F32 && pair_takes_rows(ms, n, k, true, sms) && pair_kernels_enabled()) {
         CUtensorMap map_e;
         P.bn = pick_pair_bn(ms, n, true, true, sms);
         if (int rc = make_map_columns(&map_b, b, dtype, n, k, ld_b, (uint32_t)P.bn / 2)) return rc;

@@ -50,6 +50,14 @@ def test_products_of_more_tiles_than_pairs(ms, n, k, col):
     test_products(ms, n, k, col, torch.float16)
 
 
+@pytest.mark.parametrize("dtype", list(ROUND), ids=["f16", "bf16"])
+@pytest.mark.parametrize("col", [False, True])
+@pytest.mark.parametrize("ms,n", [(384, 4096), (384, 4097), (384, 6272), (384, 6273), (1152, 2048), (1152, 2049)])
+def test_products_of_one_k_step(ms, n, col, dtype):
+    """96 and 99, 147 and 150, 144 and 153 tiles of 128 x 128: either side of what single CTAs take in one round of 148."""
+    test_products(ms, n, 128, col, dtype)
+
+
 @pytest.mark.parametrize("ms,n,k,splits", [(128, 256, 192, 0), (384, 264, 1088, 3), (1152, 1152, 1984, 0), (384, 520, 1024, 0), (640, 264, 1088, 0), (384, 264, 64, 5)])
 @pytest.mark.parametrize("col", [False, True])
 def test_weight_gradient(ms, n, k, splits, col):
