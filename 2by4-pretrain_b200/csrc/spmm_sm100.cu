@@ -1569,7 +1569,8 @@ spmm_pair_acc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                         tma_load_columns_pair(sa, &map_a, it * 64, mrow / 64, full_leader);
                     }
                     tma_load_2d_pair(sa + OFF_E, &map_e, 0, (int)(((int64_t)mblk * P.k_atoms + it * (F8 ? 2 : 1)) * 2), full_leader);
-                    // this CTA's 128 columns of B: two boxes of 64 columns x 128 K-rows, or of 128 columns x 128 bytes of K
+                    // this CTA's 128 columns of B, 32 KB: one request for two columns of 128 bytes (float8: of K; 16 bits: 64 columns x 128
+                    // K-rows each), two where the operand's columns are not whole ones (see make_map_columns)
                     if constexpr (F8) {
                         tma_load_columns_pair(sb, &map_b, bcol, 2 * it, full_leader);
                     } else if (P.whole_columns) {
